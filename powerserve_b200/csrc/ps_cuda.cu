@@ -68,7 +68,7 @@ struct LayerDev {
     // octet-interleaved copies for the row-walker mat-vec (ps_rw.cuh): q|k|v rows, o, gate|up slots, down
     uint8_t *rw_qkv = nullptr, *rw_o = nullptr, *rw_gu = nullptr, *rw_down = nullptr;
     // fp16-expanded tensor-core operands for the prefill GEMM (ps_tc.cuh): q|k|v rows, o, gate, up, down
-    uint8_t *tc_qkv = nullptr, *tc_o = nullptr, *tc_gate = nullptr, *tc_up = nullptr, *tc_down = nullptr;
+    uint8_t *tc_qkv = nullptr, *tc_o = nullptr, *tc_gu = nullptr, *tc_down = nullptr; // packed blocks of the tcgen05 GEMM (gate rows, then up rows from the next tile border)
     // octet copies for the 32-block mat-vec (ps_mv32.cuh; all-Q4_0 / all-Q8_0 models): q|k|v rows, o, gate|up rows, down
     uint8_t *mv_qkv = nullptr, *mv_o = nullptr, *mv_gu = nullptr, *mv_down = nullptr;
 };
@@ -127,7 +127,9 @@ struct ps_cuda_ctx {
     int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_scores_batch_min = 2;
     bool tc_ok = false;        // tensor-core prefill operands are resident
     uint8_t *tc_b = nullptr;   // B operand blocks of the current activation batch
-    size_t tc_b_bytes = 0;
+    float *tc_part = nullptr;  // pass groups' numbers of the tiles in flight
+    size_t tc_part_bytes = 0;
+    int *tc_cnt = nullptr;     // per tile: pass groups that have finished
     int *err_dev = nullptr;    // device-detected failures, [0] tcgen05 pipeline time-out, [1] peer wait gave up, [2] step-kernel barrier time-out
     int err_seen[3] = {};      // sticky host copy of the flags (counters "tc_error" / "tp_error" / "step_error")
     int *h_err = nullptr;      // pinned mirror, read after every forward / decode (a set flag becomes PS_CUDA_ERR_CUDA)
@@ -138,7 +140,7 @@ struct ps_cuda_ctx {
     double kt_ms = 0.0;                 // summed mat-vec kernel time of the last decode call
     int64_t kt_launches = 0;
     uint8_t *rw_out = nullptr; // lm_head, octet-interleaved
-    uint8_t *tc_out = nullptr; // lm_head, fp16-expanded tensor-core operand (batches of 16+ columns that want logits: session batches, verify batches)
+    uint8_t *tc_out = nullptr; // lm_head, packed for the tcgen05 GEMM (batches that want logits: session batches, verify batches)
     bool fused_ok = false;   // every matmul weight (and the embedding) is Q4_K: the fused decode path applies
     int opt_attn_group = 0;  // opt-in: decode attention as ONE group-synchronised kernel per layer (ps_k_attn_group); bit-exact, but 23 us vs 11.7 us per layer at ctx 2048
     unsigned long long *ag_ctr = nullptr; // [n_layers][n_kv_heads] arrival counters of the kv-head groups
@@ -703,6 +705,89 @@ int rwm_single(ps_cuda_ctx *ctx, const uint8_t *w, int n_rows, int K, int slot, 
     a.seg[0] = {dst, bias, 0, n_rows, 0};
     a.residual = residual;
     return launch_rwm(ctx, a);
+}
+
+// ---- tcgen05 GEMM of token batches (ps_tc.cuh)
+constexpr int TC_CNT = 16384;                        // tiles whose pass groups run as separate units
+constexpr size_t TC_PART_MAX = (size_t)96 << 20;
+int64_t tc_tiles(int64_t rows) { return (rows + PS_TC_M - 1) / PS_TC_M; }
+int64_t tc_nbp(int64_t K) { return (K / 256 + 1) & ~(int64_t)1; } // super-blocks, rounded up to whole steps
+size_t tc_a_bytes(int64_t rows, int64_t K) { return (size_t)tc_tiles(rows) * (size_t)tc_nbp(K) * PS_TC_A_BLOCK; }
+int tc_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t n_rows, int64_t K, int64_t tile0) {
+    ps_k_tc_pack_a<<<dim3((unsigned)tc_nbp(K), (unsigned)tc_tiles(n_rows)), 256, 0, ctx->stream>>>(dst, w, n_rows, K / 256, tile0);
+    PS_LAUNCH_CK();
+    return 0;
+}
+// column-tile width of a batch: the fewest padded columns, counting a tile's own cost (its weights are de-quantised once per tile, about
+// the work of 40 columns)
+int tc_width(int bs) {
+    int best = 128;
+    int64_t cost = INT64_MAX;
+    for (int nt : {128, 96, 64, 32, 16}) {
+        const int64_t c = (int64_t)((bs + nt - 1) / nt) * (nt + 40);
+        if (c < cost) { cost = c; best = nt; }
+    }
+    return best;
+}
+int tc_prep_b(ps_cuda_ctx *ctx, const float *x, int K, int bs) {
+    const int nt = tc_width(bs), n_ct = (bs + nt - 1) / nt;
+    ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x, K, bs, nt);
+    PS_LAUNCH_CK();
+    return 0;
+}
+template <int NT> int tc_launch(ps_cuda_ctx *ctx, PsTcArgs &a) {
+    static bool attr[64] = {};
+    if (!attr[ctx->device]) {
+        PS_CK(cudaFuncSetAttribute(ps_k_tc_gemm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PsTc<NT>::SMEM));
+        attr[ctx->device] = true;
+    }
+    // passes per unit: fewer passes cover the GPU with a small matrix and even out the last wave, more save the hand-over of a tile's numbers
+    // (a unit that hands over costs about four steps more: its 128 x NT floats go through L2 and the tile's last unit reads all of them)
+    int64_t best = INT64_MAX;
+    const int slots = ctx->n_sm * PsTc<NT>::CTAS;
+    for (int pp : {6, 2, 1}) {
+        const int64_t units = (int64_t)a.n_tiles * (PS_TC_PASSES / pp), rounds = (units + slots - 1) / slots;
+        if (pp < 6 && (a.n_tiles > TC_CNT || (size_t)units * PS_TC_M * NT * 4 > ctx->tc_part_bytes)) continue;
+        const int64_t cost = rounds * ((int64_t)pp * a.nbp + (pp < 6 ? 4 : 0));
+        if (cost < best) { best = cost; a.pp = pp; }
+    }
+    const int units = a.n_tiles * (PS_TC_PASSES / a.pp);
+    ps_k_tc_gemm<NT><<<(unsigned)std::min(units, slots), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
+    PS_LAUNCH_CK();
+    return 0;
+}
+// segments give their rows in the padded row space of the packed matrix (tile borders between them)
+int tc_gemm(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int64_t n_tiles, int64_t K, int bs, const PsRwSeg *segs, int n_seg, const float *residual) {
+    PsTcArgs a{};
+    const int nt = tc_width(bs);
+    a.err = ctx->tc_err_dev;
+    a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = (bs + nt - 1) / nt; a.n_tiles = (int)n_tiles * a.n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
+    a.part = ctx->tc_part; a.cnt = ctx->tc_cnt;
+    for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
+    ctx->n_tc++;
+    switch (nt) {
+    case 128: return tc_launch<128>(ctx, a);
+    case 96: return tc_launch<96>(ctx, a);
+    case 64: return tc_launch<64>(ctx, a);
+    case 32: return tc_launch<32>(ctx, a);
+    default: return tc_launch<16>(ctx, a);
+    }
+}
+int tc_single(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int64_t n_rows, int64_t K, float *dst, int bs, const float *residual) {
+    PsRwSeg sg = {dst, nullptr, 0, (int)n_rows, 0};
+    return tc_gemm(ctx, a_blocks, tc_tiles(n_rows), K, bs, &sg, 1, residual);
+}
+int tc_qkv(ps_cuda_ctx *ctx, const LayerDev &ld, int64_t q_rows, int64_t kv_rows, int64_t K, int bs) {
+    const bool bias = ctx->d.qkv_bias != 0;
+    const int k0 = (int)tc_tiles(q_rows) * PS_TC_M, v0 = k0 + (int)tc_tiles(kv_rows) * PS_TC_M;
+    const PsRwSeg sg[3] = {{ctx->q, bias ? ld.q_bias : nullptr, 0, (int)q_rows, 0}, {ctx->k, bias ? ld.k_bias : nullptr, k0, k0 + (int)kv_rows, 0},
+                           {ctx->v, bias ? ld.v_bias : nullptr, v0, v0 + (int)kv_rows, 0}};
+    return tc_gemm(ctx, ld.tc_qkv, tc_tiles(q_rows) + 2 * tc_tiles(kv_rows), K, bs, sg, 3, nullptr);
+}
+int tc_gate_up(ps_cuda_ctx *ctx, const LayerDev &ld, int64_t rows, int64_t K, int bs) {
+    const int u0 = (int)tc_tiles(rows) * PS_TC_M;
+    const PsRwSeg sg[2] = {{ctx->g, nullptr, 0, (int)rows, 0}, {ctx->u, nullptr, u0, u0 + (int)rows, 0}};
+    return tc_gemm(ctx, ld.tc_gu, 2 * tc_tiles(rows), K, bs, sg, 2, nullptr);
 }
 
 // one decode step on the token in tokens_dev[0] at position pos_dev[0]; `pick`: run
@@ -1743,39 +1828,6 @@ float *ps_cuda_kv_v(ps_cuda_ctx *ctx, int layer) { return (layer >= 0 && layer <
 
 // ---------------------------------------------------------------------------------------------- whole model
 // ---- tcgen05 prefill GEMM (ps_tc.cuh)
-static int tc_expand(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t n_rows, int64_t K, int64_t tile0) {
-    ps_k_tc_expand_a<<<dim3((unsigned)(K / 256), (unsigned)((n_rows + PS_TC_M - 1) / PS_TC_M)), 256, 0, ctx->stream>>>(dst, w, n_rows, K / 256, tile0);
-    PS_LAUNCH_CK();
-    return 0;
-}
-static int tc_prep_b(ps_cuda_ctx *ctx, const float *x, int K, int bs) {
-    const int n_cg = (bs + PS_TC_N - 1) / PS_TC_N;
-    ps_k_tc_prep_b<<<dim3((unsigned)((K / 256 + 3) / 4), (unsigned)(n_cg * PS_TC_N)), 128, 0, ctx->stream>>>(ctx->tc_b, x, K, bs);
-    PS_LAUNCH_CK();
-    return 0;
-}
-static int tc_gemm(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int n_rows, int K, int bs, const PsRwSeg *segs, int n_seg, const float *residual) {
-    static bool attr[64] = {};
-    if (!attr[ctx->device]) {
-        PS_CK(cudaFuncSetAttribute(ps_k_tc_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, PS_TC_STAGES * PS_TC_STAGE));
-        attr[ctx->device] = true;
-    }
-    PsTcArgs a{};
-    a.err = ctx->tc_err_dev;
-    a.a = a_blocks; a.b = ctx->tc_b; a.nb = K / 256; a.n_cg = (bs + PS_TC_N - 1) / PS_TC_N; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
-    for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
-    const int n_tiles = (n_rows + PS_TC_M - 1) / PS_TC_M;
-    a.n_units = n_tiles * a.n_cg;
-    ps_k_tc_gemm<<<(unsigned)std::min(a.n_units, ctx->n_sm), PS_TC_THREADS, PS_TC_STAGES * PS_TC_STAGE, ctx->stream>>>(a);
-    PS_LAUNCH_CK();
-    ctx->n_tc++;
-    return 0;
-}
-static int tc_single(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int n_rows, int K, float *dst, int bs, const float *residual) {
-    PsRwSeg sg = {dst, nullptr, 0, n_rows, 0};
-    return tc_gemm(ctx, a_blocks, n_rows, K, bs, &sg, 1, residual);
-}
-
 int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
     PS_NO_ARCH("ps_cuda_bind_model");
     const ps_cuda_model_desc &d = ctx->d;
@@ -1898,36 +1950,37 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
             if ((rc = rw_repack(ctx, ld.rw_gu, ld.wup, ffn_l, dim, 0, 1, 2))) return rc;
             if ((rc = rw_repack(ctx, ld.rw_down, ld.wdown, dim_l, ffn, 0, 0, 1))) return rc;
         }
-        // fp16-expanded tensor-core operands for the prefill GEMM (2 B / weight of this rank's rows; only if HBM has room)
+        // packed blocks of the batch GEMM (1.11x the GGUF bytes of this rank's rows; only if HBM has room)
         ctx->tc_ok = false;
-        if (ctx->opt_tc && qdim_l % PS_TC_M == 0 && kvd_l % PS_TC_M == 0) {
-            auto a_bytes = [](int64_t rows, int64_t K) { return (size_t)((rows + PS_TC_M - 1) / PS_TC_M) * (size_t)(K / 256) * PS_TC_A_BLOCK; };
-            const size_t per_layer = a_bytes(qdim_l + 2 * kvd_l, dim) + a_bytes(dim_l, qdim) + 2 * a_bytes(ffn_l, dim) + a_bytes(dim_l, ffn);
+        if (ctx->opt_tc) {
+            const size_t per_layer = tc_a_bytes(qdim_l, dim) + 2 * tc_a_bytes(kvd_l, dim) + tc_a_bytes(dim_l, qdim) + 2 * tc_a_bytes(ffn_l, dim) + tc_a_bytes(dim_l, ffn);
             size_t free_b = 0, total_b = 0;
             PS_CK(cudaMemGetInfo(&free_b, &total_b));
             if (per_layer * (size_t)d.n_layers + ((size_t)8 << 30) < free_b) {
                 for (LayerDev &ld : ctx->layers) {
-                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_qkv, a_bytes(qdim_l + 2 * kvd_l, dim)))) return rc;
-                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_o, a_bytes(dim_l, qdim)))) return rc;
-                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_gate, a_bytes(ffn_l, dim)))) return rc;
-                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_up, a_bytes(ffn_l, dim)))) return rc;
-                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_down, a_bytes(dim_l, ffn)))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_qkv, ld.wq, qdim_l, dim, 0))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_qkv, ld.wk, kvd_l, dim, qdim_l / PS_TC_M))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_qkv, ld.wv, kvd_l, dim, (qdim_l + kvd_l) / PS_TC_M))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_o, ld.wo, dim_l, qdim, 0))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_gate, ld.wgate, ffn_l, dim, 0))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_up, ld.wup, ffn_l, dim, 0))) return rc;
-                    if ((rc = tc_expand(ctx, ld.tc_down, ld.wdown, dim_l, ffn, 0))) return rc;
+                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_qkv, tc_a_bytes(qdim_l, dim) + 2 * tc_a_bytes(kvd_l, dim)))) return rc;
+                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_o, tc_a_bytes(dim_l, qdim)))) return rc;
+                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_gu, 2 * tc_a_bytes(ffn_l, dim)))) return rc;
+                    if ((rc = dev_alloc(ctx, (void **)&ld.tc_down, tc_a_bytes(dim_l, ffn)))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_qkv, ld.wq, qdim_l, dim, 0))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_qkv, ld.wk, kvd_l, dim, tc_tiles(qdim_l)))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_qkv, ld.wv, kvd_l, dim, tc_tiles(qdim_l) + tc_tiles(kvd_l)))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_o, ld.wo, dim_l, qdim, 0))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_gu, ld.wgate, ffn_l, dim, 0))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_gu, ld.wup, ffn_l, dim, tc_tiles(ffn_l)))) return rc;
+                    if ((rc = tc_pack(ctx, ld.tc_down, ld.wdown, dim_l, ffn, 0))) return rc;
                 }
-                const size_t bb = (size_t)((d.max_batch + PS_TC_N - 1) / PS_TC_N) * (size_t)(ctx->maxK / 256) * PS_TC_B_BLOCK;
-                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_b, bb))) return rc;
-                PS_CK(cudaMemsetAsync(ctx->tc_b, 0, bb, ctx->stream)); // the mins tiles are zero outside each lane's four K positions
-                ctx->tc_b_bytes = bb;
+                const size_t cols = (size_t)(d.max_batch + 127) / 128 * 128; // no choice of tc_width pads a batch further
+                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_b, cols * (size_t)tc_nbp(ctx->maxK) * 644))) return rc;
+                const int64_t rows = std::max(std::max(tc_tiles(qdim_l) + 2 * tc_tiles(kvd_l), 2 * tc_tiles(ffn_l)), std::max(tc_tiles(dim_l), tc_tiles(vocab_l))) * PS_TC_M;
+                ctx->tc_part_bytes = std::max(std::min(TC_PART_MAX, (size_t)rows * cols * 4 * PS_TC_PASSES), (size_t)ctx->n_sm * PS_TC_M * 128 * 4);
+                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_part, ctx->tc_part_bytes))) return rc;
+                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_cnt, TC_CNT * 4))) return rc;
+                PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, TC_CNT * 4, ctx->stream));
                 ctx->tc_ok = true;
-                if (tp == 1 && a_bytes(vocab_l, dim) + ((size_t)8 << 30) < free_b - per_layer * (size_t)d.n_layers) { // lm_head too (1 GB for the 8B model)
-                    if ((rc = dev_alloc(ctx, (void **)&ctx->tc_out, a_bytes(vocab_l, dim)))) return rc;
-                    if ((rc = tc_expand(ctx, ctx->tc_out, ctx->w_out, vocab_l, dim, 0))) return rc;
+                if (tp == 1 && tc_a_bytes(vocab_l, dim) + ((size_t)8 << 30) < free_b - per_layer * (size_t)d.n_layers) { // lm_head too
+                    if ((rc = dev_alloc(ctx, (void **)&ctx->tc_out, tc_a_bytes(vocab_l, dim)))) return rc;
+                    if ((rc = tc_pack(ctx, ctx->tc_out, ctx->w_out, vocab_l, dim, 0))) return rc;
                 }
             }
         }
@@ -2006,7 +2059,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     const bool tree = tree_base >= 0;
     const int64_t n_kv = sess ? (int64_t)sess->n_kv_max : tree ? (int64_t)tree_base + bs : (int64_t)pos0 + bs; // pos.back() + 1 (session batch: the longest row)
     const float kq_scale = 1.0f / sqrtf((float)hs);
-    const bool tc = ctx->tc_ok && ctx->opt_tc && ctx->opt_fused && bs >= ctx->opt_tc_min; // tensor-core GEMM on the fp16-expanded operands
+    const bool tc = ctx->tc_ok && ctx->opt_tc && ctx->opt_fused && bs >= ctx->opt_tc_min; // tensor-core GEMM on the packed blocks
     const bool rw = ctx->fused_ok && ctx->opt_fused && (bs > 1 || tree); // octet-interleaved copies exist: multi-column row-walker
     int rc;
     ps_k_get_embedding<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
@@ -2023,10 +2076,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         PS_LAUNCH_CK();
         if (tc) {
             if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            PsRwSeg sg[3] = {{ctx->q, d.qkv_bias ? ld.q_bias : nullptr, 0, (int)qdim, 0},
-                             {ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)qdim, (int)(qdim + kvd), 0},
-                             {ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)(qdim + kvd), (int)(qdim + 2 * kvd), 0}};
-            if ((rc = tc_gemm(ctx, ld.tc_qkv, (int)(qdim + 2 * kvd), (int)dim, bs, sg, 3, nullptr))) return rc;
+            if ((rc = tc_qkv(ctx, ld, qdim, kvd, dim, bs))) return rc;
         } else if (rw) { // q | k | v rows in one pass over the concatenated octets
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             PsRwmArgs a{};
@@ -2087,8 +2137,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         PS_LAUNCH_CK();
         if (tc) {
             if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_gate, (int)ffn, (int)dim, ctx->g, bs, nullptr))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_up, (int)ffn, (int)dim, ctx->u, bs, nullptr))) return rc;
+            if ((rc = tc_gate_up(ctx, ld, ffn, dim, bs))) return rc;
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;
@@ -2187,7 +2236,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
                          {ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)(qdim_l + kvd), (int)(qdim_l + 2 * kvd), 0}};
         if (tc) {
             if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_gemm(ctx, ld.tc_qkv, (int)(qdim_l + 2 * kvd), (int)dim, bs, sg, 3, nullptr))) return rc;
+            if ((rc = tc_qkv(ctx, ld, qdim_l, kvd, dim, bs))) return rc;
         } else {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             PsRwmArgs a{};
@@ -2220,8 +2269,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         PS_LAUNCH_CK();
         if (tc) {
             if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_gate, (int)ffn_l, (int)dim, ctx->g, bs, nullptr))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_up, (int)ffn_l, (int)dim, ctx->u, bs, nullptr))) return rc;
+            if ((rc = tc_gate_up(ctx, ld, ffn_l, dim, bs))) return rc;
         } else {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn_l, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;

@@ -1,157 +1,279 @@
-// ps_tc.cuh — tcgen05 (5th-gen tensor core) GEMM for prefill chunks: dst{N, bs} = W{K, N} . x{K, bs}, Q4_K weights x Q8_K
+// ps_tc.cuh — tcgen05 (5th-gen tensor core) GEMM for token batches: dst{N, bs} = W{K, N} . x{K, bs}, Q4_K weights x Q8_K
 // activations, BIT-IDENTICAL to ggml_vec_dot_q4_K_q8_K per column (ggml-quants.c:7809-7872).
 //
 // The reference's result is not a plain dot product: per super-block i and AVX lane l it forms the INTEGER
 //   S_l = sum_{j<8} sc_j * sum_{t<4} q4[j][4l+t] * q8[j][4l+t]            (and P_k = m_2k*bs_2k + m_2k+1*bs_2k+1 for the mins)
 // and then advances 8 + 4 fp32 FMA chains, acc_l = fma(d_x*d_y, (float)S_l, acc_l).  The integer part is a dense
 // contraction, and it is EXACT on the tensor cores in fp16/fp32: the operands sc_j*q4 (<= 945) and q8 (|.| <= 127) are
-// integers that fp16 represents exactly, every product is exact in fp32 and a 32-term sum stays below 2^24.  So:
-//   * A operand (weights): per (128-row tile, super-block, lane l) a K = 32 fp16 tile of sc_j*q4, expanded ONCE at bind time
-//     into HBM in the UMMA canonical K-major layout (2 B / weight: 15 GB for Llama-3.1-8B — the 180 GB part pays for zero
-//     dequantisation work on the prefill path); the mins use one shared K = 16 tile of the m_j.
-//   * B operand (activations): per (16-column group, super-block, lane) the q8 bytes as fp16, plus half-block sums for the
-//     mins, written per forward call by ps_k_tc_prep_b (same quantiser as everywhere else).
-//   * per super-block: 16 + 4 tcgen05.mma (M = 128, N = 16, K = 16) into 12 x 16 TMEM columns (double-buffered); 16
-//     epilogue warps read the exact integers back (12 tcgen05.ld in flight, one wait) and advance the FMA chains in
-//     registers, one (row, column) pair's 12 chains in ONE thread — the final hsum_float_8 order needs no shuffles.
-//     The tile is 128 x 16 because the chains, not the MMAs, set the budget: 12 fp32 accumulators per output element
-//     (24.5 K registers per tile) plus the 24.5 K registers the TMEM read-back lands in fill the register file.
-// Pipeline: persistent CTAs over (row tile, column group) units; TMA producer warp (2 stages, one bulk copy per operand
-// block) -> single-thread MMA issuer -> epilogue warps, linked by mbarriers (smem full/empty, tmem full/empty x 2).
+// integers that fp16 represents exactly, every product is exact in fp32 and a 32-term sum stays below 2^24.
+//
+// What bounds it.  The 12 FMAs per (row, column, super-block) are CUDA-core work that nothing replaces, and 12 accumulators per output
+// limit a tile that holds them all to 128 x 32; such a tile re-reads (and would have to de-quantise) its weights for every 32 columns.
+// So a tile is 128 rows x NT columns (up to 128) and its chains are taken in six PASSES over K of two chains each - the lane pairs
+// (0,4) (2,6) (1,5) (3,7), which hsum_float_8 adds first, and the mins pairs (0,2) (1,3) - with 2 x NT / 4 accumulators a thread.  A
+// pass needs only its own quarter of the quants.  A pass ends with ONE number per output; the six are added in the reference's order
+//   ((r04 + r26) + (r15 + r37)) + (m02 + m13).
+//   * weights stay packed (20 480 B per 128 rows x 256, 1.11x the GGUF bytes): de-quantising warps (thread = row) turn the 16 bytes of a
+//     (row, lane) into 32 halves - (1024 + nibble) by bit insertion, one HFMA2 per two values for the subtraction and the scale - and
+//     write them with tcgen05.st straight into TENSOR MEMORY, from where tcgen05.mma takes its A operand: neither the expanded weights
+//     nor their re-reads cross shared memory, whose bandwidth would otherwise be the first limit.
+//   * activations (B): q8 as fp16 in canonical K-major tiles, written once per GEMM input by ps_k_tc_prep_b; TMA bulk copies.
+//   * accumulators: a ring of three tensor-memory entries (two chains x half of the columns), so that the MMAs of one half run while
+//     the epilogue warps of the other half drain theirs; packed fma.rn.f32x2 advances two columns' chains per instruction.
+// Pipeline: TMA producer -> de-quantising warps -> single-thread MMA issuer -> epilogue warps, linked by mbarriers.
+// Work: a unit is (row tile, column tile, pass group); 1, 2 or 6 passes a unit, so that small matrices still cover the GPU.  The unit
+// of a tile that finishes last adds the others' numbers (thread-private order in global memory) and stores.
 #pragma once
 #include "ps_rw.cuh"
 
 #define PS_TC_M 128
-#define PS_TC_N 16
-#define PS_TC_EPI_WARPS 16
-#define PS_TC_THREADS ((PS_TC_EPI_WARPS + 2) * 32)
-// operand blocks in global / shared memory (bytes)
-#define PS_TC_A_TILE (PS_TC_M * 16 * 2)                    // one MMA's A operand: 128 rows x K16 fp16 = 4096
-#define PS_TC_B_TILE (PS_TC_N * 16 * 2)                    // one MMA's B operand: 16 cols x K16 fp16 = 512
-#define PS_TC_A_BLOCK (16 * PS_TC_A_TILE + PS_TC_A_TILE + PS_TC_M * 8)  // 8 lanes x 2 + mins tile + (xd, xmin) per row = 70656
-#define PS_TC_B_BLOCK (16 * PS_TC_B_TILE + 4 * PS_TC_B_TILE + PS_TC_N * 4) // 8 lanes x 2 + 4 mins tiles + yd per column = 10304
-#define PS_TC_STAGE (PS_TC_A_BLOCK + PS_TC_B_BLOCK)        // 80960
-#define PS_TC_STAGES 2
+// K is taken in steps of TWO super-blocks (one stage, one bulk copy per operand; an odd count is padded by a super-block of zeros, which
+// leaves every chain as it is: fma(0, 0, acc)).  nbp = super-blocks rounded up to even.
+// packed weights of a 128-row tile: [4 lane passes][nbp][2 lanes][128 rows][16 B quants], [nbp][128 rows][8 fp16 scales], [nbp][128 d],
+// [nbp][128 rows][8 mins], [nbp][128 -dmin]
+#define PS_TC_A_Q 4096
+#define PS_TC_A_SC 2048
+#define PS_TC_A_MN 1024
+#define PS_TC_A_D 512
+#define PS_TC_A_BLOCK (4 * PS_TC_A_Q + PS_TC_A_SC + PS_TC_A_MN + 2 * PS_TC_A_D) // 20480 per (row tile, super-block)
+#define PS_TC_A_OFF_SC(nbp) ((size_t)(nbp) * (4 * PS_TC_A_Q))
+#define PS_TC_A_OFF_D(nbp) ((size_t)(nbp) * (4 * PS_TC_A_Q + PS_TC_A_SC))
+#define PS_TC_A_OFF_MN(nbp) ((size_t)(nbp) * (4 * PS_TC_A_Q + PS_TC_A_SC + PS_TC_A_D))
+#define PS_TC_A_OFF_DM(nbp) ((size_t)(nbp) * (4 * PS_TC_A_Q + PS_TC_A_SC + PS_TC_A_D + PS_TC_A_MN))
+// activations of an NT-column tile: [4 lane passes][nbp][NT * 128 B], [2 mins passes][nbp][NT * 64 B], [nbp][NT d]
+#define PS_TC_B_BLOCK(NT) ((NT) * 644)
+#define PS_TC_PASSES 6
+// lane pass p takes the AVX lanes l and l + 4 with l = 0, 2, 1, 3; this is the pass of lane l
+PS_HD int ps_tc_pass(int l) { return ((l & 1) << 1) | ((l >> 1) & 1); }
 
-// canonical K-major, no-swizzle UMMA tile: [k-chunk (2)][8-row group][8 rows][8 fp16]  (cute: ((8,n),2):((1,SBO),LBO))
-PS_HD int ps_tc_tile_off(int row, int k16, int n_rows) { return ((k16 >> 3) * (n_rows >> 3) + (row >> 3)) * 128 + (row & 7) * 16 + (k16 & 7) * 2; }
+// configuration by column-tile width
+template <int NT> struct PsTc {
+    static constexpr int NH = NT >= 64 ? 2 : 1;                 // column halves, each with epilogue warps of its own
+    static constexpr int CW = NT / NH;                          // columns of a tensor-memory entry (N of one MMA)
+    static constexpr int EW = NT >= 64 ? 16 : 8;                // epilogue warps
+    static constexpr int EC = NT * 4 / EW;                      // columns a thread owns (its warp's lane quadrant gives the row)
+    static constexpr int NE = 3, NA = 3;                        // tensor-memory rings: accumulator entries, A buffers
+    static constexpr int NS = 3;                                // stages of two super-blocks (NE and NA divide 2 NS: the MMA loop is unrolled by it)
+    static constexpr int ND = 2;                                // de-quantising warpgroups: one per super-block of a step
+    static constexpr int THREADS = (EW + 4 * ND + 4) * 32;
+    static constexpr bool SPLIT = NT >= 96;                     // setmaxnreg: EC accumulator pairs do not fit an even share of the registers
+    static constexpr int TM_A = NE * 2 * CW;                    // first tensor-memory column of the A buffers
+    static constexpr int TM_USED = TM_A + NA * 32;
+    static constexpr int TM_COLS = TM_USED <= 256 ? 256 : 512;
+    static constexpr int STAGE_SC = 2 * PS_TC_A_Q;              // quants, scales, B of the two super-blocks (a mins pass: mins at the front, B)
+    static constexpr int STAGE_B = STAGE_SC + 2 * PS_TC_A_SC;
+    static constexpr int STAGE = STAGE_B + 2 * NT * 128;
+    static constexpr int NY = 2 * NS;                           // the factors' ring: the epilogue still reads them when the stage has been refilled
+    static constexpr int FACT = 2 * (PS_TC_A_D + NT * 4);       // d or -dmin of the rows, d of the columns
+    static constexpr int STASH = EW * 32 * EC * 4;              // a pass's numbers while the next pass of its pair runs
+    static constexpr int SMEM = NS * STAGE + NY * FACT + STASH;
+    static constexpr int CTAS = 1;
+};
 
 // ---------------------------------------------------------------------------------------------------- operand builders
-// A blocks of a matrix: [row tile][super-block][PS_TC_A_BLOCK].  One CTA per (row tile, super-block); rows >= n_rows are zero.
-__global__ void __launch_bounds__(256) ps_k_tc_expand_a(uint8_t *__restrict__ dst, const uint8_t *__restrict__ w, int64_t n_rows, int64_t nb,
-                                                        int64_t tile0) {
-    const int64_t i = blockIdx.x, rt = blockIdx.y;
-    uint8_t *out = dst + ((tile0 + rt) * nb + i) * PS_TC_A_BLOCK;
-    for (int idx = threadIdx.x; idx < PS_TC_M * 8; idx += blockDim.x) { // (row, sub-block j)
-        const int row = idx >> 3, j = idx & 7;
+// packed blocks of a matrix, row tile by row tile.  One CTA per (super-block, row tile); rows >= n_rows and super-blocks >= nb are zero.
+__global__ void __launch_bounds__(256) ps_k_tc_pack_a(uint8_t *__restrict__ dst, const uint8_t *__restrict__ w, int64_t n_rows, int64_t nb, int64_t tile0) {
+    const int64_t i = blockIdx.x, rt = blockIdx.y, nbp = gridDim.x;
+    uint8_t *out = dst + (tile0 + rt) * nbp * PS_TC_A_BLOCK;
+    for (int idx = threadIdx.x; idx < PS_TC_M * 8; idx += blockDim.x) { // (row, AVX lane l); also sub-block j = l
+        const int row = idx >> 3, l = idx & 7, j = l;
         const int64_t n = rt * PS_TC_M + row;
-        const bool live = n < n_rows;
+        const bool live = n < n_rows && i < nb;
         const uint8_t *blk = w + (n * nb + i) * PS_Q4_K_BYTES;
         int sc = 0, mn = 0;
+        uint4 q = make_uint4(0, 0, 0, 0);
         if (live) { // get_scale_min_k4 (ggml-quants.c:1912-1919)
             const uint8_t *s = blk + 4;
             if (j < 4) { sc = s[j] & 63; mn = s[j + 4] & 63; }
             else { sc = (s[j + 4] & 0xF) | ((s[j - 4] >> 6) << 4); mn = (s[j + 4] >> 4) | ((s[j] >> 6) << 4); }
+            const uint32_t *qs = reinterpret_cast<const uint32_t *>(blk + 16) + l; // word g: sub-block 2g (low nibbles), 2g + 1 (high)
+            q = make_uint4(qs[0], qs[8], qs[16], qs[24]);
         }
-        for (int e = 0; e < 32; e++) { // element e of sub-block j -> lane l = e / 4, t = e % 4
-            int q = 0;
-            if (live) {
-                const uint8_t b = blk[16 + 32 * (j >> 1) + e];
-                q = (j & 1) ? (b >> 4) : (b & 0xF);
-            }
-            const int l = e >> 2, t = e & 3, k32 = 4 * j + t;
-            uint8_t *tile = out + (size_t)(2 * l + (k32 >> 4)) * PS_TC_A_TILE;
-            *reinterpret_cast<__half *>(tile + ps_tc_tile_off(row, k32 & 15, PS_TC_M)) = __int2half_rn(sc * q); // <= 945: exact
-        }
-        // mins tile (shared by the four mins MMAs): K position 4k + u holds m_{2k + u/2}
-        uint8_t *mt = out + (size_t)16 * PS_TC_A_TILE;
-        const int k = j >> 1, u0 = (j & 1) * 2;
-        *reinterpret_cast<__half *>(mt + ps_tc_tile_off(row, 4 * k + u0, PS_TC_M)) = __int2half_rn(mn);
-        *reinterpret_cast<__half *>(mt + ps_tc_tile_off(row, 4 * k + u0 + 1, PS_TC_M)) = __int2half_rn(mn);
+        *reinterpret_cast<uint4 *>(out + (ps_tc_pass(l) * nbp + i) * PS_TC_A_Q + (l >> 2) * 2048 + row * 16) = q;
+        // even sub-blocks are read from low nibbles, odd ones from high nibbles (16 x the value): the odd scales are stored / 16
+        reinterpret_cast<__half *>(out + PS_TC_A_OFF_SC(nbp) + i * PS_TC_A_SC)[row * 8 + j] = __float2half_rn((j & 1) ? (float)sc * 0.0625f : (float)sc);
+        out[PS_TC_A_OFF_MN(nbp) + i * PS_TC_A_MN + row * 8 + j] = (uint8_t)mn;
         if (j == 0) {
-            float *xs = reinterpret_cast<float *>(out + (size_t)17 * PS_TC_A_TILE) + 2 * row;
-            xs[0] = live ? ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk)) : 0.f;
-            xs[1] = live ? ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 2)) : 0.f;
+            reinterpret_cast<float *>(out + PS_TC_A_OFF_D(nbp) + i * PS_TC_A_D)[row] = live ? ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk)) : 0.f;
+            reinterpret_cast<float *>(out + PS_TC_A_OFF_DM(nbp) + i * PS_TC_A_D)[row] = live ? -ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 2)) : 0.f;
         }
     }
 }
 
-// B blocks of an activation batch: [column group][super-block][PS_TC_B_BLOCK]; one warp per (column, super-block):
-// quantize_row_q8_K (the shared warp quantiser), then the q8 bytes as fp16 in the lane tiles, the half-block sums in the
-// mins tiles (zero outside lane k's four K positions) and d in the tail.  Columns >= bs are zero.
-__global__ void __launch_bounds__(128) ps_k_tc_prep_b(uint8_t *__restrict__ dst, const float *__restrict__ x, int64_t K, int bs) {
+// activation operand of a batch, column tile by column tile; one warp per (super-block, column): quantize_row_q8_K
+// (the shared warp quantiser), the q8 of AVX lane l as 32 halves in the order the weights come out of their words - word g = k / 8:
+// (2g: t 0, 2) (2g + 1: t 0, 2) (2g: t 1, 3) (2g + 1: t 1, 3) - then half-block sums for the mins and d.  Columns >= bs are zero.
+// Tiles are canonical K-major without swizzle: [k / 8][column][8 halves].
+__device__ __forceinline__ void ps_tc_store_b(uint8_t *__restrict__ out, int NT, int64_t nbp, int64_t i, int c, int lane, const uint32_t words[2], float yd) {
+    // thread (g, l) of the warp builds the 16-byte piece g of lane l: it needs the words (sub-block 2g, l) and (2g + 1, l); natural word
+    // (j, l) is words[j / 4] of thread (j % 4) * 8 + l
+    const int g = lane >> 3, l = lane & 7, src = ((2 * g) & 3) * 8 + l;
+    const uint32_t a0 = __shfl_sync(PS_FULL, words[0], src), a1 = __shfl_sync(PS_FULL, words[1], src);
+    const uint32_t b0 = __shfl_sync(PS_FULL, words[0], src + 8), b1 = __shfl_sync(PS_FULL, words[1], src + 8);
+    const uint32_t a = g < 2 ? a0 : a1, b = g < 2 ? b0 : b1;
+    auto h2 = [](uint32_t w, int t0, int t1) {
+        const __half2 h = __halves2half2(__int2half_rn((int)(signed char)(w >> (8 * t0))), __int2half_rn((int)(signed char)(w >> (8 * t1))));
+        return *reinterpret_cast<const uint32_t *>(&h);
+    };
+    *reinterpret_cast<uint4 *>(out + (ps_tc_pass(l) * nbp + i) * NT * 128 + (size_t)(l >> 2) * NT * 64 + ((size_t)g * NT + c) * 16) =
+        make_uint4(h2(a, 0, 2), h2(b, 0, 2), h2(a, 1, 3), h2(b, 1, 3));
+    // half-block sums: threads of one sub-block, lanes l = 0..3 -> elements 0..15, l = 4..7 -> elements 16..31
+    uint32_t hs[2]; // this thread's sub-blocks lane / 8 and 4 + lane / 8: (first half, second half) as half2
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        int s = __dp4a((int)words[h], 0x01010101, 0);
+        s += __shfl_xor_sync(PS_FULL, s, 1);
+        s += __shfl_xor_sync(PS_FULL, s, 2);
+        const int s0 = __shfl_sync(PS_FULL, s, lane & 24), s1 = __shfl_sync(PS_FULL, s, (lane & 24) + 4);
+        const __half2 v = __halves2half2(__int2half_rn(s0), __int2half_rn(s1)); // |.| <= 2032: exact
+        hs[h] = *reinterpret_cast<const uint32_t *>(&v);
+    }
+    // mins chain k (sub-blocks 2k, 2k + 1): K positions 4k .. 4k + 3 hold its four half sums, the others are zero
+    const uint32_t m0 = __shfl_sync(PS_FULL, hs[0], (lane & 1) * 16), m1 = __shfl_sync(PS_FULL, hs[0], (lane & 1) * 16 + 8);
+    const uint32_t m2 = __shfl_sync(PS_FULL, hs[1], (lane & 1) * 16), m3 = __shfl_sync(PS_FULL, hs[1], (lane & 1) * 16 + 8);
+    if (lane < 4) { // thread k: chain k; pass 4 + (k & 1), chain k / 2 of the pass
+        const int k = lane;
+        const uint32_t v0 = k < 2 ? m0 : m2, v1 = k < 2 ? m1 : m3;
+        uint8_t *t = out + nbp * NT * 512 + ((k & 1) * nbp + i) * NT * 64 + (size_t)(k >> 1) * NT * 32;
+        const uint4 mine = (k & 1) ? make_uint4(0, 0, v0, v1) : make_uint4(v0, v1, 0, 0), none = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(t + (size_t)c * 16) = k < 2 ? mine : none;
+        *reinterpret_cast<uint4 *>(t + ((size_t)NT + c) * 16) = k < 2 ? none : mine;
+    }
+    if (lane == 0) reinterpret_cast<float *>(out + nbp * NT * 640)[i * NT + c] = yd;
+}
+__global__ void __launch_bounds__(128) ps_k_tc_prep_b(uint8_t *__restrict__ dst, const float *__restrict__ x, int64_t K, int bs, int NT) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nb = K / 256, i = (int64_t)blockIdx.x * 4 + warp;
-    const int col = blockIdx.y, cg = col / PS_TC_N, c = col % PS_TC_N;
-    if (i >= nb) return;
-    uint8_t *out = dst + ((int64_t)cg * nb + i) * PS_TC_B_BLOCK;
+    const int64_t nb = K / 256, nbp = (nb + 1) & ~(int64_t)1, i = (int64_t)blockIdx.x * 4 + warp;
+    const int col = blockIdx.y, ct = col / NT, c = col % NT;
+    if (i >= nbp) return;
     uint32_t words[2] = {0, 0}, bsp = 0;
     float yd = 0.f;
-    if (col < bs) {
+    if (col < bs && i < nb) {
         float e[8];
         ps_rw_load8(x + (int64_t)col * K + i * 256, lane, e);
         ps_quant_block_q8k_regs(e, lane, words, yd, bsp);
     }
-    // natural word `lane` = (sub-block j = lane / 8, AVX lane l = lane % 8); second word: sub-block 4 + lane / 8
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        const int j = 4 * h + (lane >> 3), l = lane & 7;
-        int hsum = 0;
-#pragma unroll
-        for (int t = 0; t < 4; t++) {
-            const int q = (int)(signed char)((words[h] >> (8 * t)) & 0xff);
-            const int k32 = 4 * j + t;
-            uint8_t *tile = out + (size_t)(2 * l + (k32 >> 4)) * PS_TC_B_TILE;
-            *reinterpret_cast<__half *>(tile + ps_tc_tile_off(c, k32 & 15, PS_TC_N)) = __int2half_rn(q);
-            hsum += q;
-        }
-        // half-block sums of sub-block j: lanes l = 0..3 -> elements 0..15, l = 4..7 -> elements 16..31
-        hsum += __shfl_xor_sync(PS_FULL, hsum, 1);
-        hsum += __shfl_xor_sync(PS_FULL, hsum, 2);
-        const int k = j >> 1, u = (j & 1) * 2 + (l >> 2);
-        if ((l & 3) == 0) { // lane k's tile gets the value at K position 4k + u; the other K positions of that tile stay zero
-            uint8_t *tile = out + (size_t)(16 + k) * PS_TC_B_TILE;
-            *reinterpret_cast<__half *>(tile + ps_tc_tile_off(c, 4 * k + u, PS_TC_N)) = __int2half_rn(hsum); // |.| <= 2032: exact
-        }
-    }
-    if (lane == 0) reinterpret_cast<float *>(out + (size_t)20 * PS_TC_B_TILE)[c] = yd;
+    ps_tc_store_b(dst + ct * nbp * PS_TC_B_BLOCK(NT), NT, nbp, i, c, lane, words, yd);
 }
 
+// ---------------------------------------------------------------------------------------------------- GEMM
+#define PS_TC_SEGS 3
 struct PsTcArgs {
-    const uint8_t *a;   // [row tiles][nb][PS_TC_A_BLOCK]
-    const uint8_t *b;   // [column groups][nb][PS_TC_B_BLOCK]
-    int nb, n_cg, n_units; // units = row tiles x column groups
-    PsRwSeg seg[3];     // dst of a segment is [bs][rows of the segment]
+    const uint8_t *a;   // [row tiles][nbp * PS_TC_A_BLOCK]
+    const uint8_t *b;   // [column tiles][nbp * PS_TC_B_BLOCK(NT)]
+    int nbp, n_ct, n_tiles, pp; // super-blocks (even); column tiles; row tiles x column tiles; passes a unit takes (1, 2 or 6)
+    PsRwSeg seg[PS_TC_SEGS]; // rows row_begin .. row_end of the padded row space; dst of a segment is [bs][rows of the segment]
     int n_seg, bs;
     const float *residual;
-    int *err;           // set to 1 if a pipeline wait timed out (results invalid)
+    float *part;        // [tile][units of a tile][EC][epilogue threads]
+    int *cnt;           // per tile: units that have finished (left at zero)
+    int *err;           // set if a pipeline wait gave up (results invalid)
 };
 
-// Persistent CTAs; unit u = (row tile u / n_cg, column group u % n_cg), so that the column groups sharing an A tile run at
-// the same time on neighbouring CTAs (A comes out of L2 for all but the first).
-__global__ void __launch_bounds__(PS_TC_THREADS, 1) ps_k_tc_gemm(const PsTcArgs a) {
+typedef unsigned long long ps_f2; // two packed floats
+PS_D ps_f2 ps_f2_pack(float a, float b) { ps_f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+PS_D void ps_f2_unpack(ps_f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+PS_D ps_f2 ps_f2_mul(ps_f2 a, ps_f2 b) { ps_f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+PS_D ps_f2 ps_f2_add(ps_f2 a, ps_f2 b) { ps_f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+PS_D ps_f2 ps_f2_fma(ps_f2 a, ps_f2 b, ps_f2 c) { ps_f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+// eight columns of one row of two accumulators, as pairs of columns, with the wait for them
+PS_D void ps_tc_ld8x2(uint32_t t0, uint32_t t1, ps_f2 v[8]) {
+    asm volatile(
+        "{\n\t.reg .b32 a<8>;\n\t.reg .b32 b<8>;\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {a0,a1,a2,a3,a4,a5,a6,a7}, [%8];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {b0,b1,b2,b3,b4,b5,b6,b7}, [%9];\n\t"
+        "tcgen05.wait::ld.sync.aligned;\n\t"
+        "mov.b64 %0, {a0,a1};\n\tmov.b64 %1, {a2,a3};\n\tmov.b64 %2, {a4,a5};\n\tmov.b64 %3, {a6,a7};\n\t"
+        "mov.b64 %4, {b0,b1};\n\tmov.b64 %5, {b2,b3};\n\tmov.b64 %6, {b4,b5};\n\tmov.b64 %7, {b6,b7};\n\t}"
+        : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7])
+        : "r"(t0), "r"(t1)
+        : "memory");
+}
+PS_D void ps_tc_st8(uint32_t taddr, const uint32_t v[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                 "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+PS_D void ps_tc_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+PS_D uint32_t ps_h2_fma(uint32_t a, uint32_t b, uint32_t c) { uint32_t r; asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c)); return r; }
+PS_D uint32_t ps_h2_mul(uint32_t a, uint32_t b) { uint32_t r; asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b)); return r; }
+
+// two words of nibbles of one (row, lane) -> 16 halves sc_j * q4 (two per register); s[j]: the scale of sub-block j twice (odd ones / 16),
+// o[j] = -1024 s[j].  (1024 + n) s - 1024 s is exact: both terms are below 65504 and the fused result is an integer <= 945.
+PS_D void ps_tc_dequant8(uint32_t w0, uint32_t w1, const uint32_t s[4], const uint32_t o[4], uint32_t v[8]) {
+    const uint32_t w[2] = {w0, w1};
+#pragma unroll
+    for (int g = 0; g < 2; g++) {
+        const uint32_t a = w[g], b = w[g] >> 8;
+        v[4 * g + 0] = ps_h2_fma((a & 0x000F000Fu) | 0x64006400u, s[2 * g], o[2 * g]);
+        v[4 * g + 1] = ps_h2_fma((a & 0x00F000F0u) | 0x64006400u, s[2 * g + 1], o[2 * g + 1]);
+        v[4 * g + 2] = ps_h2_fma((b & 0x000F000Fu) | 0x64006400u, s[2 * g], o[2 * g]);
+        v[4 * g + 3] = ps_h2_fma((b & 0x00F000F0u) | 0x64006400u, s[2 * g + 1], o[2 * g + 1]);
+    }
+}
+
+template <int N> PS_D void ps_reg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> PS_D void ps_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// every lane waits for a barrier of its own; bounded like ps_tc_wait.  One such poll costs what a wait for one barrier does (about 80 cycles
+// even when the phase is complete)
+PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity) {
+    for (int spin = 0; spin < (1 << 22); spin++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (__all_sync(PS_FULL, ok)) return true;
+    }
+    return false;
+}
+
+// position in a ring of N: index and the parity of the round
+template <int N> struct PsRing {
+    int i = 0;
+    uint32_t round = 0;
+    PS_D void step() {
+        if (++i == N) { i = 0; round ^= 1; }
+    }
+};
+
+// Persistent CTAs over units u = tile * (6 / pp) + group; tile = row tile * n_ct + column tile.
+template <int NT>
+__global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gemm(const PsTcArgs a) {
+    using T = PsTc<NT>;
     extern __shared__ __align__(1024) uint8_t ps_tc_smem[];
-    __shared__ __align__(8) uint64_t bar_full[PS_TC_STAGES], bar_empty[PS_TC_STAGES], bar_tmem_full[2], bar_tmem_empty[2];
+    __shared__ __align__(8) uint64_t bar_full[T::NS], bar_empty[T::NS], bar_a_full[T::NA], bar_a_empty[T::NA], bar_d_full[T::NE], bar_d_empty[T::NE], bar_y_empty[T::NY], bar_done;
     __shared__ uint32_t tmem_base_smem;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int nb = a.nb;
-    const int my_units = (a.n_units > (int)blockIdx.x) ? (a.n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    const int n_steps = my_units * nb; // (unit, super-block) steps of this CTA, in order
+    __shared__ int sh_last;
+    const int tid = threadIdx.x, warp = __shfl_sync(PS_FULL, tid >> 5, 0), lane = tid & 31;
+    const int ns = a.nbp >> 1, pp = a.pp, nu = PS_TC_PASSES / pp; // steps of a pass, units of a tile
+    const int n_units = a.n_tiles * nu;
+    constexpr int W_TMA = T::EW + 4 * T::ND, W_MMA = W_TMA + 1;
+    uint8_t *const ps_tc_fact = ps_tc_smem + (size_t)T::NS * T::STAGE;
 
     if (tid == 0) {
-        for (int s = 0; s < PS_TC_STAGES; s++) {
+        for (int s = 0; s < T::NS; s++) {
             ps_mbar_init(&bar_full[s], 1);
-            ps_mbar_init(&bar_empty[s], 1 + PS_TC_EPI_WARPS); // the MMA commit + every epilogue warp (they read xd / yd from the stage)
+            ps_mbar_init(&bar_empty[s], 4 * T::ND + 1); // the de-quantising warps, the MMA commit
         }
-        for (int b = 0; b < 2; b++) {
-            ps_mbar_init(&bar_tmem_full[b], 1);
-            ps_mbar_init(&bar_tmem_empty[b], PS_TC_EPI_WARPS);
+        for (int s = 0; s < T::NA; s++) {
+            ps_mbar_init(&bar_a_full[s], 4);
+            ps_mbar_init(&bar_a_empty[s], 1);
         }
+        for (int s = 0; s < T::NE; s++) {
+            ps_mbar_init(&bar_d_full[s], 1);
+            ps_mbar_init(&bar_d_empty[s], T::EW / T::NH);
+        }
+        for (int s = 0; s < T::NY; s++) ps_mbar_init(&bar_y_empty[s], T::EW);
+        ps_mbar_init(&bar_done, 1);
         ps_fence_barrier_init();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == PS_TC_EPI_WARPS + 1) { // the MMA warp owns the tensor memory: 512 columns (2 x 12 x 16 used)
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(ps_smem_u32(&tmem_base_smem)) : "memory");
+    if (warp == W_MMA) { // the MMA warp owns the tensor memory
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ps_smem_u32(&tmem_base_smem)), "n"(T::TM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     ps_tc_fence_before();
@@ -159,89 +281,284 @@ __global__ void __launch_bounds__(PS_TC_THREADS, 1) ps_k_tc_gemm(const PsTcArgs 
     ps_tc_fence_after();
     const uint32_t tmem_base = tmem_base_smem;
 
-    if (warp == PS_TC_EPI_WARPS) {
-        // ===== TMA producer
-        if (lane == 0) {
-            for (int g = 0; g < n_steps; g++) {
-                const int u = (int)blockIdx.x + (g / nb) * (int)gridDim.x, i = g % nb, s = g % PS_TC_STAGES;
-                if (g >= PS_TC_STAGES && !ps_tc_wait(&bar_empty[s], ((g / PS_TC_STAGES) - 1) & 1)) { *a.err = 1; break; }
-                uint8_t *st = ps_tc_smem + (size_t)s * PS_TC_STAGE;
-                ps_mbar_expect_tx(&bar_full[s], PS_TC_STAGE);
-                ps_bulk_g2s(st, a.a + ((size_t)(u / a.n_cg) * nb + i) * PS_TC_A_BLOCK, PS_TC_A_BLOCK, &bar_full[s]);
-                ps_bulk_g2s(st + PS_TC_A_BLOCK, a.b + ((size_t)(u % a.n_cg) * nb + i) * PS_TC_B_BLOCK, PS_TC_B_BLOCK, &bar_full[s]);
+    if (warp >= W_TMA) {
+        if (T::SPLIT) ps_reg_dec<24>();
+        if (warp == W_TMA) {
+            // ===== TMA producer
+            PsRing<T::NS> st;
+            PsRing<T::NY> sy;
+            int g = 0;
+            bool ok = true;
+            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+                const int tile = u / nu, p0 = (u % nu) * pp;
+                const uint8_t *pa = a.a + (size_t)(tile / a.n_ct) * a.nbp * PS_TC_A_BLOCK, *pb = a.b + (size_t)(tile % a.n_ct) * a.nbp * PS_TC_B_BLOCK(NT);
+                for (int p = p0; p < p0 + pp && ok; p++) {
+                    const bool lanes = p < 4;
+                    const uint8_t *aq = pa + (lanes ? (size_t)p * a.nbp * PS_TC_A_Q : PS_TC_A_OFF_MN(a.nbp)), *as = pa + PS_TC_A_OFF_SC(a.nbp);
+                    const uint8_t *ad = pa + (lanes ? PS_TC_A_OFF_D(a.nbp) : PS_TC_A_OFF_DM(a.nbp));
+                    const uint8_t *bq = pb + (lanes ? (size_t)p * a.nbp * (NT * 128) : (size_t)a.nbp * (NT * 512) + (size_t)(p - 4) * a.nbp * (NT * 64));
+                    const uint8_t *by = pb + (size_t)a.nbp * (NT * 640);
+                    const uint32_t na = lanes ? 2 * PS_TC_A_Q : 2 * PS_TC_A_MN, nbb = lanes ? 2 * NT * 128 : 2 * NT * 64;
+                    const uint32_t total = na + (lanes ? 2 * PS_TC_A_SC : 0) + 2 * PS_TC_A_D + nbb + 2 * NT * 4;
+                    for (int i = 0; i < ns; i++, g++, st.step(), sy.step()) {
+                        const bool fy = (lane & 1) && g >= T::NY; // odd lanes wait for the factors' slot
+                        if (g >= T::NS && !ps_tc_wait_all(ps_smem_u32(fy ? &bar_y_empty[sy.i] : &bar_empty[st.i]), (fy ? sy.round : st.round) ^ 1)) { *a.err = 1; ok = false; break; }
+                        uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE, *sf = ps_tc_fact + sy.i * T::FACT;
+                        uint64_t *bar = &bar_full[st.i];
+                        if (ps_elect_one()) {
+                            ps_mbar_expect_tx(bar, total);
+                            ps_bulk_g2s(sm, aq, na, bar);
+                            ps_bulk_g2s(sm + T::STAGE_B, bq, nbb, bar);
+                            if (lanes) ps_bulk_g2s(sm + T::STAGE_SC, as, 2 * PS_TC_A_SC, bar);
+                            ps_bulk_g2s(sf, ad, 2 * PS_TC_A_D, bar);
+                            ps_bulk_g2s(sf + 2 * PS_TC_A_D, by, 2 * NT * 4, bar);
+                        }
+                        __syncwarp();
+                        aq += na;
+                        bq += nbb;
+                        as += 2 * PS_TC_A_SC;
+                        ad += 2 * PS_TC_A_D;
+                        by += 2 * NT * 4;
+                    }
+                }
             }
-        }
-    } else if (warp == PS_TC_EPI_WARPS + 1) {
-        // ===== MMA issuer (one thread)
-        if (lane == 0) {
-            // kind::f16, D = F32 (c_format 1 @ bit 4), A = B = F16 (0), K-major both, N >> 3 @ bit 17, M >> 4 @ bit 24
-            const uint32_t idesc = (1u << 4) | ((uint32_t)(PS_TC_N >> 3) << 17) | ((uint32_t)(PS_TC_M >> 4) << 24);
-            for (int g = 0; g < n_steps; g++) {
-                const int s = g % PS_TC_STAGES, tb = g & 1;
-                if (!ps_tc_wait(&bar_full[s], (g / PS_TC_STAGES) & 1)) { *a.err = 2; break; }
-                if (g >= 2 && !ps_tc_wait(&bar_tmem_empty[tb], ((g >> 1) - 1) & 1)) { *a.err = 3; break; } // that accumulator buffer has been drained
-                ps_tc_fence_after();
-                const uint32_t sa = ps_smem_u32(ps_tc_smem + (size_t)s * PS_TC_STAGE), sb = sa + PS_TC_A_BLOCK;
-                const uint32_t td = tmem_base + tb * (12 * PS_TC_N);
-#pragma unroll 1
-                for (int l = 0; l < 8; l++)
+            // copies in flight end before the CTA does (they have, unless a wait gave up)
+            for (int k = g > T::NS ? g - T::NS : 0; k < g; k++)
+                if (!ps_tc_wait(&bar_full[k % T::NS], (k / T::NS) & 1)) { *a.err = 5; break; }
+        } else if (warp == W_MMA) {
+            // ===== MMA issuer.  The warp stays converged and one thread, chosen by elect.sync, issues; ring positions are constants of the
+            // unrolled loop.  So descriptors and barrier addresses live in uniform registers: with one thread looping under `lane == 0` an
+            // issue took 280 cycles whatever its size, where tcgen05.mma itself takes 32 here.
+            // kind::f16, D = F32 (bit 4), A = B = F16, K-major both, N >> 3 @ bit 17, M >> 4 @ bit 24
+            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(T::CW >> 3) << 17) | ((uint32_t)(PS_TC_M >> 4) << 24);
+            const uint64_t desc0 = ps_tc_smem_desc(ps_smem_u32(ps_tc_smem + T::STAGE_B), NT * 16, 128);
+            const int n_steps = n_units > (int)blockIdx.x ? ((n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * pp * ns : 0;
+            int u = blockIdx.x, p = (u % nu) * pp, p_end = p + pp, left = ns;
+            bool ok = true;
+            for (int g0 = 0; g0 < n_steps && ok; g0 += T::NS) {
+                const uint32_t round = (uint32_t)(g0 / T::NS) & 1; // of the stages; the other rings' parities are constants
 #pragma unroll
-                    for (int h = 0; h < 2; h++)
-                        ps_tc_mma_f16(td + l * PS_TC_N, ps_tc_smem_desc(sa + (2 * l + h) * PS_TC_A_TILE, (PS_TC_M / 8) * 128, 128),
-                                      ps_tc_smem_desc(sb + (2 * l + h) * PS_TC_B_TILE, (PS_TC_N / 8) * 128, 128), idesc, h);
-#pragma unroll 1
-                for (int k = 0; k < 4; k++)
-                    ps_tc_mma_f16(td + (8 + k) * PS_TC_N, ps_tc_smem_desc(sa + 16 * PS_TC_A_TILE, (PS_TC_M / 8) * 128, 128),
-                                  ps_tc_smem_desc(sb + (16 + k) * PS_TC_B_TILE, (PS_TC_N / 8) * 128, 128), idesc, 0);
-                ps_tc_commit(&bar_empty[s]);        // operands consumed
-                ps_tc_commit(&bar_tmem_full[tb]);   // accumulators of this super-block complete
+                for (int j = 0; j < T::NS; j++) {
+                    if (g0 + j >= n_steps || !ok) break;
+                    const bool lanes = p < 4;
+#pragma unroll
+                    for (int x = 0; x < 2; x++) { // the step's super-blocks
+                        const int k = 2 * j + x, ra = k % T::NA;
+                        const uint32_t ta = tmem_base + T::TM_A + ra * 32;
+                        const uint64_t ds = desc0 + (uint64_t)(j * (T::STAGE >> 4)) + (x ? (lanes ? NT * 8 : NT * 4) : 0);
+#pragma unroll
+                        for (int h = 0; h < T::NH; h++) {
+                            const int e = k * T::NH + h, re = e % T::NE;
+                            // lane 0: the accumulator entry (free from the start in the first round), lane 1: A, the others: the stage
+                            const bool fd = lane == 0 && (g0 > 0 || e >= T::NE), fa = lane == 1;
+                            const uint32_t bar = ps_smem_u32(fd ? &bar_d_empty[re] : fa ? &bar_a_full[ra] : &bar_full[j]);
+                            if (!ps_tc_wait_all(bar, fd ? ((e / T::NE) & 1) ^ 1 : fa ? (k / T::NA) & 1 : round)) { *a.err = 2; ok = false; break; }
+                            ps_tc_fence_after();
+                            const uint32_t td = tmem_base + re * (2 * T::CW);
+                            const uint64_t dh = ds + h * (T::CW / 8) * 8;
+                            if (ps_elect_one()) {
+                                if (lanes) {
+                                    ps_tc_mma_f16_ta(td, ta, dh, idesc, 0);
+                                    ps_tc_mma_f16_ta(td, ta + 8, dh + NT * 2, idesc, 1);
+                                    ps_tc_mma_f16_ta(td + T::CW, ta + 16, dh + NT * 4, idesc, 0);
+                                    ps_tc_mma_f16_ta(td + T::CW, ta + 24, dh + NT * 6, idesc, 1);
+                                } else {
+                                    ps_tc_mma_f16_ta(td, ta, dh, idesc, 0);
+                                    ps_tc_mma_f16_ta(td + T::CW, ta, dh + NT * 2, idesc, 0);
+                                }
+                                ps_tc_commit(&bar_d_full[re]);
+                                if (h == T::NH - 1) ps_tc_commit(&bar_a_empty[ra]);
+                                if (h == T::NH - 1 && x == 1) ps_tc_commit(&bar_empty[j]);
+                            }
+                            __syncwarp();
+                        }
+                        if (!ok) break;
+                    }
+                    if (--left == 0) { // next pass, next unit
+                        left = ns;
+                        if (++p == p_end) {
+                            u += gridDim.x;
+                            p = (u % nu) * pp;
+                            p_end = p + pp;
+                        }
+                    }
+                }
+            }
+            if (ps_elect_one()) ps_tc_commit(&bar_done); // MMAs in flight end before the tensor memory is given back
+            __syncwarp();
+            if (!ps_tc_wait(&bar_done, 0)) *a.err = 6;
+        }
+    } else if (warp >= T::EW) {
+        // ===== de-quantising warps: warpgroup d takes super-block d of every step; thread = row (warp % 4 is its tensor-memory lane quadrant)
+        if (T::SPLIT) ps_reg_dec<48>();
+        const int d = (warp - T::EW) >> 2, quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + T::TM_A;
+        PsRing<T::NS> st;
+        PsRing<T::NA> ra;
+        if (d) ra.step();
+        int g = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const int p0 = (u % nu) * pp;
+            for (int p = p0; p < p0 + pp && ok; p++) {
+                for (int i = 0; i < ns; i++, g++) {
+                    const bool fa = (lane & 1) && 2 * g + d >= T::NA; // odd lanes wait for the A buffer
+                    if (!ps_tc_wait_all(ps_smem_u32(fa ? &bar_a_empty[ra.i] : &bar_full[st.i]), fa ? ra.round ^ 1 : st.round)) { *a.err = 7; ok = false; break; }
+                    ps_tc_fence_after();
+                    const uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE;
+                    const uint32_t td = t_lane + ra.i * 32;
+                    if (p < 4) {
+                        sm += d * PS_TC_A_Q;
+                        const uint4 q0 = *reinterpret_cast<const uint4 *>(sm + row * 16), q1 = *reinterpret_cast<const uint4 *>(sm + 2048 + row * 16);
+                        const uint4 sc = *reinterpret_cast<const uint4 *>(sm + T::STAGE_SC - d * (PS_TC_A_Q - PS_TC_A_SC) + row * 16);
+                        __syncwarp();
+                        if (lane == 0) ps_mbar_arrive(&bar_empty[st.i]);
+#pragma unroll
+                        for (int k = 0; k < 2; k++) { // words 2k, 2k + 1 of both lanes
+                            uint32_t s2[4], o2[4], v[8];
+                            const uint32_t s0 = k ? sc.z : sc.x, s1 = k ? sc.w : sc.y;
+#pragma unroll
+                            for (int j = 0; j < 4; j++) {
+                                s2[j] = __byte_perm(j < 2 ? s0 : s1, 0, (j & 1) ? 0x3232 : 0x1010);
+                                o2[j] = ps_h2_mul(s2[j], 0xE400E400u); // x -1024
+                            }
+                            ps_tc_dequant8(k ? q0.z : q0.x, k ? q0.w : q0.y, s2, o2, v);
+                            ps_tc_st8(td + 8 * k, v);
+                            ps_tc_dequant8(k ? q1.z : q1.x, k ? q1.w : q1.y, s2, o2, v);
+                            ps_tc_st8(td + 16 + 8 * k, v);
+                        }
+                    } else { // K positions 4k + u hold m_(2k + u / 2): column 2k + u / 2 is that minimum twice
+                        const uint2 mn = *reinterpret_cast<const uint2 *>(sm + d * PS_TC_A_MN + row * 8);
+                        __syncwarp();
+                        if (lane == 0) ps_mbar_arrive(&bar_empty[st.i]);
+                        uint32_t v[8];
+#pragma unroll
+                        for (int j = 0; j < 8; j++) {
+                            const uint32_t w = __byte_perm(j < 4 ? mn.x : mn.y, 0x64646464u, 0x4040 + 0x0101 * (j & 3)); // 1024 + m, twice
+                            v[j] = ps_h2_fma(w, 0x3C003C00u, 0xE400E400u);
+                        }
+                        ps_tc_st8(td, v);
+                    }
+                    ps_tc_st_wait();
+                    ps_tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) ps_mbar_arrive(&bar_a_full[ra.i]);
+                    st.step();
+                    ra.step();
+                    ra.step();
+                }
             }
         }
     } else {
-        // ===== epilogue: warp w owns TMEM lanes 32 * (w % 4) .. +31 (rows) and columns 4 * (w / 4) .. +3 of every accumulator
-        const int row = 32 * (warp & 3) + lane, c0 = 4 * (warp >> 2);
-        const uint32_t t_lane = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + c0;
-        int g = 0;
+        // ===== epilogue: warp w owns tensor-memory lanes 32 * (w % 4) .. +31 (rows) and EC columns of half h
+        if (T::SPLIT) ps_reg_inc<96>();
+        constexpr int WPH = T::EW / T::NH; // warps of a half
+        const int h = warp / WPH, quad = warp & 3, cg = (warp % WPH) >> 2, row = quad * 32 + lane, c0 = h * T::CW + cg * T::EC;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + cg * T::EC;
+        float *stash = reinterpret_cast<float *>(ps_tc_fact + T::NY * T::FACT) + tid; // [EC][epilogue threads]
+        constexpr int ET = T::EW * 32;
+        PsRing<T::NY> sy;
+        PsRing<T::NE> re;
+        if (h) re.step();
         bool ok = true;
-        for (int mu = 0; mu < my_units && ok; mu++) {
-            const int u = (int)blockIdx.x + mu * (int)gridDim.x, rt = u / a.n_cg, cg = u % a.n_cg;
-            float acc[4][12];
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const int tile = u / nu, p0 = (u % nu) * pp;
+            float *part = a.part + ((size_t)tile * nu + u % nu) * (T::EC * ET) + tid;
+            float *whole = a.part + (size_t)blockIdx.x * (T::EC * ET) + tid; // pp = 6: the sum of the pass pairs so far
+            ps_f2 acc[2][T::EC / 2];
+            for (int p = p0; p < p0 + pp && ok; p++) {
 #pragma unroll
-            for (int c = 0; c < 4; c++)
+                for (int c = 0; c < T::EC / 2; c++) acc[0][c] = acc[1][c] = 0ull;
+                for (int i = 0; i < ns && ok; i++, sy.step()) {
+                    const uint8_t *sf = ps_tc_fact + sy.i * T::FACT;
+#pragma unroll 1
+                    for (int x = 0; x < 2; x++) {
+                        if (!ps_tc_wait(&bar_d_full[re.i], re.round)) { *a.err = 4; ok = false; break; } // the factors came with the stage
+                        ps_tc_fence_after();
+                        const float xd = *reinterpret_cast<const float *>(sf + x * PS_TC_A_D + row * 4);
+                        const ps_f2 x2 = ps_f2_pack(xd, xd);
+                        const ulonglong2 *yd = reinterpret_cast<const ulonglong2 *>(sf + 2 * PS_TC_A_D + (x * NT + c0) * 4);
+                        const uint32_t td = t_lane + re.i * (2 * T::CW);
 #pragma unroll
-                for (int l = 0; l < 12; l++) acc[c][l] = 0.f;
-            for (int i = 0; i < nb; i++, g++) {
-                const int s = g % PS_TC_STAGES, tb = g & 1;
-                if (!ps_tc_wait(&bar_tmem_full[tb], (g >> 1) & 1)) { *a.err = 4; ok = false; break; }
-                ps_tc_fence_after();
-                const uint8_t *st = ps_tc_smem + (size_t)s * PS_TC_STAGE;
-                const float2 xs = reinterpret_cast<const float2 *>(st + (size_t)17 * PS_TC_A_TILE)[row];
-                const float4 yd = *reinterpret_cast<const float4 *>(st + PS_TC_A_BLOCK + (size_t)20 * PS_TC_B_TILE + 4 * c0);
-                __syncwarp();
-                if (lane == 0) ps_mbar_arrive(&bar_empty[s]); // this warp no longer needs the stage
-                uint32_t v[12][4];
+                        for (int c = 0; c < T::EC; c += 8) {
+                            const ulonglong2 y0 = yd[c / 4], y1 = yd[c / 4 + 1];
+                            const ps_f2 dd[4] = {ps_f2_mul(y0.x, x2), ps_f2_mul(y0.y, x2), ps_f2_mul(y1.x, x2), ps_f2_mul(y1.y, x2)};
+                            ps_f2 v[8]; // the exact integers S_l (or P_k)
+                            ps_tc_ld8x2(td + c, td + T::CW + c, v);
+                            if (c + 8 == T::EC) { // the entry is in registers, the factors as well: both can be refilled
+                                ps_tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) {
+                                    ps_mbar_arrive(&bar_d_empty[re.i]);
+                                    if (x == 1) ps_mbar_arrive(&bar_y_empty[sy.i]);
+                                }
+                            }
 #pragma unroll
-                for (int l = 0; l < 12; l++)
-                    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(v[l][0]), "=r"(v[l][1]), "=r"(v[l][2]), "=r"(v[l][3])
-                                 : "r"(t_lane + tb * (12 * PS_TC_N) + l * PS_TC_N)
-                                 : "memory");
-                ps_tc_ld_wait();
-                ps_tc_fence_before();
-                __syncwarp();
-                if (lane == 0) ps_mbar_arrive(&bar_tmem_empty[tb]); // the integers are in registers: the buffer can be refilled
-                const float ydc[4] = {yd.x, yd.y, yd.z, yd.w};
+                            for (int k = 0; k < 4; k++) {
+                                acc[0][c / 2 + k] = ps_f2_fma(dd[k], v[k], acc[0][c / 2 + k]);
+                                acc[1][c / 2 + k] = ps_f2_fma(dd[k], v[4 + k], acc[1][c / 2 + k]);
+                            }
+                        }
+                        re.step();
+                        if (T::NH == 2) re.step();
+                    }
+                }
+                if (!ok) break;
+                // ---- the pass's number: first step of hsum_float_8 (lane l + 4 and lane l), or of the mins sum (m_k and m_k+2)
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const float d = __fmul_rn(ydc[c], xs.x), dm = __fmul_rn(-ydc[c], xs.y);
-#pragma unroll
-                    for (int l = 0; l < 12; l++) // v is the exact integer S_l (l < 8) / P_k (l >= 8)
-                        acc[c][l] = __fmaf_rn(l < 8 ? d : dm, __uint_as_float(v[l][c]), acc[c][l]);
+                for (int c = 0; c < T::EC / 2; c++) {
+                    float r0, r1;
+                    ps_f2_unpack(ps_f2_add(acc[1][c], acc[0][c]), r0, r1);
+                    if (p & 1) {
+                        if (pp > 1) { r0 = __fadd_rn(stash[(2 * c) * ET], r0); r1 = __fadd_rn(stash[(2 * c + 1) * ET], r1); }
+                        if (pp == PS_TC_PASSES) { // the running sum ((r04 + r26) + (r15 + r37)), then + (m02 + m13)
+                            if (p > 1) { r0 = __fadd_rn(whole[(2 * c) * ET], r0); r1 = __fadd_rn(whole[(2 * c + 1) * ET], r1); }
+                            if (p < 5) { whole[(2 * c) * ET] = r0; whole[(2 * c + 1) * ET] = r1; }
+                        }
+                    } else if (pp > 1) {
+                        stash[(2 * c) * ET] = r0;
+                        stash[(2 * c + 1) * ET] = r1;
+                    }
+                    acc[0][c] = ps_f2_pack(r0, r1);
                 }
             }
             if (!ok) break;
-            // ---- hsum_float_8 + mins sum (ggml-quants.c:62-68, 7862-7871), bias / residual, dst[col][row]
-            const int grow = rt * PS_TC_M + row;
+            if (nu > 1) { // hand the numbers over; the tile's last unit adds them in the fixed order
+#pragma unroll
+                for (int c = 0; c < T::EC / 2; c++) {
+                    float r0, r1;
+                    ps_f2_unpack(acc[0][c], r0, r1);
+                    __stcg(part + (2 * c) * ET, r0);
+                    __stcg(part + (2 * c + 1) * ET, r1);
+                }
+                __threadfence();
+                ps_bar_sync(1, ET);
+                if (tid == 0) {
+                    const int last = atomicAdd(a.cnt + tile, 1) == nu - 1;
+                    if (last) a.cnt[tile] = 0;
+                    sh_last = last;
+                }
+                ps_bar_sync(1, ET);
+                if (!sh_last) continue;
+                __threadfence();
+                const float *q = a.part + (size_t)tile * nu * (T::EC * ET) + tid;
+                constexpr int US = T::EC * ET;
+#pragma unroll
+                for (int c = 0; c < T::EC / 2; c++) {
+                    float r[2];
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const float *qc = q + (2 * c + k) * ET;
+                        if (nu == 3) r[k] = __fadd_rn(__fadd_rn(__ldcg(qc), __ldcg(qc + US)), __ldcg(qc + 2 * US));
+                        else
+                            r[k] = __fadd_rn(__fadd_rn(__fadd_rn(__ldcg(qc), __ldcg(qc + US)), __fadd_rn(__ldcg(qc + 2 * US), __ldcg(qc + 3 * US))),
+                                             __fadd_rn(__ldcg(qc + 4 * US), __ldcg(qc + 5 * US)));
+                    }
+                    acc[0][c] = ps_f2_pack(r[0], r[1]);
+                }
+            }
+            // ---- bias / residual, dst[col][row]
+            const int rt = tile / a.n_ct, ct = tile % a.n_ct, grow = rt * PS_TC_M + row;
             int sg = 0;
             if (a.n_seg > 1 && grow >= a.seg[1].row_begin) sg = 1;
             if (a.n_seg > 2 && grow >= a.seg[2].row_begin) sg = 2;
@@ -249,17 +566,19 @@ __global__ void __launch_bounds__(PS_TC_THREADS, 1) ps_k_tc_gemm(const PsTcArgs 
                 const int n = grow - a.seg[sg].row_begin, ld = a.seg[sg].row_end - a.seg[sg].row_begin;
                 const float bias = a.seg[sg].bias ? a.seg[sg].bias[n] : 0.f;
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int col = cg * PS_TC_N + c0 + c;
-                    if (col < a.bs) {
-                        const float r0 = __fadd_rn(acc[c][4], acc[c][0]), r1 = __fadd_rn(acc[c][5], acc[c][1]);
-                        const float r2 = __fadd_rn(acc[c][6], acc[c][2]), r3 = __fadd_rn(acc[c][7], acc[c][3]);
-                        float res = __fadd_rn(__fadd_rn(r0, r2), __fadd_rn(r1, r3));
-                        res = __fadd_rn(res, __fadd_rn(__fadd_rn(acc[c][8], acc[c][10]), __fadd_rn(acc[c][9], acc[c][11])));
-                        const size_t o = (size_t)col * ld + n;
-                        if (a.seg[sg].bias) res = __fadd_rn(res, bias);
-                        if (a.residual) res = __fadd_rn(a.residual[o], res);
-                        a.seg[sg].dst[o] = res;
+                for (int c = 0; c < T::EC / 2; c++) {
+                    float r[2];
+                    ps_f2_unpack(acc[0][c], r[0], r[1]);
+#pragma unroll
+                    for (int k = 0; k < 2; k++) {
+                        const int col = ct * NT + c0 + 2 * c + k;
+                        if (col < a.bs) {
+                            const size_t o = (size_t)col * ld + n;
+                            float res = r[k];
+                            if (a.seg[sg].bias) res = __fadd_rn(res, bias);
+                            if (a.residual) res = __fadd_rn(a.residual[o], res);
+                            a.seg[sg].dst[o] = res;
+                        }
                     }
                 }
             }
@@ -267,8 +586,8 @@ __global__ void __launch_bounds__(PS_TC_THREADS, 1) ps_k_tc_gemm(const PsTcArgs 
     }
     ps_tc_fence_before();
     __syncthreads();
-    if (warp == PS_TC_EPI_WARPS + 1) {
+    if (warp == W_MMA) {
         ps_tc_fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(T::TM_COLS) : "memory");
     }
 }

@@ -1,0 +1,49 @@
+"""GPU parity of the tensor-core GEMM behind token batches (powerserve_b200/csrc/ps_tc.cuh) at the edges of its tiling: batches on both
+sides of every column-tile width and over more than one column tile, matrices whose rows do not fill a 128-row tile (q | k | v segments
+that start on tile borders, biases), an odd number of super-blocks, and shapes for which a unit of work takes one, two or all six
+passes.  Oracle: the plain-C restatement of the reference; tolerance zero (the contract of this path)."""
+import numpy as np
+import pytest
+
+from powerserve_b200 import capi, gguf, synth
+from tests import _libs as L
+from tests import _model as M
+
+pytestmark = pytest.mark.gpu
+
+# 3 and 5 super-blocks; q 6, k and v 1.5 row tiles, gate / up 10, output 50 (all passes in one unit) and a bit
+ODD = synth.ModelShape("tc-odd", "llama", 768, 1280, 2, 8, 2, 96, 6400 + 24, False, 0, 5e5, 1e-5, gguf.GGML_Q4_K, n_ctx=512, qkv_bias=True)
+
+
+@pytest.fixture(scope="module")
+def odd(tmp_path_factory):
+    d = synth.write_model_dir(str(tmp_path_factory.mktemp("tc_odd")), ODD, seed=5)
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=200)
+    yield om, cm
+    om.close()
+    cm.close()
+
+
+@pytest.mark.parametrize("bs", [6, 16, 17, 32, 33, 64, 65, 96, 97, 128, 129, 200])
+def test_batch_widths(odd, bs):
+    om, cm = odd
+    tokens = synth.random_prompt(ODD.vocab_size, bs, seed=bs)
+    om.reset()
+    cm.reset()
+    n = cm.be.counter("tc_gemm_launches")
+    got = cm.forward(tokens)
+    assert cm.be.counter("tc_gemm_launches") > n
+    L.assert_bit_equal(got, om.forward(tokens), f"{bs} tokens")
+
+
+def test_two_passes_a_unit():
+    """layer shapes of an 8B model: 48 row tiles of q | k | v, three units of two passes each"""
+    d = M.model_dir("slice-8b")
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=32)
+    tokens = synth.random_prompt(2048, 20, seed=3)
+    L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), "8B slice, 20 tokens")
+    again = cm.forward(tokens[:9])          # the counters of the tiles are left as they were found
+    assert np.isfinite(again).all() and cm.be.counter("tc_error") == 0
+    L.assert_bit_equal(again, om.forward(tokens[:9]), "8B slice, 9 more tokens")
+    om.close()
+    cm.close()
