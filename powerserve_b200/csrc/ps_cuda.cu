@@ -115,8 +115,7 @@ struct ps_cuda_ctx {
     float *g = nullptr, *u = nullptr, *kq = nullptr, *logits = nullptr;
     const float *logits_last = nullptr; // where the last forward left its [bs][vocab] logits (ps_cuda_logits_dev)
     int logits_rows = 0;                // rows of that buffer
-    float *topk_val = nullptr;          // device top-k scratch: candidates [slices][k], then the result [k]
-    int *topk_idx = nullptr;
+    unsigned long long *topk_cand = nullptr; // device top-k scratch: keys of the slices' best, then the result: ids [PS_TOPK_MAX], values [PS_TOPK_MAX]
     uint32_t *aqs = nullptr, *absp = nullptr;
     float *ad = nullptr;
     int32_t *tokens_dev = nullptr, *pos_dev = nullptr, *ids_dev = nullptr;
@@ -2704,19 +2703,17 @@ int ps_cuda_sample_topk(ps_cuda_ctx *ctx, int row, int k, float *logits_out, int
     if (!logits_out || !tokens_out) return fail(ctx, PS_CUDA_ERR_INVALID, "sample_topk: null output");
     PS_CK(cudaSetDevice(ctx->device));
     const int n_slices = (vocab + PS_TOPK_SLICE - 1) / PS_TOPK_SLICE;
-    if (!ctx->topk_val) {
-        const size_t n = (size_t)((ctx->d.vocab_size + PS_TOPK_SLICE - 1) / PS_TOPK_SLICE + 1) * PS_TOPK_MAX;
+    if (!ctx->topk_cand) {
         int rc;
-        if ((rc = dev_alloc(ctx, (void **)&ctx->topk_val, n * 4)) || (rc = dev_alloc(ctx, (void **)&ctx->topk_idx, n * 4))) return rc;
+        if ((rc = dev_alloc(ctx, (void **)&ctx->topk_cand, (size_t)(n_slices + 1) * PS_TOPK_MAX * 8))) return rc;
     }
-    float *res_val = ctx->topk_val + (size_t)n_slices * PS_TOPK_MAX;
-    int *res_idx = ctx->topk_idx + (size_t)n_slices * PS_TOPK_MAX;
-    ps_k_topk_stage1<<<n_slices, 256, 0, ctx->stream>>>(ctx->logits_last + (size_t)row * vocab, vocab, k, ctx->topk_val, ctx->topk_idx);
+    int *res = reinterpret_cast<int *>(ctx->topk_cand + (size_t)n_slices * PS_TOPK_MAX);
+    const float *logits = ctx->logits_last + (size_t)row * vocab;
+    ps_k_topk_stage1<<<n_slices, 1024, 0, ctx->stream>>>(logits, vocab, k, ctx->topk_cand);
     PS_LAUNCH_CK();
-    ps_k_topk_stage2<<<1, 256, 0, ctx->stream>>>(ctx->topk_val, ctx->topk_idx, n_slices * k, k, res_val, res_idx);
+    ps_k_topk_stage2<<<1, 1024, 0, ctx->stream>>>(ctx->topk_cand, n_slices * k, k, logits, res, reinterpret_cast<float *>(res + PS_TOPK_MAX));
     PS_LAUNCH_CK();
-    PS_CK(cudaMemcpyAsync(ctx->h_ids, res_idx, (size_t)k * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    PS_CK(cudaMemcpyAsync(ctx->h_ids + PS_TOPK_MAX, res_val, (size_t)k * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    PS_CK(cudaMemcpyAsync(ctx->h_ids, res, PS_TOPK_MAX * 8, cudaMemcpyDeviceToHost, ctx->stream));
     int rc = sync_and_check(ctx);
     if (rc) return rc;
     memcpy(tokens_out, ctx->h_ids, (size_t)k * 4);

@@ -1224,70 +1224,56 @@ __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, con
 // ====================================================================================================================
 // Device-side top-k: TopKSampler (src/sampler/sampler.cpp:39-56: partial_sort by logit, descending) on the
 // device, so that k (logit, token) pairs cross PCIe instead of the vocabulary's logits and the host never builds a
-// vocabulary-sized ProbArray (prob_array.hpp:43-49).  Two stages of repeated arg-max: every CTA extracts the k largest of
-// its slice (kept in shared memory), then one CTA merges the candidates.  Order: logit descending, equal logits by
-// ascending token id (std::partial_sort leaves that order unspecified).
+// vocabulary-sized ProbArray (prob_array.hpp:43-49).  Order: logit descending, equal logits by ascending token id (std::partial_sort
+// leaves that order unspecified); NaNs are never chosen.
+// Latency bounds both stages (one 0.5 MB read).  k rounds of a block-wide arg-max took 50 us a slice and 70 us for the merge at k = 40 and
+// 128 256 logits; sorting takes as many rounds as log2 squared whatever k is.  A value and its id make one 64-bit key (larger = better),
+// every CTA sorts its slice and hands on its k best, one CTA sorts those.
 // ====================================================================================================================
 #define PS_TOPK_MAX 64
 #define PS_TOPK_SLICE 2048
-// the block's (largest value, lowest index) among the entries of v[0..n) that are not NaN (NaN marks "already taken");
-// returns the position in every thread, -1 if nothing is left
-PS_D bool ps_topk_better(float x, int id, float best, int bi) { return x == x && (!(best == best) || x > best || (x == best && id < bi)); }
-PS_D int ps_block_argmax_smem(const float *v, const int *idx, int n, float *sv, int *si, int *sp) {
-    float best = __int_as_float(0x7fc00000);
-    int bi = 0x7fffffff, bp = -1;
-    for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const float x = v[t];
-        const int id = idx ? idx[t] : t;
-        if (ps_topk_better(x, id, best, bi)) { best = x; bi = id; bp = t; }
-    }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        const float ov = __shfl_xor_sync(PS_FULL, best, o);
-        const int oi = __shfl_xor_sync(PS_FULL, bi, o), op = __shfl_xor_sync(PS_FULL, bp, o);
-        if (ps_topk_better(ov, oi, best, bi)) { best = ov; bi = oi; bp = op; }
-    }
-    const int warp = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { sv[warp] = best; si[warp] = bi; sp[warp] = bp; }
-    __syncthreads();
-    best = sv[0]; bi = si[0]; bp = sp[0];
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++)
-        if (ps_topk_better(sv[w], si[w], best, bi)) { best = sv[w]; bi = si[w]; bp = sp[w]; }
-    __syncthreads();
-    return bp;
+#define PS_TOPK_MERGE 4096
+PS_D unsigned long long ps_topk_key(float v, int id) { // 0: not a candidate
+    const uint32_t u = v == 0.f ? 0u : __float_as_uint(v);
+    if (v != v) return 0ull;
+    return ((unsigned long long)((u & 0x80000000u) ? ~u : (u | 0x80000000u)) << 32) | (uint32_t)~(uint32_t)id;
 }
-// stage 1: CTA b -> cand_val / cand_idx [b][k] = the k largest of logits[b * SLICE, (b + 1) * SLICE) (padded with -inf, id 0x7fffffff)
-__global__ void __launch_bounds__(256) ps_k_topk_stage1(const float *__restrict__ logits, int n, int k, float *__restrict__ cand_val, int *__restrict__ cand_idx) {
-    __shared__ float s_v[PS_TOPK_SLICE];
-    __shared__ float sv[8];
-    __shared__ int si[8], sp[8];
-    const int lo = blockIdx.x * PS_TOPK_SLICE, m = min(PS_TOPK_SLICE, n - lo);
-    for (int t = threadIdx.x; t < m; t += blockDim.x) s_v[t] = logits[lo + t];
+// descending bitonic sort of N (a power of two) keys in shared memory by the whole block
+template <int N> PS_D void ps_block_sort(unsigned long long *v) {
+    for (int size = 2; size <= N; size <<= 1)
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+            __syncthreads();
+            for (int t = threadIdx.x; t < N / 2; t += blockDim.x) {
+                const int i = 2 * t - (t & (stride - 1)), j = i + stride;
+                const unsigned long long x = v[i], y = v[j];
+                if ((x < y) == ((i & size) == 0)) { v[i] = y; v[j] = x; }
+            }
+        }
     __syncthreads();
-    for (int r = 0; r < k; r++) {
-        const int p = ps_block_argmax_smem(s_v, nullptr, m, sv, si, sp); // ids inside a slice ascend with the position
-        if (threadIdx.x == 0) {
-            const bool live = p >= 0;
-            cand_val[blockIdx.x * k + r] = live ? s_v[p] : __int_as_float(0x7fc00000); // NaN = no candidate (slice shorter than k)
-            cand_idx[blockIdx.x * k + r] = live ? lo + p : 0x7fffffff;
-            if (live) s_v[p] = __int_as_float(0x7fc00000); // a quiet NaN marks "taken"
-        }
-        __syncthreads();
-    }
 }
-// stage 2: one CTA merges n_cand candidates into out_val / out_idx [k]
-__global__ void __launch_bounds__(256) ps_k_topk_stage2(float *__restrict__ cand_val, const int *__restrict__ cand_idx, int n_cand, int k, float *__restrict__ out_val,
-                                                        int *__restrict__ out_idx) {
-    __shared__ float sv[8];
-    __shared__ int si[8], sp[8];
-    for (int r = 0; r < k; r++) {
-        const int p = ps_block_argmax_smem(cand_val, cand_idx, n_cand, sv, si, sp);
-        if (threadIdx.x == 0) {
-            out_val[r] = p >= 0 ? cand_val[p] : -INFINITY;
-            out_idx[r] = p >= 0 ? cand_idx[p] : -1;
-            if (p >= 0) cand_val[p] = __int_as_float(0x7fc00000);
-        }
-        __syncthreads();
+// stage 1: CTA b -> keys of the k largest of logits[b * SLICE, (b + 1) * SLICE)
+__global__ void __launch_bounds__(1024) ps_k_topk_stage1(const float *__restrict__ logits, int n, int k, unsigned long long *__restrict__ cand) {
+    __shared__ unsigned long long v[PS_TOPK_SLICE];
+    const int lo = blockIdx.x * PS_TOPK_SLICE;
+    for (int t = threadIdx.x; t < PS_TOPK_SLICE; t += blockDim.x) v[t] = lo + t < n ? ps_topk_key(logits[lo + t], lo + t) : 0ull;
+    ps_block_sort<PS_TOPK_SLICE>(v);
+    for (int t = threadIdx.x; t < k; t += blockDim.x) cand[blockIdx.x * k + t] = v[t];
+}
+// stage 2: one CTA merges n_cand candidates (in rounds that keep the k best so far at the front) into ids [k] and values [k]
+__global__ void __launch_bounds__(1024) ps_k_topk_stage2(const unsigned long long *__restrict__ cand, int n_cand, int k, const float *__restrict__ logits, int *__restrict__ out_idx,
+                                                         float *__restrict__ out_val) {
+    __shared__ unsigned long long v[PS_TOPK_MERGE];
+    int have = 0;
+    for (int lo = 0; lo < n_cand; have = k) {
+        const int m = min(PS_TOPK_MERGE - have, n_cand - lo);
+        for (int t = threadIdx.x; t < PS_TOPK_MERGE - have; t += blockDim.x) v[have + t] = t < m ? cand[lo + t] : 0ull;
+        ps_block_sort<PS_TOPK_MERGE>(v);
+        lo += m;
+    }
+    for (int t = threadIdx.x; t < k; t += blockDim.x) {
+        const int id = v[t] ? (int)~(uint32_t)v[t] : -1;
+        out_idx[t] = id;
+        out_val[t] = id >= 0 ? logits[id] : -INFINITY;
     }
 }
 
