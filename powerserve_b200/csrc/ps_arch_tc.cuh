@@ -129,10 +129,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
     constexpr int STAGES = NA == 1 ? 6 : 4;
     constexpr int STAGE_BYTES = (NA + 1) * PT_BLOCK;
     extern __shared__ __align__(1024) uint8_t pt_smem_raw[];
-    __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_tmem_full[2], bar_tmem_empty[2];
+    __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_tmem_full[2], bar_tmem_empty[2], bar_done;
     __shared__ uint32_t tmem_base_smem;
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)pt_smem_raw + 1023) & ~(uintptr_t)1023);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nkb = a.nkb, n_ct = a.n_ct_dev ? min(*a.n_ct_dev, a.n_ct) : a.n_ct;
     const int n_units = n_ct * a.n_rt;
     const int n_sub = max(a.n_sub, 1), tn = PT_N / n_sub; // tokens of a unit
@@ -141,6 +141,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
     if (tid == 0) {
         for (int s = 0; s < STAGES; s++) { ps_mbar_init(&bar_full[s], 1); ps_mbar_init(&bar_empty[s], 1); }
         for (int b = 0; b < 2; b++) { ps_mbar_init(&bar_tmem_full[b], 1); ps_mbar_init(&bar_tmem_empty[b], 4); }
+        ps_mbar_init(&bar_done, 1);
         ps_fence_barrier_init();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -154,57 +155,69 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
     const uint32_t tmem_base = tmem_base_smem;
 
     if (warp == 4) {
-        // ===== producer: one bulk copy per operand block
-        if (lane == 0) {
-            int g = 0;
-            bool ok = true;
-            for (int mu = 0; mu < my_units && ok; mu++) {
-                const int u = (int)blockIdx.x + mu * (int)gridDim.x, ct = u / a.n_rt, rt = u % a.n_rt;
-                const int64_t grp = a.tile_e ? a.tile_e[ct] : 0;
-                const uint8_t *pa0 = a.a0 + ((grp * a.n_rt + rt) * nkb) * (int64_t)PT_BLOCK;
-                const uint8_t *pa1 = NA == 2 ? a.a1 + ((grp * a.n_rt + rt) * nkb) * (int64_t)PT_BLOCK : nullptr;
-                const uint8_t *pb = a.b + ((int64_t)(ct / n_sub) * nkb) * PT_BLOCK + (ct % n_sub) * tn * 16;
-                for (int sg = 1; sg < a.seg.n; sg++)
-                    if (rt >= a.seg.rt[sg]) pb += a.seg.set_bytes;
-                for (int kb = 0; kb < nkb; kb++, g++) {
-                    const int s = g % STAGES;
-                    if (g >= STAGES && !ps_tc_wait(&bar_empty[s], ((g / STAGES) - 1) & 1)) { *a.err = 1; ok = false; break; }
-                    uint8_t *st = smem + (size_t)s * STAGE_BYTES;
-                    ps_mbar_expect_tx(&bar_full[s], NA * PT_BLOCK + PT_BLOCK / n_sub);
-                    ps_bulk_g2s(st, pa0 + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[s]);
-                    if (NA == 2) ps_bulk_g2s(st + PT_BLOCK, pa1 + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[s]);
-                    if (n_sub == 1) ps_bulk_g2s(st + NA * PT_BLOCK, pb + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[s]);
+        // ===== producer: one bulk copy per operand block.  Producer and issuer stay converged warps and act through one elected thread: under
+        // `lane == 0` descriptors and addresses go through vector registers and an MMA took 280 cycles to issue (128 x 128 x 16 itself: 64)
+        PsRing<STAGES> st;
+        int g = 0;
+        bool ok = true;
+        for (int mu = 0; mu < my_units && ok; mu++) {
+            const int u = (int)blockIdx.x + mu * (int)gridDim.x, ct = u / a.n_rt, rt = u % a.n_rt;
+            const int64_t grp = a.tile_e ? a.tile_e[ct] : 0;
+            const uint8_t *pa0 = a.a0 + ((grp * a.n_rt + rt) * nkb) * (int64_t)PT_BLOCK;
+            const uint8_t *pa1 = NA == 2 ? a.a1 + ((grp * a.n_rt + rt) * nkb) * (int64_t)PT_BLOCK : nullptr;
+            const uint8_t *pb = a.b + ((int64_t)(ct / n_sub) * nkb) * PT_BLOCK + (ct % n_sub) * tn * 16;
+            for (int sg = 1; sg < a.seg.n; sg++)
+                if (rt >= a.seg.rt[sg]) pb += a.seg.set_bytes;
+            for (int kb = 0; kb < nkb; kb++, g++, st.step()) {
+                if (g >= STAGES && !ps_tc_wait(&bar_empty[st.i], st.round ^ 1)) { *a.err = 1; ok = false; break; }
+                uint8_t *sm = smem + (size_t)st.i * STAGE_BYTES;
+                uint64_t *bar = &bar_full[st.i];
+                if (ps_elect_one()) {
+                    ps_mbar_expect_tx(bar, NA * PT_BLOCK + PT_BLOCK / n_sub);
+                    ps_bulk_g2s(sm, pa0, PT_BLOCK, bar);
+                    if (NA == 2) ps_bulk_g2s(sm + PT_BLOCK, pa1, PT_BLOCK, bar);
+                    if (n_sub == 1) ps_bulk_g2s(sm + NA * PT_BLOCK, pb, PT_BLOCK, bar);
                     else // the part's tokens of every k-chunk, at the places they have in the whole tile
-                        for (int c = 0; c < 8; c++) ps_bulk_g2s(st + NA * PT_BLOCK + c * 2048, pb + (int64_t)kb * PT_BLOCK + c * 2048, (uint32_t)(tn * 16), &bar_full[s]);
+#pragma unroll
+                        for (int c = 0; c < 8; c++) ps_bulk_g2s(sm + NA * PT_BLOCK + c * 2048, pb + c * 2048, (uint32_t)(tn * 16), bar);
                 }
+                __syncwarp();
+                pa0 += PT_BLOCK;
+                pa1 += PT_BLOCK;
+                pb += PT_BLOCK;
             }
         }
+        for (int k = g > STAGES ? g - STAGES : 0; k < g; k++) // copies in flight end before the CTA does (they have, unless a wait gave up)
+            if (!ps_tc_wait(&bar_full[k % STAGES], (k / STAGES) & 1)) { *a.err = 5; break; }
     } else if (warp == 5) {
         // ===== MMA issuer: kind::f16 with bfloat16 operands (a_format = b_format = 1), fp32 accumulators, K-major both
-        if (lane == 0) {
-            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(PT_M >> 4) << 24);
-            int g = 0;
-            bool ok = true;
-            for (int mu = 0; mu < my_units && ok; mu++) {
-                const int tb = mu & 1;
-                if (mu >= 2 && !ps_tc_wait(&bar_tmem_empty[tb], ((mu >> 1) - 1) & 1)) { *a.err = 3; break; }
-                const uint32_t td = tmem_base + tb * (NA * PT_N);
-                for (int kb = 0; kb < nkb; kb++, g++) {
-                    const int s = g % STAGES;
-                    if (!ps_tc_wait(&bar_full[s], (g / STAGES) & 1)) { *a.err = 2; ok = false; break; }
-                    ps_tc_fence_after();
-                    const uint32_t sa = ps_smem_u32(smem + (size_t)s * STAGE_BYTES), sb = sa + NA * PT_BLOCK;
+        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(tn >> 3) << 17) | ((uint32_t)(PT_M >> 4) << 24);
+        const uint64_t desc0 = ps_tc_smem_desc(ps_smem_u32(smem), 2048, 128);
+        PsRing<STAGES> st;
+        bool ok = true;
+        for (int mu = 0; mu < my_units && ok; mu++) {
+            const int tb = mu & 1;
+            if (mu >= 2 && !ps_tc_wait(&bar_tmem_empty[tb], ((mu >> 1) - 1) & 1)) { *a.err = 3; break; }
+            const uint32_t td = tmem_base + tb * (NA * PT_N);
+            for (int kb = 0; kb < nkb; kb++, st.step()) {
+                if (!ps_tc_wait(&bar_full[st.i], st.round)) { *a.err = 2; ok = false; break; }
+                ps_tc_fence_after();
+                const uint64_t da = desc0 + (uint64_t)(st.i * (STAGE_BYTES >> 4));
+                if (ps_elect_one()) {
 #pragma unroll
                     for (int j = 0; j < PT_KB / 16; j++) {
-                        const uint64_t bd = ps_tc_smem_desc(sb + j * 4096, 2048, 128);
-                        ps_tc_mma_f16(td, ps_tc_smem_desc(sa + j * 4096, 2048, 128), bd, idesc, (kb | j) != 0);
-                        if (NA == 2) ps_tc_mma_f16(td + PT_N, ps_tc_smem_desc(sa + PT_BLOCK + j * 4096, 2048, 128), bd, idesc, (kb | j) != 0);
+                        ps_tc_mma_f16(td, da + j * 256, da + NA * (PT_BLOCK >> 4) + j * 256, idesc, (kb | j) != 0);
+                        if (NA == 2) ps_tc_mma_f16(td + PT_N, da + (PT_BLOCK >> 4) + j * 256, da + NA * (PT_BLOCK >> 4) + j * 256, idesc, (kb | j) != 0);
                     }
-                    ps_tc_commit(&bar_empty[s]);
+                    ps_tc_commit(&bar_empty[st.i]);
+                    if (kb == nkb - 1) ps_tc_commit(&bar_tmem_full[tb]);
                 }
-                if (ok) ps_tc_commit(&bar_tmem_full[tb]);
+                __syncwarp();
             }
         }
+        if (ps_elect_one()) ps_tc_commit(&bar_done); // MMAs in flight end before the tensor memory is given back
+        __syncwarp();
+        if (!ps_tc_wait(&bar_done, 0)) *a.err = 6;
     } else {
         // ===== epilogue: warp w reads tensor-memory lanes 32 w .. 32 w + 31 = 32 consecutive output features
         for (int mu = 0; mu < my_units; mu++) {

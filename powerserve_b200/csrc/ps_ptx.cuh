@@ -95,3 +95,11 @@ PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity) {
     return false;
 }
 
+// position in a ring of N: index and the parity of the round
+template <int N> struct PsRing {
+    int i = 0;
+    uint32_t round = 0;
+    PS_D void step() {
+        if (++i == N) { i = 0; round ^= 1; }
+    }
+};

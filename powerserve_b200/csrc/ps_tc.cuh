@@ -231,15 +231,6 @@ PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity) {
     return false;
 }
 
-// position in a ring of N: index and the parity of the round
-template <int N> struct PsRing {
-    int i = 0;
-    uint32_t round = 0;
-    PS_D void step() {
-        if (++i == N) { i = 0; round ^= 1; }
-    }
-};
-
 // Persistent CTAs over units u = tile * (6 / pp) + group; tile = row tile * n_ct + column tile.
 template <int NT>
 __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gemm(const PsTcArgs a) {
