@@ -313,12 +313,40 @@ int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t
     return 0;
 }
 
-template <int TYPE>
-int launch_mm_t(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t N, int64_t bs, const float *bias, const float *residual) {
-    if (bs == 1) return launch_mm<TYPE, 1>(ctx, dst, w, K, N, bs, bias, residual);
-    if (bs == 2) return launch_mm<TYPE, 2>(ctx, dst, w, K, N, bs, bias, residual);
-    if (bs <= 4) return launch_mm<TYPE, 4>(ctx, dst, w, K, N, bs, bias, residual);
-    return launch_mm<TYPE, 8>(ctx, dst, w, K, N, bs, bias, residual);
+// one column: a warp per row (ps_k_matmul_q); more: a thread per AVX lane of a row (ps_k_matmul_qb).  Columns a thread keeps: as few as the
+// batch needs, up to eight (the accumulators of two rows x eight columns, twice that with mins, leave the loads in flight their registers)
+template <int TYPE, int C> int launch_mb(ps_cuda_ctx *ctx, PsMbArgs a) {
+    constexpr int R = 2, ROWS = PS_MB_WARPS * 4 * R;
+    static bool attr_set[64] = {};
+    const size_t smem = ps_mb_smem<TYPE>(a.K, C);
+    if (smem > 48 * 1024 && !attr_set[ctx->device]) {
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_qb<TYPE, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_set[ctx->device] = true;
+    }
+    int cta = 0;
+    for (int t = 0; t < a.n_seg; t++) { a.seg[t].cta0 = cta; cta += (a.seg[t].n + ROWS - 1) / ROWS; }
+    ps_k_matmul_qb<TYPE, R, C><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), PS_MB_WARPS * 32, smem, ctx->stream>>>(a);
+    PS_LAUNCH_CK();
+    return 0;
+}
+template <int TYPE> int launch_mb_t(ps_cuda_ctx *ctx, const PsMbArgs &a) {
+    if (a.bs <= 2) return launch_mb<TYPE, 2>(ctx, a);
+    if (a.bs <= 4 || ps_mb_smem<TYPE>(a.K, 8) > 200 * 1024) return launch_mb<TYPE, 4>(ctx, a);
+    return launch_mb<TYPE, 8>(ctx, a);
+}
+// up to three matrices of one type that read the same quantised input
+int matmul_qb(ps_cuda_ctx *ctx, int wtype, int64_t K, int64_t bs, const PsMbSeg *segs, int n_seg, const float *residual) {
+    PsMbArgs a{};
+    for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
+    a.n_seg = n_seg; a.bs = (int)bs; a.K = K; a.aqs = ctx->aqs; a.ad = ctx->ad; a.absp = ctx->absp; a.residual = residual;
+    switch (wtype) {
+    case 12: return launch_mb_t<12>(ctx, a);
+    case 13: return launch_mb_t<13>(ctx, a);
+    case 14: return launch_mb_t<14>(ctx, a);
+    case 2: return launch_mb_t<2>(ctx, a);
+    case 8: return launch_mb_t<8>(ctx, a);
+    default: return fail(ctx, PS_CUDA_ERR_UNSUPPORTED, "matmul: unsupported weight type %d", wtype);
+    }
 }
 
 // quantise bs activation columns of K elements into the context's scratch (type of the WEIGHT decides the format)
@@ -340,12 +368,16 @@ int quantize_act(ps_cuda_ctx *ctx, int wtype, const float *x, int64_t K, int64_t
 // matmul on already-quantised activations (the reference re-quantises the same input for q, k, v and for gate, up;
 // the bytes are identical, so once is enough)
 int matmul_q(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int wtype, int64_t K, int64_t N, int64_t bs, const float *bias, const float *residual) {
+    if (bs > 1) {
+        const PsMbSeg sg = {w, dst, bias, (int)N, 0};
+        return matmul_qb(ctx, wtype, K, bs, &sg, 1, residual);
+    }
     switch (wtype) {
-    case 12: return launch_mm_t<12>(ctx, dst, w, K, N, bs, bias, residual);
-    case 13: return launch_mm_t<13>(ctx, dst, w, K, N, bs, bias, residual);
-    case 14: return launch_mm_t<14>(ctx, dst, w, K, N, bs, bias, residual);
-    case 2: return launch_mm_t<2>(ctx, dst, w, K, N, bs, bias, residual);
-    case 8: return launch_mm_t<8>(ctx, dst, w, K, N, bs, bias, residual);
+    case 12: return launch_mm<12, 1>(ctx, dst, w, K, N, 1, bias, residual);
+    case 13: return launch_mm<13, 1>(ctx, dst, w, K, N, 1, bias, residual);
+    case 14: return launch_mm<14, 1>(ctx, dst, w, K, N, 1, bias, residual);
+    case 2: return launch_mm<2, 1>(ctx, dst, w, K, N, 1, bias, residual);
+    case 8: return launch_mm<8, 1>(ctx, dst, w, K, N, 1, bias, residual);
     default: return fail(ctx, PS_CUDA_ERR_UNSUPPORTED, "matmul: unsupported weight type %d", wtype);
     }
 }
@@ -2086,9 +2118,15 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = launch_rwm(ctx, a))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tq, ctx->xn, dim, bs))) return rc;
-            if ((rc = matmul_q(ctx, ctx->q, ld.wq, ld.tq, dim, qdim, bs, d.qkv_bias ? ld.q_bias : nullptr, nullptr))) return rc;
-            if ((rc = matmul_q(ctx, ctx->k, ld.wk, ld.tk, dim, kvd, bs, d.qkv_bias ? ld.k_bias : nullptr, nullptr))) return rc;
-            if ((rc = matmul_q(ctx, ctx->v, ld.wv, ld.tv, dim, kvd, bs, d.qkv_bias ? ld.v_bias : nullptr, nullptr))) return rc;
+            const PsMbSeg sg[3] = {{ld.wq, ctx->q, d.qkv_bias ? ld.q_bias : nullptr, (int)qdim, 0}, {ld.wk, ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)kvd, 0},
+                                   {ld.wv, ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)kvd, 0}};
+            if (bs > 1 && ld.tq == ld.tk && ld.tq == ld.tv) {
+                if ((rc = matmul_qb(ctx, ld.tq, dim, bs, sg, 3, nullptr))) return rc;
+            } else {
+                const int ty[3] = {ld.tq, ld.tk, ld.tv};
+                for (int t = 0; t < 3; t++)
+                    if ((rc = matmul_q(ctx, sg[t].dst, sg[t].w, ty[t], dim, sg[t].n, bs, sg[t].bias, nullptr))) return rc;
+            }
         }
         ps_k_rope<<<dim3((unsigned)nh, (unsigned)bs), 64, 0, ctx->stream>>>(ctx->qr, ctx->q, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
         PS_LAUNCH_CK();
@@ -2143,8 +2181,13 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 1, 2, ctx->u, bs, nullptr, nullptr))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tgate, ctx->xn, dim, bs))) return rc;
-            if ((rc = matmul_q(ctx, ctx->g, ld.wgate, ld.tgate, dim, ffn, bs, nullptr, nullptr))) return rc;
-            if ((rc = matmul_q(ctx, ctx->u, ld.wup, ld.tup, dim, ffn, bs, nullptr, nullptr))) return rc;
+            if (bs > 1 && ld.tgate == ld.tup) {
+                const PsMbSeg sg[2] = {{ld.wgate, ctx->g, nullptr, (int)ffn, 0}, {ld.wup, ctx->u, nullptr, (int)ffn, 0}};
+                if ((rc = matmul_qb(ctx, ld.tgate, dim, bs, sg, 2, nullptr))) return rc;
+            } else {
+                if ((rc = matmul_q(ctx, ctx->g, ld.wgate, ld.tgate, dim, ffn, bs, nullptr, nullptr))) return rc;
+                if ((rc = matmul_q(ctx, ctx->u, ld.wup, ld.tup, dim, ffn, bs, nullptr, nullptr))) return rc;
+            }
         }
         ps_k_silu_hadamard<<<grid1d(ffn * bs), 256, 0, ctx->stream>>>(ctx->g, ctx->g, ctx->u, ffn * bs);
         PS_LAUNCH_CK();

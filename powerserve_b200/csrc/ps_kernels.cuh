@@ -436,6 +436,164 @@ __global__ void __launch_bounds__(256) ps_k_matmul_q(const uint8_t *__restrict__
     }
 }
 
+// The same for a batch (two columns and more): a thread owns ONE AVX lane of R rows and advances their chains for C columns, so nothing
+// travels between lanes and a weight word is unpacked once for C columns; the eight lanes of a row add up at the end.  The old
+// layout - 32 lanes to a row, four blocks side by side - spent two shuffles per chain step and column and re-read the row for
+// every eight columns.  Bound by instruction issue: with 32-element blocks a chain step is dp4a (its start value 1.5 * 2^23 makes the
+// sum a float that one subtraction turns into the exact integer), subtraction, factor, FMA; one 16-byte shared-memory load brings
+// four steps.  4 x 8 rows a CTA: the 896-row matrices of a 0.5B model then fill 112 CTAs at 32 columns.
+// Up to three matrices of one type that read the same input run in one launch (q | k | v, gate | up).
+#define PS_MB_WARPS 4
+struct PsMbSeg { const uint8_t *w; float *dst; const float *bias; int n, cta0; };
+struct PsMbArgs {
+    PsMbSeg seg[3];
+    int n_seg, bs;
+    int64_t K;
+    const uint32_t *aqs; const float *ad; const uint32_t *absp;
+    const float *residual;
+};
+template <int TYPE> PS_HD size_t ps_mb_smem(int64_t K, int C) {
+    if (PsBlk<TYPE>::ELEMS == 256) return (size_t)C * (size_t)(K + K / 256 * 20);
+    const int64_t nbg = (K / 32 + 3) / 4; // groups of four blocks, the last one padded with zeros
+    return (size_t)C * (size_t)nbg * (128 + 16);
+}
+template <int TYPE, int R, int C>
+__global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArgs a) {
+    using B = PsBlk<TYPE>;
+    constexpr bool KQ = (B::ELEMS == 256);
+    extern __shared__ __align__(16) uint8_t smem[];
+    const int nb = (int)(a.K / B::ELEMS), col0 = blockIdx.y * C, ncol = min(C, a.bs - col0);
+    int sg = 0;
+    if (a.n_seg > 1 && (int)blockIdx.x >= a.seg[1].cta0) sg = 1;
+    if (a.n_seg > 2 && (int)blockIdx.x >= a.seg[2].cta0) sg = 2;
+    const PsMbSeg &seg = a.seg[sg];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 7;
+    const int row0 = (((int)blockIdx.x - seg.cta0) * PS_MB_WARPS + warp) * 4 * R + (lane >> 3); // rows row0, row0 + 4, ...
+    float acc[R][C], accm[B::HAS_MIN ? R : 1][C];
+#pragma unroll
+    for (int t = 0; t < R; t++)
+#pragma unroll
+        for (int c = 0; c < C; c++) { acc[t][c] = 0.f; if (B::HAS_MIN) accm[t][c] = 0.f; }
+    if constexpr (KQ) {
+        uint4 *s_qs = reinterpret_cast<uint4 *>(smem);                              // [C][nb][2][8] as quantised
+        float *s_d = reinterpret_cast<float *>(s_qs + (size_t)C * nb * 16);         // [C][nb]
+        uint32_t *s_bsp = reinterpret_cast<uint32_t *>(s_d + (size_t)C * nb);       // [C][nb * 4]
+        for (int c = 0; c < C; c++) {
+            const bool in = c < ncol;
+            const uint4 *src = reinterpret_cast<const uint4 *>(a.aqs + (int64_t)(col0 + c) * nb * 64);
+            for (int t = threadIdx.x; t < nb * 16; t += blockDim.x) s_qs[c * nb * 16 + t] = in ? src[t] : make_uint4(0, 0, 0, 0);
+            for (int t = threadIdx.x; t < nb; t += blockDim.x) s_d[c * nb + t] = in ? a.ad[(int64_t)(col0 + c) * nb + t] : 0.f;
+            for (int t = threadIdx.x; t < nb * 4; t += blockDim.x) s_bsp[c * nb * 4 + t] = in ? a.absp[(int64_t)(col0 + c) * nb * 4 + t] : 0u;
+        }
+        __syncthreads();
+        const uint8_t *wr[R];
+#pragma unroll
+        for (int t = 0; t < R; t++) wr[t] = seg.w + (int64_t)min(row0 + 4 * t, seg.n - 1) * nb * B::BYTES; // rows past the end repeat the last one
+        B next[R];
+#pragma unroll
+        for (int t = 0; t < R; t++) next[t].load(wr[t], l);
+        for (int i = 0; i < nb; i++) {
+            B blk[R];
+#pragma unroll
+            for (int t = 0; t < R; t++) {
+                blk[t] = next[t];
+                next[t].load(wr[t] + (int64_t)min(i + 1, nb - 1) * B::BYTES, l);
+            }
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const PsActQ8K x{s_qs + c * nb * 16, s_d + c * nb, s_bsp + c * nb * 4};
+#pragma unroll
+                for (int t = 0; t < R; t++) {
+                    int S, P;
+                    float d, dm;
+                    blk[t].partial(x, i, l, S, d, P, dm);
+                    acc[t][c] = __fmaf_rn(d, __int2float_rn(S), acc[t][c]);
+                    if constexpr (B::HAS_MIN && B::MIN_SCALAR) { // summs += dmin * hsum(prod): multiply, then add (Q5_K); lane l holds prod lane l % 4
+                        P += __shfl_xor_sync(PS_FULL, P, 1);
+                        P += __shfl_xor_sync(PS_FULL, P, 2);
+                        accm[t][c] = __fadd_rn(accm[t][c], __fmul_rn(dm, __int2float_rn(P)));
+                    } else if constexpr (B::HAS_MIN) {
+                        accm[t][c] = __fmaf_rn(dm, __int2float_rn(P), accm[t][c]);
+                    }
+                }
+            }
+        }
+    } else {
+        const int nbg = (nb + 3) / 4;
+        uint32_t *s_qs = reinterpret_cast<uint32_t *>(smem);                        // [C][group][8 lanes][4 blocks]
+        float *s_d = reinterpret_cast<float *>(s_qs + (size_t)C * nbg * 32);        // [C][group][4 blocks]
+        for (int c = 0; c < C; c++) {
+            const uint32_t *src = a.aqs + (int64_t)(col0 + c) * nb * 8;
+            for (int t = threadIdx.x; t < nbg * 32; t += blockDim.x) {
+                const int i = t >> 3, w = t & 7; // natural order: word w of block i
+                s_qs[c * nbg * 32 + ((i >> 2) * 8 + w) * 4 + (i & 3)] = c < ncol && i < nb ? src[t] : 0u;
+            }
+            for (int t = threadIdx.x; t < nbg * 4; t += blockDim.x) s_d[c * nbg * 4 + t] = c < ncol && t < nb ? a.ad[(int64_t)(col0 + c) * nb + t] : 0.f;
+        }
+        __syncthreads();
+        const uint8_t *wr[R];
+#pragma unroll
+        for (int t = 0; t < R; t++) wr[t] = seg.w + (int64_t)min(row0 + 4 * t, seg.n - 1) * nb * B::BYTES;
+        B next[R][4];
+        auto fetch = [&](int g) { // blocks past the end repeat the last one: their activation words and factors are zero
+#pragma unroll
+            for (int t = 0; t < R; t++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) next[t][b].load(wr[t] + (int64_t)min(4 * g + b, nb - 1) * B::BYTES, l);
+        };
+        fetch(0);
+        for (int g = 0; g < nbg; g++) {
+            int q[R][4];
+            float xd[R][4];
+#pragma unroll
+            for (int t = 0; t < R; t++)
+#pragma unroll
+                for (int b = 0; b < 4; b++) { q[t][b] = (int)next[t][b].q; xd[t][b] = next[t][b].xd; }
+            fetch(min(g + 1, nbg - 1));
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const uint4 y = *reinterpret_cast<const uint4 *>(s_qs + ((size_t)(c * nbg + g) * 8 + l) * 4);
+                const float4 yd = *reinterpret_cast<const float4 *>(s_d + (size_t)(c * nbg + g) * 4);
+                const int yw[4] = {(int)y.x, (int)y.y, (int)y.z, (int)y.w};
+                const float ydv[4] = {yd.x, yd.y, yd.z, yd.w};
+#pragma unroll
+                for (int b = 0; b < 4; b++)
+#pragma unroll
+                    for (int t = 0; t < R; t++) {
+                        const float S = __fsub_rn(__int_as_float(__dp4a(q[t][b], yw[b], 0x4B400000)), 12582912.f); // |sum| < 2^17: exact
+                        acc[t][c] = __fmaf_rn(__fmul_rn(xd[t][b], ydv[b]), S, acc[t][c]);
+                    }
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < R; t++) {
+        const int n = row0 + 4 * t;
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            // hsum_float_8 over the row's eight lanes: (x4 + x0), (x6 + x2), (x5 + x1), (x7 + x3)
+            float r = acc[t][c];
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 4));
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 2));
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 1));
+            if constexpr (B::HAS_MIN && B::MIN_SCALAR) {
+                r = __fadd_rn(r, accm[t][c]); // hsum_float_8(acc) + summs
+            } else if constexpr (B::HAS_MIN) { // (m0 + m2) + (m1 + m3); lane l holds m_(l % 4)
+                float m = accm[t][c];
+                m = __fadd_rn(m, __shfl_xor_sync(PS_FULL, m, 2));
+                m = __fadd_rn(m, __shfl_xor_sync(PS_FULL, m, 1));
+                r = __fadd_rn(r, m);
+            }
+            if (l == c % 8 && c < ncol && n < seg.n) {
+                const int64_t o = (int64_t)(col0 + c) * seg.n + n;
+                if (seg.bias) r = __fadd_rn(r, seg.bias[n]);      // GGMLBackend::add with row broadcast (Qwen2 q/k/v bias)
+                if (a.residual) r = __fadd_rn(a.residual[o], r);  // residual add: x + W.h  (powerserve_compute_forward_add)
+                seg.dst[o] = r;
+            }
+        }
+    }
+}
+
 // ====================================================================================================================
 // Small fp32 operators
 // ====================================================================================================================
