@@ -1140,6 +1140,15 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
     return 0;
 }
 
+// fp32-FMA products: 64 x 64 tiles, or 32 x 64 ones where 64-row tiles would leave SMs without a tile (150 tokens x 1024 outputs, K 1024 and
+// 2048 in turn: 48 tiles of 64 rows 104 us, 80 of 32 rows 81 us; with more tiles than SMs the wider tile reads its operands less often)
+static bool pa_narrow_tiles(int n_sm, int N, int bs, int heads) { return (int64_t)((N + PA_TN - 1) / PA_TN) * ((bs + PA_TM - 1) / PA_TM) * heads < n_sm; }
+template <bool ROUND, typename... Args> static void pa_launch_linear(int n_sm, int N, int bs, int heads, cudaStream_t st, Args... args) {
+    const unsigned nt = (unsigned)((N + PA_TN - 1) / PA_TN);
+    if (pa_narrow_tiles(n_sm, N, bs, heads)) pa_k_linear<ROUND, 32><<<dim3(nt, (unsigned)((bs + 31) / 32), (unsigned)heads), 256, 0, st>>>(args...);
+    else pa_k_linear<ROUND><<<dim3(nt, (unsigned)((bs + PA_TM - 1) / PA_TM), (unsigned)heads), 256, 0, st>>>(args...);
+}
+
 template <bool ROUND>
 static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_head, std::string &err) {
     const ps_cuda_arch_desc &d = a->d;
@@ -1194,13 +1203,13 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     // y = X W^T for a batch: tensor cores on rounded operands, or the fp32-FMA tiles
     auto linear = [&](const float *X, int ldx, int K, const bf16 *W, const uint8_t *Wt, int N, float *Cout, int ldc) -> int {
         if (tc) return tc_dense(X, ldx, bs, K, Wt, N, nullptr, Cout, ldc);
-        pa_k_linear<ROUND><<<dim3(cdiv(N, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(X, ldx, W, nullptr, Cout, ldc, bs, N, K, 0, 0);
+        pa_launch_linear<ROUND>(a->n_sm, N, bs, 1, st, X, ldx, W, nullptr, Cout, ldc, bs, N, K, 0, 0);
         PA_LAUNCH();
         return 0;
     };
     // per-head products (blockIdx.z = head): fp32-FMA tiles in both modes
     auto linear_heads = [&](const float *X, int ldx, int x_gs, int K, const bf16 *W, int N, float *Cout, int ldc, int c_gs, int heads) -> int {
-        pa_k_linear<ROUND><<<dim3(cdiv(N, PA_TN), cdiv(bs, PA_TM), (unsigned)heads), blk, 0, st>>>(X, ldx, W, nullptr, Cout, ldc, bs, N, K, x_gs, c_gs);
+        pa_launch_linear<ROUND>(a->n_sm, N, bs, (int)heads, st, X, ldx, W, nullptr, Cout, ldc, bs, N, K, x_gs, c_gs);
         PA_LAUNCH();
         return 0;
     };
@@ -1506,7 +1515,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             if (tc) {
                 if ((rc = tc_dense(a->x, dim, bs, dim, w.t_tg, td, nullptr, a->tg, td, &gelu, 0, 0, &mul))) return rc;
             } else {
-                pa_k_linear<ROUND><<<dim3(cdiv(td, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(a->x, dim, w.wtg, nullptr, a->tg, td, bs, td, dim, 0, 0, 0, 0, gelu, mul);
+                pa_launch_linear<ROUND>(a->n_sm, td, bs, 1, st, a->x, dim, w.wtg, nullptr, a->tg, td, bs, td, dim, 0, 0, 0, 0, gelu, mul);
                 PA_LAUNCH();
             }
             if ((rc = linear(a->tg, td, td, w.wtp, w.t_tp, dim, a->ty, dim))) return rc;
@@ -1564,7 +1573,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                 PA_LAUNCH();
                 for (int k = 0; k < w.seg.n; k++) {
                     const int r0 = w.seg.row[k], n = w.seg.row[k + 1] - r0;
-                    pa_k_linear<ROUND><<<dim3(cdiv(n, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(k ? a->mixb + (int64_t)(k - 1) * B * dim : a->h, dim, w.wqkv + (int64_t)r0 * dim, nullptr, a->qkv + r0, w.pw, bs, n, dim, 0,
+                    pa_launch_linear<ROUND>(a->n_sm, n, bs, 1, st, k ? a->mixb + (int64_t)(k - 1) * B * dim : a->h, dim, w.wqkv + (int64_t)r0 * dim, nullptr, a->qkv + r0, w.pw, bs, n, dim, 0,
                                                                                             0, r0 == w1_off ? 0 : 1 << 30, 0, tanh_act);
                     PA_LAUNCH();
                 }
@@ -1787,7 +1796,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             if (tc) {
                 if ((rc = tc_dense(a->h, dim, bs, dim, w.t_qkv, n1, w.bqkv, a->qkv, w.ldp, w.upn > 0 ? &act : nullptr, w.pw, gap))) return rc;
             } else {
-                pa_k_linear<ROUND><<<dim3(cdiv(n1, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(a->h, dim, w.wqkv, w.bqkv, a->qkv, w.ldp, bs, n1, dim, 0, 0, w.pw, gap, act);
+                pa_launch_linear<ROUND>(a->n_sm, n1, bs, 1, st, a->h, dim, w.wqkv, w.bqkv, a->qkv, w.ldp, bs, n1, dim, 0, 0, w.pw, gap, act);
                 PA_LAUNCH();
             }
         }
@@ -1802,7 +1811,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             } else {
                 pa_k_short_conv<<<dim3(cdiv(g.W, 256), bs), 256, 0, st>>>(g.x, w.ldp, w.conv_w, w.conv_b, g.W, g.taps, g.ring, 0, a->cv, g.W, io.pos_dev, 1);
                 PA_LAUNCH();
-                pa_k_linear<false><<<dim3(cdiv(2 * g.bsz, PA_TN), cdiv(bs, PA_TM), (unsigned)l.rec_blocks), blk, 0, st>>>(a->cv, g.W, w.wri, nullptr, a->gts, 2 * g.W, bs, 2 * g.bsz, g.bsz, g.bsz, 2 * g.bsz);
+                pa_launch_linear<false>(a->n_sm, 2 * g.bsz, bs, (int)l.rec_blocks, st, a->cv, g.W, w.wri, nullptr, a->gts, 2 * g.W, bs, 2 * g.bsz, g.bsz, g.bsz, 2 * g.bsz);
                 PA_LAUNCH();
                 pa_k_rglru_scan<<<cdiv(g.W, 32), PA_GG_THREADS, 0, st>>>(g);
                 PA_LAUNCH();
@@ -1930,7 +1939,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             int rc = tc_dense(a->h, dim, bs, dim, w.t_qkv, nqkv, w.bqkv, a->qkv, nqkv);
             if (rc) return rc;
         } else {
-            pa_k_linear<ROUND><<<dim3(cdiv(nqkv, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(a->h, dim, w.wqkv, w.bqkv, a->qkv, nqkv, bs, nqkv, dim);
+            pa_launch_linear<ROUND>(a->n_sm, nqkv, bs, 1, st, a->h, dim, w.wqkv, w.bqkv, a->qkv, nqkv, bs, nqkv, dim);
         }
         PA_LAUNCH();
         if (!single) {
@@ -1964,7 +1973,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             int rc = tc_dense(a->att, w.od, bs, w.od, w.t_o, dim, w.bo, a->ao, dim);
             if (rc) return rc;
         } else {
-            pa_k_linear<ROUND><<<dim3(cdiv(dim, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(a->att, w.od, w.wo, w.bo, a->ao, dim, bs, dim, w.od);
+            pa_launch_linear<ROUND>(a->n_sm, dim, bs, 1, st, a->att, w.od, w.wo, w.bo, a->ao, dim, bs, dim, w.od);
         }
         PA_LAUNCH();
         // ---- routed feed-forward on the same normed input
@@ -2015,7 +2024,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             int rc = tc_dense(a->h, dim, bs, dim, a->t_head, d.vocab_size, nullptr, a->logits, d.vocab_size);
             if (rc) return rc;
         } else {
-            pa_k_linear<ROUND><<<dim3(cdiv(d.vocab_size, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(a->h, dim, a->head, nullptr, a->logits, d.vocab_size, bs, d.vocab_size, dim);
+            pa_launch_linear<ROUND>(a->n_sm, d.vocab_size, bs, 1, st, a->h, dim, a->head, nullptr, a->logits, d.vocab_size, bs, d.vocab_size, dim);
         }
         PA_LAUNCH();
     }
