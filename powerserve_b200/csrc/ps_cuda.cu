@@ -382,6 +382,32 @@ int matmul_q(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int wtype, int64_t 
     }
 }
 
+// the same on the octet copies of an all-Q4_0 / all-Q8_0 model (ps_k_matmul_ob); *done = false: a row octet does not fit shared memory
+template <int TYPE, int C> int launch_mo(ps_cuda_ctx *ctx, PsMbArgs a, bool *done) {
+    static bool attr_set[64] = {};
+    int warps = PS_MB_WARPS;
+    while (warps > 1 && ps_mo_smem<TYPE>(a.K, C, warps) > 200 * 1024) warps >>= 1;
+    const size_t smem = ps_mo_smem<TYPE>(a.K, C, warps);
+    if (smem > 200 * 1024) return 0;
+    if (!attr_set[ctx->device]) {
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_ob<TYPE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_set[ctx->device] = true;
+    }
+    int cta = 0;
+    for (int t = 0; t < a.n_seg; t++) { a.seg[t].cta0 = cta; cta += (a.seg[t].n + 8 * warps - 1) / (8 * warps); }
+    ps_k_matmul_ob<TYPE, C><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), (unsigned)(warps * 32), smem, ctx->stream>>>(a);
+    PS_LAUNCH_CK();
+    *done = true;
+    return 0;
+}
+int matmul_ob(ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int n_seg, const float *residual, bool *done) {
+    PsMbArgs a{};
+    for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
+    a.n_seg = n_seg; a.bs = (int)bs; a.K = K; a.aqs = ctx->aqs; a.ad = ctx->ad; a.residual = residual; a.err = ctx->tc_err_dev;
+    if (ctx->mv_type == 2) return bs <= 2 ? launch_mo<2, 2>(ctx, a, done) : bs <= 4 ? launch_mo<2, 4>(ctx, a, done) : launch_mo<2, 8>(ctx, a, done);
+    return bs <= 2 ? launch_mo<8, 2>(ctx, a, done) : bs <= 4 ? launch_mo<8, 4>(ctx, a, done) : launch_mo<8, 8>(ctx, a, done);
+}
+
 int grid1d(int64_t n, int block = 256) { return (int)std::min<int64_t>((n + block - 1) / block, 148 * 8); }
 
 } // namespace
@@ -2091,6 +2117,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     const int64_t n_kv = sess ? (int64_t)sess->n_kv_max : tree ? (int64_t)tree_base + bs : (int64_t)pos0 + bs; // pos.back() + 1 (session batch: the longest row)
     const float kq_scale = 1.0f / sqrtf((float)hs);
     const bool tc = ctx->tc_ok && ctx->opt_tc && ctx->opt_fused && bs >= ctx->opt_tc_min; // tensor-core GEMM on the packed blocks
+    const bool mo = bs > 1 && mv_usable(ctx); // octet copies of a 32-block model
     const bool rw = ctx->fused_ok && ctx->opt_fused && (bs > 1 || tree); // octet-interleaved copies exist: multi-column row-walker
     int rc;
     ps_k_get_embedding<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
@@ -2120,7 +2147,15 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = quantize_act(ctx, ld.tq, ctx->xn, dim, bs))) return rc;
             const PsMbSeg sg[3] = {{ld.wq, ctx->q, d.qkv_bias ? ld.q_bias : nullptr, (int)qdim, 0}, {ld.wk, ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)kvd, 0},
                                    {ld.wv, ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)kvd, 0}};
-            if (bs > 1 && ld.tq == ld.tk && ld.tq == ld.tv) {
+            bool done = false;
+            if (mo) {
+                const size_t ob = mv_bytes(ctx->mv_type, 8, dim); // an octet's bytes
+                const PsMbSeg so[3] = {{ld.mv_qkv, ctx->q, sg[0].bias, (int)qdim, 0}, {ld.mv_qkv + ob * (size_t)(qdim / 8), ctx->k, sg[1].bias, (int)kvd, 0},
+                                       {ld.mv_qkv + ob * (size_t)((qdim + kvd) / 8), ctx->v, sg[2].bias, (int)kvd, 0}};
+                if ((rc = matmul_ob(ctx, dim, bs, so, 3, nullptr, &done))) return rc;
+            }
+            if (done) {
+            } else if (bs > 1 && ld.tq == ld.tk && ld.tq == ld.tv) {
                 if ((rc = matmul_qb(ctx, ld.tq, dim, bs, sg, 3, nullptr))) return rc;
             } else {
                 const int ty[3] = {ld.tq, ld.tk, ld.tv};
@@ -2168,7 +2203,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rwm_single(ctx, ld.rw_o, (int)dim, (int)qdim, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.to, ctx->att, qdim, bs))) return rc;
-            if ((rc = matmul_q(ctx, ctx->x, ld.wo, ld.to, qdim, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wo.att
+            bool done = false;
+            const PsMbSeg so = {ld.mv_o, ctx->x, nullptr, (int)dim, 0};
+            if (mo && (rc = matmul_ob(ctx, qdim, bs, &so, 1, ctx->x, &done))) return rc;
+            if (!done && (rc = matmul_q(ctx, ctx->x, ld.wo, ld.to, qdim, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wo.att
         }
         ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.ffn_norm, dim, d.norm_eps);
         PS_LAUNCH_CK();
@@ -2181,7 +2219,13 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 1, 2, ctx->u, bs, nullptr, nullptr))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tgate, ctx->xn, dim, bs))) return rc;
-            if (bs > 1 && ld.tgate == ld.tup) {
+            bool done = false;
+            if (mo) {
+                const PsMbSeg so[2] = {{ld.mv_gu, ctx->g, nullptr, (int)ffn, 0}, {ld.mv_gu + mv_bytes(ctx->mv_type, 8, dim) * (size_t)(ffn / 8), ctx->u, nullptr, (int)ffn, 0}};
+                if ((rc = matmul_ob(ctx, dim, bs, so, 2, nullptr, &done))) return rc;
+            }
+            if (done) {
+            } else if (bs > 1 && ld.tgate == ld.tup) {
                 const PsMbSeg sg[2] = {{ld.wgate, ctx->g, nullptr, (int)ffn, 0}, {ld.wup, ctx->u, nullptr, (int)ffn, 0}};
                 if ((rc = matmul_qb(ctx, ld.tgate, dim, bs, sg, 2, nullptr))) return rc;
             } else {
@@ -2199,7 +2243,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rwm_single(ctx, ld.rw_down, (int)dim, (int)ffn, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tdown, ctx->g, ffn, bs))) return rc;
-            if ((rc = matmul_q(ctx, ctx->x, ld.wdown, ld.tdown, ffn, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wdown.h
+            bool done = false;
+            const PsMbSeg so = {ld.mv_down, ctx->x, nullptr, (int)dim, 0};
+            if (mo && (rc = matmul_ob(ctx, ffn, bs, &so, 1, ctx->x, &done))) return rc;
+            if (!done && (rc = matmul_q(ctx, ctx->x, ld.wdown, ld.tdown, ffn, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wdown.h
         }
     }
     if (lm_head) {
@@ -2213,7 +2260,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rwm_single(ctx, ctx->rw_out, d.vocab_size, (int)dim, 0, 1, ctx->logits, bs, nullptr, nullptr))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ctx->t_out, ctx->xn, dim, bs))) return rc;
-            if ((rc = matmul_q(ctx, ctx->logits, ctx->w_out, ctx->t_out, dim, d.vocab_size, bs, nullptr, nullptr))) return rc;
+            bool done = false;
+            const PsMbSeg so = {ctx->mv_out, ctx->logits, nullptr, d.vocab_size, 0};
+            if (mo && (rc = matmul_ob(ctx, dim, bs, &so, 1, nullptr, &done))) return rc;
+            if (!done && (rc = matmul_q(ctx, ctx->logits, ctx->w_out, ctx->t_out, dim, d.vocab_size, bs, nullptr, nullptr))) return rc;
         }
     }
     return 0;

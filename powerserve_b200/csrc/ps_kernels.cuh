@@ -451,11 +451,58 @@ struct PsMbArgs {
     int64_t K;
     const uint32_t *aqs; const float *ad; const uint32_t *absp;
     const float *residual;
+    int *err;           // (ps_k_matmul_ob) set if a copy did not arrive
 };
 template <int TYPE> PS_HD size_t ps_mb_smem(int64_t K, int C) {
     if (PsBlk<TYPE>::ELEMS == 256) return (size_t)C * (size_t)(K + K / 256 * 20);
     const int64_t nbg = (K / 32 + 3) / 4; // groups of four blocks, the last one padded with zeros
     return (size_t)C * (size_t)nbg * (128 + 16);
+}
+// Staging of the activations in shared memory: eight 16-byte loads of a thread are in flight together.  (One load at a time, column by
+// column, it took longer than the products: 28 of 44 us at K = 4864.)
+template <typename T> PS_D void ps_mb_copy(T *dst, const T *__restrict__ src, int n, int n_live, T zero) { // dst[0 .. n), zeros from n_live on
+    for (int t0 = threadIdx.x; t0 < n; t0 += 8 * blockDim.x) {
+        T v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int t = t0 + u * blockDim.x;
+            v[u] = t < n_live ? src[t] : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int t = t0 + u * blockDim.x;
+            if (t < n) dst[t] = v[u];
+        }
+    }
+}
+// columns of 32-element blocks into [C][group of four blocks][8 lanes][4 blocks]; src: the first column, [column][nb][8 words]
+template <int C> PS_D void ps_mb_stage32(uint32_t *s_qs, float *s_d, const uint32_t *__restrict__ src, const float *__restrict__ d, int nb, int nbg, int ncol) {
+    const int per = nbg * 8, n = C * per; // 16-byte pieces: half a block each
+    for (int t0 = threadIdx.x; t0 < n; t0 += 8 * blockDim.x) {
+        uint4 v[8];
+        int at[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int t = t0 + u * blockDim.x, c = t / per, r = t - c * per, i = r >> 1;
+            v[u] = c < ncol && i < nb ? *reinterpret_cast<const uint4 *>(src + ((size_t)c * nb + i) * 8 + (r & 1) * 4) : make_uint4(0, 0, 0, 0);
+            at[u] = t < n ? c * nbg * 32 + ((i >> 2) * 8 + (r & 1) * 4) * 4 + (i & 3) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (at[u] >= 0) { s_qs[at[u]] = v[u].x; s_qs[at[u] + 4] = v[u].y; s_qs[at[u] + 8] = v[u].z; s_qs[at[u] + 12] = v[u].w; }
+    }
+    const int m = C * nbg * 4;
+    for (int t0 = threadIdx.x; t0 < m; t0 += 8 * blockDim.x) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int t = t0 + u * blockDim.x, c = t / (nbg * 4), i = t - c * nbg * 4;
+            v[u] = c < ncol && i < nb ? d[(size_t)c * nb + i] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (t0 + u * (int)blockDim.x < m) s_d[t0 + u * blockDim.x] = v[u];
+    }
 }
 template <int TYPE, int R, int C>
 __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArgs a) {
@@ -478,13 +525,9 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
         uint4 *s_qs = reinterpret_cast<uint4 *>(smem);                              // [C][nb][2][8] as quantised
         float *s_d = reinterpret_cast<float *>(s_qs + (size_t)C * nb * 16);         // [C][nb]
         uint32_t *s_bsp = reinterpret_cast<uint32_t *>(s_d + (size_t)C * nb);       // [C][nb * 4]
-        for (int c = 0; c < C; c++) {
-            const bool in = c < ncol;
-            const uint4 *src = reinterpret_cast<const uint4 *>(a.aqs + (int64_t)(col0 + c) * nb * 64);
-            for (int t = threadIdx.x; t < nb * 16; t += blockDim.x) s_qs[c * nb * 16 + t] = in ? src[t] : make_uint4(0, 0, 0, 0);
-            for (int t = threadIdx.x; t < nb; t += blockDim.x) s_d[c * nb + t] = in ? a.ad[(int64_t)(col0 + c) * nb + t] : 0.f;
-            for (int t = threadIdx.x; t < nb * 4; t += blockDim.x) s_bsp[c * nb * 4 + t] = in ? a.absp[(int64_t)(col0 + c) * nb * 4 + t] : 0u;
-        }
+        ps_mb_copy(s_qs, reinterpret_cast<const uint4 *>(a.aqs) + (int64_t)col0 * nb * 16, C * nb * 16, ncol * nb * 16, make_uint4(0, 0, 0, 0));
+        ps_mb_copy(s_d, a.ad + (int64_t)col0 * nb, C * nb, ncol * nb, 0.f);
+        ps_mb_copy(s_bsp, a.absp + (int64_t)col0 * nb * 4, C * nb * 4, ncol * nb * 4, 0u);
         __syncthreads();
         const uint8_t *wr[R];
 #pragma unroll
@@ -522,14 +565,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
         const int nbg = (nb + 3) / 4;
         uint32_t *s_qs = reinterpret_cast<uint32_t *>(smem);                        // [C][group][8 lanes][4 blocks]
         float *s_d = reinterpret_cast<float *>(s_qs + (size_t)C * nbg * 32);        // [C][group][4 blocks]
-        for (int c = 0; c < C; c++) {
-            const uint32_t *src = a.aqs + (int64_t)(col0 + c) * nb * 8;
-            for (int t = threadIdx.x; t < nbg * 32; t += blockDim.x) {
-                const int i = t >> 3, w = t & 7; // natural order: word w of block i
-                s_qs[c * nbg * 32 + ((i >> 2) * 8 + w) * 4 + (i & 3)] = c < ncol && i < nb ? src[t] : 0u;
-            }
-            for (int t = threadIdx.x; t < nbg * 4; t += blockDim.x) s_d[c * nbg * 4 + t] = c < ncol && t < nb ? a.ad[(int64_t)(col0 + c) * nb + t] : 0.f;
-        }
+        ps_mb_stage32<C>(s_qs, s_d, a.aqs + (int64_t)col0 * nb * 8, a.ad + (int64_t)col0 * nb, nb, nbg, ncol);
         __syncthreads();
         const uint8_t *wr[R];
 #pragma unroll

@@ -362,3 +362,94 @@ __global__ void __launch_bounds__(64) ps_k_rope_kv(float *__restrict__ qr, const
         }
     }
 }
+
+// ---------------------------------------------------------------------------------------------------- token batches
+// ps_k_matmul_qb's product (a thread = one AVX lane of two rows, C columns in registers) on the octet copies: a warp's eight rows are
+// ONE contiguous stream, which it requests whole at the start - bulk copies in PS_MO_CHUNKS pieces with a barrier each - while the CTA stages
+// the activations; rows of a 0.5B model are 4 to 22 KB.  On the GGUF bytes the kernel waited a memory round trip for every four
+// blocks of a row, with one warp per scheduler to hide it: 896 x 4864 on 32 columns 84 us.
+#define PS_MO_CHUNKS 8
+template <int TYPE> PS_HD size_t ps_mo_smem(int64_t K, int C, int warps) { return ps_mb_smem<TYPE>(K, C) + (size_t)warps * (size_t)(K / 32) * PsMv32<TYPE>::BLK; }
+template <int TYPE, int C>
+__global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArgs a) {
+    using G = PsMv32<TYPE>;
+    constexpr int R = 2;
+    extern __shared__ __align__(16) uint8_t smem[];
+    __shared__ __align__(8) uint64_t bar[PS_MB_WARPS][PS_MO_CHUNKS];
+    const int nb = (int)(a.K / 32), nbg = (nb + 3) / 4, col0 = blockIdx.y * C, ncol = min(C, a.bs - col0), warps = blockDim.x >> 5;
+    int sg = 0;
+    if (a.n_seg > 1 && (int)blockIdx.x >= a.seg[1].cta0) sg = 1;
+    if (a.n_seg > 2 && (int)blockIdx.x >= a.seg[2].cta0) sg = 2;
+    const PsMbSeg &seg = a.seg[sg];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 7, r0 = lane >> 3;
+    const int oct = ((int)blockIdx.x - seg.cta0) * warps + warp, n_oct = (seg.n + 7) / 8;
+    const int cg = (nbg + PS_MO_CHUNKS - 1) / PS_MO_CHUNKS; // groups of four blocks per piece
+    uint32_t *s_qs = reinterpret_cast<uint32_t *>(smem);                        // [C][group][8 lanes][4 blocks]
+    float *s_d = reinterpret_cast<float *>(s_qs + (size_t)C * nbg * 32);        // [C][group][4 blocks]
+    uint8_t *sw = smem + ps_mb_smem<TYPE>(a.K, C) + (size_t)warp * nb * G::BLK; // the warp's octet
+    if (lane == 0) {
+        for (int p = 0; p < PS_MO_CHUNKS; p++) ps_mbar_init(&bar[warp][p], 1);
+        ps_fence_barrier_init();
+        if (oct < n_oct)
+            for (int p = 0, b0 = 0; b0 < nb; p++, b0 += 4 * cg) {
+                const uint32_t bytes = (uint32_t)(min(4 * cg, nb - b0) * G::BLK);
+                ps_mbar_expect_tx(&bar[warp][p], bytes);
+                ps_bulk_g2s(sw + (size_t)b0 * G::BLK, seg.w + ((size_t)oct * nb + b0) * G::BLK, bytes, &bar[warp][p]);
+            }
+    }
+    ps_mb_stage32<C>(s_qs, s_d, a.aqs + (int64_t)col0 * nb * 8, a.ad + (int64_t)col0 * nb, nb, nbg, ncol);
+    __syncthreads();
+    if (oct >= n_oct) return;
+    float acc[R][C];
+#pragma unroll
+    for (int t = 0; t < R; t++)
+#pragma unroll
+        for (int c = 0; c < C; c++) acc[t][c] = 0.f;
+    for (int g = 0; g < nbg; g++) {
+        if (g % cg == 0 && !ps_tc_wait(&bar[warp][g / cg], 0)) { *a.err = 9; break; }
+        int q[R][4];
+        float xd[R][4];
+#pragma unroll
+        for (int b = 0; b < 4; b++) {
+            const uint8_t *blk = sw + (size_t)min(4 * g + b, nb - 1) * G::BLK; // past the end: the last block again, its activations are zero
+#pragma unroll
+            for (int t = 0; t < R; t++) {
+                const int row = r0 + 4 * t;
+                const uint32_t w = *reinterpret_cast<const uint32_t *>(blk + row * G::QB + (TYPE == 2 ? (l & 3) : l) * 4);
+                q[t][b] = TYPE == 2 ? (int)__vsub4((l < 4) ? (w & 0x0f0f0f0fu) : ((w >> 4) & 0x0f0f0f0fu), 0x08080808u) : (int)w;
+                xd[t][b] = ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 8 * G::QB + 2 * row));
+            }
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const uint4 y = *reinterpret_cast<const uint4 *>(s_qs + ((size_t)(c * nbg + g) * 8 + l) * 4);
+            const float4 yd = *reinterpret_cast<const float4 *>(s_d + (size_t)(c * nbg + g) * 4);
+            const int yw[4] = {(int)y.x, (int)y.y, (int)y.z, (int)y.w};
+            const float ydv[4] = {yd.x, yd.y, yd.z, yd.w};
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+#pragma unroll
+                for (int t = 0; t < R; t++) {
+                    const float S = __fsub_rn(__int_as_float(__dp4a(q[t][b], yw[b], 0x4B400000)), 12582912.f); // |sum| < 2^17: exact
+                    acc[t][c] = __fmaf_rn(__fmul_rn(xd[t][b], ydv[b]), S, acc[t][c]);
+                }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < R; t++) {
+        const int n = oct * 8 + r0 + 4 * t;
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            float r = acc[t][c]; // hsum_float_8 over the row's eight lanes
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 4));
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 2));
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 1));
+            if (l == c % 8 && c < ncol && n < seg.n) {
+                const int64_t o = (int64_t)(col0 + c) * seg.n + n;
+                if (seg.bias) r = __fadd_rn(r, seg.bias[n]);
+                if (a.residual) r = __fadd_rn(a.residual[o], r);
+                seg.dst[o] = r;
+            }
+        }
+    }
+}

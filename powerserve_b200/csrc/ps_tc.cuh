@@ -522,30 +522,43 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                     __stcg(part + (2 * c) * ET, r0);
                     __stcg(part + (2 * c + 1) * ET, r1);
                 }
-                __threadfence();
+                // one thread fences for all (fences are cumulative over the barrier): 512 of them, each waiting for its own stores, cost more
+                // than the stores
                 ps_bar_sync(1, ET);
                 if (tid == 0) {
+                    __threadfence();
                     const int last = atomicAdd(a.cnt + tile, 1) == nu - 1;
                     if (last) a.cnt[tile] = 0;
                     sh_last = last;
+                    __threadfence();
                 }
                 ps_bar_sync(1, ET);
                 if (!sh_last) continue;
-                __threadfence();
                 const float *q = a.part + (size_t)tile * nu * (T::EC * ET) + tid;
                 constexpr int US = T::EC * ET;
 #pragma unroll
-                for (int c = 0; c < T::EC / 2; c++) {
-                    float r[2];
+                for (int cb = 0; cb < T::EC; cb += 8) { // the loads of eight columns together
+                    float r[8];
+                    if (nu == 3) {
+                        float x[3][8];
 #pragma unroll
-                    for (int k = 0; k < 2; k++) {
-                        const float *qc = q + (2 * c + k) * ET;
-                        if (nu == 3) r[k] = __fadd_rn(__fadd_rn(__ldcg(qc), __ldcg(qc + US)), __ldcg(qc + 2 * US));
-                        else
-                            r[k] = __fadd_rn(__fadd_rn(__fadd_rn(__ldcg(qc), __ldcg(qc + US)), __fadd_rn(__ldcg(qc + 2 * US), __ldcg(qc + 3 * US))),
-                                             __fadd_rn(__ldcg(qc + 4 * US), __ldcg(qc + 5 * US)));
+                        for (int w = 0; w < 3; w++)
+#pragma unroll
+                            for (int k = 0; k < 8; k++) x[w][k] = __ldcg(q + w * US + (cb + k) * ET);
+#pragma unroll
+                        for (int k = 0; k < 8; k++) r[k] = __fadd_rn(__fadd_rn(x[0][k], x[1][k]), x[2][k]);
+                    } else {
+                        float x[6][8];
+#pragma unroll
+                        for (int w = 0; w < 6; w++)
+#pragma unroll
+                            for (int k = 0; k < 8; k++) x[w][k] = __ldcg(q + w * US + (cb + k) * ET);
+#pragma unroll
+                        for (int k = 0; k < 8; k++)
+                            r[k] = __fadd_rn(__fadd_rn(__fadd_rn(x[0][k], x[1][k]), __fadd_rn(x[2][k], x[3][k])), __fadd_rn(x[4][k], x[5][k]));
                     }
-                    acc[0][c] = ps_f2_pack(r[0], r[1]);
+#pragma unroll
+                    for (int k = 0; k < 4; k++) acc[0][cb / 2 + k] = ps_f2_pack(r[2 * k], r[2 * k + 1]);
                 }
             }
             // ---- bias / residual, dst[col][row]
