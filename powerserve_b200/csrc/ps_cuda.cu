@@ -799,13 +799,14 @@ template <int NT> int tc_launch(ps_cuda_ctx *ctx, PsTcArgs &a) {
         attr[ctx->device] = true;
     }
     // passes per unit: fewer passes cover the GPU with a small matrix and even out the last wave, more save the hand-over of a tile's numbers
-    // (a unit that hands over costs about four steps more: its 128 x NT floats go through L2 and the tile's last unit reads all of them)
+    // (a unit that hands over costs about as much as seven super-blocks: its 128 x NT floats go through L2 and the tile's last unit reads all of
+    // them; 224 row tiles x 16 super-blocks at 16 columns: 88 us with one pass a unit, 78 with two, 74 with six)
     int64_t best = INT64_MAX;
     const int slots = ctx->n_sm * PsTc<NT>::CTAS;
     for (int pp : {6, 2, 1}) {
         const int64_t units = (int64_t)a.n_tiles * (PS_TC_PASSES / pp), rounds = (units + slots - 1) / slots;
         if (pp < 6 && (a.n_tiles > TC_CNT || (size_t)units * PS_TC_M * NT * 4 > ctx->tc_part_bytes)) continue;
-        const int64_t cost = rounds * ((int64_t)pp * a.nbp + (pp < 6 ? 4 : 0));
+        const int64_t cost = rounds * ((int64_t)pp * a.nbp + (pp < 6 ? 7 : 0));
         if (cost < best) { best = cost; a.pp = pp; }
     }
     const int units = a.n_tiles * (PS_TC_PASSES / a.pp);

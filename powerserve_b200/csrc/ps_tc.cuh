@@ -48,11 +48,13 @@ PS_HD int ps_tc_pass(int l) { return ((l & 1) << 1) | ((l >> 1) & 1); }
 
 // configuration by column-tile width
 template <int NT> struct PsTc {
-    static constexpr int NH = NT >= 64 ? 2 : 1;                 // column halves, each with epilogue warps of its own
+    // column halves, each with epilogue warps of its own.  An entry costs the issuing warp about as much whatever its width, so one wide entry
+    // is better where tensor memory holds enough of them (64 columns, 448 row tiles' worth of units: 134 us with two halves, 108 with one)
+    static constexpr int NH = NT >= 97 ? 2 : 1;
     static constexpr int CW = NT / NH;                          // columns of a tensor-memory entry (N of one MMA)
     static constexpr int EW = NT >= 64 ? 16 : 8;                // epilogue warps
     static constexpr int EC = NT * 4 / EW;                      // columns a thread owns (its warp's lane quadrant gives the row)
-    static constexpr int NE = 3, NA = 3;                        // tensor-memory rings: accumulator entries, A buffers
+    static constexpr int NE = NT == 96 && NH == 1 ? 2 : 3, NA = 3; // tensor-memory rings: accumulator entries, A buffers
     static constexpr int NS = 3;                                // stages of two super-blocks (NE and NA divide 2 NS: the MMA loop is unrolled by it)
     static constexpr int ND = 2;                                // de-quantising warpgroups: one per super-block of a step
     static constexpr int THREADS = (EW + 4 * ND + 4) * 32;
@@ -322,6 +324,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
             // issue took 280 cycles whatever its size, where tcgen05.mma itself takes 32 here.
             // kind::f16, D = F32 (bit 4), A = B = F16, K-major both, N >> 3 @ bit 17, M >> 4 @ bit 24
             constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(T::CW >> 3) << 17) | ((uint32_t)(PS_TC_M >> 4) << 24);
+            constexpr bool ODD = (2 * T::NS * T::NH / T::NE) & 1; // the entries' ring turns an odd number of times in the unrolled loop
             const uint64_t desc0 = ps_tc_smem_desc(ps_smem_u32(ps_tc_smem + T::STAGE_B), NT * 16, 128);
             const int n_steps = n_units > (int)blockIdx.x ? ((n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * pp * ns : 0;
             int u = blockIdx.x, p = (u % nu) * pp, p_end = p + pp, left = ns;
@@ -343,7 +346,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                             // lane 0: the accumulator entry (free from the start in the first round), lane 1: A, the others: the stage
                             const bool fd = lane == 0 && (g0 > 0 || e >= T::NE), fa = lane == 1;
                             const uint32_t bar = ps_smem_u32(fd ? &bar_d_empty[re] : fa ? &bar_a_full[ra] : &bar_full[j]);
-                            if (!ps_tc_wait_all(bar, fd ? ((e / T::NE) & 1) ^ 1 : fa ? (k / T::NA) & 1 : round)) { *a.err = 2; ok = false; break; }
+                            if (!ps_tc_wait_all(bar, fd ? ((e / T::NE) & 1) ^ 1 ^ (ODD ? round : 0) : fa ? (k / T::NA) & 1 : round)) { *a.err = 2; ok = false; break; }
                             ps_tc_fence_after();
                             const uint32_t td = tmem_base + re * (2 * T::CW);
                             const uint64_t dh = ds + h * (T::CW / 8) * 8;
