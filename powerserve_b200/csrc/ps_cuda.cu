@@ -67,7 +67,6 @@ struct LayerDev {
     int tq, tk, tv, to, tgate, tup, tdown;
     // octet-interleaved copies for the row-walker mat-vec (ps_rw.cuh): q|k|v rows, o, gate|up slots, down
     uint8_t *rw_qkv = nullptr, *rw_o = nullptr, *rw_gu = nullptr, *rw_down = nullptr;
-    // fp16-expanded tensor-core operands for the prefill GEMM (ps_tc.cuh): q|k|v rows, o, gate, up, down
     uint8_t *tc_qkv = nullptr, *tc_o = nullptr, *tc_gu = nullptr, *tc_down = nullptr; // packed blocks of the tcgen05 GEMM (gate rows, then up rows from the next tile border)
     // octet copies for the 32-block mat-vec (ps_mv32.cuh; all-Q4_0 / all-Q8_0 models): q|k|v rows, o, gate|up rows, down
     uint8_t *mv_qkv = nullptr, *mv_o = nullptr, *mv_gu = nullptr, *mv_down = nullptr;
@@ -251,6 +250,7 @@ int dev_alloc(ps_cuda_ctx *ctx, void **p, size_t bytes) {
 
 // Failures detected on the device (tcgen05 pipeline time-out, a peer wait or a grid barrier that gave up) become a C-ABI
 // status: the flags ride along with the call's final device-to-host copy.  Call with work enqueued; synchronises.
+constexpr int TC_CNT = 16384; // batch GEMM: tiles whose pass groups run as separate units (a counter each)
 int sync_and_check(ps_cuda_ctx *ctx) {
     PS_CK(cudaMemcpyAsync(ctx->h_err, ctx->err_dev, 16, cudaMemcpyDeviceToHost, ctx->stream));
     PS_CK(cudaStreamSynchronize(ctx->stream));
@@ -259,6 +259,7 @@ int sync_and_check(ps_cuda_ctx *ctx) {
         for (int k = 0; k < 3; k++) ctx->err_seen[k] |= ctx->h_err[k];
         PS_CK(cudaMemsetAsync(ctx->err_dev, 0, 16, ctx->stream));
         if (ctx->ag_ctr) PS_CK(cudaMemsetAsync(ctx->ag_ctr, 0, (size_t)ctx->d.n_layers * ctx->nkv_l * 8, ctx->stream)); // a group that gave up leaves its counter mid-instance
+        if (ctx->tc_cnt) PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, TC_CNT * 4, ctx->stream)); // a GEMM that gave up leaves its tiles' counters part-way
         return fail(ctx, PS_CUDA_ERR_CUDA, "device-side failure:%s%s%s (wait site %d; results of this call are invalid)", tc ? " tcgen05 pipeline time-out" : "",
                     tp ? " tensor-parallel peer wait gave up" : "", st ? " decode-step wait gave up" : "", st);
     }
@@ -765,7 +766,6 @@ int rwm_single(ps_cuda_ctx *ctx, const uint8_t *w, int n_rows, int K, int slot, 
 }
 
 // ---- tcgen05 GEMM of token batches (ps_tc.cuh)
-constexpr int TC_CNT = 16384;                        // tiles whose pass groups run as separate units
 constexpr size_t TC_PART_MAX = (size_t)96 << 20;
 int64_t tc_tiles(int64_t rows) { return (rows + PS_TC_M - 1) / PS_TC_M; }
 int64_t tc_nbp(int64_t K) { return (K / 256 + 1) & ~(int64_t)1; } // super-blocks, rounded up to whole steps
@@ -1885,7 +1885,6 @@ float *ps_cuda_kv_k(ps_cuda_ctx *ctx, int layer) { return (layer >= 0 && layer <
 float *ps_cuda_kv_v(ps_cuda_ctx *ctx, int layer) { return (layer >= 0 && layer < ctx->d.n_layers) ? ctx->vct[layer] : nullptr; }
 
 // ---------------------------------------------------------------------------------------------- whole model
-// ---- tcgen05 prefill GEMM (ps_tc.cuh)
 int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
     PS_NO_ARCH("ps_cuda_bind_model");
     const ps_cuda_model_desc &d = ctx->d;
