@@ -8,7 +8,7 @@
 // Why this shape (B200): the op is an HBM stream of 144-byte blocks with ~85 warp instructions of work per 8 row-blocks -
 // at 6.5 TB/s an SM must retire a block every ~6 cycles, so the kernel is as much issue-bound as bandwidth-bound.  The
 // earlier design (one thread per block, shared-memory hand-off to separate fp32 chain threads, CTA-wide barriers per
-// tile, 8 warps) measured 20-27 % issue utilisation and 3x instruction overhead (profiles/r01b_*).  Here:
+// tile, 8 warps) measured 20-27 % issue utilisation and 3x instruction overhead (profiles/set1b_*).  Here:
 //   * FOUR threads own one weight row: thread q of the quad owns AVX lanes 2q, 2q+1 of the reference's __m256 accumulator
 //     (and lane q of the __m128 mins accumulator) and walks the row's super-blocks IN ORDER, so the fp32 FMA chains of
 //     the reference live in three registers per thread — no hand-off, no chain phase, no barrier inside the stream.

@@ -1,6 +1,6 @@
 """Summarise an .ncu-rep (ncu --set full) into the text table kept under profiles/: one column per captured launch.
 
-    python tools/ncu_summary.py gpurun_out/decode_kernels.ncu-rep "header line" ... > profiles/rNN_ncu_....txt
+    python tools/ncu_summary.py decode_kernels.ncu-rep "header line" ... > profiles/...txt
 """
 import csv
 import subprocess
