@@ -453,7 +453,9 @@ int ps_cuda_arch_tap(ps_cuda_ctx *ctx, int layer, float *host, int bs);
  * Kernel choice for batches (prefill chunks, verify batches; every choice computes the same bits): "attn_tile" = 0 runs
  * the first-generation batch attention kernels instead of the register-tiled ones; "tc_min" = n is the narrowest batch that takes
  * the tcgen05 GEMM (default 6; narrower ones walk with the multi-column row-walker); "scores_batch_min" (default 2) and
- * "pv_batch_min" (default 3) are the narrowest batches for the query-blocked scores / P.V kernels. */
+ * "pv_batch_min" (default 3) are the narrowest batches for the query-blocked scores / P.V kernels.
+ * "give_up_warp" = w (default -1: none): in the batch products that copy ahead, warp w of every CTA takes its first wait as run out, so that
+ * tests reach the error status (PS_CUDA_ERR_CUDA, counter "tc_error"); later calls without it are unaffected. */
 int ps_cuda_set_option(ps_cuda_ctx *ctx, const char *name, int value);
 /* counters: "kernel_launches" (kernels enqueued since create), "graph_replays", "h2d_bytes", "d2h_bytes",
  * "last_device_ns" (CUDA-event time, on the context stream, of the last forward / decode_greedy call),

@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
             for (int sg = 1; sg < a.seg.n; sg++)
                 if (rt >= a.seg.rt[sg]) pb += a.seg.set_bytes;
             for (int kb = 0; kb < nkb; kb++, g++, st.step()) {
-                if (g >= STAGES && !ps_tc_wait(&bar_empty[st.i], st.round ^ 1)) { *a.err = 1; ok = false; break; }
+                if (g >= STAGES && !ps_tc_wait_warp(&bar_empty[st.i], st.round ^ 1)) { *a.err = 1; ok = false; break; }
                 uint8_t *sm = smem + (size_t)st.i * STAGE_BYTES;
                 uint64_t *bar = &bar_full[st.i];
                 if (ps_elect_one()) {
@@ -197,10 +197,10 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
         bool ok = true;
         for (int mu = 0; mu < my_units && ok; mu++) {
             const int tb = mu & 1;
-            if (mu >= 2 && !ps_tc_wait(&bar_tmem_empty[tb], ((mu >> 1) - 1) & 1)) { *a.err = 3; break; }
+            if (mu >= 2 && !ps_tc_wait_warp(&bar_tmem_empty[tb], ((mu >> 1) - 1) & 1)) { *a.err = 3; break; }
             const uint32_t td = tmem_base + tb * (NA * PT_N);
             for (int kb = 0; kb < nkb; kb++, st.step()) {
-                if (!ps_tc_wait(&bar_full[st.i], st.round)) { *a.err = 2; ok = false; break; }
+                if (!ps_tc_wait_warp(&bar_full[st.i], st.round)) { *a.err = 2; ok = false; break; }
                 ps_tc_fence_after();
                 const uint64_t da = desc0 + (uint64_t)(st.i * (STAGE_BYTES >> 4));
                 if (ps_elect_one()) {
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
         // ===== epilogue: warp w reads tensor-memory lanes 32 w .. 32 w + 31 = 32 consecutive output features
         for (int mu = 0; mu < my_units; mu++) {
             const int u = (int)blockIdx.x + mu * (int)gridDim.x, ct = u / a.n_rt, rt = u % a.n_rt, tb = mu & 1;
-            if (!ps_tc_wait(&bar_tmem_full[tb], (mu >> 1) & 1)) { *a.err = 4; break; }
+            if (!ps_tc_wait_warp(&bar_tmem_full[tb], (mu >> 1) & 1)) { *a.err = 4; break; }
             ps_tc_fence_after();
             int n = rt * PT_M + 32 * warp + lane, n_end = a.N;
             for (int sg = 0; sg < a.seg.n; sg++) // the segment's own rows

@@ -122,7 +122,7 @@ struct ps_cuda_ctx {
     float *h_logits = nullptr;                                          // pinned staging for logits
     size_t h_logits_cap = 0;
     // options / counters
-    int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_scores_batch_min = 2;
+    int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_scores_batch_min = 2, opt_give_up = -1;
     bool tc_ok = false;        // tensor-core prefill operands are resident
     uint8_t *tc_b = nullptr;   // B operand blocks of the current activation batch
     float *tc_part = nullptr;  // pass groups' numbers of the tiles in flight
@@ -251,6 +251,7 @@ int dev_alloc(ps_cuda_ctx *ctx, void **p, size_t bytes) {
 // Failures detected on the device (tcgen05 pipeline time-out, a peer wait or a grid barrier that gave up) become a C-ABI
 // status: the flags ride along with the call's final device-to-host copy.  Call with work enqueued; synchronises.
 constexpr int TC_CNT = 16384; // batch GEMM: tiles whose pass groups run as separate units (a counter each)
+uint32_t give_up_cycles(const ps_cuda_ctx *ctx) { return ctx->opt_give_up >= 0 ? 1u << 24 : PS_TC_WAIT_CYCLES; } // option "give_up_warp": the other waits run out within 10 ms
 int sync_and_check(ps_cuda_ctx *ctx) {
     PS_CK(cudaMemcpyAsync(ctx->h_err, ctx->err_dev, 16, cudaMemcpyDeviceToHost, ctx->stream));
     PS_CK(cudaStreamSynchronize(ctx->stream));
@@ -820,7 +821,7 @@ int tc_gemm(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int64_t n_tiles, int64_t 
     const int nt = tc_width(bs);
     a.err = ctx->tc_err_dev;
     a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = (bs + nt - 1) / nt; a.n_tiles = (int)n_tiles * a.n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
-    a.part = ctx->tc_part; a.cnt = ctx->tc_cnt;
+    a.part = ctx->tc_part; a.cnt = ctx->tc_cnt; a.give_up = ctx->opt_give_up; a.limit = give_up_cycles(ctx);
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
     ctx->n_tc++;
     switch (nt) {
@@ -2929,6 +2930,7 @@ int ps_cuda_set_option(ps_cuda_ctx *ctx, const char *name, int value) {
     else if (!strcmp(name, "mv_kpar")) ctx->opt_mv_kpar = value;         // 1 (default): 32-block mat-vec launches with one octet per CTA and long rows share the row's blocks among the CTA's warps
     else if (!strcmp(name, "rwm_tile")) ctx->opt_rwm_tile = value;       // 1 (default): the multi-column row-walker shrinks its row tile so that narrow batches use every SM; 0: 16-octet tiles
     else if (!strcmp(name, "scores_batch_min")) ctx->opt_scores_batch_min = std::max(1, value); // batches at least this wide use the query-blocked scores kernel
+    else if (!strcmp(name, "give_up_warp")) ctx->opt_give_up = value; // tests of the way out of a pipeline whose wait has run out
     else if (!strcmp(name, "tc_min")) ctx->opt_tc_min = std::max(2, value); // narrowest batch that takes the tcgen05 GEMM (narrower ones: multi-column row-walker)
     else if (!strcmp(name, "attn_tile")) ctx->opt_attn_tile = value; // register-tiled scores / P.V kernels for batches (0: the first-generation kernels, for A/B)
     else if (!strcmp(name, "pv_batch_min")) ctx->opt_pv_batch_min = value; // batches at least this wide use the query-blocked P.V kernel (prefill), narrower ones the per-(head, dim) warp kernel

@@ -81,18 +81,39 @@ PS_D void ps_tc_ld8(uint32_t taddr, float v[8]) { // 32 lanes x 8 consecutive co
 }
 PS_D void ps_tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// bounded mbarrier wait: a mis-sequenced pipeline must never hang the GPU (returns false after ~2^22 polls)
-PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity) {
-    for (int spin = 0; spin < (1 << 22); spin++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(ps_smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (ok) return true;
-    }
+// bounded mbarrier wait: a mis-sequenced pipeline must never hang the GPU.  Gives up (returns false) after 2^31 SM cycles, about a second: a
+// poll itself may suspend the thread for microseconds, so a number of polls says little about the time
+#define PS_TC_WAIT_CYCLES 0x80000000u
+PS_D uint32_t ps_clock32() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+    return t;
+}
+PS_D bool ps_tc_poll(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity, uint32_t cycles = PS_TC_WAIT_CYCLES) {
+    if (ps_tc_poll(ps_smem_u32(bar), parity)) return true;
+    const uint32_t t0 = ps_clock32();
+    do {
+        if (ps_tc_poll(ps_smem_u32(bar), parity)) return true;
+    } while (ps_clock32() - t0 < cycles);
     return false;
+}
+// the same by a converged warp that goes on together: giving up is the warp's decision, not a lane's (elect.sync and the .aligned tcgen05
+// instructions that follow need all lanes)
+PS_D bool ps_tc_wait_warp(uint64_t *bar, uint32_t parity, uint32_t cycles = PS_TC_WAIT_CYCLES) { return __all_sync(0xffffffffu, ps_tc_wait(bar, parity, cycles)); }
+// named barrier that says whether `ok` holds in every one of its n threads
+PS_D bool ps_bar_all(int id, int n, bool ok) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %3, 0;\n\tbar.red.and.pred q, %1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r) : "r"(id), "r"(n), "r"((uint32_t)ok) : "memory");
+    return r != 0;
 }
 
 // position in a ring of N: index and the parity of the round

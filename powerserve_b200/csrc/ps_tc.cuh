@@ -172,6 +172,8 @@ struct PsTcArgs {
     float *part;        // [tile][units of a tile][EC][epilogue threads]
     int *cnt;           // per tile: units that have finished (left at zero)
     int *err;           // set if a pipeline wait gave up (results invalid)
+    int give_up;        // warp whose first wait counts as run out (-1: none): how a test reaches the way out
+    uint32_t limit;     // cycles a wait lasts at most
 };
 
 typedef unsigned long long ps_f2; // two packed floats
@@ -222,16 +224,12 @@ template <int N> PS_D void ps_reg_dec() { asm volatile("setmaxnreg.dec.sync.alig
 
 // every lane waits for a barrier of its own; bounded like ps_tc_wait.  One such poll costs what a wait for one barrier does (about 80 cycles
 // even when the phase is complete)
-PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity) {
-    for (int spin = 0; spin < (1 << 22); spin++) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(ok)
-            : "r"(bar), "r"(parity)
-            : "memory");
-        if (__all_sync(PS_FULL, ok)) return true;
-    }
+PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity, uint32_t cycles) {
+    if (__all_sync(PS_FULL, ps_tc_poll(bar, parity))) return true;
+    const uint32_t t0 = __shfl_sync(PS_FULL, ps_clock32(), 0);
+    do {
+        if (__all_sync(PS_FULL, ps_tc_poll(bar, parity))) return true;
+    } while (__shfl_sync(PS_FULL, ps_clock32(), 0) - t0 < cycles);
     return false;
 }
 
@@ -283,7 +281,8 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
             PsRing<T::NS> st;
             PsRing<T::NY> sy;
             int g = 0;
-            bool ok = true;
+            bool ok = warp != a.give_up;
+            if (!ok) *a.err = 1;
             for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
                 const int tile = u / nu, p0 = (u % nu) * pp;
                 const uint8_t *pa = a.a + (size_t)(tile / a.n_ct) * a.nbp * PS_TC_A_BLOCK, *pb = a.b + (size_t)(tile % a.n_ct) * a.nbp * PS_TC_B_BLOCK(NT);
@@ -297,7 +296,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                     const uint32_t total = na + (lanes ? 2 * PS_TC_A_SC : 0) + 2 * PS_TC_A_D + nbb + 2 * NT * 4;
                     for (int i = 0; i < ns; i++, g++, st.step(), sy.step()) {
                         const bool fy = (lane & 1) && g >= T::NY; // odd lanes wait for the factors' slot
-                        if (g >= T::NS && !ps_tc_wait_all(ps_smem_u32(fy ? &bar_y_empty[sy.i] : &bar_empty[st.i]), (fy ? sy.round : st.round) ^ 1)) { *a.err = 1; ok = false; break; }
+                        if (g >= T::NS && !ps_tc_wait_all(ps_smem_u32(fy ? &bar_y_empty[sy.i] : &bar_empty[st.i]), (fy ? sy.round : st.round) ^ 1, a.limit)) { *a.err = 1; ok = false; break; }
                         uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE, *sf = ps_tc_fact + sy.i * T::FACT;
                         uint64_t *bar = &bar_full[st.i];
                         if (ps_elect_one()) {
@@ -330,7 +329,8 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
             const uint64_t desc0 = ps_tc_smem_desc(ps_smem_u32(ps_tc_smem + T::STAGE_B), NT * 16, 128);
             const int n_steps = n_units > (int)blockIdx.x ? ((n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * pp * ns : 0;
             int u = blockIdx.x, p = (u % nu) * pp, p_end = p + pp, left = ns;
-            bool ok = true;
+            bool ok = warp != a.give_up;
+            if (!ok) *a.err = 2;
             for (int g0 = 0; g0 < n_steps && ok; g0 += T::NS) {
                 const uint32_t round = (uint32_t)(g0 / T::NS) & 1; // of the stages; the other rings' parities are constants
 #pragma unroll
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                             // lane 0: the accumulator entry (free from the start in the first round), lane 1: A, the others: the stage
                             const bool fd = lane == 0 && (g0 > 0 || e >= T::NE), fa = lane == 1;
                             const uint32_t bar = ps_smem_u32(fd ? &bar_d_empty[re] : fa ? &bar_a_full[ra] : &bar_full[j]);
-                            if (!ps_tc_wait_all(bar, fd ? ((e / T::NE) & 1) ^ 1 ^ (ODD ? round : 0) : fa ? (k / T::NA) & 1 : round)) { *a.err = 2; ok = false; break; }
+                            if (!ps_tc_wait_all(bar, fd ? ((e / T::NE) & 1) ^ 1 ^ (ODD ? round : 0) : fa ? (k / T::NA) & 1 : round, a.limit)) { *a.err = 2; ok = false; break; }
                             ps_tc_fence_after();
                             const uint32_t td = tmem_base + re * (2 * T::CW);
                             const uint64_t dh = ds + h * (T::CW / 8) * 8;
@@ -393,13 +393,14 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
         PsRing<T::NA> ra;
         if (d) ra.step();
         int g = 0;
-        bool ok = true;
+        bool ok = warp != a.give_up;
+        if (!ok) *a.err = 7;
         for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
             const int p0 = (u % nu) * pp;
             for (int p = p0; p < p0 + pp && ok; p++) {
                 for (int i = 0; i < ns; i++, g++) {
                     const bool fa = (lane & 1) && 2 * g + d >= T::NA; // odd lanes wait for the A buffer
-                    if (!ps_tc_wait_all(ps_smem_u32(fa ? &bar_a_empty[ra.i] : &bar_full[st.i]), fa ? ra.round ^ 1 : st.round)) { *a.err = 7; ok = false; break; }
+                    if (!ps_tc_wait_all(ps_smem_u32(fa ? &bar_a_empty[ra.i] : &bar_full[st.i]), fa ? ra.round ^ 1 : st.round, a.limit)) { *a.err = 7; ok = false; break; }
                     ps_tc_fence_after();
                     const uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE;
                     const uint32_t td = t_lane + ra.i * 32;
@@ -456,8 +457,9 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
         PsRing<T::NY> sy;
         PsRing<T::NE> re;
         if (h) re.step();
-        bool ok = true;
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+        bool ok = warp != a.give_up;
+        if (!ok) *a.err = 4;
+        for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
             const int tile = u / nu, p0 = (u % nu) * pp;
             float *part = a.part + ((size_t)tile * nu + u % nu) * (T::EC * ET) + tid;
             float *whole = a.part + (size_t)blockIdx.x * (T::EC * ET) + tid; // pp = 6: the sum of the pass pairs so far
@@ -469,7 +471,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                     const uint8_t *sf = ps_tc_fact + sy.i * T::FACT;
 #pragma unroll 1
                     for (int x = 0; x < 2; x++) {
-                        if (!ps_tc_wait(&bar_d_full[re.i], re.round)) { *a.err = 4; ok = false; break; } // the factors came with the stage
+                        if (!ps_tc_wait_warp(&bar_d_full[re.i], re.round, a.limit)) { *a.err = 4; ok = false; break; } // the factors came with the stage
                         ps_tc_fence_after();
                         const float xd = *reinterpret_cast<const float *>(sf + x * PS_TC_A_D + row * 4);
                         const ps_f2 x2 = ps_f2_pack(xd, xd);
@@ -518,7 +520,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                     acc[0][c] = ps_f2_pack(r0, r1);
                 }
             }
-            if (!ok) break;
+            if (nu == 1 && !ok) break;
             if (nu > 1) { // hand the numbers over; the tile's last unit adds them in the fixed order
 #pragma unroll
                 for (int c = 0; c < T::EC / 2; c++) {
@@ -528,8 +530,8 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gem
                     __stcg(part + (2 * c + 1) * ET, r1);
                 }
                 // one thread fences for all (fences are cumulative over the barrier): 512 of them, each waiting for its own stores, cost more
-                // than the stores
-                ps_bar_sync(1, ET);
+                // than the stores.  A warp that gave up comes here too, and all of them leave: no warp waits at a barrier that another has passed by
+                if (!ps_bar_all(1, ET, ok)) break;
                 if (tid == 0) {
                     __threadfence();
                     const int last = atomicAdd(a.cnt + tile, 1) == nu - 1;

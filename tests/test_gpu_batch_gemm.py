@@ -47,3 +47,23 @@ def test_two_passes_a_unit():
     L.assert_bit_equal(again, om.forward(tokens[:9]), "8B slice, 9 more tokens")
     om.close()
     cm.close()
+
+
+@pytest.mark.parametrize("bs", [16, 64, 128])
+def test_a_warp_that_gives_up_ends_the_call(odd, bs):
+    """one warp of every CTA takes its first wait as run out - an epilogue warp while the others of its tile go on to hand numbers over, a
+    de-quantising warp, the copies' warp, the issuing one: every other wait ends by its own limit, the call reports the time-out, and the
+    next call on the same context has all bits"""
+    om, cm = odd
+    tokens = synth.random_prompt(ODD.vocab_size, bs, seed=bs)
+    om.reset()
+    want = om.forward(tokens)
+    epilogue = 8 if bs < 64 else 16
+    for warp in (0, epilogue - 1, epilogue, epilogue + 8, epilogue + 9):
+        cm.reset()
+        cm.be.set_option("give_up_warp", warp)
+        with pytest.raises(capi.PsCudaError, match="tcgen05 pipeline time-out"):
+            cm.forward(tokens)
+        cm.be.set_option("give_up_warp", -1)
+        cm.reset()
+        L.assert_bit_equal(cm.forward(tokens), want, f"after warp {warp} gave up")
