@@ -223,14 +223,16 @@ template <int N> PS_D void ps_reg_inc() { asm volatile("setmaxnreg.inc.sync.alig
 template <int N> PS_D void ps_reg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // every lane waits for a barrier of its own; bounded like ps_tc_wait.  One such poll costs what a wait for one barrier does (about 80 cycles
-// even when the phase is complete)
+// even when the phase is complete).  The vote orders no memory: what a lane acquired with its barrier reaches the other lanes at the __syncwarp
 PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity, uint32_t cycles) {
-    if (__all_sync(PS_FULL, ps_tc_poll(bar, parity))) return true;
-    const uint32_t t0 = __shfl_sync(PS_FULL, ps_clock32(), 0);
-    do {
-        if (__all_sync(PS_FULL, ps_tc_poll(bar, parity))) return true;
-    } while (__shfl_sync(PS_FULL, ps_clock32(), 0) - t0 < cycles);
-    return false;
+    bool ok = __all_sync(PS_FULL, ps_tc_poll(bar, parity));
+    if (!ok) {
+        const uint32_t t0 = __shfl_sync(PS_FULL, ps_clock32(), 0);
+        do ok = __all_sync(PS_FULL, ps_tc_poll(bar, parity));
+        while (!ok && __shfl_sync(PS_FULL, ps_clock32(), 0) - t0 < cycles);
+    }
+    __syncwarp();
+    return ok;
 }
 
 // Persistent CTAs over units u = tile * (6 / pp) + group; tile = row tile * n_ct + column tile.

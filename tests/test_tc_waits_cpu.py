@@ -38,3 +38,8 @@ def test_epilogue_warps_meet_before_they_leave():
     plain = [m.start() for m in re.finditer(r"ps_bar_sync\(1, ET\);", body)]
     assert len(waits) == 1 and len(plain) == 1 and waits[0] < plain[0]
     assert not re.search(r"if \(!ok\) break;\s*if \(nu > 1\)", body)
+
+
+def test_lanes_share_what_they_acquired():
+    body = _body(_source("ps_tc.cuh"), "bool ps_tc_wait_all")
+    assert "ps_tc_poll" in body and re.search(r"__syncwarp\(\);\s*return ok;\s*\}$", body) and body.count("return") == 1
