@@ -128,7 +128,7 @@ struct ps_cuda_ctx {
     float *tc_part = nullptr;  // pass groups' numbers of the tiles in flight
     size_t tc_part_bytes = 0;
     int *tc_cnt = nullptr;     // per tile: pass groups that have finished
-    int *err_dev = nullptr;    // device-detected failures, [0] tcgen05 pipeline time-out, [1] peer wait gave up, [2] step-kernel barrier time-out
+    int *err_dev = nullptr;    // device-detected failures, [0] tcgen05 pipeline time-out (PS_ERR_COPY: a copy of a batch product), [1] peer wait gave up, [2] step-kernel barrier time-out
     int err_seen[3] = {};      // sticky host copy of the flags (counters "tc_error" / "tp_error" / "step_error")
     int *h_err = nullptr;      // pinned mirror, read after every forward / decode (a set flag becomes PS_CUDA_ERR_CUDA)
     int *tc_err_dev = nullptr; // = err_dev + 0 (counter "tc_error")
@@ -248,7 +248,7 @@ int dev_alloc(ps_cuda_ctx *ctx, void **p, size_t bytes) {
     return 0;
 }
 
-// Failures detected on the device (tcgen05 pipeline time-out, a peer wait or a grid barrier that gave up) become a C-ABI
+// Failures detected on the device (tcgen05 pipeline or copy time-out, a peer wait or a grid barrier that gave up) become a C-ABI
 // status: the flags ride along with the call's final device-to-host copy.  Call with work enqueued; synchronises.
 constexpr int TC_CNT = 16384; // batch GEMM: tiles whose pass groups run as separate units (a counter each)
 uint32_t give_up_cycles(const ps_cuda_ctx *ctx) { return ctx->opt_give_up >= 0 ? 1u << 24 : PS_TC_WAIT_CYCLES; } // option "give_up_warp": the other waits run out within 10 ms
@@ -261,7 +261,7 @@ int sync_and_check(ps_cuda_ctx *ctx) {
         PS_CK(cudaMemsetAsync(ctx->err_dev, 0, 16, ctx->stream));
         if (ctx->ag_ctr) PS_CK(cudaMemsetAsync(ctx->ag_ctr, 0, (size_t)ctx->d.n_layers * ctx->nkv_l * 8, ctx->stream)); // a group that gave up leaves its counter mid-instance
         if (ctx->tc_cnt) PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, TC_CNT * 4, ctx->stream)); // a GEMM that gave up leaves its tiles' counters part-way
-        return fail(ctx, PS_CUDA_ERR_CUDA, "device-side failure:%s%s%s (wait site %d; results of this call are invalid)", tc ? " tcgen05 pipeline time-out" : "",
+        return fail(ctx, PS_CUDA_ERR_CUDA, "device-side failure:%s%s%s (wait site %d; results of this call are invalid)", tc == PS_ERR_COPY ? " copy of a batch product did not arrive" : tc ? " tcgen05 pipeline time-out" : "",
                     tp ? " tensor-parallel peer wait gave up" : "", st ? " decode-step wait gave up" : "", st);
     }
     return 0;
@@ -405,7 +405,7 @@ template <int TYPE, int C> int launch_mo(ps_cuda_ctx *ctx, PsMbArgs a, bool *don
 int matmul_ob(ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int n_seg, const float *residual, bool *done) {
     PsMbArgs a{};
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
-    a.n_seg = n_seg; a.bs = (int)bs; a.K = K; a.aqs = ctx->aqs; a.ad = ctx->ad; a.residual = residual; a.err = ctx->tc_err_dev;
+    a.n_seg = n_seg; a.bs = (int)bs; a.K = K; a.aqs = ctx->aqs; a.ad = ctx->ad; a.residual = residual; a.err = ctx->tc_err_dev; a.give_up = ctx->opt_give_up;
     if (ctx->mv_type == 2) return bs <= 2 ? launch_mo<2, 2>(ctx, a, done) : bs <= 4 ? launch_mo<2, 4>(ctx, a, done) : launch_mo<2, 8>(ctx, a, done);
     return bs <= 2 ? launch_mo<8, 2>(ctx, a, done) : bs <= 4 ? launch_mo<8, 4>(ctx, a, done) : launch_mo<8, 8>(ctx, a, done);
 }

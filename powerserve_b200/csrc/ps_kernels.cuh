@@ -452,6 +452,7 @@ struct PsMbArgs {
     const uint32_t *aqs; const float *ad; const uint32_t *absp;
     const float *residual;
     int *err;           // (ps_k_matmul_ob) set if a copy did not arrive
+    int give_up;        // (ps_k_matmul_ob) warp whose first wait counts as run out (-1: none): how a test reaches the way out
 };
 template <int TYPE> PS_HD size_t ps_mb_smem(int64_t K, int C) {
     if (PsBlk<TYPE>::ELEMS == 256) return (size_t)C * (size_t)(K + K / 256 * 20);

@@ -369,6 +369,7 @@ __global__ void __launch_bounds__(64) ps_k_rope_kv(float *__restrict__ qr, const
 // the activations; rows of a 0.5B model are 4 to 22 KB.  On the GGUF bytes the kernel waited a memory round trip for every four
 // blocks of a row, with one warp per scheduler to hide it: 896 x 4864 on 32 columns 84 us.
 #define PS_MO_CHUNKS 8
+#define PS_ERR_COPY 9 // error code: a bulk copy of ps_k_matmul_ob did not arrive
 template <int TYPE> PS_HD size_t ps_mo_smem(int64_t K, int C, int warps) { return ps_mb_smem<TYPE>(K, C) + (size_t)warps * (size_t)(K / 32) * PsMv32<TYPE>::BLK; }
 template <int TYPE, int C>
 __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArgs a) {
@@ -405,8 +406,9 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
     for (int t = 0; t < R; t++)
 #pragma unroll
         for (int c = 0; c < C; c++) acc[t][c] = 0.f;
-    for (int g = 0; g < nbg; g++) {
-        if (g % cg == 0 && !ps_tc_wait(&bar[warp][g / cg], 0)) { *a.err = 9; break; }
+    bool ok = warp != a.give_up;
+    for (int g = 0; g < nbg && ok; g++) {
+        if (g % cg == 0 && !ps_tc_wait_warp(&bar[warp][g / cg], 0)) { ok = false; break; }
         int q[R][4];
         float xd[R][4];
 #pragma unroll
@@ -434,6 +436,11 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
                     acc[t][c] = __fmaf_rn(__fmul_rn(xd[t][b], ydv[b]), S, acc[t][c]);
                 }
         }
+    }
+    if (!ok) { // the other pieces arrive before this shared memory can become another CTA's (or the limit passes for each)
+        *a.err = PS_ERR_COPY;
+        for (int p = 0; p * 4 * cg < nb; p++) ps_tc_wait(&bar[warp][p], 0);
+        return;
     }
 #pragma unroll
     for (int t = 0; t < R; t++) {

@@ -1,4 +1,4 @@
-"""Waits of the tensor-core pipelines, read from the source: what no run on a GPU shows reliably.
+"""Waits of the kernels that copy ahead, read from the source: what no run on a GPU shows reliably.
 
 A wait gives up after a limit.  In a warp that stays converged - it elects a thread, or runs `.sync.aligned` tensor-memory instructions -
 giving up has to be one decision of the whole warp, and a warp whose lanes poll different barriers has to pass what each lane acquired on to
@@ -43,3 +43,9 @@ def test_epilogue_warps_meet_before_they_leave():
 def test_lanes_share_what_they_acquired():
     body = _body(_source("ps_tc.cuh"), "bool ps_tc_wait_all")
     assert "ps_tc_poll" in body and re.search(r"__syncwarp\(\);\s*return ok;\s*\}$", body) and body.count("return") == 1
+
+
+def test_copies_arrive_before_the_shared_memory_is_given_up():
+    body = _body(_source("ps_mv32.cuh"), "ps_k_matmul_ob(const PsMbArgs a)")
+    out = _body(body, "if (!ok)")
+    assert re.search(r"for \(int p = 0; p \* 4 \* cg < nb; p\+\+\) ps_tc_wait\(&bar\[warp\]\[p\], 0\);\s*return;", out)
