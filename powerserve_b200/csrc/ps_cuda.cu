@@ -114,7 +114,7 @@ struct ps_cuda_ctx {
     float *g = nullptr, *u = nullptr, *kq = nullptr, *logits = nullptr;
     const float *logits_last = nullptr; // where the last forward left its [bs][vocab] logits (ps_cuda_logits_dev)
     int logits_rows = 0;                // rows of that buffer
-    unsigned long long *topk_cand = nullptr; // device top-k scratch: keys of the slices' best, then the result: ids [PS_TOPK_MAX], values [PS_TOPK_MAX]
+    unsigned long long *topk_cand = nullptr; // device top-k scratch: keys of the slices' best, then the result: ids [k], values [k]
     uint32_t *aqs = nullptr, *absp = nullptr;
     float *ad = nullptr;
     int32_t *tokens_dev = nullptr, *pos_dev = nullptr, *ids_dev = nullptr;
@@ -2808,13 +2808,13 @@ int ps_cuda_sample_topk(ps_cuda_ctx *ctx, int row, int k, float *logits_out, int
     const float *logits = ctx->logits_last + (size_t)row * vocab;
     ps_k_topk_stage1<<<n_slices, 1024, 0, ctx->stream>>>(logits, vocab, k, ctx->topk_cand);
     PS_LAUNCH_CK();
-    ps_k_topk_stage2<<<1, 1024, 0, ctx->stream>>>(ctx->topk_cand, n_slices * k, k, logits, res, reinterpret_cast<float *>(res + PS_TOPK_MAX));
+    ps_k_topk_stage2<<<1, 1024, 0, ctx->stream>>>(ctx->topk_cand, n_slices * k, k, logits, res, reinterpret_cast<float *>(res + k));
     PS_LAUNCH_CK();
-    PS_CK(cudaMemcpyAsync(ctx->h_ids, res, PS_TOPK_MAX * 8, cudaMemcpyDeviceToHost, ctx->stream));
+    PS_CK(cudaMemcpyAsync(ctx->h_ids, res, (size_t)k * 8, cudaMemcpyDeviceToHost, ctx->stream));
     int rc = sync_and_check(ctx);
     if (rc) return rc;
     memcpy(tokens_out, ctx->h_ids, (size_t)k * 4);
-    memcpy(logits_out, ctx->h_ids + PS_TOPK_MAX, (size_t)k * 4);
+    memcpy(logits_out, ctx->h_ids + k, (size_t)k * 4);
     ctx->d2h += (int64_t)k * 8;
     return 0;
 }
