@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
 #pragma unroll
         for (int t = 0; t < R; t++) wr[t] = seg.w + (int64_t)min(row0 + 4 * t, seg.n - 1) * nb * B::BYTES;
         B next[R][4];
-        auto fetch = [&](int g) { // blocks past the end repeat the last one: their activation words and factors are zero
+        auto fetch = [&](int g) { // blocks past the end repeat the last one's words, against activation words of zero
 #pragma unroll
             for (int t = 0; t < R; t++)
 #pragma unroll
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
 #pragma unroll
             for (int t = 0; t < R; t++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) { q[t][b] = (int)next[t][b].q; xd[t][b] = next[t][b].xd; }
+                for (int b = 0; b < 4; b++) { q[t][b] = (int)next[t][b].q; xd[t][b] = 4 * g + b < nb ? next[t][b].xd : 0.f; } // (an infinite factor would make the zeros NaN)
             fetch(min(g + 1, nbg - 1));
 #pragma unroll
             for (int c = 0; c < C; c++) {

@@ -413,13 +413,13 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
         float xd[R][4];
 #pragma unroll
         for (int b = 0; b < 4; b++) {
-            const uint8_t *blk = sw + (size_t)min(4 * g + b, nb - 1) * G::BLK; // past the end: the last block again, its activations are zero
+            const uint8_t *blk = sw + (size_t)min(4 * g + b, nb - 1) * G::BLK; // past the end: the last block's words again, against zeros
 #pragma unroll
             for (int t = 0; t < R; t++) {
                 const int row = r0 + 4 * t;
                 const uint32_t w = *reinterpret_cast<const uint32_t *>(blk + row * G::QB + (TYPE == 2 ? (l & 3) : l) * 4);
                 q[t][b] = TYPE == 2 ? (int)__vsub4((l < 4) ? (w & 0x0f0f0f0fu) : ((w >> 4) & 0x0f0f0f0fu), 0x08080808u) : (int)w;
-                xd[t][b] = ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 8 * G::QB + 2 * row));
+                xd[t][b] = 4 * g + b < nb ? ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 8 * G::QB + 2 * row)) : 0.f;
             }
         }
 #pragma unroll

@@ -32,3 +32,55 @@ def test_a_warp_that_gives_up_ends_the_call(quant, tmp_path):
         cm.reset()
     om.close()
     cm.close()
+
+
+def _product(be, t, w, K, N, x, bs):
+    ref = np.zeros(N * bs, np.float32)
+    L.oracle().ps_or_matmul(t, L.vptr(w), K, N, L.fptr(x), bs, L.fptr(ref))
+    wd = be.register_weight(w, t, K, N)
+    xd, dd = be.upload(x), be.empty(N * bs)
+    be.matmul(dd, wd, t, K, N, xd, bs)
+    got = dd.numpy()
+    xd.free()
+    dd.free()
+    be.unregister_weight(w)
+    return got, ref
+
+
+@pytest.mark.parametrize("t", [L.Q8_0, L.Q4_0])
+@pytest.mark.parametrize("blocks", [1, 3, 4, 6])
+def test_infinite_scale_in_the_last_block(t, blocks):
+    """a damaged file's scale: an infinity stays one, whatever the number of blocks (groups of four are filled up with zeros)"""
+    be = capi.CudaBackend(capi.ModelDesc(256, 512, 1, 4, 4, 64, 512, 64, 1e-5, 64, 0, 1e4, 1.0, 1.0, 0, 8, 0, 1))
+    rng = np.random.default_rng(blocks)
+    K, N, bs = 32 * blocks, 21, 5
+    w = synth.random_blocks(rng, t, N, K, 0.1).reshape(N, blocks, -1)
+    w[::2, -1, :2] = np.frombuffer(np.float16(np.inf).tobytes(), np.uint8)
+    w[::2, -1, 2:] = 1 if t == L.Q8_0 else 0x99     # quants of one sign: every lane's sum is positive
+    got, ref = _product(be, t, np.ascontiguousarray(w.reshape(-1)), K, N, (1 + rng.random(K * bs)).astype(np.float32), bs)
+    assert np.isinf(ref.reshape(bs, N)[:, ::2]).all() and np.isfinite(ref.reshape(bs, N)[:, 1::2]).all()
+    L.assert_bit_equal(got, ref, f"type {t}, {blocks} blocks")
+    be.close()
+
+
+@pytest.mark.parametrize("quant", [gguf.GGML_Q8_0, gguf.GGML_Q4_0])
+def test_infinite_scale_in_the_head(quant, tmp_path, monkeypatch):
+    """the same on octet copies: rows of the head whose last of five blocks has an infinite scale; a logit is infinite where its eight lanes agree"""
+    def damaged(shape, seed=0, plain=synth.generate_tensors):
+        tensors = plain(shape, seed)
+        raw = next(d for n, _, _, d in tensors if n == "output.weight").view(np.uint8).reshape(2048, 5, -1)
+        raw[:, 4, :2] = np.frombuffer(np.float16(np.inf).tobytes(), np.uint8)
+        return tensors
+
+    monkeypatch.setattr(synth, "generate_tensors", damaged)
+    d = synth.write_model_dir(str(tmp_path / "m"), _shape(quant, 160, 320, 5, 2048), seed=3)
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=8)
+    assert cm.be.counter("mv32_ok") == 1
+    for bs in (2, 4, 8):
+        tokens = synth.random_prompt(2048, bs, seed=bs)
+        om.reset()
+        cm.reset()
+        want, got = om.forward(tokens), cm.forward(tokens)
+        assert np.isinf(want).any() and np.array_equal(want, got, equal_nan=True)
+    om.close()
+    cm.close()
