@@ -332,9 +332,10 @@ template <int TYPE, int C> int launch_mb(ps_cuda_ctx *ctx, PsMbArgs a) {
     return 0;
 }
 template <int TYPE> int launch_mb_t(ps_cuda_ctx *ctx, const PsMbArgs &a) {
-    if (a.bs <= 2) return launch_mb<TYPE, 2>(ctx, a);
-    if (a.bs <= 4 || ps_mb_smem<TYPE>(a.K, 8) > 200 * 1024) return launch_mb<TYPE, 4>(ctx, a);
-    return launch_mb<TYPE, 8>(ctx, a);
+    const auto fits = [&](int C) { return ps_mb_smem<TYPE>(a.K, C) <= 200 * 1024; }; // (the columns live in shared memory)
+    if (a.bs > 4 && fits(8)) return launch_mb<TYPE, 8>(ctx, a);
+    if (a.bs > 2 && fits(4)) return launch_mb<TYPE, 4>(ctx, a);
+    return launch_mb<TYPE, 2>(ctx, a);
 }
 // up to three matrices of one type that read the same quantised input
 int matmul_qb(ps_cuda_ctx *ctx, int wtype, int64_t K, int64_t bs, const PsMbSeg *segs, int n_seg, const float *residual) {

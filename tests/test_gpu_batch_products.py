@@ -84,3 +84,32 @@ def test_infinite_scale_in_the_head(quant, tmp_path, monkeypatch):
         assert np.isinf(want).any() and np.array_equal(want, got, equal_nan=True)
     om.close()
     cm.close()
+
+
+# 200 KB of shared memory: eight columns up to K = 22 656 (32-element blocks) or 23 552 (256), four up to 45 440 or 47 360, two beyond
+@pytest.mark.parametrize("t,K", [(L.Q8_0, 22656), (L.Q8_0, 22688), (L.Q8_0, 45472), (L.Q4_0, 45504), (L.Q6_K, 23808), (L.Q4_K, 47616)])
+@pytest.mark.parametrize("bs", [2, 3, 4, 8])
+def test_long_rows(t, K, bs):
+    be = capi.CudaBackend(capi.ModelDesc(256, K, 1, 4, 4, 64, 512, 64, 1e-5, 64, 0, 1e4, 1.0, 1.0, 0, 8, 0, 1))
+    rng = np.random.default_rng(K + bs)
+    w = synth.random_blocks(rng, t, 41, K, K ** -0.5).reshape(-1)
+    got, ref = _product(be, t, w, K, 41, rng.standard_normal(K * bs).astype(np.float32), bs)
+    L.assert_bit_equal(got, ref, f"type {t} K {K} bs {bs}")
+    be.close()
+
+
+@pytest.mark.parametrize("quant", [gguf.GGML_Q8_0, gguf.GGML_Q4_0])
+@pytest.mark.parametrize("ffn", [5152, 11040, 23008, 31008])
+def test_long_octets(quant, ffn, tmp_path):
+    """the down product on octet copies: beside eight staged columns there is room for the octets of four, two or one warp, or for none (then
+    ps_k_matmul_qb takes it); two and four columns leave more"""
+    d = synth.write_model_dir(str(tmp_path / "m"), _shape(quant, 256, ffn, 4, 512), seed=ffn)
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=8)
+    assert cm.be.counter("mv32_ok") == 1
+    for bs in (2, 3, 8):
+        tokens = synth.random_prompt(512, bs, seed=bs)
+        om.reset()
+        cm.reset()
+        L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"ffn {ffn} bs {bs}")
+    om.close()
+    cm.close()
