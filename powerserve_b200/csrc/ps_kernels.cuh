@@ -1439,9 +1439,10 @@ __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, con
 // device, so that k (logit, token) pairs cross PCIe instead of the vocabulary's logits and the host never builds a
 // vocabulary-sized ProbArray (prob_array.hpp:43-49).  Order: logit descending, equal logits by ascending token id (std::partial_sort
 // leaves that order unspecified); NaNs are never chosen.
-// Latency bounds both stages (one 0.5 MB read).  k rounds of a block-wide arg-max took 50 us a slice and 70 us for the merge at k = 40 and
-// 128 256 logits; sorting takes as many rounds as log2 squared whatever k is.  A value and its id make one 64-bit key (larger = better),
-// every CTA sorts its slice and hands on its k best, one CTA sorts those.
+// Latency bounds both stages (one 0.5 MB read).  A value and its id make one 64-bit key (larger = better); every CTA hands on the k best of its
+// slice, one CTA those of all.  Keys stay in registers and k rounds of a block-wide maximum take them out: two 32-bit warp reductions, a
+// barrier, two more.  Whole call, 128 256 logits, k = 1 / 8 / 40 / 64: 31 / 41 / 53 / 66 us; a block-wide sort of the slice 78 whatever k is
+// (74 to 135 for the largest vocabularies), rounds over keys in shared memory 34 / 56 / 144 / 242.
 // ====================================================================================================================
 #define PS_TOPK_MAX 64
 #define PS_TOPK_SLICE 2048
@@ -1451,17 +1452,31 @@ PS_D unsigned long long ps_topk_key(float v, int id) { // 0: not a candidate
     if (v != v) return 0ull;
     return ((unsigned long long)((u & 0x80000000u) ? ~u : (u | 0x80000000u)) << 32) | (uint32_t)~(uint32_t)id;
 }
-// descending bitonic sort of N (a power of two) keys in shared memory by the whole block
-template <int N> PS_D void ps_block_sort(unsigned long long *v) {
-    for (int size = 2; size <= N; size <<= 1)
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            __syncthreads();
-            for (int t = threadIdx.x; t < N / 2; t += blockDim.x) {
-                const int i = 2 * t - (t & (stride - 1)), j = i + stride;
-                const unsigned long long x = v[i], y = v[j];
-                if ((x < y) == ((i & size) == 0)) { v[i] = y; v[j] = x; }
-            }
-        }
+// the k largest of N keys in shared memory to its front, descending (0 where there are no more); 1024 threads
+template <int N> PS_D void ps_block_best(unsigned long long *v, int k) {
+    __shared__ unsigned long long part[2][32]; // each warp's best, by turns: a round's values are read before the next but one writes them
+    constexpr int P = N / 1024;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const auto warp_max = [](unsigned long long m) {
+        const uint32_t hi = __reduce_max_sync(PS_FULL, (uint32_t)(m >> 32)), lo = __reduce_max_sync(PS_FULL, (uint32_t)(m >> 32) == hi ? (uint32_t)m : 0u);
+        return ((unsigned long long)hi << 32) | lo;
+    };
+    unsigned long long x[P];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < P; i++) x[i] = v[threadIdx.x + 1024 * i];
+    for (int r = 0; r < k; r++) {
+        unsigned long long m = x[0];
+#pragma unroll
+        for (int i = 1; i < P; i++) m = x[i] > m ? x[i] : m;
+        m = warp_max(m);
+        if (lane == 0) part[r & 1][warp] = m;
+        __syncthreads();
+        m = warp_max(part[r & 1][lane]);
+#pragma unroll
+        for (int i = 0; i < P; i++) x[i] = x[i] == m ? 0ull : x[i]; // (keys differ by their ids)
+        if (threadIdx.x == 0) v[r] = m;
+    }
     __syncthreads();
 }
 // stage 1: CTA b -> keys of the k largest of logits[b * SLICE, (b + 1) * SLICE)
@@ -1469,7 +1484,7 @@ __global__ void __launch_bounds__(1024) ps_k_topk_stage1(const float *__restrict
     __shared__ unsigned long long v[PS_TOPK_SLICE];
     const int lo = blockIdx.x * PS_TOPK_SLICE;
     for (int t = threadIdx.x; t < PS_TOPK_SLICE; t += blockDim.x) v[t] = lo + t < n ? ps_topk_key(logits[lo + t], lo + t) : 0ull;
-    ps_block_sort<PS_TOPK_SLICE>(v);
+    ps_block_best<PS_TOPK_SLICE>(v, k);
     for (int t = threadIdx.x; t < k; t += blockDim.x) cand[blockIdx.x * k + t] = v[t];
 }
 // stage 2: one CTA merges n_cand candidates (in rounds that keep the k best so far at the front) into ids [k] and values [k]
@@ -1480,7 +1495,7 @@ __global__ void __launch_bounds__(1024) ps_k_topk_stage2(const unsigned long lon
     for (int lo = 0; lo < n_cand; have = k) {
         const int m = min(PS_TOPK_MERGE - have, n_cand - lo);
         for (int t = threadIdx.x; t < PS_TOPK_MERGE - have; t += blockDim.x) v[have + t] = t < m ? cand[lo + t] : 0ull;
-        ps_block_sort<PS_TOPK_MERGE>(v);
+        ps_block_best<PS_TOPK_MERGE>(v, k);
         lo += m;
     }
     for (int t = threadIdx.x; t < k; t += blockDim.x) {

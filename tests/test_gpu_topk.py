@@ -36,3 +36,18 @@ def test_planted_rows(vocab):
     vals, ids = m.sample_topk(3)
     assert list(ids) == [9, -1, -1] and vals[0] == 2.0 and np.all(np.isneginf(vals[1:]))
     m.close()
+
+
+def test_every_k():
+    """all k that a call takes, one after the other on one row: each is the front of the same order"""
+    shape = synth.ModelShape("topk", "llama", 256, 256, 1, 4, 4, 64, 5000, True, 0, 1e4, 1e-5, gguf.GGML_Q8_0, n_ctx=32)
+    tensors = {n: gguf.GGUFTensor(n, t, tuple(s), np.ascontiguousarray(d).view(np.uint8).reshape(-1)) for n, t, s, d in synth.generate_tensors(shape, 1)}
+    m = capi.CudaModel(desc=capi.desc_from_model_json(synth.model_json(shape), max_batch=2, n_ctx=32), tensors=tensors)
+    m.forward_lazy([1])
+    row = (np.random.default_rng(2).integers(-40, 40, 5000) * 0.25).astype(np.float32)
+    m.be._ck(m.be.L.ps_cuda_memcpy_h2d(m.be.h, m.be.logits_dev(), row.ctypes.data, row.nbytes))
+    order = np.lexsort((np.arange(5000), -row))
+    for k in list(range(1, 65)) + [3, 1]:
+        vals, ids = m.sample_topk(k)
+        assert list(ids) == list(order[:k]) and np.array_equal(vals, row[order[:k]]), k
+    m.close()
