@@ -1329,8 +1329,8 @@ __global__ void ps_k_sess_kv_store(float *const *__restrict__ kc_ptrs, float *co
     }
 }
 
-// scores of column c: kq_c {n_kv_c, 1, n_heads} at kq + c * col_stride; one warp per (cache position, kv head)
-__global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q, int hs,
+// scores of column c: kq_c {n_kv_c, 1, n_heads} at kq + c * col_stride; one warp per (cache position, kv head), HB heads of the group at a time
+template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q, int hs,
                                                         int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t col_stride) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z, g = blockIdx.y;
     const int64_t n_kv = (int64_t)pos[c] + 1, j = (int64_t)blockIdx.x * 4 + warp;
@@ -1340,7 +1340,7 @@ __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, 
     float kv[8];
 #pragma unroll
     for (int s = 0; s < 8; s++) kv[s] = (s < steps) ? krow[32 * s + lane] : 0.f;
-#pragma unroll 4
+#pragma unroll HB
     for (int hh = 0; hh < r2; hh++) {
         const int h = g * r2 + hh;
         const float *qv = q + ((int64_t)c * n_heads + h) * hs;
@@ -1395,8 +1395,8 @@ __global__ void __launch_bounds__(256) ps_k_sess_softmax(float *__restrict__ kq,
     for (int64_t j = threadIdx.x; j < ne0; j += blockDim.x) dp[j] = __fmul_rn(dp[j], inv);
 }
 
-// P.V of column c: out[c][h * hs + d]; one warp per (kv head g, d)
-__global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, const float *const *__restrict__ vct_ptrs, const float *__restrict__ kq, int hs,
+// P.V of column c: out[c][h * hs + d]; one warp per (kv head g, d), which takes HB of the group's heads at a time
+template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, const float *const *__restrict__ vct_ptrs, const float *__restrict__ kq, int hs,
                                                     int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t n_ctx, int64_t col_stride) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z;
     const int d = blockIdx.x * 4 + warp, g = blockIdx.y;
@@ -1405,31 +1405,33 @@ __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, con
     const int64_t n_kv = (int64_t)pos[c] + 1, np = n_kv & ~(int64_t)31;
     const int rem = (int)(n_kv - np);
     const float *vrow = vct_ptrs[c] + ((int64_t)g * hs + d) * n_ctx;
-    // Bound by memory latency.  Four heads of the group share a V row and their loads are in flight together; the leftover products are formed
+    // Bound by memory latency.  HB heads of the group share a V row and their loads are in flight together; the leftover products are formed
     // by the lanes and only their additions run one after the other (one head at a time, with lane 0 loading every leftover itself,
-    // 64 sessions of 100 to 200 positions took 75 us a layer of an 8B model).
-    for (int h0 = 0; h0 < r2; h0 += 4) {
-        const float *pr[4];
-        float sum[4], left[4];
+    // 64 sessions of 100 to 200 positions took 75 us a layer of an 8B model).  Four heads at a time, two or one where the group has no more: an absent
+    // head costs as much as a present one (64 sessions of 500 positions, a layer of 32 query and 32 kv heads: 805 us with four, 658 with one, 770
+    // with the loads of each head in turn)
+    for (int h0 = 0; h0 < r2; h0 += HB) {
+        const float *pr[HB];
+        float sum[HB], left[HB];
 #pragma unroll
-        for (int t = 0; t < 4; t++) { pr[t] = kq + c * col_stride + (int64_t)(g * r2 + min(h0 + t, r2 - 1)) * n_kv; sum[t] = 0.f; }
+        for (int t = 0; t < HB; t++) { pr[t] = kq + c * col_stride + (int64_t)(g * r2 + min(h0 + t, r2 - 1)) * n_kv; sum[t] = 0.f; }
         const float vl = lane < rem ? vrow[np + lane] : 0.f;
 #pragma unroll
-        for (int t = 0; t < 4; t++) left[t] = lane < rem ? __fmul_rn(vl, pr[t][np + lane]) : 0.f;
-#pragma unroll 2
+        for (int t = 0; t < HB; t++) left[t] = lane < rem ? __fmul_rn(vl, pr[t][np + lane]) : 0.f;
+#pragma unroll (HB == 4 ? 2 : 4)
         for (int64_t s = 0; s < np; s += 32) {
             const float v = vrow[s + lane];
 #pragma unroll
-            for (int t = 0; t < 4; t++) sum[t] = __fmaf_rn(v, pr[t][s + lane], sum[t]);
+            for (int t = 0; t < HB; t++) sum[t] = __fmaf_rn(v, pr[t][s + lane], sum[t]);
         }
 #pragma unroll
-        for (int t = 0; t < 4; t++) sum[t] = ps_f32x8_reduce(sum[t]);
+        for (int t = 0; t < HB; t++) sum[t] = ps_f32x8_reduce(sum[t]);
         for (int j = 0; j < rem; j++) // leftovers: mul, then add
 #pragma unroll
-            for (int t = 0; t < 4; t++) sum[t] = __fadd_rn(sum[t], __shfl_sync(PS_FULL, left[t], j));
+            for (int t = 0; t < HB; t++) sum[t] = __fadd_rn(sum[t], __shfl_sync(PS_FULL, left[t], j));
         if (lane == 0)
 #pragma unroll
-            for (int t = 0; t < 4; t++)
+            for (int t = 0; t < HB; t++)
                 if (h0 + t < r2) out[((int64_t)c * n_heads + g * r2 + h0 + t) * hs + d] = sum[t];
     }
 }

@@ -55,3 +55,25 @@ def test_batched_sessions_equal_single_sequence_decoding(preset, n_sess):
     for sid in sids[1:]:
         cm.session_destroy(sid)
     cm.close()
+
+
+@pytest.mark.parametrize("preset", ["tiny-q8", "tiny-qwen2-r7"])
+def test_heads_of_a_group_taken_together(preset):
+    """one query head per kv head, and seven (P.V takes four of a group at a time, and the rest): rows of 32 positions and leftovers"""
+    d = M.model_dir(preset)
+    vocab = synth.PRESETS[preset].vocab_size
+    cm = capi.CudaModel(d, max_batch=16)
+    prompts = [synth.random_prompt(vocab, n, seed=n) for n in (2, 32, 33, 64, 78)]
+    want = [alone(cm, p, 3, 16) for p in prompts]
+    sids = [0] + [cm.session_create() for _ in prompts[1:]]
+    for sid, p in zip(sids, prompts):
+        cm.session_select(sid)
+        cm.reset()
+        cm.prefill(p, 16)
+    toks = [int(p[-1]) for p in prompts]
+    for step in range(3):
+        lg, ids = cm.forward_sessions(sids, toks)
+        for col, w in enumerate(want):
+            L.assert_bit_equal(lg[col], w[1][step], f"{preset}: session {col} step {step}")
+        toks = [int(t) for t in ids]
+    cm.close()
