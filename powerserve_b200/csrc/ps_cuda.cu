@@ -777,51 +777,51 @@ int tc_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t n_rows, in
     PS_LAUNCH_CK();
     return 0;
 }
-// column-tile width of a batch: the fewest padded columns, counting a tile's own cost (its weights are de-quantised once per tile, about
-// the work of 40 columns)
-int tc_width(int bs) {
-    int best = 128;
+// How a product is cut: column-tile width and passes per unit, by the rounds that the GPU's CTAs (one an SM) need for all units and what a
+// round takes.  An entry (a super-block of a pass) takes 975, 662, 559, 428 or 376 ns at 128, 96, 64, 32 or 16 columns (224 row tiles x 16
+// super-blocks: 187, 127, 107, 82 and 72 us), so wide tiles are cheaper per column while there are units for every SM.  A small matrix is done in
+// one round whatever the width, and there a narrow tile ends first (a layer of 512 x 1536 on 128 columns: 156 us with 128-column tiles, 124 as
+// chosen here; 2048 x 8192: 261 and 253).  A narrower width has to promise a tenth: at 4096 x 14336 it promised 9 % and took 10 us more.
+// Fewer passes a unit cover the GPU with a small matrix and even out the last round, more save the hand-over of a tile's numbers: a unit that
+// hands over costs about seven entries more, because its 128 x width floats go through L2 and the tile's last unit reads all of them (224 row
+// tiles x 16 super-blocks at 16 columns: 88 us with one pass a unit, 78 with two, 74 with six)
+struct TcPlan { int nt, pp; };
+TcPlan tc_plan(const ps_cuda_ctx *ctx, int64_t row_tiles, int64_t K, int bs) {
+    static const struct { int nt, ns; } width[] = {{128, 975}, {96, 662}, {64, 559}, {32, 428}, {16, 376}};
+    TcPlan best = {128, PS_TC_PASSES};
     int64_t cost = INT64_MAX;
-    for (int nt : {128, 96, 64, 32, 16}) {
-        const int64_t c = (int64_t)((bs + nt - 1) / nt) * (nt + 40);
-        if (c < cost) { cost = c; best = nt; }
+    for (const auto &w : width) {
+        const int64_t tiles = row_tiles * ((bs + w.nt - 1) / w.nt);
+        for (int pp : {6, 2, 1}) {
+            const int64_t units = tiles * (PS_TC_PASSES / pp), rounds = (units + ctx->n_sm - 1) / ctx->n_sm;
+            if (pp < 6 && (tiles > TC_CNT || (size_t)units * PS_TC_M * w.nt * 4 > ctx->tc_part_bytes)) continue;
+            const int64_t c = rounds * (pp * tc_nbp(K) + (pp < 6 ? 7 : 0)) * w.ns;
+            if (w.nt == best.nt ? c < cost : c * 10 < cost * 9) { cost = c; best = {w.nt, pp}; }
+        }
     }
     return best;
 }
-int tc_prep_b(ps_cuda_ctx *ctx, const float *x, int K, int bs) {
-    const int nt = tc_width(bs), n_ct = (bs + nt - 1) / nt;
-    ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x, K, bs, nt);
-    PS_LAUNCH_CK();
-    return 0;
-}
-template <int NT> int tc_launch(ps_cuda_ctx *ctx, PsTcArgs &a) {
+
+template <int NT> int tc_launch(ps_cuda_ctx *ctx, const PsTcArgs &a) {
     static bool attr[64] = {};
     if (!attr[ctx->device]) {
         PS_CK(cudaFuncSetAttribute(ps_k_tc_gemm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PsTc<NT>::SMEM));
         attr[ctx->device] = true;
     }
-    // passes per unit: fewer passes cover the GPU with a small matrix and even out the last wave, more save the hand-over of a tile's numbers
-    // (a unit that hands over costs about as much as seven super-blocks: its 128 x NT floats go through L2 and the tile's last unit reads all of
-    // them; 224 row tiles x 16 super-blocks at 16 columns: 88 us with one pass a unit, 78 with two, 74 with six)
-    int64_t best = INT64_MAX;
-    const int slots = ctx->n_sm * PsTc<NT>::CTAS;
-    for (int pp : {6, 2, 1}) {
-        const int64_t units = (int64_t)a.n_tiles * (PS_TC_PASSES / pp), rounds = (units + slots - 1) / slots;
-        if (pp < 6 && (a.n_tiles > TC_CNT || (size_t)units * PS_TC_M * NT * 4 > ctx->tc_part_bytes)) continue;
-        const int64_t cost = rounds * ((int64_t)pp * a.nbp + (pp < 6 ? 7 : 0));
-        if (cost < best) { best = cost; a.pp = pp; }
-    }
     const int units = a.n_tiles * (PS_TC_PASSES / a.pp);
-    ps_k_tc_gemm<NT><<<(unsigned)std::min(units, slots), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
+    ps_k_tc_gemm<NT><<<(unsigned)std::min(units, ctx->n_sm), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
     PS_LAUNCH_CK();
     return 0;
 }
-// segments give their rows in the padded row space of the packed matrix (tile borders between them)
-int tc_gemm(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int64_t n_tiles, int64_t K, int bs, const PsRwSeg *segs, int n_seg, const float *residual) {
+// quantises the input and multiplies; segments give their rows in the padded row space of the packed matrix (tile borders between them)
+int tc_gemm(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n_tiles, int64_t K, int bs, const PsRwSeg *segs, int n_seg, const float *residual) {
     PsTcArgs a{};
-    const int nt = tc_width(bs);
+    const TcPlan plan = tc_plan(ctx, n_tiles, K, bs);
+    const int nt = plan.nt, n_ct = (bs + nt - 1) / nt;
+    ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x, K, bs, nt);
+    PS_LAUNCH_CK();
     a.err = ctx->tc_err_dev;
-    a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = (bs + nt - 1) / nt; a.n_tiles = (int)n_tiles * a.n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
+    a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = n_ct; a.n_tiles = (int)n_tiles * n_ct; a.pp = plan.pp; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
     a.part = ctx->tc_part; a.cnt = ctx->tc_cnt; a.give_up = ctx->opt_give_up; a.limit = give_up_cycles(ctx);
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
     ctx->n_tc++;
@@ -833,21 +833,21 @@ int tc_gemm(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int64_t n_tiles, int64_t 
     default: return tc_launch<16>(ctx, a);
     }
 }
-int tc_single(ps_cuda_ctx *ctx, const uint8_t *a_blocks, int64_t n_rows, int64_t K, float *dst, int bs, const float *residual) {
+int tc_single(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n_rows, int64_t K, float *dst, int bs, const float *residual) {
     PsRwSeg sg = {dst, nullptr, 0, (int)n_rows, 0};
-    return tc_gemm(ctx, a_blocks, tc_tiles(n_rows), K, bs, &sg, 1, residual);
+    return tc_gemm(ctx, x, a_blocks, tc_tiles(n_rows), K, bs, &sg, 1, residual);
 }
-int tc_qkv(ps_cuda_ctx *ctx, const LayerDev &ld, int64_t q_rows, int64_t kv_rows, int64_t K, int bs) {
+int tc_qkv(ps_cuda_ctx *ctx, const float *x, const LayerDev &ld, int64_t q_rows, int64_t kv_rows, int64_t K, int bs) {
     const bool bias = ctx->d.qkv_bias != 0;
     const int k0 = (int)tc_tiles(q_rows) * PS_TC_M, v0 = k0 + (int)tc_tiles(kv_rows) * PS_TC_M;
     const PsRwSeg sg[3] = {{ctx->q, bias ? ld.q_bias : nullptr, 0, (int)q_rows, 0}, {ctx->k, bias ? ld.k_bias : nullptr, k0, k0 + (int)kv_rows, 0},
                            {ctx->v, bias ? ld.v_bias : nullptr, v0, v0 + (int)kv_rows, 0}};
-    return tc_gemm(ctx, ld.tc_qkv, tc_tiles(q_rows) + 2 * tc_tiles(kv_rows), K, bs, sg, 3, nullptr);
+    return tc_gemm(ctx, x, ld.tc_qkv, tc_tiles(q_rows) + 2 * tc_tiles(kv_rows), K, bs, sg, 3, nullptr);
 }
-int tc_gate_up(ps_cuda_ctx *ctx, const LayerDev &ld, int64_t rows, int64_t K, int bs) {
+int tc_gate_up(ps_cuda_ctx *ctx, const float *x, const LayerDev &ld, int64_t rows, int64_t K, int bs) {
     const int u0 = (int)tc_tiles(rows) * PS_TC_M;
     const PsRwSeg sg[2] = {{ctx->g, nullptr, 0, (int)rows, 0}, {ctx->u, nullptr, u0, u0 + (int)rows, 0}};
-    return tc_gemm(ctx, ld.tc_gu, 2 * tc_tiles(rows), K, bs, sg, 2, nullptr);
+    return tc_gemm(ctx, x, ld.tc_gu, 2 * tc_tiles(rows), K, bs, sg, 2, nullptr);
 }
 
 // one decode step on the token in tokens_dev[0] at position pos_dev[0]; `pick`: run
@@ -2029,7 +2029,7 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
                     if ((rc = tc_pack(ctx, ld.tc_gu, ld.wup, ffn_l, dim, tc_tiles(ffn_l)))) return rc;
                     if ((rc = tc_pack(ctx, ld.tc_down, ld.wdown, dim_l, ffn, 0))) return rc;
                 }
-                const size_t cols = (size_t)(d.max_batch + 127) / 128 * 128; // no choice of tc_width pads a batch further
+                const size_t cols = (size_t)d.max_batch + 127; // (whole column tiles of any width)
                 if ((rc = dev_alloc(ctx, (void **)&ctx->tc_b, cols * (size_t)tc_nbp(ctx->maxK) * 644))) return rc;
                 const int64_t rows = std::max(std::max(tc_tiles(qdim_l) + 2 * tc_tiles(kvd_l), 2 * tc_tiles(ffn_l)), std::max(tc_tiles(dim_l), tc_tiles(vocab_l))) * PS_TC_M;
                 ctx->tc_part_bytes = std::max(std::min(TC_PART_MAX, (size_t)rows * cols * 4 * PS_TC_PASSES), (size_t)ctx->n_sm * PS_TC_M * 128 * 4);
@@ -2138,8 +2138,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.attn_norm, dim, d.norm_eps);
         PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_qkv(ctx, ld, qdim, kvd, dim, bs))) return rc;
+            if ((rc = tc_qkv(ctx, ctx->xn, ld, qdim, kvd, dim, bs))) return rc;
         } else if (rw) { // q | k | v rows in one pass over the concatenated octets
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             PsRwmArgs a{};
@@ -2203,8 +2202,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         PS_LAUNCH_CK();
         }
         if (tc) {
-            if ((rc = tc_prep_b(ctx, ctx->att, (int)qdim, bs))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_o, (int)dim, (int)qdim, ctx->x, bs, ctx->x))) return rc;
+            if ((rc = tc_single(ctx, ctx->att, ld.tc_o, (int)dim, (int)qdim, ctx->x, bs, ctx->x))) return rc;
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->att, (int)qdim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_o, (int)dim, (int)qdim, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
@@ -2218,8 +2216,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.ffn_norm, dim, d.norm_eps);
         PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_gate_up(ctx, ld, ffn, dim, bs))) return rc;
+            if ((rc = tc_gate_up(ctx, ctx->xn, ld, ffn, dim, bs))) return rc;
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;
@@ -2243,8 +2240,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         ps_k_silu_hadamard<<<grid1d(ffn * bs), 256, 0, ctx->stream>>>(ctx->g, ctx->g, ctx->u, ffn * bs);
         PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_prep_b(ctx, ctx->g, (int)ffn, bs))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_down, (int)dim, (int)ffn, ctx->x, bs, ctx->x))) return rc;
+            if ((rc = tc_single(ctx, ctx->g, ld.tc_down, (int)dim, (int)ffn, ctx->x, bs, ctx->x))) return rc;
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->g, (int)ffn, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_down, (int)dim, (int)ffn, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
@@ -2260,8 +2256,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ctx->w_out_norm, dim, d.norm_eps);
         PS_LAUNCH_CK();
         if (tc && ctx->tc_out) {
-            if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_single(ctx, ctx->tc_out, d.vocab_size, (int)dim, ctx->logits, bs, nullptr))) return rc;
+            if ((rc = tc_single(ctx, ctx->xn, ctx->tc_out, d.vocab_size, (int)dim, ctx->logits, bs, nullptr))) return rc;
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ctx->rw_out, d.vocab_size, (int)dim, 0, 1, ctx->logits, bs, nullptr, nullptr))) return rc;
@@ -2334,8 +2329,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
                          {ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)qdim_l, (int)(qdim_l + kvd), 0},
                          {ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)(qdim_l + kvd), (int)(qdim_l + 2 * kvd), 0}};
         if (tc) {
-            if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_qkv(ctx, ld, qdim_l, kvd, dim, bs))) return rc;
+            if ((rc = tc_qkv(ctx, ctx->xn, ld, qdim_l, kvd, dim, bs))) return rc;
         } else {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             PsRwmArgs a{};
@@ -2357,8 +2351,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         PS_LAUNCH_CK();
         if ((rc = tp_gather_rows(ctx, attb, ctx->att, bs, qdim_l))) return rc;                      // exchange 1: attention output
         if (tc) {
-            if ((rc = tc_prep_b(ctx, attb, (int)qdim, bs))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_o, (int)dim_l, (int)qdim, xl, bs, xl))) return rc;       // x[rows of this rank] += Wo[rows] . att
+            if ((rc = tc_single(ctx, attb, ld.tc_o, (int)dim_l, (int)qdim, xl, bs, xl))) return rc;       // x[rows of this rank] += Wo[rows] . att
         } else {
             if ((rc = rwm_quantize(ctx, attb, (int)qdim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_o, (int)dim_l, (int)qdim, 0, 1, xl, bs, nullptr, xl))) return rc;
@@ -2367,8 +2360,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, x, ld.ffn_norm, dim, d.norm_eps);
         PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_prep_b(ctx, ctx->xn, (int)dim, bs))) return rc;
-            if ((rc = tc_gate_up(ctx, ld, ffn_l, dim, bs))) return rc;
+            if ((rc = tc_gate_up(ctx, ctx->xn, ld, ffn_l, dim, bs))) return rc;
         } else {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn_l, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;
@@ -2378,8 +2370,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         PS_LAUNCH_CK();
         if ((rc = tp_gather_rows(ctx, hb, ctx->g, bs, ffn_l))) return rc;                             // exchange 3: FFN hidden vector
         if (tc) {
-            if ((rc = tc_prep_b(ctx, hb, (int)ffn, bs))) return rc;
-            if ((rc = tc_single(ctx, ld.tc_down, (int)dim_l, (int)ffn, xl, bs, xl))) return rc;     // x[rows] += Wdown[rows] . h
+            if ((rc = tc_single(ctx, hb, ld.tc_down, (int)dim_l, (int)ffn, xl, bs, xl))) return rc;     // x[rows] += Wdown[rows] . h
         } else {
             if ((rc = rwm_quantize(ctx, hb, (int)ffn, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_down, (int)dim_l, (int)ffn, 0, 1, xl, bs, nullptr, xl))) return rc;
