@@ -133,6 +133,7 @@ struct ps_cuda_ctx {
     int *h_err = nullptr;      // pinned mirror, read after every forward / decode (a set flag becomes PS_CUDA_ERR_CUDA)
     int *tc_err_dev = nullptr; // = err_dev + 0 (counter "tc_error")
     int64_t n_tc = 0;          // tcgen05 GEMM launches (counter "tc_gemm_launches")
+    int64_t n_tc_pp[7] = {};   // by passes a unit takes (counters "tc_gemm_pass1", "tc_gemm_pass2", "tc_gemm_pass6")
     std::vector<cudaEvent_t> kt_events; // option "ktime": event pairs around every row-walker mat-vec launch
     size_t kt_used = 0;
     double kt_ms = 0.0;                 // summed mat-vec kernel time of the last decode call
@@ -825,6 +826,7 @@ int tc_gemm(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n
     a.part = ctx->tc_part; a.cnt = ctx->tc_cnt; a.give_up = ctx->opt_give_up; a.limit = give_up_cycles(ctx);
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
     ctx->n_tc++;
+    ctx->n_tc_pp[plan.pp]++;
     switch (nt) {
     case 128: return tc_launch<128>(ctx, a);
     case 96: return tc_launch<96>(ctx, a);
@@ -2988,6 +2990,7 @@ int64_t ps_cuda_get_counter(ps_cuda_ctx *ctx, const char *name) {
     if (!strcmp(name, "matvec_kernel_launches")) return ctx->kt_launches;
     if (!strcmp(name, "tp_allgathers")) return ctx->n_gather;
     if (!strcmp(name, "tc_gemm_launches")) return ctx->n_tc;
+    if (!strncmp(name, "tc_gemm_pass", 12) && name[12] >= '1' && name[12] <= '6' && !name[13]) return ctx->n_tc_pp[name[12] - '0'];
     if (!strcmp(name, "tc_ok")) return ctx->tc_ok ? 1 : 0;
     if (!strcmp(name, "tc_error")) {
         int v = 0;

@@ -42,6 +42,7 @@ def test_two_passes_a_unit():
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=32)
     tokens = synth.random_prompt(2048, 20, seed=3)
     L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), "8B slice, 20 tokens")
+    assert cm.be.counter("tc_gemm_pass2") > 0
     again = cm.forward(tokens[:9])          # the counters of the tiles are left as they were found
     assert np.isfinite(again).all() and cm.be.counter("tc_error") == 0
     L.assert_bit_equal(again, om.forward(tokens[:9]), "8B slice, 9 more tokens")
@@ -67,3 +68,23 @@ def test_a_warp_that_gives_up_ends_the_call(odd, bs):
         cm.be.set_option("give_up_warp", -1)
         cm.reset()
         L.assert_bit_equal(cm.forward(tokens), want, f"after warp {warp} gave up")
+
+
+def test_every_number_of_passes(odd):
+    """what the widths above are spread over: units of one pass and of all six (the head's 51 row tiles)"""
+    cm = odd[1]
+    cm.reset()
+    n = [cm.be.counter(f"tc_gemm_pass{p}") for p in (1, 6)]
+    cm.forward(synth.random_prompt(ODD.vocab_size, 40, seed=40))
+    assert cm.be.counter("tc_gemm_pass1") > n[0] and cm.be.counter("tc_gemm_pass6") > n[1]
+
+
+@pytest.mark.parametrize("bs", [97, 128])
+def test_widest_tiles(bs):
+    """products large enough for column tiles of 128 at any number of passes (an 8B layer's)"""
+    d = M.model_dir("slice-8b")
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=128)
+    tokens = synth.random_prompt(2048, bs, seed=bs)
+    L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"8B slice, {bs} tokens")
+    om.close()
+    cm.close()
