@@ -297,21 +297,16 @@ void build_rope_table(const ps_cuda_model_desc &d, std::vector<float> &t, const 
     }
 }
 
-template <int TYPE, int C> size_t mm_smem(int64_t K) {
-    const int64_t nb = K / PsBlk<TYPE>::ELEMS;
-    return (size_t)C * (size_t)(K + nb * 4 + (PsBlk<TYPE>::ELEMS == 256 ? nb * 16 : 0));
-}
-
-template <int TYPE, int C>
-int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t N, int64_t bs, const float *bias, const float *residual) {
+template <int TYPE>
+int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t N, const float *bias, const float *residual) {
     static bool attr_set[64] = {};
-    const size_t smem = mm_smem<TYPE, C>(K);
+    const int64_t nb = K / PsBlk<TYPE>::ELEMS;
+    const size_t smem = (size_t)(K + nb * 4 + (PsBlk<TYPE>::ELEMS == 256 ? nb * 16 : 0));
     if (smem > 48 * 1024 && !attr_set[ctx->device]) {
-        PS_CK(cudaFuncSetAttribute(ps_k_matmul_q<TYPE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_q<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[ctx->device] = true;
     }
-    dim3 grid((unsigned)((N + 7) / 8), (unsigned)((bs + C - 1) / C));
-    ps_k_matmul_q<TYPE, C><<<grid, 256, smem, ctx->stream>>>(w, K, N, bs, ctx->aqs, ctx->ad, ctx->absp, dst, bias, residual);
+    ps_k_matmul_q<TYPE><<<(unsigned)((N + 7) / 8), 256, smem, ctx->stream>>>(w, K, N, ctx->aqs, ctx->ad, ctx->absp, dst, bias, residual);
     PS_LAUNCH_CK();
     return 0;
 }
@@ -377,11 +372,11 @@ int matmul_q(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int wtype, int64_t 
         return matmul_qb(ctx, wtype, K, bs, &sg, 1, residual);
     }
     switch (wtype) {
-    case 12: return launch_mm<12, 1>(ctx, dst, w, K, N, 1, bias, residual);
-    case 13: return launch_mm<13, 1>(ctx, dst, w, K, N, 1, bias, residual);
-    case 14: return launch_mm<14, 1>(ctx, dst, w, K, N, 1, bias, residual);
-    case 2: return launch_mm<2, 1>(ctx, dst, w, K, N, 1, bias, residual);
-    case 8: return launch_mm<8, 1>(ctx, dst, w, K, N, 1, bias, residual);
+    case 12: return launch_mm<12>(ctx, dst, w, K, N, bias, residual);
+    case 13: return launch_mm<13>(ctx, dst, w, K, N, bias, residual);
+    case 14: return launch_mm<14>(ctx, dst, w, K, N, bias, residual);
+    case 2: return launch_mm<2>(ctx, dst, w, K, N, bias, residual);
+    case 8: return launch_mm<8>(ctx, dst, w, K, N, bias, residual);
     default: return fail(ctx, PS_CUDA_ERR_UNSUPPORTED, "matmul: unsupported weight type %d", wtype);
     }
 }

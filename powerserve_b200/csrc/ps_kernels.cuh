@@ -339,100 +339,76 @@ template <> struct PsBlk<8> {
     }
 };
 
-// dst{N, bs} = W{K, N} . x{K, bs}; one warp per weight row, C activation columns per pass (gridDim.y passes).
-// Shared memory holds the C quantised columns.  Row results are bit-identical for every C (each column has its own
-// chain), which tests/test_gpu_ops.py checks.
-template <int TYPE, int C>
-__global__ void __launch_bounds__(256) ps_k_matmul_q(const uint8_t *__restrict__ w, int64_t K, int64_t N, int64_t bs,
-                                                     const uint32_t *__restrict__ aqs, const float *__restrict__ ad,
-                                                     const uint32_t *__restrict__ absp, float *__restrict__ dst,
-                                                     const float *__restrict__ bias, const float *__restrict__ residual) {
+// dst{N} = W{K, N} . x{K}, one column: one warp per weight row, four blocks of it side by side.  Shared memory holds the quantised column.
+template <int TYPE>
+__global__ void __launch_bounds__(256) ps_k_matmul_q(const uint8_t *__restrict__ w, int64_t K, int64_t N, const uint32_t *__restrict__ aqs, const float *__restrict__ ad,
+                                                     const uint32_t *__restrict__ absp, float *__restrict__ dst, const float *__restrict__ bias,
+                                                     const float *__restrict__ residual) {
     using B = PsBlk<TYPE>;
     constexpr bool KQ = (B::ELEMS == 256);
     extern __shared__ __align__(16) uint8_t smem[];
     const int64_t nb = K / B::ELEMS;
-    const int64_t col0 = (int64_t)blockIdx.y * C;
-    const int ncol = (int)min((int64_t)C, bs - col0);
-    // ---- stage the quantised activation columns
-    const int64_t qwords = K / 4;                       // words of quants per column
-    uint32_t *s_qs = reinterpret_cast<uint32_t *>(smem);                      // [C][K/4]
-    float *s_d = reinterpret_cast<float *>(s_qs + (int64_t)C * qwords);       // [C][nb]
-    uint32_t *s_bsp = reinterpret_cast<uint32_t *>(s_d + (int64_t)C * nb);    // [C][nb*4] (K-quants only)
-    for (int c = 0; c < ncol; c++) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(aqs + (col0 + c) * qwords);
-        uint4 *dstq = reinterpret_cast<uint4 *>(s_qs + c * qwords);
-        for (int64_t t = threadIdx.x; t < qwords / 4; t += blockDim.x) dstq[t] = src[t];
-        for (int64_t t = threadIdx.x; t < nb; t += blockDim.x) s_d[c * nb + t] = ad[(col0 + c) * nb + t];
-        if (KQ)
-            for (int64_t t = threadIdx.x; t < nb * 4; t += blockDim.x) s_bsp[c * nb * 4 + t] = absp[(col0 + c) * nb * 4 + t];
-    }
+    const int64_t qwords = K / 4;                                             // words of quants
+    uint32_t *s_qs = reinterpret_cast<uint32_t *>(smem);                      // [K/4]
+    float *s_d = reinterpret_cast<float *>(s_qs + qwords);                    // [nb]
+    uint32_t *s_bsp = reinterpret_cast<uint32_t *>(s_d + nb);                 // [nb*4] (K-quants only)
+    for (int64_t t = threadIdx.x; t < qwords / 4; t += blockDim.x) reinterpret_cast<uint4 *>(s_qs)[t] = reinterpret_cast<const uint4 *>(aqs)[t];
+    for (int64_t t = threadIdx.x; t < nb; t += blockDim.x) s_d[t] = ad[t];
+    if (KQ)
+        for (int64_t t = threadIdx.x; t < nb * 4; t += blockDim.x) s_bsp[t] = absp[t];
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l = lane & 7, b = lane >> 3;
     const int64_t n = (int64_t)blockIdx.x * 8 + warp;
     if (n >= N) return;
     const uint8_t *wrow = w + n * nb * B::BYTES;
-    float acc[C], accm[C];
-#pragma unroll
-    for (int c = 0; c < C; c++) { acc[c] = 0.f; accm[c] = 0.f; }
+    float acc = 0.f, accm = 0.f;
     for (int64_t i0 = 0; i0 < nb; i0 += 4) {
         const int64_t i = i0 + b;
-        const bool valid = i < nb;
-        B blk;
-        if (valid) blk.load(wrow + i * B::BYTES, l);
+        int S = 0, P = 0;
+        float d = 0.f, dm = 0.f;
+        if (i < nb) {
+            B blk;
+            blk.load(wrow + i * B::BYTES, l);
+            if constexpr (KQ) {
+                PsActQ8K a{reinterpret_cast<const uint4 *>(s_qs), s_d, s_bsp};
+                blk.partial(a, i, l, S, d, P, dm);
+            } else {
+                PsActQ80 a{s_qs, s_d};
+                blk.partial(a, i, l, S, d, P, dm);
+            }
+        }
+        // advance the 8 (+4) accumulator chains over the (up to) four blocks of this step, in row order
         const int nvalid = (int)min((int64_t)4, nb - i0);
+        for (int bb = 0; bb < nvalid; bb++) {
+            const int Sb = __shfl_sync(PS_FULL, S, bb * 8 + l);
+            const float db = __shfl_sync(PS_FULL, d, bb * 8 + l);
+            acc = __fmaf_rn(db, __int2float_rn(Sb), acc);
+            if constexpr (B::HAS_MIN && B::MIN_SCALAR) { // summs += dmin * hsum(prod): multiply, then add (Q5_K)
+                int Pt = 0;
 #pragma unroll
-        for (int c = 0; c < C; c++) {
-            if (c < ncol) {
-                int S = 0, P = 0;
-                float d = 0.f, dm = 0.f;
-                if (valid) {
-                    if constexpr (KQ) {
-                        PsActQ8K a{reinterpret_cast<const uint4 *>(s_qs + c * qwords), s_d + c * nb, s_bsp + c * nb * 4};
-                        blk.partial(a, i, l, S, d, P, dm);
-                    } else {
-                        PsActQ80 a{s_qs + c * qwords, s_d + c * nb};
-                        blk.partial(a, i, l, S, d, P, dm);
-                    }
-                }
-                // advance the 8 (+4) accumulator chains over the (up to) four blocks of this step, in row order
-                for (int bb = 0; bb < nvalid; bb++) {
-                    const int Sb = __shfl_sync(PS_FULL, S, bb * 8 + l);
-                    const float db = __shfl_sync(PS_FULL, d, bb * 8 + l);
-                    acc[c] = __fmaf_rn(db, __int2float_rn(Sb), acc[c]);
-                    if constexpr (B::HAS_MIN && B::MIN_SCALAR) { // summs += dmin * hsum(prod): multiply, then add (Q5_K)
-                        int Pt = 0;
-#pragma unroll
-                        for (int k = 0; k < 4; k++) Pt += __shfl_sync(PS_FULL, P, bb * 8 + k);
-                        const float dmb = __shfl_sync(PS_FULL, dm, bb * 8 + l);
-                        accm[c] = __fadd_rn(accm[c], __fmul_rn(dmb, __int2float_rn(Pt)));
-                    } else if constexpr (B::HAS_MIN) {
-                        const int Pb = __shfl_sync(PS_FULL, P, bb * 8 + (l & 3));
-                        const float dmb = __shfl_sync(PS_FULL, dm, bb * 8 + l);
-                        accm[c] = __fmaf_rn(dmb, __int2float_rn(Pb), accm[c]);
-                    }
-                }
+                for (int k = 0; k < 4; k++) Pt += __shfl_sync(PS_FULL, P, bb * 8 + k);
+                const float dmb = __shfl_sync(PS_FULL, dm, bb * 8 + l);
+                accm = __fadd_rn(accm, __fmul_rn(dmb, __int2float_rn(Pt)));
+            } else if constexpr (B::HAS_MIN) {
+                const int Pb = __shfl_sync(PS_FULL, P, bb * 8 + (l & 3));
+                const float dmb = __shfl_sync(PS_FULL, dm, bb * 8 + l);
+                accm = __fmaf_rn(dmb, __int2float_rn(Pb), accm);
             }
         }
     }
-#pragma unroll
-    for (int c = 0; c < C; c++) {
-        if (c < ncol) {
-            float r = ps_hsum8_lanes(acc[c]);
-            if constexpr (B::HAS_MIN && B::MIN_SCALAR) {
-                r = __fadd_rn(r, accm[c]); // hsum_float_8(acc) + summs
-            } else if constexpr (B::HAS_MIN) {
-                // acc_m = add(acc_m, movehl(acc_m)); add_ss(acc_m, movehdup(acc_m))   (ggml-quants.c:7868-7871)
-                const float m0 = __shfl_sync(PS_FULL, accm[c], 0), m1 = __shfl_sync(PS_FULL, accm[c], 1);
-                const float m2 = __shfl_sync(PS_FULL, accm[c], 2), m3 = __shfl_sync(PS_FULL, accm[c], 3);
-                r = __fadd_rn(r, __fadd_rn(__fadd_rn(m0, m2), __fadd_rn(m1, m3)));
-            }
-            if (lane == 0) {
-                const int64_t o = (col0 + c) * N + n;
-                if (bias) r = __fadd_rn(r, bias[n]);          // GGMLBackend::add with row broadcast (Qwen2 q/k/v bias)
-                if (residual) r = __fadd_rn(residual[o], r);  // residual add: x + W.h  (powerserve_compute_forward_add)
-                dst[o] = r;
-            }
-        }
+    float r = ps_hsum8_lanes(acc);
+    if constexpr (B::HAS_MIN && B::MIN_SCALAR) {
+        r = __fadd_rn(r, accm); // hsum_float_8(acc) + summs
+    } else if constexpr (B::HAS_MIN) {
+        // acc_m = add(acc_m, movehl(acc_m)); add_ss(acc_m, movehdup(acc_m))   (ggml-quants.c:7868-7871)
+        const float m0 = __shfl_sync(PS_FULL, accm, 0), m1 = __shfl_sync(PS_FULL, accm, 1);
+        const float m2 = __shfl_sync(PS_FULL, accm, 2), m3 = __shfl_sync(PS_FULL, accm, 3);
+        r = __fadd_rn(r, __fadd_rn(__fadd_rn(m0, m2), __fadd_rn(m1, m3)));
+    }
+    if (lane == 0) {
+        if (bias) r = __fadd_rn(r, bias[n]);          // GGMLBackend::add with row broadcast (Qwen2 q/k/v bias)
+        if (residual) r = __fadd_rn(residual[n], r);  // residual add: x + W.h  (powerserve_compute_forward_add)
+        dst[n] = r;
     }
 }
 

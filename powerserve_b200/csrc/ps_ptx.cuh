@@ -70,15 +70,6 @@ PS_D void ps_tc_commit(uint64_t *bar) {
 }
 PS_D void ps_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 PS_D void ps_tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-PS_D void ps_tc_ld8(uint32_t taddr, float v[8]) { // 32 lanes x 8 consecutive columns, one row (lane) per thread
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr)
-                 : "memory");
-#pragma unroll
-    for (int t = 0; t < 8; t++) v[t] = __uint_as_float(r[t]);
-}
 PS_D void ps_tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // bounded mbarrier wait: a mis-sequenced pipeline must never hang the GPU.  Gives up (returns false) after 2^31 SM cycles, about a second: a

@@ -56,7 +56,7 @@ template <int NT> struct PsTc {
     static constexpr int CW = NT / NH;                          // columns of a tensor-memory entry (N of one MMA)
     static constexpr int EW = NT >= 64 ? 16 : 8;                // epilogue warps
     static constexpr int EC = NT * 4 / EW;                      // columns a thread owns (its warp's lane quadrant gives the row)
-    static constexpr int NE = NT == 96 && NH == 1 ? 2 : 3, NA = 3; // tensor-memory rings: accumulator entries, A buffers
+    static constexpr int NE = NT == 96 ? 2 : 3, NA = 3; // tensor-memory rings: accumulator entries, A buffers
     static constexpr int NS = 3;                                // stages of two super-blocks (NE and NA divide 2 NS: the MMA loop is unrolled by it)
     static constexpr int ND = 2;                                // de-quantising warpgroups: one per super-block of a step
     static constexpr int THREADS = (EW + 4 * ND + 4) * 32;
@@ -71,7 +71,6 @@ template <int NT> struct PsTc {
     static constexpr int FACT = 2 * (PS_TC_A_D + NT * 4);       // d or -dmin of the rows, d of the columns
     static constexpr int STASH = EW * 32 * EC * 4;              // a pass's numbers while the next pass of its pair runs
     static constexpr int SMEM = NS * STAGE + NY * FACT + STASH;
-    static constexpr int CTAS = 1;
 };
 
 // ---------------------------------------------------------------------------------------------------- operand builders
@@ -237,7 +236,7 @@ PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity, uint32_t cycles) {
 
 // Persistent CTAs over units u = tile * (6 / pp) + group; tile = row tile * n_ct + column tile.
 template <int NT>
-__global__ void __launch_bounds__(PsTc<NT>::THREADS, PsTc<NT>::CTAS) ps_k_tc_gemm(const PsTcArgs a) {
+__global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcArgs a) {
     using T = PsTc<NT>;
     extern __shared__ __align__(1024) uint8_t ps_tc_smem[];
     __shared__ __align__(8) uint64_t bar_full[T::NS], bar_empty[T::NS], bar_a_full[T::NA], bar_a_empty[T::NA], bar_d_full[T::NE], bar_d_empty[T::NE], bar_y_empty[T::NY], bar_done;
