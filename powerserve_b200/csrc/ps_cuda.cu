@@ -313,19 +313,24 @@ int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t
 
 // one column: a warp per row (ps_k_matmul_q); more: a thread per AVX lane of a row (ps_k_matmul_qb).  Columns a thread keeps: as few as the
 // batch needs, up to eight (the accumulators of two rows x eight columns, twice that with mins, leave the loads in flight their registers)
-template <int TYPE, int C> int launch_mb(ps_cuda_ctx *ctx, PsMbArgs a) {
+template <int TYPE, int C, bool REST> int launch_mb_r(ps_cuda_ctx *ctx, PsMbArgs a) {
     constexpr int R = 2, ROWS = PS_MB_WARPS * 4 * R;
     static bool attr_set[64] = {};
     const size_t smem = ps_mb_smem<TYPE>(a.K, C);
     if (smem > 48 * 1024 && !attr_set[ctx->device]) {
-        PS_CK(cudaFuncSetAttribute(ps_k_matmul_qb<TYPE, R, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_qb<TYPE, R, C, REST>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[ctx->device] = true;
     }
     int cta = 0;
     for (int t = 0; t < a.n_seg; t++) { a.seg[t].cta0 = cta; cta += (a.seg[t].n + ROWS - 1) / ROWS; }
-    ps_k_matmul_qb<TYPE, R, C><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), PS_MB_WARPS * 32, smem, ctx->stream>>>(a);
+    ps_k_matmul_qb<TYPE, R, C, REST><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), PS_MB_WARPS * 32, smem, ctx->stream>>>(a);
     PS_LAUNCH_CK();
     return 0;
+}
+template <int TYPE, int C> int launch_mb(ps_cuda_ctx *ctx, const PsMbArgs &a) {
+    if constexpr (PsBlk<TYPE>::ELEMS == 32) // (a kernel of its own for a rest of blocks: a mask in the loop cost 4 to 16 %)
+        if (a.K % 128) return launch_mb_r<TYPE, C, true>(ctx, a);
+    return launch_mb_r<TYPE, C, false>(ctx, a);
 }
 template <int TYPE> int launch_mb_t(ps_cuda_ctx *ctx, const PsMbArgs &a) {
     const auto fits = [&](int C) { return ps_mb_smem<TYPE>(a.K, C) <= 200 * 1024; }; // (the columns live in shared memory)
@@ -382,22 +387,25 @@ int matmul_q(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int wtype, int64_t 
 }
 
 // the same on the octet copies of an all-Q4_0 / all-Q8_0 model (ps_k_matmul_ob); *done = false: a row octet does not fit shared memory
-template <int TYPE, int C> int launch_mo(ps_cuda_ctx *ctx, PsMbArgs a, bool *done) {
+template <int TYPE, int C, bool REST> int launch_mo_r(ps_cuda_ctx *ctx, PsMbArgs a, bool *done) {
     static bool attr_set[64] = {};
     int warps = PS_MB_WARPS;
     while (warps > 1 && ps_mo_smem<TYPE>(a.K, C, warps) > 200 * 1024) warps >>= 1;
     const size_t smem = ps_mo_smem<TYPE>(a.K, C, warps);
     if (smem > 200 * 1024) return 0;
     if (!attr_set[ctx->device]) {
-        PS_CK(cudaFuncSetAttribute(ps_k_matmul_ob<TYPE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_ob<TYPE, C, REST>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[ctx->device] = true;
     }
     int cta = 0;
     for (int t = 0; t < a.n_seg; t++) { a.seg[t].cta0 = cta; cta += (a.seg[t].n + 8 * warps - 1) / (8 * warps); }
-    ps_k_matmul_ob<TYPE, C><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), (unsigned)(warps * 32), smem, ctx->stream>>>(a);
+    ps_k_matmul_ob<TYPE, C, REST><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), (unsigned)(warps * 32), smem, ctx->stream>>>(a);
     PS_LAUNCH_CK();
     *done = true;
     return 0;
+}
+template <int TYPE, int C> int launch_mo(ps_cuda_ctx *ctx, const PsMbArgs &a, bool *done) {
+    return a.K % 128 ? launch_mo_r<TYPE, C, true>(ctx, a, done) : launch_mo_r<TYPE, C, false>(ctx, a, done);
 }
 int matmul_ob(ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int n_seg, const float *residual, bool *done) {
     PsMbArgs a{};

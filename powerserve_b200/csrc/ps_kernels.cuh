@@ -481,7 +481,8 @@ template <int C> PS_D void ps_mb_stage32(uint32_t *s_qs, float *s_d, const uint3
             if (t0 + u * (int)blockDim.x < m) s_d[t0 + u * blockDim.x] = v[u];
     }
 }
-template <int TYPE, int R, int C>
+// REST: 32-element blocks whose number is no multiple of four
+template <int TYPE, int R, int C, bool REST>
 __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArgs a) {
     using B = PsBlk<TYPE>;
     constexpr bool KQ = (B::ELEMS == 256);
@@ -548,7 +549,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
 #pragma unroll
         for (int t = 0; t < R; t++) wr[t] = seg.w + (int64_t)min(row0 + 4 * t, seg.n - 1) * nb * B::BYTES;
         B next[R][4];
-        auto fetch = [&](int g) { // blocks past the end repeat the last one's words, against activation words of zero
+        auto fetch = [&](int g) { // blocks past the end repeat the last one against activation words of zero
 #pragma unroll
             for (int t = 0; t < R; t++)
 #pragma unroll
@@ -561,7 +562,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
 #pragma unroll
             for (int t = 0; t < R; t++)
 #pragma unroll
-                for (int b = 0; b < 4; b++) { q[t][b] = (int)next[t][b].q; xd[t][b] = 4 * g + b < nb ? next[t][b].xd : 0.f; } // (an infinite factor would make the zeros NaN)
+                for (int b = 0; b < 4; b++) { q[t][b] = (int)next[t][b].q; xd[t][b] = !REST || 4 * g + b < nb ? next[t][b].xd : 0.f; } // (Inf x 0 would be NaN)
             fetch(min(g + 1, nbg - 1));
 #pragma unroll
             for (int c = 0; c < C; c++) {

@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(64) ps_k_rope_kv(float *__restrict__ qr, const
 #define PS_MO_CHUNKS 8
 #define PS_ERR_COPY 9 // error code: a bulk copy of ps_k_matmul_ob did not arrive
 template <int TYPE> PS_HD size_t ps_mo_smem(int64_t K, int C, int warps) { return ps_mb_smem<TYPE>(K, C) + (size_t)warps * (size_t)(K / 32) * PsMv32<TYPE>::BLK; }
-template <int TYPE, int C>
+template <int TYPE, int C, bool REST>
 __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArgs a) {
     using G = PsMv32<TYPE>;
     constexpr int R = 2;
@@ -406,20 +406,20 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
     for (int t = 0; t < R; t++)
 #pragma unroll
         for (int c = 0; c < C; c++) acc[t][c] = 0.f;
-    bool ok = warp != a.give_up;
-    for (int g = 0; g < nbg && ok; g++) {
-        if (g % cg == 0 && !ps_tc_wait_warp(&bar[warp][g / cg], 0)) { ok = false; break; }
+    bool ok = true;
+    for (int g = 0; g < nbg; g++) {
+        if (g % cg == 0 && (!ps_tc_wait_warp(&bar[warp][g / cg], 0) || warp == a.give_up)) { ok = false; break; }
         int q[R][4];
         float xd[R][4];
 #pragma unroll
         for (int b = 0; b < 4; b++) {
-            const uint8_t *blk = sw + (size_t)min(4 * g + b, nb - 1) * G::BLK; // past the end: the last block's words again, against zeros
+            const uint8_t *blk = sw + (size_t)min(4 * g + b, nb - 1) * G::BLK; // past the end: the last block again, against zeros
 #pragma unroll
             for (int t = 0; t < R; t++) {
                 const int row = r0 + 4 * t;
                 const uint32_t w = *reinterpret_cast<const uint32_t *>(blk + row * G::QB + (TYPE == 2 ? (l & 3) : l) * 4);
                 q[t][b] = TYPE == 2 ? (int)__vsub4((l < 4) ? (w & 0x0f0f0f0fu) : ((w >> 4) & 0x0f0f0f0fu), 0x08080808u) : (int)w;
-                xd[t][b] = 4 * g + b < nb ? ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 8 * G::QB + 2 * row)) : 0.f;
+                xd[t][b] = !REST || 4 * g + b < nb ? ps_half_bits_to_float(*reinterpret_cast<const unsigned short *>(blk + 8 * G::QB + 2 * row)) : 0.f;
             }
         }
 #pragma unroll
