@@ -313,8 +313,8 @@ int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t
 
 // one column: a warp per row (ps_k_matmul_q); more: a thread per AVX lane of a row (ps_k_matmul_qb).  Columns a thread keeps: as few as the
 // batch needs, up to eight (the accumulators of two rows x eight columns, twice that with mins, leave the loads in flight their registers)
-template <int TYPE, int C, bool REST> int launch_mb_r(ps_cuda_ctx *ctx, PsMbArgs a) {
-    constexpr int R = 2, ROWS = PS_MB_WARPS * 4 * R;
+template <int TYPE, int C, int R, bool REST = false> int launch_mb_r(ps_cuda_ctx *ctx, PsMbArgs a) {
+    constexpr int ROWS = PS_MB_WARPS * 4 * R;
     static bool attr_set[64] = {};
     const size_t smem = ps_mb_smem<TYPE>(a.K, C);
     if (smem > 48 * 1024 && !attr_set[ctx->device]) {
@@ -327,10 +327,21 @@ template <int TYPE, int C, bool REST> int launch_mb_r(ps_cuda_ctx *ctx, PsMbArgs
     PS_LAUNCH_CK();
     return 0;
 }
+// rows a thread takes: two, or one where 32-row CTAs would not reach every SM and 16-row ones are all resident together.  Q6_K, 2 / 3 / 8 columns:
+// 4096 x 1024 19 / 21 / 26 us with two rows, 15 / 15 / 19 with one (a warp per row: 14 / 15 / 25); 8192 x 2048 27 / 32 / 40 and 21 / 22 / 27 (19 / 23 /
+// 42).  On eight columns the four- and five-bit formats hide the loads (Q4_K 4096 x 4096, 5 columns: 19 us with two rows, 21 with one; Q6_K: 25
+// and 21), and 32-element blocks are four to a step
 template <int TYPE, int C> int launch_mb(ps_cuda_ctx *ctx, const PsMbArgs &a) {
+    if constexpr (PsBlk<TYPE>::ELEMS == 256 && (C <= 4 || TYPE == 14)) {
+        int64_t wide = 0, narrow = 0;
+        const int64_t cols = (a.bs + C - 1) / C;
+        for (int t = 0; t < a.n_seg; t++) { wide += (a.seg[t].n + 31) / 32; narrow += (a.seg[t].n + 15) / 16; }
+        const int64_t resident = 227 * 1024 / (int64_t)(ps_mb_smem<TYPE>(a.K, C) + 1024);
+        if (wide * cols < ctx->n_sm && narrow * cols <= resident * ctx->n_sm) return launch_mb_r<TYPE, C, 1>(ctx, a);
+    }
     if constexpr (PsBlk<TYPE>::ELEMS == 32) // (a kernel of its own for a rest of blocks: a mask in the loop cost 4 to 16 %)
-        if (a.K % 128) return launch_mb_r<TYPE, C, true>(ctx, a);
-    return launch_mb_r<TYPE, C, false>(ctx, a);
+        if (a.K % 128) return launch_mb_r<TYPE, C, 2, true>(ctx, a);
+    return launch_mb_r<TYPE, C, 2>(ctx, a);
 }
 template <int TYPE> int launch_mb_t(ps_cuda_ctx *ctx, const PsMbArgs &a) {
     const auto fits = [&](int C) { return ps_mb_smem<TYPE>(a.K, C) <= 200 * 1024; }; // (the columns live in shared memory)

@@ -418,6 +418,7 @@ __global__ void __launch_bounds__(256) ps_k_matmul_q(const uint8_t *__restrict__
 // every eight columns.  Bound by instruction issue: with 32-element blocks a chain step is dp4a (its start value 1.5 * 2^23 makes the
 // sum a float that one subtraction turns into the exact integer), subtraction, factor, FMA; one 16-byte shared-memory load brings
 // four steps.  4 x 8 rows a CTA: the 896-row matrices of a 0.5B model then fill 112 CTAs at 32 columns.
+// R = 1 (one row a thread, half as many rows a CTA) where there are few CTAs and the super-blocks of a row are one chain of latencies.
 // Up to three matrices of one type that read the same input run in one launch (q | k | v, gate | up).
 #define PS_MB_WARPS 4
 struct PsMbSeg { const uint8_t *w; float *dst; const float *bias; int n, cta0; };

@@ -113,3 +113,16 @@ def test_long_octets(quant, ffn, tmp_path):
         L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"ffn {ffn} bs {bs}")
     om.close()
     cm.close()
+
+
+@pytest.mark.parametrize("t", [L.Q4_K, L.Q5_K, L.Q6_K])
+@pytest.mark.parametrize("bs", [2, 4, 7])
+def test_rows_of_a_thread(t, bs):
+    """one row a thread up to 147 CTAs of 32 rows, two beyond, and two where the columns leave room for few CTAs an SM"""
+    be = capi.CudaBackend(capi.ModelDesc(256, 14336, 1, 4, 4, 64, 512, 64, 1e-5, 64, 0, 1e4, 1.0, 1.0, 0, 8, 0, 1))
+    rng = np.random.default_rng(bs)
+    for K, N in [(512, 4704), (512, 4705), (256, 17), (14336, 2400)]:
+        w = synth.random_blocks(rng, t, N, K, K ** -0.5).reshape(-1)
+        got, ref = _product(be, t, w, K, N, rng.standard_normal(K * bs).astype(np.float32), bs)
+        L.assert_bit_equal(got, ref, f"type {t} {K} x {N} bs {bs}")
+    be.close()
