@@ -406,9 +406,11 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
     for (int t = 0; t < R; t++)
 #pragma unroll
         for (int c = 0; c < C; c++) acc[t][c] = 0.f;
-    bool ok = true;
+    if (warp == a.give_up) *a.err = PS_ERR_COPY;
     for (int g = 0; g < nbg; g++) {
-        if (g % cg == 0 && (!ps_tc_wait_warp(&bar[warp][g / cg], 0) || warp == a.give_up)) { ok = false; break; }
+        // after a wait that gave up the results are invalid; the loop goes on and waits for the other pieces, each within its limit, so that none is in
+        // flight when this shared memory becomes another CTA's
+        if (g % cg == 0 && !ps_tc_wait(&bar[warp][g / cg], 0)) *a.err = PS_ERR_COPY;
         int q[R][4];
         float xd[R][4];
 #pragma unroll
@@ -436,11 +438,6 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
                     acc[t][c] = __fmaf_rn(__fmul_rn(xd[t][b], ydv[b]), S, acc[t][c]);
                 }
         }
-    }
-    if (!ok) { // the other pieces arrive before this shared memory can become another CTA's (or the limit passes for each)
-        *a.err = PS_ERR_COPY;
-        for (int p = 0; p * 4 * cg < nb; p++) ps_tc_wait(&bar[warp][p], 0);
-        return;
     }
 #pragma unroll
     for (int t = 0; t < R; t++) {

@@ -72,14 +72,8 @@ PS_D void ps_tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync
 PS_D void ps_tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 PS_D void ps_tc_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// bounded mbarrier wait: a mis-sequenced pipeline must never hang the GPU.  Gives up (returns false) after 2^31 SM cycles, about a second: a
-// poll itself may suspend the thread for microseconds, so a number of polls says little about the time
-#define PS_TC_WAIT_CYCLES 0x80000000u
-PS_D uint32_t ps_clock32() {
-    uint32_t t;
-    asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
-    return t;
-}
+// bounded mbarrier wait: a mis-sequenced pipeline must never hang the GPU.  A poll that fails has suspended the thread for 7 800 cycles, so
+// 2^18 polls are about a second; then it gives up (returns false)
 PS_D bool ps_tc_poll(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -89,17 +83,28 @@ PS_D bool ps_tc_poll(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity, uint32_t cycles = PS_TC_WAIT_CYCLES) {
-    if (ps_tc_poll(ps_smem_u32(bar), parity)) return true;
-    const uint32_t t0 = ps_clock32();
-    do {
+PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity) {
+    for (int spin = 0; spin < (1 << 18); spin++)
         if (ps_tc_poll(ps_smem_u32(bar), parity)) return true;
-    } while (ps_clock32() - t0 < cycles);
     return false;
 }
 // the same by a converged warp that goes on together: giving up is the warp's decision, not a lane's (elect.sync and the .aligned tcgen05
-// instructions that follow need all lanes)
-PS_D bool ps_tc_wait_warp(uint64_t *bar, uint32_t parity, uint32_t cycles = PS_TC_WAIT_CYCLES) { return __all_sync(0xffffffffu, ps_tc_wait(bar, parity, cycles)); }
+// instructions that follow need all lanes).  The limit is a time here, 2^31 SM cycles unless a test asks for less
+#define PS_TC_WAIT_CYCLES 0x80000000u
+PS_D uint32_t ps_clock32() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%clock;" : "=r"(t));
+    return t;
+}
+PS_D bool ps_tc_wait_warp(uint64_t *bar, uint32_t parity, uint32_t cycles = PS_TC_WAIT_CYCLES) {
+    bool ok = ps_tc_poll(ps_smem_u32(bar), parity);
+    if (!ok) {
+        const uint32_t t0 = ps_clock32();
+        do ok = ps_tc_poll(ps_smem_u32(bar), parity);
+        while (!ok && ps_clock32() - t0 < cycles);
+    }
+    return __all_sync(0xffffffffu, ok);
+}
 // named barrier that says whether `ok` holds in every one of its n threads
 PS_D bool ps_bar_all(int id, int n, bool ok) {
     uint32_t r;
