@@ -2092,8 +2092,9 @@ struct SessRun { int n_kv_max; };
 static void launch_batch_scores(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int64_t n_kv, int bs) {
     if (bs >= ctx->opt_scores_batch_min) {
         const int r2 = nh / nkv;
-        // queries a CTA keeps in shared memory: as many as fit, fewer (down to four) while the grid leaves the GPU idle - 32 queries of a 0.5B
-        // model over 32 keys: 4 CTAs 18 us
+        // queries a CTA keeps in shared memory: as many as fit, fewer (down to four) while the grid leaves the GPU idle (32 queries of a 0.5B
+        // model over 32 keys would be 4 CTAs: 172 us a layer, 162 with the rule; 128 queries, 2048 wide: 250 and 241).  Once, twice or four times
+        // the SMs as the border are within 1 % of one another
         int qb = std::max(1, std::min(bs, 8192 / (r2 * hs)));
         while (qb > 4 && (int64_t)((n_kv + 31) / 32) * nkv * ((bs + qb - 1) / qb) < 2 * ctx->n_sm) qb = std::max(4, (qb + 1) / 2);
         const dim3 grid((unsigned)((n_kv + 31) / 32), (unsigned)nkv, (unsigned)((bs + qb - 1) / qb));
@@ -2137,7 +2138,9 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     const bool tree = tree_base >= 0;
     const int64_t n_kv = sess ? (int64_t)sess->n_kv_max : tree ? (int64_t)tree_base + bs : (int64_t)pos0 + bs; // pos.back() + 1 (session batch: the longest row)
     const float kq_scale = 1.0f / sqrtf((float)hs);
-    const bool tc = ctx->tc_ok && ctx->opt_tc && ctx->opt_fused && bs >= ctx->opt_tc_min; // tensor-core GEMM on the packed blocks
+    // tensor-core GEMM on the packed blocks.  Row-walker / GEMM, us a layer: 8B 188 / 221 on 4 columns, 241 / 223 on 5, 263 / 223 on 6; 2048 x 8192
+    // 125 / 123, 158 / 124, 165 / 125; 512 x 1536 87 / 92, 93 / 92, 98 / 93
+    const bool tc = ctx->tc_ok && ctx->opt_tc && ctx->opt_fused && bs >= ctx->opt_tc_min;
     const bool mo = bs > 1 && mv_usable(ctx); // octet copies of a 32-block model
     const bool rw = ctx->fused_ok && ctx->opt_fused && (bs > 1 || tree); // octet-interleaved copies exist: multi-column row-walker
     int rc;
@@ -2489,7 +2492,8 @@ int ps_cuda_forward(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t *pos,
 // KV position is shared state.  Here a context can hold several independent KV sets ("sessions") over ONE set of weights:
 // ps_cuda_session_select makes one of them the target of every single-sequence call (forward / decode_greedy / kv_*: prefill
 // and bookkeeping work unchanged), and ps_cuda_forward_sessions advances n sessions by one token each in ONE forward pass -
-// the weight stream is read once for the n columns (multi-column row-walker for n < 16, tcgen05 GEMM from 16 up), attention
+// the weight stream is read once for the n columns (Q4_K: multi-column row-walker, tcgen05 GEMM from option tc_min up; other formats:
+// ps_k_matmul_ob or ps_k_matmul_qb), attention
 // runs per column over its own session's cache.  A session's logits are bit-identical to decoding it alone with batch 1.
 static int refresh_kv_tables(ps_cuda_ctx *ctx) {
     const ps_cuda_model_desc &d = ctx->d;

@@ -367,7 +367,8 @@ __global__ void __launch_bounds__(64) ps_k_rope_kv(float *__restrict__ qr, const
 // ps_k_matmul_qb's product (a thread = one AVX lane of two rows, C columns in registers) on the octet copies: a warp's eight rows are
 // ONE contiguous stream, which it requests whole at the start - bulk copies in PS_MO_CHUNKS pieces with a barrier each - while the CTA stages
 // the activations; rows of a 0.5B model are 4 to 22 KB.  On the GGUF bytes the kernel waited a memory round trip for every four
-// blocks of a row, with one warp per scheduler to hide it: 896 x 4864 on 32 columns 84 us.
+// blocks of a row, with one warp per scheduler to hide it: 896 x 4864 on 32 columns 84 us.  Pieces, us a layer on 4 / 32 / 128 columns: eight 108 /
+// 150 / 312, sixteen 109 / 153 / 316, two 105 / 145 / 297 (0.5B, Q4_0); 138 / 541 / 1892, 145 / 563 / 1978, 135 / 525 / 1836 (2048 x 8192, Q8_0).
 #define PS_MO_CHUNKS 8
 #define PS_ERR_COPY 9 // error code: a bulk copy of ps_k_matmul_ob did not arrive
 template <int TYPE> PS_HD size_t ps_mo_smem(int64_t K, int C, int warps) { return ps_mb_smem<TYPE>(K, C) + (size_t)warps * (size_t)(K / 32) * PsMv32<TYPE>::BLK; }

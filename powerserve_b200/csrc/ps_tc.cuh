@@ -13,15 +13,17 @@
 // (0,4) (2,6) (1,5) (3,7), which hsum_float_8 adds first, and the mins pairs (0,2) (1,3) - with 2 x NT / 4 accumulators a thread.  A
 // pass needs only its own quarter of the quants.  A pass ends with ONE number per output; the six are added in the reference's order
 //   ((r04 + r26) + (r15 + r37)) + (m02 + m13).
-//   * weights stay packed (20 480 B per 128 rows x 256, 1.11x the GGUF bytes): de-quantising warps (thread = row) turn the 16 bytes of a
+//   * weights stay packed (20 480 B per 128 rows x 256, 1.11x the GGUF bytes; a tile reads 29 696, since every lane pass takes all scales and every
+//     pass its factors): de-quantising warps (thread = row) turn the 16 bytes of a
 //     (row, lane) into 32 halves - (1024 + nibble) by bit insertion, one HFMA2 per two values for the subtraction and the scale - and
 //     write them with tcgen05.st straight into TENSOR MEMORY, from where tcgen05.mma takes its A operand: neither the expanded weights
 //     nor their re-reads cross shared memory, whose bandwidth would otherwise be the first limit.
 //   * activations (B): q8 as fp16 in canonical K-major tiles, written once per GEMM input by ps_k_tc_prep_b; TMA bulk copies.
 //   * accumulators: a ring of two or three tensor-memory entries of two chains (at 128 columns each entry is one half of the columns, and the
 //     MMAs of one half run while the epilogue warps of the other drain theirs); packed fma.rn.f32x2 advances two columns' chains per instruction.
-// Measured, 8B layer (q|k|v, o, gate|up, down): 128 columns 595 -> 385 us; 16 columns 196 -> 162.  What is left is mostly
-// synchronisation: stripped to its barriers the kernel keeps two thirds of its time (about 800 cycles per accumulator entry).
+// Measured, 8B layer (q|k|v, o, gate|up, down): 128 columns 595 -> 391 us; 16 columns 196 -> 161.  What is left is mostly
+// synchronisation: stripped to its barriers the kernel keeps two thirds of its time (about 800 cycles per accumulator entry).  128 columns
+// spill 80 bytes at the 72 registers that 28 warps leave a thread; no other width spills.
 // Pipeline: TMA producer -> de-quantising warps -> single-thread MMA issuer -> epilogue warps, linked by mbarriers.
 // Work: a unit is (row tile, column tile, pass group); 1, 2 or 6 passes a unit, so that small matrices still cover the GPU.  The unit
 // of a tile that finishes last adds the others' numbers (thread-private order in global memory) and stores.
