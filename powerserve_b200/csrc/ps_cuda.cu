@@ -125,15 +125,14 @@ struct ps_cuda_ctx {
     int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_scores_batch_min = 2, opt_give_up = -1;
     bool tc_ok = false;        // tensor-core prefill operands are resident
     uint8_t *tc_b = nullptr;   // B operand blocks of the current activation batch
-    float *tc_part = nullptr;  // pass groups' numbers of the tiles in flight
-    size_t tc_part_bytes = 0;
-    int *tc_cnt = nullptr;     // per tile: pass groups that have finished
+    float *tc_part = nullptr;  // numbers of the tiles that CTAs share: a slot per CTA
+    int *tc_cnt = nullptr;     // per slot: passes handed over
     int *err_dev = nullptr;    // device-detected failures, [0] tcgen05 pipeline time-out (PS_ERR_COPY: a copy of a batch product), [1] peer wait gave up, [2] step-kernel barrier time-out
     int err_seen[3] = {};      // sticky host copy of the flags (counters "tc_error" / "tp_error" / "step_error")
     int *h_err = nullptr;      // pinned mirror, read after every forward / decode (a set flag becomes PS_CUDA_ERR_CUDA)
     int *tc_err_dev = nullptr; // = err_dev + 0 (counter "tc_error")
     int64_t n_tc = 0;          // tcgen05 GEMM launches (counter "tc_gemm_launches")
-    int64_t n_tc_pp[7] = {};   // by passes a unit takes (counters "tc_gemm_pass1", "tc_gemm_pass2", "tc_gemm_pass6")
+    int64_t n_tc_pp[7] = {};   // by a CTA's share of passes: one, two, more (counters "tc_gemm_pass1", "tc_gemm_pass2", "tc_gemm_pass6")
     std::vector<cudaEvent_t> kt_events; // option "ktime": event pairs around every row-walker mat-vec launch
     size_t kt_used = 0;
     double kt_ms = 0.0;                 // summed mat-vec kernel time of the last decode call
@@ -251,7 +250,6 @@ int dev_alloc(ps_cuda_ctx *ctx, void **p, size_t bytes) {
 
 // Failures detected on the device (tcgen05 pipeline or copy time-out, a peer wait or a grid barrier that gave up) become a C-ABI
 // status: the flags ride along with the call's final device-to-host copy.  Call with work enqueued; synchronises.
-constexpr int TC_CNT = 16384; // batch GEMM: tiles whose pass groups run as separate units (a counter each)
 uint32_t give_up_cycles(const ps_cuda_ctx *ctx) { return ctx->opt_give_up >= 0 ? 1u << 24 : PS_TC_WAIT_CYCLES; } // option "give_up_warp": the other waits run out within 10 ms
 int sync_and_check(ps_cuda_ctx *ctx) {
     PS_CK(cudaMemcpyAsync(ctx->h_err, ctx->err_dev, 16, cudaMemcpyDeviceToHost, ctx->stream));
@@ -261,7 +259,7 @@ int sync_and_check(ps_cuda_ctx *ctx) {
         for (int k = 0; k < 3; k++) ctx->err_seen[k] |= ctx->h_err[k];
         PS_CK(cudaMemsetAsync(ctx->err_dev, 0, 16, ctx->stream));
         if (ctx->ag_ctr) PS_CK(cudaMemsetAsync(ctx->ag_ctr, 0, (size_t)ctx->d.n_layers * ctx->nkv_l * 8, ctx->stream)); // a group that gave up leaves its counter mid-instance
-        if (ctx->tc_cnt) PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, TC_CNT * 4, ctx->stream)); // a GEMM that gave up leaves its tiles' counters part-way
+        if (ctx->tc_cnt) PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, (size_t)ctx->n_sm * 4, ctx->stream)); // a GEMM that gave up leaves its counters part-way
         return fail(ctx, PS_CUDA_ERR_CUDA, "device-side failure:%s%s%s (wait site %d; results of this call are invalid)", tc == PS_ERR_COPY ? " copy of a batch product did not arrive" : tc ? " tcgen05 pipeline time-out" : "",
                     tp ? " tensor-parallel peer wait gave up" : "", st ? " decode-step wait gave up" : "", st);
     }
@@ -783,7 +781,6 @@ int rwm_single(ps_cuda_ctx *ctx, const uint8_t *w, int n_rows, int K, int slot, 
 }
 
 // ---- tcgen05 GEMM of token batches (ps_tc.cuh)
-constexpr size_t TC_PART_MAX = (size_t)96 << 20;
 int64_t tc_tiles(int64_t rows) { return (rows + PS_TC_M - 1) / PS_TC_M; }
 int64_t tc_nbp(int64_t K) { return (K / 256 + 1) & ~(int64_t)1; } // super-blocks, rounded up to whole steps
 size_t tc_a_bytes(int64_t rows, int64_t K) { return (size_t)tc_tiles(rows) * (size_t)tc_nbp(K) * PS_TC_A_BLOCK; }
@@ -792,39 +789,30 @@ int tc_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t n_rows, in
     PS_LAUNCH_CK();
     return 0;
 }
-// How a product is cut: column-tile width and passes per unit, by the rounds that the GPU's CTAs (one an SM) need for all units and what a
-// round takes.  An entry (a super-block of a pass) takes 975, 662, 559, 428 or 376 ns at 128, 96, 64, 32 or 16 columns (224 row tiles x 16
-// super-blocks: 187, 127, 107, 82 and 72 us), so wide tiles are cheaper per column while there are units for every SM.  A small matrix is done in
-// one round whatever the width, and there a narrow tile ends first (a layer of 512 x 1536 on 128 columns: 156 us with 128-column tiles, 124 as
-// chosen here; 2048 x 8192: 261 and 253).  A narrower width has to promise a tenth: at 4096 x 14336 it promised 9 % and took 10 us more.
-// Fewer passes a unit cover the GPU with a small matrix and even out the last round, more save the hand-over of a tile's numbers: a unit that
-// hands over costs about seven entries more, because its 128 x width floats go through L2 and the tile's last unit reads all of them (224 row
-// tiles x 16 super-blocks at 16 columns: 88 us with one pass a unit, 78 with two, 74 with six)
-struct TcPlan { int nt, pp; };
+// Column-tile width of a product.  Its passes are cut into one share per CTA, and a pass takes so many ns a super-block (16 to 64 columns: 203, 232, 264, 308)
+// and half a microsecond for its end.  So wide tiles are cheaper per column while every SM has a few passes, and of a small matrix, where a share is one
+// or two passes whatever the width, a narrow tile ends first (4096 x 4096 on 64 columns: 26.6 us with 64-column tiles, 25.6 with 32)
+struct TcPlan { int nt, share; };
 TcPlan tc_plan(const ps_cuda_ctx *ctx, int64_t row_tiles, int64_t K, int bs) {
-    static const struct { int nt, ns; } width[] = {{128, 975}, {96, 662}, {64, 559}, {32, 428}, {16, 376}};
-    TcPlan best = {128, PS_TC_PASSES};
+    static const struct { int nt, ns; } width[] = {{64, 308}, {48, 264}, {32, 232}, {16, 203}};
+    TcPlan best = {};
     int64_t cost = INT64_MAX;
     for (const auto &w : width) {
-        const int64_t tiles = row_tiles * ((bs + w.nt - 1) / w.nt);
-        for (int pp : {6, 2, 1}) {
-            const int64_t units = tiles * (PS_TC_PASSES / pp), rounds = (units + ctx->n_sm - 1) / ctx->n_sm;
-            if (pp < 6 && (tiles > TC_CNT || (size_t)units * PS_TC_M * w.nt * 4 > ctx->tc_part_bytes)) continue;
-            const int64_t c = rounds * (pp * tc_nbp(K) + (pp < 6 ? 7 : 0)) * w.ns;
-            if (w.nt == best.nt ? c < cost : c * 10 < cost * 9) { cost = c; best = {w.nt, pp}; }
-        }
+        const int64_t passes = row_tiles * ((bs + w.nt - 1) / w.nt) * PS_TC_PASSES, share = (passes + ctx->n_sm - 1) / ctx->n_sm;
+        const int64_t c = share * (tc_nbp(K) * w.ns + 500);
+        if (c < cost) { cost = c; best = {w.nt, (int)share}; }
     }
     return best;
 }
 
-template <int NT> int tc_launch(ps_cuda_ctx *ctx, const PsTcArgs &a) {
+template <int NT> int tc_launch(ps_cuda_ctx *ctx, PsTcArgs a) {
     static bool attr[64] = {};
     if (!attr[ctx->device]) {
         PS_CK(cudaFuncSetAttribute(ps_k_tc_gemm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PsTc<NT>::SMEM));
         attr[ctx->device] = true;
     }
-    const int units = a.n_tiles * (PS_TC_PASSES / a.pp);
-    ps_k_tc_gemm<NT><<<(unsigned)std::min(units, ctx->n_sm), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
+    if (a.give_up >= 0) a.give_up %= PsTc<NT>::THREADS / 32; // (a test's option; widths have 20 or 28 warps)
+    ps_k_tc_gemm<NT><<<(unsigned)std::min(a.n_tiles * PS_TC_PASSES, ctx->n_sm), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
     PS_LAUNCH_CK();
     return 0;
 }
@@ -836,15 +824,14 @@ int tc_gemm(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n
     ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x, K, bs, nt);
     PS_LAUNCH_CK();
     a.err = ctx->tc_err_dev;
-    a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = n_ct; a.n_tiles = (int)n_tiles * n_ct; a.pp = plan.pp; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
+    a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = n_ct; a.n_tiles = (int)n_tiles * n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
     a.part = ctx->tc_part; a.cnt = ctx->tc_cnt; a.give_up = ctx->opt_give_up; a.limit = give_up_cycles(ctx);
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
     ctx->n_tc++;
-    ctx->n_tc_pp[plan.pp]++;
+    ctx->n_tc_pp[plan.share > 2 ? PS_TC_PASSES : plan.share]++;
     switch (nt) {
-    case 128: return tc_launch<128>(ctx, a);
-    case 96: return tc_launch<96>(ctx, a);
     case 64: return tc_launch<64>(ctx, a);
+    case 48: return tc_launch<48>(ctx, a);
     case 32: return tc_launch<32>(ctx, a);
     default: return tc_launch<16>(ctx, a);
     }
@@ -2045,13 +2032,11 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
                     if ((rc = tc_pack(ctx, ld.tc_gu, ld.wup, ffn_l, dim, tc_tiles(ffn_l)))) return rc;
                     if ((rc = tc_pack(ctx, ld.tc_down, ld.wdown, dim_l, ffn, 0))) return rc;
                 }
-                const size_t cols = (size_t)d.max_batch + 127; // (whole column tiles of any width)
+                const size_t cols = (size_t)d.max_batch + 63; // (whole column tiles of any width)
                 if ((rc = dev_alloc(ctx, (void **)&ctx->tc_b, cols * (size_t)tc_nbp(ctx->maxK) * 644))) return rc;
-                const int64_t rows = std::max(std::max(tc_tiles(qdim_l) + 2 * tc_tiles(kvd_l), 2 * tc_tiles(ffn_l)), std::max(tc_tiles(dim_l), tc_tiles(vocab_l))) * PS_TC_M;
-                ctx->tc_part_bytes = std::max(std::min(TC_PART_MAX, (size_t)rows * cols * 4 * PS_TC_PASSES), (size_t)ctx->n_sm * PS_TC_M * 128 * 4);
-                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_part, ctx->tc_part_bytes))) return rc;
-                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_cnt, TC_CNT * 4))) return rc;
-                PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, TC_CNT * 4, ctx->stream));
+                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_part, (size_t)ctx->n_sm * PS_TC_PASSES * PS_TC_M * 64 * 4))) return rc;
+                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_cnt, (size_t)ctx->n_sm * 4))) return rc;
+                PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, (size_t)ctx->n_sm * 4, ctx->stream));
                 ctx->tc_ok = true;
                 if (tp == 1 && tc_a_bytes(vocab_l, dim) + ((size_t)8 << 30) < free_b - per_layer * (size_t)d.n_layers) { // lm_head too
                     if ((rc = dev_alloc(ctx, (void **)&ctx->tc_out, tc_a_bytes(vocab_l, dim)))) return rc;

@@ -9,8 +9,8 @@
 //
 // What bounds it.  The 12 FMAs per (row, column, super-block) are CUDA-core work that nothing replaces, and 12 accumulators per output
 // limit a tile that holds them all to 128 x 32; such a tile re-reads (and would have to de-quantise) its weights for every 32 columns.
-// So a tile is 128 rows x NT columns (up to 128) and its chains are taken in six PASSES over K of two chains each - the lane pairs
-// (0,4) (2,6) (1,5) (3,7), which hsum_float_8 adds first, and the mins pairs (0,2) (1,3) - with 2 x NT / 4 accumulators a thread.  A
+// So a tile is 128 rows x NT columns (up to 64) and its chains are taken in six PASSES over K of two chains each - the lane pairs
+// (0,4) (2,6) (1,5) (3,7), which hsum_float_8 adds first, and the mins pairs (0,2) (1,3) - with 2 x NT / 2 accumulators a thread.  A
 // pass needs only its own quarter of the quants.  A pass ends with ONE number per output; the six are added in the reference's order
 //   ((r04 + r26) + (r15 + r37)) + (m02 + m13).
 //   * weights stay packed (20 480 B per 128 rows x 256, 1.11x the GGUF bytes; a tile reads 29 696, since every lane pass takes all scales and every
@@ -19,14 +19,18 @@
 //     write them with tcgen05.st straight into TENSOR MEMORY, from where tcgen05.mma takes its A operand: neither the expanded weights
 //     nor their re-reads cross shared memory, whose bandwidth would otherwise be the first limit.
 //   * activations (B): q8 as fp16 in canonical K-major tiles, written once per GEMM input by ps_k_tc_prep_b; TMA bulk copies.
-//   * accumulators: a ring of two or three tensor-memory entries of two chains (at 128 columns each entry is one half of the columns, and the
-//     MMAs of one half run while the epilogue warps of the other drain theirs); packed fma.rn.f32x2 advances two columns' chains per instruction.
-// Measured, 8B layer (q|k|v, o, gate|up, down): 128 columns 595 -> 391 us; 16 columns 196 -> 161.  What is left is mostly
-// synchronisation: stripped to its barriers the kernel keeps two thirds of its time (about 800 cycles per accumulator entry).  128 columns
-// spill 80 bytes at the 72 registers that 28 warps leave a thread; no other width spills.
-// Pipeline: TMA producer -> de-quantising warps -> single-thread MMA issuer -> epilogue warps, linked by mbarriers.
-// Work: a unit is (row tile, column tile, pass group); 1, 2 or 6 passes a unit, so that small matrices still cover the GPU.  The unit
-// of a tile that finishes last adds the others' numbers (thread-private order in global memory) and stores.
+//   * accumulators: a ring of tensor-memory entries; packed fma.rn.f32x2 advances two columns' chains per instruction.
+// Pipeline: TMA producer -> de-quantising warps -> single-thread MMA issuer -> epilogue warps, linked by four kinds of mbarrier: a stage is
+// full / empty, an entry may be computed (go: its A written, its accumulators drained) / is computed (done).
+// Work: all passes of all tiles in a row, cut into one contiguous share per CTA, so that the shares differ by one pass at most and a CTA hands numbers
+// over for two tiles at most, whatever the matrix.  The CTA that finishes a shared tile last adds the numbers and stores.
+//
+// Measured (time that each further super-block of a pass adds, at 1.92 GHz; 128 rows x 16 / 32 / 48 / 64 columns): 390 / 450 / 510 / 590 cycles, where a kernel with
+// two units of work to a tile, epilogue warps of half the columns and a barrier per hand-over needed 720 to 820 at any width.  Where it goes (64 columns): the
+// epilogue's own work 270 (16 FMUL2 and 32 FFMA2 a warp, 192 of pipe time), de-quantising 140 in a lane pass, and what the roles need for their waits and rings:
+// 630 of 1 800 instructions.  28 672 x 4096 on 16 / 32 / 64 / 128 columns: 86 / 108 / 104 / 168 -> 45 / 55 / 80 / 138 us; 4096 x 14 336 on 128: 104 -> 80.
+// An epilogue that reads more than eight columns at a time spills or moves registers (64 columns: 590 cycles with 8, 655 with 16, 676 with 32, 700 with two
+// buffers of 8); the end of a pass is met once per pass with cold instructions, so its loops hold no branches (64 columns: 12 us a tile with, 3.5 without).
 #pragma once
 #include "ps_rw.cuh"
 
@@ -52,27 +56,31 @@ PS_HD int ps_tc_pass(int l) { return ((l & 1) << 1) | ((l >> 1) & 1); }
 
 // configuration by column-tile width
 template <int NT> struct PsTc {
-    // column halves, each with epilogue warps of its own.  An entry costs the issuing warp about as much whatever its width, so one wide entry
-    // is better where tensor memory holds enough of them (64 columns, 448 row tiles' worth of units: 134 us with two halves, 108 with one)
-    static constexpr int NH = NT >= 97 ? 2 : 1;
-    static constexpr int CW = NT / NH;                          // columns of a tensor-memory entry (N of one MMA)
-    static constexpr int EW = NT >= 64 ? 16 : 8;                // epilogue warps
+    static constexpr int EW = 8;                                // epilogue warps
     static constexpr int EC = NT * 4 / EW;                      // columns a thread owns (its warp's lane quadrant gives the row)
-    static constexpr int NE = NT == 96 ? 2 : 3, NA = 3; // tensor-memory rings: accumulator entries, A buffers
-    static constexpr int NS = 3;                                // stages of two super-blocks (NE and NA divide 2 NS: the MMA loop is unrolled by it)
-    static constexpr int ND = 2;                                // de-quantising warpgroups: one per super-block of a step
+    // super-blocks of an entry: with two, every role waits half as often (48 columns: 510 cycles a super-block).  At 64 columns tensor memory holds three
+    // entries of one super-block, or one of two
+    static constexpr int XE = NT <= 48 ? 2 : 1;
+    static constexpr int NE = XE == 1 ? 3 : NT == 16 ? 4 : 2;   // ring of accumulator entries with their A
+    // de-quantising warpgroups, one per super-block of a step.  Where the epilogue is short they set the pace: four then take every second step
+    // (16 columns: 450 -> 390 cycles, 32: 464 -> 450; 48 columns 510 -> 530, so two)
+    static constexpr int ND = NT <= 32 ? 4 : 2;
+    static constexpr int NS = NT <= 48 ? 6 : 5;                 // stages of two super-blocks (even where ND is 4: a group then sees every use of its slots)
     static constexpr int THREADS = (EW + 4 * ND + 4) * 32;
-    static constexpr bool SPLIT = NT >= 96;                     // setmaxnreg: EC accumulator pairs do not fit an even share of the registers
-    static constexpr int TM_A = NE * 2 * CW;                    // first tensor-memory column of the A buffers
-    static constexpr int TM_USED = TM_A + NA * 32;
+    // registers a thread of the epilogue and of the de-quantising warps (setmaxnreg; the rest has 24): they add up to what the block is launched with
+    static constexpr int R_EPI = ND == 4 ? 128 : 160, R_DEQ = ND == 4 ? 56 : 64;
+    static constexpr int TM_E = XE * 2 * NT;                    // tensor-memory columns of an entry's accumulators
+    static constexpr int TM_A = NE * TM_E;                      // first column of the A buffers
+    static constexpr int TM_USED = TM_A + NE * XE * 32;
     static constexpr int TM_COLS = TM_USED <= 256 ? 256 : 512;
     static constexpr int STAGE_SC = 2 * PS_TC_A_Q;              // quants, scales, B of the two super-blocks (a mins pass: mins at the front, B)
     static constexpr int STAGE_B = STAGE_SC + 2 * PS_TC_A_SC;
     static constexpr int STAGE = STAGE_B + 2 * NT * 128;
-    static constexpr int NY = 2 * NS;                           // the factors' ring: the epilogue still reads them when the stage has been refilled
+    static constexpr int NY = NS + (XE == 1 ? 2 : NE); // the factors' ring: the epilogue still reads them when the stage has been refilled
     static constexpr int FACT = 2 * (PS_TC_A_D + NT * 4);       // d or -dmin of the rows, d of the columns
-    static constexpr int STASH = EW * 32 * EC * 4;              // a pass's numbers while the next pass of its pair runs
-    static constexpr int SMEM = NS * STAGE + NY * FACT + STASH;
+    static constexpr int STASH = EW * 32 * EC * 4;              // numbers of a tile: the pass before, the sum of the pairs before
+    static constexpr int SMEM = NS * STAGE + NY * FACT + 2 * STASH;
+    static_assert(TM_USED <= 512 && SMEM <= 230000 && (ND == 2 || NS % 2 == 0), "");
 };
 
 // ---------------------------------------------------------------------------------------------------- operand builders
@@ -166,12 +174,12 @@ __global__ void __launch_bounds__(128) ps_k_tc_prep_b(uint8_t *__restrict__ dst,
 struct PsTcArgs {
     const uint8_t *a;   // [row tiles][nbp * PS_TC_A_BLOCK]
     const uint8_t *b;   // [column tiles][nbp * PS_TC_B_BLOCK(NT)]
-    int nbp, n_ct, n_tiles, pp; // super-blocks (even); column tiles; row tiles x column tiles; passes a unit takes (1, 2 or 6)
+    int nbp, n_ct, n_tiles; // super-blocks (even); column tiles; row tiles x column tiles
     PsRwSeg seg[PS_TC_SEGS]; // rows row_begin .. row_end of the padded row space; dst of a segment is [bs][rows of the segment]
     int n_seg, bs;
     const float *residual;
-    float *part;        // [tile][units of a tile][EC][epilogue threads]
-    int *cnt;           // per tile: units that have finished (left at zero)
+    float *part;        // [CTA][pass][EC][epilogue threads]: numbers of the shared tile that begins in a CTA's share (there is one at most)
+    int *cnt;           // [CTA]: how many of its passes have been handed over (left at zero)
     int *err;           // set if a pipeline wait gave up (results invalid)
     int give_up;        // warp whose first wait counts as run out (-1: none): how a test reaches the way out
     uint32_t limit;     // cycles a wait lasts at most
@@ -184,19 +192,17 @@ PS_D ps_f2 ps_f2_mul(ps_f2 a, ps_f2 b) { ps_f2 r; asm("mul.rn.f32x2 %0, %1, %2;"
 PS_D ps_f2 ps_f2_add(ps_f2 a, ps_f2 b) { ps_f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 PS_D ps_f2 ps_f2_fma(ps_f2 a, ps_f2 b, ps_f2 c) { ps_f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
-// eight columns of one row of two accumulators, as pairs of columns, with the wait for them
-PS_D void ps_tc_ld8x2(uint32_t t0, uint32_t t1, ps_f2 v[8]) {
-    asm volatile(
-        "{\n\t.reg .b32 a<8>;\n\t.reg .b32 b<8>;\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {a0,a1,a2,a3,a4,a5,a6,a7}, [%8];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {b0,b1,b2,b3,b4,b5,b6,b7}, [%9];\n\t"
-        "tcgen05.wait::ld.sync.aligned;\n\t"
-        "mov.b64 %0, {a0,a1};\n\tmov.b64 %1, {a2,a3};\n\tmov.b64 %2, {a4,a5};\n\tmov.b64 %3, {a6,a7};\n\t"
-        "mov.b64 %4, {b0,b1};\n\tmov.b64 %5, {b2,b3};\n\tmov.b64 %6, {b4,b5};\n\tmov.b64 %7, {b6,b7};\n\t}"
-        : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]), "=l"(v[4]), "=l"(v[5]), "=l"(v[6]), "=l"(v[7])
-        : "r"(t0), "r"(t1)
-        : "memory");
+// eight columns of one row of an accumulator; they are there after ps_tc_ld_wait, and ps_tc_pass keeps whatever reads them behind it
+PS_D void ps_tc_ld(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
 }
+PS_D void ps_tc_pass(uint32_t (&v)[8]) {
+    asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])::"memory");
+}
+PS_D ps_f2 ps_f2_bits(uint32_t a, uint32_t b) { ps_f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
 PS_D void ps_tc_st8(uint32_t taddr, const uint32_t v[8]) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
                  "r"(v[5]), "r"(v[6]), "r"(v[7])
@@ -236,36 +242,53 @@ PS_D bool ps_tc_wait_all(uint32_t bar, uint32_t parity, uint32_t cycles) {
     return ok;
 }
 
-// Persistent CTAs over units u = tile * (6 / pp) + group; tile = row tile * n_ct + column tile.
+PS_D int ps_add_acq_rel(int *p, int v) {
+    int r;
+    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(r) : "l"(p), "r"(v) : "memory");
+    return r;
+}
+// the CTA's passes: q = tile * 6 + pass, a contiguous share of all of them
+PS_D int ps_tc_share(int c, int n_cta, int n_tiles) { return (int)((int64_t)n_tiles * PS_TC_PASSES * c / n_cta); }
+// does a share begin at pass q?
+PS_D bool ps_tc_cut(int q, int n_cta, int n_tiles) {
+    const int64_t n = (int64_t)n_tiles * PS_TC_PASSES;
+    return ps_tc_share((int)(((int64_t)q * n_cta + n - 1) / n), n_cta, n_tiles) == q;
+}
+
+// the CTA whose share holds pass q
+PS_D int ps_tc_owner(int q, int n_cta, int n_tiles) {
+    const int64_t n = (int64_t)n_tiles * PS_TC_PASSES;
+    return (int)(((int64_t)(q + 1) * n_cta + n - 1) / n) - 1;
+}
+
 template <int NT>
 __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcArgs a) {
     using T = PsTc<NT>;
     extern __shared__ __align__(1024) uint8_t ps_tc_smem[];
-    __shared__ __align__(8) uint64_t bar_full[T::NS], bar_empty[T::NS], bar_a_full[T::NA], bar_a_empty[T::NA], bar_d_full[T::NE], bar_d_empty[T::NE], bar_y_empty[T::NY], bar_done;
+    // full: a stage has been copied; empty: its MMAs are complete; go: an entry's A is in tensor memory and its accumulators have been read;
+    // done: its MMAs are complete (accumulators readable, A writable)
+    __shared__ __align__(8) uint64_t bar_full[T::NS], bar_empty[T::NS], bar_go[T::NE], bar_done[T::NE], bar_end;
     __shared__ uint32_t tmem_base_smem;
     __shared__ int sh_last;
     const int tid = threadIdx.x, warp = __shfl_sync(PS_FULL, tid >> 5, 0), lane = tid & 31;
-    const int ns = a.nbp >> 1, pp = a.pp, nu = PS_TC_PASSES / pp; // steps of a pass, units of a tile
-    const int n_units = a.n_tiles * nu;
+    const int ns = a.nbp >> 1; // steps of a pass
+    const int q0 = ps_tc_share(blockIdx.x, gridDim.x, a.n_tiles), q1 = ps_tc_share(blockIdx.x + 1, gridDim.x, a.n_tiles);
     constexpr int W_TMA = T::EW + 4 * T::ND, W_MMA = W_TMA + 1;
     uint8_t *const ps_tc_fact = ps_tc_smem + (size_t)T::NS * T::STAGE;
 
     if (tid == 0) {
         for (int s = 0; s < T::NS; s++) {
             ps_mbar_init(&bar_full[s], 1);
-            ps_mbar_init(&bar_empty[s], 4 * T::ND + 1); // the de-quantising warps, the MMA commit
-        }
-        for (int s = 0; s < T::NA; s++) {
-            ps_mbar_init(&bar_a_full[s], 4);
-            ps_mbar_init(&bar_a_empty[s], 1);
+            ps_mbar_init(&bar_empty[s], 1);
         }
         for (int s = 0; s < T::NE; s++) {
-            ps_mbar_init(&bar_d_full[s], 1);
-            ps_mbar_init(&bar_d_empty[s], T::EW / T::NH);
+            ps_mbar_init(&bar_go[s], 4 * T::XE + T::EW);
+            ps_mbar_init(&bar_done[s], 1);
         }
-        for (int s = 0; s < T::NY; s++) ps_mbar_init(&bar_y_empty[s], T::EW);
-        ps_mbar_init(&bar_done, 1);
+        ps_mbar_init(&bar_end, 1);
         ps_fence_barrier_init();
+        for (int s = 0; s < T::NE; s++) // the entries are free at first
+            for (int w = 0; w < T::EW; w++) ps_mbar_arrive(&bar_go[s]);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == W_MMA) { // the MMA warp owns the tensor memory
@@ -278,7 +301,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcA
     const uint32_t tmem_base = tmem_base_smem;
 
     if (warp >= W_TMA) {
-        if (T::SPLIT) ps_reg_dec<24>();
+        ps_reg_dec<24>();
         if (warp == W_TMA) {
             // ===== TMA producer
             PsRing<T::NS> st;
@@ -286,317 +309,323 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcA
             int g = 0;
             bool ok = warp != a.give_up;
             if (!ok) *a.err = 1;
-            for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-                const int tile = u / nu, p0 = (u % nu) * pp;
+            for (int q = q0; q < q1 && ok; q++) {
+                const int tile = q / PS_TC_PASSES, p = q % PS_TC_PASSES;
+                const bool lanes = p < 4;
                 const uint8_t *pa = a.a + (size_t)(tile / a.n_ct) * a.nbp * PS_TC_A_BLOCK, *pb = a.b + (size_t)(tile % a.n_ct) * a.nbp * PS_TC_B_BLOCK(NT);
-                for (int p = p0; p < p0 + pp && ok; p++) {
-                    const bool lanes = p < 4;
-                    const uint8_t *aq = pa + (lanes ? (size_t)p * a.nbp * PS_TC_A_Q : PS_TC_A_OFF_MN(a.nbp)), *as = pa + PS_TC_A_OFF_SC(a.nbp);
-                    const uint8_t *ad = pa + (lanes ? PS_TC_A_OFF_D(a.nbp) : PS_TC_A_OFF_DM(a.nbp));
-                    const uint8_t *bq = pb + (lanes ? (size_t)p * a.nbp * (NT * 128) : (size_t)a.nbp * (NT * 512) + (size_t)(p - 4) * a.nbp * (NT * 64));
-                    const uint8_t *by = pb + (size_t)a.nbp * (NT * 640);
-                    const uint32_t na = lanes ? 2 * PS_TC_A_Q : 2 * PS_TC_A_MN, nbb = lanes ? 2 * NT * 128 : 2 * NT * 64;
-                    const uint32_t total = na + (lanes ? 2 * PS_TC_A_SC : 0) + 2 * PS_TC_A_D + nbb + 2 * NT * 4;
-                    for (int i = 0; i < ns; i++, g++, st.step(), sy.step()) {
-                        const bool fy = (lane & 1) && g >= T::NY; // odd lanes wait for the factors' slot
-                        if (g >= T::NS && !ps_tc_wait_all(ps_smem_u32(fy ? &bar_y_empty[sy.i] : &bar_empty[st.i]), (fy ? sy.round : st.round) ^ 1, a.limit)) { *a.err = 1; ok = false; break; }
-                        uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE, *sf = ps_tc_fact + sy.i * T::FACT;
-                        uint64_t *bar = &bar_full[st.i];
-                        if (ps_elect_one()) {
-                            ps_mbar_expect_tx(bar, total);
-                            ps_bulk_g2s(sm, aq, na, bar);
-                            ps_bulk_g2s(sm + T::STAGE_B, bq, nbb, bar);
-                            if (lanes) ps_bulk_g2s(sm + T::STAGE_SC, as, 2 * PS_TC_A_SC, bar);
-                            ps_bulk_g2s(sf, ad, 2 * PS_TC_A_D, bar);
-                            ps_bulk_g2s(sf + 2 * PS_TC_A_D, by, 2 * NT * 4, bar);
-                        }
-                        __syncwarp();
-                        aq += na;
-                        bq += nbb;
-                        as += 2 * PS_TC_A_SC;
-                        ad += 2 * PS_TC_A_D;
-                        by += 2 * NT * 4;
+                const uint8_t *aq = pa + (lanes ? (size_t)p * a.nbp * PS_TC_A_Q : PS_TC_A_OFF_MN(a.nbp)), *as = pa + PS_TC_A_OFF_SC(a.nbp);
+                const uint8_t *ad = pa + (lanes ? PS_TC_A_OFF_D(a.nbp) : PS_TC_A_OFF_DM(a.nbp));
+                const uint8_t *bq = pb + (lanes ? (size_t)p * a.nbp * (NT * 128) : (size_t)a.nbp * (NT * 512) + (size_t)(p - 4) * a.nbp * (NT * 64));
+                const uint8_t *by = pb + (size_t)a.nbp * (NT * 640);
+                const uint32_t na = lanes ? 2 * PS_TC_A_Q : 2 * PS_TC_A_MN, nbb = lanes ? 2 * NT * 128 : 2 * NT * 64;
+                const uint32_t total = na + (lanes ? 2 * PS_TC_A_SC : 0) + 2 * PS_TC_A_D + nbb + 2 * NT * 4;
+                for (int i = 0; i < ns; i++, g++, st.step(), sy.step()) {
+                    // the MMAs of stage g - NS are complete: its operands have been read; entries three super-blocks before have been drained, and
+                    // with them the factors of stage g - NS - 2
+                    if (g >= T::NS && !ps_tc_wait_warp(&bar_empty[st.i], st.round ^ 1, a.limit)) { *a.err = 1; ok = false; break; }
+                    uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE, *sf = ps_tc_fact + sy.i * T::FACT;
+                    uint64_t *bar = &bar_full[st.i];
+                    if (ps_elect_one()) {
+                        ps_mbar_expect_tx(bar, total);
+                        ps_bulk_g2s(sm, aq, na, bar);
+                        ps_bulk_g2s(sm + T::STAGE_B, bq, nbb, bar);
+                        if (lanes) ps_bulk_g2s(sm + T::STAGE_SC, as, 2 * PS_TC_A_SC, bar);
+                        ps_bulk_g2s(sf, ad, 2 * PS_TC_A_D, bar);
+                        ps_bulk_g2s(sf + 2 * PS_TC_A_D, by, 2 * NT * 4, bar);
                     }
+                    __syncwarp();
+                    aq += na;
+                    bq += nbb;
+                    as += 2 * PS_TC_A_SC;
+                    ad += 2 * PS_TC_A_D;
+                    by += 2 * NT * 4;
                 }
             }
             // copies in flight end before the CTA does (they have, unless a wait gave up)
             for (int k = g > T::NS ? g - T::NS : 0; k < g; k++)
                 if (!ps_tc_wait(&bar_full[k % T::NS], (k / T::NS) & 1)) { *a.err = 5; break; }
         } else if (warp == W_MMA) {
-            // ===== MMA issuer.  The warp stays converged and one thread, chosen by elect.sync, issues; ring positions are constants of the
-            // unrolled loop.  So descriptors and barrier addresses live in uniform registers: with one thread looping under `lane == 0` an
-            // issue took 280 cycles whatever its size, where tcgen05.mma itself takes 32 here.
+            // ===== MMA issuer.  The warp stays converged and one thread, chosen by elect.sync, issues, so that descriptors and barrier addresses
+            // live in uniform registers
             // kind::f16, D = F32 (bit 4), A = B = F16, K-major both, N >> 3 @ bit 17, M >> 4 @ bit 24
-            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(T::CW >> 3) << 17) | ((uint32_t)(PS_TC_M >> 4) << 24);
-            constexpr bool ODD = (2 * T::NS * T::NH / T::NE) & 1; // the entries' ring turns an odd number of times in the unrolled loop
+            constexpr uint32_t idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(PS_TC_M >> 4) << 24);
             const uint64_t desc0 = ps_tc_smem_desc(ps_smem_u32(ps_tc_smem + T::STAGE_B), NT * 16, 128);
-            const int n_steps = n_units > (int)blockIdx.x ? ((n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1) * pp * ns : 0;
-            int u = blockIdx.x, p = (u % nu) * pp, p_end = p + pp, left = ns;
+            PsRing<T::NS> st;
+            PsRing<T::NE> re;
             bool ok = warp != a.give_up;
             if (!ok) *a.err = 2;
-            for (int g0 = 0; g0 < n_steps && ok; g0 += T::NS) {
-                const uint32_t round = (uint32_t)(g0 / T::NS) & 1; // of the stages; the other rings' parities are constants
+            for (int q = q0; q < q1 && ok; q++) {
+                const bool lanes = q % PS_TC_PASSES < 4;
+                for (int i = 0; i < ns && ok; i++, st.step()) {
+                    const uint64_t ds = desc0 + (uint64_t)(st.i * (T::STAGE >> 4));
 #pragma unroll
-                for (int j = 0; j < T::NS; j++) {
-                    if (g0 + j >= n_steps || !ok) break;
-                    const bool lanes = p < 4;
+                    for (int e = 0; e < 2 / T::XE; e++, re.step()) {
+                        const uint32_t ta = tmem_base + T::TM_A + re.i * (T::XE * 32), td = tmem_base + re.i * T::TM_E;
+                        // (the de-quantising warps have waited for the stage, B with it)
+                        if (!ps_tc_wait_warp(&bar_go[re.i], re.round, a.limit)) { *a.err = 2; ok = false; break; }
+                        ps_tc_fence_after();
+                        if (ps_elect_one()) {
+                            if (lanes) {
 #pragma unroll
-                    for (int x = 0; x < 2; x++) { // the step's super-blocks
-                        const int k = 2 * j + x, ra = k % T::NA;
-                        const uint32_t ta = tmem_base + T::TM_A + ra * 32;
-                        const uint64_t ds = desc0 + (uint64_t)(j * (T::STAGE >> 4)) + (x ? (lanes ? NT * 8 : NT * 4) : 0);
-#pragma unroll
-                        for (int h = 0; h < T::NH; h++) {
-                            const int e = k * T::NH + h, re = e % T::NE;
-                            // lane 0: the accumulator entry (free from the start in the first round), lane 1: A, the others: the stage
-                            const bool fd = lane == 0 && (g0 > 0 || e >= T::NE), fa = lane == 1;
-                            const uint32_t bar = ps_smem_u32(fd ? &bar_d_empty[re] : fa ? &bar_a_full[ra] : &bar_full[j]);
-                            if (!ps_tc_wait_all(bar, fd ? ((e / T::NE) & 1) ^ 1 ^ (ODD ? round : 0) : fa ? (k / T::NA) & 1 : round, a.limit)) { *a.err = 2; ok = false; break; }
-                            ps_tc_fence_after();
-                            const uint32_t td = tmem_base + re * (2 * T::CW);
-                            const uint64_t dh = ds + h * (T::CW / 8) * 8;
-                            if (ps_elect_one()) {
-                                if (lanes) {
-                                    ps_tc_mma_f16_ta(td, ta, dh, idesc, 0);
-                                    ps_tc_mma_f16_ta(td, ta + 8, dh + NT * 2, idesc, 1);
-                                    ps_tc_mma_f16_ta(td + T::CW, ta + 16, dh + NT * 4, idesc, 0);
-                                    ps_tc_mma_f16_ta(td + T::CW, ta + 24, dh + NT * 6, idesc, 1);
-                                } else {
-                                    ps_tc_mma_f16_ta(td, ta, dh, idesc, 0);
-                                    ps_tc_mma_f16_ta(td + T::CW, ta, dh + NT * 2, idesc, 0);
+                                for (int k = 0; k < 2 * T::XE; k++) { // super-block k / 2 of the entry, chain k % 2
+                                    const uint64_t dk = ds + (2 * T::XE * e + k) * (NT * 4);
+                                    ps_tc_mma_f16_ta(td + k * NT, ta + k * 16, dk, idesc, 0);
+                                    ps_tc_mma_f16_ta(td + k * NT, ta + k * 16 + 8, dk + NT * 2, idesc, 1);
                                 }
-                                ps_tc_commit(&bar_d_full[re]);
-                                if (h == T::NH - 1) ps_tc_commit(&bar_a_empty[ra]);
-                                if (h == T::NH - 1 && x == 1) ps_tc_commit(&bar_empty[j]);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < 2 * T::XE; k++) ps_tc_mma_f16_ta(td + k * NT, ta + (k >> 1) * 32, ds + (2 * T::XE * e + k) * (NT * 2), idesc, 0);
                             }
-                            __syncwarp();
+                            ps_tc_commit(&bar_done[re.i]);
+                            if (e == 2 / T::XE - 1) ps_tc_commit(&bar_empty[st.i]);
                         }
-                        if (!ok) break;
-                    }
-                    if (--left == 0) { // next pass, next unit
-                        left = ns;
-                        if (++p == p_end) {
-                            u += gridDim.x;
-                            p = (u % nu) * pp;
-                            p_end = p + pp;
-                        }
+                        __syncwarp();
                     }
                 }
             }
-            if (ps_elect_one()) ps_tc_commit(&bar_done); // MMAs in flight end before the tensor memory is given back
+            if (ps_elect_one()) ps_tc_commit(&bar_end); // MMAs in flight end before the tensor memory is given back
             __syncwarp();
-            if (!ps_tc_wait(&bar_done, 0)) *a.err = 6;
+            if (!ps_tc_wait(&bar_end, 0)) *a.err = 6;
         }
     } else if (warp >= T::EW) {
-        // ===== de-quantising warps: warpgroup d takes super-block d of every step; thread = row (warp % 4 is its tensor-memory lane quadrant)
-        if (T::SPLIT) ps_reg_dec<48>();
-        const int d = (warp - T::EW) >> 2, quad = warp & 3, row = quad * 32 + lane;
-        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + T::TM_A;
+        // ===== de-quantising warps: a warpgroup takes super-block d of a step, of every second step where there are four; thread = row (warp % 4 is its
+        // tensor-memory lane quadrant)
+        ps_reg_dec<T::R_DEQ>();
+        const int group = (warp - T::EW) >> 2, d = group & 1, quad = warp & 3, row = quad * 32 + lane;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + T::TM_A + (T::XE == 2 ? d * 32 : 0);
         PsRing<T::NS> st;
-        PsRing<T::NA> ra;
-        if (d) ra.step();
-        int g = 0;
+        PsRing<T::NE> re;
+        constexpr int EN = 2 / T::XE; // entries of a step
+        if (T::XE == 1 && d) re.step();
         bool ok = warp != a.give_up;
         if (!ok) *a.err = 7;
-        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
-            const int p0 = (u % nu) * pp;
-            for (int p = p0; p < p0 + pp && ok; p++) {
-                for (int i = 0; i < ns; i++, g++) {
-                    const bool fa = (lane & 1) && 2 * g + d >= T::NA; // odd lanes wait for the A buffer
-                    if (!ps_tc_wait_all(ps_smem_u32(fa ? &bar_a_empty[ra.i] : &bar_full[st.i]), fa ? ra.round ^ 1 : st.round, a.limit)) { *a.err = 7; ok = false; break; }
-                    ps_tc_fence_after();
-                    const uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE;
-                    const uint32_t td = t_lane + ra.i * 32;
-                    if (p < 4) {
-                        sm += d * PS_TC_A_Q;
-                        const uint4 q0 = *reinterpret_cast<const uint4 *>(sm + row * 16), q1 = *reinterpret_cast<const uint4 *>(sm + 2048 + row * 16);
-                        const uint4 sc = *reinterpret_cast<const uint4 *>(sm + T::STAGE_SC - d * (PS_TC_A_Q - PS_TC_A_SC) + row * 16);
-                        __syncwarp();
-                        if (lane == 0) ps_mbar_arrive(&bar_empty[st.i]);
-#pragma unroll
-                        for (int k = 0; k < 2; k++) { // words 2k, 2k + 1 of both lanes
-                            uint32_t s2[4], o2[4], v[8];
-                            const uint32_t s0 = k ? sc.z : sc.x, s1 = k ? sc.w : sc.y;
-#pragma unroll
-                            for (int j = 0; j < 4; j++) {
-                                s2[j] = __byte_perm(j < 2 ? s0 : s1, 0, (j & 1) ? 0x3232 : 0x1010);
-                                o2[j] = ps_h2_mul(s2[j], 0xE400E400u); // x -1024
-                            }
-                            ps_tc_dequant8(k ? q0.z : q0.x, k ? q0.w : q0.y, s2, o2, v);
-                            ps_tc_st8(td + 8 * k, v);
-                            ps_tc_dequant8(k ? q1.z : q1.x, k ? q1.w : q1.y, s2, o2, v);
-                            ps_tc_st8(td + 16 + 8 * k, v);
-                        }
-                    } else { // K positions 4k + u hold m_(2k + u / 2): column 2k + u / 2 is that minimum twice
-                        const uint2 mn = *reinterpret_cast<const uint2 *>(sm + d * PS_TC_A_MN + row * 8);
-                        __syncwarp();
-                        if (lane == 0) ps_mbar_arrive(&bar_empty[st.i]);
-                        uint32_t v[8];
-#pragma unroll
-                        for (int j = 0; j < 8; j++) {
-                            const uint32_t w = __byte_perm(j < 4 ? mn.x : mn.y, 0x64646464u, 0x4040 + 0x0101 * (j & 3)); // 1024 + m, twice
-                            v[j] = ps_h2_fma(w, 0x3C003C00u, 0xE400E400u);
-                        }
-                        ps_tc_st8(td, v);
-                    }
-                    ps_tc_st_wait();
-                    ps_tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) ps_mbar_arrive(&bar_a_full[ra.i]);
+        int g = 0, fresh = T::NE - (T::XE == 1 ? d : 0); // entries ahead whose A buffer has not been used
+        for (int q = q0; q < q1 && ok; q++) {
+            const bool lanes = q % PS_TC_PASSES < 4;
+            for (int i = 0; i < ns; i++, g++) {
+                const bool used = fresh <= 0;
+                fresh -= used ? 0 : EN;
+                if (T::ND == 4 && ((g ^ (group >> 1)) & 1)) { // the other two groups' step
                     st.step();
-                    ra.step();
-                    ra.step();
+                    re.step();
+                    continue;
                 }
+                // one wait for two things: even lanes wait for the stage, odd ones for the A buffer
+                const bool fa = (lane & 1) && used;
+                if (!ps_tc_wait_all(ps_smem_u32(fa ? &bar_done[re.i] : &bar_full[st.i]), fa ? re.round ^ 1 : st.round, a.limit)) { *a.err = 7; ok = false; break; }
+                ps_tc_fence_after();
+                const uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE;
+                const uint32_t td = t_lane + re.i * (T::XE * 32);
+                uint32_t v[4][8];
+                if (lanes) {
+                    sm += d * PS_TC_A_Q;
+                    const uint4 w0 = *reinterpret_cast<const uint4 *>(sm + row * 16), w1 = *reinterpret_cast<const uint4 *>(sm + 2048 + row * 16);
+                    const uint4 sc = *reinterpret_cast<const uint4 *>(sm + T::STAGE_SC - d * (PS_TC_A_Q - PS_TC_A_SC) + row * 16);
+#pragma unroll
+                    for (int k = 0; k < 2; k++) { // words 2k, 2k + 1 of both lanes
+                        uint32_t s2[4], o2[4];
+                        const uint32_t s0 = k ? sc.z : sc.x, s1 = k ? sc.w : sc.y;
+#pragma unroll
+                        for (int j = 0; j < 4; j++) {
+                            s2[j] = __byte_perm(j < 2 ? s0 : s1, 0, (j & 1) ? 0x3232 : 0x1010);
+                            o2[j] = ps_h2_mul(s2[j], 0xE400E400u); // x -1024
+                        }
+                        ps_tc_dequant8(k ? w0.z : w0.x, k ? w0.w : w0.y, s2, o2, v[k]);
+                        ps_tc_dequant8(k ? w1.z : w1.x, k ? w1.w : w1.y, s2, o2, v[2 + k]);
+                    }
+                } else { // K positions 4k + u hold m_(2k + u / 2): column 2k + u / 2 is that minimum twice
+                    const uint2 mn = *reinterpret_cast<const uint2 *>(sm + d * PS_TC_A_MN + row * 8);
+#pragma unroll
+                    for (int j = 0; j < 8; j++) {
+                        const uint32_t w = __byte_perm(j < 4 ? mn.x : mn.y, 0x64646464u, 0x4040 + 0x0101 * (j & 3)); // 1024 + m, twice
+                        v[0][j] = ps_h2_fma(w, 0x3C003C00u, 0xE400E400u);
+                    }
+                }
+                ps_tc_st8(td, v[0]);
+                if (lanes) {
+                    ps_tc_st8(td + 8, v[1]);
+                    ps_tc_st8(td + 16, v[2]);
+                    ps_tc_st8(td + 24, v[3]);
+                }
+                ps_tc_st_wait();
+                ps_tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ps_mbar_arrive(&bar_go[re.i]);
+                st.step();
+                for (int k = 0; k < EN; k++) re.step();
             }
         }
     } else {
-        // ===== epilogue: warp w owns tensor-memory lanes 32 * (w % 4) .. +31 (rows) and EC columns of half h
-        if (T::SPLIT) ps_reg_inc<96>();
-        constexpr int WPH = T::EW / T::NH; // warps of a half
-        const int h = warp / WPH, quad = warp & 3, cg = (warp % WPH) >> 2, row = quad * 32 + lane, c0 = h * T::CW + cg * T::EC;
-        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + cg * T::EC;
-        float *stash = reinterpret_cast<float *>(ps_tc_fact + T::NY * T::FACT) + tid; // [EC][epilogue threads]
-        constexpr int ET = T::EW * 32;
+        // ===== epilogue: warp w owns tensor-memory lanes 32 * (w % 4) .. +31 (rows) and EC columns
+        ps_reg_inc<T::R_EPI>();
+        const int quad = warp & 3, row = quad * 32 + lane, c0 = (warp >> 2) * T::EC;
+        const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + c0;
+        constexpr int ET = T::EW * 32, US = T::EC * ET;
+        float *stash = reinterpret_cast<float *>(ps_tc_fact + T::NY * T::FACT) + tid, *whole = stash + US; // [EC][epilogue threads]
         PsRing<T::NY> sy;
         PsRing<T::NE> re;
-        if (h) re.step();
         bool ok = warp != a.give_up;
         if (!ok) *a.err = 4;
-        for (int u = blockIdx.x; u < n_units; u += gridDim.x) {
-            const int tile = u / nu, p0 = (u % nu) * pp;
-            float *part = a.part + ((size_t)tile * nu + u % nu) * (T::EC * ET) + tid;
-            float *whole = a.part + (size_t)blockIdx.x * (T::EC * ET) + tid; // pp = 6: the sum of the pass pairs so far
-            ps_f2 acc[2][T::EC / 2];
-            for (int p = p0; p < p0 + pp && ok; p++) {
+        int pend = -1, pend_slot = 0, old = 0; // the shared tile handed over last, its slot, and (thread 0) how many of its passes were there by then
+        ps_f2 acc[2][T::EC / 2];
+        for (int q = q0; q < q1; q++) {
+            const int tile = q / PS_TC_PASSES, p = q % PS_TC_PASSES;
 #pragma unroll
-                for (int c = 0; c < T::EC / 2; c++) acc[0][c] = acc[1][c] = 0ull;
-                for (int i = 0; i < ns && ok; i++, sy.step()) {
-                    const uint8_t *sf = ps_tc_fact + sy.i * T::FACT;
-#pragma unroll 1
-                    for (int x = 0; x < 2; x++) {
-                        if (!ps_tc_wait_warp(&bar_d_full[re.i], re.round, a.limit)) { *a.err = 4; ok = false; break; } // the factors came with the stage
-                        ps_tc_fence_after();
-                        const float xd = *reinterpret_cast<const float *>(sf + x * PS_TC_A_D + row * 4);
-                        const ps_f2 x2 = ps_f2_pack(xd, xd);
-                        const ulonglong2 *yd = reinterpret_cast<const ulonglong2 *>(sf + 2 * PS_TC_A_D + (x * NT + c0) * 4);
-                        const uint32_t td = t_lane + re.i * (2 * T::CW);
+            for (int c = 0; c < T::EC / 2; c++) acc[0][c] = acc[1][c] = 0ull;
+            for (int i = 0; i < ns && ok; i++, sy.step()) {
+                const uint8_t *sf = ps_tc_fact + sy.i * T::FACT;
+                // one wait a step: entries are complete in order
+                const int e0 = re.i;
+                if (T::XE == 1) re.step();
+                const int e1 = re.i;
+                if (!ps_tc_wait_warp(&bar_done[e1], re.round, a.limit)) { *a.err = 4; ok = false; break; }
+                re.step();
+                ps_tc_fence_after();
+                const uint32_t td[2] = {t_lane + e0 * T::TM_E, t_lane + e1 * T::TM_E + (T::XE == 2 ? 2 * NT : 0)};
 #pragma unroll
-                        for (int c = 0; c < T::EC; c += 8) {
-                            const ulonglong2 y0 = yd[c / 4], y1 = yd[c / 4 + 1];
-                            const ps_f2 dd[4] = {ps_f2_mul(y0.x, x2), ps_f2_mul(y0.y, x2), ps_f2_mul(y1.x, x2), ps_f2_mul(y1.y, x2)};
-                            ps_f2 v[8]; // the exact integers S_l (or P_k)
-                            ps_tc_ld8x2(td + c, td + T::CW + c, v);
-                            if (c + 8 == T::EC) { // the entry is in registers, the factors as well: both can be refilled
-                                ps_tc_fence_before();
-                                __syncwarp();
-                                if (lane == 0) {
-                                    ps_mbar_arrive(&bar_d_empty[re.i]);
-                                    if (x == 1) ps_mbar_arrive(&bar_y_empty[sy.i]);
-                                }
-                            }
+                for (int x = 0; x < 2; x++) {
+                    // (the factors came with the stage, and stay until this warp has drained the entry)
+                    const float xd = *reinterpret_cast<const float *>(sf + x * PS_TC_A_D + row * 4);
+                    const ps_f2 x2 = ps_f2_pack(xd, xd);
 #pragma unroll
-                            for (int k = 0; k < 4; k++) {
-                                acc[0][c / 2 + k] = ps_f2_fma(dd[k], v[k], acc[0][c / 2 + k]);
-                                acc[1][c / 2 + k] = ps_f2_fma(dd[k], v[4 + k], acc[1][c / 2 + k]);
-                            }
+                    for (int c = 0; c < T::EC; c += 8) {
+                        uint32_t v0[8], v1[8];
+                        ps_tc_ld(td[x] + c, v0);
+                        ps_tc_ld(td[x] + NT + c, v1);
+                        const ulonglong2 *yd = reinterpret_cast<const ulonglong2 *>(sf + 2 * PS_TC_A_D + (x * NT + c0 + c) * 4);
+                        const ulonglong2 y0 = yd[0], y1 = yd[1];
+                        const ps_f2 dd[4] = {ps_f2_mul(y0.x, x2), ps_f2_mul(y0.y, x2), ps_f2_mul(y1.x, x2), ps_f2_mul(y1.y, x2)};
+                        ps_tc_ld_wait();
+                        ps_tc_pass(v0);
+                        ps_tc_pass(v1);
+                        if ((x == 1 || T::XE == 1) && c + 8 == T::EC) { // the entry is in registers
+                            ps_tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) ps_mbar_arrive(&bar_go[x ? e1 : e0]);
                         }
-                        re.step();
-                        if (T::NH == 2) re.step();
-                    }
-                }
-                if (!ok) break;
-                // ---- the pass's number: first step of hsum_float_8 (lane l + 4 and lane l), or of the mins sum (m_k and m_k+2)
 #pragma unroll
-                for (int c = 0; c < T::EC / 2; c++) {
-                    float r0, r1;
-                    ps_f2_unpack(ps_f2_add(acc[1][c], acc[0][c]), r0, r1);
-                    if (p & 1) {
-                        if (pp > 1) { r0 = __fadd_rn(stash[(2 * c) * ET], r0); r1 = __fadd_rn(stash[(2 * c + 1) * ET], r1); }
-                        if (pp == PS_TC_PASSES) { // the running sum ((r04 + r26) + (r15 + r37)), then + (m02 + m13)
-                            if (p > 1) { r0 = __fadd_rn(whole[(2 * c) * ET], r0); r1 = __fadd_rn(whole[(2 * c + 1) * ET], r1); }
-                            if (p < 5) { whole[(2 * c) * ET] = r0; whole[(2 * c + 1) * ET] = r1; }
+                        for (int k = 0; k < 4; k++) {
+                            acc[0][c / 2 + k] = ps_f2_fma(dd[k], ps_f2_bits(v0[2 * k], v0[2 * k + 1]), acc[0][c / 2 + k]);
+                            acc[1][c / 2 + k] = ps_f2_fma(dd[k], ps_f2_bits(v1[2 * k], v1[2 * k + 1]), acc[1][c / 2 + k]);
                         }
-                    } else if (pp > 1) {
-                        stash[(2 * c) * ET] = r0;
-                        stash[(2 * c + 1) * ET] = r1;
                     }
-                    acc[0][c] = ps_f2_pack(r0, r1);
                 }
             }
-            if (nu == 1 && !ok) break;
-            if (nu > 1) { // hand the numbers over; the tile's last unit adds them in the fixed order
+            // ---- the pass's number: first step of hsum_float_8 (lane l + 4 and lane l), or of the mins sum (m_k and m_k+2); then
+            // ((r04 + r26) + (r15 + r37)) + (m02 + m13)
+            const bool alone = q - p >= q0 && q - p + PS_TC_PASSES <= q1; // a tile of this CTA alone; of any other, pairs or single numbers are written down
+            const bool end = p == PS_TC_PASSES - 1 || q + 1 == q1;       // the CTA's part of the tile ends
+            const int slot = alone ? 0 : ps_tc_owner(q - p, gridDim.x, a.n_tiles);
+            float *part = a.part + ((size_t)slot * PS_TC_PASSES + p) * US + tid;
+            // (loops without branches inside: the code is met once a pass, and every line of it is fetched anew)
+            auto each = [&](auto f) {
 #pragma unroll
                 for (int c = 0; c < T::EC / 2; c++) {
                     float r0, r1;
                     ps_f2_unpack(acc[0][c], r0, r1);
-                    __stcg(part + (2 * c) * ET, r0);
-                    __stcg(part + (2 * c + 1) * ET, r1);
+                    f(2 * c * ET, r0);
+                    f((2 * c + 1) * ET, r1);
+                    acc[0][c] = ps_f2_pack(r0, r1);
                 }
-                // one thread fences for all (fences are cumulative over the barrier): 512 of them, each waiting for its own stores, cost more
-                // than the stores.  A warp that gave up comes here too, and all of them leave: no warp waits at a barrier that another has passed by
-                if (!ps_bar_all(1, ET, ok)) break;
-                if (tid == 0) {
-                    __threadfence();
-                    const int last = atomicAdd(a.cnt + tile, 1) == nu - 1;
-                    if (last) a.cnt[tile] = 0;
-                    sh_last = last;
-                    __threadfence();
-                }
-                ps_bar_sync(1, ET);
-                if (!sh_last) continue;
-                const float *q = a.part + (size_t)tile * nu * (T::EC * ET) + tid;
-                constexpr int US = T::EC * ET;
+            };
 #pragma unroll
-                for (int cb = 0; cb < T::EC; cb += 8) { // the loads of eight columns together
-                    float r[8];
-                    if (nu == 3) {
-                        float x[3][8];
-#pragma unroll
-                        for (int w = 0; w < 3; w++)
-#pragma unroll
-                            for (int k = 0; k < 8; k++) x[w][k] = __ldcg(q + w * US + (cb + k) * ET);
-#pragma unroll
-                        for (int k = 0; k < 8; k++) r[k] = __fadd_rn(__fadd_rn(x[0][k], x[1][k]), x[2][k]);
-                    } else {
-                        float x[6][8];
-#pragma unroll
-                        for (int w = 0; w < 6; w++)
-#pragma unroll
-                            for (int k = 0; k < 8; k++) x[w][k] = __ldcg(q + w * US + (cb + k) * ET);
-#pragma unroll
-                        for (int k = 0; k < 8; k++)
-                            r[k] = __fadd_rn(__fadd_rn(__fadd_rn(x[0][k], x[1][k]), __fadd_rn(x[2][k], x[3][k])), __fadd_rn(x[4][k], x[5][k]));
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++) acc[0][cb / 2 + k] = ps_f2_pack(r[2 * k], r[2 * k + 1]);
-                }
+            for (int c = 0; c < T::EC / 2; c++) acc[0][c] = ps_f2_add(acc[1][c], acc[0][c]);
+            if (!(p & 1)) each([&](int o, float &r) { stash[o] = r; });
+            else if (q > q0) each([&](int o, float &r) { r = __fadd_rn(stash[o], r); });
+            if (!alone) {
+                if ((p & 1) || end) each([&](int o, float &r) { __stcg(part + o, r); });
+            } else if (p & 1) {
+                if (p > 1) each([&](int o, float &r) { r = __fadd_rn(whole[o], r); });
+                if (!end) each([&](int o, float &r) { whole[o] = r; });
             }
-            // ---- bias / residual, dst[col][row]
-            const int rt = tile / a.n_ct, ct = tile % a.n_ct, grow = rt * PS_TC_M + row;
-            int sg = 0;
-            if (a.n_seg > 1 && grow >= a.seg[1].row_begin) sg = 1;
-            if (a.n_seg > 2 && grow >= a.seg[2].row_begin) sg = 2;
-            if (grow < a.seg[sg].row_end) {
+            if (!end) continue;
+            // ---- the CTA's part of the tile ends: a tile of its own is stored.  Of a shared one, thread 0 tells for all (its release is cumulative
+            // over the barrier) and learns at the CTA's next part, or at its end, when the answer has long come, whether its part was the tile's
+            // last; if so the CTA adds the tile's numbers
+            bool met = true;
+#pragma unroll 1
+            for (int r = alone ? 0 : 1; r < 3; r++) {
+                int t = tile;
+                if (r == 0) {
+                    r = 1; // nothing to tell
+                    if (!ok) continue;
+                } else {
+                    if (r == 2 && (q + 1 < q1 || pend < 0)) break;
+                    // a warp that gave up comes here too, and all of them leave: no warp waits at a barrier that another has passed by
+                    met = false;
+                    if (!ps_bar_all(1, ET, ok)) break;
+                    met = true;
+                    if (tid == 0) {
+                        const int last = pend >= 0 && old == PS_TC_PASSES;
+                        if (last) a.cnt[pend_slot] = 0;
+                        sh_last = last;
+                    }
+                    ps_bar_sync(1, ET);
+                    const bool last = sh_last;
+                    t = pend;
+                    const float *w = a.part + (size_t)pend_slot * PS_TC_PASSES * US + tid;
+                    pend = r == 2 ? -1 : tile;
+                    pend_slot = slot;
+                    if (r == 1 && tid == 0) {
+                        const int n = q + 1 - max(q0, q - p);
+                        old = ps_add_acq_rel(a.cnt + slot, n) + n;
+                    }
+                    if (!last) continue;
+                    const int b = t * PS_TC_PASSES;
+                    const bool cut[3] = {ps_tc_cut(b + 1, gridDim.x, a.n_tiles), ps_tc_cut(b + 3, gridDim.x, a.n_tiles), ps_tc_cut(b + 5, gridDim.x, a.n_tiles)};
+#pragma unroll
+                    for (int cb = 0; cb < T::EC; cb += 8) { // the loads of eight columns together
+                        float y[3][8], z[3][8];
+#pragma unroll
+                        for (int j = 0; j < 3; j++)
+#pragma unroll
+                            for (int k = 0; k < 8; k++) y[j][k] = __ldcg(w + (2 * j + 1) * US + (cb + k) * ET);
+#pragma unroll
+                        for (int j = 0; j < 3; j++)
+                            if (cut[j])
+#pragma unroll
+                                for (int k = 0; k < 8; k++) z[j][k] = __ldcg(w + 2 * j * US + (cb + k) * ET);
+#pragma unroll
+                        for (int j = 0; j < 3; j++)
+                            if (cut[j])
+#pragma unroll
+                                for (int k = 0; k < 8; k++) y[j][k] = __fadd_rn(z[j][k], y[j][k]);
+#pragma unroll
+                        for (int k = 0; k < 8; k += 2)
+                            acc[0][(cb + k) / 2] = ps_f2_pack(__fadd_rn(__fadd_rn(y[0][k], y[1][k]), y[2][k]), __fadd_rn(__fadd_rn(y[0][k + 1], y[1][k + 1]), y[2][k + 1]));
+                    }
+                }
+                // bias / residual, dst[col][row]
+                const int rt = t / a.n_ct, ct = t % a.n_ct, grow = rt * PS_TC_M + row;
+                int sg = 0;
+                if (a.n_seg > 1 && grow >= a.seg[1].row_begin) sg = 1;
+                if (a.n_seg > 2 && grow >= a.seg[2].row_begin) sg = 2;
+                const int n_col = grow < a.seg[sg].row_end ? a.bs - (ct * NT + c0) : 0; // columns of this thread that exist
                 const int n = grow - a.seg[sg].row_begin, ld = a.seg[sg].row_end - a.seg[sg].row_begin;
-                const float bias = a.seg[sg].bias ? a.seg[sg].bias[n] : 0.f;
+                const size_t o0 = (size_t)(ct * NT + c0) * ld + n;
+                auto columns = [&](auto f) {
+                    size_t o = o0;
 #pragma unroll
-                for (int c = 0; c < T::EC / 2; c++) {
-                    float r[2];
-                    ps_f2_unpack(acc[0][c], r[0], r[1]);
-#pragma unroll
-                    for (int k = 0; k < 2; k++) {
-                        const int col = ct * NT + c0 + 2 * c + k;
-                        if (col < a.bs) {
-                            const size_t o = (size_t)col * ld + n;
-                            float res = r[k];
-                            if (a.seg[sg].bias) res = __fadd_rn(res, bias);
-                            if (a.residual) res = __fadd_rn(a.residual[o], res);
-                            a.seg[sg].dst[o] = res;
-                        }
+                    for (int c = 0; c < T::EC / 2; c++) {
+                        float r0, r1;
+                        ps_f2_unpack(acc[0][c], r0, r1);
+                        if (2 * c < n_col) f(o, r0);
+                        if (2 * c + 1 < n_col) f(o + ld, r1);
+                        acc[0][c] = ps_f2_pack(r0, r1);
+                        o += 2 * (size_t)ld;
                     }
+                };
+                if (a.seg[sg].bias) {
+                    const float bias = n_col > 0 ? a.seg[sg].bias[n] : 0.f;
+                    columns([&](size_t, float &v) { v = __fadd_rn(v, bias); });
                 }
+                if (a.residual) columns([&](size_t o, float &v) { v = __fadd_rn(a.residual[o], v); });
+                float *dst = a.seg[sg].dst;
+                columns([&](size_t o, float &v) { dst[o] = v; });
             }
+            if (!met) break;
         }
+        ps_tc_ld_wait();
     }
     ps_tc_fence_before();
     __syncthreads();
