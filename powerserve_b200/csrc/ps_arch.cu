@@ -1141,12 +1141,37 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
 }
 
 // fp32-FMA products: 64 x 64 tiles, or 32 x 64 ones where 64-row tiles would leave SMs without a tile (150 tokens x 1024 outputs, K 1024 and
-// 2048 in turn: 48 tiles of 64 rows 104 us, 80 of 32 rows 81 us; with more tiles than SMs the wider tile reads its operands less often)
-static bool pa_narrow_tiles(int n_sm, int N, int bs, int heads) { return (int64_t)((N + PA_TN - 1) / PA_TN) * ((bs + PA_TM - 1) / PA_TM) * heads < n_sm; }
-template <bool ROUND, typename... Args> static void pa_launch_linear(int n_sm, int N, int bs, int heads, cudaStream_t st, Args... args) {
+// 2048 in turn: 48 tiles of 64 rows 104 us, 80 of 32 rows 81 us; with more tiles than SMs the wider tile reads its operands less often).
+// K is cut where the rows of the weights alone give few tiles: by the weights' shape only, so that a token's sums do not depend on its batch.  One tile of
+// tokens then makes up to four CTAs an SM (2 layers of 1024 / 1536 / 2048 wide models on 48 tokens: uncut 737 / 1061 / 1339 us, one CTA an SM 418 / 644 /
+// 943, two 392 / 544 / 740, four 393 / 510 / 653); a cut keeps 128 k or more, since the sums travel through the cluster's shared memory (about 2 us)
+static int pa_cuts(int64_t N, int K) {
+    int S = 1;
+    while (S < 8 && 2 * S * N <= 4 * 148 * PA_TN && K >= 2 * S * 128) S *= 2;
+    return S;
+}
+static bool pa_narrow_tiles(int n_sm, int64_t N, int bs) { return ((N + PA_TN - 1) / PA_TN) * ((bs + PA_TM - 1) / PA_TM) < n_sm; }
+template <typename... KArgs, typename... Args>
+static cudaError_t pa_launch_cut(int S, void (*kern)(KArgs...), dim3 grid, cudaStream_t st, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = grid; cfg.blockDim = dim3(256); cfg.stream = st;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = (unsigned)S;
+    cfg.attrs = at;
+    cfg.numAttrs = S > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, (KArgs)args...);
+}
+template <bool ROUND>
+static void pa_launch_linear(int n_sm, int N, int bs, int heads, cudaStream_t st, const float *A, int lda, const bf16 *W, const float *bias, float *C, int ldc, int M, int n, int K,
+                             int a_gs = 0, int c_gs = 0, int act_from = 1 << 30, int gap = 0, PaAct act = PaAct{}, PaRowMul mul = PaRowMul{}) {
     const unsigned nt = (unsigned)((N + PA_TN - 1) / PA_TN);
-    if (pa_narrow_tiles(n_sm, N, bs, heads)) pa_k_linear<ROUND, 32><<<dim3(nt, (unsigned)((bs + 31) / 32), (unsigned)heads), 256, 0, st>>>(args...);
-    else pa_k_linear<ROUND><<<dim3(nt, (unsigned)((bs + PA_TM - 1) / PA_TM), (unsigned)heads), 256, 0, st>>>(args...);
+    const int S = pa_cuts((int64_t)nt * PA_TN * heads, K);
+    const bool narrow = pa_narrow_tiles(n_sm, (int64_t)nt * PA_TN * heads * S, bs);
+    const int tm = narrow ? 32 : PA_TM;
+    pa_launch_cut(S, narrow ? pa_k_linear<ROUND, 32> : pa_k_linear<ROUND, PA_TM>, dim3(nt, (unsigned)((bs + tm - 1) / tm), (unsigned)(heads * S)), st, A, lda, W, bias, C, ldc, M, n, K, S,
+                  a_gs, c_gs, act_from, gap, act, mul);
 }
 
 template <bool ROUND>
@@ -1312,16 +1337,27 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         }
         return 0;
     };
+    // its first half on the fp32-FMA tiles
+    auto dense_up = [&](const float *X, const bf16 *wg, const bf16 *wu, int ff, const PaAct &act) -> int {
+        const int64_t rows = (int64_t)cdiv(ff, PA_TN) * PA_TN * (wg ? 2 : 1); // (a gated tile has two products)
+        const int S = pa_cuts(rows, dim);
+        const bool narrow = pa_narrow_tiles(a->n_sm, rows * S / (wg ? 2 : 1), bs);
+        const dim3 grid(cdiv(ff, PA_TN), cdiv(bs, narrow ? 32 : PA_TM), (unsigned)S);
+        if (wg) pa_launch_cut(S, narrow ? pa_k_dense_up<ROUND, 2, 32> : pa_k_dense_up<ROUND, 2, PA_TM>, grid, st, X, dim, wg, wu, a->y, bs, ff, dim, act, S);
+        else pa_launch_cut(S, narrow ? pa_k_dense_up<ROUND, 1, 32> : pa_k_dense_up<ROUND, 1, PA_TM>, grid, st, X, dim, (const bf16 *)nullptr, wu, a->y, bs, ff, dim, act, S);
+        PA_LAUNCH();
+        return 0;
+    };
     // the dense feed-forward of a batch: gate | up (or up alone) with the activation in the product's epilogue, then down
     auto dense_batch = [&](const float *X, const bf16 *wg, const bf16 *wu, const bf16 *wd, const uint8_t *tg, const uint8_t *tu, const uint8_t *td, int ff, const PaAct &act,
                            float *out) -> int {
+        int rc_up;
         if (!wg) { // no gate
             if (tc) {
                 int rc = tc_dense(X, dim, bs, dim, tu, ff, nullptr, a->y, ff, &act);
                 if (rc) return rc;
             } else {
-                pa_k_dense_up1<ROUND><<<dim3(cdiv(ff, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(X, dim, wu, a->y, bs, ff, dim, act);
-                PA_LAUNCH();
+                if ((rc_up = dense_up(X, nullptr, wu, ff, act))) return rc_up;
             }
             return linear(a->y, ff, ff, wd, td, dim, out, dim);
         }
@@ -1335,7 +1371,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             const int ctas = cut_tiles(g);
             pa_k_tc_gemm<2><<<ctas, PT_THREADS, PT_SMEM, st>>>(g);
         } else {
-            pa_k_dense_up<ROUND><<<dim3(cdiv(ff, PA_TN), cdiv(bs, PA_TM)), blk, 0, st>>>(X, dim, wg, wu, a->y, bs, ff, dim, act);
+            if ((rc_up = dense_up(X, wg, wu, ff, act))) return rc_up;
         }
         PA_LAUNCH();
         return linear(a->y, ff, ff, wd, td, dim, out, dim);

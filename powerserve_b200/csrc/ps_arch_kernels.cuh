@@ -7,7 +7,7 @@
 // the latent attention's norms and rotations (half-split or neighbouring pairs).  Pooled windows: pa_k_pool_blocks forms the mean key /
 // value of every block of positions that a batch completes; the scores / soft-max / P.V kernels take the blocks as further keys behind
 // the tokens.  Rotated heads: pa_k_embed forms the angles of a forward pass, pa_k_qkv_post rotates q / k / values, pa_k_pv turns the heads'
-// outputs back.  pa_k_dense_up1 is the first half of a feed-forward without a gate.
+// outputs back.
 // The single-token kernels (bs == 1) live in ps_arch_decode.cuh.
 #pragma once
 
@@ -178,6 +178,9 @@ __device__ __forceinline__ void pa_fetch8(const bf16 *row, bool vec, int k, int 
         for (int c = 0; c < 8; c++) v[c] = (row && k + c < K) ? pa_ld(row + k + c) : 0.f;
     }
 }
+// A thread stages AV consecutive k of a row, one word each: without the swizzle four threads of a warp met in a bank at every store (a quarter
+// of the shared memory's time).  Rows move by multiples of AV with every AV k, so the 16-byte reads stay whole
+template <int AV> __device__ __forceinline__ int pa_swz(int k) { return AV == 8 ? ((k >> 3) & 3) << 3 : ((k >> 2) & 7) << 2; }
 template <bool ROUND, typename BT, int NB, int TM = PA_TM>
 __device__ __forceinline__ void pa_tile_mm(float (&acc)[NB][TM / 16][4], const float *arow, float ascale, const BT *brow0, const BT *brow1, int K, float (*As)[PA_LD],
                                            float (*Bs)[PA_TK][PA_LD]) {
@@ -193,31 +196,31 @@ __device__ __forceinline__ void pa_tile_mm(float (&acc)[NB][TM / 16][4], const f
     fetch(0);
     for (int k0 = 0; k0 < K; k0 += PA_TK) {
 #pragma unroll
-        for (int c = 0; c < AV; c++) As[ka + c][la] = pa_rnd<ROUND>(ra[c] * ascale);
+        for (int c = 0; c < AV; c++) As[ka + c][la ^ pa_swz<AV>(ka)] = pa_rnd<ROUND>(ra[c] * ascale);
 #pragma unroll
         for (int c = 0; c < 8; c++) {
-            Bs[0][kq + c][lr] = rb[0][c];
-            if (NB == 2) Bs[NB - 1][kq + c][lr] = rb[NB - 1][c];
+            Bs[0][kq + c][lr ^ pa_swz<8>(kq)] = rb[0][c];
+            if (NB == 2) Bs[NB - 1][kq + c][lr ^ pa_swz<8>(kq)] = rb[NB - 1][c];
         }
         __syncthreads();
         if (k0 + PA_TK < K) fetch(k0 + PA_TK);
         float av[2][TY], bv[2][NB][4]; // the next k's operands are read while this one is computed
         auto frag = [&](int k, int w) {
             if (TY == 4) {
-                const float4 a4 = *reinterpret_cast<const float4 *>(&As[k][ty * TY]);
+                const float4 a4 = *reinterpret_cast<const float4 *>(&As[k][(ty * TY) ^ pa_swz<AV>(k)]);
                 av[w][0] = a4.x; av[w][1] = a4.y; av[w][TY - 2] = a4.z; av[w][TY - 1] = a4.w;
             } else {
-                const float2 a2 = *reinterpret_cast<const float2 *>(&As[k][ty * TY]);
+                const float2 a2 = *reinterpret_cast<const float2 *>(&As[k][(ty * TY) ^ pa_swz<AV>(k)]);
                 av[w][0] = a2.x; av[w][1] = a2.y;
             }
 #pragma unroll
             for (int nb = 0; nb < NB; nb++) {
-                const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[nb][k][tx * 4]);
+                const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[nb][k][(tx * 4) ^ pa_swz<8>(k)]);
                 bv[w][nb][0] = b4.x; bv[w][nb][1] = b4.y; bv[w][nb][2] = b4.z; bv[w][nb][3] = b4.w;
             }
         };
         frag(0, 0);
-#pragma unroll 8
+#pragma unroll
         for (int k = 0; k < PA_TK; k++) {
             const int w = k & 1;
             if (k + 1 < PA_TK) frag(k + 1, w ^ 1);
@@ -235,6 +238,70 @@ __device__ __forceinline__ void pa_tile_mm(float (&acc)[NB][TM / 16][4], const f
 #define PA_TILE_SMEM(NB)                          \
     __shared__ __align__(16) float As[PA_TK][PA_LD]; \
     __shared__ __align__(16) float Bs[NB][PA_TK][PA_LD]
+
+// A tile whose K is cut over the CTAs of a cluster (ranks along z).  A product of few tiles leaves SMs empty or with two warps a scheduler, which
+// wait for operands most of the time; the cuts fill them.  Every rank leaves its sums in shared memory, then rank r adds rows r * TM / S ..
+// of all ranks, in rank order, so that the result does not depend on the cluster's timing, and `store` gets four columns of a row at a time.
+// 150 tokens x 1024 outputs: K 1024 and 2048 81 us on average uncut, 27 in eight cuts; 2048 gate and up rows, K 1024: 97 and 66 us
+__device__ __forceinline__ uint32_t pa_cluster_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
+__device__ __forceinline__ void pa_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory"); // release / acquire
+}
+__device__ __forceinline__ float4 pa_cluster_ld(const float *p, int rank) {
+    uint32_t at;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
+    return v;
+}
+// shared memory of such a tile: the operands' stages, then the sums
+template <int NB, int TM> struct PaTileMem {
+    static constexpr int N = (1 + NB) * PA_TK * PA_LD > NB * TM * PA_TN ? (1 + NB) * PA_TK * PA_LD : NB * TM * PA_TN;
+};
+// k-range of a rank: whole steps of the tile core
+__device__ __forceinline__ int pa_cut_begin(int K, int rank, int S) { return min(K, (K + S * PA_TK - 1) / (S * PA_TK) * PA_TK * rank); }
+
+template <bool ROUND, int NB, int TM, typename F>
+__device__ __forceinline__ void pa_tile_cut(float *sm, const float *arow, const bf16 *brow0, const bf16 *brow1, int K, int S, F store) {
+    constexpr int TY = TM / 16;
+    float(*As)[PA_LD] = reinterpret_cast<float(*)[PA_LD]>(sm);
+    float(*Bs)[PA_TK][PA_LD] = reinterpret_cast<float(*)[PA_TK][PA_LD]>(sm + PA_TK * PA_LD);
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, rank = S > 1 ? (int)pa_cluster_rank() : 0;
+    const int k0 = pa_cut_begin(K, rank, S), k1 = pa_cut_begin(K, rank + 1, S);
+    float acc[NB][TY][4] = {};
+    if (k0 < k1) pa_tile_mm<ROUND, bf16, NB, TM>(acc, arow ? arow + k0 : nullptr, 1.0f, brow0 ? brow0 + k0 : nullptr, brow1 ? brow1 + k0 : nullptr, k1 - k0, As, Bs);
+    if (S == 1) {
+#pragma unroll
+        for (int i = 0; i < TY; i++) {
+            float4 v[NB];
+#pragma unroll
+            for (int nb = 0; nb < NB; nb++) v[nb] = make_float4(acc[nb][i][0], acc[nb][i][1], acc[nb][i][2], acc[nb][i][3]);
+            store(ty * TY + i, tx * 4, v);
+        }
+        return;
+    }
+#pragma unroll
+    for (int nb = 0; nb < NB; nb++)
+#pragma unroll
+        for (int i = 0; i < TY; i++)
+            *reinterpret_cast<float4 *>(sm + (nb * TM + ty * TY + i) * PA_TN + tx * 4) = make_float4(acc[nb][i][0], acc[nb][i][1], acc[nb][i][2], acc[nb][i][3]);
+    pa_cluster_sync();
+    for (int e = tid; e < TM / S * 16; e += 256) {
+        const int row = TM / S * rank + (e >> 4), col = (e & 15) * 4;
+        float4 v[NB];
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++) {
+            const float *at = sm + (nb * TM + row) * PA_TN + col;
+            v[nb] = pa_cluster_ld(at, 0);
+            for (int r = 1; r < S; r++) {
+                const float4 u = pa_cluster_ld(at, r);
+                v[nb].x += u.x; v[nb].y += u.y; v[nb].z += u.z; v[nb].w += u.w;
+            }
+        }
+        store(row, col, v);
+    }
+    pa_cluster_sync(); // nobody leaves while its sums are read
+}
 
 // ---------------------------------------------------------------------------------------------------------------- small ops
 // keep (null or [tokens] rows of stride ld_keep) receives the same rows once more: the embedding output that later passes of a looped model add back
@@ -505,38 +572,34 @@ __global__ void __launch_bounds__(256) pa_k_rope_q(const float *__restrict__ q, 
 }
 
 // ---------------------------------------------------------------------------------------------------------------- dense
-// C[m][n] = sum_k A[m][k] W[n][k] + bias[n].  blockIdx.z walks groups (per-head products): group z reads the columns of A from
+// C[m][n] = sum_k A[m][k] W[n][k] + bias[n].  blockIdx.z walks groups (per-head products) of S cuts of K: group z reads the columns of A from
 // z * a_gs on, the matrix z of N x K weights, and writes the columns of C from z * c_gs on.  Rows n >= act_from leave through the
 // one-argument activation, `gap` columns further on; mul multiplies the outputs by a table row per token.
 template <bool ROUND, int TM = PA_TM>
 __global__ void __launch_bounds__(256) pa_k_linear(const float *__restrict__ A, int lda, const bf16 *__restrict__ W, const float *__restrict__ bias, float *__restrict__ C, int ldc,
-                                                   int M, int N, int K, int a_gs = 0, int c_gs = 0, int act_from = 1 << 30, int gap = 0, PaAct act = PaAct{},
-                                                   PaRowMul mul = PaRowMul{}) {
-    PA_TILE_SMEM(1);
-    constexpr int TY = TM / 16;
-    const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM), tx = tid & 15, ty = tid >> 4;
+                                                   int M, int N, int K, int S, int a_gs, int c_gs, int act_from, int gap, PaAct act, PaRowMul mul) {
+    __shared__ __align__(16) float sm[PaTileMem<1, TM>::N];
+    const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM), z = blockIdx.z / S;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * PA_TN;
-    A += (int64_t)blockIdx.z * a_gs;
-    C += (int64_t)blockIdx.z * c_gs;
-    W += (int64_t)blockIdx.z * N * K;
-    float acc[1][TY][4] = {};
+    A += (int64_t)z * a_gs;
+    C += (int64_t)z * c_gs;
+    W += (int64_t)z * N * K;
     const float *arow = (m0 + la < M) ? A + (int64_t)(m0 + la) * lda : nullptr;
     const bf16 *brow = (n0 + lr < N) ? W + (int64_t)(n0 + lr) * K : nullptr;
-    pa_tile_mm<ROUND, bf16, 1, TM>(acc, arow, 1.0f, brow, nullptr, K, As, Bs);
-#pragma unroll
-    for (int i = 0; i < TY; i++) {
-        const int m = m0 + ty * TY + i;
-        if (m >= M) continue;
+    pa_tile_cut<ROUND, 1, TM>(sm, arow, brow, nullptr, K, S, [&](int row, int col, const float4 (&sum)[1]) {
+        const int m = m0 + row;
+        if (m >= M) return;
+        const float s4[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
+            const int n = n0 + col + j;
             if (n >= N) continue;
-            float v = acc[0][i][j] + (bias ? bias[n] : 0.f);
+            float v = s4[j] + (bias ? bias[n] : 0.f);
             if (n >= act_from) v = pa_act1(v, act);
             if (mul.table) v *= pa_ld(mul.table + (int64_t)mul.tok[m] * mul.ld + n);
             C[(int64_t)m * ldc + (n < act_from ? n : n + gap)] = v;
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------------------------------------------- router
@@ -792,48 +855,26 @@ __global__ void __launch_bounds__(256) pa_k_expert_down(const float *__restrict_
     }
 }
 
-// dense gated feed-forward, first half: y[m][n] = act(gate[n] . h_m, up[n] . h_m)
-template <bool ROUND>
+// dense feed-forward, first half: y[m][n] = act(gate[n] . h_m, up[n] . h_m); NB = 1: no gate, act(up[n] . h_m).  blockIdx.z: the S cuts of K
+template <bool ROUND, int NB, int TM = PA_TM>
 __global__ void __launch_bounds__(256) pa_k_dense_up(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff,
-                                                     int dim, PaAct act) {
-    PA_TILE_SMEM(2);
-    const int tid = threadIdx.x, lr = tid >> 2, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * PA_TM, n0 = blockIdx.x * PA_TN;
-    float acc[2][4][4] = {};
-    const float *arow = (m0 + lr < M) ? h + (int64_t)(m0 + lr) * ldh : nullptr;
+                                                     int dim, PaAct act, int S) {
+    __shared__ __align__(16) float sm[PaTileMem<NB, TM>::N];
+    const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM);
+    const int m0 = blockIdx.y * TM, n0 = blockIdx.x * PA_TN;
+    const float *arow = (m0 + la < M) ? h + (int64_t)(m0 + la) * ldh : nullptr;
     const bool nin = n0 + lr < ff;
-    pa_tile_mm<ROUND, bf16, 2>(acc, arow, 1.0f, nin ? Wg + (int64_t)(n0 + lr) * dim : nullptr, nin ? Wu + (int64_t)(n0 + lr) * dim : nullptr, dim, As, Bs);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n < ff) y[(int64_t)m * ff + n] = pa_expert_act(acc[0][i][j], acc[1][i][j], act);
-        }
-    }
-}
-
-// feed-forward without a gate, first half: y[m][n] = act(up[n] . h_m)
-template <bool ROUND>
-__global__ void __launch_bounds__(256) pa_k_dense_up1(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff, int dim, PaAct act) {
-    PA_TILE_SMEM(1);
-    const int tid = threadIdx.x, lr = tid >> 2, tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * PA_TM, n0 = blockIdx.x * PA_TN;
-    float acc[1][4][4] = {};
-    const float *arow = (m0 + lr < M) ? h + (int64_t)(m0 + lr) * ldh : nullptr;
-    pa_tile_mm<ROUND, bf16, 1>(acc, arow, 1.0f, (n0 + lr < ff) ? Wu + (int64_t)(n0 + lr) * dim : nullptr, nullptr, dim, As, Bs);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
+    const bf16 *up = nin ? Wu + (int64_t)(n0 + lr) * dim : nullptr;
+    pa_tile_cut<ROUND, NB, TM>(sm, arow, NB == 2 ? (nin ? Wg + (int64_t)(n0 + lr) * dim : nullptr) : up, up, dim, S, [&](int row, int col, const float4 (&sum)[NB]) {
+        const int m = m0 + row;
+        if (m >= M) return;
+        const float s0[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w}, s1[4] = {sum[NB - 1].x, sum[NB - 1].y, sum[NB - 1].z, sum[NB - 1].w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n < ff) y[(int64_t)m * ff + n] = pa_act1(acc[0][i][j], act);
+            const int n = n0 + col + j;
+            if (n < ff) y[(int64_t)m * ff + n] = NB == 2 ? pa_expert_act(s0[j], s1[j], act) : pa_act1(s0[j], act);
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------------------------------------------- attention
