@@ -1259,7 +1259,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     const float *add_tok = nullptr, *add_vec = nullptr;
     auto seam = [&](float *h_out, const float *w_in, int ldh = 0) -> int {
         if (!pend_y && !h_out && !add_tok && !add_vec) return 0;
-        pa_k_seam_norm<<<bs, 256, 0, st>>>(a->x, pend_y, pend_w, h_out, w_in, dim, groups, d.norm_eps, center, add_tok, add_vec, a->res_scale, ldh > 0 ? ldh : dim);
+        pa_k_seam_norm<<<dim3((unsigned)bs, (unsigned)groups), 256, 0, st>>>(a->x, pend_y, pend_w, h_out, w_in, dim, groups, d.norm_eps, center, add_tok, add_vec, a->res_scale, ldh > 0 ? ldh : dim);
         PA_LAUNCH();
         pend_y = pend_w = add_tok = add_vec = nullptr;
         return 0;
