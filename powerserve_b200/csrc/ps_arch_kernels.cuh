@@ -141,13 +141,16 @@ __device__ __forceinline__ float pa_act1(float z, PaAct act) {
 }
 
 // ---------------------------------------------------------------------------------------------------------------- tile core
-// acc[i][j] += sum_k A(ty * TY + i, k) * B(tx * 4 + j, k) for the CTA's TM x 64 tile (TM = 64 or 32, TY = TM / 16), k ascending.  Every
-// thread stages TM / 8 k-values of ONE A row and 8 of ONE B row per step: `arow` points at row tid / (256 / TM) of the tile, `brow` at row
-// tid >> 2 (null = outside: zeros).
-// Bound by latency where a grid has fewer tiles than there are SMs (two warps a scheduler): four scalar loads per operand used to be waited
-// for at every 16 k.  Now the next step's values travel in registers while this one is computed, 32 k a step, by 16-byte loads where
-// the row allows them, and the next k's operands are read from shared memory one k ahead.  150 tokens x 1024 outputs, K 1024 and 2048 in
-// turn: 130 -> 104 us a product (32-row tiles: 81); P.V of 256 queries x 1024 keys x 16 heads 80 -> 50 us.
+// Sums over k of A(m, k) B(n, k) for the CTA's TM x 64 tile (TM = 64 or 32; NB = 2: two B operands).  A step is 32 k: every thread stages TM / 8 k-values of
+// ONE A row and 8 of ONE B row - `arow` points at row tid / (256 / TM) of the tile, `brow` at row tid >> 2 (null = outside: zeros) - by 16-byte loads
+// where the row allows them, and holds the next step's values in registers while this one is computed.
+// Bound by shared memory: a 16-byte read costs four of its cycles, shared addresses or not, so what counts is how many products a thread makes of
+// one.  The threads are G groups that share the k of a step, each with the whole tile: a thread of four groups owns 8 x 8 outputs (32 rows: 4 x 8) and
+// needs a sixteenth of a read per product, where 4 x 4 outputs over all k need an eighth.  The groups' sums meet at the end.
+// It pays for 32-row tiles and long sums: 8 / 48 / 128 tokens of two 1024-wide Vanapel layers in float32 358 / 363 / 428 us with 4 x 4 outputs
+// everywhere, 327 / 338 / 418 now; P.V of 256 queries x 1024 keys x 16 heads 43 -> 36 us.  At 64 rows and short cuts the meeting costs what the reads
+// save (and 128 registers halve the CTAs an SM holds), so those stay with one group of 4 x 4 outputs.  So do rounded operands, whose products the
+// tensor cores make: their sums stay in the order of k
 __device__ __forceinline__ void pa_fetch8(const float *row, bool vec, int k, int K, float v[8]) {
     if (vec && k + 8 <= K) {
         const float4 x = *reinterpret_cast<const float4 *>(row + k), y = *reinterpret_cast<const float4 *>(row + k + 4);
@@ -181,11 +184,24 @@ __device__ __forceinline__ void pa_fetch8(const bf16 *row, bool vec, int k, int 
 // A thread stages AV consecutive k of a row, one word each: without the swizzle four threads of a warp met in a bank at every store (a quarter
 // of the shared memory's time).  Rows move by multiples of AV with every AV k, so the 16-byte reads stay whole
 template <int AV> __device__ __forceinline__ int pa_swz(int k) { return AV == 8 ? ((k >> 3) & 3) << 3 : ((k >> 2) & 7) << 2; }
-template <bool ROUND, typename BT, int NB, int TM = PA_TM>
-__device__ __forceinline__ void pa_tile_mm(float (&acc)[NB][TM / 16][4], const float *arow, float ascale, const BT *brow0, const BT *brow1, int K, float (*As)[PA_LD],
-                                           float (*Bs)[PA_TK][PA_LD]) {
-    constexpr int TY = TM / 16, AV = TM / 8, AT = 256 / TM; // rows of a thread; k-values of A it stages; threads of an A row
-    const int tid = threadIdx.x, lr = tid >> 2, kq = (tid & 3) * 8, la = tid / AT, ka = (tid % AT) * AV, tx = tid & 15, ty = tid >> 4;
+template <int NB, int TM, bool GROUPS = false> struct PaTile {
+    static constexpr int MY = GROUPS ? TM / 8 : TM / 16, MX = NB == 1 && GROUPS ? 8 : 4; // outputs of a thread
+    static constexpr int TY = TM / MY, TX = PA_TN / MX;      // threads along the rows and the columns
+    static constexpr int G = 256 / (TY * TX), KG = PA_TK / G; // groups, k of a step each
+    static constexpr int N = (1 + NB) * PA_TK * PA_LD > NB * TM * PA_TN ? (1 + NB) * PA_TK * PA_LD : NB * TM * PA_TN; // floats of shared memory: the operands, later the sums
+    typedef float Acc[NB][MY][MX];
+    static __device__ __forceinline__ int ty() { return (threadIdx.x / TX) % TY; }
+    static __device__ __forceinline__ int tx() { return threadIdx.x % TX; }
+    static __device__ __forceinline__ int group() { return threadIdx.x / (TY * TX); }
+};
+template <bool ROUND, typename BT, int NB, int TM, bool GROUPS = false>
+__device__ __forceinline__ void pa_tile_mm(typename PaTile<NB, TM, GROUPS>::Acc &acc, const float *arow, float ascale, const BT *brow0, const BT *brow1, int K, float *sm) {
+    using T = PaTile<NB, TM, GROUPS>;
+    float(*As)[PA_LD] = reinterpret_cast<float(*)[PA_LD]>(sm);
+    float(*Bs)[PA_TK][PA_LD] = reinterpret_cast<float(*)[PA_TK][PA_LD]>(sm + PA_TK * PA_LD);
+    constexpr int AV = TM / 8, AT = 256 / TM; // k-values of A a thread stages; threads of an A row
+    const int tid = threadIdx.x, lr = tid >> 2, kq = (tid & 3) * 8, la = tid / AT, ka = (tid % AT) * AV, kg = T::group() * T::KG;
+    const int ya = (T::ty() * T::MY) ^ pa_swz<AV>(kg), xb = (T::tx() * 4) ^ pa_swz<8>(kg);
     const bool va = arow && ((uintptr_t)arow & 15) == 0, vb0 = brow0 && ((uintptr_t)brow0 & 15) == 0, vb1 = NB == 2 && brow1 && ((uintptr_t)brow1 & 15) == 0;
     float ra[8], rb[NB][8];
     auto fetch = [&](int k0) {
@@ -204,40 +220,71 @@ __device__ __forceinline__ void pa_tile_mm(float (&acc)[NB][TM / 16][4], const f
         }
         __syncthreads();
         if (k0 + PA_TK < K) fetch(k0 + PA_TK);
-        float av[2][TY], bv[2][NB][4]; // the next k's operands are read while this one is computed
-        auto frag = [&](int k, int w) {
-            if (TY == 4) {
-                const float4 a4 = *reinterpret_cast<const float4 *>(&As[k][(ty * TY) ^ pa_swz<AV>(k)]);
-                av[w][0] = a4.x; av[w][1] = a4.y; av[w][TY - 2] = a4.z; av[w][TY - 1] = a4.w;
-            } else {
-                const float2 a2 = *reinterpret_cast<const float2 *>(&As[k][(ty * TY) ^ pa_swz<AV>(k)]);
-                av[w][0] = a2.x; av[w][1] = a2.y;
-            }
 #pragma unroll
-            for (int nb = 0; nb < NB; nb++) {
-                const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[nb][k][(tx * 4) ^ pa_swz<8>(k)]);
-                bv[w][nb][0] = b4.x; bv[w][nb][1] = b4.y; bv[w][nb][2] = b4.z; bv[w][nb][3] = b4.w;
-            }
-        };
-        frag(0, 0);
+        for (int k = 0; k < T::KG; k++) { // (the swizzle of kg + k is that of kg and that of k: KG is a multiple of eight)
+            float av[T::MY], bv[NB][T::MX];
 #pragma unroll
-        for (int k = 0; k < PA_TK; k++) {
-            const int w = k & 1;
-            if (k + 1 < PA_TK) frag(k + 1, w ^ 1);
+            for (int i = 0; i < T::MY; i += 4) {
+                if (T::MY == 2) {
+                    const float2 a2 = *reinterpret_cast<const float2 *>(&As[kg + k][ya ^ pa_swz<AV>(k)]);
+                    av[0] = a2.x; av[1] = a2.y;
+                    break;
+                }
+                const float4 a4 = *reinterpret_cast<const float4 *>(&As[kg + k][(ya ^ pa_swz<AV>(k)) + i]);
+                av[i] = a4.x; av[i + 1] = a4.y; av[(i + 2) % T::MY] = a4.z; av[(i + 3) % T::MY] = a4.w;
+            }
 #pragma unroll
             for (int nb = 0; nb < NB; nb++)
 #pragma unroll
-                for (int i = 0; i < TY; i++)
+                for (int j = 0; j < T::MX; j += 4) {
+                    const float4 b4 = *reinterpret_cast<const float4 *>(&Bs[nb][kg + k][(xb ^ pa_swz<8>(k)) ^ (j * 8)]);
+                    bv[nb][j] = b4.x; bv[nb][j + 1] = b4.y; bv[nb][j + 2] = b4.z; bv[nb][j + 3] = b4.w;
+                }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) acc[nb][i][j] = fmaf(av[w][i], bv[w][nb][j], acc[nb][i][j]);
+            for (int nb = 0; nb < NB; nb++)
+#pragma unroll
+                for (int i = 0; i < T::MY; i++)
+#pragma unroll
+                    for (int j = 0; j < T::MX; j++) acc[nb][i][j] = fmaf(av[i], bv[nb][j], acc[nb][i][j]);
         }
         __syncthreads();
     }
 }
-
-#define PA_TILE_SMEM(NB)                          \
-    __shared__ __align__(16) float As[PA_TK][PA_LD]; \
-    __shared__ __align__(16) float Bs[NB][PA_TK][PA_LD]
+// the groups' sums, added in the groups' order, row by row in shared memory
+template <int NB, int TM, bool GROUPS>
+__device__ __forceinline__ void pa_tile_gather(const typename PaTile<NB, TM, GROUPS>::Acc &acc, float *sm) {
+    using T = PaTile<NB, TM, GROUPS>;
+    const int g = T::group();
+#pragma unroll 1
+    for (int r = 0; r < T::G; r++) {
+        if (g == r)
+#pragma unroll
+            for (int nb = 0; nb < NB; nb++)
+#pragma unroll
+                for (int i = 0; i < T::MY; i++)
+#pragma unroll
+                    for (int j = 0; j < T::MX; j += 4) {
+                        float4 *at = reinterpret_cast<float4 *>(sm + (nb * TM + T::ty() * T::MY + i) * PA_TN + T::tx() * 4 + j * 8);
+                        float4 v = make_float4(acc[nb][i][j], acc[nb][i][j + 1], acc[nb][i][j + 2], acc[nb][i][j + 3]);
+                        if (r) {
+                            const float4 u = *at;
+                            v.x = u.x + v.x; v.y = u.y + v.y; v.z = u.z + v.z; v.w = u.w + v.w;
+                        }
+                        *at = v;
+                    }
+        __syncthreads();
+    }
+}
+// ... and handed to `store` four columns of a row at a time
+template <int NB, int TM, bool GROUPS, typename F> __device__ __forceinline__ void pa_tile_store(const typename PaTile<NB, TM, GROUPS>::Acc &acc, float *sm, F store) {
+    pa_tile_gather<NB, TM, GROUPS>(acc, sm);
+    for (int e = threadIdx.x; e < TM * 16; e += 256) {
+        float4 v[NB];
+#pragma unroll
+        for (int nb = 0; nb < NB; nb++) v[nb] = *reinterpret_cast<const float4 *>(sm + (nb * TM + (e >> 4)) * PA_TN + (e & 15) * 4);
+        store(e >> 4, (e & 15) * 4, v);
+    }
+}
 
 // A tile whose K is cut over the CTAs of a cluster (ranks along z).  A product of few tiles leaves SMs empty or with two warps a scheduler, which
 // wait for operands most of the time; the cuts fill them.  Every rank leaves its sums in shared memory, then rank r adds rows r * TM / S ..
@@ -254,37 +301,18 @@ __device__ __forceinline__ float4 pa_cluster_ld(const float *p, int rank) {
     asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
-// shared memory of such a tile: the operands' stages, then the sums
-template <int NB, int TM> struct PaTileMem {
-    static constexpr int N = (1 + NB) * PA_TK * PA_LD > NB * TM * PA_TN ? (1 + NB) * PA_TK * PA_LD : NB * TM * PA_TN;
-};
 // k-range of a rank: whole steps of the tile core
 __device__ __forceinline__ int pa_cut_begin(int K, int rank, int S) { return min(K, (K + S * PA_TK - 1) / (S * PA_TK) * PA_TK * rank); }
 
 template <bool ROUND, int NB, int TM, typename F>
 __device__ __forceinline__ void pa_tile_cut(float *sm, const float *arow, const bf16 *brow0, const bf16 *brow1, int K, int S, F store) {
-    constexpr int TY = TM / 16;
-    float(*As)[PA_LD] = reinterpret_cast<float(*)[PA_LD]>(sm);
-    float(*Bs)[PA_TK][PA_LD] = reinterpret_cast<float(*)[PA_TK][PA_LD]>(sm + PA_TK * PA_LD);
-    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, rank = S > 1 ? (int)pa_cluster_rank() : 0;
+    const int tid = threadIdx.x, rank = S > 1 ? (int)pa_cluster_rank() : 0;
     const int k0 = pa_cut_begin(K, rank, S), k1 = pa_cut_begin(K, rank + 1, S);
-    float acc[NB][TY][4] = {};
-    if (k0 < k1) pa_tile_mm<ROUND, bf16, NB, TM>(acc, arow ? arow + k0 : nullptr, 1.0f, brow0 ? brow0 + k0 : nullptr, brow1 ? brow1 + k0 : nullptr, k1 - k0, As, Bs);
-    if (S == 1) {
-#pragma unroll
-        for (int i = 0; i < TY; i++) {
-            float4 v[NB];
-#pragma unroll
-            for (int nb = 0; nb < NB; nb++) v[nb] = make_float4(acc[nb][i][0], acc[nb][i][1], acc[nb][i][2], acc[nb][i][3]);
-            store(ty * TY + i, tx * 4, v);
-        }
-        return;
-    }
-#pragma unroll
-    for (int nb = 0; nb < NB; nb++)
-#pragma unroll
-        for (int i = 0; i < TY; i++)
-            *reinterpret_cast<float4 *>(sm + (nb * TM + ty * TY + i) * PA_TN + tx * 4) = make_float4(acc[nb][i][0], acc[nb][i][1], acc[nb][i][2], acc[nb][i][3]);
+    constexpr bool GR = TM == 32 && !ROUND;
+    typename PaTile<NB, TM, GR>::Acc acc = {};
+    if (k0 < k1) pa_tile_mm<ROUND, bf16, NB, TM, GR>(acc, arow ? arow + k0 : nullptr, 1.0f, brow0 ? brow0 + k0 : nullptr, brow1 ? brow1 + k0 : nullptr, k1 - k0, sm);
+    if (S == 1) return pa_tile_store<NB, TM, GR>(acc, sm, store);
+    pa_tile_gather<NB, TM, GR>(acc, sm);
     pa_cluster_sync();
     for (int e = tid; e < TM / S * 16; e += 256) {
         const int row = TM / S * rank + (e >> 4), col = (e & 15) * 4;
@@ -575,9 +603,9 @@ __global__ void __launch_bounds__(256) pa_k_rope_q(const float *__restrict__ q, 
 // z * a_gs on, the matrix z of N x K weights, and writes the columns of C from z * c_gs on.  Rows n >= act_from leave through the
 // one-argument activation, `gap` columns further on; mul multiplies the outputs by a table row per token.
 template <bool ROUND, int TM = PA_TM>
-__global__ void __launch_bounds__(256) pa_k_linear(const float *__restrict__ A, int lda, const bf16 *__restrict__ W, const float *__restrict__ bias, float *__restrict__ C, int ldc,
+__global__ void __launch_bounds__(256, TM == 32 ? 2 : 4) pa_k_linear(const float *__restrict__ A, int lda, const bf16 *__restrict__ W, const float *__restrict__ bias, float *__restrict__ C, int ldc,
                                                    int M, int N, int K, int S, int a_gs, int c_gs, int act_from, int gap, PaAct act, PaRowMul mul) {
-    __shared__ __align__(16) float sm[PaTileMem<1, TM>::N];
+    __shared__ __align__(16) float sm[PaTile<1, TM>::N];
     const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM), z = blockIdx.z / S;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * PA_TN;
     A += (int64_t)z * a_gs;
@@ -799,66 +827,66 @@ __global__ void __launch_bounds__(256) pa_k_dispatch(const int *__restrict__ sel
 
 // y[r][n] = act(gate_e . z_r, up_e . z_r), z_r = w_r * h[token_r] (route_on_input) or h[token_r]; NB = 1: no gate, act(up_e . z_r)
 template <bool ROUND, int NB>
-__global__ void __launch_bounds__(256) pa_k_expert_up(const float *__restrict__ h, int ldh, const int *__restrict__ row_token, const float *__restrict__ row_w,
+__global__ void __launch_bounds__(256, NB == 2 ? 2 : 4) pa_k_expert_up(const float *__restrict__ h, int ldh, const int *__restrict__ row_token, const float *__restrict__ row_w,
                                                       const int *__restrict__ tile_e, const int *__restrict__ tile_row0, const int *__restrict__ tile_end,
                                                       const int *__restrict__ n_tiles, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int ff,
                                                       int dim, int on_input, PaAct act) {
-    PA_TILE_SMEM(NB);
+    __shared__ __align__(16) float sm[PaTile<NB, PA_TM>::N];
     if ((int)blockIdx.y >= *n_tiles) return;
-    const int tid = threadIdx.x, lr = tid >> 2, tx = tid & 15, ty = tid >> 4;
+    const int lr = threadIdx.x >> 2;
     const int e = tile_e[blockIdx.y], r0 = tile_row0[blockIdx.y], rend = tile_end[blockIdx.y], n0 = blockIdx.x * PA_TN;
-    float acc[NB][4][4] = {};
+    typename PaTile<NB, PA_TM>::Acc acc = {};
     const bool rin = r0 + lr < rend;
     const float *arow = rin ? h + (int64_t)row_token[r0 + lr] * ldh : nullptr;
     const float ascale = (rin && on_input) ? row_w[r0 + lr] : 1.0f;
     const int64_t wofs = ((int64_t)e * ff + n0 + lr) * dim;
     const bool nin = n0 + lr < ff;
-    pa_tile_mm<ROUND, bf16, NB>(acc, arow, ascale, nin ? (NB == 2 ? Wg : Wu) + wofs : nullptr, nin ? Wu + wofs : nullptr, dim, As, Bs);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = r0 + ty * 4 + i;
-        if (r >= rend) continue;
+    pa_tile_mm<ROUND, bf16, NB, PA_TM>(acc, arow, ascale, nin ? (NB == 2 ? Wg : Wu) + wofs : nullptr, nin ? Wu + wofs : nullptr, dim, sm);
+    pa_tile_store<NB, PA_TM, false>(acc, sm, [&](int row, int col, const float4 (&sum)[NB]) {
+        const int r = r0 + row;
+        if (r >= rend) return;
+        const float s0[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w}, s1[4] = {sum[NB - 1].x, sum[NB - 1].y, sum[NB - 1].z, sum[NB - 1].w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n < ff) y[(int64_t)r * ff + n] = NB == 2 ? pa_expert_act(acc[0][i][j], acc[NB - 1][i][j], act) : pa_act1(acc[0][i][j], act);
+            const int n = n0 + col + j;
+            if (n < ff) y[(int64_t)r * ff + n] = NB == 2 ? pa_expert_act(s0[j], s1[j], act) : pa_act1(s0[j], act);
         }
-    }
+    });
 }
 
 // slot[token_r][slot_r][n] = down_e . y_r  (times w_r when the score weighs the OUTPUT)
 template <bool ROUND>
-__global__ void __launch_bounds__(256) pa_k_expert_down(const float *__restrict__ y, int ff_ld, const int *__restrict__ row_token, const int *__restrict__ row_slot,
+__global__ void __launch_bounds__(256, 4) pa_k_expert_down(const float *__restrict__ y, int ff_ld, const int *__restrict__ row_token, const int *__restrict__ row_slot,
                                                         const float *__restrict__ row_w, const int *__restrict__ tile_e, const int *__restrict__ tile_row0,
                                                         const int *__restrict__ tile_end, const int *__restrict__ n_tiles, const bf16 *__restrict__ Wd, float *__restrict__ slot,
                                                         int top, int dim, int ff, int on_input) {
-    PA_TILE_SMEM(1);
+    __shared__ __align__(16) float sm[PaTile<1, PA_TM>::N];
     if ((int)blockIdx.y >= *n_tiles) return;
-    const int tid = threadIdx.x, lr = tid >> 2, tx = tid & 15, ty = tid >> 4;
+    const int lr = threadIdx.x >> 2;
     const int e = tile_e[blockIdx.y], r0 = tile_row0[blockIdx.y], rend = tile_end[blockIdx.y], n0 = blockIdx.x * PA_TN;
-    float acc[1][4][4] = {};
+    PaTile<1, PA_TM>::Acc acc = {};
     const float *arow = (r0 + lr < rend) ? y + (int64_t)(r0 + lr) * ff_ld : nullptr;
     const bf16 *brow = (n0 + lr < dim) ? Wd + ((int64_t)e * dim + n0 + lr) * ff : nullptr;
-    pa_tile_mm<ROUND, bf16, 1>(acc, arow, 1.0f, brow, nullptr, ff, As, Bs);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int r = r0 + ty * 4 + i;
-        if (r >= rend) continue;
+    pa_tile_mm<ROUND, bf16, 1, PA_TM>(acc, arow, 1.0f, brow, nullptr, ff, sm);
+    pa_tile_store<1, PA_TM, false>(acc, sm, [&](int row, int col, const float4 (&sum)[1]) {
+        const int r = r0 + row;
+        if (r >= rend) return;
         const float w = on_input ? 1.0f : row_w[r];
         float *dst = slot + ((int64_t)row_token[r] * top + row_slot[r]) * dim;
+        const float s4[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n < dim) dst[n] = acc[0][i][j] * w;
+            const int n = n0 + col + j;
+            if (n < dim) dst[n] = s4[j] * w;
         }
-    }
+    });
 }
 
 // dense feed-forward, first half: y[m][n] = act(gate[n] . h_m, up[n] . h_m); NB = 1: no gate, act(up[n] . h_m).  blockIdx.z: the S cuts of K
 template <bool ROUND, int NB, int TM = PA_TM>
-__global__ void __launch_bounds__(256) pa_k_dense_up(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff,
+__global__ void __launch_bounds__(256, NB == 2 || TM == 32 ? 2 : 4) pa_k_dense_up(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff,
                                                      int dim, PaAct act, int S) {
-    __shared__ __align__(16) float sm[PaTileMem<NB, TM>::N];
+    __shared__ __align__(16) float sm[PaTile<NB, TM>::N];
     const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM);
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * PA_TN;
     const float *arow = (m0 + la < M) ? h + (int64_t)(m0 + la) * ldh : nullptr;
@@ -898,51 +926,49 @@ __device__ __forceinline__ float pa_sink_logit(const PaAttn &at, int h) { return
 
 // S[h][i][j] = score of query i (position pos[i]) and cache row j <= pos[i], before the heads are mixed.  Key tiles from
 // `tok_tiles` on are tiles of pooled blocks: S[h][i][pool_off + b] = score of query i and the mean key of block b.
-__global__ void __launch_bounds__(256) pa_k_scores(PaAttn at, const float *__restrict__ qkv, int ldq, const float *__restrict__ kc, int kd, float *__restrict__ S,
+__global__ void __launch_bounds__(256, 3) pa_k_scores(PaAttn at, const float *__restrict__ qkv, int ldq, const float *__restrict__ kc, int kd, float *__restrict__ S,
                                                    const int32_t *__restrict__ pos, int bs, int key_tile0, int tok_tiles) {
-    PA_TILE_SMEM(1);
-    const int tid = threadIdx.x, lr = tid >> 2, tx = tid & 15, ty = tid >> 4;
+    __shared__ __align__(16) float sm[PaTile<1, PA_TM>::N];
+    const int lr = threadIdx.x >> 2;
     const int h = blockIdx.z, g = h / (at.H / at.G), m0 = blockIdx.y * PA_TM;
     const int pos0 = pos[0], last = pos0 + min(m0 + PA_TM, bs) - 1; // the tile's furthest query
+    PaTile<1, PA_TM>::Acc acc = {};
+    const float *arow = (m0 + lr < bs) ? qkv + (int64_t)(m0 + lr) * ldq + h * at.dq : nullptr;
     if ((int)blockIdx.x >= tok_tiles) {
         const int b0 = ((int)blockIdx.x - tok_tiles) * PA_TN, nv = pa_pool_vis(at, last);
         if (b0 >= nv) return;
-        float acc[1][4][4] = {};
-        const float *arow = (m0 + lr < bs) ? qkv + (int64_t)(m0 + lr) * ldq + h * at.dq : nullptr;
         const float *brow = (b0 + lr < nv) ? kc + (int64_t)(at.n_ctx + b0 + lr) * kd + g * at.dq : nullptr;
-        pa_tile_mm<false, float, 1>(acc, arow, 1.0f, brow, nullptr, at.dq, As, Bs);
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const int m = m0 + ty * 4 + i;
-            if (m >= bs) continue;
+        pa_tile_mm<false, float, 1, PA_TM>(acc, arow, 1.0f, brow, nullptr, at.dq, sm);
+        pa_tile_store<1, PA_TM, false>(acc, sm, [&](int row, int col, const float4 (&sum)[1]) {
+            const int m = m0 + row;
+            if (m >= bs) return;
             const int nvm = pa_pool_vis(at, pos0 + m);
-            float *row = S + ((int64_t)h * at.B + m) * at.ldS + at.pool_off;
+            float *out = S + ((int64_t)h * at.B + m) * at.ldS + at.pool_off;
+            const float s4[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w};
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int b = b0 + tx * 4 + j;
-                if (b < nvm) row[b] = acc[0][i][j] * at.scale * (at.temp ? at.temp[h] : 1.0f);
+                const int b = b0 + col + j;
+                if (b < nvm) out[b] = s4[j] * at.scale * (at.temp ? at.temp[h] : 1.0f);
             }
-        }
+        });
         return;
     }
     const int n0 = (blockIdx.x + key_tile0) * PA_TN;
     if (n0 > last || n0 + PA_TN <= pa_first_key(at, pos0 + m0)) return; // (the tile's first query sees furthest back)
-    float acc[1][4][4] = {};
-    const float *arow = (m0 + lr < bs) ? qkv + (int64_t)(m0 + lr) * ldq + h * at.dq : nullptr;
     const float *brow = (n0 + lr <= last) ? kc + (int64_t)(n0 + lr) * kd + g * at.dq : nullptr;
-    pa_tile_mm<false, float, 1>(acc, arow, 1.0f, brow, nullptr, at.dq, As, Bs);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= bs) continue;
-        const int p = pos0 + m;
-        float *row = S + ((int64_t)h * at.B + m) * at.ldS;
+    pa_tile_mm<false, float, 1, PA_TM>(acc, arow, 1.0f, brow, nullptr, at.dq, sm);
+    pa_tile_store<1, PA_TM, false>(acc, sm, [&](int row, int col, const float4 (&sum)[1]) {
+        const int m = m0 + row, p = pos0 + m;
+        if (m >= bs) return;
+        const int first = pa_first_key(at, p);
+        float *out = S + ((int64_t)h * at.B + m) * at.ldS;
+        const float s4[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int n = n0 + tx * 4 + j;
-            if (n <= p && n >= pa_first_key(at, p)) row[n] = pa_score(at, acc[0][i][j], h, p - n);
+            const int n = n0 + col + j;
+            if (n <= p && n >= first) out[n] = pa_score(at, s4[j], h, p - n);
         }
-    }
+    });
 }
 
 // per query: mix the heads' scores (b_h = sum_g T[h][g] a_g), soft-max every head's row (optionally with a sink term in the
@@ -1013,14 +1039,14 @@ __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__rest
 
 // att[i][h * dv + c] = sum_j P[h][i][j] V^T[g * dv + c][j].  With rotated values a tile's 64 columns are 32 pairs (m, m + dv / 2), two pairs to a
 // thread, which turns them back by its query's position; then the head's gate and the factor on the heads' outputs.
-__global__ void __launch_bounds__(256) pa_k_pv(PaAttn at, const float *__restrict__ S, const float *__restrict__ vct, float *__restrict__ att, int od,
+__global__ void __launch_bounds__(256, 2) pa_k_pv(PaAttn at, const float *__restrict__ S, const float *__restrict__ vct, float *__restrict__ att, int od,
                                                const int32_t *__restrict__ pos, int bs) {
-    PA_TILE_SMEM(1);
-    const int tid = threadIdx.x, lr = tid >> 2, tx = tid & 15, ty = tid >> 4;
+    __shared__ __align__(16) float sm[PaTile<1, PA_TM, true>::N];
+    const int lr = threadIdx.x >> 2;
     const int h = blockIdx.z, g = h / (at.H / at.G), m0 = blockIdx.y * PA_TM, n0 = blockIdx.x * PA_TN;
     const int n_keys = pos[0] + min(m0 + PA_TM, bs); // keys the tile's furthest query sees (the rows are zero beyond their own)
     const int k0 = pa_first_key(at, pos[0] + m0);    // ... and the first key its first query sees (zero before a row's own)
-    float acc[1][4][4] = {};
+    PaTile<1, PA_TM, true>::Acc acc = {};
     const float *arow = (m0 + lr < bs) ? S + ((int64_t)h * at.B + m0 + lr) * at.ldS + k0 : nullptr;
     // value dim of the tile's column j (dv or more: outside)
     const int vh = at.vrope.dims >> 1;
@@ -1031,34 +1057,34 @@ __global__ void __launch_bounds__(256) pa_k_pv(PaAttn at, const float *__restric
     };
     const int cb = col(lr);
     const float *brow = (cb < at.dv) ? vct + (int64_t)(g * at.dv + cb) * at.n_ctx + k0 : nullptr;
-    pa_tile_mm<false, float, 1>(acc, arow, 1.0f, brow, nullptr, n_keys - k0, As, Bs);
+    pa_tile_mm<false, float, 1, PA_TM, true>(acc, arow, 1.0f, brow, nullptr, n_keys - k0, sm);
     const int nv = pa_pool_vis(at, n_keys - 1); // pooled blocks of the tile's furthest query: their weights times the mean value rows
     if (nv > 0) {
         const float *arow2 = (m0 + lr < bs) ? S + ((int64_t)h * at.B + m0 + lr) * at.ldS + at.pool_off : nullptr;
         const float *brow2 = (n0 + lr < at.dv) ? vct + (int64_t)at.G * at.dv * at.n_ctx + (int64_t)(g * at.dv + n0 + lr) * at.n_pool : nullptr;
-        pa_tile_mm<false, float, 1>(acc, arow2, 1.0f, brow2, nullptr, nv, As, Bs);
+        pa_tile_mm<false, float, 1, PA_TM, true>(acc, arow2, 1.0f, brow2, nullptr, nv, sm);
     }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= bs) continue;
+    pa_tile_store<1, PA_TM, true>(acc, sm, [&](int row, int c4, const float4 (&sum)[1]) {
+        const int m = m0 + row;
+        if (m >= bs) return;
+        float s4[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w};
         float f = at.gate ? pa_sigmoid(at.gate[(int64_t)m * at.ld_gate + h]) : 1.0f;
         if (at.out_scale != 0.f) f *= at.out_scale;
         if (vh > 0) {
 #pragma unroll
             for (int j = 0; j < 2; j++) {
-                const int d = n0 / 2 + tx * 2 + j;
+                const int d = n0 / 2 + c4 / 2 + j;
                 if (d >= vh) continue;
                 const float2 cs = at.vrope.cs[(int64_t)m * at.vrope.ld_cs + d];
-                const float a = acc[0][i][j], b = acc[0][i][j + 2];
-                acc[0][i][j] = a * cs.x + b * cs.y;
-                acc[0][i][j + 2] = b * cs.x - a * cs.y;
+                const float a = s4[j], b = s4[j + 2];
+                s4[j] = a * cs.x + b * cs.y;
+                s4[j + 2] = b * cs.x - a * cs.y;
             }
         }
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const int n = col(tx * 4 + j);
-            if (n < at.dv) att[(int64_t)m * od + h * at.dv + n] = acc[0][i][j] * f;
+            const int n = col(c4 + j);
+            if (n < at.dv) att[(int64_t)m * od + h * at.dv + n] = s4[j] * f;
         }
-    }
+    });
 }
