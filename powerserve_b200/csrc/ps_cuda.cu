@@ -110,7 +110,7 @@ struct ps_cuda_ctx {
     float *rope_table = nullptr;
     // workspace
     int64_t maxK = 0;
-    float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *qr = nullptr, *kr = nullptr, *att = nullptr;
+    float *x = nullptr, *xn = nullptr, *q = nullptr, *k = nullptr, *v = nullptr, *qr = nullptr, *att = nullptr;
     float *g = nullptr, *u = nullptr, *kq = nullptr, *logits = nullptr;
     const float *logits_last = nullptr; // where the last forward left its [bs][vocab] logits (ps_cuda_logits_dev)
     int logits_rows = 0;                // rows of that buffer
@@ -363,16 +363,20 @@ int matmul_qb(ps_cuda_ctx *ctx, int wtype, int64_t K, int64_t bs, const PsMbSeg 
 }
 
 // quantise bs activation columns of K elements into the context's scratch (type of the WEIGHT decides the format)
-int quantize_act(ps_cuda_ctx *ctx, int wtype, const float *x, int64_t K, int64_t bs) {
+dim3 embed_grid(int64_t tokens, int64_t dim) { return dim3((unsigned)tokens, (unsigned)((dim + 1023) / 1024)); } // four elements a thread
+
+// what a product takes: x; silu(x) * u; or x normed with the weights `norm`
+struct ActIn { const float *x, *u = nullptr, *norm = nullptr; };
+int quantize_act(ps_cuda_ctx *ctx, int wtype, const ActIn &in, int64_t K, int64_t bs) {
     if (K > ctx->maxK || bs > ctx->d.max_batch) return fail(ctx, PS_CUDA_ERR_INVALID, "activation %lldx%lld exceeds workspace", (long long)K, (long long)bs);
     if (wtype == 12 || wtype == 13 || wtype == 14) {
         if (K % 256) return fail(ctx, PS_CUDA_ERR_INVALID, "K=%lld is not a multiple of 256", (long long)K);
-        dim3 grid((unsigned)((K / 256 + 3) / 4), (unsigned)bs);
-        ps_k_quantize_q8k<<<grid, 128, 0, ctx->stream>>>(x, K, ctx->aqs, ctx->ad, ctx->absp);
+        if (in.norm) ps_k_norm_quantize<true><<<(unsigned)bs, 512, 0, ctx->stream>>>(in.x, in.norm, K, ctx->d.norm_eps, ctx->aqs, ctx->ad, ctx->absp);
+        else ps_k_quantize_q8k<<<dim3((unsigned)((K / 256 + 3) / 4), (unsigned)bs), 128, 0, ctx->stream>>>(in.x, in.u, K, ctx->aqs, ctx->ad, ctx->absp);
     } else {
         if (K % 32) return fail(ctx, PS_CUDA_ERR_INVALID, "K=%lld is not a multiple of 32", (long long)K);
-        dim3 grid((unsigned)((K / 32 + 15) / 16), (unsigned)bs);
-        ps_k_quantize_q80<<<grid, 128, 0, ctx->stream>>>(x, K, ctx->aqs, ctx->ad);
+        if (in.norm) ps_k_norm_quantize<false><<<(unsigned)bs, 512, 0, ctx->stream>>>(in.x, in.norm, K, ctx->d.norm_eps, ctx->aqs, ctx->ad, nullptr);
+        else ps_k_quantize_q80<<<dim3((unsigned)((K / 32 + 15) / 16), (unsigned)bs), 128, 0, ctx->stream>>>(in.x, in.u, K, ctx->aqs, ctx->ad);
     }
     PS_LAUNCH_CK();
     return 0;
@@ -780,6 +784,33 @@ int rwm_single(ps_cuda_ctx *ctx, const uint8_t *w, int n_rows, int K, int slot, 
     return launch_rwm(ctx, a);
 }
 
+// rotations of a batch's q and k, K and V rows into the layer's caches (a tree's at slots base .., a copy kept aside; a session batch's into each one's own)
+int launch_rope_kv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int bs, int64_t base = -1, bool stage = false, bool sess = false) {
+    const ps_cuda_model_desc &d = ctx->d;
+    const int kvd = nkv * d.head_size;
+    PsRopeKv a{};
+    a.q = ctx->q; a.k = ctx->k; a.v = ctx->v; a.qr = ctx->qr; a.kc = ctx->kc[L]; a.vct = ctx->vct[L];
+    if (sess) {
+        a.kc_ptrs = ctx->sess_ptrs_dev + (size_t)L * 2 * d.max_batch;
+        a.vct_ptrs = a.kc_ptrs + d.max_batch;
+    }
+    if (stage) {
+        const size_t lstride = (size_t)std::min<int64_t>(d.max_batch, 32) * (size_t)kvd;
+        a.k_stage = ctx->k_stage + L * lstride;
+        a.v_stage = ctx->v_stage + L * lstride;
+    }
+    a.pos = ctx->pos_dev; a.table = ctx->rope_table; a.nh = nh; a.nkv = nkv; a.head_size = d.head_size; a.n_dims = d.rope_n_dims; a.neox = d.rope_type & 2; a.bs = bs;
+    a.n_ctx = d.n_ctx; a.base = base;
+    ps_k_rope_kv_batch<<<(unsigned)(((nh + nkv) * (d.head_size / 2) + 255) / 256 * bs + (kvd + 31) / 32 * ((bs + 31) / 32)), 256, 0, ctx->stream>>>(a);
+    PS_LAUNCH_CK();
+    return 0;
+}
+int rms_norm(ps_cuda_ctx *ctx, const float *w, int bs) { // of x into xn
+    ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, w, ctx->d.dim, ctx->d.norm_eps);
+    PS_LAUNCH_CK();
+    return 0;
+}
+
 // ---- tcgen05 GEMM of token batches (ps_tc.cuh)
 int64_t tc_tiles(int64_t rows) { return (rows + PS_TC_M - 1) / PS_TC_M; }
 int64_t tc_nbp(int64_t K) { return (K / 256 + 1) & ~(int64_t)1; } // super-blocks, rounded up to whole steps
@@ -817,11 +848,12 @@ template <int NT> int tc_launch(ps_cuda_ctx *ctx, PsTcArgs a) {
     return 0;
 }
 // quantises the input and multiplies; segments give their rows in the padded row space of the packed matrix (tile borders between them)
-int tc_gemm(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n_tiles, int64_t K, int bs, const PsRwSeg *segs, int n_seg, const float *residual) {
+int tc_gemm(ps_cuda_ctx *ctx, const ActIn &x, const uint8_t *a_blocks, int64_t n_tiles, int64_t K, int bs, const PsRwSeg *segs, int n_seg, const float *residual) {
     PsTcArgs a{};
     const TcPlan plan = tc_plan(ctx, n_tiles, K, bs);
     const int nt = plan.nt, n_ct = (bs + nt - 1) / nt;
-    ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x, K, bs, nt);
+    if (x.norm) ps_k_tc_norm_b<<<(unsigned)(n_ct * nt), 512, 0, ctx->stream>>>(ctx->tc_b, x.x, x.norm, K, ctx->d.norm_eps, bs, nt);
+    else ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x.x, x.u, K, bs, nt);
     PS_LAUNCH_CK();
     a.err = ctx->tc_err_dev;
     a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = n_ct; a.n_tiles = (int)n_tiles * n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
@@ -836,18 +868,18 @@ int tc_gemm(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n
     default: return tc_launch<16>(ctx, a);
     }
 }
-int tc_single(ps_cuda_ctx *ctx, const float *x, const uint8_t *a_blocks, int64_t n_rows, int64_t K, float *dst, int bs, const float *residual) {
+int tc_single(ps_cuda_ctx *ctx, const ActIn &x, const uint8_t *a_blocks, int64_t n_rows, int64_t K, float *dst, int bs, const float *residual) {
     PsRwSeg sg = {dst, nullptr, 0, (int)n_rows, 0};
     return tc_gemm(ctx, x, a_blocks, tc_tiles(n_rows), K, bs, &sg, 1, residual);
 }
-int tc_qkv(ps_cuda_ctx *ctx, const float *x, const LayerDev &ld, int64_t q_rows, int64_t kv_rows, int64_t K, int bs) {
+int tc_qkv(ps_cuda_ctx *ctx, const ActIn &x, const LayerDev &ld, int64_t q_rows, int64_t kv_rows, int64_t K, int bs) {
     const bool bias = ctx->d.qkv_bias != 0;
     const int k0 = (int)tc_tiles(q_rows) * PS_TC_M, v0 = k0 + (int)tc_tiles(kv_rows) * PS_TC_M;
     const PsRwSeg sg[3] = {{ctx->q, bias ? ld.q_bias : nullptr, 0, (int)q_rows, 0}, {ctx->k, bias ? ld.k_bias : nullptr, k0, k0 + (int)kv_rows, 0},
                            {ctx->v, bias ? ld.v_bias : nullptr, v0, v0 + (int)kv_rows, 0}};
     return tc_gemm(ctx, x, ld.tc_qkv, tc_tiles(q_rows) + 2 * tc_tiles(kv_rows), K, bs, sg, 3, nullptr);
 }
-int tc_gate_up(ps_cuda_ctx *ctx, const float *x, const LayerDev &ld, int64_t rows, int64_t K, int bs) {
+int tc_gate_up(ps_cuda_ctx *ctx, const ActIn &x, const LayerDev &ld, int64_t rows, int64_t K, int bs) {
     const int u0 = (int)tc_tiles(rows) * PS_TC_M;
     const PsRwSeg sg[2] = {{ctx->g, nullptr, 0, (int)rows, 0}, {ctx->u, nullptr, u0, u0 + (int)rows, 0}};
     return tc_gemm(ctx, x, ld.tc_gu, 2 * tc_tiles(rows), K, bs, sg, 2, nullptr);
@@ -959,7 +991,7 @@ int decode_step_mv32(ps_cuda_ctx *ctx, bool lm_head, bool pick) {
     const int dim = d.dim, hs = d.head_size, nh = d.n_heads, nkv = d.n_kv_heads, kvd = hs * nkv, qdim = nh * hs, ffn = d.ffn_dim;
     int rc;
     ctx->trace_launch = 0;
-    ps_k_get_embedding<<<1, 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, (int64_t)dim, ctx->tokens_dev);
+    ps_k_get_embedding<<<embed_grid(1, dim), 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, (int64_t)dim, ctx->tokens_dev);
     PS_LAUNCH_CK();
     for (int L = 0; L < d.n_layers; L++) {
         const LayerDev &ld = ctx->layers[L];
@@ -1049,39 +1081,26 @@ int decode_step_ops(ps_cuda_ctx *ctx, bool lm_head, bool pick) {
     const int64_t dim = d.dim, hs = d.head_size, nh = d.n_heads, nkv = d.n_kv_heads, kvd = hs * nkv, qdim = nh * hs, ffn = d.ffn_dim;
     int rc;
     ctx->trace_launch = 0;
-    ps_k_get_embedding<<<1, 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev); // every embedding type, token from device memory
+    ps_k_get_embedding<<<embed_grid(1, dim), 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev); // every embedding type, token from device memory
     PS_LAUNCH_CK();
     for (int L = 0; L < d.n_layers; L++) {
         const LayerDev &ld = ctx->layers[L];
-        ps_k_rmsnorm<<<1, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.attn_norm, dim, d.norm_eps);
-        PS_LAUNCH_CK();
-        if ((rc = quantize_act(ctx, ld.tq, ctx->xn, dim, 1))) return rc;
+        if ((rc = quantize_act(ctx, ld.tq, {ctx->x, nullptr, ld.attn_norm}, dim, 1))) return rc;
         if ((rc = matmul_q(ctx, ctx->q, ld.wq, ld.tq, dim, qdim, 1, d.qkv_bias ? ld.q_bias : nullptr, nullptr))) return rc;
         if ((rc = matmul_q(ctx, ctx->k, ld.wk, ld.tk, dim, kvd, 1, d.qkv_bias ? ld.k_bias : nullptr, nullptr))) return rc;
         if ((rc = matmul_q(ctx, ctx->v, ld.wv, ld.tv, dim, kvd, 1, d.qkv_bias ? ld.v_bias : nullptr, nullptr))) return rc;
-        ps_k_rope<<<dim3((unsigned)nh, 1), 64, 0, ctx->stream>>>(ctx->qr, ctx->q, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
-        PS_LAUNCH_CK();
-        ps_k_rope<<<dim3((unsigned)nkv, 1), 64, 0, ctx->stream>>>(ctx->kr, ctx->k, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
-        PS_LAUNCH_CK();
-        ps_k_kv_store<<<grid1d(kvd), 256, 0, ctx->stream>>>(ctx->kc[L], ctx->vct[L], ctx->kr, ctx->v, kvd, d.n_ctx, ctx->pos_dev, 1);
-        PS_LAUNCH_CK();
+        if ((rc = launch_rope_kv(ctx, L, (int)nh, (int)nkv, 1))) return rc;
         if ((rc = launch_attn_any(ctx, L, ctx->qr))) return rc;
-        if ((rc = quantize_act(ctx, ld.to, ctx->att, qdim, 1))) return rc;
+        if ((rc = quantize_act(ctx, ld.to, {ctx->att}, qdim, 1))) return rc;
         if ((rc = matmul_q(ctx, ctx->x, ld.wo, ld.to, qdim, dim, 1, nullptr, ctx->x))) return rc;
-        ps_k_rmsnorm<<<1, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.ffn_norm, dim, d.norm_eps);
-        PS_LAUNCH_CK();
-        if ((rc = quantize_act(ctx, ld.tgate, ctx->xn, dim, 1))) return rc;
+        if ((rc = quantize_act(ctx, ld.tgate, {ctx->x, nullptr, ld.ffn_norm}, dim, 1))) return rc;
         if ((rc = matmul_q(ctx, ctx->g, ld.wgate, ld.tgate, dim, ffn, 1, nullptr, nullptr))) return rc;
         if ((rc = matmul_q(ctx, ctx->u, ld.wup, ld.tup, dim, ffn, 1, nullptr, nullptr))) return rc;
-        ps_k_silu_hadamard<<<grid1d(ffn), 256, 0, ctx->stream>>>(ctx->g, ctx->g, ctx->u, ffn);
-        PS_LAUNCH_CK();
-        if ((rc = quantize_act(ctx, ld.tdown, ctx->g, ffn, 1))) return rc;
+        if ((rc = quantize_act(ctx, ld.tdown, {ctx->g, ctx->u}, ffn, 1))) return rc;
         if ((rc = matmul_q(ctx, ctx->x, ld.wdown, ld.tdown, ffn, dim, 1, nullptr, ctx->x))) return rc;
     }
     if (lm_head) {
-        ps_k_rmsnorm<<<1, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ctx->w_out_norm, dim, d.norm_eps);
-        PS_LAUNCH_CK();
-        if ((rc = quantize_act(ctx, ctx->t_out, ctx->xn, dim, 1))) return rc;
+        if ((rc = quantize_act(ctx, ctx->t_out, {ctx->x, nullptr, ctx->w_out_norm}, dim, 1))) return rc;
         if ((rc = matmul_q(ctx, ctx->logits, ctx->w_out, ctx->t_out, dim, d.vocab_size, 1, nullptr, nullptr))) return rc;
         if (pick) {
             const int n_part = std::min(ctx->n_sm, (d.vocab_size + 255) / 256);
@@ -1330,7 +1349,6 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
     PS_AL(ctx->k, 4 * kvd * B);
     PS_AL(ctx->v, 4 * kvd * B);
     PS_AL(ctx->qr, 4 * qdim * B);
-    PS_AL(ctx->kr, 4 * kvd * B);
     PS_AL(ctx->att, 4 * qdim * B);
     PS_AL(ctx->g, 4 * (int64_t)d.ffn_dim * B);
     PS_AL(ctx->u, 4 * (int64_t)d.ffn_dim * B);
@@ -1674,7 +1692,7 @@ int ps_cuda_get_embedding(ps_cuda_ctx *ctx, float *dst, const void *w, int wtype
     if (!type_ok(wtype) || dim % blk_elems(wtype)) return fail(ctx, PS_CUDA_ERR_INVALID, "get_embedding: bad type/dim");
     int rc = stage_ints(ctx, ctx->tokens_dev, ctx->h_tokens, tokens, bs);
     if (rc) return rc;
-    ps_k_get_embedding<<<(unsigned)bs, 256, 0, ctx->stream>>>(dst, (const uint8_t *)w, wtype, dim, ctx->tokens_dev);
+    ps_k_get_embedding<<<embed_grid(bs, dim), 256, 0, ctx->stream>>>(dst, (const uint8_t *)w, wtype, dim, ctx->tokens_dev);
     PS_LAUNCH_CK();
     return 0;
 }
@@ -1689,7 +1707,7 @@ int ps_cuda_rmsnorm(ps_cuda_ctx *ctx, float *dst, const float *x, const float *w
 int ps_cuda_matmul(ps_cuda_ctx *ctx, float *dst, const void *w, int wtype, int64_t K, int64_t N, const float *x, int64_t bs) {
     PS_NO_ARCH("ps_cuda_matmul");
     if (bs <= 0 || N <= 0) return fail(ctx, PS_CUDA_ERR_INVALID, "matmul: empty shape");
-    int rc = quantize_act(ctx, wtype, x, K, bs);
+    int rc = quantize_act(ctx, wtype, {x}, K, bs);
     if (rc) return rc;
     return matmul_q(ctx, dst, (const uint8_t *)w, wtype, K, N, bs, nullptr, nullptr);
 }
@@ -2129,7 +2147,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     const bool mo = bs > 1 && mv_usable(ctx); // octet copies of a 32-block model
     const bool rw = ctx->fused_ok && ctx->opt_fused && (bs > 1 || tree); // octet-interleaved copies exist: multi-column row-walker
     int rc;
-    ps_k_get_embedding<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
+    ps_k_get_embedding<<<embed_grid(bs, dim), 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
     PS_LAUNCH_CK();
     static bool attr[64] = {};
     if (!attr[ctx->device]) {
@@ -2139,11 +2157,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     }
     for (int L = 0; L < d.n_layers; L++) {
         const LayerDev &ld = ctx->layers[L];
-        ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.attn_norm, dim, d.norm_eps);
-        PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_qkv(ctx, ctx->xn, ld, qdim, kvd, dim, bs))) return rc;
+            if ((rc = tc_qkv(ctx, {ctx->x, nullptr, ld.attn_norm}, ld, qdim, kvd, dim, bs))) return rc;
         } else if (rw) { // q | k | v rows in one pass over the concatenated octets
+            if ((rc = rms_norm(ctx, ld.attn_norm, bs))) return rc;
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             PsRwmArgs a{};
             a.w = ld.rw_qkv; a.n_oct = (int)((qdim + 2 * kvd) / 8); a.K = (int)dim; a.slot = 0; a.n_slots = 1; a.n_seg = 3; a.bs = bs;
@@ -2152,7 +2169,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             a.seg[2] = {ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)(qdim + kvd), (int)(qdim + 2 * kvd), 0};
             if ((rc = launch_rwm(ctx, a))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.tq, ctx->xn, dim, bs))) return rc;
+            if ((rc = quantize_act(ctx, ld.tq, {ctx->x, nullptr, ld.attn_norm}, dim, bs))) return rc;
             const PsMbSeg sg[3] = {{ld.wq, ctx->q, d.qkv_bias ? ld.q_bias : nullptr, (int)qdim, 0}, {ld.wk, ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)kvd, 0},
                                    {ld.wv, ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)kvd, 0}};
             bool done = false;
@@ -2171,21 +2188,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
                     if ((rc = matmul_q(ctx, sg[t].dst, sg[t].w, ty[t], dim, sg[t].n, bs, sg[t].bias, nullptr))) return rc;
             }
         }
-        ps_k_rope<<<dim3((unsigned)nh, (unsigned)bs), 64, 0, ctx->stream>>>(ctx->qr, ctx->q, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
-        PS_LAUNCH_CK();
-        ps_k_rope<<<dim3((unsigned)nkv, (unsigned)bs), 64, 0, ctx->stream>>>(ctx->kr, ctx->k, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
-        PS_LAUNCH_CK();
-        if (sess) {
-            float **pl = ctx->sess_ptrs_dev + (size_t)L * 2 * d.max_batch;
-            ps_k_sess_kv_store<<<grid1d(kvd * bs), 256, 0, ctx->stream>>>(pl, pl + d.max_batch, ctx->kr, ctx->v, kvd, d.n_ctx, ctx->pos_dev, bs);
-        } else if (tree) {
-            const size_t lstride = (size_t)std::min<int64_t>(d.max_batch, 32) * (size_t)kvd;
-            ps_k_kv_store_at<<<grid1d(kvd * bs), 256, 0, ctx->stream>>>(ctx->kc[L], ctx->vct[L], ctx->k_stage + L * lstride, ctx->v_stage + L * lstride, ctx->kr, ctx->v,
-                                                                         kvd, d.n_ctx, tree_base, bs);
-        } else {
-            ps_k_kv_store<<<grid1d(kvd * bs), 256, 0, ctx->stream>>>(ctx->kc[L], ctx->vct[L], ctx->kr, ctx->v, kvd, d.n_ctx, ctx->pos_dev, bs);
-        }
-        PS_LAUNCH_CK();
+        if ((rc = launch_rope_kv(ctx, L, (int)nh, (int)nkv, bs, tree ? tree_base : -1, tree, sess != nullptr))) return rc;
         if (sess) { // every column attends over its own session's cache at its own position
             float **pl = ctx->sess_ptrs_dev + (size_t)L * 2 * d.max_batch;
             const int64_t cs = nh * (int64_t)d.n_ctx;
@@ -2206,27 +2209,26 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         PS_LAUNCH_CK();
         }
         if (tc) {
-            if ((rc = tc_single(ctx, ctx->att, ld.tc_o, (int)dim, (int)qdim, ctx->x, bs, ctx->x))) return rc;
+            if ((rc = tc_single(ctx, {ctx->att}, ld.tc_o, (int)dim, (int)qdim, ctx->x, bs, ctx->x))) return rc;
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->att, (int)qdim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_o, (int)dim, (int)qdim, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.to, ctx->att, qdim, bs))) return rc;
+            if ((rc = quantize_act(ctx, ld.to, {ctx->att}, qdim, bs))) return rc;
             bool done = false;
             const PsMbSeg so = {ld.mv_o, ctx->x, nullptr, (int)dim, 0};
             if (mo && (rc = matmul_ob(ctx, qdim, bs, &so, 1, ctx->x, &done))) return rc;
             if (!done && (rc = matmul_q(ctx, ctx->x, ld.wo, ld.to, qdim, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wo.att
         }
-        ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ld.ffn_norm, dim, d.norm_eps);
-        PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_gate_up(ctx, ctx->xn, ld, ffn, dim, bs))) return rc;
+            if ((rc = tc_gate_up(ctx, {ctx->x, nullptr, ld.ffn_norm}, ld, ffn, dim, bs))) return rc;
         } else if (rw) {
+            if ((rc = rms_norm(ctx, ld.ffn_norm, bs))) return rc;
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 1, 2, ctx->u, bs, nullptr, nullptr))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.tgate, ctx->xn, dim, bs))) return rc;
+            if ((rc = quantize_act(ctx, ld.tgate, {ctx->x, nullptr, ld.ffn_norm}, dim, bs))) return rc;
             bool done = false;
             if (mo) {
                 const PsMbSeg so[2] = {{ld.mv_gu, ctx->g, nullptr, (int)ffn, 0}, {ld.mv_gu + mv_bytes(ctx->mv_type, 8, dim) * (size_t)(ffn / 8), ctx->u, nullptr, (int)ffn, 0}};
@@ -2241,15 +2243,15 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
                 if ((rc = matmul_q(ctx, ctx->u, ld.wup, ld.tup, dim, ffn, bs, nullptr, nullptr))) return rc;
             }
         }
-        ps_k_silu_hadamard<<<grid1d(ffn * bs), 256, 0, ctx->stream>>>(ctx->g, ctx->g, ctx->u, ffn * bs);
-        PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_single(ctx, ctx->g, ld.tc_down, (int)dim, (int)ffn, ctx->x, bs, ctx->x))) return rc;
+            if ((rc = tc_single(ctx, {ctx->g, ctx->u}, ld.tc_down, (int)dim, (int)ffn, ctx->x, bs, ctx->x))) return rc;
         } else if (rw) {
+            ps_k_silu_hadamard<<<grid1d(ffn * bs), 256, 0, ctx->stream>>>(ctx->g, ctx->g, ctx->u, ffn * bs);
+            PS_LAUNCH_CK();
             if ((rc = rwm_quantize(ctx, ctx->g, (int)ffn, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_down, (int)dim, (int)ffn, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.tdown, ctx->g, ffn, bs))) return rc;
+            if ((rc = quantize_act(ctx, ld.tdown, {ctx->g, ctx->u}, ffn, bs))) return rc;
             bool done = false;
             const PsMbSeg so = {ld.mv_down, ctx->x, nullptr, (int)dim, 0};
             if (mo && (rc = matmul_ob(ctx, ffn, bs, &so, 1, ctx->x, &done))) return rc;
@@ -2257,15 +2259,14 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         }
     }
     if (lm_head) {
-        ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, ctx->w_out_norm, dim, d.norm_eps);
-        PS_LAUNCH_CK();
         if (tc && ctx->tc_out) {
-            if ((rc = tc_single(ctx, ctx->xn, ctx->tc_out, d.vocab_size, (int)dim, ctx->logits, bs, nullptr))) return rc;
+            if ((rc = tc_single(ctx, {ctx->x, nullptr, ctx->w_out_norm}, ctx->tc_out, d.vocab_size, (int)dim, ctx->logits, bs, nullptr))) return rc;
         } else if (rw) {
+            if ((rc = rms_norm(ctx, ctx->w_out_norm, bs))) return rc;
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ctx->rw_out, d.vocab_size, (int)dim, 0, 1, ctx->logits, bs, nullptr, nullptr))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ctx->t_out, ctx->xn, dim, bs))) return rc;
+            if ((rc = quantize_act(ctx, ctx->t_out, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs))) return rc;
             bool done = false;
             const PsMbSeg so = {ctx->mv_out, ctx->logits, nullptr, d.vocab_size, 0};
             if (mo && (rc = matmul_ob(ctx, dim, bs, &so, 1, nullptr, &done))) return rc;
@@ -2321,7 +2322,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
     float *x = ctx->tp_xb, *xl = ctx->tp_xl, *attb = ctx->tp_attb, *hb = ctx->tp_hb; // batch-sized twins of the single-token exchange buffers
     static bool attr[64] = {};
     if (!attr[ctx->device]) { PS_CK(cudaFuncSetAttribute(ps_k_softmax_ext, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024)); attr[ctx->device] = true; }
-    ps_k_get_embedding<<<(unsigned)bs, 256, 0, ctx->stream>>>(x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
+    ps_k_get_embedding<<<embed_grid(bs, dim), 256, 0, ctx->stream>>>(x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
     PS_LAUNCH_CK();
     ps_k_tp_slice<<<grid1d(bs * dim_l), 256, 0, ctx->stream>>>(xl, x, bs, dim, dim_l, rank);
     PS_LAUNCH_CK();
@@ -2333,7 +2334,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
                          {ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)qdim_l, (int)(qdim_l + kvd), 0},
                          {ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)(qdim_l + kvd), (int)(qdim_l + 2 * kvd), 0}};
         if (tc) {
-            if ((rc = tc_qkv(ctx, ctx->xn, ld, qdim_l, kvd, dim, bs))) return rc;
+            if ((rc = tc_qkv(ctx, {ctx->xn}, ld, qdim_l, kvd, dim, bs))) return rc;
         } else {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             PsRwmArgs a{};
@@ -2341,12 +2342,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
             for (int t = 0; t < 3; t++) a.seg[t] = sg[t];
             if ((rc = launch_rwm(ctx, a))) return rc;
         }
-        ps_k_rope<<<dim3((unsigned)nh, (unsigned)bs), 64, 0, ctx->stream>>>(ctx->qr, ctx->q, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
-        PS_LAUNCH_CK();
-        ps_k_rope<<<dim3((unsigned)nkv, (unsigned)bs), 64, 0, ctx->stream>>>(ctx->kr, ctx->k, (int)hs, d.rope_n_dims, d.rope_type & 2, ctx->pos_dev, ctx->rope_table);
-        PS_LAUNCH_CK();
-        ps_k_kv_store<<<grid1d(kvd * bs), 256, 0, ctx->stream>>>(ctx->kc[L], ctx->vct[L], ctx->kr, ctx->v, kvd, d.n_ctx, ctx->pos_dev, bs);
-        PS_LAUNCH_CK();
+        if ((rc = launch_rope_kv(ctx, L, (int)nh, (int)nkv, bs))) return rc;
         launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs);
         PS_LAUNCH_CK();
         ps_k_softmax_ext<<<(unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->stream>>>(ctx->kq, ctx->kq, nullptr, ctx->pos_dev, n_kv, bs, kq_scale);
@@ -2355,7 +2351,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         PS_LAUNCH_CK();
         if ((rc = tp_gather_rows(ctx, attb, ctx->att, bs, qdim_l))) return rc;                      // exchange 1: attention output
         if (tc) {
-            if ((rc = tc_single(ctx, attb, ld.tc_o, (int)dim_l, (int)qdim, xl, bs, xl))) return rc;       // x[rows of this rank] += Wo[rows] . att
+            if ((rc = tc_single(ctx, {attb}, ld.tc_o, (int)dim_l, (int)qdim, xl, bs, xl))) return rc;       // x[rows of this rank] += Wo[rows] . att
         } else {
             if ((rc = rwm_quantize(ctx, attb, (int)qdim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_o, (int)dim_l, (int)qdim, 0, 1, xl, bs, nullptr, xl))) return rc;
@@ -2364,7 +2360,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, x, ld.ffn_norm, dim, d.norm_eps);
         PS_LAUNCH_CK();
         if (tc) {
-            if ((rc = tc_gate_up(ctx, ctx->xn, ld, ffn_l, dim, bs))) return rc;
+            if ((rc = tc_gate_up(ctx, {ctx->xn}, ld, ffn_l, dim, bs))) return rc;
         } else {
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn_l, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;
@@ -2374,7 +2370,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         PS_LAUNCH_CK();
         if ((rc = tp_gather_rows(ctx, hb, ctx->g, bs, ffn_l))) return rc;                             // exchange 3: FFN hidden vector
         if (tc) {
-            if ((rc = tc_single(ctx, hb, ld.tc_down, (int)dim_l, (int)ffn, xl, bs, xl))) return rc;     // x[rows] += Wdown[rows] . h
+            if ((rc = tc_single(ctx, {hb}, ld.tc_down, (int)dim_l, (int)ffn, xl, bs, xl))) return rc;     // x[rows] += Wdown[rows] . h
         } else {
             if ((rc = rwm_quantize(ctx, hb, (int)ffn, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_down, (int)dim_l, (int)ffn, 0, 1, xl, bs, nullptr, xl))) return rc;

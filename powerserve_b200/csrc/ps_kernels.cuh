@@ -66,19 +66,10 @@ PS_D float ps_f32x8_reduce(float v) {
 //   bsp [nb][4] uint32   : int16 pair (s_{2k}, s_{2k+1}), s_j = sum of the 32 quants of sub-block j
 //                          (== hadd_epi16 of block_q8_K::bsums, ggml-quants.c:7829-7830)
 
-// quantize_row_q8_K_ref (libs/ggml/src/ggml-quants.c:3799-3837).  One warp per 256-block.
-__global__ void __launch_bounds__(128) ps_k_quantize_q8k(const float *__restrict__ x, int64_t K, uint32_t *__restrict__ qs,
-                                                         float *__restrict__ dq, uint32_t *__restrict__ bsp) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nb = K / 256;
-    const int64_t i = (int64_t)blockIdx.x * 4 + warp;
-    const int64_t col = blockIdx.y;
-    if (i >= nb) return;
+// quantize_row_q8_K_ref (libs/ggml/src/ggml-quants.c:3799-3837), one warp per 256-block: lane (jj, l) holds elements 32 jj + 4 l .. + 3 and 128 further on
+__device__ __forceinline__ void ps_store_q8k(const float e[8], int lane, int64_t i, int64_t col, int64_t nb, uint32_t *__restrict__ qs, float *__restrict__ dq,
+                                             uint32_t *__restrict__ bsp) {
     const int l = lane & 7, jj = lane >> 3;
-    const float *xb = x + col * K + i * 256;
-    const float4 v0 = *reinterpret_cast<const float4 *>(xb + 32 * jj + 4 * l);
-    const float4 v1 = *reinterpret_cast<const float4 *>(xb + 32 * (jj + 4) + 4 * l);
-    const float e[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
     const int idx0 = 32 * jj + 4 * l, idx1 = 32 * (jj + 4) + 4 * l;
     float amax = 0.f;
 #pragma unroll
@@ -140,16 +131,8 @@ __global__ void __launch_bounds__(128) ps_k_quantize_q8k(const float *__restrict
 // quantize_row_q8_0, AVX2 branch (libs/ggml/src/ggml-quants.c:957-1017): d = max|x| / 127 stored as fp16,
 // id = 127 / max|x|, round-half-to-even.  One warp handles four 32-blocks (lane = 8*b + l owns word l of block b).
 // Layout: qs [nb32][8] uint32 natural order, d [nb32] float holding fp16(d) widened back (what the dot product reads).
-__global__ void __launch_bounds__(128) ps_k_quantize_q80(const float *__restrict__ x, int64_t K, uint32_t *__restrict__ qs,
-                                                         float *__restrict__ dq) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nb = K / 32;
-    const int64_t i = ((int64_t)blockIdx.x * 4 + warp) * 4 + (lane >> 3);
-    const int64_t col = blockIdx.y;
+__device__ __forceinline__ void ps_store_q80(float4 v, bool valid, int lane, int64_t i, int64_t col, int64_t nb, uint32_t *__restrict__ qs, float *__restrict__ dq) {
     const int l = lane & 7;
-    const bool valid = i < nb;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid) v = *reinterpret_cast<const float4 *>(x + col * K + i * 32 + 4 * l);
     float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 #pragma unroll
     for (int o = 1; o < 8; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(PS_FULL, amax, o));
@@ -160,6 +143,35 @@ __global__ void __launch_bounds__(128) ps_k_quantize_q80(const float *__restrict
     const int q2 = __float2int_rn(__fmul_rn(v.z, id)), q3 = __float2int_rn(__fmul_rn(v.w, id));
     qs[(col * nb + i) * 8 + l] = (uint32_t)(q0 & 0xff) | ((uint32_t)(q1 & 0xff) << 8) | ((uint32_t)(q2 & 0xff) << 16) | ((uint32_t)(q3 & 0xff) << 24);
     if (l == 0) dq[col * nb + i] = __half2float(__float2half_rn(d));
+}
+
+// four (or eight: 128 further on) elements of what a product takes: x, or silu(x) * u where u is given
+__device__ __forceinline__ float4 ps_act4(const float *__restrict__ x, const float *__restrict__ u) {
+    float4 v = *reinterpret_cast<const float4 *>(x);
+    if (u) {
+        const float4 w = *reinterpret_cast<const float4 *>(u);
+        v = make_float4(ps_silu_mul(v.x, w.x), ps_silu_mul(v.y, w.y), ps_silu_mul(v.z, w.z), ps_silu_mul(v.w, w.w));
+    }
+    return v;
+}
+__device__ __forceinline__ void ps_act8(const float *__restrict__ x, const float *__restrict__ u, int lane, float e[8]) {
+    const float4 a = ps_act4(x + 4 * lane, u ? u + 4 * lane : nullptr), b = ps_act4(x + 128 + 4 * lane, u ? u + 128 + 4 * lane : nullptr);
+    e[0] = a.x; e[1] = a.y; e[2] = a.z; e[3] = a.w; e[4] = b.x; e[5] = b.y; e[6] = b.z; e[7] = b.w;
+}
+__global__ void __launch_bounds__(128) ps_k_quantize_q8k(const float *__restrict__ x, const float *__restrict__ u, int64_t K, uint32_t *__restrict__ qs, float *__restrict__ dq,
+                                                         uint32_t *__restrict__ bsp) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nb = K / 256, i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5), col = blockIdx.y, at = col * K + i * 256;
+    if (i >= nb) return;
+    float e[8];
+    ps_act8(x + at, u ? u + at : nullptr, lane, e);
+    ps_store_q8k(e, lane, i, col, nb, qs, dq, bsp);
+}
+__global__ void __launch_bounds__(128) ps_k_quantize_q80(const float *__restrict__ x, const float *__restrict__ u, int64_t K, uint32_t *__restrict__ qs, float *__restrict__ dq) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nb = K / 32, i = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + (lane >> 3), col = blockIdx.y, at = col * K + i * 32 + 4 * (lane & 7);
+    const bool valid = i < nb;
+    ps_store_q80(valid ? ps_act4(x + at, u ? u + at : nullptr) : make_float4(0.f, 0.f, 0.f, 0.f), valid, lane, i, col, nb, qs, dq);
 }
 
 // ====================================================================================================================
@@ -613,13 +625,14 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
 // Small fp32 operators
 // ====================================================================================================================
 // GGMLBackend::get_embedding (src/backend/ggml/ggml_wrapper.cpp:181-211) + dequantize_row_* (ggml-quants.c:1536,
-// 1630, 2569, 2991).  One CTA per token row.
+// 1630, 2569, 2991).  blockIdx.x: token, blockIdx.y: its share of the row (an element's address and scales are a chain of loads; 16 of them one after
+// the other took 8.6 us on rows of 4096).
 __global__ void __launch_bounds__(256) ps_k_get_embedding(float *__restrict__ dst, const uint8_t *__restrict__ w, int type,
                                                           int64_t dim, const int32_t *__restrict__ tokens) {
     const int64_t tok = tokens[blockIdx.x];
     const uint8_t *row = w + tok * ps_row_bytes(type, dim);
     float *y = dst + (int64_t)blockIdx.x * dim;
-    for (int64_t e = threadIdx.x; e < dim; e += blockDim.x) {
+    for (int64_t e = (int64_t)blockIdx.y * 256 + threadIdx.x; e < dim; e += (int64_t)gridDim.y * 256) {
         float v;
         if (type == 0) {
             v = reinterpret_cast<const float *>(row)[e];
@@ -692,71 +705,134 @@ PS_D double ps_block_sum_double(double v, double *sh) {
 }
 
 // powerserve_compute_forward_rms_norm_f32 (libs/ggml/src/ggml.c:12667-12721): y = x * (w * 1/sqrtf(mean(x^2)+eps)),
-// the sum of fp32 squares accumulated in double.  One CTA per row.
+// the sum of fp32 squares accumulated in double.  One CTA per row, the first 256 threads add (the tree of the others' zeros changes nothing): the factor 1/sqrtf(..)
+__device__ __forceinline__ float ps_rms_scale(const float *__restrict__ xr, int64_t dim, float eps, double *sh) {
+    double s = 0.0;
+    if (threadIdx.x < 256)
+#pragma unroll 8
+        for (int64_t e = threadIdx.x; e < dim; e += 256) s += (double)__fmul_rn(xr[e], xr[e]);
+    const double sum = ps_block_sum_double(s, sh);
+    const float mean = (float)(sum / (double)dim);
+    return __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+}
 __global__ void __launch_bounds__(256) ps_k_rmsnorm(float *__restrict__ dst, const float *__restrict__ x, const float *__restrict__ w,
                                                     int64_t dim, float eps) {
     __shared__ double sh[32];
     const float *xr = x + (int64_t)blockIdx.x * dim;
     float *yr = dst + (int64_t)blockIdx.x * dim;
-    double s = 0.0;
-    for (int64_t e = threadIdx.x; e < dim; e += blockDim.x) s += (double)__fmul_rn(xr[e], xr[e]);
-    const double sum = ps_block_sum_double(s, sh);
-    const float mean = (float)(sum / (double)dim);
-    const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
-    for (int64_t e = threadIdx.x; e < dim; e += blockDim.x) yr[e] = __fmul_rn(xr[e], __fmul_rn(w[e], scale));
+    const float scale = ps_rms_scale(xr, dim, eps, sh);
+    for (int64_t e = threadIdx.x; e < dim; e += 256) yr[e] = __fmul_rn(xr[e], __fmul_rn(w[e], scale));
+}
+__device__ __forceinline__ float4 ps_norm4(const float *__restrict__ x, const float *__restrict__ w, float scale) {
+    const float4 v = *reinterpret_cast<const float4 *>(x), g = *reinterpret_cast<const float4 *>(w);
+    return make_float4(__fmul_rn(v.x, __fmul_rn(g.x, scale)), __fmul_rn(v.y, __fmul_rn(g.y, scale)), __fmul_rn(v.z, __fmul_rn(g.z, scale)), __fmul_rn(v.w, __fmul_rn(g.w, scale)));
+}
+// The norm and the quantiser of the products behind it in one launch (one CTA a row): on batches both are a few microseconds of latency, and a launch and
+// a trip through memory lay between them (32 rows of 896: 5.3 + 3.2 us, together 5.7)
+template <bool Q8K> __global__ void __launch_bounds__(512) ps_k_norm_quantize(const float *__restrict__ x, const float *__restrict__ w, int64_t dim, float eps, uint32_t *__restrict__ qs,
+                                                                             float *__restrict__ dq, uint32_t *__restrict__ bsp) {
+    __shared__ double sh[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t col = blockIdx.x, nb = dim / (Q8K ? 256 : 32);
+    const float *xr = x + col * dim;
+    const float scale = ps_rms_scale(xr, dim, eps, sh);
+    if (Q8K) {
+        for (int64_t i = warp; i < nb; i += 16) {
+            const int64_t at = i * 256 + 4 * lane;
+            const float4 a = ps_norm4(xr + at, w + at, scale), b = ps_norm4(xr + at + 128, w + at + 128, scale);
+            const float e[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+            ps_store_q8k(e, lane, i, col, nb, qs, dq, bsp);
+        }
+    } else {
+        for (int64_t i0 = warp * 4; i0 < nb; i0 += 64) {
+            const int64_t i = i0 + (lane >> 3), at = i * 32 + 4 * (lane & 7);
+            ps_store_q80(i < nb ? ps_norm4(xr + at, w + at, scale) : make_float4(0.f, 0.f, 0.f, 0.f), i < nb, lane, i, col, nb, qs, dq);
+        }
+    }
 }
 
 // ggml_compute_forward_rope_f32 (libs/ggml/src/ggml.c:15368-15497) with the cos/sin cache of ggml_rope_cache_init
 // (:15342-15356) precomputed for every position by the host (ps_cuda.cu: build_rope_table) — table[pos][i0] = cos,
 // table[pos][i0+1] = sin.  src/dst {head_size, n_heads, bs}; grid (n_heads, bs).
+// pair p of a head: where its two elements lie and what they become
+struct PsPair { int a, b; float ya, yb; };
+__device__ __forceinline__ PsPair ps_rope_pair(const float *__restrict__ s, int p, int n_dims, int neox, const float *__restrict__ cache) {
+    const int i0 = 2 * p;
+    if (i0 >= n_dims) return {i0, i0 + 1, s[i0], s[i0 + 1]};
+    const float c = cache[i0], sn = cache[i0 + 1];
+    const int a = neox ? p : i0, b = neox ? p + n_dims / 2 : i0 + 1;
+    const float x0 = s[a], x1 = s[b];
+    return {a, b, __fadd_rn(__fmul_rn(x0, c), -__fmul_rn(x1, sn)),  // x0*c - x1*s  (not fused in the reference)
+            __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c))};         // x0*s + x1*c
+}
 __global__ void ps_k_rope(float *__restrict__ dst, const float *__restrict__ src, int head_size, int n_dims, int neox,
                           const int32_t *__restrict__ pos, const float *__restrict__ table) {
     const int64_t row = (int64_t)blockIdx.y * gridDim.x + blockIdx.x;
-    const float *s = src + row * head_size;
     float *d = dst + row * head_size;
-    const float *cache = table + (int64_t)pos[blockIdx.y] * head_size;
     for (int p = threadIdx.x; p < head_size / 2; p += blockDim.x) {
-        const int i0 = 2 * p;
-        if (i0 < n_dims) {
-            const float c = cache[i0], sn = cache[i0 + 1];
-            const int a = neox ? p : i0, bidx = neox ? p + n_dims / 2 : i0 + 1;
-            const float x0 = s[a], x1 = s[bidx];
-            d[a] = __fadd_rn(__fmul_rn(x0, c), -__fmul_rn(x1, sn));    // x0*c - x1*s  (not fused in the reference)
-            d[bidx] = __fadd_rn(__fmul_rn(x0, sn), __fmul_rn(x1, c));  // x0*s + x1*c
-        } else {
-            d[i0] = s[i0];
-            d[i0 + 1] = s[i0 + 1];
-        }
+        const PsPair v = ps_rope_pair(src + row * head_size, p, n_dims, neox, table + (int64_t)pos[blockIdx.y] * head_size);
+        d[v.a] = v.ya;
+        d[v.b] = v.yb;
     }
 }
 
-// KV store: the two COPY ops of NormAttention::build (src/model/module/norm_attention.cpp:79-105).
-// K cache [n_ctx][kv_dim] <- rope(k) rows at pos0..; V cache TRANSPOSED [kv_dim][n_ctx] <- v columns at pos0..
-__global__ void ps_k_kv_store(float *__restrict__ kc, float *__restrict__ vct, const float *__restrict__ k, const float *__restrict__ v,
-                              int64_t kv_dim, int64_t n_ctx, const int32_t *__restrict__ pos, int64_t bs) {
-    const int64_t pos0 = pos[0];
-    const int64_t total = kv_dim * bs;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / kv_dim, e = t % kv_dim;
-        kc[(pos0 + i) * kv_dim + e] = k[t];
-        vct[e * n_ctx + pos0 + i] = v[t];
+// Rotations and cache stores of a batch in one launch - the two COPY ops of NormAttention::build (src/model/module/norm_attention.cpp:79-105): K cache
+// [n_ctx][kv_dim] <- rope(k) rows, V cache TRANSPOSED [kv_dim][n_ctx] <- v columns (three launches of 3 to 5 us each before): the first CTAs rotate a token's q into qr and k into the K cache, a pair a thread, further ones
+// carry 32 channels x 32 tokens of v to the transposed cache, through shared memory so that both sides are whole lines.
+// Cache rows: token i goes to slot base + i (base < 0: pos[0] + i) of kc / vct, or, with per-token caches (sessions), to row pos[i] of kc_ptrs[i] /
+// vct_ptrs[i].  k_stage / v_stage (or null) get the rotated k and the v rows once more (`copy` of a tree's tokens).
+struct PsRopeKv {
+    const float *q, *k, *v;
+    float *qr, *kc, *vct;
+    float *const *kc_ptrs, *const *vct_ptrs;
+    float *k_stage, *v_stage;
+    const int32_t *pos;
+    const float *table;
+    int nh, nkv, head_size, n_dims, neox, bs;
+    int64_t n_ctx, base;
+};
+__global__ void __launch_bounds__(256) ps_k_rope_kv_batch(const PsRopeKv a) {
+    const int hs = a.head_size, kvd = a.nkv * hs, half = hs / 2, per = (a.nh + a.nkv) * half, n_p = (per + 255) / 256; // pairs of a token, CTAs for them
+    const int64_t slot0 = a.base >= 0 ? a.base : (int64_t)a.pos[0];
+    if ((int)blockIdx.x < n_p * a.bs) {
+        const int i = blockIdx.x / n_p, t = blockIdx.x % n_p * 256 + threadIdx.x, h = t / half, p = t % half;
+        if (t >= per) return;
+        const float *cache = a.table + (int64_t)a.pos[i] * hs;
+        if (h < a.nh) {
+            const int64_t at = ((int64_t)i * a.nh + h) * hs;
+            const PsPair v = ps_rope_pair(a.q + at, p, a.n_dims, a.neox, cache);
+            a.qr[at + v.a] = v.ya;
+            a.qr[at + v.b] = v.yb;
+            return;
+        }
+        const int64_t e = (int64_t)(h - a.nh) * hs, at = (int64_t)i * kvd + e;
+        const PsPair v = ps_rope_pair(a.k + at, p, a.n_dims, a.neox, cache);
+        float *d = (a.kc_ptrs ? a.kc_ptrs[i] + (int64_t)a.pos[i] * kvd : a.kc + (slot0 + i) * kvd) + e;
+        d[v.a] = v.ya;
+        d[v.b] = v.yb;
+        if (a.k_stage) {
+            a.k_stage[at + v.a] = v.ya;
+            a.k_stage[at + v.b] = v.yb;
+        }
+        return;
     }
+    __shared__ float tile[32][33];
+    const int b = blockIdx.x - n_p * a.bs, n_e = (kvd + 31) / 32, e0 = b % n_e * 32, i0 = b / n_e * 32, c = threadIdx.x & 31, r = threadIdx.x >> 5;
+    for (int i = r; i < 32; i += 8)
+        if (i0 + i < a.bs && e0 + c < kvd) {
+            const int64_t at = (int64_t)(i0 + i) * kvd + e0 + c;
+            tile[i][c] = a.v[at];
+            if (a.v_stage) a.v_stage[at] = a.v[at];
+        }
+    __syncthreads();
+    if (i0 + c >= a.bs) return;
+    float *vt = a.vct_ptrs ? a.vct_ptrs[i0 + c] + a.pos[i0 + c] : a.vct + slot0 + i0 + c;
+    for (int e = r; e < 32; e += 8)
+        if (e0 + e < kvd) vt[(e0 + e) * a.n_ctx] = tile[c][e];
 }
 
 // ---- speculative decode: the KV cache as KVCacheInterface sees it (src/core/kv_cache.hpp:97-276) - cache
 // SLOTS decoupled from token positions, a per-slot mask, and the last batch's K / V kept aside for `copy`.
-// KV store of a batch at cache slots base .. base + bs - 1 (save_tokens) + a copy into the per-layer staging rows
-__global__ void ps_k_kv_store_at(float *__restrict__ kc, float *__restrict__ vct, float *__restrict__ k_stage, float *__restrict__ v_stage,
-                                 const float *__restrict__ k, const float *__restrict__ v, int64_t kv_dim, int64_t n_ctx, int64_t base, int64_t bs) {
-    const int64_t total = kv_dim * bs;
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t i = t / kv_dim, e = t % kv_dim;
-        kc[(base + i) * kv_dim + e] = k[t];
-        vct[e * n_ctx + base + i] = v[t];
-        k_stage[t] = k[t];
-        v_stage[t] = v[t];
-    }
-}
 // KVCacheInterface::copy (kv_cache.hpp:120-127, 188-203): token `src` of the last batch -> cache slot `dst`, every layer.
 // kv = [2 * n_layers] device pointers (K caches, then transposed V caches); stage = [n_layers][max_batch][kv_dim] x 2.
 __global__ void ps_k_kv_copy_slot(float *const *__restrict__ kv, int n_layers, const float *__restrict__ k_stage, const float *__restrict__ v_stage,
@@ -1294,19 +1370,10 @@ __global__ void __launch_bounds__(128) ps_k_matmul_f32(float *__restrict__ dst, 
 // Server-side batching: one token of each of n independent SESSIONS per forward pass.  The weight
 // products run once for the n columns (one weight stream); attention is per column over that session's OWN cache at its OWN
 // position.  Column `c` = blockIdx.z; kc_ptrs / vct_ptrs hold the session's cache of the current layer, pos[c] its
-// position.  The arithmetic of every column is that of the bs = 1 operator-table kernels above (ps_k_kv_store,
+// position.  The arithmetic of every column is that of the bs = 1 operator-table kernels above (ps_k_rope,
 // ps_k_attn_scores, ps_k_softmax_ext with the position mask, ps_k_attn_pv), so a session's result does not depend on which
 // other sessions share the batch.
 // ====================================================================================================================
-__global__ void ps_k_sess_kv_store(float *const *__restrict__ kc_ptrs, float *const *__restrict__ vct_ptrs, const float *__restrict__ k,
-                                   const float *__restrict__ v, int64_t kv_dim, int64_t n_ctx, const int32_t *__restrict__ pos, int n) {
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < kv_dim * n; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = t / kv_dim, e = t % kv_dim, p = pos[c];
-        kc_ptrs[c][p * kv_dim + e] = k[t];
-        vct_ptrs[c][e * n_ctx + p] = v[t];
-    }
-}
-
 // scores of column c: kq_c {n_kv_c, 1, n_heads} at kq + c * col_stride; one warp per (cache position, kv head), HB heads of the group at a time
 template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q, int hs,
                                                         int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t col_stride) {
