@@ -424,8 +424,14 @@ int matmul_ob(ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int 
     PsMbArgs a{};
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
     a.n_seg = n_seg; a.bs = (int)bs; a.K = K; a.aqs = ctx->aqs; a.ad = ctx->ad; a.residual = residual; a.err = ctx->tc_err_dev; a.give_up = ctx->opt_give_up;
-    if (ctx->mv_type == 2) return bs <= 2 ? launch_mo<2, 2>(ctx, a, done) : bs <= 4 ? launch_mo<2, 4>(ctx, a, done) : launch_mo<2, 8>(ctx, a, done);
-    return bs <= 2 ? launch_mo<8, 2>(ctx, a, done) : bs <= 4 ? launch_mo<8, 4>(ctx, a, done) : launch_mo<8, 8>(ctx, a, done);
+    // eight columns a warp; four where octets x groups of eight leave a scheduler fewer than two warps: the blocks of a row are a chain, and a warp alone waits for
+    // most of a step (896 rows on 32 columns, K 896 / 4864: 14.8 / 30.5 us with eight, 11.8 / 25.2 with four, 10.7 / 31.3 with two; 1152 rows 11.2, 9.6, 10.1;
+    // 9728 rows 32.3, 39.8, 53.7.  A row a thread and two warps an octet instead: 13.5 / 25.7 with eight columns, 11.3 / 24.5 with four)
+    int64_t walks = 0;
+    for (int t = 0; t < n_seg; t++) walks += (segs[t].n + 7) / 8;
+    const int C = bs <= 2 ? 2 : bs <= 4 || walks * ((bs + 7) / 8) < 8 * ctx->n_sm ? 4 : 8;
+    if (ctx->mv_type == 2) return C == 2 ? launch_mo<2, 2>(ctx, a, done) : C == 4 ? launch_mo<2, 4>(ctx, a, done) : launch_mo<2, 8>(ctx, a, done);
+    return C == 2 ? launch_mo<8, 2>(ctx, a, done) : C == 4 ? launch_mo<8, 4>(ctx, a, done) : launch_mo<8, 8>(ctx, a, done);
 }
 
 int grid1d(int64_t n, int block = 256) { return (int)std::min<int64_t>((n + block - 1) / block, 148 * 8); }
