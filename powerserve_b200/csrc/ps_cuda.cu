@@ -2123,16 +2123,18 @@ static int launch_batch_pv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int
         static bool pv_attr[64] = {};
         if (!pv_attr[ctx->device]) {
             PS_CK(cudaFuncSetAttribute(ps_k_attn_pv_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            PS_CK(cudaFuncSetAttribute(ps_k_attn_pv_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            for (const auto k : {ps_k_attn_pv_tile<true, 4>, ps_k_attn_pv_tile<true, 6>, ps_k_attn_pv_tile<false, 4>}) PS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
             pv_attr[ctx->device] = true;
         }
         dim3 grid((unsigned)((bs + PS_PV_QB - 1) / PS_PV_QB), (unsigned)nh);
         const dim3 grid1 = grid;
-        const bool tile = ctx->opt_attn_tile && hs % PS_PVT_D == 0 && PS_PVT_RING + (size_t)PS_PVT_Q * n_kv * 4 <= 200 * 1024;
+        const bool tile = ctx->opt_attn_tile && hs % PS_PVT_D == 0 && PS_PVT_RING(4) + (size_t)PS_PVT_Q * n_kv * 4 <= 200 * 1024;
         if (tile)
             while ((int)(grid.x * grid.y * grid.z) * 2 <= ctx->n_sm * 2 && (int)grid.z * 2 * 8 * PS_PVT_D <= hs) grid.z *= 2; // narrow batch: split the dim groups over more CTAs
         static_assert(PS_PV_QB == PS_PVT_Q, "both P.V kernels block the queries by 8");
-        if (tile) ps_k_attn_pv_tile<<<grid, 256, PS_PVT_RING + (size_t)PS_PVT_Q * n_kv * 4, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
+        const bool vec = n_ctx % 4 == 0 && ((uintptr_t)ctx->vct[L] & 15) == 0, deep = vec && PS_PVT_RING(6) + (size_t)PS_PVT_Q * n_kv * 4 <= 112 * 1024; // (two CTAs an SM)
+        const auto pv = deep ? ps_k_attn_pv_tile<true, 6> : vec ? ps_k_attn_pv_tile<true, 4> : ps_k_attn_pv_tile<false, 4>;
+        if (tile) pv<<<grid, 256, (deep ? PS_PVT_RING(6) : PS_PVT_RING(4)) + (size_t)PS_PVT_Q * n_kv * 4, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
         else ps_k_attn_pv_batch<<<grid1, 256, (size_t)PS_PV_QB * n_kv * 4, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
     } else {
         ps_k_attn_pv<<<dim3((unsigned)((hs + 3) / 4), (unsigned)nkv), 128, 0, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);

@@ -9,6 +9,14 @@
 
 #define PS_FULL 0xffffffffu
 
+// two packed floats: one instruction for two results, rounded like the single ones
+typedef unsigned long long ps_f2;
+PS_D ps_f2 ps_f2_pack(float a, float b) { ps_f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+PS_D void ps_f2_unpack(ps_f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+PS_D ps_f2 ps_f2_mul(ps_f2 a, ps_f2 b) { ps_f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+PS_D ps_f2 ps_f2_add(ps_f2 a, ps_f2 b) { ps_f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+PS_D ps_f2 ps_f2_fma(ps_f2 a, ps_f2 b, ps_f2 c) { ps_f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
 // ggml block sizes in bytes (libs/ggml/src/ggml-common.h:158-162, 200-204, 299-310, 335-340)
 #define PS_Q4_0_BYTES 18
 #define PS_Q8_0_BYTES 34
@@ -1188,23 +1196,30 @@ PS_D void ps_rs_stage(float (&a)[N], bool up, int mask) {
 
 #define PS_PVT_Q 8 // queries per CTA
 #define PS_PVT_D 8 // output dims per warp tile
-#define PS_PVT_DEPTH 4 // V^T chunks in flight per warp (cp.async ring in shared memory: no registers held by loads in flight)
-#define PS_PVT_RING (8 * PS_PVT_DEPTH * PS_PVT_D * 32 * 4) // bytes: 8 warps x depth x 8 rows x 32 positions
+#define PS_PVT_RING(DEPTH) (8 * (DEPTH) * PS_PVT_D * 32 * 4) // bytes: 8 warps x depth (cp.async ring: no registers held by loads in flight) x 8 rows x 32 positions
 PS_D void ps_cp_async4(float *dst_smem, const float *src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src) : "memory");
+}
+PS_D void ps_cp_async16(float *dst_smem, const float *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst_smem)), "l"(src) : "memory");
 }
 PS_D void ps_cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> PS_D void ps_cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// VEC: rows of V^T start on 16-byte lines (n_ctx a multiple of four), so a warp fetches a chunk with two copies of 16 bytes a lane; by words it
+// takes eight, which cost shared memory more than everything else in the loop; pairs of queries are packed floats.  DEPTH chunks of a row are on their way:
+// a chunk takes a warp about 200 cycles, memory about 800.  32 heads x 128 queries x 2048 keys, head size 128: 107 us by words, 92 by lines and
+// pairs and four chunks; a pass of two such layers 1108 -> 1082 us with pairs and six
+template <bool VEC, int DEPTH>
 __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ out, const float *__restrict__ vct, const float *__restrict__ p,
                                                             int hs, int n_heads, int n_kv_heads, int64_t n_kv, int64_t n_ctx, int bs) {
-    // [ring: 8 warps][PS_PVT_DEPTH][PS_PVT_D][32] V^T chunks, then the probabilities, position-major: s_p4[j] = queries 0..3
+    // [ring: 8 warps][DEPTH][PS_PVT_D][32] V^T chunks, then the probabilities, position-major: s_p4[j] = queries 0..3
     // at position j, s_p4[n_kv + j] = queries 4..7, so a lane fetches its eight probabilities of a chunk with two
     // conflict-free 16-byte loads off one address register
     extern __shared__ __align__(16) float4 s_pvt[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    float *ring = reinterpret_cast<float *>(s_pvt) + warp * (PS_PVT_DEPTH * PS_PVT_D * 32) + lane; // every lane reads back only what it copied itself
-    float4 *s_p4 = s_pvt + PS_PVT_RING / 16;
+    float *const ring = reinterpret_cast<float *>(s_pvt) + warp * (DEPTH * PS_PVT_D * 32);
+    float4 *s_p4 = s_pvt + PS_PVT_RING(DEPTH) / 16;
     const int i0 = blockIdx.x * PS_PVT_Q, h = blockIdx.y, g = h / (n_heads / n_kv_heads);
     const int nq = min(PS_PVT_Q, bs - i0);
     const int nkv = (int)n_kv;
@@ -1212,19 +1227,25 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
     const int np = nc << 5;
     // hs is a multiple of PS_PVT_D (launch condition); gridDim.z CTAs share the dim groups of a (query block, head) when the batch is narrow
     const int d_first = ((int)blockIdx.z * 8 + warp) * PS_PVT_D, d_step = (int)gridDim.z * 8 * PS_PVT_D;
-    const float *vp[PS_PVT_D]; // one running pointer per V^T row: the copies below only add immediates
-    auto issue = [&](bool in, int slot, int off) { // a chunk of the current dim group -> ring slot (always one group per call, possibly empty)
-        if (in) {
+    constexpr int ROWS = VEC ? 4 : 1, NV = PS_PVT_D / ROWS;   // rows a copy instruction covers
+    const float *vp = nullptr; // this lane's word (VEC: four words, of row lane / 8) of the group's first row
+    auto start = [&](int d0) { vp = vct + ((int64_t)g * hs + d0 + (VEC ? lane >> 3 : 0)) * n_ctx + (VEC ? (lane & 7) * 4 : lane); };
+    auto issue = [&](int c, int slot) { // chunk c of the current dim group -> a ring slot (always one group per call, possibly empty)
+        if (c < nc) {
+            float *to = ring + slot * (PS_PVT_D * 32) + (VEC ? (lane >> 3) * 32 + (lane & 7) * 4 : lane);
 #pragma unroll
-            for (int di = 0; di < PS_PVT_D; di++) ps_cp_async4(ring + (slot * PS_PVT_D + di) * 32, vp[di] + off);
+            for (int k = 0; k < NV; k++) {
+                const float *from = vp + (int64_t)(k * ROWS) * n_ctx + 32 * c;
+                if (VEC) ps_cp_async16(to + k * ROWS * 32, from);
+                else ps_cp_async4(to + k * ROWS * 32, from);
+            }
         }
         ps_cp_async_commit();
     };
     if (d_first < hs) { // the first dim group's V^T chunks are on their way while the probabilities are staged
+        start(d_first);
 #pragma unroll
-        for (int di = 0; di < PS_PVT_D; di++) vp[di] = vct + ((int64_t)g * hs + d_first + di) * n_ctx + lane;
-#pragma unroll
-        for (int k = 0; k < PS_PVT_DEPTH - 1; k++) issue(k < nc, k, 32 * k);
+        for (int k = 0; k < DEPTH - 1; k++) issue(k, k);
     }
     {
         const float *pr = p + ((int64_t)h * bs + i0) * n_kv;
@@ -1238,40 +1259,40 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
     }
     __syncthreads();
     for (int d0 = d_first; d0 < hs; d0 += d_step) {
-        const float4 *sp = s_p4 + lane;
-        float acc[PS_PVT_D * PS_PVT_Q]; // [di][qi]
+        const ulonglong2 *sp = reinterpret_cast<const ulonglong2 *>(s_p4) + lane;
+        ps_f2 acc2[PS_PVT_D][PS_PVT_Q / 2]; // [di][pair of queries]
 #pragma unroll
-        for (int k = 0; k < PS_PVT_D * PS_PVT_Q; k++) acc[k] = 0.f;
-        for (int c0 = 0; c0 < nc; c0 += PS_PVT_DEPTH) {
+        for (int di = 0; di < PS_PVT_D; di++)
 #pragma unroll
-            for (int k = 0; k < PS_PVT_DEPTH; k++) {
-                const int c = c0 + k;
-                if (c < nc) { // warp-uniform
-                    issue(c + PS_PVT_DEPTH - 1 < nc, (k + PS_PVT_DEPTH - 1) % PS_PVT_DEPTH, 32 * (k + PS_PVT_DEPTH - 1)); // refills the slot consumed one chunk ago
-                    ps_cp_async_wait<PS_PVT_DEPTH - 1>();                                // chunk c has landed
-                    float v[PS_PVT_D];
+            for (int k = 0; k < PS_PVT_Q / 2; k++) acc2[di][k] = 0ull;
+        int slot = 0;
+#pragma unroll 2
+        for (int c = 0; c < nc; c++) {
+            ps_cp_async_wait<DEPTH - 2>(); // chunk c has landed: this lane's part, then everyone's, and the chunk before has been read
+            __syncwarp();
+            issue(c + DEPTH - 1, slot == 0 ? DEPTH - 1 : slot - 1); // into the slot of the chunk before
+            const float *rv = ring + slot * (PS_PVT_D * 32) + lane;
+            slot = slot + 1 == DEPTH ? 0 : slot + 1;
+            const ulonglong2 lo = sp[32 * c], hi = sp[nkv + 32 * c];
+            const ps_f2 pp[PS_PVT_Q / 2] = {lo.x, lo.y, hi.x, hi.y};
 #pragma unroll
-                    for (int di = 0; di < PS_PVT_D; di++) v[di] = ring[(k * PS_PVT_D + di) * 32];
-                    const float4 lo = sp[32 * k], hi = sp[nkv + 32 * k];
-                    const float pp[PS_PVT_Q] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+            for (int di = 0; di < PS_PVT_D; di++) {
+                const float v = rv[di * 32];
+                const ps_f2 v2 = ps_f2_pack(v, v);
 #pragma unroll
-                    for (int di = 0; di < PS_PVT_D; di++)
-#pragma unroll
-                        for (int qi = 0; qi < PS_PVT_Q; qi++) acc[di * PS_PVT_Q + qi] = __fmaf_rn(v[di], pp[qi], acc[di * PS_PVT_Q + qi]);
-                }
+                for (int k = 0; k < PS_PVT_Q / 2; k++) acc2[di][k] = ps_f2_fma(v2, pp[k], acc2[di][k]);
             }
-#pragma unroll
-            for (int di = 0; di < PS_PVT_D; di++) vp[di] += 32 * PS_PVT_DEPTH;
-            sp += 32 * PS_PVT_DEPTH;
         }
         ps_cp_async_wait<0>();
+        __syncwarp();
         if (d0 + d_step < hs) { // next dim group of this warp: its first chunks fly during the reduction below
-            const int64_t adv = (int64_t)d_step * n_ctx - (int64_t)((nc + PS_PVT_DEPTH - 1) / PS_PVT_DEPTH) * (32 * PS_PVT_DEPTH);
+            start(d0 + d_step);
 #pragma unroll
-            for (int di = 0; di < PS_PVT_D; di++) vp[di] += adv;
-#pragma unroll
-            for (int k = 0; k < PS_PVT_DEPTH - 1; k++) issue(k < nc, k, 32 * k);
+            for (int k = 0; k < DEPTH - 1; k++) issue(k, k);
         }
+        float acc[PS_PVT_D * PS_PVT_Q]; // [di][qi]
+#pragma unroll
+        for (int k = 0; k < PS_PVT_D * PS_PVT_Q / 2; k++) ps_f2_unpack(acc2[k / 4][k % 4], acc[2 * k], acc[2 * k + 1]);
         // GGML_F32x8_REDUCE as a reduce-scatter: 64 sums -> 2 per lane.  Flat index = qi + 8 * di; the stages peel index
         // bits 5, 4, 3 (lane bits 4, 3, 2), then bit 2 (lane bit 0, stage xor 1) and bit 1 (lane bit 1, stage xor 2).
         ps_rs_stage<64>(acc, lane & 16, 16);

@@ -206,13 +206,6 @@ struct PsTcArgs {
     uint32_t limit;     // cycles a wait lasts at most
 };
 
-typedef unsigned long long ps_f2; // two packed floats
-PS_D ps_f2 ps_f2_pack(float a, float b) { ps_f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-PS_D void ps_f2_unpack(ps_f2 v, float &a, float &b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-PS_D ps_f2 ps_f2_mul(ps_f2 a, ps_f2 b) { ps_f2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-PS_D ps_f2 ps_f2_add(ps_f2 a, ps_f2 b) { ps_f2 r; asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-PS_D ps_f2 ps_f2_fma(ps_f2 a, ps_f2 b, ps_f2 c) { ps_f2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
-
 // eight columns of one row of an accumulator; they are there after ps_tc_ld_wait, and ps_tc_pass keeps whatever reads them behind it
 PS_D void ps_tc_ld(uint32_t taddr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
