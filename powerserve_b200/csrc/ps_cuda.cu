@@ -2200,13 +2200,14 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         if (sess) { // every column attends over its own session's cache at its own position
             float **pl = ctx->sess_ptrs_dev + (size_t)L * 2 * d.max_batch;
             const int64_t cs = nh * (int64_t)d.n_ctx;
-            const auto scores = nh / nkv == 1 ? ps_k_sess_scores<1> : nh / nkv == 2 ? ps_k_sess_scores<2> : ps_k_sess_scores<4>;
-            scores<<<dim3((unsigned)((n_kv + 3) / 4), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->stream>>>(ctx->kq, pl, ctx->qr, (int)hs, (int)nh, (int)nkv, ctx->pos_dev, cs);
+            static void (*const scores[])(float *, const float *const *, const float *, int, int, const int32_t *, int64_t) = {
+                ps_k_sess_scores<1>, ps_k_sess_scores<2>, ps_k_sess_scores<3>, ps_k_sess_scores<4>, ps_k_sess_scores<5>, ps_k_sess_scores<6>, ps_k_sess_scores<7>, ps_k_sess_scores<8>};
+            scores[hs / 32 - 1]<<<dim3((unsigned)((n_kv + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->stream>>>(ctx->kq, pl, ctx->qr, (int)nh, (int)nkv, ctx->pos_dev, cs);
             PS_LAUNCH_CK();
             ps_k_sess_softmax<<<dim3((unsigned)nh, (unsigned)bs), 256, (size_t)n_kv * 4, ctx->stream>>>(ctx->kq, ctx->pos_dev, cs, kq_scale);
             PS_LAUNCH_CK();
             const auto pv = nh / nkv == 1 ? ps_k_sess_pv<1> : nh / nkv == 2 ? ps_k_sess_pv<2> : ps_k_sess_pv<4>;
-            pv<<<dim3((unsigned)((hs + 3) / 4), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->stream>>>(ctx->att, pl + d.max_batch, ctx->kq, (int)hs, (int)nh, (int)nkv, ctx->pos_dev, d.n_ctx, cs);
+            pv<<<dim3((unsigned)((hs + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->stream>>>(ctx->att, pl + d.max_batch, ctx->kq, (int)hs, (int)nh, (int)nkv, ctx->pos_dev, d.n_ctx, cs);
             PS_LAUNCH_CK();
         } else {
         launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs);

@@ -1395,27 +1395,46 @@ __global__ void __launch_bounds__(128) ps_k_matmul_f32(float *__restrict__ dst, 
 // ps_k_attn_scores, ps_k_softmax_ext with the position mask, ps_k_attn_pv), so a session's result does not depend on which
 // other sessions share the batch.
 // ====================================================================================================================
-// scores of column c: kq_c {n_kv_c, 1, n_heads} at kq + c * col_stride; one warp per (cache position, kv head), HB heads of the group at a time
-template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q, int hs,
-                                                        int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t col_stride) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z, g = blockIdx.y;
-    const int64_t n_kv = (int64_t)pos[c] + 1, j = (int64_t)blockIdx.x * 4 + warp;
-    if (j >= n_kv) return;
-    const int r2 = n_heads / n_kv_heads, steps = hs / 32;
-    const float *krow = kc_ptrs[c] + j * (int64_t)(hs * n_kv_heads) + g * hs;
-    float kv[8];
+// scores of column c: kq_c {n_kv_c, 1, n_heads} at kq + c * col_stride; a warp takes eight cache rows of a kv head against every query head of the group,
+// its sums reduced as in ps_k_attn_scores_tile (a warp a row: 20 shuffles and as many loads for four numbers; 64 sessions of 100 to 200 positions, a layer
+// of 32 query and 8 kv heads: 47.6 us; with P.V below 94 a layer, now about 39)
+template <int STEPS> __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q,
+                                                                           int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t col_stride) {
+    constexpr int hs = 32 * STEPS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z, g = blockIdx.y, code = lane >> 2;
+    const int64_t n_kv = (int64_t)pos[c] + 1, j0 = ((int64_t)blockIdx.x * 4 + warp) * 8;
+    if (j0 >= n_kv) return;
+    const int r2 = n_heads / n_kv_heads;
+    const float *base = kc_ptrs[c] + g * hs + lane;
+    float kv[8][STEPS]; // slot t: row t ^ code of the eight
 #pragma unroll
-    for (int s = 0; s < 8; s++) kv[s] = (s < steps) ? krow[32 * s + lane] : 0.f;
-#pragma unroll HB
+    for (int t = 0; t < 8; t++) {
+        const int64_t j = j0 + (t ^ code);
+#pragma unroll
+        for (int s = 0; s < STEPS; s++) kv[t][s] = j < n_kv ? base[j * (int64_t)(hs * n_kv_heads) + 32 * s] : 0.f;
+    }
+    const bool writer = (lane & 3) == 0 && j0 + code < n_kv;
+    const float *qv = q + ((int64_t)c * n_heads + g * r2) * hs + lane;
+    float *dst = kq + c * col_stride + (int64_t)(g * r2) * n_kv + j0 + code;
+#pragma unroll 2
     for (int hh = 0; hh < r2; hh++) {
-        const int h = g * r2 + hh;
-        const float *qv = q + ((int64_t)c * n_heads + h) * hs;
-        float sum = 0.f;
+        float qe[STEPS], sum[8];
 #pragma unroll
-        for (int s = 0; s < 8; s++)
-            if (s < steps) sum = __fmaf_rn(kv[s], qv[32 * s + lane], sum); // ggml_vec_dot_f32 lane chain
-        sum = ps_f32x8_reduce(sum);
-        if (lane == 0) kq[c * col_stride + (int64_t)h * n_kv + j] = sum;
+        for (int s = 0; s < STEPS; s++) qe[s] = qv[hh * hs + 32 * s];
+#pragma unroll
+        for (int t = 0; t < 8; t++) {
+            sum[t] = 0.f;
+#pragma unroll
+            for (int s = 0; s < STEPS; s++) sum[t] = __fmaf_rn(kv[t][s], qe[s], sum[t]); // ggml_vec_dot_f32 lane chain
+        }
+#pragma unroll
+        for (int t = 0; t < 4; t++) sum[t] = __fadd_rn(sum[t], __shfl_xor_sync(PS_FULL, sum[t + 4], 16));
+#pragma unroll
+        for (int t = 0; t < 2; t++) sum[t] = __fadd_rn(sum[t], __shfl_xor_sync(PS_FULL, sum[t + 2], 8));
+        sum[0] = __fadd_rn(sum[0], __shfl_xor_sync(PS_FULL, sum[1], 4));
+        sum[0] = __fadd_rn(sum[0], __shfl_xor_sync(PS_FULL, sum[0], 1));
+        sum[0] = __fadd_rn(sum[0], __shfl_xor_sync(PS_FULL, sum[0], 2));
+        if (writer) dst[(int64_t)hh * n_kv] = sum[0];
     }
 }
 
@@ -1461,44 +1480,73 @@ __global__ void __launch_bounds__(256) ps_k_sess_softmax(float *__restrict__ kq,
     for (int64_t j = threadIdx.x; j < ne0; j += blockDim.x) dp[j] = __fmul_rn(dp[j], inv);
 }
 
-// P.V of column c: out[c][h * hs + d]; one warp per (kv head g, d), which takes HB of the group's heads at a time
+// P.V of column c: out[c][h * hs + d]; a warp takes eight dims of a kv head and HB of the group's heads at a time (four, two or one where the group has no
+// more: an absent head costs as much as a present one).  A chunk of 32 positions is eight rows of V and HB of weights for 8 HB products; with a dim a warp
+// the weights were read 128 times over and every sum took five shuffles (64 sessions of 100 to 200 positions, a layer of 32 query and 8 kv heads: 46.6 us).  After the reduction lane (dim, head) owns one sum and adds the leftover products to it in order
 template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, const float *const *__restrict__ vct_ptrs, const float *__restrict__ kq, int hs,
                                                     int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t n_ctx, int64_t col_stride) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z;
-    const int d = blockIdx.x * 4 + warp, g = blockIdx.y;
-    if (d >= hs) return;
+    __shared__ float s_left[4][8 + HB][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z, g = blockIdx.y, d0 = (blockIdx.x * 4 + warp) * 8;
+    if (d0 >= hs) return; // (hs is a multiple of eight)
     const int r2 = n_heads / n_kv_heads;
     const int64_t n_kv = (int64_t)pos[c] + 1, np = n_kv & ~(int64_t)31;
     const int rem = (int)(n_kv - np);
-    const float *vrow = vct_ptrs[c] + ((int64_t)g * hs + d) * n_ctx;
-    // Bound by memory latency.  HB heads of the group share a V row and their loads are in flight together; the leftover products are formed
-    // by the lanes and only their additions run one after the other (one head at a time, with lane 0 loading every leftover itself,
-    // 64 sessions of 100 to 200 positions took 75 us a layer of an 8B model).  Four heads at a time, two or one where the group has no more: an absent
-    // head costs as much as a present one (64 sessions of 500 positions, a layer of 32 query and 32 kv heads: 805 us with four, 658 with one, 770
-    // with the loads of each head in turn)
+    const float *vrow = vct_ptrs[c] + ((int64_t)g * hs + d0) * n_ctx + lane;
     for (int h0 = 0; h0 < r2; h0 += HB) {
         const float *pr[HB];
-        float sum[HB], left[HB];
+        float sum[8 * HB]; // [dim][head]
 #pragma unroll
-        for (int t = 0; t < HB; t++) { pr[t] = kq + c * col_stride + (int64_t)(g * r2 + min(h0 + t, r2 - 1)) * n_kv; sum[t] = 0.f; }
-        const float vl = lane < rem ? vrow[np + lane] : 0.f;
+        for (int t = 0; t < HB; t++) pr[t] = kq + c * col_stride + (int64_t)(g * r2 + min(h0 + t, r2 - 1)) * n_kv + lane;
 #pragma unroll
-        for (int t = 0; t < HB; t++) left[t] = lane < rem ? __fmul_rn(vl, pr[t][np + lane]) : 0.f;
-#pragma unroll (HB == 4 ? 2 : 4)
+        for (int k = 0; k < 8 * HB; k++) sum[k] = 0.f;
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 8 + HB; k++) s_left[warp][k][lane] = lane < rem ? (k < 8 ? vrow[k * n_ctx + np] : pr[k < 8 ? 0 : k - 8][np]) : 0.f;
+#pragma unroll 2
         for (int64_t s = 0; s < np; s += 32) {
-            const float v = vrow[s + lane];
+            float v[8], w[HB];
 #pragma unroll
-            for (int t = 0; t < HB; t++) sum[t] = __fmaf_rn(v, pr[t][s + lane], sum[t]);
+            for (int k = 0; k < 8; k++) v[k] = vrow[k * n_ctx + s];
+#pragma unroll
+            for (int t = 0; t < HB; t++) w[t] = pr[t][s];
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+#pragma unroll
+                for (int t = 0; t < HB; t++) sum[k * HB + t] = __fmaf_rn(v[k], w[t], sum[k * HB + t]);
         }
+        // GGML_F32x8_REDUCE as a reduce-scatter: lane bits 4, 3, 2 keep the dim, then (stages xor 1, xor 2) bits 0 and 1 the head
+        ps_rs_stage<8 * HB>(sum, lane & 16, 16);
+        float a4[4 * HB], a2[2 * HB], a1[HB];
 #pragma unroll
-        for (int t = 0; t < HB; t++) sum[t] = ps_f32x8_reduce(sum[t]);
-        for (int j = 0; j < rem; j++) // leftovers: mul, then add
+        for (int k = 0; k < 4 * HB; k++) a4[k] = sum[k];
+        ps_rs_stage<4 * HB>(a4, lane & 8, 8);
 #pragma unroll
-            for (int t = 0; t < HB; t++) sum[t] = __fadd_rn(sum[t], __shfl_sync(PS_FULL, left[t], j));
-        if (lane == 0)
+        for (int k = 0; k < 2 * HB; k++) a2[k] = a4[k];
+        ps_rs_stage<2 * HB>(a2, lane & 4, 4);
 #pragma unroll
-            for (int t = 0; t < HB; t++)
-                if (h0 + t < r2) out[((int64_t)c * n_heads + g * r2 + h0 + t) * hs + d] = sum[t];
+        for (int t = 0; t < HB; t++) a1[t] = a2[t];
+        float r = a1[0];
+        int mine = 0;
+        if (HB == 4) {
+            ps_rs_stage<HB>(a1, lane & 1, 1);
+            float b[2] = {a1[0], a1[1 % HB]};
+            ps_rs_stage<2>(b, lane & 2, 2);
+            r = b[0];
+            mine = 2 * (lane & 1) + ((lane >> 1) & 1);
+        } else {
+            if (HB == 2) {
+                ps_rs_stage<HB>(a1, lane & 1, 1);
+                r = a1[0];
+                mine = lane & 1;
+            } else {
+                r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 1));
+            }
+            r = __fadd_rn(r, __shfl_xor_sync(PS_FULL, r, 2));
+        }
+        __syncwarp();
+        const float *lv = s_left[warp][lane >> 2], *lp = s_left[warp][8 + mine];
+        for (int j = 0; j < rem; j++) r = __fadd_rn(r, __fmul_rn(lv[j], lp[j])); // leftovers: mul, then add, in order
+        if (h0 + mine < r2 && (HB == 4 || (lane & (HB == 2 ? 2 : 3)) == 0)) out[((int64_t)c * n_heads + g * r2 + h0 + mine) * hs + d0 + (lane >> 2)] = r;
     }
 }
 
