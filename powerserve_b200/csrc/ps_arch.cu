@@ -1144,7 +1144,8 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
 // 2048 in turn: 48 tiles of 64 rows 104 us, 80 of 32 rows 81 us; with more tiles than SMs the wider tile reads its operands less often).
 // K is cut where the rows of the weights alone give few tiles: by the weights' shape only, so that a token's sums do not depend on its batch.  One tile of
 // tokens then makes up to four CTAs an SM (2 layers of 1024 / 1536 / 2048 wide models on 48 tokens: uncut 737 / 1061 / 1339 us, one CTA an SM 418 / 644 /
-// 943, two 392 / 544 / 740, four 393 / 510 / 653); a cut keeps 128 k or more, since the sums travel through the cluster's shared memory (about 2 us)
+// 943, two 392 / 544 / 740, four 393 / 510 / 653); a cut keeps 128 k or more, since the sums travel through the cluster's shared memory (about 2 us).
+// Float32 mode alone: in bfloat16 mode what these kernels do (per-head products, gates) leads into rounded operands and keeps its one order of k
 static int pa_cuts(int64_t N, int K) {
     int S = 1;
     while (S < 8 && 2 * S * N <= 4 * 148 * PA_TN && K >= 2 * S * 128) S *= 2;
@@ -1163,11 +1164,11 @@ static cudaError_t pa_launch_cut(int S, void (*kern)(KArgs...), dim3 grid, cudaS
     cfg.numAttrs = S > 1 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, (KArgs)args...);
 }
-template <bool ROUND>
+template <bool ROUND, bool CUT = !ROUND>
 static void pa_launch_linear(int n_sm, int N, int bs, int heads, cudaStream_t st, const float *A, int lda, const bf16 *W, const float *bias, float *C, int ldc, int M, int n, int K,
                              int a_gs = 0, int c_gs = 0, int act_from = 1 << 30, int gap = 0, PaAct act = PaAct{}, PaRowMul mul = PaRowMul{}) {
     const unsigned nt = (unsigned)((N + PA_TN - 1) / PA_TN);
-    const int S = pa_cuts((int64_t)nt * PA_TN * heads, K);
+    const int S = CUT ? pa_cuts((int64_t)nt * PA_TN * heads, K) : 1;
     const bool narrow = pa_narrow_tiles(n_sm, (int64_t)nt * PA_TN * heads * S, bs);
     const int tm = narrow ? 32 : PA_TM;
     pa_launch_cut(S, narrow ? pa_k_linear<ROUND, 32> : pa_k_linear<ROUND, PA_TM>, dim3(nt, (unsigned)((bs + tm - 1) / tm), (unsigned)(heads * S)), st, A, lda, W, bias, C, ldc, M, n, K, S,
@@ -1249,7 +1250,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         PA_LAUNCH();
         pa_k_mix_softmax<<<bs, 256, 4 * (size_t)at.H * at.H, st>>>(at, a->S, io.pos_dev, bs);
         PA_LAUNCH();
-        pa_k_pv<<<dim3(cdiv(at.dv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st>>>(at, a->S, io.vct[li], out, aw, io.pos_dev, bs);
+        pa_k_pv<!ROUND><<<dim3(cdiv(at.dv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st>>>(at, a->S, io.vct[li], out, aw, io.pos_dev, bs);
         PA_LAUNCH();
         return 0;
     };
@@ -1340,7 +1341,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     // its first half on the fp32-FMA tiles
     auto dense_up = [&](const float *X, const bf16 *wg, const bf16 *wu, int ff, const PaAct &act) -> int {
         const int64_t rows = (int64_t)cdiv(ff, PA_TN) * PA_TN * (wg ? 2 : 1); // (a gated tile has two products)
-        const int S = pa_cuts(rows, dim);
+        const int S = ROUND ? 1 : pa_cuts(rows, dim);
         const bool narrow = pa_narrow_tiles(a->n_sm, rows * S / (wg ? 2 : 1), bs);
         const dim3 grid(cdiv(ff, PA_TN), cdiv(bs, narrow ? 32 : PA_TM), (unsigned)S);
         if (wg) pa_launch_cut(S, narrow ? pa_k_dense_up<ROUND, 2, 32> : pa_k_dense_up<ROUND, 2, PA_TM>, grid, st, X, dim, wg, wu, a->y, bs, ff, dim, act, S);
@@ -1847,7 +1848,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             } else {
                 pa_k_short_conv<<<dim3(cdiv(g.W, 256), bs), 256, 0, st>>>(g.x, w.ldp, w.conv_w, w.conv_b, g.W, g.taps, g.ring, 0, a->cv, g.W, io.pos_dev, 1);
                 PA_LAUNCH();
-                pa_launch_linear<false>(a->n_sm, 2 * g.bsz, bs, (int)l.rec_blocks, st, a->cv, g.W, w.wri, nullptr, a->gts, 2 * g.W, bs, 2 * g.bsz, g.bsz, g.bsz, 2 * g.bsz);
+                pa_launch_linear<false, !ROUND>(a->n_sm, 2 * g.bsz, bs, (int)l.rec_blocks, st, a->cv, g.W, w.wri, nullptr, a->gts, 2 * g.W, bs, 2 * g.bsz, g.bsz, g.bsz, 2 * g.bsz);
                 PA_LAUNCH();
                 pa_k_rglru_scan<<<cdiv(g.W, 32), PA_GG_THREADS, 0, st>>>(g);
                 PA_LAUNCH();
@@ -1996,7 +1997,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             PA_LAUNCH();
             pa_k_mix_softmax<<<bs, 256, 4 * (size_t)H * H, st>>>(at, a->S, io.pos_dev, bs);
             PA_LAUNCH();
-            pa_k_pv<<<dim3(cdiv(dv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st>>>(at, a->S, io.vct[li], a->att, w.od, io.pos_dev, bs);
+            pa_k_pv<!ROUND><<<dim3(cdiv(dv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st>>>(at, a->S, io.vct[li], a->att, w.od, io.pos_dev, bs);
             PA_LAUNCH();
         }
         if (single) {

@@ -1039,14 +1039,17 @@ __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__rest
 
 // att[i][h * dv + c] = sum_j P[h][i][j] V^T[g * dv + c][j].  With rotated values a tile's 64 columns are 32 pairs (m, m + dv / 2), two pairs to a
 // thread, which turns them back by its query's position; then the head's gate and the factor on the heads' outputs.
-__global__ void __launch_bounds__(256, 2) pa_k_pv(PaAttn at, const float *__restrict__ S, const float *__restrict__ vct, float *__restrict__ att, int od,
+// GROUPS: four groups of threads share the keys of a step (256 queries x 1024 keys x 16 heads 43 -> 36 us).  Not in bfloat16 mode: the heads' outputs are the
+// rounded operand of the next product, where another order of the keys moves logits by 1e-4, and they are to be the same however a prompt is cut
+template <bool GROUPS>
+__global__ void __launch_bounds__(256, GROUPS ? 2 : 3) pa_k_pv(PaAttn at, const float *__restrict__ S, const float *__restrict__ vct, float *__restrict__ att, int od,
                                                const int32_t *__restrict__ pos, int bs) {
-    __shared__ __align__(16) float sm[PaTile<1, PA_TM, true>::N];
+    __shared__ __align__(16) float sm[PaTile<1, PA_TM, GROUPS>::N];
     const int lr = threadIdx.x >> 2;
     const int h = blockIdx.z, g = h / (at.H / at.G), m0 = blockIdx.y * PA_TM, n0 = blockIdx.x * PA_TN;
     const int n_keys = pos[0] + min(m0 + PA_TM, bs); // keys the tile's furthest query sees (the rows are zero beyond their own)
     const int k0 = pa_first_key(at, pos[0] + m0);    // ... and the first key its first query sees (zero before a row's own)
-    PaTile<1, PA_TM, true>::Acc acc = {};
+    typename PaTile<1, PA_TM, GROUPS>::Acc acc = {};
     const float *arow = (m0 + lr < bs) ? S + ((int64_t)h * at.B + m0 + lr) * at.ldS + k0 : nullptr;
     // value dim of the tile's column j (dv or more: outside)
     const int vh = at.vrope.dims >> 1;
@@ -1057,14 +1060,14 @@ __global__ void __launch_bounds__(256, 2) pa_k_pv(PaAttn at, const float *__rest
     };
     const int cb = col(lr);
     const float *brow = (cb < at.dv) ? vct + (int64_t)(g * at.dv + cb) * at.n_ctx + k0 : nullptr;
-    pa_tile_mm<false, float, 1, PA_TM, true>(acc, arow, 1.0f, brow, nullptr, n_keys - k0, sm);
+    pa_tile_mm<false, float, 1, PA_TM, GROUPS>(acc, arow, 1.0f, brow, nullptr, n_keys - k0, sm);
     const int nv = pa_pool_vis(at, n_keys - 1); // pooled blocks of the tile's furthest query: their weights times the mean value rows
     if (nv > 0) {
         const float *arow2 = (m0 + lr < bs) ? S + ((int64_t)h * at.B + m0 + lr) * at.ldS + at.pool_off : nullptr;
         const float *brow2 = (n0 + lr < at.dv) ? vct + (int64_t)at.G * at.dv * at.n_ctx + (int64_t)(g * at.dv + n0 + lr) * at.n_pool : nullptr;
-        pa_tile_mm<false, float, 1, PA_TM, true>(acc, arow2, 1.0f, brow2, nullptr, nv, sm);
+        pa_tile_mm<false, float, 1, PA_TM, GROUPS>(acc, arow2, 1.0f, brow2, nullptr, nv, sm);
     }
-    pa_tile_store<1, PA_TM, true>(acc, sm, [&](int row, int c4, const float4 (&sum)[1]) {
+    pa_tile_store<1, PA_TM, GROUPS>(acc, sm, [&](int row, int c4, const float4 (&sum)[1]) {
         const int m = m0 + row;
         if (m >= bs) return;
         float s4[4] = {sum[0].x, sum[0].y, sum[0].z, sum[0].w};
