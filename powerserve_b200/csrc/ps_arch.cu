@@ -1145,7 +1145,8 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
 // K is cut where the rows of the weights alone give few tiles: by the weights' shape only, so that a token's sums do not depend on its batch.  One tile of
 // tokens then makes up to four CTAs an SM (2 layers of 1024 / 1536 / 2048 wide models on 48 tokens: uncut 737 / 1061 / 1339 us, one CTA an SM 418 / 644 /
 // 943, two 392 / 544 / 740, four 393 / 510 / 653); a cut keeps 128 k or more, since the sums travel through the cluster's shared memory (about 2 us).
-// Float32 mode alone: in bfloat16 mode what these kernels do (per-head products, gates) leads into rounded operands and keeps its one order of k
+// Float32 mode alone: in bfloat16 mode what these kernels do (per-head products, gates) leads into rounded operands and keeps its one order of k.
+// 148 are a B200's SMs; the device's own number would let a GPU with fewer cut, and add, otherwise
 static int pa_cuts(int64_t N, int K) {
     int S = 1;
     while (S < 8 && 2 * S * N <= 4 * 148 * PA_TN && K >= 2 * S * 128) S *= 2;

@@ -145,12 +145,12 @@ __device__ __forceinline__ float pa_act1(float z, PaAct act) {
 // ONE A row and 8 of ONE B row - `arow` points at row tid / (256 / TM) of the tile, `brow` at row tid >> 2 (null = outside: zeros) - by 16-byte loads
 // where the row allows them, and holds the next step's values in registers while this one is computed.
 // Bound by shared memory: a 16-byte read costs four of its cycles, shared addresses or not, so what counts is how many products a thread makes of
-// one.  The threads are G groups that share the k of a step, each with the whole tile: a thread of four groups owns 8 x 8 outputs (32 rows: 4 x 8) and
-// needs a sixteenth of a read per product, where 4 x 4 outputs over all k need an eighth.  The groups' sums meet at the end.
-// It pays for 32-row tiles and long sums: 8 / 48 / 128 tokens of two 1024-wide Vanapel layers in float32 358 / 363 / 428 us with 4 x 4 outputs
-// everywhere, 327 / 338 / 418 now; P.V of 256 queries x 1024 keys x 16 heads 43 -> 36 us.  At 64 rows and short cuts the meeting costs what the reads
-// save (and 128 registers halve the CTAs an SM holds), so those stay with one group of 4 x 4 outputs.  So do rounded operands, whose products the
-// tensor cores make: their sums stay in the order of k
+// one.  GROUPS (P.V in float32 mode): four groups of threads share the k of a step, each with the whole 64 x 64 tile, so that a thread owns 8 x 8 outputs and
+// needs a sixteenth of a read per product, where 4 x 4 outputs over all k need an eighth.  The groups' sums meet at the end: it pays for long sums (256
+// queries x 1024 keys x 16 heads 43 -> 36 us), and not for the short cuts of the dense products at 64 rows (27 -> 39 us, 128 registers halve the CTAs an SM
+// holds).  Nor may 32-row tiles have groups where 64-row ones have none, since the batch decides between the two: one order of k for both, so that a
+// token's sums do not depend on its batch (8 / 48 / 150 tokens of two 1024-wide Vanapel layers in float32: 297 / 319 / 522 us with groups in 32-row tiles,
+// 317 / 335 / 532 without, 300 / 318 / 586 with groups in both)
 __device__ __forceinline__ void pa_fetch8(const float *row, bool vec, int k, int K, float v[8]) {
     if (vec && k + 8 <= K) {
         const float4 x = *reinterpret_cast<const float4 *>(row + k), y = *reinterpret_cast<const float4 *>(row + k + 4);
@@ -308,11 +308,10 @@ template <bool ROUND, int NB, int TM, typename F>
 __device__ __forceinline__ void pa_tile_cut(float *sm, const float *arow, const bf16 *brow0, const bf16 *brow1, int K, int S, F store) {
     const int tid = threadIdx.x, rank = S > 1 ? (int)pa_cluster_rank() : 0;
     const int k0 = pa_cut_begin(K, rank, S), k1 = pa_cut_begin(K, rank + 1, S);
-    constexpr bool GR = TM == 32 && !ROUND;
-    typename PaTile<NB, TM, GR>::Acc acc = {};
-    if (k0 < k1) pa_tile_mm<ROUND, bf16, NB, TM, GR>(acc, arow ? arow + k0 : nullptr, 1.0f, brow0 ? brow0 + k0 : nullptr, brow1 ? brow1 + k0 : nullptr, k1 - k0, sm);
-    if (S == 1) return pa_tile_store<NB, TM, GR>(acc, sm, store);
-    pa_tile_gather<NB, TM, GR>(acc, sm);
+    typename PaTile<NB, TM>::Acc acc = {};
+    if (k0 < k1) pa_tile_mm<ROUND, bf16, NB, TM>(acc, arow ? arow + k0 : nullptr, 1.0f, brow0 ? brow0 + k0 : nullptr, brow1 ? brow1 + k0 : nullptr, k1 - k0, sm);
+    if (S == 1) return pa_tile_store<NB, TM, false>(acc, sm, store);
+    pa_tile_gather<NB, TM, false>(acc, sm);
     pa_cluster_sync();
     for (int e = tid; e < TM / S * 16; e += 256) {
         const int row = TM / S * rank + (e >> 4), col = (e & 15) * 4;
@@ -603,7 +602,7 @@ __global__ void __launch_bounds__(256) pa_k_rope_q(const float *__restrict__ q, 
 // z * a_gs on, the matrix z of N x K weights, and writes the columns of C from z * c_gs on.  Rows n >= act_from leave through the
 // one-argument activation, `gap` columns further on; mul multiplies the outputs by a table row per token.
 template <bool ROUND, int TM = PA_TM>
-__global__ void __launch_bounds__(256, TM == 32 ? 2 : 4) pa_k_linear(const float *__restrict__ A, int lda, const bf16 *__restrict__ W, const float *__restrict__ bias, float *__restrict__ C, int ldc,
+__global__ void __launch_bounds__(256, 4) pa_k_linear(const float *__restrict__ A, int lda, const bf16 *__restrict__ W, const float *__restrict__ bias, float *__restrict__ C, int ldc,
                                                    int M, int N, int K, int S, int a_gs, int c_gs, int act_from, int gap, PaAct act, PaRowMul mul) {
     __shared__ __align__(16) float sm[PaTile<1, TM>::N];
     const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM), z = blockIdx.z / S;
@@ -884,7 +883,7 @@ __global__ void __launch_bounds__(256, 4) pa_k_expert_down(const float *__restri
 
 // dense feed-forward, first half: y[m][n] = act(gate[n] . h_m, up[n] . h_m); NB = 1: no gate, act(up[n] . h_m).  blockIdx.z: the S cuts of K
 template <bool ROUND, int NB, int TM = PA_TM>
-__global__ void __launch_bounds__(256, NB == 2 || TM == 32 ? 2 : 4) pa_k_dense_up(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff,
+__global__ void __launch_bounds__(256, NB == 2 ? 2 : 4) pa_k_dense_up(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff,
                                                      int dim, PaAct act, int S) {
     __shared__ __align__(16) float sm[PaTile<NB, TM>::N];
     const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM);
@@ -922,6 +921,8 @@ __device__ __forceinline__ int pa_first_key(const PaAttn &at, int p) {
     if (at.chunk > 0) lo = max(lo, p - p % at.chunk);
     return lo;
 }
+// first key of a tile of queries whose first one stands at p: on a step of the tile core, so that a key's group of threads is the same in every portion
+__device__ __forceinline__ int pa_tile_first_key(const PaAttn &at, int p) { return pa_first_key(at, p) / PA_TK * PA_TK; }
 __device__ __forceinline__ float pa_sink_logit(const PaAttn &at, int h) { return at.sink_v ? at.sink_v[h] : 0.f; }
 
 // S[h][i][j] = score of query i (position pos[i]) and cache row j <= pos[i], before the heads are mixed.  Key tiles from
@@ -994,7 +995,7 @@ __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__rest
     extern __shared__ float Ts[];
     const int i = blockIdx.x, H = at.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = pos[i] + 1, n_end = pos[0] + bs, lo = pa_first_key(at, pos[i]);
-    const int lo_tile = pa_first_key(at, pos[0] + i / PA_TM * PA_TM); // P.V walks whole tiles of queries: from the tile's first key on
+    const int lo_tile = pa_tile_first_key(at, pos[0] + i / PA_TM * PA_TM); // P.V walks whole tiles of queries: from the tile's first key on
     if (at.mix) {
         for (int t = threadIdx.x; t < H * H; t += 256) Ts[t] = at.mix[t];
         __syncthreads();
@@ -1040,7 +1041,7 @@ __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__rest
 // att[i][h * dv + c] = sum_j P[h][i][j] V^T[g * dv + c][j].  With rotated values a tile's 64 columns are 32 pairs (m, m + dv / 2), two pairs to a
 // thread, which turns them back by its query's position; then the head's gate and the factor on the heads' outputs.
 // GROUPS: four groups of threads share the keys of a step (256 queries x 1024 keys x 16 heads 43 -> 36 us).  Not in bfloat16 mode: the heads' outputs are the
-// rounded operand of the next product, where another order of the keys moves logits by 1e-4, and they are to be the same however a prompt is cut
+// rounded operand of the next product, where another order of the keys moves logits by 1e-4
 template <bool GROUPS>
 __global__ void __launch_bounds__(256, GROUPS ? 2 : 3) pa_k_pv(PaAttn at, const float *__restrict__ S, const float *__restrict__ vct, float *__restrict__ att, int od,
                                                const int32_t *__restrict__ pos, int bs) {
@@ -1048,7 +1049,7 @@ __global__ void __launch_bounds__(256, GROUPS ? 2 : 3) pa_k_pv(PaAttn at, const 
     const int lr = threadIdx.x >> 2;
     const int h = blockIdx.z, g = h / (at.H / at.G), m0 = blockIdx.y * PA_TM, n0 = blockIdx.x * PA_TN;
     const int n_keys = pos[0] + min(m0 + PA_TM, bs); // keys the tile's furthest query sees (the rows are zero beyond their own)
-    const int k0 = pa_first_key(at, pos[0] + m0);    // ... and the first key its first query sees (zero before a row's own)
+    const int k0 = pa_tile_first_key(at, pos[0] + m0); // ... and the first key its first query sees (zero before a row's own)
     typename PaTile<1, PA_TM, GROUPS>::Acc acc = {};
     const float *arow = (m0 + lr < bs) ? S + ((int64_t)h * at.B + m0 + lr) * at.ldS + k0 : nullptr;
     // value dim of the tile's column j (dv or more: outside)

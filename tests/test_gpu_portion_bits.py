@@ -9,7 +9,7 @@ from powerserve_b200 import arch, arch_synth
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("dtype,width,ff", [("bfloat16", 264, 200)])
+@pytest.mark.parametrize("dtype,width,ff", [("bfloat16", 264, 200), ("float32", 264, 200), ("float32", 1032, 648)])
 def test_portions(tmp_path, dtype, width, ff):
     layers = [arch_synth.vanapel_attention_layer(6, 2, 44, 44, window=40, ff=ff, limit=7.0), arch_synth.vanapel_latent_layer(6, 44, 8, 40, 72, 260, ff=ff, limit=7.0)]
     cfg = arch_synth.vanapel_config(width, 130, layers, groups=1)
