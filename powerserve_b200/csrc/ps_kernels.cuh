@@ -1480,6 +1480,8 @@ __global__ void __launch_bounds__(256) ps_k_sess_softmax(float *__restrict__ kq,
     for (int64_t j = threadIdx.x; j < ne0; j += blockDim.x) dp[j] = __fmul_rn(dp[j], inv);
 }
 
+// a load that stays where it is written: before the ones that follow it and before what is made of it
+PS_D float ps_ld_now(const float *p) { float v; asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p)); return v; }
 // P.V of column c: out[c][h * hs + d]; a warp takes eight dims of a kv head and HB of the group's heads at a time (four, two or one where the group has no
 // more: an absent head costs as much as a present one).  A chunk of 32 positions is eight rows of V and HB of weights for 8 HB products; with a dim a warp
 // the weights were read 128 times over and every sum took five shuffles (64 sessions of 100 to 200 positions, a layer of 32 query and 8 kv heads: 46.6 us).  After the reduction lane (dim, head) owns one sum and adds the leftover products to it in order
@@ -1500,19 +1502,32 @@ template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__r
 #pragma unroll
         for (int k = 0; k < 8 * HB; k++) sum[k] = 0.f;
         __syncwarp();
+        float left[8 + HB];
 #pragma unroll
-        for (int k = 0; k < 8 + HB; k++) s_left[warp][k][lane] = lane < rem ? (k < 8 ? vrow[k * n_ctx + np] : pr[k < 8 ? 0 : k - 8][np]) : 0.f;
-#pragma unroll 2
-        for (int64_t s = 0; s < np; s += 32) {
-            float v[8], w[HB];
+        for (int k = 0; k < 8 + HB; k++) left[k] = lane < rem ? ps_ld_now(k < 8 ? vrow + k * n_ctx + np : pr[k < 8 ? 0 : k - 8] + np) : 0.f;
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = vrow[k * n_ctx + s];
+        for (int k = 0; k < 8 + HB; k++) s_left[warp][k][lane] = left[k];
+        // Bound by memory latency: four chunks' loads are on their way together.  Left to itself the compiler puts the loads of one head between its products, one
+        // waited for after the other (cold caches, a session of 1000 positions, 16 kv heads with a query head each 100 us, two heads each 37, four 23; now 11, 11, 12)
+        constexpr int U = 4;
+        for (int64_t s = 0; s < np; s += 32 * U) {
+            float v[U][8], w[U][HB];
 #pragma unroll
-            for (int t = 0; t < HB; t++) w[t] = pr[t][s];
+            for (int c = 0; c < U; c++)
+                if (s + 32 * c < np) {
 #pragma unroll
-            for (int k = 0; k < 8; k++)
+                    for (int k = 0; k < 8; k++) v[c][k] = ps_ld_now(vrow + k * n_ctx + s + 32 * c);
 #pragma unroll
-                for (int t = 0; t < HB; t++) sum[k * HB + t] = __fmaf_rn(v[k], w[t], sum[k * HB + t]);
+                    for (int t = 0; t < HB; t++) w[c][t] = ps_ld_now(pr[t] + s + 32 * c);
+                }
+#pragma unroll
+            for (int c = 0; c < U; c++)
+                if (s + 32 * c < np) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+#pragma unroll
+                        for (int t = 0; t < HB; t++) sum[k * HB + t] = __fmaf_rn(v[c][k], w[c][t], sum[k * HB + t]);
+                }
         }
         // GGML_F32x8_REDUCE as a reduce-scatter: lane bits 4, 3, 2 keep the dim, then (stages xor 1, xor 2) bits 0 and 1 the head
         ps_rs_stage<8 * HB>(sum, lane & 16, 16);
