@@ -842,13 +842,12 @@ TcPlan tc_plan(const ps_cuda_ctx *ctx, int64_t row_tiles, int64_t K, int bs) {
     return best;
 }
 
-template <int NT> int tc_launch(ps_cuda_ctx *ctx, PsTcArgs a) {
+template <int NT> int tc_launch(ps_cuda_ctx *ctx, const PsTcArgs &a) {
     static bool attr[64] = {};
     if (!attr[ctx->device]) {
         PS_CK(cudaFuncSetAttribute(ps_k_tc_gemm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PsTc<NT>::SMEM));
         attr[ctx->device] = true;
     }
-    if (a.give_up >= 0) a.give_up %= PsTc<NT>::THREADS / 32; // (a test's option; widths have 20 or 28 warps)
     ps_k_tc_gemm<NT><<<(unsigned)std::min(a.n_tiles * PS_TC_PASSES, ctx->n_sm), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
     PS_LAUNCH_CK();
     return 0;

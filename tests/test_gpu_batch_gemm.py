@@ -1,7 +1,7 @@
 """GPU parity of the tensor-core GEMM behind token batches (powerserve_b200/csrc/ps_tc.cuh) at the edges of its tiling: batches on both
 sides of every column-tile width and over more than one column tile, matrices whose rows do not fill a 128-row tile (q | k | v segments
-that start on tile borders, biases), an odd number of super-blocks, and shapes for which a unit of work takes one, two or all six
-passes.  Oracle: the plain-C restatement of the reference; tolerance zero (the contract of this path)."""
+that start on tile borders, biases), an odd number of super-blocks, and shapes for which a CTA's share is one pass, two or more.
+Oracle: the plain-C restatement of the reference; tolerance zero (the contract of this path)."""
 import numpy as np
 import pytest
 
@@ -11,7 +11,7 @@ from tests import _model as M
 
 pytestmark = pytest.mark.gpu
 
-# 3 and 5 super-blocks; q 6, k and v 1.5 row tiles, gate / up 10, output 50 (all passes in one unit) and a bit
+# 3 and 5 super-blocks; q 6, k and v 1.5 row tiles, gate / up 10, output 50 and a bit
 ODD = synth.ModelShape("tc-odd", "llama", 768, 1280, 2, 8, 2, 96, 6400 + 24, False, 0, 5e5, 1e-5, gguf.GGML_Q4_K, n_ctx=512, qkv_bias=True)
 
 
@@ -36,31 +36,33 @@ def test_batch_widths(odd, bs):
     L.assert_bit_equal(got, om.forward(tokens), f"{bs} tokens")
 
 
-def test_two_passes_a_unit():
-    """layer shapes of an 8B model: 48 row tiles of q | k | v, three units of two passes each"""
+def test_shares_of_two_passes():
+    """layer shapes of an 8B model: 48 row tiles of q | k | v, 288 passes for 148 SMs"""
     d = M.model_dir("slice-8b")
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=32)
     tokens = synth.random_prompt(2048, 20, seed=3)
     L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), "8B slice, 20 tokens")
     assert cm.be.counter("tc_gemm_pass2") > 0
-    again = cm.forward(tokens[:9])          # the counters of the tiles are left as they were found
+    again = cm.forward(tokens[:9])          # the counters of the shared tiles are left as they were found
     assert np.isfinite(again).all() and cm.be.counter("tc_error") == 0
     L.assert_bit_equal(again, om.forward(tokens[:9]), "8B slice, 9 more tokens")
     om.close()
     cm.close()
 
 
-@pytest.mark.parametrize("bs", [16, 64, 128])
-def test_a_warp_that_gives_up_ends_the_call(odd, bs):
-    """one warp of every CTA takes its first wait as run out - an epilogue warp while the others of its tile go on to hand numbers over, a
-    de-quantising warp, the copies' warp, the issuing one: every other wait ends by its own limit, the call reports the time-out, and the
-    next call on the same context has all bits"""
-    om, cm = odd
-    tokens = synth.random_prompt(ODD.vocab_size, bs, seed=bs)
-    om.reset()
+@pytest.mark.parametrize("width", [16, 32, 48, 64])
+def test_a_warp_that_gives_up_ends_the_call(width):
+    """one warp of every CTA takes its first wait as run out - the first and the last epilogue warp while the others of the tile go on to hand numbers
+    over, the first and the last de-quantising one, the copies' warp, the issuing one: every other wait ends by its own limit, the call reports the
+    time-out, and the next call on the same context has all bits.  All products of an 8B layer on `width` tokens take tiles of that many columns;
+    a number behind the last warp of theirs is nobody's, and the call goes through."""
+    d = M.model_dir("slice-8b")
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=64)
+    tokens = synth.random_prompt(2048, width, seed=width)
     want = om.forward(tokens)
-    epilogue = 8 if bs < 64 else 16
-    for warp in (0, epilogue - 1, epilogue, epilogue + 8, epilogue + 9):
+    om.close()
+    copies = 8 + (16 if width <= 32 else 8)                  # epilogue, then de-quantising warps
+    for warp in (0, 7, 8, copies - 1, copies, copies + 1):
         cm.reset()
         cm.be.set_option("give_up_warp", warp)
         with pytest.raises(capi.PsCudaError, match="tcgen05 pipeline time-out"):
@@ -68,10 +70,15 @@ def test_a_warp_that_gives_up_ends_the_call(odd, bs):
         cm.be.set_option("give_up_warp", -1)
         cm.reset()
         L.assert_bit_equal(cm.forward(tokens), want, f"after warp {warp} gave up")
+    for warp in (copies + 4, 40):
+        cm.reset()
+        cm.be.set_option("give_up_warp", warp)
+        L.assert_bit_equal(cm.forward(tokens), want, f"no warp {warp}")
+    cm.close()
 
 
-def test_every_number_of_passes(odd):
-    """what the widths above are spread over: units of one pass and of all six (the head's 51 row tiles)"""
+def test_shares_of_one_pass_and_of_more_than_two(odd):
+    """what the widths above are spread over: 4 to 10 row tiles, and the head's 51"""
     cm = odd[1]
     cm.reset()
     n = [cm.be.counter(f"tc_gemm_pass{p}") for p in (1, 6)]
@@ -80,8 +87,8 @@ def test_every_number_of_passes(odd):
 
 
 @pytest.mark.parametrize("bs", [97, 128])
-def test_widest_tiles(bs):
-    """products large enough for column tiles of 128 at any number of passes (an 8B layer's)"""
+def test_two_column_tiles_of_64(bs):
+    """an 8B layer's products on more tokens than the widest tile has columns"""
     d = M.model_dir("slice-8b")
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=128)
     tokens = synth.random_prompt(2048, bs, seed=bs)
