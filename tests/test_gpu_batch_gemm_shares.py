@@ -9,8 +9,9 @@ from tests import _model as M
 
 pytestmark = pytest.mark.gpu
 
-# row tiles: q | k | v 3, o 2, gate | up 38, down 2, head 101 (and a part of one); 1 and 9.5 super-blocks of 256
-SHAPE = synth.ModelShape("tc-shares", "llama", 256, 2432 // 256 * 256 + 256, 1, 4, 2, 64, 128 * 100 + 8, False, 0, 5e5, 1e-5, gguf.GGML_Q4_K, n_ctx=512)
+# row tiles: q | k | v 4, o 2, gate | up 52, down 2, head 101 (the last one has 8 rows); super-blocks of 256: one, and the down product's 13, an odd
+# count whose last step is half padding when the rings of five or six stages have gone round
+SHAPE = synth.ModelShape("tc-shares", "llama", 256, 256 * 13, 1, 4, 2, 64, 128 * 100 + 8, False, 0, 5e5, 1e-5, gguf.GGML_Q4_K, n_ctx=512)
 
 
 @pytest.fixture(scope="module")
