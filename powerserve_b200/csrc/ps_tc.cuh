@@ -206,14 +206,14 @@ struct PsTcArgs {
     uint32_t limit;     // cycles a wait lasts at most
 };
 
-// eight columns of one row of an accumulator; they are there after ps_tc_ld_wait, and ps_tc_pass keeps whatever reads them behind it
+// eight columns of one row of an accumulator; they are there after ps_tc_ld_wait, and ps_tc_keep keeps whatever reads them behind it
 PS_D void ps_tc_ld(uint32_t taddr, uint32_t (&v)[8]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                  : "r"(taddr)
                  : "memory");
 }
-PS_D void ps_tc_pass(uint32_t (&v)[8]) {
+PS_D void ps_tc_keep(uint32_t (&v)[8]) {
     asm volatile("" : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])::"memory");
 }
 PS_D ps_f2 ps_f2_bits(uint32_t a, uint32_t b) { ps_f2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
@@ -510,8 +510,8 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcA
                         const ulonglong2 y0 = yd[0], y1 = yd[1];
                         const ps_f2 dd[4] = {ps_f2_mul(y0.x, x2), ps_f2_mul(y0.y, x2), ps_f2_mul(y1.x, x2), ps_f2_mul(y1.y, x2)};
                         ps_tc_ld_wait();
-                        ps_tc_pass(v0);
-                        ps_tc_pass(v1);
+                        ps_tc_keep(v0);
+                        ps_tc_keep(v1);
                         if ((x == 1 || T::XE == 1) && c + 8 == T::EC) { // the entry is in registers
                             ps_tc_fence_before();
                             __syncwarp();
