@@ -125,7 +125,8 @@ struct ps_cuda_ctx {
     int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_scores_batch_min = 2, opt_give_up = -1;
     bool tc_ok = false;        // tensor-core prefill operands are resident
     uint8_t *tc_b = nullptr;   // B operand blocks of the current activation batch
-    float *tc_part = nullptr;  // numbers of the tiles that CTAs share: a slot per CTA
+    float *tc_part = nullptr;  // numbers of the tiles that CTAs share: a slot per CTA, for tiles of up to tc_nt columns
+    int tc_nt = 64;            // widest column tile that max_batch tokens need
     int *tc_cnt = nullptr;     // per slot: passes handed over
     int *err_dev = nullptr;    // device-detected failures, [0] tcgen05 pipeline time-out (PS_ERR_COPY: a copy of a batch product), [1] peer wait gave up, [2] step-kernel barrier time-out
     int err_seen[3] = {};      // sticky host copy of the flags (counters "tc_error" / "tp_error" / "step_error")
@@ -835,6 +836,7 @@ TcPlan tc_plan(const ps_cuda_ctx *ctx, int64_t row_tiles, int64_t K, int bs) {
     TcPlan best = {};
     int64_t cost = INT64_MAX;
     for (const auto &w : width) {
+        if (w.nt > ctx->tc_nt) continue;
         const int64_t passes = row_tiles * ((bs + w.nt - 1) / w.nt) * PS_TC_PASSES, share = (passes + ctx->n_sm - 1) / ctx->n_sm;
         const int64_t c = share * (tc_nbp(K) * w.ns + 500);
         if (c < cost) { cost = c; best = {w.nt, (int)share}; }
@@ -2057,7 +2059,8 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
                 }
                 const size_t cols = (size_t)d.max_batch + 63; // (whole column tiles of any width)
                 if ((rc = dev_alloc(ctx, (void **)&ctx->tc_b, cols * (size_t)tc_nbp(ctx->maxK) * 644))) return rc;
-                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_part, (size_t)ctx->n_sm * PS_TC_PASSES * PS_TC_M * 64 * 4))) return rc;
+                ctx->tc_nt = std::min(64, (d.max_batch + 15) & ~15);
+                if ((rc = dev_alloc(ctx, (void **)&ctx->tc_part, (size_t)ctx->n_sm * PS_TC_PASSES * PS_TC_M * ctx->tc_nt * 4))) return rc;
                 if ((rc = dev_alloc(ctx, (void **)&ctx->tc_cnt, (size_t)ctx->n_sm * 4))) return rc;
                 PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, (size_t)ctx->n_sm * 4, ctx->stream));
                 ctx->tc_ok = true;

@@ -95,3 +95,16 @@ def test_two_column_tiles_of_64(bs):
     L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"8B slice, {bs} tokens")
     om.close()
     cm.close()
+
+
+def test_workspace_follows_the_batch():
+    """the numbers of shared tiles need a slot per SM for tiles of as many columns as max_batch has, up to 64: 7 MB for 16, 29 MB for 64"""
+    import torch
+    d, used = M.model_dir("tiny-llama"), {}
+    for batch in (16, 64, 16, 64):      # (the first model of a process brings the kernels' own memory along)
+        before = torch.cuda.mem_get_info()[0]
+        cm = capi.CudaModel(d, max_batch=batch)
+        used[batch] = before - torch.cuda.mem_get_info()[0]
+        cm.close()
+    slot = 148 * 6 * 128 * 4
+    assert used[64] - used[16] > 0.8 * slot * (64 - 16), used
