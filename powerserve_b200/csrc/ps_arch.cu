@@ -1343,6 +1343,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     auto dense_up = [&](const float *X, const bf16 *wg, const bf16 *wu, int ff, const PaAct &act) -> int {
         const int64_t rows = (int64_t)cdiv(ff, PA_TN) * PA_TN * (wg ? 2 : 1); // (a gated tile has two products)
         const int S = ROUND ? 1 : pa_cuts(rows, dim);
+        // (gate | up of 1024 x 1024 on 8 / 64 tokens: 18.7 / 19.6 us in 32-row tiles, 22.1 / 22.7 in 64-row ones; 512 x 2048: 23.4 / 31.2 and 26.5 / 27.4)
         const bool narrow = pa_narrow_tiles(a->n_sm, rows * S / (wg ? 2 : 1), bs);
         const dim3 grid(cdiv(ff, PA_TN), cdiv(bs, narrow ? 32 : PA_TM), (unsigned)S);
         if (wg) pa_launch_cut(S, narrow ? pa_k_dense_up<ROUND, 2, 32> : pa_k_dense_up<ROUND, 2, PA_TM>, grid, st, X, dim, wg, wu, a->y, bs, ff, dim, act, S);

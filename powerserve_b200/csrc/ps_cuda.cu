@@ -829,7 +829,10 @@ int tc_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t n_rows, in
 }
 // Column-tile width of a product.  Its passes are cut into one share per CTA, and a pass takes so many ns a super-block (16 to 64 columns: 203, 232, 264, 308)
 // and half a microsecond for its end.  So wide tiles are cheaper per column while every SM has a few passes, and of a small matrix, where a share is one
-// or two passes whatever the width, a narrow tile ends first (4096 x 4096 on 64 columns: 26.6 us with 64-column tiles, 25.6 with 32)
+// or two passes whatever the width, a narrow tile ends first.  What a launch takes besides, with cold caches 9 to 20 us for its start, its first copies and
+// the last shared tile, is not in the estimate: 28672 x 4096 on 64 columns is estimated at 54 us and takes 71.  Over the products of 1B and 8B layers on 8 to
+// 128 columns the choice is the fastest width or within 3 % of it, except where CTAs of one or two passes share tiles and a wide tile's hand-over counts
+// (4096 x 4096 on 64 columns: 27 us with 64-column tiles, 25 with 32; 2048 x 2048 on 48 / 64: 16.6 / 18.6 with 48 / 64, 13.9 / 15.6 with 16 / 32)
 struct TcPlan { int nt, share; };
 TcPlan tc_plan(const ps_cuda_ctx *ctx, int64_t row_tiles, int64_t K, int bs) {
     static const struct { int nt, ns; } width[] = {{64, 308}, {48, 264}, {32, 232}, {16, 203}};

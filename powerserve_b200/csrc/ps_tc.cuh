@@ -28,7 +28,7 @@
 // Measured (time that each further super-block of a pass adds, at 1.92 GHz; 128 rows x 16 / 32 / 48 / 64 columns): 390 / 450 / 510 / 590 cycles, where a kernel with
 // two units of work to a tile, epilogue warps of half the columns and a barrier per hand-over needed 720 to 820 at any width.  Where it goes (64 columns): the
 // epilogue's own work 270 (16 FMUL2 and 32 FFMA2 a warp, 192 of pipe time), de-quantising 140 in a lane pass, and what the roles need for their waits and rings:
-// 630 of 1 800 instructions.  28 672 x 4096 on 16 / 32 / 64 / 128 columns: 86 / 108 / 104 / 168 -> 45 / 55 / 80 / 138 us; 4096 x 14 336 on 128: 104 -> 80.
+// 630 of 1 800 instructions.  28 672 x 4096 on 16 / 32 / 64 / 128 columns: 86 / 108 / 104 / 168 -> 45 / 53 / 71 / 126 us; 4096 x 14 336 on 128: 104 -> 76.
 // An epilogue that reads more than eight columns at a time spills or moves registers (64 columns: 590 cycles with 8, 655 with 16, 676 with 32, 700 with two
 // buffers of 8); the end of a pass is met once per pass with cold instructions, so its loops hold no branches (64 columns: 12 us a tile with, 3.5 without).
 #pragma once
