@@ -400,11 +400,42 @@ int matmul_q(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int wtype, int64_t 
     }
 }
 
-// the same on the octet copies of an all-Q4_0 / all-Q8_0 model (ps_k_matmul_ob); *done = false: a row octet does not fit shared memory
+// matmul_q on the octet copies of an all-Q4_0 / all-Q8_0 model (ps_k_matmul_ob):
+template <int TYPE> int mo_warps(int64_t K, int C) { // warps of a CTA: their octets and the activations fit shared memory
+    int warps = PS_MB_WARPS;
+    while (warps > 1 && ps_mo_smem<TYPE>(K, C, warps) > 200 * 1024) warps >>= 1;
+    return warps;
+}
+// Four columns a warp where eight do?  The blocks of a row are a chain, and with eight columns octets x groups of eight may leave a scheduler fewer than two warps,
+// which wait for most of a step (896 rows on 32 columns, K 896 / 4864: 14.8 / 30.5 us with eight, 11.8 / 25.2 with four, 10.7 / 31.3 with two; 9728 rows 32.3, 39.8,
+// 53.7.  A row a thread and two warps an octet instead: 13.5 / 25.7 with eight columns, 11.3 / 24.5 with four).  Then four are faster if a CTA gets more warps
+// that way (long rows), or if their CTAs, twice as many, need no further round of the SMs and are not more than about three to an SM (Q8_0, K 2048, 3072 rows on 8 / 16
+// columns, two CTAs to an SM: 13.9 / 17.1 us with eight, 12.3 / 21.4 with four; Q8_0, K 1536, 1536 rows on 32 / 48: 18.9 / 19.8 and 15.5 / 23.5; Q4_0, K 896,
+// 1152 rows on 48 / 64: 12.4 / 12.8 and 10.9 / 13.3).  Where eight columns leave no room for one octet the GGUF rows' kernel takes over, two to three times as fast as
+// four columns with one octet a CTA (Q8_0, K 14336, 4096 rows on 8 / 16 columns: 135 / 227 us and 310 / 607)
+template <int TYPE> bool mo_four_columns(const ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int n_seg) {
+    int64_t walks = 0;
+    for (int t = 0; t < n_seg; t++) walks += (segs[t].n + 7) / 8;
+    if (walks * ((bs + 7) / 8) >= 8 * ctx->n_sm) return false;
+    const int w4 = mo_warps<TYPE>(K, 4), w8 = mo_warps<TYPE>(K, 8);
+    if (w4 > w8) return true;
+    auto ctas = [&](int C, int warps) {
+        int64_t n = 0;
+        for (int t = 0; t < n_seg; t++) n += (segs[t].n + 8 * warps - 1) / (8 * warps);
+        return n * ((bs + C - 1) / C);
+    };
+    auto rounds = [&](int64_t n, int C, int warps) { // of CTAs that fit an SM's 227 KB (barriers and a KB of its own besides)
+        const int64_t most = ctx->n_sm * std::max<int64_t>(1, 227 * 1024 / (int64_t)(ps_mo_smem<TYPE>(K, C, warps) + 1536));
+        return (n + most - 1) / most;
+    };
+    if (ps_mo_smem<TYPE>(K, 8, w8) > 200 * 1024) return false;
+    const int64_t n4 = ctas(4, w4), r8 = rounds(ctas(8, w8), 8, w8);
+    return rounds(n4, 4, w4) <= r8 && (r8 > 1 || 5 * n4 <= 16 * ctx->n_sm);
+}
+// *done = false: a row octet does not fit shared memory
 template <int TYPE, int C, bool REST> int launch_mo_r(ps_cuda_ctx *ctx, PsMbArgs a, bool *done) {
     static bool attr_set[64] = {};
-    int warps = PS_MB_WARPS;
-    while (warps > 1 && ps_mo_smem<TYPE>(a.K, C, warps) > 200 * 1024) warps >>= 1;
+    const int warps = mo_warps<TYPE>(a.K, C);
     const size_t smem = ps_mo_smem<TYPE>(a.K, C, warps);
     if (smem > 200 * 1024) return 0;
     if (!attr_set[ctx->device]) {
@@ -425,12 +456,7 @@ int matmul_ob(ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int 
     PsMbArgs a{};
     for (int t = 0; t < n_seg; t++) a.seg[t] = segs[t];
     a.n_seg = n_seg; a.bs = (int)bs; a.K = K; a.aqs = ctx->aqs; a.ad = ctx->ad; a.residual = residual; a.err = ctx->tc_err_dev; a.give_up = ctx->opt_give_up;
-    // eight columns a warp; four where octets x groups of eight leave a scheduler fewer than two warps: the blocks of a row are a chain, and a warp alone waits for
-    // most of a step (896 rows on 32 columns, K 896 / 4864: 14.8 / 30.5 us with eight, 11.8 / 25.2 with four, 10.7 / 31.3 with two; 1152 rows 11.2, 9.6, 10.1;
-    // 9728 rows 32.3, 39.8, 53.7.  A row a thread and two warps an octet instead: 13.5 / 25.7 with eight columns, 11.3 / 24.5 with four)
-    int64_t walks = 0;
-    for (int t = 0; t < n_seg; t++) walks += (segs[t].n + 7) / 8;
-    const int C = bs <= 2 ? 2 : bs <= 4 || walks * ((bs + 7) / 8) < 8 * ctx->n_sm ? 4 : 8;
+    const int C = bs <= 2 ? 2 : bs <= 4 || (ctx->mv_type == 2 ? mo_four_columns<2>(ctx, K, bs, segs, n_seg) : mo_four_columns<8>(ctx, K, bs, segs, n_seg)) ? 4 : 8;
     if (ctx->mv_type == 2) return C == 2 ? launch_mo<2, 2>(ctx, a, done) : C == 4 ? launch_mo<2, 4>(ctx, a, done) : launch_mo<2, 8>(ctx, a, done);
     return C == 2 ? launch_mo<8, 2>(ctx, a, done) : C == 4 ? launch_mo<8, 4>(ctx, a, done) : launch_mo<8, 8>(ctx, a, done);
 }

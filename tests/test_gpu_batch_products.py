@@ -1,5 +1,7 @@
 """GPU parity of the products of token batches that run on the CUDA cores (ps_k_matmul_qb on GGUF rows, ps_k_matmul_ob on octet copies)
 where their shapes change, and their way out.  Oracle: the plain-C restatement of the reference; tolerance zero."""
+import time
+
 import numpy as np
 import pytest
 
@@ -126,3 +128,44 @@ def test_rows_of_a_thread(t, bs):
         got, ref = _product(be, t, w, K, N, rng.standard_normal(K * bs).astype(np.float32), bs)
         L.assert_bit_equal(got, ref, f"type {t} {K} x {N} bs {bs}")
     be.close()
+
+
+def test_rows_too_long_for_eight_octets_of_q8_0(tmp_path):
+    """rows of 14336 Q8_0 weights: eight columns' activations leave no room for a single octet, four leave room for one, whose CTAs of one warp take two to three
+    times as long as the kernel on the GGUF bytes.  72 tokens are the most at which the octet kernel would take four columns by its number of
+    warps alone, at 80 it never does: the portions' times are to be alike, and all bits the same."""
+    shape = synth.ModelShape("q8-long-rows", "llama", 1024, 14336, 1, 16, 2, 64, 264, False, 0, 1e4, 1e-5, gguf.GGML_Q8_0, n_ctx=128)
+    d = synth.write_model_dir(str(tmp_path), shape, seed=12)
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=80)
+    took = {}
+    for n in (72, 80):
+        tokens = synth.random_prompt(264, n, seed=n)
+        om.reset()
+        cm.reset()
+        L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"{n} tokens")
+        best = 1e9
+        for _ in range(20):
+            cm.reset()
+            t0 = time.perf_counter()
+            cm.forward(tokens, lm_head=False)
+            best = min(best, time.perf_counter() - t0)
+        took[n] = best
+    om.close()
+    cm.close()
+    assert took[72] < 1.25 * took[80], took
+
+
+@pytest.mark.parametrize("quant", [gguf.GGML_Q4_0, gguf.GGML_Q8_0])
+@pytest.mark.parametrize("dim,ffn", [(1536, 1536), (1024, 2816)])
+def test_four_and_eight_columns_a_warp(tmp_path, quant, dim, ffn):
+    """portions on both sides of the rule: CTAs of four columns that fit the SMs, that would share them, that have more warps than those of eight"""
+    shape = synth.ModelShape("columns", "llama", dim, ffn, 1, dim // 64, 2, 64, 264, False, 0, 1e4, 1e-5, quant, n_ctx=128)
+    d = synth.write_model_dir(str(tmp_path), shape, seed=13)
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=80)
+    for n in (5, 12, 32, 48, 65, 72):
+        tokens = synth.random_prompt(264, n, seed=n)
+        om.reset()
+        cm.reset()
+        L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"{n} tokens")
+    om.close()
+    cm.close()
