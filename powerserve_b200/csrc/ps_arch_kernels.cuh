@@ -150,7 +150,7 @@ __device__ __forceinline__ float pa_act1(float z, PaAct act) {
 // queries x 1024 keys x 16 heads 43 -> 36 us), and not for the short cuts of the dense products at 64 rows (27 -> 39 us, 128 registers halve the CTAs an SM
 // holds).  Nor may 32-row tiles have groups where 64-row ones have none, since the batch decides between the two: one order of k for both, so that a
 // token's sums do not depend on its batch (8 / 48 / 150 tokens of two 1024-wide Vanapel layers in float32: 297 / 319 / 522 us with groups in 32-row tiles,
-// 317 / 335 / 532 without, 300 / 318 / 586 with groups in both)
+// 311 / 328 / 520 without; groups in both: the small batches as before, 150 tokens 10 % slower)
 __device__ __forceinline__ void pa_fetch8(const float *row, bool vec, int k, int K, float v[8]) {
     if (vec && k + 8 <= K) {
         const float4 x = *reinterpret_cast<const float4 *>(row + k), y = *reinterpret_cast<const float4 *>(row + k + 4);

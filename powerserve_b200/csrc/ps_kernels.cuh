@@ -1397,7 +1397,7 @@ __global__ void __launch_bounds__(128) ps_k_matmul_f32(float *__restrict__ dst, 
 // ====================================================================================================================
 // scores of column c: kq_c {n_kv_c, 1, n_heads} at kq + c * col_stride; a warp takes eight cache rows of a kv head against every query head of the group,
 // its sums reduced as in ps_k_attn_scores_tile (a warp a row: 20 shuffles and as many loads for four numbers; 64 sessions of 100 to 200 positions, a layer
-// of 32 query and 8 kv heads: 47.6 us; with P.V below 94 a layer, now about 39)
+// of 32 query and 8 kv heads: 47.6 us; with P.V below 94 a layer, now 34)
 template <int STEPS> __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q,
                                                                            int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t col_stride) {
     constexpr int hs = 32 * STEPS;
