@@ -296,6 +296,30 @@ void build_rope_table(const ps_cuda_model_desc &d, std::vector<float> &t, const 
     }
 }
 
+// launch with programmatic dependence on the kernel before (ps_grid_dep): its start-up, and in some kernels the first weights, overlap that one's end
+template <typename... KArgs, typename... Args>
+int launch_k(ps_cuda_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = (ctx->opt_pdl && !ctx->opt_ktime) ? 1 : 0;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+    ctx->n_launch++;
+    if (e != cudaSuccess) return fail(ctx, PS_CUDA_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
+    return 0;
+}
+
+#define PS_DEP(kern, grid, block, smem, ...)                                                                 \
+    do {                                                                                                     \
+        if (int rc_ = launch_k(ctx, kern, dim3(grid), dim3(block), smem, __VA_ARGS__)) return rc_;           \
+    } while (0)
+
 template <int TYPE>
 int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t N, const float *bias, const float *residual) {
     static bool attr_set[64] = {};
@@ -305,8 +329,7 @@ int launch_mm(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int64_t K, int64_t
         PS_CK(cudaFuncSetAttribute(ps_k_matmul_q<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[ctx->device] = true;
     }
-    ps_k_matmul_q<TYPE><<<(unsigned)((N + 7) / 8), 256, smem, ctx->stream>>>(w, K, N, ctx->aqs, ctx->ad, ctx->absp, dst, bias, residual);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_matmul_q<TYPE>, (unsigned)((N + 7) / 8), 256, smem, w, K, N, ctx->aqs, ctx->ad, ctx->absp, dst, bias, residual);
     return 0;
 }
 
@@ -322,8 +345,7 @@ template <int TYPE, int C, int R, bool REST = false> int launch_mb_r(ps_cuda_ctx
     }
     int cta = 0;
     for (int t = 0; t < a.n_seg; t++) { a.seg[t].cta0 = cta; cta += (a.seg[t].n + ROWS - 1) / ROWS; }
-    ps_k_matmul_qb<TYPE, R, C, REST><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), PS_MB_WARPS * 32, smem, ctx->stream>>>(a);
-    PS_LAUNCH_CK();
+    PS_DEP((ps_k_matmul_qb<TYPE, R, C, REST>), dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), PS_MB_WARPS * 32, smem, a);
     return 0;
 }
 // rows a thread takes: two, or one where 32-row CTAs would not reach every SM and 16-row ones are all resident together.  Q6_K, 2 / 3 / 8 columns:
@@ -372,14 +394,13 @@ int quantize_act(ps_cuda_ctx *ctx, int wtype, const ActIn &in, int64_t K, int64_
     if (K > ctx->maxK || bs > ctx->d.max_batch) return fail(ctx, PS_CUDA_ERR_INVALID, "activation %lldx%lld exceeds workspace", (long long)K, (long long)bs);
     if (wtype == 12 || wtype == 13 || wtype == 14) {
         if (K % 256) return fail(ctx, PS_CUDA_ERR_INVALID, "K=%lld is not a multiple of 256", (long long)K);
-        if (in.norm) ps_k_norm_quantize<true><<<(unsigned)bs, 512, 0, ctx->stream>>>(in.x, in.norm, K, ctx->d.norm_eps, ctx->aqs, ctx->ad, ctx->absp);
-        else ps_k_quantize_q8k<<<dim3((unsigned)((K / 256 + 3) / 4), (unsigned)bs), 128, 0, ctx->stream>>>(in.x, in.u, K, ctx->aqs, ctx->ad, ctx->absp);
+        if (in.norm) PS_DEP(ps_k_norm_quantize<true>, (unsigned)bs, 512, 0, in.x, in.norm, K, ctx->d.norm_eps, ctx->aqs, ctx->ad, ctx->absp);
+        else PS_DEP(ps_k_quantize_q8k, dim3((unsigned)((K / 256 + 3) / 4), (unsigned)bs), 128, 0, in.x, in.u, K, ctx->aqs, ctx->ad, ctx->absp);
     } else {
         if (K % 32) return fail(ctx, PS_CUDA_ERR_INVALID, "K=%lld is not a multiple of 32", (long long)K);
-        if (in.norm) ps_k_norm_quantize<false><<<(unsigned)bs, 512, 0, ctx->stream>>>(in.x, in.norm, K, ctx->d.norm_eps, ctx->aqs, ctx->ad, nullptr);
-        else ps_k_quantize_q80<<<dim3((unsigned)((K / 32 + 15) / 16), (unsigned)bs), 128, 0, ctx->stream>>>(in.x, in.u, K, ctx->aqs, ctx->ad);
+        if (in.norm) PS_DEP(ps_k_norm_quantize<false>, (unsigned)bs, 512, 0, in.x, in.norm, K, ctx->d.norm_eps, ctx->aqs, ctx->ad, nullptr);
+        else PS_DEP(ps_k_quantize_q80, dim3((unsigned)((K / 32 + 15) / 16), (unsigned)bs), 128, 0, in.x, in.u, K, ctx->aqs, ctx->ad);
     }
-    PS_LAUNCH_CK();
     return 0;
 }
 
@@ -444,8 +465,7 @@ template <int TYPE, int C, bool REST> int launch_mo_r(ps_cuda_ctx *ctx, PsMbArgs
     }
     int cta = 0;
     for (int t = 0; t < a.n_seg; t++) { a.seg[t].cta0 = cta; cta += (a.seg[t].n + 8 * warps - 1) / (8 * warps); }
-    ps_k_matmul_ob<TYPE, C, REST><<<dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), (unsigned)(warps * 32), smem, ctx->stream>>>(a);
-    PS_LAUNCH_CK();
+    PS_DEP((ps_k_matmul_ob<TYPE, C, REST>), dim3((unsigned)cta, (unsigned)((a.bs + C - 1) / C)), (unsigned)(warps * 32), smem, a);
     *done = true;
     return 0;
 }
@@ -470,24 +490,6 @@ int grid1d(int64_t n, int block = 256) { return (int)std::min<int64_t>((n + bloc
 // Llama-3.1-8B instead of ~650, chained with programmatic dependent launch and replayed as one CUDA graph.
 // ====================================================================================================================
 namespace {
-
-template <typename... KArgs, typename... Args>
-int launch_k(ps_cuda_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = (ctx->opt_pdl && !ctx->opt_ktime) ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-    ctx->n_launch++;
-    if (e != cudaSuccess) return fail(ctx, PS_CUDA_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e));
-    return 0;
-}
 
 // timeline slot of the next fused-path launch (nullptr when option "trace" is off)
 long long *tl_slot(ps_cuda_ctx *ctx) {
@@ -834,13 +836,11 @@ int launch_rope_kv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int bs, int64_t bas
     }
     a.pos = ctx->pos_dev; a.table = ctx->rope_table; a.nh = nh; a.nkv = nkv; a.head_size = d.head_size; a.n_dims = d.rope_n_dims; a.neox = d.rope_type & 2; a.bs = bs;
     a.n_ctx = d.n_ctx; a.base = base;
-    ps_k_rope_kv_batch<<<(unsigned)(((nh + nkv) * (d.head_size / 2) + 255) / 256 * bs + (kvd + 31) / 32 * ((bs + 31) / 32)), 256, 0, ctx->stream>>>(a);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_rope_kv_batch, (unsigned)(((nh + nkv) * (d.head_size / 2) + 255) / 256 * bs + (kvd + 31) / 32 * ((bs + 31) / 32)), 256, 0, a);
     return 0;
 }
 int rms_norm(ps_cuda_ctx *ctx, const float *w, int bs) { // of x into xn
-    ps_k_rmsnorm<<<(unsigned)bs, 256, 0, ctx->stream>>>(ctx->xn, ctx->x, w, ctx->d.dim, ctx->d.norm_eps);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_rmsnorm, (unsigned)bs, 256, 0, ctx->xn, ctx->x, w, ctx->d.dim, ctx->d.norm_eps);
     return 0;
 }
 
@@ -879,8 +879,7 @@ template <int NT> int tc_launch(ps_cuda_ctx *ctx, const PsTcArgs &a) {
         PS_CK(cudaFuncSetAttribute(ps_k_tc_gemm<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, PsTc<NT>::SMEM));
         attr[ctx->device] = true;
     }
-    ps_k_tc_gemm<NT><<<(unsigned)std::min(a.n_tiles * PS_TC_PASSES, ctx->n_sm), PsTc<NT>::THREADS, PsTc<NT>::SMEM, ctx->stream>>>(a);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_tc_gemm<NT>, (unsigned)std::min(a.n_tiles * PS_TC_PASSES, ctx->n_sm), PsTc<NT>::THREADS, PsTc<NT>::SMEM, a);
     return 0;
 }
 // quantises the input and multiplies; segments give their rows in the padded row space of the packed matrix (tile borders between them)
@@ -888,9 +887,8 @@ int tc_gemm(ps_cuda_ctx *ctx, const ActIn &x, const uint8_t *a_blocks, int64_t n
     PsTcArgs a{};
     const TcPlan plan = tc_plan(ctx, n_tiles, K, bs);
     const int nt = plan.nt, n_ct = (bs + nt - 1) / nt;
-    if (x.norm) ps_k_tc_norm_b<<<(unsigned)(n_ct * nt), 512, 0, ctx->stream>>>(ctx->tc_b, x.x, x.norm, K, ctx->d.norm_eps, bs, nt);
-    else ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x.x, x.u, K, bs, nt);
-    PS_LAUNCH_CK();
+    if (x.norm) PS_DEP(ps_k_tc_norm_b, (unsigned)(n_ct * nt), 512, 0, ctx->tc_b, x.x, x.norm, K, ctx->d.norm_eps, bs, nt);
+    else PS_DEP(ps_k_tc_prep_b, dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->tc_b, x.x, x.u, K, bs, nt);
     a.err = ctx->tc_err_dev;
     a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = n_ct; a.n_tiles = (int)n_tiles * n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
     a.part = ctx->tc_part; a.cnt = ctx->tc_cnt; a.give_up = ctx->opt_give_up; a.limit = give_up_cycles(ctx);
@@ -1027,8 +1025,7 @@ int decode_step_mv32(ps_cuda_ctx *ctx, bool lm_head, bool pick) {
     const int dim = d.dim, hs = d.head_size, nh = d.n_heads, nkv = d.n_kv_heads, kvd = hs * nkv, qdim = nh * hs, ffn = d.ffn_dim;
     int rc;
     ctx->trace_launch = 0;
-    ps_k_get_embedding<<<embed_grid(1, dim), 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, (int64_t)dim, ctx->tokens_dev);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_get_embedding, embed_grid(1, dim), 256, 0, ctx->x, ctx->w_embd, ctx->t_embd, (int64_t)dim, ctx->tokens_dev);
     for (int L = 0; L < d.n_layers; L++) {
         const LayerDev &ld = ctx->layers[L];
         {   // q | k | v = W . rmsnorm(x) (+ bias)
@@ -1117,8 +1114,7 @@ int decode_step_ops(ps_cuda_ctx *ctx, bool lm_head, bool pick) {
     const int64_t dim = d.dim, hs = d.head_size, nh = d.n_heads, nkv = d.n_kv_heads, kvd = hs * nkv, qdim = nh * hs, ffn = d.ffn_dim;
     int rc;
     ctx->trace_launch = 0;
-    ps_k_get_embedding<<<embed_grid(1, dim), 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev); // every embedding type, token from device memory
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_get_embedding, embed_grid(1, dim), 256, 0, ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev); // every embedding type, token from device memory
     for (int L = 0; L < d.n_layers; L++) {
         const LayerDev &ld = ctx->layers[L];
         if ((rc = quantize_act(ctx, ld.tq, {ctx->x, nullptr, ld.attn_norm}, dim, 1))) return rc;
@@ -2128,8 +2124,8 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
 struct SessRun { int n_kv_max; };
 // Scores and P.V of a batch over one cache (prefill chunk, verify batch): register-tiled kernels (option attn_tile, on
 // by default), else the first-generation kernels; narrow batches use the per-position / per-(head, dim) warp kernels.  nh / nkv
-// are the heads THIS rank owns.  The caller checks the launch (PS_LAUNCH_CK) after launch_batch_scores.
-static void launch_batch_scores(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int64_t n_kv, int bs) {
+// are the heads THIS rank owns.
+static int launch_batch_scores(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int64_t n_kv, int bs) {
     if (bs >= ctx->opt_scores_batch_min) {
         const int r2 = nh / nkv;
         // queries a CTA keeps in shared memory: as many as fit, fewer (down to four) while the grid leaves the GPU idle (32 queries of a 0.5B
@@ -2139,14 +2135,15 @@ static void launch_batch_scores(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs
         while (qb > 4 && (int64_t)((n_kv + 31) / 32) * nkv * ((bs + qb - 1) / qb) < 2 * ctx->n_sm) qb = std::max(4, (qb + 1) / 2);
         const dim3 grid((unsigned)((n_kv + 31) / 32), (unsigned)nkv, (unsigned)((bs + qb - 1) / qb));
         const size_t smem = (size_t)qb * r2 * hs * 4;
-        if (ctx->opt_attn_tile && hs == 128) ps_k_attn_scores_tile<4><<<grid, 128, smem, ctx->stream>>>(ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
-        else if (ctx->opt_attn_tile && hs == 64) ps_k_attn_scores_tile<2><<<grid, 128, smem, ctx->stream>>>(ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
-        else if (ctx->opt_attn_tile && hs == 32) ps_k_attn_scores_tile<1><<<grid, 128, smem, ctx->stream>>>(ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
-        else if (ctx->opt_attn_tile && hs == 256) ps_k_attn_scores_tile<8><<<grid, 128, smem, ctx->stream>>>(ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
-        else ps_k_attn_scores_batch<<<grid, 128, (size_t)qb * r2 * hs * 4, ctx->stream>>>(ctx->kq, ctx->kc[L], ctx->qr, hs, nh, nkv, n_kv, bs, qb);
+        if (ctx->opt_attn_tile && hs == 128) PS_DEP(ps_k_attn_scores_tile<4>, grid, 128, smem, ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
+        else if (ctx->opt_attn_tile && hs == 64) PS_DEP(ps_k_attn_scores_tile<2>, grid, 128, smem, ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
+        else if (ctx->opt_attn_tile && hs == 32) PS_DEP(ps_k_attn_scores_tile<1>, grid, 128, smem, ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
+        else if (ctx->opt_attn_tile && hs == 256) PS_DEP(ps_k_attn_scores_tile<8>, grid, 128, smem, ctx->kq, ctx->kc[L], ctx->qr, nh, nkv, n_kv, bs, qb);
+        else PS_DEP(ps_k_attn_scores_batch, grid, 128, (size_t)qb * r2 * hs * 4, ctx->kq, ctx->kc[L], ctx->qr, hs, nh, nkv, n_kv, bs, qb);
     } else {
-        ps_k_attn_scores<<<dim3((unsigned)((n_kv + 3) / 4), (unsigned)nkv), 128, 0, ctx->stream>>>(ctx->kq, ctx->kc[L], ctx->qr, hs, nh, nkv, n_kv, bs);
+        PS_DEP(ps_k_attn_scores, dim3((unsigned)((n_kv + 3) / 4), (unsigned)nkv), 128, 0, ctx->kq, ctx->kc[L], ctx->qr, hs, nh, nkv, n_kv, bs);
     }
+    return 0;
 }
 static int launch_batch_pv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int64_t n_kv, int bs, int batch_min) {
     const int64_t n_ctx = ctx->d.n_ctx;
@@ -2165,12 +2162,11 @@ static int launch_batch_pv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int
         static_assert(PS_PV_QB == PS_PVT_Q, "both P.V kernels block the queries by 8");
         const bool vec = n_ctx % 4 == 0 && ((uintptr_t)ctx->vct[L] & 15) == 0, deep = vec && PS_PVT_RING(6) + (size_t)PS_PVT_Q * n_kv * 4 <= 112 * 1024; // (two CTAs an SM)
         const auto pv = deep ? ps_k_attn_pv_tile<true, 6> : vec ? ps_k_attn_pv_tile<true, 4> : ps_k_attn_pv_tile<false, 4>;
-        if (tile) pv<<<grid, 256, (deep ? PS_PVT_RING(6) : PS_PVT_RING(4)) + (size_t)PS_PVT_Q * n_kv * 4, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
-        else ps_k_attn_pv_batch<<<grid1, 256, (size_t)PS_PV_QB * n_kv * 4, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
+        if (tile) PS_DEP(pv, grid, 256, (deep ? PS_PVT_RING(6) : PS_PVT_RING(4)) + (size_t)PS_PVT_Q * n_kv * 4, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
+        else PS_DEP(ps_k_attn_pv_batch, grid1, 256, (size_t)PS_PV_QB * n_kv * 4, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
     } else {
-        ps_k_attn_pv<<<dim3((unsigned)((hs + 3) / 4), (unsigned)nkv), 128, 0, ctx->stream>>>(ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
+        PS_DEP(ps_k_attn_pv, dim3((unsigned)((hs + 3) / 4), (unsigned)nkv), 128, 0, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
     }
-    PS_LAUNCH_CK();
     return 0;
 }
 
@@ -2186,8 +2182,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     const bool mo = bs > 1 && mv_usable(ctx); // octet copies of a 32-block model
     const bool rw = ctx->fused_ok && ctx->opt_fused && (bs > 1 || tree); // octet-interleaved copies exist: multi-column row-walker
     int rc;
-    ps_k_get_embedding<<<embed_grid(bs, dim), 256, 0, ctx->stream>>>(ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_get_embedding, embed_grid(bs, dim), 256, 0, ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
     static bool attr[64] = {};
     if (!attr[ctx->device]) {
         PS_CK(cudaFuncSetAttribute(ps_k_softmax_ext, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
@@ -2233,20 +2228,14 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             const int64_t cs = nh * (int64_t)d.n_ctx;
             static void (*const scores[])(float *, const float *const *, const float *, int, int, const int32_t *, int64_t) = {
                 ps_k_sess_scores<1>, ps_k_sess_scores<2>, ps_k_sess_scores<3>, ps_k_sess_scores<4>, ps_k_sess_scores<5>, ps_k_sess_scores<6>, ps_k_sess_scores<7>, ps_k_sess_scores<8>};
-            scores[hs / 32 - 1]<<<dim3((unsigned)((n_kv + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->stream>>>(ctx->kq, pl, ctx->qr, (int)nh, (int)nkv, ctx->pos_dev, cs);
-            PS_LAUNCH_CK();
-            ps_k_sess_softmax<<<dim3((unsigned)nh, (unsigned)bs), 256, (size_t)n_kv * 4, ctx->stream>>>(ctx->kq, ctx->pos_dev, cs, kq_scale);
-            PS_LAUNCH_CK();
+            PS_DEP(scores[hs / 32 - 1], dim3((unsigned)((n_kv + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->kq, pl, ctx->qr, (int)nh, (int)nkv, ctx->pos_dev, cs);
+            PS_DEP(ps_k_sess_softmax, dim3((unsigned)nh, (unsigned)bs), 256, (size_t)n_kv * 4, ctx->kq, ctx->pos_dev, cs, kq_scale);
             const auto pv = nh / nkv == 1 ? ps_k_sess_pv<1> : nh / nkv == 2 ? ps_k_sess_pv<2> : ps_k_sess_pv<4>;
-            pv<<<dim3((unsigned)((hs + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->stream>>>(ctx->att, pl + d.max_batch, ctx->kq, (int)hs, (int)nh, (int)nkv, ctx->pos_dev, d.n_ctx, cs);
-            PS_LAUNCH_CK();
+            PS_DEP(pv, dim3((unsigned)((hs + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->att, pl + d.max_batch, ctx->kq, (int)hs, (int)nh, (int)nkv, ctx->pos_dev, d.n_ctx, cs);
         } else {
-        launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs);
-        PS_LAUNCH_CK();
-        ps_k_softmax_ext<<<(unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->stream>>>(ctx->kq, ctx->kq, tree ? ctx->tree_bias : nullptr, ctx->pos_dev, n_kv, bs, kq_scale);
-        PS_LAUNCH_CK();
+        if ((rc = launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs))) return rc;
+        PS_DEP(ps_k_softmax_ext, (unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->kq, ctx->kq, tree ? ctx->tree_bias : nullptr, ctx->pos_dev, n_kv, bs, kq_scale);
         if ((rc = launch_batch_pv(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs, ctx->opt_pv_batch_min))) return rc;
-        PS_LAUNCH_CK();
         }
         if (tc) {
             if ((rc = tc_single(ctx, {ctx->att}, ld.tc_o, (int)dim, (int)qdim, ctx->x, bs, ctx->x))) return rc;
@@ -2383,12 +2372,10 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
             if ((rc = launch_rwm(ctx, a))) return rc;
         }
         if ((rc = launch_rope_kv(ctx, L, (int)nh, (int)nkv, bs))) return rc;
-        launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs);
-        PS_LAUNCH_CK();
+        if ((rc = launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs))) return rc;
         ps_k_softmax_ext<<<(unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->stream>>>(ctx->kq, ctx->kq, nullptr, ctx->pos_dev, n_kv, bs, kq_scale);
         PS_LAUNCH_CK();
         if ((rc = launch_batch_pv(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs, 0))) return rc;
-        PS_LAUNCH_CK();
         if ((rc = tp_gather_rows(ctx, attb, ctx->att, bs, qdim_l))) return rc;                      // exchange 1: attention output
         if (tc) {
             if ((rc = tc_single(ctx, {attb}, ld.tc_o, (int)dim_l, (int)qdim, xl, bs, xl))) return rc;       // x[rows of this rank] += Wo[rows] . att
@@ -2659,8 +2646,7 @@ int ps_cuda_forward_sessions(ps_cuda_ctx *ctx, const int32_t *session_ids, const
     ctx->logits_last = ctx->logits;
     ctx->logits_rows = lm_head ? n : 0;
     if (lm_head && greedy_ids) {
-        ps_k_argmax<<<n, 1024, 0, ctx->stream>>>(ctx->logits, d.vocab_size, ctx->ids_dev, ctx->ids_dev + d.max_batch); // one CTA per column
-        PS_LAUNCH_CK();
+        PS_DEP(ps_k_argmax, n, 1024, 0, ctx->logits, d.vocab_size, ctx->ids_dev, ctx->ids_dev + d.max_batch); // one CTA per column
         PS_CK(cudaMemcpyAsync(ctx->h_ids, ctx->ids_dev, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     }
     PS_CK(cudaEventRecord(ctx->ev1, ctx->stream));
@@ -2724,16 +2710,13 @@ int ps_cuda_forward_tree(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t 
         ctx->slot_mask_dirty = false;
     }
     PS_CK(cudaEventRecord(ctx->ev0, ctx->stream));
-    ps_k_tree_mask<<<dim3((unsigned)std::min<int64_t>((base + bs + 255) / 256, 64), (unsigned)bs), 256, 0, ctx->stream>>>(ctx->tree_bias, ctx->slot_mask_dev, ctx->tree_dev, base, bs,
-                                                                                                                        base + bs);
-    PS_LAUNCH_CK();
+    PS_DEP(ps_k_tree_mask, dim3((unsigned)std::min<int64_t>((base + bs + 255) / 256, 64), (unsigned)bs), 256, 0, ctx->tree_bias, ctx->slot_mask_dev, ctx->tree_dev, base, bs, base + bs);
     int rc = forward_ops(ctx, bs, lm_head, 0, base);
     if (rc) return rc;
     PS_CK(cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->logits_last = ctx->logits;
     if (lm_head == 2) { // greedy ids only (ProbArray + greedy_sample with top_k = 1 per row, first maximum): bs ints come back instead of bs x vocab floats
-        ps_k_argmax<<<bs, 1024, 0, ctx->stream>>>(ctx->logits, ctx->d.vocab_size, ctx->ids_dev, ctx->ids_dev + 2048); // one CTA per tree node
-        PS_LAUNCH_CK();
+        PS_DEP(ps_k_argmax, bs, 1024, 0, ctx->logits, ctx->d.vocab_size, ctx->ids_dev, ctx->ids_dev + 2048); // one CTA per tree node
         PS_CK(cudaMemcpyAsync(ctx->h_ids, ctx->ids_dev, (size_t)bs * 4, cudaMemcpyDeviceToHost, ctx->stream));
         if ((rc = sync_and_check(ctx))) return rc;
         memcpy(logits_host, ctx->h_ids, (size_t)bs * 4);

@@ -6,6 +6,7 @@
 // them, and the fp32 accumulation chains are replayed in the reference's order (see ps_math.cuh).
 #pragma once
 #include "ps_math.cuh"
+#include "ps_ptx.cuh"
 
 #define PS_FULL 0xffffffffu
 
@@ -168,6 +169,7 @@ __device__ __forceinline__ void ps_act8(const float *__restrict__ x, const float
 }
 __global__ void __launch_bounds__(128) ps_k_quantize_q8k(const float *__restrict__ x, const float *__restrict__ u, int64_t K, uint32_t *__restrict__ qs, float *__restrict__ dq,
                                                          uint32_t *__restrict__ bsp) {
+    ps_grid_dep();
     const int lane = threadIdx.x & 31;
     const int64_t nb = K / 256, i = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5), col = blockIdx.y, at = col * K + i * 256;
     if (i >= nb) return;
@@ -176,6 +178,7 @@ __global__ void __launch_bounds__(128) ps_k_quantize_q8k(const float *__restrict
     ps_store_q8k(e, lane, i, col, nb, qs, dq, bsp);
 }
 __global__ void __launch_bounds__(128) ps_k_quantize_q80(const float *__restrict__ x, const float *__restrict__ u, int64_t K, uint32_t *__restrict__ qs, float *__restrict__ dq) {
+    ps_grid_dep();
     const int lane = threadIdx.x & 31;
     const int64_t nb = K / 32, i = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * 4 + (lane >> 3), col = blockIdx.y, at = col * K + i * 32 + 4 * (lane & 7);
     const bool valid = i < nb;
@@ -364,6 +367,7 @@ template <int TYPE>
 __global__ void __launch_bounds__(256) ps_k_matmul_q(const uint8_t *__restrict__ w, int64_t K, int64_t N, const uint32_t *__restrict__ aqs, const float *__restrict__ ad,
                                                      const uint32_t *__restrict__ absp, float *__restrict__ dst, const float *__restrict__ bias,
                                                      const float *__restrict__ residual) {
+    ps_grid_dep();
     using B = PsBlk<TYPE>;
     constexpr bool KQ = (B::ELEMS == 256);
     extern __shared__ __align__(16) uint8_t smem[];
@@ -505,6 +509,7 @@ template <int C> PS_D void ps_mb_stage32(uint32_t *s_qs, float *s_d, const uint3
 // REST: 32-element blocks whose number is no multiple of four
 template <int TYPE, int R, int C, bool REST>
 __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArgs a) {
+    ps_grid_dep();
     using B = PsBlk<TYPE>;
     constexpr bool KQ = (B::ELEMS == 256);
     extern __shared__ __align__(16) uint8_t smem[];
@@ -637,6 +642,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_qb(const PsMbArg
 // the other took 8.6 us on rows of 4096).
 __global__ void __launch_bounds__(256) ps_k_get_embedding(float *__restrict__ dst, const uint8_t *__restrict__ w, int type,
                                                           int64_t dim, const int32_t *__restrict__ tokens) {
+    ps_grid_dep();
     const int64_t tok = tokens[blockIdx.x];
     const uint8_t *row = w + tok * ps_row_bytes(type, dim);
     float *y = dst + (int64_t)blockIdx.x * dim;
@@ -725,6 +731,7 @@ __device__ __forceinline__ float ps_rms_scale(const float *__restrict__ xr, int6
 }
 __global__ void __launch_bounds__(256) ps_k_rmsnorm(float *__restrict__ dst, const float *__restrict__ x, const float *__restrict__ w,
                                                     int64_t dim, float eps) {
+    ps_grid_dep();
     __shared__ double sh[32];
     const float *xr = x + (int64_t)blockIdx.x * dim;
     float *yr = dst + (int64_t)blockIdx.x * dim;
@@ -739,6 +746,7 @@ __device__ __forceinline__ float4 ps_norm4(const float *__restrict__ x, const fl
 // a trip through memory lay between them (32 rows of 896: 5.3 + 3.2 us, together 5.7)
 template <bool Q8K> __global__ void __launch_bounds__(512) ps_k_norm_quantize(const float *__restrict__ x, const float *__restrict__ w, int64_t dim, float eps, uint32_t *__restrict__ qs,
                                                                              float *__restrict__ dq, uint32_t *__restrict__ bsp) {
+    ps_grid_dep();
     __shared__ double sh[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t col = blockIdx.x, nb = dim / (Q8K ? 256 : 32);
@@ -800,6 +808,7 @@ struct PsRopeKv {
     int64_t n_ctx, base;
 };
 __global__ void __launch_bounds__(256) ps_k_rope_kv_batch(const PsRopeKv a) {
+    ps_grid_dep();
     const int hs = a.head_size, kvd = a.nkv * hs, half = hs / 2, per = (a.nh + a.nkv) * half, n_p = (per + 255) / 256; // pairs of a token, CTAs for them
     const int64_t slot0 = a.base >= 0 ? a.base : (int64_t)a.pos[0];
     if ((int)blockIdx.x < n_p * a.bs) {
@@ -864,6 +873,7 @@ __global__ void ps_k_kv_move_slot(float *const *__restrict__ kv, int n_layers, i
 // tree[i][j - base].  mask {n_kv, bs}, 0 or -inf, the layout softmax_ext expects.
 __global__ void ps_k_tree_mask(float *__restrict__ mask, const uint8_t *__restrict__ slot_mask, const uint8_t *__restrict__ tree, int64_t base,
                                int64_t bs, int64_t n_kv) {
+    ps_grid_dep();
     const int64_t i = blockIdx.y;
     for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < n_kv; j += (int64_t)gridDim.x * blockDim.x) {
         const bool vis = j < base ? !slot_mask[j] : tree[i * bs + (j - base)] != 0;
@@ -883,6 +893,7 @@ __global__ void ps_k_get_mask(float *__restrict__ mask, int64_t n_kv, const int3
 // every batch column.  kq {n_kv, bs, n_heads}.
 __global__ void __launch_bounds__(128) ps_k_attn_scores(float *__restrict__ kq, const float *__restrict__ kc, const float *__restrict__ q,
                                                         int hs, int n_heads, int n_kv_heads, int64_t n_kv, int bs) {
+    ps_grid_dep();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t j = (int64_t)blockIdx.x * 4 + warp;
     const int g = blockIdx.y;
@@ -935,6 +946,7 @@ __global__ void __launch_bounds__(128) ps_k_attn_scores(float *__restrict__ kq, 
 // nullptr -> no mask at all (GGMLBackend::softmax: ggml_compute_forward_soft_max_f32 with src1 == NULL).
 __global__ void __launch_bounds__(256) ps_k_softmax_ext(float *__restrict__ dst, const float *__restrict__ x, const float *__restrict__ mask,
                                                         const int32_t *__restrict__ pos, int64_t ne0, int64_t ne1, float scale) {
+    ps_grid_dep();
     extern __shared__ float wp[];
     __shared__ double sh[32];
     __shared__ float shf[32];
@@ -981,6 +993,7 @@ __global__ void __launch_bounds__(256) ps_k_softmax_ext(float *__restrict__ dst,
 // One warp per (kv head g, d): the V^T row is streamed once for all heads of the group and all columns.
 __global__ void __launch_bounds__(128) ps_k_attn_pv(float *__restrict__ out, const float *__restrict__ vct, const float *__restrict__ p,
                                                     int hs, int n_heads, int n_kv_heads, int64_t n_kv, int64_t n_ctx, int bs) {
+    ps_grid_dep();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int d = blockIdx.x * 4 + warp, g = blockIdx.y;
     if (d >= hs) return;
@@ -1007,6 +1020,7 @@ __global__ void __launch_bounds__(128) ps_k_attn_pv(float *__restrict__ out, con
 // (ggml_vec_dot_f32 lane order and GGML_F32x8_REDUCE order, exactly as in ps_k_attn_scores).
 __global__ void __launch_bounds__(128) ps_k_attn_scores_batch(float *__restrict__ kq, const float *__restrict__ kc, const float *__restrict__ q,
                                                               int hs, int n_heads, int n_kv_heads, int64_t n_kv, int bs, int qb) {
+    ps_grid_dep();
     extern __shared__ float s_qb[]; // [qb * r2][hs]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = blockIdx.y, r2 = n_heads / n_kv_heads, steps = hs / 32;
@@ -1066,6 +1080,7 @@ __global__ void __launch_bounds__(128) ps_k_attn_scores_batch(float *__restrict_
 #define PS_PV_QB 8
 __global__ void __launch_bounds__(256) ps_k_attn_pv_batch(float *__restrict__ out, const float *__restrict__ vct, const float *__restrict__ p,
                                                           int hs, int n_heads, int n_kv_heads, int64_t n_kv, int64_t n_ctx, int bs) {
+    ps_grid_dep();
     extern __shared__ float s_pq[]; // [PS_PV_QB][n_kv]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int i0 = blockIdx.x * PS_PV_QB, h = blockIdx.y, g = h / (n_heads / n_kv_heads);
@@ -1134,6 +1149,7 @@ __global__ void __launch_bounds__(256) ps_k_attn_pv_batch(float *__restrict__ ou
 template <int STEPS> // head size / 32: the loops below carry no run-time predicates
 __global__ void __launch_bounds__(128) ps_k_attn_scores_tile(float *__restrict__ kq, const float *__restrict__ kc, const float *__restrict__ q,
                                                              int n_heads, int n_kv_heads, int64_t n_kv, int bs, int qb) {
+    ps_grid_dep();
     extern __shared__ float s_qb[]; // [qb * r2][hs]
     constexpr int hs = 32 * STEPS;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, c = lane >> 2;
@@ -1213,6 +1229,7 @@ template <int N> PS_D void ps_cp_async_wait() { asm volatile("cp.async.wait_grou
 template <bool VEC, int DEPTH>
 __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ out, const float *__restrict__ vct, const float *__restrict__ p,
                                                             int hs, int n_heads, int n_kv_heads, int64_t n_kv, int64_t n_ctx, int bs) {
+    ps_grid_dep();
     // [ring: 8 warps][DEPTH][PS_PVT_D][32] V^T chunks, then the probabilities, position-major: s_p4[j] = queries 0..3
     // at position j, s_p4[n_kv + j] = queries 4..7, so a lane fetches its eight probabilities of a chunk with two
     // conflict-free 16-byte loads off one address register
@@ -1400,6 +1417,7 @@ __global__ void __launch_bounds__(128) ps_k_matmul_f32(float *__restrict__ dst, 
 // of 32 query and 8 kv heads: 47.6 us; with P.V below 94 a layer, now 34)
 template <int STEPS> __global__ void __launch_bounds__(128) ps_k_sess_scores(float *__restrict__ kq, const float *const *__restrict__ kc_ptrs, const float *__restrict__ q,
                                                                            int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t col_stride) {
+    ps_grid_dep();
     constexpr int hs = 32 * STEPS;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z, g = blockIdx.y, code = lane >> 2;
     const int64_t n_kv = (int64_t)pos[c] + 1, j0 = ((int64_t)blockIdx.x * 4 + warp) * 8;
@@ -1440,6 +1458,7 @@ template <int STEPS> __global__ void __launch_bounds__(128) ps_k_sess_scores(flo
 
 // softmax_ext of column c with the position mask of GET_MASK (every j <= pos: + 0.0f), rows of n_kv_c; grid (n_heads, n)
 __global__ void __launch_bounds__(256) ps_k_sess_softmax(float *__restrict__ kq, const int32_t *__restrict__ pos, int64_t col_stride, float scale) {
+    ps_grid_dep();
     extern __shared__ float wp[];
     __shared__ double sh[32];
     __shared__ float shf[32];
@@ -1487,6 +1506,7 @@ PS_D float ps_ld_now(const float *p) { float v; asm volatile("ld.global.f32 %0, 
 // the weights were read 128 times over and every sum took five shuffles (64 sessions of 100 to 200 positions, a layer of 32 query and 8 kv heads: 46.6 us).  After the reduction lane (dim, head) owns one sum and adds the leftover products to it in order
 template <int HB> __global__ void __launch_bounds__(128) ps_k_sess_pv(float *__restrict__ out, const float *const *__restrict__ vct_ptrs, const float *__restrict__ kq, int hs,
                                                     int n_heads, int n_kv_heads, const int32_t *__restrict__ pos, int64_t n_ctx, int64_t col_stride) {
+    ps_grid_dep();
     __shared__ float s_left[4][8 + HB][32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c = blockIdx.z, g = blockIdx.y, d0 = (blockIdx.x * 4 + warp) * 8;
     if (d0 >= hs) return; // (hs is a multiple of eight)
@@ -1639,6 +1659,7 @@ __global__ void __launch_bounds__(1024) ps_k_topk_stage2(const unsigned long lon
 // greedy pick (Model::decode with top_k = 1: ProbArray + greedy_sample, src/model/llama/llama_model.cpp:124-128):
 // first maximum wins.  One CTA; writes the id to `out[step]` and to `next_token` (device feedback for the next step).
 __global__ void __launch_bounds__(1024) ps_k_argmax(const float *__restrict__ logits, int64_t n, int32_t *__restrict__ out, int32_t *__restrict__ next_token) {
+    ps_grid_dep();
     __shared__ float sv[32];
     __shared__ int si[32];
     // one CTA per logits row (gridDim.x rows: the columns of a session batch); a single row for the decode loop

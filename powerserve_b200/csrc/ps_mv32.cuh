@@ -399,6 +399,7 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
                 ps_bulk_g2s(sw + (size_t)b0 * G::BLK, seg.w + ((size_t)oct * nb + b0) * G::BLK, bytes, &bar[warp][p]);
             }
     }
+    ps_grid_dep(); // (the weights are on their way)
     ps_mb_stage32<C>(s_qs, s_d, a.aqs + (int64_t)col0 * nb * 8, a.ad + (int64_t)col0 * nb, nb, nbg, ncol);
     __syncthreads();
     if (oct >= n_oct) return;

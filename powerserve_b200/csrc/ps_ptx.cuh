@@ -37,6 +37,13 @@ PS_D void ps_bulk_g2s(void *dst_smem, const void *src_gmem, uint32_t bytes, uint
 PS_D void ps_fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 PS_D void ps_grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 PS_D void ps_grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Programmatic dependent launch.  A kernel launched by launch_k / pa_launch_dep may start while the one before it in the stream still runs; nothing
+// that other kernels write is read, and nothing they read is written, before this wait, which ends when the kernel before is complete (and, as that one
+// waited too, all before it).  Every kernel launched that way waits in all threads that touch global memory.  After it the next kernel may start
+PS_D void ps_grid_dep() {
+    ps_grid_dep_wait();
+    ps_grid_dep_launch();
+}
 PS_D void ps_bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 
 // ---------------------------------------------------------------------------------------------------- tcgen05 helpers

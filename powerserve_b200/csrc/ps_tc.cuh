@@ -155,6 +155,7 @@ __device__ __forceinline__ void ps_tc_store_b(uint8_t *__restrict__ out, int NT,
     if (lane == 0) reinterpret_cast<float *>(out + nbp * NT * 640)[i * NT + c] = yd;
 }
 __global__ void __launch_bounds__(128) ps_k_tc_prep_b(uint8_t *__restrict__ dst, const float *__restrict__ x, const float *__restrict__ u, int64_t K, int bs, int NT) {
+    ps_grid_dep();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nb = K / 256, nbp = (nb + 1) & ~(int64_t)1, i = (int64_t)blockIdx.x * 4 + warp;
     const int col = blockIdx.y, ct = col / NT, c = col % NT;
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(128) ps_k_tc_prep_b(uint8_t *__restrict__ dst,
 }
 // the same behind a norm, one CTA a column (128 columns of 4096: 7.0 + 4.2 us as two launches, together 6.2)
 __global__ void __launch_bounds__(512) ps_k_tc_norm_b(uint8_t *__restrict__ dst, const float *__restrict__ x, const float *__restrict__ w, int64_t dim, float eps, int bs, int NT) {
+    ps_grid_dep();
     __shared__ double sh[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t nb = dim / 256, nbp = (nb + 1) & ~(int64_t)1;
@@ -275,6 +277,34 @@ PS_D int ps_tc_owner(int q, int n_cta, int n_tiles) {
     return (int)(((int64_t)(q + 1) * n_cta + n - 1) / n) - 1;
 }
 
+// where the operands of pass q lie, and the copies of its step i into a stage
+template <int NT> struct PsTcSrc {
+    const uint8_t *aq, *as, *ad, *bq, *by;
+    bool lanes;
+    PS_D PsTcSrc(const PsTcArgs &a, int q) {
+        const int tile = q / PS_TC_PASSES, p = q % PS_TC_PASSES;
+        const uint8_t *pa = a.a + (size_t)(tile / a.n_ct) * a.nbp * PS_TC_A_BLOCK, *pb = a.b + (size_t)(tile % a.n_ct) * a.nbp * PS_TC_B_BLOCK(NT);
+        lanes = p < 4;
+        aq = pa + (lanes ? (size_t)p * a.nbp * PS_TC_A_Q : PS_TC_A_OFF_MN(a.nbp));
+        as = pa + PS_TC_A_OFF_SC(a.nbp);
+        ad = pa + (lanes ? PS_TC_A_OFF_D(a.nbp) : PS_TC_A_OFF_DM(a.nbp));
+        bq = pb + (lanes ? (size_t)p * a.nbp * (NT * 128) : (size_t)a.nbp * (NT * 512) + (size_t)(p - 4) * a.nbp * (NT * 64));
+        by = pb + (size_t)a.nbp * (NT * 640);
+    }
+    PS_D void weights(int i, uint8_t *sm, uint8_t *sf, uint64_t *bar) const {
+        const uint32_t na = lanes ? 2 * PS_TC_A_Q : 2 * PS_TC_A_MN;
+        ps_mbar_expect_tx(bar, na + (lanes ? 2 * PS_TC_A_SC : 0) + 2 * PS_TC_A_D + (lanes ? 2 * NT * 128 : 2 * NT * 64) + 2 * NT * 4);
+        ps_bulk_g2s(sm, aq + (size_t)i * na, na, bar);
+        if (lanes) ps_bulk_g2s(sm + PsTc<NT>::STAGE_SC, as + (size_t)i * (2 * PS_TC_A_SC), 2 * PS_TC_A_SC, bar);
+        ps_bulk_g2s(sf, ad + (size_t)i * (2 * PS_TC_A_D), 2 * PS_TC_A_D, bar);
+    }
+    PS_D void columns(int i, uint8_t *sm, uint8_t *sf, uint64_t *bar) const {
+        const uint32_t nb = lanes ? 2 * NT * 128 : 2 * NT * 64;
+        ps_bulk_g2s(sm + PsTc<NT>::STAGE_B, bq + (size_t)i * nb, nb, bar);
+        ps_bulk_g2s(sf + 2 * PS_TC_A_D, by + (size_t)i * (2 * NT * 4), 2 * NT * 4, bar);
+    }
+};
+
 template <int NT>
 __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcArgs a) {
     using T = PsTc<NT>;
@@ -320,45 +350,37 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcA
             // ===== TMA producer
             PsRing<T::NS> st;
             PsRing<T::NY> sy;
-            int g = 0;
+            int g = 0, ahead = 0;
             bool ok = warp != a.give_up;
             if (!ok) *a.err = 1;
+            // the weights of the first steps do not depend on the kernel before: they are asked for while it still runs
+            if (ok && q0 < q1) {
+                const PsTcSrc<NT> src(a, q0);
+                ahead = min(ns, T::NS);
+                if (ps_elect_one())
+                    for (int i = 0; i < ahead; i++) src.weights(i, ps_tc_smem + (size_t)i * T::STAGE, ps_tc_fact + i * T::FACT, &bar_full[i]);
+                __syncwarp();
+            }
+            ps_grid_dep();
             for (int q = q0; q < q1 && ok; q++) {
-                const int tile = q / PS_TC_PASSES, p = q % PS_TC_PASSES;
-                const bool lanes = p < 4;
-                const uint8_t *pa = a.a + (size_t)(tile / a.n_ct) * a.nbp * PS_TC_A_BLOCK, *pb = a.b + (size_t)(tile % a.n_ct) * a.nbp * PS_TC_B_BLOCK(NT);
-                const uint8_t *aq = pa + (lanes ? (size_t)p * a.nbp * PS_TC_A_Q : PS_TC_A_OFF_MN(a.nbp)), *as = pa + PS_TC_A_OFF_SC(a.nbp);
-                const uint8_t *ad = pa + (lanes ? PS_TC_A_OFF_D(a.nbp) : PS_TC_A_OFF_DM(a.nbp));
-                const uint8_t *bq = pb + (lanes ? (size_t)p * a.nbp * (NT * 128) : (size_t)a.nbp * (NT * 512) + (size_t)(p - 4) * a.nbp * (NT * 64));
-                const uint8_t *by = pb + (size_t)a.nbp * (NT * 640);
-                const uint32_t na = lanes ? 2 * PS_TC_A_Q : 2 * PS_TC_A_MN, nbb = lanes ? 2 * NT * 128 : 2 * NT * 64;
-                const uint32_t total = na + (lanes ? 2 * PS_TC_A_SC : 0) + 2 * PS_TC_A_D + nbb + 2 * NT * 4;
+                const PsTcSrc<NT> src(a, q);
                 for (int i = 0; i < ns; i++, g++, st.step(), sy.step()) {
                     // the MMAs of stage g - NS are complete: its operands have been read; entries three super-blocks before have been drained, and
                     // with them the factors of stage g - NS - 2
                     if (g >= T::NS && !ps_tc_wait_warp(&bar_empty[st.i], st.round ^ 1, a.limit)) { *a.err = 1; ok = false; break; }
                     uint8_t *sm = ps_tc_smem + (size_t)st.i * T::STAGE, *sf = ps_tc_fact + sy.i * T::FACT;
-                    uint64_t *bar = &bar_full[st.i];
                     if (ps_elect_one()) {
-                        ps_mbar_expect_tx(bar, total);
-                        ps_bulk_g2s(sm, aq, na, bar);
-                        ps_bulk_g2s(sm + T::STAGE_B, bq, nbb, bar);
-                        if (lanes) ps_bulk_g2s(sm + T::STAGE_SC, as, 2 * PS_TC_A_SC, bar);
-                        ps_bulk_g2s(sf, ad, 2 * PS_TC_A_D, bar);
-                        ps_bulk_g2s(sf + 2 * PS_TC_A_D, by, 2 * NT * 4, bar);
+                        if (g >= ahead) src.weights(i, sm, sf, &bar_full[st.i]);
+                        src.columns(i, sm, sf, &bar_full[st.i]);
                     }
                     __syncwarp();
-                    aq += na;
-                    bq += nbb;
-                    as += 2 * PS_TC_A_SC;
-                    ad += 2 * PS_TC_A_D;
-                    by += 2 * NT * 4;
                 }
             }
             // copies in flight end before the CTA does (they have, unless a wait gave up)
             for (int k = g > T::NS ? g - T::NS : 0; k < g; k++)
                 if (!ps_tc_wait(&bar_full[k % T::NS], (k / T::NS) & 1)) { *a.err = 5; break; }
         } else if (warp == W_MMA) {
+            ps_grid_dep_wait();
             // ===== MMA issuer.  The warp stays converged and one thread, chosen by elect.sync, issues, so that descriptors and barrier addresses
             // live in uniform registers
             // kind::f16, D = F32 (bit 4), A = B = F16, K-major both, N >> 3 @ bit 17, M >> 4 @ bit 24
@@ -405,6 +427,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcA
         // ===== de-quantising warps: a warpgroup takes super-block d of a step, of every second step where there are four; thread = row (warp % 4 is its
         // tensor-memory lane quadrant)
         ps_reg_dec<T::R_DEQ>();
+        ps_grid_dep_wait(); // (nothing here reads global memory: the limits of the waits below count from here)
         const int group = (warp - T::EW) >> 2, d = group & 1, quad = warp & 3, row = quad * 32 + lane;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + T::TM_A + (T::XE == 2 ? d * 32 : 0);
         PsRing<T::NS> st;
@@ -472,6 +495,7 @@ __global__ void __launch_bounds__(PsTc<NT>::THREADS, 1) ps_k_tc_gemm(const PsTcA
     } else {
         // ===== epilogue: warp w owns tensor-memory lanes 32 * (w % 4) .. +31 (rows) and EC columns
         ps_reg_inc<T::R_EPI>();
+        ps_grid_dep_wait();
         const int quad = warp & 3, row = quad * 32 + lane, c0 = (warp >> 2) * T::EC;
         const uint32_t t_lane = tmem_base + ((uint32_t)(quad * 32) << 16) + c0;
         constexpr int ET = T::EW * 32, US = T::EC * ET;
