@@ -21,6 +21,7 @@
 typedef __nv_bfloat16 bf16;
 namespace cg = cooperative_groups;
 
+#include "ps_ptx.cuh"
 #include "ps_arch_kernels.cuh"
 #include "ps_arch_decode.cuh"
 #include "ps_arch_recur.cuh"
@@ -298,6 +299,8 @@ cudaError_t pa_launch_cluster(bool pdl, int n_cl, void (*kern)(KArgs...), dim3 g
     cfg.numAttrs = pdl ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
 }
+// pdl: programmatic dependence on the kernel before (ps_grid_dep).  Not for pa_k_pv, whose few CTAs compute for tens of microseconds: those that come
+// early crowd on the SMs that are free first (16 heads x 256 queries x 1024 keys: a pass 372 us early, 316 when the soft-max has gone)
 template <typename... KArgs, typename... Args>
 cudaError_t pa_launch_dep(bool pdl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg{};
@@ -1154,25 +1157,32 @@ static int pa_cuts(int64_t N, int K) {
 }
 static bool pa_narrow_tiles(int n_sm, int64_t N, int bs) { return ((N + PA_TN - 1) / PA_TN) * ((bs + PA_TM - 1) / PA_TM) < n_sm; }
 template <typename... KArgs, typename... Args>
-static cudaError_t pa_launch_cut(int S, void (*kern)(KArgs...), dim3 grid, cudaStream_t st, Args... args) {
+static cudaError_t pa_launch_cut(bool pdl, int S, void (*kern)(KArgs...), dim3 grid, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     cfg.gridDim = grid; cfg.blockDim = dim3(256); cfg.stream = st;
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = (unsigned)S;
     cfg.attrs = at;
-    cfg.numAttrs = S > 1 ? 1 : 0;
+    if (pdl) {
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs++;
+    }
+    if (S > 1) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        at[cfg.numAttrs].val.clusterDim.x = at[cfg.numAttrs].val.clusterDim.y = 1;
+        at[cfg.numAttrs].val.clusterDim.z = (unsigned)S;
+        cfg.numAttrs++;
+    }
     return cudaLaunchKernelEx(&cfg, kern, (KArgs)args...);
 }
 template <bool ROUND, bool CUT = !ROUND>
-static void pa_launch_linear(int n_sm, int N, int bs, int heads, cudaStream_t st, const float *A, int lda, const bf16 *W, const float *bias, float *C, int ldc, int M, int n, int K,
+static void pa_launch_linear(bool pdl, int n_sm, int N, int bs, int heads, cudaStream_t st, const float *A, int lda, const bf16 *W, const float *bias, float *C, int ldc, int M, int n, int K,
                              int a_gs = 0, int c_gs = 0, int act_from = 1 << 30, int gap = 0, PaAct act = PaAct{}, PaRowMul mul = PaRowMul{}) {
     const unsigned nt = (unsigned)((N + PA_TN - 1) / PA_TN);
     const int S = CUT ? pa_cuts((int64_t)nt * PA_TN * heads, K) : 1;
     const bool narrow = pa_narrow_tiles(n_sm, (int64_t)nt * PA_TN * heads * S, bs);
     const int tm = narrow ? 32 : PA_TM;
-    pa_launch_cut(S, narrow ? pa_k_linear<ROUND, 32> : pa_k_linear<ROUND, PA_TM>, dim3(nt, (unsigned)((bs + tm - 1) / tm), (unsigned)(heads * S)), st, A, lda, W, bias, C, ldc, M, n, K, S,
+    pa_launch_cut(pdl, S, narrow ? pa_k_linear<ROUND, 32> : pa_k_linear<ROUND, PA_TM>, dim3(nt, (unsigned)((bs + tm - 1) / tm), (unsigned)(heads * S)), st, A, lda, W, bias, C, ldc, M, n, K, S,
                   a_gs, c_gs, act_from, gap, act, mul);
 }
 
@@ -1215,14 +1225,14 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     auto tc_dense = [&](const float *X, int ldx, int M, int K, const uint8_t *wt, int N, const float *bias, float *C, int ldc, const PaAct *act1 = nullptr, int act_from = 0,
                         int gap = 0, const PaRowMul *mul = nullptr) -> int {
         const int nkb = (K + PT_KB - 1) / PT_KB, n_ct = (M + PT_N - 1) / PT_N, n_rt = (N + PT_M - 1) / PT_M;
-        pa_k_tc_prep_x<<<dim3((unsigned)nkb, (unsigned)n_ct), 256, 0, st>>>(a->tcx, X, ldx, M, K, nkb, nullptr, nullptr, nullptr, nullptr, nullptr);
+        pa_launch_dep(pdl, pa_k_tc_prep_x, dim3((unsigned)nkb, (unsigned)n_ct), dim3(256), 0, st, a->tcx, X, ldx, M, K, nkb, nullptr, nullptr, nullptr, nullptr, nullptr);
         PA_LAUNCH();
         PtArgs g{};
         g.a0 = wt; g.b = a->tcx; g.nkb = nkb; g.n_rt = n_rt; g.n_ct = n_ct; g.M = M; g.N = N; g.mode = PT_MODE_DENSE; g.C = C; g.ldc = ldc; g.bias = bias; g.err = io.err_dev;
         if (act1) { g.act = *act1; g.act1 = 1; g.act_from = act_from; g.gap = gap; }
         if (mul) g.mul = *mul;
         const int ctas = cut_tiles(g);
-        pa_k_tc_gemm<1><<<ctas, PT_THREADS, PT_SMEM, st>>>(g);
+        pa_launch_dep(pdl, pa_k_tc_gemm<1>, dim3(ctas), dim3(PT_THREADS), PT_SMEM, st, g);
         PA_LAUNCH();
         return 0;
     };
@@ -1230,13 +1240,13 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     // y = X W^T for a batch: tensor cores on rounded operands, or the fp32-FMA tiles
     auto linear = [&](const float *X, int ldx, int K, const bf16 *W, const uint8_t *Wt, int N, float *Cout, int ldc) -> int {
         if (tc) return tc_dense(X, ldx, bs, K, Wt, N, nullptr, Cout, ldc);
-        pa_launch_linear<ROUND>(a->n_sm, N, bs, 1, st, X, ldx, W, nullptr, Cout, ldc, bs, N, K, 0, 0);
+        pa_launch_linear<ROUND>(pdl, a->n_sm, N, bs, 1, st, X, ldx, W, nullptr, Cout, ldc, bs, N, K, 0, 0);
         PA_LAUNCH();
         return 0;
     };
     // per-head products (blockIdx.z = head): fp32-FMA tiles in both modes
     auto linear_heads = [&](const float *X, int ldx, int x_gs, int K, const bf16 *W, int N, float *Cout, int ldc, int c_gs, int heads) -> int {
-        pa_launch_linear<ROUND>(a->n_sm, N, bs, (int)heads, st, X, ldx, W, nullptr, Cout, ldc, bs, N, K, x_gs, c_gs);
+        pa_launch_linear<ROUND>(pdl, a->n_sm, N, bs, (int)heads, st, X, ldx, W, nullptr, Cout, ldc, bs, N, K, x_gs, c_gs);
         PA_LAUNCH();
         return 0;
     };
@@ -1247,11 +1257,11 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         const int tile0 = lo0 / PA_TN, tok_tiles = (int)cdiv(n_kv, PA_TN) - tile0;
         // pooled blocks the batch's last query sees: further key tiles behind the token tiles
         const int nv = (at.pool > 0 && n_kv - at.window >= at.pool) ? (n_kv - at.window) / at.pool : 0;
-        pa_k_scores<<<dim3(tok_tiles + cdiv(nv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st>>>(at, q, ldq, io.kc[li], kd, a->S, io.pos_dev, bs, tile0, tok_tiles);
+        pa_launch_dep(pdl, pa_k_scores, dim3(tok_tiles + cdiv(nv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st, at, q, ldq, io.kc[li], kd, a->S, io.pos_dev, bs, tile0, tok_tiles);
         PA_LAUNCH();
-        pa_k_mix_softmax<<<bs, 256, 4 * (size_t)at.H * at.H, st>>>(at, a->S, io.pos_dev, bs);
+        pa_launch_dep(pdl, pa_k_mix_softmax, dim3(bs), dim3(256), 4 * (size_t)at.H * at.H, st, at, a->S, io.pos_dev, bs);
         PA_LAUNCH();
-        pa_k_pv<!ROUND><<<dim3(cdiv(at.dv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st>>>(at, a->S, io.vct[li], out, aw, io.pos_dev, bs);
+        pa_launch_dep(false, pa_k_pv<!ROUND>, dim3(cdiv(at.dv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st, at, a->S, io.vct[li], out, aw, io.pos_dev, bs);
         PA_LAUNCH();
         return 0;
     };
@@ -1261,7 +1271,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     const float *add_tok = nullptr, *add_vec = nullptr;
     auto seam = [&](float *h_out, const float *w_in, int ldh = 0) -> int {
         if (!pend_y && !h_out && !add_tok && !add_vec) return 0;
-        pa_k_seam_norm<<<dim3((unsigned)bs, (unsigned)groups), 256, 0, st>>>(a->x, pend_y, pend_w, h_out, w_in, dim, groups, d.norm_eps, center, add_tok, add_vec, a->res_scale, ldh > 0 ? ldh : dim);
+        pa_launch_dep(pdl, pa_k_seam_norm, dim3((unsigned)bs, (unsigned)groups), dim3(256), 0, st, a->x, pend_y, pend_w, h_out, w_in, dim, groups, d.norm_eps, center, add_tok, add_vec, a->res_scale, ldh > 0 ? ldh : dim);
         PA_LAUNCH();
         pend_y = pend_w = add_tok = add_vec = nullptr;
         return 0;
@@ -1301,40 +1311,37 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         const int top = l.top_k, E = l.n_experts, ff = l.expert_ff, n = bs * top;
         if (tc) {
             const int max_tiles = n / PT_N + E + 1, nkb1 = (dim + PT_KB - 1) / PT_KB, nkb2 = (ff + PT_KB - 1) / PT_KB;
-            pa_k_dispatch<<<1, 256, 0, st>>>(a->sel_e, a->sel_w, n, top, E, PT_N, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles);
+            pa_launch_dep(pdl, pa_k_dispatch, dim3(1), dim3(256), 0, st, a->sel_e, a->sel_w, n, top, E, PT_N, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles);
             PA_LAUNCH();
-            pa_k_tc_prep_x<<<dim3((unsigned)nkb1, (unsigned)max_tiles), 256, 0, st>>>(a->tcx, X, dim, n, dim, nkb1, a->n_tiles, a->tile_row0, a->tile_end, a->row_token,
-                                                                                    l.route_on_input ? a->row_w : nullptr);
+            pa_launch_dep(pdl, pa_k_tc_prep_x, dim3((unsigned)nkb1, (unsigned)max_tiles), dim3(256), 0, st, a->tcx, X, dim, n, dim, nkb1, a->n_tiles, a->tile_row0, a->tile_end, a->row_token, l.route_on_input ? a->row_w : nullptr);
             PA_LAUNCH();
             PtArgs g{};
             g.a0 = w.t_gate; g.a1 = w.t_up; g.b = a->tcx; g.nkb = nkb1; g.n_rt = (ff + PT_M - 1) / PT_M; g.n_ct = max_tiles; g.n_ct_dev = a->n_tiles;
             g.tile_e = a->tile_e; g.tile_row0 = a->tile_row0; g.tile_end = a->tile_end; g.M = n; g.N = ff; g.mode = PT_MODE_EXPERT_UP; g.C = a->y; g.ldc = ff;
             g.act = pa_act_of(l); g.err = io.err_dev;
             if (w.t_gate) {
-                pa_k_tc_gemm<2><<<std::min(a->n_sm, max_tiles * g.n_rt), PT_THREADS, PT_SMEM, st>>>(g);
+                pa_launch_dep(pdl, pa_k_tc_gemm<2>, dim3(std::min(a->n_sm, max_tiles * g.n_rt)), dim3(PT_THREADS), PT_SMEM, st, g);
             } else { // no gate
                 g.a0 = w.t_up; g.a1 = nullptr;
-                pa_k_tc_gemm<1><<<std::min(a->n_sm, max_tiles * g.n_rt), PT_THREADS, PT_SMEM, st>>>(g);
+                pa_launch_dep(pdl, pa_k_tc_gemm<1>, dim3(std::min(a->n_sm, max_tiles * g.n_rt)), dim3(PT_THREADS), PT_SMEM, st, g);
             }
             PA_LAUNCH();
-            pa_k_tc_prep_x<<<dim3((unsigned)nkb2, (unsigned)max_tiles), 256, 0, st>>>(a->tcx, a->y, ff, n, ff, nkb2, a->n_tiles, a->tile_row0, a->tile_end, nullptr, nullptr);
+            pa_launch_dep(pdl, pa_k_tc_prep_x, dim3((unsigned)nkb2, (unsigned)max_tiles), dim3(256), 0, st, a->tcx, a->y, ff, n, ff, nkb2, a->n_tiles, a->tile_row0, a->tile_end, nullptr, nullptr);
             PA_LAUNCH();
             PtArgs g2{};
             g2.a0 = w.t_down; g2.b = a->tcx; g2.nkb = nkb2; g2.n_rt = (dim + PT_M - 1) / PT_M; g2.n_ct = max_tiles; g2.n_ct_dev = a->n_tiles;
             g2.tile_e = a->tile_e; g2.tile_row0 = a->tile_row0; g2.tile_end = a->tile_end; g2.M = n; g2.N = dim; g2.mode = PT_MODE_EXPERT_DOWN; g2.C = a->slot; g2.ldc = dim;
             g2.row_token = a->row_token; g2.row_slot = a->row_slot; g2.row_w = a->row_w; g2.top = top; g2.on_input = l.route_on_input; g2.err = io.err_dev;
-            pa_k_tc_gemm<1><<<std::min(a->n_sm, max_tiles * g2.n_rt), PT_THREADS, PT_SMEM, st>>>(g2);
+            pa_launch_dep(pdl, pa_k_tc_gemm<1>, dim3(std::min(a->n_sm, max_tiles * g2.n_rt)), dim3(PT_THREADS), PT_SMEM, st, g2);
             PA_LAUNCH();
         } else {
             const int max_tiles = n / PA_TM + E + 1;
-            pa_k_dispatch<<<1, 256, 0, st>>>(a->sel_e, a->sel_w, n, top, E, PA_TM, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles);
+            pa_launch_dep(pdl, pa_k_dispatch, dim3(1), dim3(256), 0, st, a->sel_e, a->sel_w, n, top, E, PA_TM, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles);
             PA_LAUNCH();
             auto *up_kern = w.wgate ? pa_k_expert_up<ROUND, 2> : pa_k_expert_up<ROUND, 1>;
-            up_kern<<<dim3(cdiv(ff, PA_TN), max_tiles), blk, 0, st>>>(X, dim, a->row_token, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles, w.wgate, w.wup, a->y, ff, dim,
-                                                                      l.route_on_input, pa_act_of(l));
+            pa_launch_dep(pdl, up_kern, dim3(cdiv(ff, PA_TN), max_tiles), blk, 0, st, X, dim, a->row_token, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles, w.wgate, w.wup, a->y, ff, dim, l.route_on_input, pa_act_of(l));
             PA_LAUNCH();
-            pa_k_expert_down<ROUND><<<dim3(cdiv(dim, PA_TN), max_tiles), blk, 0, st>>>(a->y, ff, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end,
-                                                                                      a->n_tiles, w.wdown, a->slot, top, dim, ff, l.route_on_input);
+            pa_launch_dep(pdl, pa_k_expert_down<ROUND>, dim3(cdiv(dim, PA_TN), max_tiles), blk, 0, st, a->y, ff, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles, w.wdown, a->slot, top, dim, ff, l.route_on_input);
             PA_LAUNCH();
         }
         return 0;
@@ -1346,8 +1353,8 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         // (gate | up of 1024 x 1024 on 8 / 64 tokens: 18.7 / 19.6 us in 32-row tiles, 22.1 / 22.7 in 64-row ones; 512 x 2048: 23.4 / 31.2 and 26.5 / 27.4)
         const bool narrow = pa_narrow_tiles(a->n_sm, rows * S / (wg ? 2 : 1), bs);
         const dim3 grid(cdiv(ff, PA_TN), cdiv(bs, narrow ? 32 : PA_TM), (unsigned)S);
-        if (wg) pa_launch_cut(S, narrow ? pa_k_dense_up<ROUND, 2, 32> : pa_k_dense_up<ROUND, 2, PA_TM>, grid, st, X, dim, wg, wu, a->y, bs, ff, dim, act, S);
-        else pa_launch_cut(S, narrow ? pa_k_dense_up<ROUND, 1, 32> : pa_k_dense_up<ROUND, 1, PA_TM>, grid, st, X, dim, (const bf16 *)nullptr, wu, a->y, bs, ff, dim, act, S);
+        if (wg) pa_launch_cut(pdl, S, narrow ? pa_k_dense_up<ROUND, 2, 32> : pa_k_dense_up<ROUND, 2, PA_TM>, grid, st, X, dim, wg, wu, a->y, bs, ff, dim, act, S);
+        else pa_launch_cut(pdl, S, narrow ? pa_k_dense_up<ROUND, 1, 32> : pa_k_dense_up<ROUND, 1, PA_TM>, grid, st, X, dim, (const bf16 *)nullptr, wu, a->y, bs, ff, dim, act, S);
         PA_LAUNCH();
         return 0;
     };
@@ -1366,13 +1373,13 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         }
         if (tc) {
             const int nkb = (dim + PT_KB - 1) / PT_KB, n_ct = (bs + PT_N - 1) / PT_N;
-            pa_k_tc_prep_x<<<dim3((unsigned)nkb, (unsigned)n_ct), 256, 0, st>>>(a->tcx, X, dim, bs, dim, nkb, nullptr, nullptr, nullptr, nullptr, nullptr);
+            pa_launch_dep(pdl, pa_k_tc_prep_x, dim3((unsigned)nkb, (unsigned)n_ct), dim3(256), 0, st, a->tcx, X, dim, bs, dim, nkb, nullptr, nullptr, nullptr, nullptr, nullptr);
             PA_LAUNCH();
             PtArgs g{};
             g.a0 = tg; g.a1 = tu; g.b = a->tcx; g.nkb = nkb; g.n_rt = (ff + PT_M - 1) / PT_M; g.n_ct = n_ct; g.M = bs; g.N = ff; g.mode = PT_MODE_EXPERT_UP;
             g.C = a->y; g.ldc = ff; g.act = act; g.err = io.err_dev;
             const int ctas = cut_tiles(g);
-            pa_k_tc_gemm<2><<<ctas, PT_THREADS, PT_SMEM, st>>>(g);
+            pa_launch_dep(pdl, pa_k_tc_gemm<2>, dim3(ctas), dim3(PT_THREADS), PT_SMEM, st, g);
         } else {
             if ((rc_up = dense_up(X, wg, wu, ff, act))) return rc_up;
         }
@@ -1414,7 +1421,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         if (latent) {
             const int rq = l.q_rank, rk = l.kv_rank, dr = l.rot_dim, dn = l.qk_dim, lqw = H * (dn + dr);
             const PaRope rope{w.rope_freq, l.rope_dims, w.rope_mscale, l.rope_interleaved};
-            pa_k_latent_post<<<bs, 256, 0, st>>>(a->qkv, w.pw, rq, rk, dr, w.dq_norm, w.dkv_norm, d.norm_eps, rope, a->cq, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev);
+            pa_launch_dep(pdl, pa_k_latent_post, dim3(bs), dim3(256), 0, st, a->qkv, w.pw, rq, rk, dr, w.dq_norm, w.dkv_norm, d.norm_eps, rope, a->cq, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev);
             PA_LAUNCH();
             if (single) {
                 PaMv mv{};
@@ -1428,17 +1435,16 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                 if ((rc = linear_heads(a->lq, lqw, dn + dr, dn, w.wukt, rk, a->qa, w.qd, rk + dr, H))) return rc; // W_uk folded into the query
             }
             if (dr > 0) {
-                pa_k_rope_q<<<bs, 256, 0, st>>>(a->lq, lqw, a->qa, H, dn, dr, rk, rope, io.pos_dev);
+                pa_launch_dep(pdl, pa_k_rope_q, dim3(bs), dim3(256), 0, st, a->lq, lqw, a->qa, H, dn, dr, rk, rope, io.pos_dev);
                 PA_LAUNCH();
             }
             at.dq = rk + dr; at.dv = rk; q = a->qa; ldq = w.qd;
         } else {
             at.dq = l.qk_dim; at.dv = l.v_dim;
             if (l.qk_norm || l.v_mix)
-                pa_k_qkv_post<<<bs, 256, 0, st>>>(a->qkv, w.pw, H, G, l.qk_dim, l.v_dim, l.qk_norm, d.norm_eps, l.v_mix, w.vmix, a->vsrc, a->vsrc_w, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev,
-                                                   nullptr, nullptr, 0.f, 1.f);
+                pa_launch_dep(pdl, pa_k_qkv_post, dim3(bs), dim3(256), 0, st, a->qkv, w.pw, H, G, l.qk_dim, l.v_dim, l.qk_norm, d.norm_eps, l.v_mix, w.vmix, a->vsrc, a->vsrc_w, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, nullptr, nullptr, 0.f, 1.f, PaRope{}, PaRope{});
             else
-                pa_k_kv_store<<<dim3(cdiv(w.kd + w.vd, 256), bs), 256, 0, st>>>(a->qkv, w.pw, w.qd, w.kd, w.vd, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.qd + w.kd);
+                pa_launch_dep(pdl, pa_k_kv_store, dim3(cdiv(w.kd + w.vd, 256), bs), dim3(256), 0, st, a->qkv, w.pw, w.qd, w.kd, w.vd, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.qd + w.kd);
             PA_LAUNCH();
         }
         if (single) {
@@ -1554,7 +1560,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             if (tc) {
                 if ((rc = tc_dense(a->x, dim, bs, dim, w.t_tg, td, nullptr, a->tg, td, &gelu, 0, 0, &mul))) return rc;
             } else {
-                pa_launch_linear<ROUND>(a->n_sm, td, bs, 1, st, a->x, dim, w.wtg, nullptr, a->tg, td, bs, td, dim, 0, 0, 0, 0, gelu, mul);
+                pa_launch_linear<ROUND>(pdl, a->n_sm, td, bs, 1, st, a->x, dim, w.wtg, nullptr, a->tg, td, bs, td, dim, 0, 0, 0, 0, gelu, mul);
                 PA_LAUNCH();
             }
             if ((rc = linear(a->tg, td, td, w.wtp, w.t_tp, dim, a->ty, dim))) return rc;
@@ -1600,19 +1606,19 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                 PtArgs g{};
                 g.seg = w.seg;
                 g.seg.set_bytes = (int64_t)n_ct * nkb * PT_BLOCK;
-                pa_k_tc_prep_shift<<<dim3((unsigned)nkb, (unsigned)n_ct, 4), 256, 0, st>>>(a->tcx, a->h, bs, dim, nkb, w.mu, ring, io.pos_dev, g.seg.set_bytes);
+                pa_launch_dep(pdl, pa_k_tc_prep_shift, dim3((unsigned)nkb, (unsigned)n_ct, 4), dim3(256), 0, st, a->tcx, a->h, bs, dim, nkb, w.mu, ring, io.pos_dev, g.seg.set_bytes);
                 PA_LAUNCH();
                 g.a0 = w.t_qkv; g.b = a->tcx; g.nkb = nkb; g.n_rt = w.seg.rt[w.seg.n]; g.n_ct = n_ct; g.M = bs; g.N = w.pw; g.mode = PT_MODE_DENSE; g.C = a->qkv; g.ldc = w.pw; g.err = io.err_dev;
                 g.act = tanh_act; g.act1 = 1; g.act_from = w1_off;
                 const int ctas = cut_tiles(g);
-                pa_k_tc_gemm<1><<<ctas, PT_THREADS, PT_SMEM, st>>>(g);
+                pa_launch_dep(pdl, pa_k_tc_gemm<1>, dim3(ctas), dim3(PT_THREADS), PT_SMEM, st, g);
                 PA_LAUNCH();
             } else {
                 pa_k_token_shift<<<dim3(cdiv(dim, 256), bs, 5), 256, 0, st>>>(a->h, dim, w.mu, ring, io.pos_dev, a->mixb, (int64_t)B * dim);
                 PA_LAUNCH();
                 for (int k = 0; k < w.seg.n; k++) {
                     const int r0 = w.seg.row[k], n = w.seg.row[k + 1] - r0;
-                    pa_launch_linear<ROUND>(a->n_sm, n, bs, 1, st, k ? a->mixb + (int64_t)(k - 1) * B * dim : a->h, dim, w.wqkv + (int64_t)r0 * dim, nullptr, a->qkv + r0, w.pw, bs, n, dim, 0,
+                    pa_launch_linear<ROUND>(pdl, a->n_sm, n, bs, 1, st, k ? a->mixb + (int64_t)(k - 1) * B * dim : a->h, dim, w.wqkv + (int64_t)r0 * dim, nullptr, a->qkv + r0, w.pw, bs, n, dim, 0,
                                                                                             0, r0 == w1_off ? 0 : 1 << 30, 0, tanh_act);
                     PA_LAUNCH();
                 }
@@ -1645,12 +1651,11 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                 PA_LAUNCH();
             } else if (heads_post) {
                 if (!single) { // (a single token's scores kernel does this)
-                    pa_k_qkv_post<<<bs, 256, 0, st>>>(q, w.pw, H, l.n_kv_heads, l.qk_dim, l.v_dim, l.qk_norm, d.norm_eps, 0, nullptr, nullptr, 0, io.kc[li],
-                                                                                                      io.vct[li], d.n_ctx, io.pos_dev, w.q_norm, w.k_norm, 0.f, 1.f, at_rope, at_vrope);
+                    pa_launch_dep(pdl, pa_k_qkv_post, dim3(bs), dim3(256), 0, st, q, w.pw, H, l.n_kv_heads, l.qk_dim, l.v_dim, l.qk_norm, d.norm_eps, 0, nullptr, nullptr, 0, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.q_norm, w.k_norm, 0.f, 1.f, at_rope, at_vrope);
                     PA_LAUNCH();
                 }
             } else if (!direct) {
-                pa_k_kv_store<<<dim3(cdiv(w.kd + w.vd, 256), bs), 256, 0, st>>>(q, w.pw, w.qd, w.kd, w.vd, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.v_off);
+                pa_launch_dep(pdl, pa_k_kv_store, dim3(cdiv(w.kd + w.vd, 256), bs), dim3(256), 0, st, q, w.pw, w.qd, w.kd, w.vd, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.v_off);
                 PA_LAUNCH();
             }
             if (l.pool > 0 && !single) { // the means of the blocks that this batch completes (at most bs / pool + 1 of them); a single token's scores kernel forms its own
@@ -1773,7 +1778,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             if ((rc = seam(raw ? nullptr : a->h, w_in))) return rc;
             const float *X = raw ? a->x : a->h;
             if (sff > 0 && (rc = dense_batch(X, w.wsg, w.wsu, w.wsd, w.t_sg, w.t_su, w.t_sd, sff, act, a->sh))) return rc;
-            pa_k_router<<<bs, 256, 0, st>>>(X, w.router, dim, rt, a->sel_e, a->sel_w, a->sgate, nullptr);
+            pa_launch_dep(pdl, pa_k_router, dim3(bs), dim3(256), 0, st, X, w.router, dim, rt, a->sel_e, a->sel_w, a->sgate, nullptr);
             PA_LAUNCH();
             if ((rc = routed_batch(X, w))) return rc;
             pa_k_moe_sum<<<dim3(cdiv(dim, 256), bs), 256, 0, st>>>(a->ffo, a->slot, top, sff > 0 ? a->sh : nullptr, rt.shared_gate ? a->sgate : nullptr, dim, a->sel_e, a->sel_w,
@@ -1835,7 +1840,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             if (tc) {
                 if ((rc = tc_dense(a->h, dim, bs, dim, w.t_qkv, n1, w.bqkv, a->qkv, w.ldp, w.upn > 0 ? &act : nullptr, w.pw, gap))) return rc;
             } else {
-                pa_launch_linear<ROUND>(a->n_sm, n1, bs, 1, st, a->h, dim, w.wqkv, w.bqkv, a->qkv, w.ldp, bs, n1, dim, 0, 0, w.pw, gap, act);
+                pa_launch_linear<ROUND>(pdl, a->n_sm, n1, bs, 1, st, a->h, dim, w.wqkv, w.bqkv, a->qkv, w.ldp, bs, n1, dim, 0, 0, w.pw, gap, act);
                 PA_LAUNCH();
             }
         }
@@ -1850,7 +1855,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             } else {
                 pa_k_short_conv<<<dim3(cdiv(g.W, 256), bs), 256, 0, st>>>(g.x, w.ldp, w.conv_w, w.conv_b, g.W, g.taps, g.ring, 0, a->cv, g.W, io.pos_dev, 1);
                 PA_LAUNCH();
-                pa_launch_linear<false, !ROUND>(a->n_sm, 2 * g.bsz, bs, (int)l.rec_blocks, st, a->cv, g.W, w.wri, nullptr, a->gts, 2 * g.W, bs, 2 * g.bsz, g.bsz, g.bsz, 2 * g.bsz);
+                pa_launch_linear<false, !ROUND>(pdl, a->n_sm, 2 * g.bsz, bs, (int)l.rec_blocks, st, a->cv, g.W, w.wri, nullptr, a->gts, 2 * g.W, bs, 2 * g.bsz, g.bsz, g.bsz, 2 * g.bsz);
                 PA_LAUNCH();
                 pa_k_rglru_scan<<<cdiv(g.W, 32), PA_GG_THREADS, 0, st>>>(g);
                 PA_LAUNCH();
@@ -1875,11 +1880,11 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                                   (const bf16 *)w.wukt, a->qa, lg, (const float *)w.dkv_norm, d.norm_eps, rope, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev);
                     PA_LAUNCH();
                 } else {
-                    pa_k_latent_post<<<bs, 256, 0, st>>>(a->qkv + H * lq, w.ldp, 0, rk, dr, nullptr, w.dkv_norm, d.norm_eps, rope, nullptr, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev);
+                    pa_launch_dep(pdl, pa_k_latent_post, dim3(bs), dim3(256), 0, st, a->qkv + H * lq, w.ldp, 0, rk, dr, nullptr, w.dkv_norm, d.norm_eps, rope, nullptr, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev);
                     PA_LAUNCH();
                     if ((rc = linear_heads(a->qkv, w.ldp, lq, dn, w.wukt, rk, a->qa, w.qd, rk + dr, H))) return rc; // W_uk folded into the query
                     if (dr > 0) {
-                        pa_k_rope_q<<<bs, 256, 0, st>>>(a->qkv, w.ldp, a->qa, H, dn, dr, rk, rope, io.pos_dev);
+                        pa_launch_dep(pdl, pa_k_rope_q, dim3(bs), dim3(256), 0, st, a->qkv, w.ldp, a->qa, H, dn, dr, rk, rope, io.pos_dev);
                         PA_LAUNCH();
                     }
                 }
@@ -1888,8 +1893,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                     at.head_norm = 1; at.qn = w.q_norm; at.kn = w.k_norm; at.eps = d.norm_eps; at.qt_coef = l.q_temp_coef; at.qt_every = l.q_temp_every; at.k_raw = a->qkv + w.qd; at.kc_out = io.kc[li];
                 }
             } else {
-                pa_k_qkv_post<<<bs, 256, 0, st>>>(a->qkv, w.ldp, H, l.n_kv_heads, l.qk_dim, l.v_dim, l.qk_norm, d.norm_eps, 0, nullptr, nullptr, 0, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.q_norm,
-                                                  w.k_norm, l.q_temp_coef, l.q_temp_every);
+                pa_launch_dep(pdl, pa_k_qkv_post, dim3(bs), dim3(256), 0, st, a->qkv, w.ldp, H, l.n_kv_heads, l.qk_dim, l.v_dim, l.qk_norm, d.norm_eps, 0, nullptr, nullptr, 0, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.q_norm, w.k_norm, l.q_temp_coef, l.q_temp_every, PaRope{}, PaRope{});
                 PA_LAUNCH();
             }
             rc = single ? attend_single(at, q, li, ho) : attend(at, q, ldq, w.kd, li, ho, ldo);
@@ -1919,7 +1923,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             pa_k_dec_expert_down<ROUND><<<cdiv(dim, PA_DV_ROWS / ksd), PA_DV_THREADS, 0, st>>>(a->y, a->sel_e, a->sel_w, l.top_k, w.wdown, nullptr, nullptr, dim, l.expert_ff, 0, ksd, a->ffo, a->ao, nullptr);
             PA_LAUNCH();
         } else {
-            pa_k_router<<<bs, 256, 0, st>>>(a->h, w.router, dim, pa_route_of(l), a->sel_e, a->sel_w, a->sgate, w.router_b);
+            pa_launch_dep(pdl, pa_k_router, dim3(bs), dim3(256), 0, st, a->h, w.router, dim, pa_route_of(l), a->sel_e, a->sel_w, a->sgate, w.router_b);
             PA_LAUNCH();
             if ((rc = routed_batch(a->h, w))) return rc;
             pa_k_moe_sum<<<dim3(cdiv(dim, 256), bs), 256, 0, st>>>(a->ffo, a->slot, l.top_k, a->ao, nullptr, dim);
@@ -1929,8 +1933,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         return 0;
     };
 
-    pa_k_embed<<<bs, 128, 0, st>>>(a->x, a->embed, io.tokens_dev, dim, d.embed_scale, a->has_pass_in ? a->xcat + dim : a->keep_embed ? a->xe : nullptr, a->has_pass_in ? 2 * dim : dim,
-                                   PaAngles{a->ang_freq, a->ang_ms, (int)a->ang_freq_h.size(), a->ang, io.pos_dev});
+    pa_launch_dep(pdl, pa_k_embed, dim3(bs), dim3(128), 0, st, a->x, a->embed, io.tokens_dev, dim, d.embed_scale, a->has_pass_in ? a->xcat + dim : a->keep_embed ? a->xe : nullptr, a->has_pass_in ? 2 * dim : dim, PaAngles{a->ang_freq, a->ang_ms, (int)a->ang_freq_h.size(), a->ang, io.pos_dev});
     PA_LAUNCH();
     for (int li = 0; li < d.n_layers; li++) {
         const PsArchLayer &w = a->L[(size_t)li];
@@ -1952,7 +1955,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         const int H = l.n_heads, G = l.n_kv_heads, dq = l.qk_dim, dv = l.v_dim, nqkv = w.qd + w.kd + w.vd;
         const bool routed = l.mlp_kind == PS_MLP_ROUTED;
         if (!single) { // (the single-token kernels norm in their prologues)
-            pa_k_norm<<<bs, 256, 0, st>>>(a->h, a->x, w.norm, dim, d.norm_eps);
+            pa_launch_dep(pdl, pa_k_norm, dim3(bs), dim3(256), 0, st, a->h, a->x, w.norm, dim, d.norm_eps);
             PA_LAUNCH();
         }
         // ---- token mixer: projections -> cache -> scores -> (mix, soft-max) -> P.V -> output projection
@@ -1978,11 +1981,11 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             int rc = tc_dense(a->h, dim, bs, dim, w.t_qkv, nqkv, w.bqkv, a->qkv, nqkv);
             if (rc) return rc;
         } else {
-            pa_launch_linear<ROUND>(a->n_sm, nqkv, bs, 1, st, a->h, dim, w.wqkv, w.bqkv, a->qkv, nqkv, bs, nqkv, dim);
+            pa_launch_linear<ROUND>(pdl, a->n_sm, nqkv, bs, 1, st, a->h, dim, w.wqkv, w.bqkv, a->qkv, nqkv, bs, nqkv, dim);
         }
         PA_LAUNCH();
         if (!single) {
-            pa_k_kv_store<<<dim3(cdiv(w.kd + w.vd, 256), bs), 256, 0, st>>>(a->qkv, nqkv, w.qd, w.kd, w.vd, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.qd + w.kd);
+            pa_launch_dep(pdl, pa_k_kv_store, dim3(cdiv(w.kd + w.vd, 256), bs), dim3(256), 0, st, a->qkv, nqkv, w.qd, w.kd, w.vd, io.kc[li], io.vct[li], d.n_ctx, io.pos_dev, w.qd + w.kd);
             PA_LAUNCH();
         }
         PaAttn at{};
@@ -1995,11 +1998,11 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             pa_launch_dep(pdl, pa_k_dec_pv, dim3(cdiv(dv, PA_DP_DIMS), G, pa_dec_pv_split(H, G)), dim3(256), pa_dec_pv_smem(H, G), st, at, (const float *)a->S, (const float *)io.vct[li], io.pos_dev, a->att, pa_dec_pv_chunk(H, G), io.err_dev);
             PA_LAUNCH();
         } else {
-            pa_k_scores<<<dim3(cdiv(n_kv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st>>>(at, a->qkv, nqkv, io.kc[li], w.kd, a->S, io.pos_dev, bs, 0, (int)cdiv(n_kv, PA_TN));
+            pa_launch_dep(pdl, pa_k_scores, dim3(cdiv(n_kv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st, at, a->qkv, nqkv, io.kc[li], w.kd, a->S, io.pos_dev, bs, 0, (int)cdiv(n_kv, PA_TN));
             PA_LAUNCH();
-            pa_k_mix_softmax<<<bs, 256, 4 * (size_t)H * H, st>>>(at, a->S, io.pos_dev, bs);
+            pa_launch_dep(pdl, pa_k_mix_softmax, dim3(bs), dim3(256), 4 * (size_t)H * H, st, at, a->S, io.pos_dev, bs);
             PA_LAUNCH();
-            pa_k_pv<!ROUND><<<dim3(cdiv(dv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st>>>(at, a->S, io.vct[li], a->att, w.od, io.pos_dev, bs);
+            pa_launch_dep(false, pa_k_pv<!ROUND>, dim3(cdiv(dv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st, at, a->S, io.vct[li], a->att, w.od, io.pos_dev, bs);
             PA_LAUNCH();
         }
         if (single) {
@@ -2012,7 +2015,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             int rc = tc_dense(a->att, w.od, bs, w.od, w.t_o, dim, w.bo, a->ao, dim);
             if (rc) return rc;
         } else {
-            pa_launch_linear<ROUND>(a->n_sm, dim, bs, 1, st, a->att, w.od, w.wo, w.bo, a->ao, dim, bs, dim, w.od);
+            pa_launch_linear<ROUND>(pdl, a->n_sm, dim, bs, 1, st, a->att, w.od, w.wo, w.bo, a->ao, dim, bs, dim, w.od);
         }
         PA_LAUNCH();
         // ---- routed feed-forward on the same normed input
@@ -2022,7 +2025,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             const int ff = l.expert_ff;
             int rc = 0;
             if (!single) {
-                pa_k_router<<<bs, 256, 0, st>>>(a->h, w.router, dim, pa_route_of(l), a->sel_e, a->sel_w, a->sgate, nullptr);
+                pa_launch_dep(pdl, pa_k_router, dim3(bs), dim3(256), 0, st, a->h, w.router, dim, pa_route_of(l), a->sel_e, a->sel_w, a->sgate, nullptr);
                 PA_LAUNCH();
             }
             if (single) {
@@ -2035,7 +2038,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             }
         }
         if (!single) {
-            pa_k_combine<<<dim3(cdiv(dim, 256), bs), 256, 0, st>>>(a->x, a->ao, a->slot, top, dim);
+            pa_launch_dep(pdl, pa_k_combine, dim3(cdiv(dim, 256), bs), dim3(256), 0, st, a->x, a->ao, a->slot, top, dim);
             PA_LAUNCH();
         }
         if (a->taps_on) {
@@ -2049,7 +2052,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                 int rc = seam(a->h, a->final_norm);
                 if (rc) return rc;
             } else {
-                pa_k_norm<<<bs, 256, 0, st>>>(a->h, a->x, a->final_norm, dim, d.norm_eps);
+                pa_launch_dep(pdl, pa_k_norm, dim3(bs), dim3(256), 0, st, a->h, a->x, a->final_norm, dim, d.norm_eps);
                 PA_LAUNCH();
             }
         }
@@ -2063,7 +2066,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
             int rc = tc_dense(a->h, dim, bs, dim, a->t_head, d.vocab_size, nullptr, a->logits, d.vocab_size);
             if (rc) return rc;
         } else {
-            pa_launch_linear<ROUND>(a->n_sm, d.vocab_size, bs, 1, st, a->h, dim, a->head, nullptr, a->logits, d.vocab_size, bs, d.vocab_size, dim);
+            pa_launch_linear<ROUND>(pdl, a->n_sm, d.vocab_size, bs, 1, st, a->h, dim, a->head, nullptr, a->logits, d.vocab_size, bs, d.vocab_size, dim);
         }
         PA_LAUNCH();
     }

@@ -334,6 +334,7 @@ __device__ __forceinline__ void pa_tile_cut(float *sm, const float *arow, const 
 // keep (null or [tokens] rows of stride ld_keep) receives the same rows once more: the embedding output that later passes of a looped model add back
 __global__ void __launch_bounds__(128) pa_k_embed(float *__restrict__ x, const bf16 *__restrict__ table, const int32_t *__restrict__ tokens, int dim, float scale,
                                                   float *__restrict__ keep, int ld_keep, PaAngles ang) {
+    ps_grid_dep();
     const int t = blockIdx.x;
     for (int i = threadIdx.x; i < ang.n; i += blockDim.x) {
         const PaRope r{ang.freq, 0, ang.mscale[i], 0, nullptr, 0};
@@ -365,6 +366,7 @@ __global__ void __launch_bounds__(128) pa_k_embed(float *__restrict__ x, const b
 
 // h = x / sqrt(mean(x^2) + eps) * w   (w already holds 1 + weight for unit-offset norms)
 __global__ void __launch_bounds__(256) pa_k_norm(float *__restrict__ h, const float *__restrict__ x, const float *__restrict__ w, int dim, float eps) {
+    ps_grid_dep();
     __shared__ float red[8];
     __shared__ float inv_s;
     const float *xr = x + (int64_t)blockIdx.x * dim;
@@ -388,6 +390,7 @@ __global__ void __launch_bounds__(256) pa_k_norm(float *__restrict__ h, const fl
 // (v_off: where the value rows start in a projected row - behind the keys, or AT the keys when the values are the keys)
 __global__ void __launch_bounds__(256) pa_k_kv_store(const float *__restrict__ qkv, int ld, int qd, int kd, int vd, float *__restrict__ kc, float *__restrict__ vct, int n_ctx,
                                                      const int32_t *__restrict__ pos, int v_off) {
+    ps_grid_dep();
     const int t = blockIdx.y, c = blockIdx.x * 256 + threadIdx.x;
     const int p = pos[t];
     const float *row = qkv + (int64_t)t * ld;
@@ -420,6 +423,7 @@ __global__ void __launch_bounds__(256) pa_k_pool_blocks(float *__restrict__ kc, 
 
 // x += mixer + sum of the feed-forward slots (fixed order)
 __global__ void __launch_bounds__(256) pa_k_combine(float *__restrict__ x, const float *__restrict__ ao, const float *__restrict__ slot, int top, int dim) {
+    ps_grid_dep();
     const int t = blockIdx.y, c = blockIdx.x * 256 + threadIdx.x;
     if (c >= dim) return;
     float y = ao[(int64_t)t * dim + c];
@@ -464,6 +468,7 @@ template <int NT = 256> __device__ __forceinline__ float pa_block_stats(const fl
 __global__ void __launch_bounds__(256) pa_k_seam_norm(float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ w_out, float *__restrict__ h,
                                                       const float *__restrict__ w_in, int dim, int groups, float eps, int center, const float *__restrict__ add_tok,
                                                       const float *__restrict__ add_vec, float y_scale, int ldh) {
+    ps_grid_dep();
     __shared__ float red[8];
     const int64_t base = (int64_t)blockIdx.x * dim;
     const int gs = dim / groups;
@@ -508,7 +513,8 @@ __device__ __forceinline__ float pa_q_temp(float coef, float every, int p) {
 __global__ void __launch_bounds__(256) pa_k_qkv_post(float *__restrict__ qkv, int ld, int H, int G, int dq, int dv, int qk_norm, float eps, int v_mix,
                                                      const float *__restrict__ lambda, float *__restrict__ v_src, int ld_src, float *__restrict__ kc,
                                                      float *__restrict__ vct, int n_ctx, const int32_t *__restrict__ pos, const float *__restrict__ qn, const float *__restrict__ kn,
-                                                     float qt_coef, float qt_every, PaRope rope = PaRope{}, PaRope vrope = PaRope{}) {
+                                                     float qt_coef, float qt_every, PaRope rope, PaRope vrope) {
+    ps_grid_dep();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = pos[t];
     float *row = qkv + (int64_t)t * ld;
     const float qt = pa_q_temp(qt_coef, qt_every, p);
@@ -567,6 +573,7 @@ __device__ __forceinline__ void pa_rope_store(const PaRope &r, const float *src,
 __global__ void __launch_bounds__(256) pa_k_latent_post(const float *__restrict__ t_in, int ld, int rq, int rk, int dr, const float *__restrict__ wq, const float *__restrict__ wk,
                                                         float eps, PaRope rope, float *__restrict__ cq, float *__restrict__ kc, float *__restrict__ vct, int n_ctx,
                                                         const int32_t *__restrict__ pos) {
+    ps_grid_dep();
     __shared__ float red[8];
     const int t = blockIdx.x, p = pos[t];
     const float *row = t_in + (int64_t)t * ld;
@@ -590,6 +597,7 @@ __global__ void __launch_bounds__(256) pa_k_latent_post(const float *__restrict_
 
 // the rotated part of every query head: q[t * ldq + h * (dn + dr) + dn ..] -> qa[t][h * (rk + dr) + rk ..], rotated by the token's position
 __global__ void __launch_bounds__(256) pa_k_rope_q(const float *__restrict__ q, int ldq, float *__restrict__ qa, int H, int dn, int dr, int rk, PaRope rope, const int32_t *__restrict__ pos) {
+    ps_grid_dep();
     const int t = blockIdx.x, p = pos[t];
     for (int e = threadIdx.x; e < H * dr; e += 256) {
         const int hh = e / dr, c = e % dr;
@@ -604,6 +612,7 @@ __global__ void __launch_bounds__(256) pa_k_rope_q(const float *__restrict__ q, 
 template <bool ROUND, int TM = PA_TM>
 __global__ void __launch_bounds__(256, 4) pa_k_linear(const float *__restrict__ A, int lda, const bf16 *__restrict__ W, const float *__restrict__ bias, float *__restrict__ C, int ldc,
                                                    int M, int N, int K, int S, int a_gs, int c_gs, int act_from, int gap, PaAct act, PaRowMul mul) {
+    ps_grid_dep();
     __shared__ __align__(16) float sm[PaTile<1, TM>::N];
     const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM), z = blockIdx.z / S;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * PA_TN;
@@ -765,6 +774,7 @@ __device__ __forceinline__ void pa_route_topk_warp(const float *__restrict__ z, 
 // last row gives sgate[token] = sigmoid(w_sg . h)
 __global__ void __launch_bounds__(256) pa_k_router(const float *__restrict__ h, const bf16 *__restrict__ Wr, int dim, PaRoute r, int *__restrict__ sel_e,
                                                    float *__restrict__ sel_w, float *__restrict__ sgate, const float *__restrict__ bias) {
+    ps_grid_dep();
     __shared__ float zs[PA_MAX_EXPERTS + 1], sc[PA_MAX_EXPERTS], sw[PA_MAX_EXPERTS];
     __shared__ int se[PA_MAX_EXPERTS];
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -798,6 +808,7 @@ __global__ void __launch_bounds__(256) pa_k_router(const float *__restrict__ h, 
 __global__ void __launch_bounds__(256) pa_k_dispatch(const int *__restrict__ sel_e, const float *__restrict__ sel_w, int n, int top, int E, int tile_rows, int *__restrict__ row_token,
                                                      int *__restrict__ row_slot, float *__restrict__ row_w, int *__restrict__ tile_e, int *__restrict__ tile_row0,
                                                      int *__restrict__ tile_end, int *__restrict__ n_tiles) {
+    ps_grid_dep();
     __shared__ int cnt[PA_MAX_EXPERTS], off[PA_MAX_EXPERTS], fill[PA_MAX_EXPERTS];
     for (int e = threadIdx.x; e < E; e += 256) { cnt[e] = 0; fill[e] = 0; }
     __syncthreads();
@@ -830,6 +841,7 @@ __global__ void __launch_bounds__(256, NB == 2 ? 2 : 4) pa_k_expert_up(const flo
                                                       const int *__restrict__ tile_e, const int *__restrict__ tile_row0, const int *__restrict__ tile_end,
                                                       const int *__restrict__ n_tiles, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int ff,
                                                       int dim, int on_input, PaAct act) {
+    ps_grid_dep();
     __shared__ __align__(16) float sm[PaTile<NB, PA_TM>::N];
     if ((int)blockIdx.y >= *n_tiles) return;
     const int lr = threadIdx.x >> 2;
@@ -859,6 +871,7 @@ __global__ void __launch_bounds__(256, 4) pa_k_expert_down(const float *__restri
                                                         const float *__restrict__ row_w, const int *__restrict__ tile_e, const int *__restrict__ tile_row0,
                                                         const int *__restrict__ tile_end, const int *__restrict__ n_tiles, const bf16 *__restrict__ Wd, float *__restrict__ slot,
                                                         int top, int dim, int ff, int on_input) {
+    ps_grid_dep();
     __shared__ __align__(16) float sm[PaTile<1, PA_TM>::N];
     if ((int)blockIdx.y >= *n_tiles) return;
     const int lr = threadIdx.x >> 2;
@@ -885,6 +898,7 @@ __global__ void __launch_bounds__(256, 4) pa_k_expert_down(const float *__restri
 template <bool ROUND, int NB, int TM = PA_TM>
 __global__ void __launch_bounds__(256, NB == 2 ? 2 : 4) pa_k_dense_up(const float *__restrict__ h, int ldh, const bf16 *__restrict__ Wg, const bf16 *__restrict__ Wu, float *__restrict__ y, int M, int ff,
                                                      int dim, PaAct act, int S) {
+    ps_grid_dep();
     __shared__ __align__(16) float sm[PaTile<NB, TM>::N];
     const int tid = threadIdx.x, lr = tid >> 2, la = tid / (256 / TM);
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * PA_TN;
@@ -929,6 +943,7 @@ __device__ __forceinline__ float pa_sink_logit(const PaAttn &at, int h) { return
 // `tok_tiles` on are tiles of pooled blocks: S[h][i][pool_off + b] = score of query i and the mean key of block b.
 __global__ void __launch_bounds__(256, 3) pa_k_scores(PaAttn at, const float *__restrict__ qkv, int ldq, const float *__restrict__ kc, int kd, float *__restrict__ S,
                                                    const int32_t *__restrict__ pos, int bs, int key_tile0, int tok_tiles) {
+    ps_grid_dep();
     __shared__ __align__(16) float sm[PaTile<1, PA_TM>::N];
     const int lr = threadIdx.x >> 2;
     const int h = blockIdx.z, g = h / (at.H / at.G), m0 = blockIdx.y * PA_TM;
@@ -992,6 +1007,7 @@ __device__ __forceinline__ void pa_mix_rows(const PaAttn &at, float *S, int i, i
 }
 
 __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__restrict__ S, const int32_t *__restrict__ pos, int bs) {
+    ps_grid_dep();
     extern __shared__ float Ts[];
     const int i = blockIdx.x, H = at.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int n = pos[i] + 1, n_end = pos[0] + bs, lo = pa_first_key(at, pos[i]);
@@ -1045,6 +1061,7 @@ __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__rest
 template <bool GROUPS>
 __global__ void __launch_bounds__(256, GROUPS ? 2 : 3) pa_k_pv(PaAttn at, const float *__restrict__ S, const float *__restrict__ vct, float *__restrict__ att, int od,
                                                const int32_t *__restrict__ pos, int bs) {
+    ps_grid_dep();
     __shared__ __align__(16) float sm[PaTile<1, PA_TM, GROUPS>::N];
     const int lr = threadIdx.x >> 2;
     const int h = blockIdx.z, g = h / (at.H / at.G), m0 = blockIdx.y * PA_TM, n0 = blockIdx.x * PA_TN;

@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256) pa_k_tc_tile_w(uint8_t *__restrict__ dst,
 __global__ void __launch_bounds__(256) pa_k_tc_prep_x(uint8_t *__restrict__ dst, const float *__restrict__ x, int ldx, int M, int K, int nkb, const int *__restrict__ n_tiles,
                                                       const int *__restrict__ tile_row0, const int *__restrict__ tile_end, const int *__restrict__ row_token,
                                                       const float *__restrict__ row_w) {
+    ps_grid_dep();
     const int kb = blockIdx.x, t = blockIdx.y;
     if (n_tiles && t >= *n_tiles) return;
     const int r0 = tile_row0 ? tile_row0[t] : t * 128, rend = tile_end ? tile_end[t] : M;
@@ -68,6 +69,7 @@ __global__ void __launch_bounds__(256) pa_k_tc_prep_x(uint8_t *__restrict__ dst,
 // token: row (pos - 1) & 1 of `ring`, zeros at position 0).  Grid (k blocks, column tiles, 4): a CTA takes 32 rows, a thread eight entries of all sets; set s starts s * set_bytes further on.
 __global__ void __launch_bounds__(256) pa_k_tc_prep_shift(uint8_t *__restrict__ dst, const float *__restrict__ x, int M, int K, int nkb, const float *__restrict__ mu,
                                                           const float *__restrict__ ring, const int32_t *__restrict__ pos, int64_t set_bytes) {
+    ps_grid_dep();
     const int kb = blockIdx.x, t = blockIdx.y, p0 = pos[0];
     const int kc = threadIdx.x & 7, row = blockIdx.z * 32 + (threadIdx.x >> 3), r = t * 128 + row, k0 = kb * PT_KB + kc * 8;
     uint8_t *out = dst + ((int64_t)t * nkb + kb) * PT_BLOCK + kc * 2048 + row * 16;
@@ -133,10 +135,8 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
     __shared__ uint32_t tmem_base_smem;
     uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)pt_smem_raw + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
-    const int nkb = a.nkb, n_ct = a.n_ct_dev ? min(*a.n_ct_dev, a.n_ct) : a.n_ct;
-    const int n_units = n_ct * a.n_rt;
+    const int nkb = a.nkb;
     const int n_sub = max(a.n_sub, 1), tn = PT_N / n_sub; // tokens of a unit
-    const int my_units = (n_units > (int)blockIdx.x) ? (n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; s++) { ps_mbar_init(&bar_full[s], 1); ps_mbar_init(&bar_empty[s], 1); }
@@ -153,6 +153,24 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
     __syncthreads();
     ps_tc_fence_after();
     const uint32_t tmem_base = tmem_base_smem;
+    // a dense product's first weights do not depend on the kernel before: they are asked for while it still runs
+    int ahead = 0;
+    if (warp == 4 && !a.n_ct_dev && !a.tile_e && (int)blockIdx.x < a.n_ct * a.n_rt) {
+        ahead = min(STAGES, nkb);
+        if (ps_elect_one()) {
+            const int64_t b0 = (int64_t)((int)blockIdx.x % a.n_rt) * nkb * PT_BLOCK;
+            for (int kb = 0; kb < ahead; kb++) {
+                ps_mbar_expect_tx(&bar_full[kb], NA * PT_BLOCK + PT_BLOCK / n_sub);
+                ps_bulk_g2s(smem + (size_t)kb * STAGE_BYTES, a.a0 + b0 + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[kb]);
+                if (NA == 2) ps_bulk_g2s(smem + (size_t)kb * STAGE_BYTES + PT_BLOCK, a.a1 + b0 + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[kb]);
+            }
+        }
+        __syncwarp();
+    }
+    ps_grid_dep();
+    const int n_ct = a.n_ct_dev ? min(*a.n_ct_dev, a.n_ct) : a.n_ct;
+    const int n_units = n_ct * a.n_rt;
+    const int my_units = (n_units > (int)blockIdx.x) ? (n_units - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
 
     if (warp == 4) {
         // ===== producer: one bulk copy per operand block.  Producer and issuer stay converged warps and act through one elected thread: under
@@ -173,9 +191,11 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
                 uint8_t *sm = smem + (size_t)st.i * STAGE_BYTES;
                 uint64_t *bar = &bar_full[st.i];
                 if (ps_elect_one()) {
-                    ps_mbar_expect_tx(bar, NA * PT_BLOCK + PT_BLOCK / n_sub);
-                    ps_bulk_g2s(sm, pa0, PT_BLOCK, bar);
-                    if (NA == 2) ps_bulk_g2s(sm + PT_BLOCK, pa1, PT_BLOCK, bar);
+                    if (g >= ahead) {
+                        ps_mbar_expect_tx(bar, NA * PT_BLOCK + PT_BLOCK / n_sub);
+                        ps_bulk_g2s(sm, pa0, PT_BLOCK, bar);
+                        if (NA == 2) ps_bulk_g2s(sm + PT_BLOCK, pa1, PT_BLOCK, bar);
+                    }
                     if (n_sub == 1) ps_bulk_g2s(sm + NA * PT_BLOCK, pb, PT_BLOCK, bar);
                     else // the part's tokens of every k-chunk, at the places they have in the whole tile
 #pragma unroll

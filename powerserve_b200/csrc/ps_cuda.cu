@@ -296,7 +296,10 @@ void build_rope_table(const ps_cuda_model_desc &d, std::vector<float> &t, const 
     }
 }
 
-// launch with programmatic dependence on the kernel before (ps_grid_dep): its start-up, and in some kernels the first weights, overlap that one's end
+// launch with programmatic dependence on the kernel before (ps_grid_dep): its start-up, and in some kernels the first weights, overlap that one's end.
+// Not for a kernel whose CTAs compute for microseconds and would all fit a part of the SMs: those that come early crowd on the SMs that are free
+// first (SiLU and packing of four 1B layers' 77 tokens, eight CTAs of 16 an SM: a pass 627 us early, 600 after the GEMM has gone; 12 tokens of two 8B
+// layers 394 and 380)
 template <typename... KArgs, typename... Args>
 int launch_k(ps_cuda_ctx *ctx, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, Args... args) {
     cudaLaunchConfig_t cfg{};
@@ -888,7 +891,10 @@ int tc_gemm(ps_cuda_ctx *ctx, const ActIn &x, const uint8_t *a_blocks, int64_t n
     const TcPlan plan = tc_plan(ctx, n_tiles, K, bs);
     const int nt = plan.nt, n_ct = (bs + nt - 1) / nt;
     if (x.norm) PS_DEP(ps_k_tc_norm_b, (unsigned)(n_ct * nt), 512, 0, ctx->tc_b, x.x, x.norm, K, ctx->d.norm_eps, bs, nt);
-    else PS_DEP(ps_k_tc_prep_b, dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->tc_b, x.x, x.u, K, bs, nt);
+    else if (x.u) { // (not early: launch_k)
+        ps_k_tc_prep_b<<<dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->stream>>>(ctx->tc_b, x.x, x.u, K, bs, nt);
+        PS_LAUNCH_CK();
+    } else PS_DEP(ps_k_tc_prep_b, dim3((unsigned)((tc_nbp(K) + 3) / 4), (unsigned)(n_ct * nt)), 128, 0, ctx->tc_b, x.x, x.u, K, bs, nt);
     a.err = ctx->tc_err_dev;
     a.a = a_blocks; a.b = ctx->tc_b; a.nbp = (int)tc_nbp(K); a.n_ct = n_ct; a.n_tiles = (int)n_tiles * n_ct; a.n_seg = n_seg; a.bs = bs; a.residual = residual;
     a.part = ctx->tc_part; a.cnt = ctx->tc_cnt; a.give_up = ctx->opt_give_up; a.limit = give_up_cycles(ctx);
