@@ -13,6 +13,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
+#include <initializer_list>
 #include <mutex>
 #include <string>
 #include <unordered_map>
@@ -70,6 +71,7 @@ struct LayerDev {
     uint8_t *tc_qkv = nullptr, *tc_o = nullptr, *tc_gu = nullptr, *tc_down = nullptr; // packed blocks of the tcgen05 GEMM (gate rows, then up rows from the next tile border)
     // octet copies for the 32-block mat-vec (ps_mv32.cuh; all-Q4_0 / all-Q8_0 models): q|k|v rows, o, gate|up rows, down
     uint8_t *mv_qkv = nullptr, *mv_o = nullptr, *mv_gu = nullptr, *mv_down = nullptr;
+    uint8_t *mt_q = nullptr, *mt_k = nullptr, *mt_v = nullptr, *mt_o = nullptr, *mt_gate = nullptr, *mt_up = nullptr, *mt_down = nullptr; // the same models' weight records of the batch products
 };
 
 } // namespace
@@ -122,7 +124,7 @@ struct ps_cuda_ctx {
     float *h_logits = nullptr;                                          // pinned staging for logits
     size_t h_logits_cap = 0;
     // options / counters
-    int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_scores_batch_min = 2, opt_give_up = -1;
+    int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_mt_min = 2, opt_scores_batch_min = 2, opt_give_up = -1;
     bool tc_ok = false;        // tensor-core prefill operands are resident
     uint8_t *tc_b = nullptr;   // B operand blocks of the current activation batch
     float *tc_part = nullptr;  // numbers of the tiles that CTAs share: a slot per CTA, for tiles of up to tc_nt columns
@@ -148,6 +150,8 @@ struct ps_cuda_ctx {
     bool mv_ok = false;      // every matmul weight is Q4_0 (or every one Q8_0): the fused 32-block decode path applies (ps_mv32.cuh)
     int mv_type = 0;
     uint8_t *mv_out = nullptr;
+    bool mt_ok = false;      // weight records of ps_k_matmul_mt are resident
+    uint8_t *mt_out = nullptr, *mt_x = nullptr; // lm_head; activation records of a batch (at the end of the same allocation)
     bool ops_graph_ok = false; // any supported mix of weight types: the graph-replayed operator-table decode step applies (decode_step_ops)
     int opt_ops_graph = 1;
     int n_sm = 148;
@@ -424,7 +428,7 @@ int matmul_q(ps_cuda_ctx *ctx, float *dst, const uint8_t *w, int wtype, int64_t 
     }
 }
 
-// matmul_q on the octet copies of an all-Q4_0 / all-Q8_0 model (ps_k_matmul_ob):
+// matmul_q on the octet copies of an all-Q4_0 / all-Q8_0 model (ps_k_matmul_ob), where HBM has no room for the records of ps_k_matmul_mt:
 template <int TYPE> int mo_warps(int64_t K, int C) { // warps of a CTA: their octets and the activations fit shared memory
     int warps = PS_MB_WARPS;
     while (warps > 1 && ps_mo_smem<TYPE>(K, C, warps) > 200 * 1024) warps >>= 1;
@@ -482,6 +486,64 @@ int matmul_ob(ps_cuda_ctx *ctx, int64_t K, int64_t bs, const PsMbSeg *segs, int 
     const int C = bs <= 2 ? 2 : bs <= 4 || (ctx->mv_type == 2 ? mo_four_columns<2>(ctx, K, bs, segs, n_seg) : mo_four_columns<8>(ctx, K, bs, segs, n_seg)) ? 4 : 8;
     if (ctx->mv_type == 2) return C == 2 ? launch_mo<2, 2>(ctx, a, done) : C == 4 ? launch_mo<2, 4>(ctx, a, done) : launch_mo<2, 8>(ctx, a, done);
     return C == 2 ? launch_mo<8, 2>(ctx, a, done) : C == 4 ? launch_mo<8, 4>(ctx, a, done) : launch_mo<8, 8>(ctx, a, done);
+}
+
+// the same on the tensor cores (ps_k_matmul_mt), quantising included
+// Column tiles of eight a CTA takes: a wider unit unpacks and stages the weights for more columns, where there are units enough (Q4_0, K 896, 9728 rows on 16 / 32 / 64 /
+// 128 columns, us: 11.2 / 17.9 / 31.2 / 58.8 with one, 11.5 / 16.4 / 27.7 / 51.5 with two, 17.3 / 17.2 / 27.6 / 47.2 with four; K 4864, 896 rows on 32 / 128: 13.3 / 30.7, 16.4 / 30.7,
+// 25.3 / 33.7; Q8_0, K 2048, 16384 rows on 24 / 32 / 128: 38 / 48 / 174, 44 / 44 / 162, 46 / 46 / 153.  ps_k_matmul_ob: 20.4 / 32 / 56 / 104; 24.8 / 106; 84 / 105 / 388)
+int mt_tiles(const ps_cuda_ctx *ctx, int64_t row_tiles, int n_ct) {
+    int nt = 1;
+    int64_t cost = 100 * (int64_t)n_ct;
+    for (int c = 2; c <= 4; c *= 2) {
+        const int64_t cols = (n_ct + c - 1) / c * c;
+        if (row_tiles * cols >= (c == 2 ? 5 : 32) * ctx->n_sm && cols * (c == 2 ? 93 : 87) < cost) { nt = c; cost = cols * (c == 2 ? 93 : 87); }
+    }
+    return nt;
+}
+template <int TYPE, int NT> int launch_mt(ps_cuda_ctx *ctx, PsMtArgs a) {
+    static int resident[64] = {}; // CTAs that the registers let an SM hold
+    constexpr int STAGE = ps_mt_stage<TYPE, NT>(), RED = ps_mt_red<NT>(), GS = ps_mt_groups<NT>();
+    if (!resident[ctx->device]) {
+        cudaFuncAttributes fa;
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_mt<TYPE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        PS_CK(cudaFuncGetAttributes(&fa, ps_k_matmul_mt<TYPE, NT>));
+        resident[ctx->device] = std::max(1, 65536 / (160 * ((fa.numRegs + 7) & ~7)));
+    }
+    a.n_units = a.n_tiles * (((a.bs + 7) / 8 + NT - 1) / NT);
+    // a CTA per unit as long as they are resident together, with at least two stages each; the ring as deep as there is room
+    const int room = 220 * 1024, most = std::min(resident[ctx->device], std::max(1, room / (2 * STAGE + RED + 1280)));
+    const int per_sm = std::min(most, (a.n_units + ctx->n_sm - 1) / ctx->n_sm);
+    a.ns = std::max(1, std::min(std::min(PS_MT_MAX_NS, (a.nbg + GS - 1) / GS * ((a.n_units + per_sm * ctx->n_sm - 1) / (per_sm * ctx->n_sm))),
+                                std::min((200 * 1024 - RED) / STAGE, (room / per_sm - RED - 1280) / STAGE)));
+    PS_DEP((ps_k_matmul_mt<TYPE, NT>), (unsigned)std::min(a.n_units, per_sm * ctx->n_sm), 160, (size_t)a.ns * STAGE + RED, a);
+    return 0;
+}
+template <int TYPE> int launch_mt_t(ps_cuda_ctx *ctx, const PsMtArgs &a) {
+    switch (mt_tiles(ctx, a.n_tiles, (a.bs + 7) / 8)) {
+    case 4: return launch_mt<TYPE, 4>(ctx, a);
+    case 2: return launch_mt<TYPE, 2>(ctx, a);
+    default: return launch_mt<TYPE, 1>(ctx, a);
+    }
+}
+int matmul_mt(ps_cuda_ctx *ctx, const ActIn &in, int64_t K, int bs, std::initializer_list<PsMtSeg> segs, const float *residual) {
+    if (in.norm) PS_DEP(ps_k_mt_norm_quantize, (unsigned)bs, 512, 0, in.x, in.norm, K, ctx->d.norm_eps, ctx->mt_x);
+    else PS_DEP(ps_k_mt_quantize, dim3((unsigned)((K / 32 + 15) / 16), (unsigned)bs), 128, 0, in.x, in.u, K, ctx->mt_x);
+    PsMtArgs a{};
+    for (const PsMtSeg &s : segs) {
+        a.seg[a.n_seg] = s;
+        a.seg[a.n_seg++].tile0 = a.n_tiles;
+        a.n_tiles += (s.n + 15) / 16;
+    }
+    a.bs = bs; a.nbg = (int)((K / 32 + 3) / 4); a.x = ctx->mt_x; a.residual = residual; a.err = ctx->tc_err_dev; a.give_up = ctx->opt_give_up;
+    return ctx->mv_type == 2 ? launch_mt_t<2>(ctx, a) : launch_mt_t<8>(ctx, a);
+}
+int mt_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t rows, int64_t K) {
+    const dim3 grid((unsigned)((K / 32 + 3) / 4), (unsigned)((rows + 15) / 16));
+    if (ctx->mv_type == 2) ps_k_mt_pack<2><<<grid, 128, 0, ctx->stream>>>(dst, w, rows, K / 32);
+    else ps_k_mt_pack<8><<<grid, 128, 0, ctx->stream>>>(dst, w, rows, K / 32);
+    PS_LAUNCH_CK();
+    return 0;
 }
 
 int grid1d(int64_t n, int block = 256) { return (int)std::min<int64_t>((n + block - 1) / block, 148 * 8); }
@@ -2045,6 +2107,26 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
             }
             if ((rc = mk(&ctx->mv_out, d.vocab_size, dim))) return rc;
             if ((rc = mv_repack_t(ctx, ctx->mv_out, ctx->w_out, d.vocab_size, dim, 0))) return rc;
+            // weight records of the batch products (1.11x or 1.06x the GGUF bytes; only if HBM has room)
+            size_t need = ps_mt_w_bytes(t0, d.vocab_size, dim) + ps_mt_x_bytes(ctx->maxK, d.max_batch), free_b = 0, total_b = 0;
+            need += (size_t)d.n_layers * (ps_mt_w_bytes(t0, qdim, dim) + 2 * ps_mt_w_bytes(t0, kvd, dim) + ps_mt_w_bytes(t0, dim, qdim) + 2 * ps_mt_w_bytes(t0, ffn, dim) + ps_mt_w_bytes(t0, dim, ffn));
+            PS_CK(cudaMemGetInfo(&free_b, &total_b));
+            ctx->mt_ok = d.max_batch > 1 && need + ((size_t)8 << 30) < free_b;
+            if (ctx->mt_ok) { // (one allocation: seven a layer took longer than the packing)
+                uint8_t *at = nullptr;
+                if ((rc = dev_alloc(ctx, (void **)&at, need))) return rc;
+                auto rec = [&](uint8_t **p, const uint8_t *w, int64_t rows, int64_t K) -> int {
+                    *p = at;
+                    at += ps_mt_w_bytes(t0, rows, K);
+                    return mt_pack(ctx, *p, w, rows, K);
+                };
+                for (LayerDev &ld : ctx->layers)
+                    if ((rc = rec(&ld.mt_q, ld.wq, qdim, dim)) || (rc = rec(&ld.mt_k, ld.wk, kvd, dim)) || (rc = rec(&ld.mt_v, ld.wv, kvd, dim)) || (rc = rec(&ld.mt_o, ld.wo, dim, qdim)) ||
+                        (rc = rec(&ld.mt_gate, ld.wgate, ffn, dim)) || (rc = rec(&ld.mt_up, ld.wup, ffn, dim)) || (rc = rec(&ld.mt_down, ld.wdown, dim, ffn)))
+                        return rc;
+                if ((rc = rec(&ctx->mt_out, ctx->w_out, d.vocab_size, dim))) return rc;
+                ctx->mt_x = at;
+            }
             PS_CK(cudaStreamSynchronize(ctx->stream));
             ctx->mv_ok = true;
         }
@@ -2186,6 +2268,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
     // 125 / 123, 158 / 124, 165 / 125; 512 x 1536 87 / 92, 93 / 92, 98 / 93
     const bool tc = ctx->tc_ok && ctx->opt_tc && ctx->opt_fused && bs >= ctx->opt_tc_min;
     const bool mo = bs > 1 && mv_usable(ctx); // octet copies of a 32-block model
+    const bool mt = mo && ctx->mt_ok && bs >= ctx->opt_mt_min; // on the tensor cores
     const bool rw = ctx->fused_ok && ctx->opt_fused && (bs > 1 || tree); // octet-interleaved copies exist: multi-column row-walker
     int rc;
     PS_DEP(ps_k_get_embedding, embed_grid(bs, dim), 256, 0, ctx->x, ctx->w_embd, ctx->t_embd, dim, ctx->tokens_dev);
@@ -2208,6 +2291,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             a.seg[1] = {ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)qdim, (int)(qdim + kvd), 0};
             a.seg[2] = {ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)(qdim + kvd), (int)(qdim + 2 * kvd), 0};
             if ((rc = launch_rwm(ctx, a))) return rc;
+        } else if (mt) {
+            const bool bias = d.qkv_bias != 0;
+            if ((rc = matmul_mt(ctx, {ctx->x, nullptr, ld.attn_norm}, dim, bs, {{ld.mt_q, ctx->q, bias ? ld.q_bias : nullptr, (int)qdim}, {ld.mt_k, ctx->k, bias ? ld.k_bias : nullptr, (int)kvd},
+                                {ld.mt_v, ctx->v, bias ? ld.v_bias : nullptr, (int)kvd}}, nullptr))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tq, {ctx->x, nullptr, ld.attn_norm}, dim, bs))) return rc;
             const PsMbSeg sg[3] = {{ld.wq, ctx->q, d.qkv_bias ? ld.q_bias : nullptr, (int)qdim, 0}, {ld.wk, ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)kvd, 0},
@@ -2248,6 +2335,8 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         } else if (rw) {
             if ((rc = rwm_quantize(ctx, ctx->att, (int)qdim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_o, (int)dim, (int)qdim, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
+        } else if (mt) {
+            if ((rc = matmul_mt(ctx, {ctx->att}, qdim, bs, {{ld.mt_o, ctx->x, nullptr, (int)dim}}, ctx->x))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.to, {ctx->att}, qdim, bs))) return rc;
             bool done = false;
@@ -2262,6 +2351,8 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 0, 2, ctx->g, bs, nullptr, nullptr))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_gu, (int)ffn, (int)dim, 1, 2, ctx->u, bs, nullptr, nullptr))) return rc;
+        } else if (mt) {
+            if ((rc = matmul_mt(ctx, {ctx->x, nullptr, ld.ffn_norm}, dim, bs, {{ld.mt_gate, ctx->g, nullptr, (int)ffn}, {ld.mt_up, ctx->u, nullptr, (int)ffn}}, nullptr))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tgate, {ctx->x, nullptr, ld.ffn_norm}, dim, bs))) return rc;
             bool done = false;
@@ -2285,6 +2376,8 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             PS_LAUNCH_CK();
             if ((rc = rwm_quantize(ctx, ctx->g, (int)ffn, bs))) return rc;
             if ((rc = rwm_single(ctx, ld.rw_down, (int)dim, (int)ffn, 0, 1, ctx->x, bs, nullptr, ctx->x))) return rc;
+        } else if (mt) {
+            if ((rc = matmul_mt(ctx, {ctx->g, ctx->u}, ffn, bs, {{ld.mt_down, ctx->x, nullptr, (int)dim}}, ctx->x))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ld.tdown, {ctx->g, ctx->u}, ffn, bs))) return rc;
             bool done = false;
@@ -2300,6 +2393,8 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = rms_norm(ctx, ctx->w_out_norm, bs))) return rc;
             if ((rc = rwm_quantize(ctx, ctx->xn, (int)dim, bs))) return rc;
             if ((rc = rwm_single(ctx, ctx->rw_out, d.vocab_size, (int)dim, 0, 1, ctx->logits, bs, nullptr, nullptr))) return rc;
+        } else if (mt) {
+            if ((rc = matmul_mt(ctx, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs, {{ctx->mt_out, ctx->logits, nullptr, d.vocab_size}}, nullptr))) return rc;
         } else {
             if ((rc = quantize_act(ctx, ctx->t_out, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs))) return rc;
             bool done = false;
@@ -2956,6 +3051,7 @@ int ps_cuda_set_option(ps_cuda_ctx *ctx, const char *name, int value) {
     else if (!strcmp(name, "scores_batch_min")) ctx->opt_scores_batch_min = std::max(1, value); // batches at least this wide use the query-blocked scores kernel
     else if (!strcmp(name, "give_up_warp")) ctx->opt_give_up = value; // tests of the way out of a pipeline whose wait has run out
     else if (!strcmp(name, "tc_min")) ctx->opt_tc_min = std::max(2, value); // narrowest batch that takes the tcgen05 GEMM (narrower ones: multi-column row-walker)
+    else if (!strcmp(name, "mt_min")) ctx->opt_mt_min = std::max(2, value); // narrowest batch of a 32-block model that multiplies on the tensor cores (narrower ones, and all where its records found no room: ps_k_matmul_ob)
     else if (!strcmp(name, "attn_tile")) ctx->opt_attn_tile = value; // register-tiled scores / P.V kernels for batches (0: the first-generation kernels, for A/B)
     else if (!strcmp(name, "pv_batch_min")) ctx->opt_pv_batch_min = value; // batches at least this wide use the query-blocked P.V kernel (prefill), narrower ones the per-(head, dim) warp kernel
     else if (!strcmp(name, "rw_unroll2")) ctx->opt_unroll2 = value; // tuning: two blocks per loop trip in the mat-vec launches with <= 8 octets per CTA

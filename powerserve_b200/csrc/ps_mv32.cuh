@@ -459,3 +459,246 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
         }
     }
 }
+
+// ---------------------------------------------------------------------------------------------------- token batches on the tensor cores
+// The same product on the tensor cores.  A block adds fl(d_x d_y) * S to each of eight chains, S the INTEGER sum of four products, and dp4a (2 cycles of the
+// FMA pipe a warp), the integer-to-float step, the factor (every lane's own) and the FMA are five cycles of that pipe for 32 chain steps.
+// mma.sync m16n8k8 makes 128 such sums, already float and exact (halves of 11 bits, products and sums of at most 17 bits in fp32), in 8 cycles of a
+// pipe that runs beside the FMAs, and leaves a factor to eight chain steps.  Its k holds two AVX lanes, l and l + 4 (k = 2t: element t of lane l, k = 2t + 1: of
+// lane l + 4), so the activation word is masked to one half for each of the two sums.  Any shape of mma.sync takes 8 cycles: 64 for 1024 chain steps.
+// Warp w of a CTA takes lanes w and w + 4 of 16 rows x 8 NT columns; the chains of a row meet in shared memory at the end.  Weights and activations
+// pass through a ring of stages that a fifth warp fills by bulk copies, over all of the CTA's tiles in a row, the first weights before the kernel
+// before has ended.  The weights have an order of their own, in which a lane reads what it needs of four blocks at once: on the octet copies half of the
+// instructions were byte loads and conversions of scales.
+// Measured (Q4_0, 896 wide, 32 / 128 columns, us a product, cold caches; dp4a before): q|k|v 5.7 / 8.9 (9.4 / 17.6), o 6.5 / 9.1 (12 / 21), gate|up 16.4 / 47 (32 / 104), down 13.3 / 31
+// (25 / 106); 32 tokens of six layers 632 -> 405 us.  HMMA pipe 30 % busy, issue 50 %: packed pairs need moves (14 instructions an MMA; with plain
+// floats 13, and Q8_0 with two column tiles 162 -> 205 us).
+//
+// weight record of (16 rows, four blocks), g = lane / 4, t = lane % 4, rows g and g + 8: [4 w][32 lanes][2 rows][4 blocks] bytes (low nibble: element t of lane w,
+// high nibble: of lane w + 4) or byte pairs (+ 128; of lanes w, w + 4), then [8 g][2 rows][4 blocks] scales.  Blocks past the row's end and rows past the matrix have scale zero
+template <int TYPE> PS_HD constexpr int ps_mt_wq() { return TYPE == 2 ? 1024 : 2048; }
+template <int TYPE> PS_HD constexpr int ps_mt_wrec() { return ps_mt_wq<TYPE>() + 256; }
+PS_HD size_t ps_mt_w_bytes(int type, int64_t rows, int64_t K) { return (size_t)((rows + 15) / 16) * (size_t)((K / 32 + 3) / 4) * (type == 2 ? ps_mt_wrec<2>() : ps_mt_wrec<8>()); }
+template <int TYPE> __global__ void __launch_bounds__(128) ps_k_mt_pack(uint8_t *__restrict__ dst, const uint8_t *__restrict__ w, int64_t n_rows, int64_t nb) { // grid (groups, tiles)
+    constexpr int SRC = PsMv32<TYPE>::SRC;
+    const int64_t g4 = blockIdx.x, tile = blockIdx.y;
+    uint8_t *out = dst + (tile * gridDim.x + g4) * ps_mt_wrec<TYPE>();
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
+    for (int r = 0; r < 2; r++) {
+        const int64_t row = tile * 16 + r * 8 + (lane >> 2);
+        for (int b = 0; b < 4; b++) {
+            const int64_t i = g4 * 4 + b;
+            const bool live = row < n_rows && i < nb;
+            const uint8_t *blk = w + (row * nb + i) * SRC;
+            if (TYPE == 2) out[(threadIdx.x * 2 + r) * 4 + b] = live ? blk[2 + 4 * wp + t] : 0x88;
+            else
+                for (int h = 0; h < 2; h++) out[((threadIdx.x * 2 + r) * 4 + b) * 2 + h] = live ? blk[2 + 16 * h + 4 * wp + t] ^ 0x80 : 0x80;
+            if (wp == 0 && t == 0)
+                reinterpret_cast<float *>(out + ps_mt_wq<TYPE>())[(lane >> 2) * 8 + r * 4 + b] = live ? ps_half_bits_to_float((uint32_t)blk[0] | (uint32_t)blk[1] << 8) : 0.f;
+        }
+    }
+}
+// activation record of (8 columns, four blocks): [4 w][8 columns][4 t][4 blocks] pairs of halves (lane w, lane w + 4), then [4 t][4 blocks][columns 2t, 2t + 1] scales
+#define PS_MT_REC 2176
+PS_HD size_t ps_mt_x_bytes(int64_t K, int64_t cols) { return (size_t)((cols + 7) / 8) * (size_t)((K / 32 + 3) / 4) * PS_MT_REC; }
+// one warp, four blocks of a column (lane = 8 b + l: word l of block b); blocks past the row's end are zeros
+PS_D void ps_mt_store(uint8_t *__restrict__ dst, float4 v, int lane, int64_t g, int64_t col, int64_t nbg) {
+    uint32_t word;
+    float d;
+    ps_mv_quant4(v, word, d);
+    const int b = lane >> 3, l = lane & 7, n = (int)(col & 7);
+    uint8_t *rec = dst + ((col >> 3) * nbg + g) * PS_MT_REC;
+    const uint32_t other = __shfl_xor_sync(PS_FULL, word, 4), lo = l < 4 ? word : other, hi = l < 4 ? other : word; // lanes l % 4 and l % 4 + 4
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int t = (l >> 2) * 2 + k;
+        const __half2 h = __halves2half2(__int2half_rn((int)(signed char)(lo >> (8 * t))), __int2half_rn((int)(signed char)(hi >> (8 * t))));
+        reinterpret_cast<__half2 *>(rec)[(((l & 3) * 8 + n) * 4 + t) * 4 + b] = h;
+    }
+    if (l == 0) reinterpret_cast<float *>(rec + 2048)[((n >> 1) * 4 + b) * 2 + (n & 1)] = d;
+}
+__global__ void __launch_bounds__(128) ps_k_mt_quantize(const float *__restrict__ x, const float *__restrict__ u, int64_t K, uint8_t *__restrict__ dst) {
+    ps_grid_dep();
+    const int lane = threadIdx.x & 31;
+    const int64_t nb = K / 32, nbg = (nb + 3) / 4, g = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5), i = g * 4 + (lane >> 3), col = blockIdx.y, at = col * K + i * 32 + 4 * (lane & 7);
+    if (g >= nbg) return;
+    ps_mt_store(dst, i < nb ? ps_act4(x + at, u ? u + at : nullptr) : make_float4(0.f, 0.f, 0.f, 0.f), lane, g, col, nbg);
+}
+__global__ void __launch_bounds__(512) ps_k_mt_norm_quantize(const float *__restrict__ x, const float *__restrict__ w, int64_t dim, float eps, uint8_t *__restrict__ dst) {
+    ps_grid_dep();
+    __shared__ double sh[32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t col = blockIdx.x, nb = dim / 32, nbg = (nb + 3) / 4;
+    const float *xr = x + col * dim;
+    const float scale = ps_rms_scale(xr, dim, eps, sh);
+    for (int64_t g = warp; g < nbg; g += 16) {
+        const int64_t i = g * 4 + (lane >> 3), at = i * 32 + 4 * (lane & 7);
+        ps_mt_store(dst, i < nb ? ps_norm4(xr + at, w + at, scale) : make_float4(0.f, 0.f, 0.f, 0.f), lane, g, col, nbg);
+    }
+}
+
+struct PsMtSeg { const uint8_t *w; float *dst; const float *bias; int n, tile0; }; // w: weight records
+struct PsMtArgs {
+    PsMtSeg seg[3];
+    int n_seg, bs, nbg, n_tiles, n_units, ns; // groups of four blocks; row tiles, x column groups: units of work; stages of the ring
+    const uint8_t *x;   // activation records
+    const float *residual;
+    int *err, give_up;
+};
+#define PS_MT_MAX_NS 8
+// groups of a stage: a wait and the issue of its copies cost some hundred cycles, a group's MMAs 64 NT (one group a stage, refilled by a thread of the first
+// warp behind a CTA barrier: 1000 cycles a group whatever NT)
+template <int NT> PS_HD constexpr int ps_mt_groups() { return NT == 1 ? 4 : 2; }
+template <int TYPE, int NT> PS_HD constexpr int ps_mt_stage() { return ps_mt_groups<NT>() * (ps_mt_wrec<TYPE>() + NT * PS_MT_REC); }
+template <int NT> PS_HD constexpr int ps_mt_red() { return 4 * 8 * NT * 16 * 4; } // [4 w][8 NT columns][16 rows] floats
+// the sums of one AVX lane: (row g, columns 2t, 2t + 1), (row g + 8, the same)
+PS_D void ps_mt_mma(float (&s)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%7,%7,%7,%7};"
+        : "=f"(s[0]), "=f"(s[1]), "=f"(s[2]), "=f"(s[3])
+        : "r"(a0), "r"(a1), "r"(b), "f"(0.f));
+}
+template <int TYPE, int NT>
+__global__ void __launch_bounds__(160) ps_k_matmul_mt(const PsMtArgs a) {
+    constexpr int GS = ps_mt_groups<NT>(), WREC = ps_mt_wrec<TYPE>(), STAGE = ps_mt_stage<TYPE, NT>(), X0 = GS * WREC;
+    extern __shared__ __align__(128) uint8_t ps_mt_smem[];
+    __shared__ __align__(8) uint64_t bar_full[PS_MT_MAX_NS], bar_empty[PS_MT_MAX_NS];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gr = lane >> 2, t = lane & 3;
+    const int nbg = a.nbg, ns = a.ns, n_st = (nbg + GS - 1) / GS, n_ct = (a.bs + 7) / 8;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < ns; s++) {
+            ps_mbar_init(&bar_full[s], 1);
+            ps_mbar_init(&bar_empty[s], 4);
+        }
+        ps_fence_barrier_init();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    __syncthreads();
+    auto seg_of = [&](int tile) { return a.n_seg > 2 && tile >= a.seg[2].tile0 ? 2 : a.n_seg > 1 && tile >= a.seg[1].tile0 ? 1 : 0; };
+    if (warp == 4) { // ===== copies
+        auto weights = [&](int u, int k, int slot) { // stage k of unit u
+            const int tile = u % a.n_tiles, n = min(GS, nbg - GS * k);
+            const PsMtSeg &seg = a.seg[seg_of(tile)];
+            ps_mbar_expect_tx(&bar_full[slot], (uint32_t)(n * (WREC + NT * PS_MT_REC)));
+            ps_bulk_g2s(ps_mt_smem + (size_t)slot * STAGE, seg.w + ((size_t)(tile - seg.tile0) * nbg + GS * k) * WREC, (uint32_t)(n * WREC), &bar_full[slot]);
+        };
+        auto columns = [&](int u, int k, int slot) {
+            const int ct0 = u / a.n_tiles * NT, n = min(GS, nbg - GS * k);
+#pragma unroll
+            for (int j = 0; j < NT; j++) // (past the last tile: that one again)
+                ps_bulk_g2s(ps_mt_smem + (size_t)slot * STAGE + X0 + j * (GS * PS_MT_REC), a.x + ((size_t)min(ct0 + j, n_ct - 1) * nbg + GS * k) * PS_MT_REC, (uint32_t)(n * PS_MT_REC),
+                            &bar_full[slot]);
+        };
+        const int ahead = min(ns, n_st);
+        if (ps_elect_one())
+            for (int k = 0; k < ahead; k++) weights(blockIdx.x, k, k);
+        __syncwarp();
+        ps_grid_dep();
+        int slot = 0, n = 0;
+        uint32_t phase = 0;
+        for (int u = blockIdx.x; u < a.n_units; u += gridDim.x)
+            for (int k = 0; k < n_st; k++, n++) {
+                if (n >= ns && !ps_tc_wait_warp(&bar_empty[slot], phase ^ 1)) *a.err = PS_ERR_COPY;
+                if (ps_elect_one()) {
+                    if (n >= ahead) weights(u, k, slot);
+                    columns(u, k, slot);
+                }
+                __syncwarp();
+                if (++slot == ns) { slot = 0; phase ^= 1; }
+            }
+        return; // (the other warps wait for every copy)
+    }
+    ps_grid_dep();
+    if (warp == a.give_up) *a.err = PS_ERR_COPY;
+    float *red = reinterpret_cast<float *>(ps_mt_smem + (size_t)ns * STAGE);
+    int slot = 0;
+    uint32_t phase = 0;
+    for (int u = blockIdx.x; u < a.n_units; u += gridDim.x) {
+        ps_f2 acc[2][2][NT]; // [lane w, w + 4][row g, g + 8][column tile]: columns 2t, 2t + 1
+#pragma unroll
+        for (int j = 0; j < NT; j++) acc[0][0][j] = acc[0][1][j] = acc[1][0][j] = acc[1][1][j] = 0ull;
+        for (int k = 0; k < n_st; k++) {
+            // after a wait that gave up the results are invalid; the loop goes on and waits for the other copies, each within its limit, so that none is in
+            // flight when this shared memory becomes another CTA's
+            if (!ps_tc_wait(&bar_full[slot], phase)) *a.err = PS_ERR_COPY;
+            const uint8_t *st = ps_mt_smem + (size_t)slot * STAGE;
+            auto group = [&](int g) {
+                const uint8_t *sw = st + g * WREC;
+                uint32_t av[2][4];  // [row g, g + 8][block]: the halves of lanes w and w + 4
+                if (TYPE == 2) { // low nibble n, high nibble m of a byte: halves 1024 + n and 1024 + 16 m, made n - 8 and m - 8
+                    const uint2 q = *reinterpret_cast<const uint2 *>(sw + (warp * 32 + lane) * 8);
+#pragma unroll
+                    for (int r = 0; r < 2; r++)
+#pragma unroll
+                        for (int b = 0; b < 4; b++) {
+                            const uint32_t h = __byte_perm(r ? q.y : q.x, 0, b | 0x4040 | b << 8) & 0x00F0000Fu | 0x64006400u;
+                            asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(av[r][b]) : "r"(h), "r"(0x2C003C00u), "r"(0xD480E408u)); // x (1, 1 / 16) + (-1032, -72)
+                        }
+                } else { // 1024 + 128 + q - 1152
+                    const uint4 q = *reinterpret_cast<const uint4 *>(sw + (warp * 32 + lane) * 16);
+                    const uint32_t w[2][2] = {{q.x, q.y}, {q.z, q.w}};
+#pragma unroll
+                    for (int r = 0; r < 2; r++)
+#pragma unroll
+                        for (int b = 0; b < 4; b++)
+                            asm("add.rn.f16x2 %0, %1, %2;" : "=r"(av[r][b]) : "r"(__byte_perm(w[r][b >> 1], 0x64646464u, (b & 1) ? 0x4342 : 0x4140)), "r"(0xE480E480u));
+                }
+                const float4 d0 = *reinterpret_cast<const float4 *>(sw + ps_mt_wq<TYPE>() + gr * 32), d1 = *reinterpret_cast<const float4 *>(sw + ps_mt_wq<TYPE>() + gr * 32 + 16);
+                const float xd[2][4] = {{d0.x, d0.y, d0.z, d0.w}, {d1.x, d1.y, d1.z, d1.w}};
+#pragma unroll
+                for (int j = 0; j < NT; j++) {
+                    const uint8_t *sx = st + X0 + (j * GS + g) * PS_MT_REC;
+                    const uint4 bq = *reinterpret_cast<const uint4 *>(sx + (warp * 32 + lane) * 16);
+                    const ulonglong2 y01 = *reinterpret_cast<const ulonglong2 *>(sx + 2048 + t * 32), y23 = *reinterpret_cast<const ulonglong2 *>(sx + 2048 + t * 32 + 16);
+                    const uint32_t bw[4] = {bq.x, bq.y, bq.z, bq.w};
+                    const ps_f2 yd[4] = {y01.x, y01.y, y23.x, y23.y};
+#pragma unroll
+                    for (int b = 0; b < 4; b++) {
+                        float s[2][4];
+                        ps_mt_mma(s[0], av[0][b], av[1][b], bw[b] & 0xFFFFu);
+                        ps_mt_mma(s[1], av[0][b], av[1][b], bw[b] & 0xFFFF0000u);
+                        const ps_f2 d[2] = {ps_f2_mul(ps_f2_pack(xd[0][b], xd[0][b]), yd[b]), ps_f2_mul(ps_f2_pack(xd[1][b], xd[1][b]), yd[b])};
+#pragma unroll
+                        for (int l = 0; l < 2; l++)
+#pragma unroll
+                            for (int r = 0; r < 2; r++) acc[l][r][j] = ps_f2_fma(d[r], ps_f2_pack(s[l][2 * r], s[l][2 * r + 1]), acc[l][r][j]);
+                    }
+                }
+            };
+            if (GS * (k + 1) <= nbg) {
+#pragma unroll(NT == 4 ? 1 : GS) // a warp is often alone on its scheduler: the loads of one group then fly beside the MMAs and FMAs of the other
+                for (int g = 0; g < GS; g++) group(g);
+            } else {
+#pragma unroll 1
+                for (int g = 0; g < nbg - GS * k; g++) group(g);
+            }
+            __syncwarp();
+            if (lane == 0) ps_mbar_arrive(&bar_empty[slot]);
+            if (++slot == ns) { slot = 0; phase ^= 1; }
+        }
+        // hsum_float_8: (x4 + x0, x5 + x1, x6 + x2, x7 + x3) -> (r0 + r2) + (r1 + r3)
+#pragma unroll
+        for (int j = 0; j < NT; j++)
+#pragma unroll
+            for (int r = 0; r < 2; r++) {
+                float p, q;
+                ps_f2_unpack(ps_f2_add(acc[1][r][j], acc[0][r][j]), p, q);
+                red[(warp * 8 * NT + 8 * j + 2 * t) * 16 + 8 * r + gr] = p;
+                red[(warp * 8 * NT + 8 * j + 2 * t + 1) * 16 + 8 * r + gr] = q;
+            }
+        ps_bar_sync(1, 128);
+        const int tile = u % a.n_tiles, ct0 = u / a.n_tiles * NT;
+        const PsMtSeg &seg = a.seg[seg_of(tile)];
+#pragma unroll
+        for (int k = 0; k < NT; k++) {
+            const int e = k * 128 + threadIdx.x, c = 8 * ct0 + (e >> 4), n = (tile - seg.tile0) * 16 + (e & 15);
+            float r = __fadd_rn(__fadd_rn(red[e], red[256 * NT + e]), __fadd_rn(red[128 * NT + e], red[384 * NT + e]));
+            if (c < a.bs && n < seg.n) {
+                const int64_t o = (int64_t)c * seg.n + n;
+                if (seg.bias) r = __fadd_rn(r, seg.bias[n]);
+                if (a.residual) r = __fadd_rn(a.residual[o], r);
+                seg.dst[o] = r;
+            }
+        }
+        if (u + (int)gridDim.x < a.n_units) ps_bar_sync(1, 128); // (the next tile's numbers go to the same place)
+    }
+}
