@@ -180,6 +180,10 @@ int ps_cuda_forward_sessions(ps_cuda_ctx *ctx, const int32_t *session_ids, const
 /* Model::decode with top_k = 1 (llama_model.cpp:119-132): forward + arg-max on the device; only the token id comes
  * back.  `n_steps` > 1 keeps feeding the produced id back in without a host round trip (ids_host gets n_steps ids). */
 int ps_cuda_decode_greedy(ps_cuda_ctx *ctx, int32_t first_token, int n_steps, int32_t *ids_host);
+/* page-locked host memory: logits buffers in it (of any of the forward calls above) are written by the device directly, others by way of a
+ * staging buffer and a copy on the host.  No context is needed; a buffer may outlive the contexts that wrote to it */
+int ps_cuda_host_alloc(size_t bytes, void **host);
+int ps_cuda_host_free(void *host);
 /* device-side logits of the last forward ([bs][vocab]) for callers that sample on the GPU */
 const float *ps_cuda_logits_dev(ps_cuda_ctx *ctx);
 /* Device-side sampling: ps_cuda_forward / ps_cuda_forward_sessions accept logits_host == NULL with

@@ -7,6 +7,8 @@ from __future__ import annotations
 import ctypes as C
 import json
 import os
+import threading
+import weakref
 from typing import Dict, List, Optional, Sequence
 
 import numpy as np
@@ -173,6 +175,8 @@ def load_library() -> C.CDLL:
         "ps_cuda_session_position": (ci, [vp, ci]),
         "ps_cuda_forward_sessions": (ci, [vp, i32p, i32p, ci, ci, fp, i32p]),
         "ps_cuda_logits_dev": (vp, [vp]),
+        "ps_cuda_host_alloc": (ci, [C.c_size_t, C.POINTER(vp)]),
+        "ps_cuda_host_free": (ci, [vp]),
         "ps_cuda_tp_unique_id": (ci, [vp]),
         "ps_cuda_tp_init": (ci, [vp, vp]),
         "ps_cuda_tp_export": (ci, [vp, vp]),
@@ -200,6 +204,54 @@ def exported_symbols() -> List[str]:
 
 def _i32(a: Sequence[int]) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(a, dtype=np.int32))
+
+
+class _LogitsPool:
+    """Page-locked buffers behind the logits arrays that a model hands out: the device writes them directly (a pageable array takes a second copy on the
+    host, 150 us for 1.6 MB).  At most two buffers of at most 16 MB; an array's buffer comes back when the array and all its views are gone, and is
+    freed if the model has been closed by then.  Whoever keeps more arrays alive, or larger ones, gets ordinary memory."""
+    MOST, LARGEST = 2, 16 << 20
+
+    def __init__(self, L):
+        self.L, self.lock, self.free, self.made, self.closed = L, threading.RLock(), [], 0, False  # (a finalizer may run inside)
+
+    def array(self, rows: int, cols: int) -> np.ndarray:
+        n = 4 * rows * cols
+        got = self._take(n) if 0 < n <= self.LARGEST else None
+        if got is None:
+            return np.empty((rows, cols), np.float32)
+        mem = (C.c_char * n).from_address(got[0])
+        weakref.finalize(mem, self._give, got).atexit = False
+        return np.frombuffer(mem, np.float32).reshape(rows, cols)
+
+    def _take(self, n: int):
+        with self.lock:
+            fit = next((b for b in self.free if b[1] >= n), None)
+            if fit is None and (self.made < self.MOST or self.free):
+                if self.made == self.MOST:      # a smaller one makes room
+                    self.L.ps_cuda_host_free(self.free.pop()[0])
+                    self.made -= 1
+                p = C.c_void_p()
+                if self.L.ps_cuda_host_alloc(n, C.byref(p)) == 0:
+                    self.made += 1
+                    return p.value, n
+            elif fit is not None:
+                self.free.remove(fit)
+            return fit
+
+    def _give(self, buf):
+        with self.lock:
+            if self.closed:
+                self.L.ps_cuda_host_free(buf[0])
+            else:
+                self.free.append(buf)
+
+    def close(self):
+        with self.lock:
+            self.closed = True
+            for b in self.free:
+                self.L.ps_cuda_host_free(b[0])
+            self.free = []
 
 
 class DeviceBuffer:
@@ -243,6 +295,7 @@ class CudaBackend:
         if rc != 0:
             raise PsCudaError(f"ps_cuda_create failed ({rc}): {self.L.ps_cuda_last_error(None).decode()}")
         self.h = h
+        self.logits_pool = _LogitsPool(self.L)
 
     def _ck(self, rc: int):
         if rc != 0:
@@ -252,6 +305,7 @@ class CudaBackend:
         if self.h:
             self.L.ps_cuda_destroy(self.h)
             self.h = None
+            self.logits_pool.close()
 
     # ---- memory
     def empty(self, n_floats: int) -> DeviceBuffer:
@@ -459,7 +513,7 @@ class CudaModel:
         t = _i32(tokens)
         bs = len(t)
         p = _i32(pos) if pos is not None else np.arange(self.position, self.position + bs, dtype=np.int32)
-        logits = np.empty((bs, self.vocab), np.float32) if lm_head else None
+        logits = self.be.logits_pool.array(bs, self.vocab) if lm_head else None
         self.be._ck(self.be.L.ps_cuda_forward(self.be.h, t.ctypes.data_as(C.POINTER(C.c_int32)), p.ctypes.data_as(C.POINTER(C.c_int32)),
                                               bs, int(lm_head), logits.ctypes.data if lm_head else None))
         return logits
@@ -469,7 +523,7 @@ class CudaModel:
         t, p = _i32(tokens), _i32(pos)
         bs = len(t)
         m = None if tree_mask is None else np.ascontiguousarray(np.asarray(tree_mask, dtype=np.uint8).reshape(bs, bs))
-        logits = np.empty((bs, self.vocab), np.float32) if lm_head else None
+        logits = self.be.logits_pool.array(bs, self.vocab) if lm_head else None
         self.be._ck(self.be.L.ps_cuda_forward_tree(self.be.h, t.ctypes.data_as(C.POINTER(C.c_int32)), p.ctypes.data_as(C.POINTER(C.c_int32)), bs,
                                                    m.ctypes.data if m is not None else None, int(lm_head), logits.ctypes.data if lm_head else None))
         return logits
@@ -498,7 +552,7 @@ class CudaModel:
         """one token of each session in ONE forward pass -> (logits [n][vocab] or None, device arg-max ids [n])"""
         sids, toks = _i32(session_ids), _i32(tokens)
         n = len(sids)
-        logits = np.empty((n, self.desc.vocab_size), np.float32) if (lm_head and want_logits) else None
+        logits = self.be.logits_pool.array(n, self.desc.vocab_size) if (lm_head and want_logits) else None
         ids = np.zeros(n, np.int32)
         self.be._ck(self.be.L.ps_cuda_forward_sessions(self.be.h, sids.ctypes.data_as(C.POINTER(C.c_int32)), toks.ctypes.data_as(C.POINTER(C.c_int32)), n,
                                                        1 if lm_head else 0, logits.ctypes.data_as(C.POINTER(C.c_float)) if logits is not None else None,

@@ -96,17 +96,17 @@ struct ps_cuda_ctx {
     int position = 0;
     // server-side batching: independent KV sets over one set of weights; the ACTIVE session's state lives in kc / vct /
     // position / slot_mask above, the others are parked here
-    struct KvSet { std::vector<float *> kc, vct; int position = 0; std::vector<uint8_t> slot_mask; };
+    struct KvSet { std::vector<float *> kc, vct; float **ptrs_dev = nullptr; int position = 0; std::vector<uint8_t> slot_mask; };
     std::unordered_map<int, KvSet> sessions;
     int cur_session = 0, next_session = 1;
     float **sess_ptrs_dev = nullptr, **h_sess_ptrs = nullptr; // [n_layers][2][max_batch] cache pointers of the current session batch
     // speculative decode (kv_cache.hpp:97-276): per-slot mask, last batch kept aside for KVCacheInterface::copy
     std::vector<uint8_t> slot_mask;      // host copy, 1 = masked (not attended)
     bool slot_mask_dirty = true;
-    uint8_t *slot_mask_dev = nullptr, *tree_dev = nullptr, *h_tree = nullptr;
+    uint8_t *slot_mask_dev = nullptr, *tree_dev = nullptr, *h_tree = nullptr, *h_mask = nullptr;
     float *tree_bias = nullptr;          // [max_batch][n_ctx] attention bias of the current tree batch
     float *k_stage = nullptr, *v_stage = nullptr; // [n_layers][max_batch][kvd_l]
-    float **kv_ptrs_dev = nullptr;       // [2 * n_layers]: K caches, then V^T caches
+    float **kv_ptrs_dev = nullptr;       // [2 * n_layers]: K caches, then V^T caches of the active set (every set has its table)
     int last_batch = 0;                  // tokens held by the staging rows
     // rope table
     float *rope_table = nullptr;
@@ -132,7 +132,7 @@ struct ps_cuda_ctx {
     int *tc_cnt = nullptr;     // per slot: passes handed over
     int *err_dev = nullptr;    // device-detected failures, [0] tcgen05 pipeline time-out (PS_ERR_COPY: a copy of a batch product), [1] peer wait gave up, [2] step-kernel barrier time-out
     int err_seen[3] = {};      // sticky host copy of the flags (counters "tc_error" / "tp_error" / "step_error")
-    int *h_err = nullptr;      // pinned mirror, read after every forward / decode (a set flag becomes PS_CUDA_ERR_CUDA)
+    int *h_err = nullptr;      // their memory: mapped host memory, so that reading them after every forward / decode takes no copy (a set flag becomes PS_CUDA_ERR_CUDA)
     int *tc_err_dev = nullptr; // = err_dev + 0 (counter "tc_error")
     int64_t n_tc = 0;          // tcgen05 GEMM launches (counter "tc_gemm_launches")
     int64_t n_tc_pp[7] = {};   // by a CTA's share of passes: one, two, more (counters "tc_gemm_pass1", "tc_gemm_pass2", "tc_gemm_pass6")
@@ -194,6 +194,7 @@ struct ps_cuda_ctx {
     int opt_attn_chunk = 0;         // testing: cap on the soft-max positions resident in shared memory (forces the chunked attention path)
     bool step_ok = false;           // the model / geometry qualifies for ps_k_step
     PsStLayer *st_layers = nullptr; // device table
+    bool st_stale = false;          // it has another set's caches
     PsStPeers *st_peers = nullptr;  // device table of the exchanged vectors on every rank
     unsigned long long *st_ll[5] = {}; // this rank's (value, epoch) vectors: x, x1, att, hq image, best
     size_t st_off[5] = {};          // tensor parallel: their offsets inside the exchange heap
@@ -254,20 +255,81 @@ int dev_alloc(ps_cuda_ctx *ctx, void **p, size_t bytes) {
 }
 
 // Failures detected on the device (tcgen05 pipeline or copy time-out, a peer wait or a grid barrier that gave up) become a C-ABI
-// status: the flags ride along with the call's final device-to-host copy.  Call with work enqueued; synchronises.
+// status: the kernels write the flags to mapped host memory.  Call with work enqueued; synchronises.
 uint32_t give_up_cycles(const ps_cuda_ctx *ctx) { return ctx->opt_give_up >= 0 ? 1u << 24 : PS_TC_WAIT_CYCLES; } // option "give_up_warp": the other waits run out within 10 ms
 int sync_and_check(ps_cuda_ctx *ctx) {
-    PS_CK(cudaMemcpyAsync(ctx->h_err, ctx->err_dev, 16, cudaMemcpyDeviceToHost, ctx->stream));
     PS_CK(cudaStreamSynchronize(ctx->stream));
-    if (ctx->h_err[0] | ctx->h_err[1] | ctx->h_err[2]) {
-        const int tc = ctx->h_err[0], tp = ctx->h_err[1], st = ctx->h_err[2];
-        for (int k = 0; k < 3; k++) ctx->err_seen[k] |= ctx->h_err[k];
-        PS_CK(cudaMemsetAsync(ctx->err_dev, 0, 16, ctx->stream));
+    volatile int *flag = ctx->h_err;
+    if (flag[0] | flag[1] | flag[2]) {
+        const int tc = flag[0], tp = flag[1], st = flag[2];
+        for (int k = 0; k < 3; k++) ctx->err_seen[k] |= flag[k];
+        for (int k = 0; k < 4; k++) flag[k] = 0;
         if (ctx->ag_ctr) PS_CK(cudaMemsetAsync(ctx->ag_ctr, 0, (size_t)ctx->d.n_layers * ctx->nkv_l * 8, ctx->stream)); // a group that gave up leaves its counter mid-instance
         if (ctx->tc_cnt) PS_CK(cudaMemsetAsync(ctx->tc_cnt, 0, (size_t)ctx->n_sm * 4, ctx->stream)); // a GEMM that gave up leaves its counters part-way
         return fail(ctx, PS_CUDA_ERR_CUDA, "device-side failure:%s%s%s (wait site %d; results of this call are invalid)", tc == PS_ERR_COPY ? " copy of a batch product did not arrive" : tc ? " tcgen05 pipeline time-out" : "",
                     tp ? " tensor-parallel peer wait gave up" : "", st ? " decode-step wait gave up" : "", st);
     }
+    return 0;
+}
+
+// What a call brings lies side by side, in pinned memory and on the device, so that one copy takes it there:
+// [max_batch tokens][max_batch positions][a tree's mask][the cache slots' mask].  The error flags are mapped host memory
+#define PS_TREE_MAX 32
+int host_buffers(ps_cuda_ctx *ctx) {
+    const size_t B = (size_t)ctx->d.max_batch, bytes = 8 * B + PS_TREE_MAX * PS_TREE_MAX + (size_t)ctx->d.n_ctx;
+    int rc = dev_alloc(ctx, (void **)&ctx->tokens_dev, bytes);
+    if (rc) return rc;
+    ctx->pos_dev = ctx->tokens_dev + B;
+    ctx->tree_dev = reinterpret_cast<uint8_t *>(ctx->pos_dev + B);
+    ctx->slot_mask_dev = ctx->tree_dev + PS_TREE_MAX * PS_TREE_MAX;
+    PS_CK(cudaMallocHost(&ctx->h_tokens, bytes));
+    ctx->h_pos = ctx->h_tokens + B;
+    ctx->h_tree = reinterpret_cast<uint8_t *>(ctx->h_pos + B);
+    ctx->h_mask = ctx->h_tree + PS_TREE_MAX * PS_TREE_MAX;
+    PS_CK(cudaMallocHost(&ctx->h_ids, 4 * 8192));
+    PS_CK(cudaHostAlloc(&ctx->h_err, 128, cudaHostAllocMapped)); // [0..2] flags, [3..] debug record of the step kernel (PS_ST_DEBUG builds)
+    memset(ctx->h_err, 0, 128);
+    PS_CK(cudaHostGetDevicePointer((void **)&ctx->err_dev, ctx->h_err, 0));
+    ctx->tc_err_dev = ctx->err_dev;
+    ctx->tp_err_dev = ctx->err_dev + 1;
+    return 0;
+}
+// tokens and positions of bs rows (they lie in the pinned buffer) to the device; tree: and its mask, and the slots' mask if it has changed
+int stage_call(ps_cuda_ctx *ctx, int bs, bool tree = false) {
+    const size_t B = (size_t)ctx->d.max_batch;
+    size_t bytes = 4 * (B + (size_t)bs);
+    if (tree) {
+        bytes = 8 * B + PS_TREE_MAX * PS_TREE_MAX;
+        if (ctx->slot_mask_dirty) {
+            memcpy(ctx->h_mask, ctx->slot_mask.data(), (size_t)ctx->d.n_ctx);
+            bytes += (size_t)ctx->d.n_ctx;
+            ctx->slot_mask_dirty = false;
+        }
+    }
+    PS_CK(cudaMemcpyAsync(ctx->tokens_dev, ctx->h_tokens, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    ctx->h2d += (int64_t)bytes;
+    return 0;
+}
+// logits of the last pass to the caller; synchronises and checks.  Pinned memory of the caller's is written directly, other memory by way of a pinned
+// buffer and a copy on the host, which for a few MB takes longer than the transfer (1.6 MB: 150 us and 30)
+int logits_to_host(ps_cuda_ctx *ctx, float *host, size_t bytes) {
+    cudaPointerAttributes at{};
+    const bool direct = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
+    if (!direct) {
+        cudaGetLastError();
+        if (bytes > ctx->h_logits_cap) {
+            if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
+            ctx->h_logits = nullptr;
+            ctx->h_logits_cap = 0;
+            PS_CK(cudaMallocHost(&ctx->h_logits, bytes));
+            ctx->h_logits_cap = bytes;
+        }
+    }
+    PS_CK(cudaMemcpyAsync(direct ? host : ctx->h_logits, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    const int rc = sync_and_check(ctx);
+    if (rc) return rc;
+    if (!direct) memcpy(host, ctx->h_logits, bytes);
+    ctx->d2h += (int64_t)bytes;
     return 0;
 }
 
@@ -1246,8 +1308,25 @@ template <int R2> int launch_step_r(ps_cuda_ctx *ctx, const PsStArgs &a, int img
     return 0;
 }
 
+int step_table(ps_cuda_ctx *ctx) {
+    const ps_cuda_model_desc &d = ctx->d;
+    std::vector<PsStLayer> tab(d.n_layers);
+    for (int L = 0; L < d.n_layers; L++) {
+        const LayerDev &ld = ctx->layers[L];
+        tab[L] = PsStLayer{ld.rw_qkv, ld.rw_o, ld.rw_gu, ld.rw_down, ld.attn_norm, ld.ffn_norm, d.qkv_bias ? ld.q_bias : nullptr,
+                           d.qkv_bias ? ld.k_bias : nullptr, d.qkv_bias ? ld.v_bias : nullptr, ctx->kc[L], ctx->vct[L]};
+    }
+    PS_CK(cudaMemcpyAsync(ctx->st_layers, tab.data(), sizeof(PsStLayer) * (size_t)d.n_layers, cudaMemcpyHostToDevice, ctx->stream));
+    PS_CK(cudaStreamSynchronize(ctx->stream)); // the host vector dies here
+    ctx->st_stale = false;
+    return 0;
+}
 // one decode step on the token in tokens_dev[0] at position pos_dev[0]; n_kv_max = the longest soft-max row this launch may see
 int launch_step(ps_cuda_ctx *ctx, int mode, int n_kv_max) {
+    if (ctx->st_stale) {
+        const int rc0 = step_table(ctx);
+        if (rc0) return rc0;
+    }
     const ps_cuda_model_desc &d = ctx->d;
     const int r2 = d.n_heads / d.n_kv_heads;
     PsStArgs a{};
@@ -1457,15 +1536,9 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
     PS_AL(ctx->aqs, ctx->maxK * B);
     PS_AL(ctx->ad, 4 * (ctx->maxK / 32) * B);
     PS_AL(ctx->absp, 4 * (ctx->maxK / 256 + 1) * 4 * B);
-    PS_AL(ctx->tokens_dev, 4 * B);
-    PS_AL(ctx->pos_dev, 4 * B);
     PS_AL(ctx->ids_dev, 4 * 4096);
     PS_AL(ctx->ctr_dev, 16);
-    PS_AL(ctx->err_dev, 128); // [0..2] flags, [3..] debug record of the step kernel (PS_ST_DEBUG builds)
-    PS_CKC(cudaMemsetAsync(ctx->err_dev, 0, 128, ctx->stream));
-    ctx->tc_err_dev = ctx->err_dev;
-    ctx->tp_err_dev = ctx->err_dev + 1;
-    PS_CKC(cudaMallocHost(&ctx->h_err, 16));
+    { int rc_ = host_buffers(ctx); if (rc_) return bail(rc_); }
     if (tp > 1) {
         auto up = [](size_t v) { return (v + 255) & ~(size_t)255; };
         ctx->off_att = 0;
@@ -1544,10 +1617,8 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
         PS_CKC(cudaMemsetAsync(ctx->ag_ctr, 0, nc * 8, ctx->stream));
     }
     {   // speculative decode: slot mask, staging rows of the last batch, cache pointer table, tree bias
-        const int64_t kvd_l = kvd / tp, tb = std::min<int64_t>(B, 32);
+        const int64_t kvd_l = kvd / tp, tb = std::min<int64_t>(B, PS_TREE_MAX);
         ctx->slot_mask.assign((size_t)d.n_ctx, 1); // nothing committed yet: every slot is masked (rollback state)
-        PS_AL(ctx->slot_mask_dev, (size_t)d.n_ctx);
-        PS_AL(ctx->tree_dev, (size_t)(tb * tb));
         PS_AL(ctx->tree_bias, 4 * (size_t)tb * (size_t)d.n_ctx);
         PS_AL(ctx->k_stage, 4 * (size_t)d.n_layers * (size_t)tb * (size_t)kvd_l);
         PS_AL(ctx->v_stage, 4 * (size_t)d.n_layers * (size_t)tb * (size_t)kvd_l);
@@ -1555,7 +1626,6 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
         std::vector<float *> ptrs(2 * (size_t)d.n_layers);
         for (int L = 0; L < d.n_layers; L++) { ptrs[L] = ctx->kc[L]; ptrs[d.n_layers + L] = ctx->vct[L]; }
         PS_CKC(cudaMemcpy(ctx->kv_ptrs_dev, ptrs.data(), sizeof(float *) * ptrs.size(), cudaMemcpyHostToDevice));
-        PS_CKC(cudaMallocHost(&ctx->h_tree, (size_t)(tb * tb)));
     }
     {
         std::vector<float> t;
@@ -1563,9 +1633,6 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
         PS_AL(ctx->rope_table, t.size() * 4);
         PS_CKC(cudaMemcpy(ctx->rope_table, t.data(), t.size() * 4, cudaMemcpyHostToDevice));
     }
-    PS_CKC(cudaMallocHost(&ctx->h_tokens, 4 * B));
-    PS_CKC(cudaMallocHost(&ctx->h_pos, 4 * B));
-    PS_CKC(cudaMallocHost(&ctx->h_ids, 4 * 8192));
     PS_CKC(cudaEventCreate(&ctx->ev0));
     PS_CKC(cudaEventCreate(&ctx->ev1));
     PS_CKC(cudaStreamSynchronize(ctx->stream));
@@ -1600,17 +1667,9 @@ int ps_cuda_create_arch(ps_cuda_ctx **out, int device, const ps_cuda_arch_desc *
         return code;
     };
     auto ck = [&](cudaError_t e, const char *what) { return e == cudaSuccess ? 0 : fail(ctx, PS_CUDA_ERR_CUDA, "%s failed: %s", what, cudaGetErrorString(e)); };
-    const int64_t B = desc->max_batch;
     if ((rc = ck(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "cudaStreamCreate"))) return bail(rc);
-    if ((rc = dev_alloc(ctx, (void **)&ctx->tokens_dev, 4 * B)) || (rc = dev_alloc(ctx, (void **)&ctx->pos_dev, 4 * B)) || (rc = dev_alloc(ctx, (void **)&ctx->ids_dev, 4 * 4096)) ||
-        (rc = dev_alloc(ctx, (void **)&ctx->ctr_dev, 16)) || (rc = dev_alloc(ctx, (void **)&ctx->err_dev, 128)) ||
+    if ((rc = host_buffers(ctx)) || (rc = dev_alloc(ctx, (void **)&ctx->ids_dev, 4 * 4096)) || (rc = dev_alloc(ctx, (void **)&ctx->ctr_dev, 16)) ||
         (rc = dev_alloc(ctx, (void **)&ctx->part_val, 4 * 1024)) || (rc = dev_alloc(ctx, (void **)&ctx->part_idx, 4 * 1024)))
-        return bail(rc);
-    if ((rc = ck(cudaMemsetAsync(ctx->err_dev, 0, 128, ctx->stream), "cudaMemsetAsync"))) return bail(rc);
-    ctx->tc_err_dev = ctx->err_dev;
-    ctx->tp_err_dev = ctx->err_dev + 1;
-    if ((rc = ck(cudaMallocHost(&ctx->h_err, 16), "cudaMallocHost")) || (rc = ck(cudaMallocHost(&ctx->h_tokens, 4 * B), "cudaMallocHost")) ||
-        (rc = ck(cudaMallocHost(&ctx->h_pos, 4 * B), "cudaMallocHost")) || (rc = ck(cudaMallocHost(&ctx->h_ids, 4 * 8192), "cudaMallocHost")))
         return bail(rc);
     { int v = 148; if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) ctx->n_sm = v; }
     ctx->kc.resize(desc->n_layers);
@@ -1665,10 +1724,8 @@ void ps_cuda_destroy(ps_cuda_ctx *ctx) {
     cudaStreamSynchronize(ctx->stream);
     for (void *p : ctx->owned) cudaFree(p);
     if (ctx->h_tokens) cudaFreeHost(ctx->h_tokens);
-    if (ctx->h_pos) cudaFreeHost(ctx->h_pos);
     if (ctx->h_ids) cudaFreeHost(ctx->h_ids);
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
-    if (ctx->h_tree) cudaFreeHost(ctx->h_tree);
     if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
     if (ctx->g_step) cudaGraphExecDestroy(ctx->g_step);
     if (ctx->g_fwd) cudaGraphExecDestroy(ctx->g_fwd);
@@ -1681,6 +1738,16 @@ void ps_cuda_destroy(ps_cuda_ctx *ctx) {
     if (ctx->arch) ps_arch_destroy(ctx->arch);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
+}
+
+int ps_cuda_host_alloc(size_t bytes, void **host) {
+    if (!host) return fail(nullptr, PS_CUDA_ERR_INVALID, "null argument");
+    const cudaError_t e = cudaHostAlloc(host, bytes ? bytes : 16, cudaHostAllocPortable);
+    return e == cudaSuccess ? 0 : fail(nullptr, PS_CUDA_ERR_OOM, "cudaHostAlloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+}
+int ps_cuda_host_free(void *host) {
+    const cudaError_t e = cudaFreeHost(host);
+    return e == cudaSuccess ? 0 : fail(nullptr, PS_CUDA_ERR_CUDA, "cudaFreeHost failed: %s", cudaGetErrorString(e));
 }
 
 int ps_cuda_sync(ps_cuda_ctx *ctx) {
@@ -2186,15 +2253,8 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
         if ((rc = dev_alloc(ctx, (void **)&ctx->rw_out, oct_bytes(vocab_l, dim, 1)))) return rc;
         if ((rc = rw_repack(ctx, ctx->rw_out, ctx->w_out, vocab_l, dim, 0, 0, 1))) return rc;
         {   // the persistent step kernel's per-layer table
-            std::vector<PsStLayer> tab(d.n_layers);
-            for (int L = 0; L < d.n_layers; L++) {
-                const LayerDev &ld = ctx->layers[L];
-                tab[L] = PsStLayer{ld.rw_qkv, ld.rw_o, ld.rw_gu, ld.rw_down, ld.attn_norm, ld.ffn_norm, d.qkv_bias ? ld.q_bias : nullptr,
-                                   d.qkv_bias ? ld.k_bias : nullptr, d.qkv_bias ? ld.v_bias : nullptr, ctx->kc[L], ctx->vct[L]};
-            }
             if (!ctx->st_layers && (rc = dev_alloc(ctx, (void **)&ctx->st_layers, sizeof(PsStLayer) * (size_t)d.n_layers))) return rc;
-            PS_CK(cudaMemcpyAsync(ctx->st_layers, tab.data(), sizeof(PsStLayer) * (size_t)d.n_layers, cudaMemcpyHostToDevice, ctx->stream));
-            PS_CK(cudaStreamSynchronize(ctx->stream)); // `tab` dies at the end of this scope
+            if ((rc = step_table(ctx))) return rc;
             ctx->step_ok = (d.head_size == 64 || d.head_size == 128) && ffn_l % 256 == 0 && d.vocab_size / 8 >= 1 && ctx->smem_optin >= 160 * 1024;
         }
         PS_CK(cudaStreamSynchronize(ctx->stream));
@@ -2537,9 +2597,7 @@ int ps_cuda_forward(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t *pos,
     PS_CK(cudaStreamSynchronize(ctx->stream));
     memcpy(ctx->h_tokens, tokens, (size_t)bs * 4);
     memcpy(ctx->h_pos, pos, (size_t)bs * 4);
-    PS_CK(cudaMemcpyAsync(ctx->tokens_dev, ctx->h_tokens, (size_t)bs * 4, cudaMemcpyHostToDevice, ctx->stream));
-    PS_CK(cudaMemcpyAsync(ctx->pos_dev, ctx->h_pos, (size_t)bs * 4, cudaMemcpyHostToDevice, ctx->stream));
-    ctx->h2d += (int64_t)bs * 8;
+    if ((rc = stage_call(ctx, bs))) return rc;
     PS_CK(cudaEventRecord(ctx->ev0, ctx->stream));
     ctx->logits_last = ctx->logits;
     if (ctx->arch) {
@@ -2574,22 +2632,7 @@ int ps_cuda_forward(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t *pos,
     if (rc) return rc;
     PS_CK(cudaEventRecord(ctx->ev1, ctx->stream));
     ctx->logits_rows = lm_head ? bs : 0;
-    if (lm_head && logits_host) {
-        const size_t bytes = (size_t)bs * ctx->d.vocab_size * 4;
-        if (bytes > ctx->h_logits_cap) {
-            if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
-            ctx->h_logits = nullptr;
-            ctx->h_logits_cap = 0;
-            PS_CK(cudaMallocHost(&ctx->h_logits, bytes));
-            ctx->h_logits_cap = bytes;
-        }
-        PS_CK(cudaMemcpyAsync(ctx->h_logits, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        if ((rc = sync_and_check(ctx))) return rc;
-        memcpy(logits_host, ctx->h_logits, bytes);
-        ctx->d2h += (int64_t)bytes;
-    } else {
-        if ((rc = sync_and_check(ctx))) return rc;
-    }
+    if ((rc = lm_head && logits_host ? logits_to_host(ctx, logits_host, (size_t)bs * ctx->d.vocab_size * 4) : sync_and_check(ctx))) return rc;
     { float ms = 0.f; PS_CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1)); ctx->last_ms = ms; }
     ctx->position = pos[0] + bs; // m_kv->advance(batch_size), llama_model.cpp:109
     kv_set_mask(ctx, 0, ctx->position, 0);
@@ -2604,29 +2647,21 @@ int ps_cuda_forward(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t *pos,
 // the weight stream is read once for the n columns (Q4_K: multi-column row-walker, tcgen05 GEMM from option tc_min up; other formats:
 // ps_k_matmul_ob or ps_k_matmul_qb), attention
 // runs per column over its own session's cache.  A session's logits are bit-identical to decoding it alone with batch 1.
-static int refresh_kv_tables(ps_cuda_ctx *ctx) {
-    const ps_cuda_model_desc &d = ctx->d;
-    if (ctx->arch) { // the executor takes the active set's pointers with every forward pass; the captured steps hold the old ones
-        PS_CK(cudaStreamSynchronize(ctx->stream));
-        if (ctx->g_step) { cudaGraphExecDestroy(ctx->g_step); ctx->g_step = nullptr; }
-        if (ctx->g_fwd) { cudaGraphExecDestroy(ctx->g_fwd); ctx->g_fwd = nullptr; }
-        return 0;
-    }
-    std::vector<float *> ptrs(2 * (size_t)d.n_layers);
-    for (int L = 0; L < d.n_layers; L++) { ptrs[L] = ctx->kc[L]; ptrs[d.n_layers + L] = ctx->vct[L]; }
-    PS_CK(cudaMemcpyAsync(ctx->kv_ptrs_dev, ptrs.data(), sizeof(float *) * ptrs.size(), cudaMemcpyHostToDevice, ctx->stream));
-    if (ctx->st_layers && ctx->bound && ctx->fused_ok) {
-        std::vector<PsStLayer> tab(d.n_layers);
-        for (int L = 0; L < d.n_layers; L++) {
-            const LayerDev &ld = ctx->layers[L];
-            tab[L] = PsStLayer{ld.rw_qkv, ld.rw_o, ld.rw_gu, ld.rw_down, ld.attn_norm, ld.ffn_norm, d.qkv_bias ? ld.q_bias : nullptr,
-                               d.qkv_bias ? ld.k_bias : nullptr, d.qkv_bias ? ld.v_bias : nullptr, ctx->kc[L], ctx->vct[L]};
-        }
-        PS_CK(cudaMemcpyAsync(ctx->st_layers, tab.data(), sizeof(PsStLayer) * (size_t)d.n_layers, cudaMemcpyHostToDevice, ctx->stream));
-    }
-    PS_CK(cudaStreamSynchronize(ctx->stream)); // the host vectors die here
-    if (ctx->g_step) { cudaGraphExecDestroy(ctx->g_step); ctx->g_step = nullptr; } // the captured steps hold the old cache pointers
+// The captured steps hold the old set's cache pointers (nothing else does that a switch has to renew: a set brings its pointer table, the
+// opt-in step kernel's table is renewed where it is launched, and a layer-list executor takes the pointers with every pass).  Two pageable copies and a
+// synchronisation a switch were 10 us: 0.6 ms where a server goes over 64 conversations
+static int drop_captured(ps_cuda_ctx *ctx) {
+    if (!ctx->g_step && !ctx->g_fwd) return 0;
+    PS_CK(cudaStreamSynchronize(ctx->stream));
+    if (ctx->g_step) { cudaGraphExecDestroy(ctx->g_step); ctx->g_step = nullptr; }
     if (ctx->g_fwd) { cudaGraphExecDestroy(ctx->g_fwd); ctx->g_fwd = nullptr; }
+    return 0;
+}
+static int kv_table(ps_cuda_ctx *ctx, float **dev, const std::vector<float *> &kc, const std::vector<float *> &vct) {
+    std::vector<float *> ptrs(kc);
+    ptrs.insert(ptrs.end(), vct.begin(), vct.end());
+    PS_CK(cudaMemcpyAsync(dev, ptrs.data(), sizeof(float *) * ptrs.size(), cudaMemcpyHostToDevice, ctx->stream));
+    PS_CK(cudaStreamSynchronize(ctx->stream)); // the host vector dies here
     return 0;
 }
 
@@ -2646,6 +2681,10 @@ int ps_cuda_session_create(ps_cuda_ctx *ctx, int *session_id) {
         PS_CK(cudaMemsetAsync(ks.kc[L], 0, kb, ctx->stream));
         PS_CK(cudaMemsetAsync(ks.vct[L], 0, vb, ctx->stream));
     }
+    if (!ctx->arch) {
+        int rc = dev_alloc(ctx, (void **)&ks.ptrs_dev, sizeof(float *) * 2 * (size_t)d.n_layers);
+        if (rc || (rc = kv_table(ctx, ks.ptrs_dev, ks.kc, ks.vct))) return rc;
+    }
     ks.slot_mask.assign((size_t)d.n_ctx, 1);
     const int id = ctx->next_session++;
     ctx->sessions.emplace(id, std::move(ks));
@@ -2660,12 +2699,14 @@ int ps_cuda_session_destroy(ps_cuda_ctx *ctx, int session_id) {
     if (it == ctx->sessions.end()) return fail(ctx, PS_CUDA_ERR_INVALID, "session_destroy: unknown session %d", session_id);
     PS_CK(cudaSetDevice(ctx->device));
     PS_CK(cudaStreamSynchronize(ctx->stream));
-    for (auto *vec : {&it->second.kc, &it->second.vct})
-        for (float *p : *vec) {
-            for (size_t i = 0; i < ctx->owned.size(); i++)
-                if (ctx->owned[i] == p) { ctx->owned.erase(ctx->owned.begin() + i); break; }
-            PS_CK(cudaFree(p));
-        }
+    std::vector<void *> all(it->second.kc.begin(), it->second.kc.end());
+    all.insert(all.end(), it->second.vct.begin(), it->second.vct.end());
+    if (it->second.ptrs_dev) all.push_back(it->second.ptrs_dev);
+    for (void *p : all) {
+        for (size_t i = 0; i < ctx->owned.size(); i++)
+            if (ctx->owned[i] == p) { ctx->owned.erase(ctx->owned.begin() + i); break; }
+        PS_CK(cudaFree(p));
+    }
     ctx->sessions.erase(it);
     return 0;
 }
@@ -2676,19 +2717,21 @@ int ps_cuda_session_select(ps_cuda_ctx *ctx, int session_id) {
     std::lock_guard<std::mutex> lock(ctx->mu);
     if (session_id == ctx->cur_session) return 0;
     auto it = ctx->sessions.find(session_id);
-    if (it == ctx->sessions.end() && session_id != 0) return fail(ctx, PS_CUDA_ERR_INVALID, "session_select: unknown session %d", session_id);
+    if (it == ctx->sessions.end()) return fail(ctx, PS_CUDA_ERR_INVALID, "session_select: unknown session %d", session_id);
     PS_CK(cudaSetDevice(ctx->device));
+    const int rc = drop_captured(ctx);
+    if (rc) return rc;
     // park the active state under its id, then load the requested one (session 0 = the context's own cache)
-    ps_cuda_ctx::KvSet cur;
-    cur.kc = ctx->kc; cur.vct = ctx->vct; cur.position = ctx->position; cur.slot_mask = ctx->slot_mask;
-    ps_cuda_ctx::KvSet next = std::move(ctx->sessions.at(session_id));
-    ctx->sessions.erase(session_id);
+    ps_cuda_ctx::KvSet cur{std::move(ctx->kc), std::move(ctx->vct), ctx->kv_ptrs_dev, ctx->position, std::move(ctx->slot_mask)};
+    ps_cuda_ctx::KvSet next = std::move(it->second);
+    ctx->sessions.erase(it);
     ctx->sessions.emplace(ctx->cur_session, std::move(cur));
-    ctx->kc = next.kc; ctx->vct = next.vct; ctx->position = next.position; ctx->slot_mask = next.slot_mask;
+    ctx->kc = std::move(next.kc); ctx->vct = std::move(next.vct); ctx->kv_ptrs_dev = next.ptrs_dev; ctx->position = next.position; ctx->slot_mask = std::move(next.slot_mask);
     ctx->slot_mask_dirty = true;
+    ctx->st_stale = true;
     ctx->last_batch = 0;
     ctx->cur_session = session_id;
-    return refresh_kv_tables(ctx);
+    return 0;
 }
 
 int ps_cuda_session_position(ps_cuda_ctx *ctx, int session_id) {
@@ -2736,10 +2779,9 @@ int ps_cuda_forward_sessions(ps_cuda_ctx *ctx, const int32_t *session_ids, const
             ctx->h_sess_ptrs[((size_t)L * 2 + 1) * d.max_batch + i] = (*vct)[L];
         }
     }
-    PS_CK(cudaMemcpyAsync(ctx->tokens_dev, ctx->h_tokens, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    PS_CK(cudaMemcpyAsync(ctx->pos_dev, ctx->h_pos, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
+    if (int rc_ = stage_call(ctx, n)) return rc_;
     PS_CK(cudaMemcpyAsync(ctx->sess_ptrs_dev, ctx->h_sess_ptrs, sizeof(float *) * 2 * (size_t)d.n_layers * (size_t)d.max_batch, cudaMemcpyHostToDevice, ctx->stream));
-    ctx->h2d += (int64_t)n * 8 + (int64_t)sizeof(float *) * 2 * d.n_layers * d.max_batch;
+    ctx->h2d += (int64_t)sizeof(float *) * 2 * d.n_layers * d.max_batch;
     PS_CK(cudaEventRecord(ctx->ev0, ctx->stream));
     SessRun sr{n_kv_max};
     int rc = forward_ops(ctx, n, lm_head, 0, -1, &sr);
@@ -2751,20 +2793,7 @@ int ps_cuda_forward_sessions(ps_cuda_ctx *ctx, const int32_t *session_ids, const
         PS_CK(cudaMemcpyAsync(ctx->h_ids, ctx->ids_dev, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     }
     PS_CK(cudaEventRecord(ctx->ev1, ctx->stream));
-    if (lm_head && logits_host) {
-        const size_t bytes = (size_t)n * d.vocab_size * 4;
-        if (bytes > ctx->h_logits_cap) {
-            if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
-            ctx->h_logits = nullptr;
-            ctx->h_logits_cap = 0;
-            PS_CK(cudaMallocHost(&ctx->h_logits, bytes));
-            ctx->h_logits_cap = bytes;
-        }
-        PS_CK(cudaMemcpyAsync(ctx->h_logits, ctx->logits, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        if ((rc = sync_and_check(ctx))) return rc;
-        memcpy(logits_host, ctx->h_logits, bytes);
-        ctx->d2h += (int64_t)bytes;
-    } else if ((rc = sync_and_check(ctx))) return rc;
+    if ((rc = lm_head && logits_host ? logits_to_host(ctx, logits_host, (size_t)n * d.vocab_size * 4) : sync_and_check(ctx))) return rc;
     if (lm_head && greedy_ids) { memcpy(greedy_ids, ctx->h_ids, (size_t)n * 4); ctx->d2h += (int64_t)n * 4; }
     { float ms = 0.f; PS_CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1)); ctx->last_ms = ms; }
     for (int i = 0; i < n; i++) { // m_kv->advance(1) of every session in the batch
@@ -2784,7 +2813,7 @@ int ps_cuda_forward_tree(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t 
     std::lock_guard<std::mutex> lock(ctx->mu);
     if (!ctx->bound) return fail(ctx, PS_CUDA_ERR_INVALID, "forward_tree: no model bound");
     if (ctx->tp > 1) return fail(ctx, PS_CUDA_ERR_UNSUPPORTED, "forward_tree: tree batches are single-GPU");
-    const int tb = std::min(ctx->d.max_batch, 32);
+    const int tb = std::min(ctx->d.max_batch, PS_TREE_MAX);
     if (bs <= 0 || bs > tb) return fail(ctx, PS_CUDA_ERR_INVALID, "forward_tree: batch %d outside [1,%d]", bs, tb);
     if (lm_head && !logits_host) return fail(ctx, PS_CUDA_ERR_INVALID, "forward_tree: lm_head requested without an output buffer");
     const int base = ctx->position;
@@ -2801,15 +2830,7 @@ int ps_cuda_forward_tree(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t 
     memcpy(ctx->h_pos, pos, (size_t)bs * 4);
     for (int i = 0; i < bs; i++)
         for (int j = 0; j < bs; j++) ctx->h_tree[i * bs + j] = tree_mask ? (tree_mask[i * bs + j] != 0) : (i >= j);
-    PS_CK(cudaMemcpyAsync(ctx->tokens_dev, ctx->h_tokens, (size_t)bs * 4, cudaMemcpyHostToDevice, ctx->stream));
-    PS_CK(cudaMemcpyAsync(ctx->pos_dev, ctx->h_pos, (size_t)bs * 4, cudaMemcpyHostToDevice, ctx->stream));
-    PS_CK(cudaMemcpyAsync(ctx->tree_dev, ctx->h_tree, (size_t)bs * bs, cudaMemcpyHostToDevice, ctx->stream));
-    ctx->h2d += (int64_t)bs * 8 + (int64_t)bs * bs;
-    if (ctx->slot_mask_dirty) { // pageable source, small: the synchronous copy keeps the host vector free to change afterwards
-        PS_CK(cudaMemcpy(ctx->slot_mask_dev, ctx->slot_mask.data(), (size_t)ctx->d.n_ctx, cudaMemcpyHostToDevice));
-        ctx->h2d += ctx->d.n_ctx;
-        ctx->slot_mask_dirty = false;
-    }
+    if (int rc_ = stage_call(ctx, bs, true)) return rc_;
     PS_CK(cudaEventRecord(ctx->ev0, ctx->stream));
     PS_DEP(ps_k_tree_mask, dim3((unsigned)std::min<int64_t>((base + bs + 255) / 256, 64), (unsigned)bs), 256, 0, ctx->tree_bias, ctx->slot_mask_dev, ctx->tree_dev, base, bs, base + bs);
     int rc = forward_ops(ctx, bs, lm_head, 0, base);
@@ -2822,20 +2843,7 @@ int ps_cuda_forward_tree(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t 
         if ((rc = sync_and_check(ctx))) return rc;
         memcpy(logits_host, ctx->h_ids, (size_t)bs * 4);
         ctx->d2h += (int64_t)bs * 4;
-    } else if (lm_head) {
-        const size_t bytes = (size_t)bs * ctx->d.vocab_size * 4;
-        if (bytes > ctx->h_logits_cap) {
-            if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
-            ctx->h_logits = nullptr;
-            ctx->h_logits_cap = 0;
-            PS_CK(cudaMallocHost(&ctx->h_logits, bytes));
-            ctx->h_logits_cap = bytes;
-        }
-        PS_CK(cudaMemcpyAsync(ctx->h_logits, ctx->logits, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-        if ((rc = sync_and_check(ctx))) return rc;
-        memcpy(logits_host, ctx->h_logits, bytes);
-        ctx->d2h += (int64_t)bytes;
-    } else if ((rc = sync_and_check(ctx))) return rc;
+    } else if ((rc = lm_head ? logits_to_host(ctx, logits_host, (size_t)bs * ctx->d.vocab_size * 4) : sync_and_check(ctx))) return rc;
     { float ms = 0.f; PS_CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1)); ctx->last_ms = ms; }
     ctx->last_batch = bs;
     kv_set_mask(ctx, base, base + bs, 0);   // advance_tokens(bs)
