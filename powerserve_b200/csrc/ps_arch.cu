@@ -125,7 +125,8 @@ struct PsArch {
     std::vector<float *> taps;
     uint8_t *t_head = nullptr, *tcx = nullptr; // lm_head operand blocks; activation blocks of the current product
     int max_k = 0;
-    int opt_tc = 1;     // bfloat16 batches (bs >= 2) run on the tcgen05 GEMM; 0 = the fp32-FMA tile kernels on rounded operands
+    int opt_tc = 1;     // batches (bs >= 2) run on the tcgen05 GEMMs; 0 = the fp32-FMA tile kernels (on rounded operands in bfloat16 mode)
+    bool tiled = false; // the operand blocks of those GEMMs are resident (float32 mode: if HBM has room and every weight is finite)
     int opt_simple = 0; // 1: every batch width takes the tiled kernels (the single-token kernels are skipped; tests compare the two)
     int n_sm = 148;
     // single-token step: the experts' gate | up product needs only the router logits, so it runs beside the attention kernels
@@ -646,11 +647,13 @@ int ps_arch_create(PsArch **out, const ps_cuda_arch_desc *desc, std::string &err
     AL(a->row_w, 4 * nrow);
     AL(a->row_token, 4 * nrow);
     AL(a->row_slot, 4 * nrow);
-    const size_t ntile = nrow / PA_TM + (size_t)std::max(a->max_e, 1) + 1;
+    const size_t ntile = nrow / 16 + (size_t)std::max(a->max_e, 1) + 1; // (16: the narrowest token tile of any kernel)
     if (a->round) {
         size_t blocks = (nrow / PT_N + (size_t)std::max(a->max_e, 1) + 1) * (size_t)((a->max_k + PT_KB - 1) / PT_KB);
         if (a->has_shift) blocks = std::max(blocks, (size_t)PT_MAX_SEG * ((size_t)B + PT_N - 1) / PT_N * (size_t)((dim + PT_KB - 1) / PT_KB) + PT_MAX_SEG * (size_t)((dim + PT_KB - 1) / PT_KB));
         AL(a->tcx, blocks * PT_BLOCK);
+    } else { // three parts of a token's k block, tiles of up to 64 tokens
+        AL(a->tcx, (nrow + (size_t)(std::max(a->max_e, 1) + 2) * 64) * (size_t)((a->max_k + PT_KB - 1) / PT_KB) * pt_xb<1>());
     }
     AL(a->tile_e, 4 * ntile);
     AL(a->tile_row0, 4 * ntile);
@@ -702,7 +705,13 @@ int ps_arch_create(PsArch **out, const ps_cuda_arch_desc *desc, std::string &err
         cudaFuncSetAttribute(pa_k_dec_token_input<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 176 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(pa_k_dec_token_input<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 176 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(pa_k_tc_gemm<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(pa_k_tc_gemm<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) != cudaSuccess) {
+        cudaFuncSetAttribute(pa_k_tc_gemm<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_tc_gemm3<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pt3<1, 16>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_tc_gemm3<1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pt3<1, 32>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_tc_gemm3<1, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pt3<1, 64>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_tc_gemm3<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pt3<2, 16>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_tc_gemm3<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pt3<2, 32>::SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_tc_gemm3<2, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Pt3<2, 64>::SMEM) != cudaSuccess) {
         cudaGetLastError();
         return bail(afail(err, PS_CUDA_ERR_CUDA, "cudaFuncSetAttribute(dynamic shared memory) failed"));
     }
@@ -1085,13 +1094,26 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
         if ((rc = aalloc(a, (void **)&a->ang_freq, 8 * n, err)) || (rc = upload_f32(a, &a->ang_ms, a->ang_ms_h, err)) || (rc = aalloc(a, (void **)&a->ang, 8 * n * (size_t)d.max_batch, err))) return rc;
         PA_CK(cudaMemcpy(a->ang_freq, a->ang_freq_h.data(), 8 * n, cudaMemcpyHostToDevice));
     }
-    if (a->round) {
-        // tensor-core operand blocks: every matrix once more in the layout the tcgen05 GEMM streams (ps_arch_tc.cuh)
+    // tensor-core operand blocks: every matrix once more in the layout the tcgen05 GEMMs stream (ps_arch_tc.cuh).  In float32 mode, whose FMA tiles can do without,
+    // a first trip counts the bytes
+    size_t need = 0;
+    int *odd = nullptr; // float32 mode: a weight that is not finite (its zero parts would turn an infinity into no number)
+    for (int trip = a->round ? 1 : 0; trip < 2; trip++) {
+        const bool count = trip == 0;
+        if (!a->round && trip == 1) {
+            size_t free_b = 0, total_b = 0;
+            PA_CK(cudaMemGetInfo(&free_b, &total_b));
+            if (need + ((size_t)8 << 30) > free_b) break;
+            if ((rc = aalloc(a, (void **)&odd, 4, err))) return rc;
+            PA_CK(cudaMemsetAsync(odd, 0, 4, stream));
+        }
         auto tile = [&](uint8_t **dst, const bf16 *src, int groups, int N, int K) -> int {
             const int n_rt = (N + PT_M - 1) / PT_M, nkb = (K + PT_KB - 1) / PT_KB;
+            need += (size_t)groups * n_rt * nkb * PT_BLOCK;
+            if (count) return 0;
             int r = aalloc(a, (void **)dst, (size_t)groups * n_rt * nkb * PT_BLOCK, err);
             if (r) return r;
-            pa_k_tc_tile_w<<<dim3((unsigned)nkb, (unsigned)n_rt, (unsigned)groups), 256, 0, stream>>>(*dst, src, N, K, n_rt, nkb);
+            pa_k_tc_tile_w<<<dim3((unsigned)nkb, (unsigned)n_rt, (unsigned)groups), 256, 0, stream>>>(*dst, src, N, K, n_rt, nkb, odd);
             PA_CK(cudaGetLastError());
             return 0;
         };
@@ -1106,12 +1128,13 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
                     return rc;
                 continue;
             }
-            if (w.seg.n > 0) { // every segment starts at a row tile of its own
+            if (w.seg.n > 0 && !a->round) { // (rows of several operand sets: the FMA tiles)
+            } else if (w.seg.n > 0) { // every segment starts at a row tile of its own
                 const int nkb = (d.dim + PT_KB - 1) / PT_KB;
                 if ((rc = aalloc(a, (void **)&w.t_qkv, (size_t)w.seg.rt[w.seg.n] * nkb * PT_BLOCK, err))) return rc;
                 for (int k = 0; k < w.seg.n; k++) {
                     const int n = w.seg.row[k + 1] - w.seg.row[k], n_rt = w.seg.rt[k + 1] - w.seg.rt[k];
-                    pa_k_tc_tile_w<<<dim3((unsigned)nkb, (unsigned)n_rt, 1), 256, 0, stream>>>(w.t_qkv + (size_t)w.seg.rt[k] * nkb * PT_BLOCK, w.wqkv + (size_t)w.seg.row[k] * d.dim, n, d.dim, n_rt, nkb);
+                    pa_k_tc_tile_w<<<dim3((unsigned)nkb, (unsigned)n_rt, 1), 256, 0, stream>>>(w.t_qkv + (size_t)w.seg.rt[k] * nkb * PT_BLOCK, w.wqkv + (size_t)w.seg.row[k] * d.dim, n, d.dim, n_rt, nkb, nullptr);
                     PA_CK(cudaGetLastError());
                 }
             } else if ((rc = tile(&w.t_qkv, w.wqkv, 1, w.pw, d.dim))) {
@@ -1130,7 +1153,11 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
                  (rc = tile(&w.t_down, w.wdown, w.d.n_experts, d.dim, w.d.expert_ff))))
                 return rc;
         }
+        if (count) continue;
         PA_CK(cudaStreamSynchronize(stream));
+        int any = 0;
+        if (odd) PA_CK(cudaMemcpy(&any, odd, 4, cudaMemcpyDeviceToHost));
+        a->tiled = !any;
     }
     for (int i = 0; i < d.n_layers; i++) { // repeated runs: the first run's weights under the run's own description
         PsArchLayer &w = a->L[(size_t)i];
@@ -1211,7 +1238,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         const int cap = a->opt_mv_cap > 0 ? a->opt_mv_cap : a->has_par && pdl && (int64_t)rows * K * 2 < ((int64_t)48 << 20) ? 2 : 4;
         return std::min(cdiv(rows, PA_DV_ROWS / ks), (unsigned)(cap * a->n_sm));
     };
-    const bool tc = ROUND && a->opt_tc && !single && !a->opt_simple;
+    const bool tc = a->tiled && a->opt_tc && !single && !a->opt_simple;
     // a dense product with few units: cut its token tiles until the grid fills the GPU.  Every cut reads the weights once more and shortens the
     // epilogue, so it pays for short sums and tiny grids (measured)
     auto cut_tiles = [&](PtArgs &g) {
@@ -1221,9 +1248,35 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         g.n_ct = (int)cdiv(g.M, PT_N / g.n_sub);
         return std::min(a->n_sm, g.n_ct * g.n_rt);
     };
+    // float32 mode (pa_k_tc_gemm3): activations in three parts, then the GEMM; g holds what is the product's own.  Tokens of a tile: the fewest (16, 32, 64) whose units
+    // fit the SMs together; of routed rows about what an expert gets
+    auto tc_split = [&](PtArgs &g, const float *X, int ldx, int K, int tn, bool routed, const int *row_token, const float *row_w) -> int {
+        g.nkb = (K + PT_KB - 1) / PT_KB; g.n_rt = (g.N + PT_M - 1) / PT_M; g.b = a->tcx; g.err = io.err_dev;
+        if (!routed) {
+            tn = 16;
+            while (tn < 64 && (int)cdiv(g.M, tn) * g.n_rt > a->n_sm) tn *= 2;
+            g.n_ct = (int)cdiv(g.M, tn);
+        }
+        pa_launch_dep(pdl, pa_k_tc_prep_split, dim3((unsigned)g.nkb, (unsigned)g.n_ct), dim3(256), 0, st, a->tcx, X, ldx, g.M, K, g.nkb, tn, routed ? a->n_tiles : nullptr,
+                      routed ? a->tile_row0 : nullptr, routed ? a->tile_end : nullptr, row_token, row_w);
+        PA_LAUNCH();
+        const dim3 grid((unsigned)std::min(a->n_sm, g.n_ct * g.n_rt));
+        auto go = [&](void (*kern)(PtArgs), int smem) { pa_launch_dep(pdl, kern, grid, dim3(PT_THREADS), smem, st, g); };
+        if (g.a1) tn == 16 ? go(pa_k_tc_gemm3<2, 16>, Pt3<2, 16>::SMEM) : tn == 32 ? go(pa_k_tc_gemm3<2, 32>, Pt3<2, 32>::SMEM) : go(pa_k_tc_gemm3<2, 64>, Pt3<2, 64>::SMEM);
+        else tn == 16 ? go(pa_k_tc_gemm3<1, 16>, Pt3<1, 16>::SMEM) : tn == 32 ? go(pa_k_tc_gemm3<1, 32>, Pt3<1, 32>::SMEM) : go(pa_k_tc_gemm3<1, 64>, Pt3<1, 64>::SMEM);
+        PA_LAUNCH();
+        return 0;
+    };
     // C[m][n] = sum_k X[m][k] W[n][k] + bias[n] on the tensor cores: round + tile the activations, then the GEMM
     auto tc_dense = [&](const float *X, int ldx, int M, int K, const uint8_t *wt, int N, const float *bias, float *C, int ldc, const PaAct *act1 = nullptr, int act_from = 0,
                         int gap = 0, const PaRowMul *mul = nullptr) -> int {
+        if (!ROUND) {
+            PtArgs g{};
+            g.a0 = wt; g.M = M; g.N = N; g.mode = PT_MODE_DENSE; g.C = C; g.ldc = ldc; g.bias = bias;
+            if (act1) { g.act = *act1; g.act1 = 1; g.act_from = act_from; g.gap = gap; }
+            if (mul) g.mul = *mul;
+            return tc_split(g, X, ldx, K, 0, false, nullptr, nullptr);
+        }
         const int nkb = (K + PT_KB - 1) / PT_KB, n_ct = (M + PT_N - 1) / PT_N, n_rt = (N + PT_M - 1) / PT_M;
         pa_launch_dep(pdl, pa_k_tc_prep_x, dim3((unsigned)nkb, (unsigned)n_ct), dim3(256), 0, st, a->tcx, X, ldx, M, K, nkb, nullptr, nullptr, nullptr, nullptr, nullptr);
         PA_LAUNCH();
@@ -1309,6 +1362,20 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
     auto routed_batch = [&](const float *X, const PsArchLayer &w) -> int {
         const ps_cuda_layer_desc &l = w.d;
         const int top = l.top_k, E = l.n_experts, ff = l.expert_ff, n = bs * top;
+        if (tc && !ROUND) {
+            const int tn = n >= 48 * E ? 64 : n >= 24 * E ? 32 : 16, max_tiles = n / tn + E + 1;
+            pa_launch_dep(pdl, pa_k_dispatch, dim3(1), dim3(256), 0, st, a->sel_e, a->sel_w, n, top, E, tn, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles);
+            PA_LAUNCH();
+            PtArgs g{};
+            g.n_ct = max_tiles; g.n_ct_dev = a->n_tiles; g.tile_e = a->tile_e; g.tile_row0 = a->tile_row0; g.tile_end = a->tile_end; g.M = n;
+            PtArgs g2 = g;
+            g.a0 = w.t_gate ? w.t_gate : w.t_up; g.a1 = w.t_gate ? w.t_up : nullptr; g.N = ff; g.mode = PT_MODE_EXPERT_UP; g.C = a->y; g.ldc = ff; g.act = pa_act_of(l);
+            int rc = tc_split(g, X, dim, dim, tn, true, a->row_token, l.route_on_input ? a->row_w : nullptr);
+            if (rc) return rc;
+            g2.a0 = w.t_down; g2.N = dim; g2.mode = PT_MODE_EXPERT_DOWN; g2.C = a->slot; g2.ldc = dim; g2.row_token = a->row_token; g2.row_slot = a->row_slot; g2.row_w = a->row_w; g2.top = top;
+            g2.on_input = l.route_on_input;
+            return tc_split(g2, a->y, ff, ff, tn, true, nullptr, nullptr);
+        }
         if (tc) {
             const int max_tiles = n / PT_N + E + 1, nkb1 = (dim + PT_KB - 1) / PT_KB, nkb2 = (ff + PT_KB - 1) / PT_KB;
             pa_launch_dep(pdl, pa_k_dispatch, dim3(1), dim3(256), 0, st, a->sel_e, a->sel_w, n, top, E, PT_N, a->row_token, a->row_slot, a->row_w, a->tile_e, a->tile_row0, a->tile_end, a->n_tiles);
@@ -1370,6 +1437,12 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                 if ((rc_up = dense_up(X, nullptr, wu, ff, act))) return rc_up;
             }
             return linear(a->y, ff, ff, wd, td, dim, out, dim);
+        }
+        if (tc && !ROUND) {
+            PtArgs g{};
+            g.a0 = tg; g.a1 = tu; g.M = bs; g.N = ff; g.mode = PT_MODE_EXPERT_UP; g.C = a->y; g.ldc = ff; g.act = act;
+            int rc = tc_split(g, X, dim, dim, 0, false, nullptr, nullptr);
+            return rc ? rc : linear(a->y, ff, ff, wd, td, dim, out, dim);
         }
         if (tc) {
             const int nkb = (dim + PT_KB - 1) / PT_KB, n_ct = (bs + PT_N - 1) / PT_N;
@@ -1601,7 +1674,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         } else if (rwkv) {
             float *ring = io.kc[li] + w.ring_off;
             if ((rc = seam(a->h, w.norm))) return rc;
-            if (tc) { // one GEMM over six operand sets
+            if (tc && ROUND) { // one GEMM over six operand sets
                 const int nkb = (dim + PT_KB - 1) / PT_KB, n_ct = (bs + PT_N - 1) / PT_N;
                 PtArgs g{};
                 g.seg = w.seg;

@@ -22,7 +22,8 @@
 
 // ---------------------------------------------------------------------------------------------------- operand builders
 // weights [groups][N][K] bf16 row-major -> blocks [group][row tile][k block][k-chunk 8][row 128][8]; zero outside N x K
-__global__ void __launch_bounds__(256) pa_k_tc_tile_w(uint8_t *__restrict__ dst, const bf16 *__restrict__ w, int N, int K, int n_rt, int nkb) {
+// odd (or null): set if a weight is an infinity or no number
+__global__ void __launch_bounds__(256) pa_k_tc_tile_w(uint8_t *__restrict__ dst, const bf16 *__restrict__ w, int N, int K, int n_rt, int nkb, int *__restrict__ odd) {
     const int kb = blockIdx.x, rt = blockIdx.y, grp = blockIdx.z;
     const bf16 *src = w + (int64_t)grp * N * K;
     uint8_t *out = dst + (((int64_t)grp * n_rt + rt) * nkb + kb) * PT_BLOCK;
@@ -31,6 +32,12 @@ __global__ void __launch_bounds__(256) pa_k_tc_tile_w(uint8_t *__restrict__ dst,
         uint16_t v[8];
 #pragma unroll
         for (int t = 0; t < 8; t++) v[t] = (n < N && k0 + t < K) ? reinterpret_cast<const uint16_t *>(src)[(int64_t)n * K + k0 + t] : (uint16_t)0;
+        if (odd) {
+            bool any = false;
+#pragma unroll
+            for (int t = 0; t < 8; t++) any |= (v[t] & 0x7F80) == 0x7F80;
+            if (any) *odd = 1;
+        }
         uint4 pk;
         pk.x = v[0] | ((uint32_t)v[1] << 16); pk.y = v[2] | ((uint32_t)v[3] << 16); pk.z = v[4] | ((uint32_t)v[5] << 16); pk.w = v[6] | ((uint32_t)v[7] << 16);
         *reinterpret_cast<uint4 *>(out + kc * 2048 + row * 16) = pk;
@@ -299,5 +306,239 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
     if (warp == 5) {
         ps_tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------- float32 mode
+// The same products without rounding.  The weights are bfloat16 as they are; an activation is cut into three bfloat16 parts, its upper, middle and lower
+// eight significant bits (exact, and no part overflows), so that three MMAs whose products are exact replace the FMAs.  What an MMA loses is the low
+// end of the fp32 accumulator (it truncates where an FMA rounds), and that grows with the number of MMAs an accumulator sees and with its size.  So an accumulator takes ONE
+// k block of 64 - lowest parts first, while it is small, the four MMAs of the upper parts last - and the epilogue adds the blocks' sums in fp32 with
+// rounding.  The order of k is the same for every number of tokens and every portion.
+// Error against 64 bits: logits of two 1024-wide Vanapel layers 8e-7 with FMA tiles, 5.8e-7 so (150 tokens at 300).
+// Bound by the epilogue, which drains an accumulator of TN tokens every 12 MMAs (24 with a gate), and by the copies: a stage of 64 k is 16 KB of weights a
+// matrix and 384 B a token.  A unit is 128 output rows x TN tokens, TN as small as fills the GPU: its epilogue is shorter and the weights come from L2.
+// MEASURED
+#define PT_SPLIT 3
+template <int TN> PS_HD constexpr int pt_xb() { return PT_SPLIT * TN * PT_KB * 2; } // bytes of a tile's k block: [part][k-chunk of 8][token TN][8]
+// activations -> [column tile][k block][part][k-chunk][token][8]; tiles as in pa_k_tc_prep_x
+__global__ void __launch_bounds__(256) pa_k_tc_prep_split(uint8_t *__restrict__ dst, const float *__restrict__ x, int ldx, int M, int K, int nkb, int TN, const int *__restrict__ n_tiles,
+                                                          const int *__restrict__ tile_row0, const int *__restrict__ tile_end, const int *__restrict__ row_token, const float *__restrict__ row_w) {
+    ps_grid_dep();
+    const int kb = blockIdx.x, t = blockIdx.y;
+    if (n_tiles && t >= *n_tiles) return;
+    const int r0 = tile_row0 ? tile_row0[t] : t * TN, rend = tile_end ? tile_end[t] : M;
+    uint8_t *out = dst + ((int64_t)t * nkb + kb) * (PT_SPLIT * TN * PT_KB * 2);
+    for (int c = threadIdx.x; c < TN * 8; c += 256) {
+        const int kc = c & 7, row = c >> 3, r = r0 + row, k0 = kb * PT_KB + kc * 8;
+        const bool in = r < rend;
+        const float *src = x + (int64_t)(in && row_token ? row_token[r] : in ? r : 0) * ldx;
+        const float sc = in && row_w ? row_w[r] : 1.0f;
+        uint32_t part[PT_SPLIT][4] = {};
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            float v = in && k0 + e < K ? src[k0 + e] * sc : 0.f;
+            const bool odd = !(fabsf(v) < INFINITY);
+            if (v != v) v = __uint_as_float(0x7FC00000u); // (a NaN's low bits alone would read as an infinity)
+#pragma unroll
+            for (int q = 0; q < PT_SPLIT; q++) {
+                const uint32_t hi = __float_as_uint(v) & 0xFFFF0000u;
+                part[q][e >> 1] |= (e & 1) ? hi : hi >> 16;
+                v = odd ? 0.f : v - __uint_as_float(hi);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < PT_SPLIT; q++) *reinterpret_cast<uint4 *>(out + (q * 8 + kc) * (TN * 16) + row * 16) = make_uint4(part[q][0], part[q][1], part[q][2], part[q][3]);
+    }
+}
+
+// a tile's sums wait in shared memory for a store loop of one copy: unrolled over its registers, with the modes' and activations' branches in every copy, a tile of 64
+// tokens took longer to store than to multiply (instructions that are fetched once)
+template <int NA, int TN> struct Pt3 {
+    static constexpr int STAGE = NA * PT_BLOCK + pt_xb<TN>(), RED = NA * TN * PT_M * 4, FIT = (224 * 1024 - RED) / STAGE, STAGES = FIT < 8 ? FIT : 8, SMEM = STAGES * STAGE + RED + 1024;
+};
+template <int NA, int TN>
+__global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm3(const __grid_constant__ PtArgs a) {
+    constexpr int XB = pt_xb<TN>(), STAGE = Pt3<NA, TN>::STAGE, STAGES = Pt3<NA, TN>::STAGES;
+    constexpr int TM = 2 * NA * TN < 32 ? 32 : 2 * NA * TN; // tensor-memory columns: two accumulator buffers
+    extern __shared__ __align__(1024) uint8_t pt_smem_raw[];
+    __shared__ __align__(8) uint64_t bar_full[STAGES], bar_empty[STAGES], bar_tmem_full[2], bar_tmem_empty[2], bar_done;
+    __shared__ uint32_t tmem_base_smem;
+    uint8_t *smem = reinterpret_cast<uint8_t *>(((uintptr_t)pt_smem_raw + 1023) & ~(uintptr_t)1023);
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int nkb = a.nkb;
+    if (tid == 0) {
+        for (int s = 0; s < STAGES; s++) { ps_mbar_init(&bar_full[s], 1); ps_mbar_init(&bar_empty[s], 1); }
+        for (int b = 0; b < 2; b++) { ps_mbar_init(&bar_tmem_full[b], 1); ps_mbar_init(&bar_tmem_empty[b], 4); }
+        ps_mbar_init(&bar_done, 1);
+        ps_fence_barrier_init();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 5) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ps_smem_u32(&tmem_base_smem)), "n"(TM) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    ps_tc_fence_before();
+    __syncthreads();
+    ps_tc_fence_after();
+    const uint32_t tmem_base = tmem_base_smem;
+    int ahead = 0; // (as in pa_k_tc_gemm)
+    if (warp == 4 && !a.n_ct_dev && !a.tile_e && (int)blockIdx.x < a.n_ct * a.n_rt) {
+        ahead = min(STAGES, nkb);
+        if (ps_elect_one()) {
+            const int64_t b0 = (int64_t)((int)blockIdx.x % a.n_rt) * nkb * PT_BLOCK;
+            for (int kb = 0; kb < ahead; kb++) {
+                ps_mbar_expect_tx(&bar_full[kb], STAGE);
+                ps_bulk_g2s(smem + (size_t)kb * STAGE, a.a0 + b0 + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[kb]);
+                if (NA == 2) ps_bulk_g2s(smem + (size_t)kb * STAGE + PT_BLOCK, a.a1 + b0 + (int64_t)kb * PT_BLOCK, PT_BLOCK, &bar_full[kb]);
+            }
+        }
+        __syncwarp();
+    }
+    ps_grid_dep();
+    const int n_ct = a.n_ct_dev ? min(*a.n_ct_dev, a.n_ct) : a.n_ct, n_units = n_ct * a.n_rt;
+
+    if (warp == 4) {
+        PsRing<STAGES> st;
+        int g = 0;
+        bool ok = true;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const int ct = u / a.n_rt, rt = u % a.n_rt;
+            const int64_t grp = a.tile_e ? a.tile_e[ct] : 0;
+            const uint8_t *pa0 = a.a0 + ((grp * a.n_rt + rt) * nkb) * (int64_t)PT_BLOCK, *pa1 = NA == 2 ? a.a1 + ((grp * a.n_rt + rt) * nkb) * (int64_t)PT_BLOCK : nullptr;
+            const uint8_t *pb = a.b + (int64_t)ct * nkb * XB;
+            for (int kb = 0; kb < nkb; kb++, g++, st.step()) {
+                if (g >= STAGES && !ps_tc_wait_warp(&bar_empty[st.i], st.round ^ 1)) { *a.err = 1; ok = false; break; }
+                uint8_t *sm = smem + (size_t)st.i * STAGE;
+                uint64_t *bar = &bar_full[st.i];
+                if (ps_elect_one()) {
+                    if (g >= ahead) {
+                        ps_mbar_expect_tx(bar, STAGE);
+                        ps_bulk_g2s(sm, pa0 + (int64_t)kb * PT_BLOCK, PT_BLOCK, bar);
+                        if (NA == 2) ps_bulk_g2s(sm + PT_BLOCK, pa1 + (int64_t)kb * PT_BLOCK, PT_BLOCK, bar);
+                    }
+                    ps_bulk_g2s(sm + NA * PT_BLOCK, pb + (int64_t)kb * XB, XB, bar);
+                }
+                __syncwarp();
+            }
+        }
+        for (int k = g > STAGES ? g - STAGES : 0; k < g; k++) // copies in flight end before the CTA does (they have, unless a wait gave up)
+            if (!ps_tc_wait(&bar_full[k % STAGES], (k / STAGES) & 1)) { *a.err = 5; break; }
+    } else if (warp == 5) {
+        constexpr uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(PT_M >> 4) << 24);
+        const uint64_t desc_a = ps_tc_smem_desc(ps_smem_u32(smem), 2048, 128), desc_b = ps_tc_smem_desc(ps_smem_u32(smem + NA * PT_BLOCK), TN * 16, 128);
+        PsRing<STAGES> st;
+        bool ok = true;
+        int m = 0;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x)
+            for (int kb = 0; kb < nkb; kb++, m++, st.step()) {
+                const int tb = m & 1;
+                if (!ps_tc_wait_warp(&bar_full[st.i], st.round)) { *a.err = 2; ok = false; break; }
+                if (m >= 2 && !ps_tc_wait_warp(&bar_tmem_empty[tb], ((m >> 1) - 1) & 1)) { *a.err = 3; ok = false; break; }
+                ps_tc_fence_after();
+                const uint64_t da = desc_a + (uint64_t)(st.i * (STAGE >> 4)), db = desc_b + (uint64_t)(st.i * (STAGE >> 4));
+                const uint32_t td = tmem_base + tb * (NA * TN);
+                if (ps_elect_one()) {
+#pragma unroll
+                    for (int q = PT_SPLIT - 1; q >= 0; q--) // lowest parts first
+#pragma unroll
+                        for (int j = 0; j < PT_KB / 16; j++) {
+                            const uint64_t dq = db + (q * 8 + 2 * j) * TN;
+                            ps_tc_mma_f16(td, da + j * 256, dq, idesc, q != PT_SPLIT - 1 || j != 0);
+                            if (NA == 2) ps_tc_mma_f16(td + TN, da + (PT_BLOCK >> 4) + j * 256, dq, idesc, q != PT_SPLIT - 1 || j != 0);
+                        }
+                    ps_tc_commit(&bar_empty[st.i]);
+                    ps_tc_commit(&bar_tmem_full[tb]);
+                }
+                __syncwarp();
+            }
+        if (ps_elect_one()) ps_tc_commit(&bar_done); // MMAs in flight end before the tensor memory is given back
+        __syncwarp();
+        if (!ps_tc_wait(&bar_done, 0)) *a.err = 6;
+    } else {
+        bool ok = true;
+        int m = 0;
+        for (int u = blockIdx.x; u < n_units && ok; u += gridDim.x) {
+            const int ct = u / a.n_rt, rt = u % a.n_rt;
+            float acc[NA][TN];
+#pragma unroll
+            for (int c = 0; c < TN; c++) acc[0][c] = acc[NA - 1][c] = 0.f;
+            for (int kb = 0; kb < nkb; kb++, m++) {
+                const int tb = m & 1;
+                if (!ps_tc_wait_warp(&bar_tmem_full[tb], (m >> 1) & 1)) { *a.err = 4; ok = false; break; }
+                ps_tc_fence_after();
+                const uint32_t t_lane = tmem_base + ((uint32_t)(32 * warp) << 16) + tb * (NA * TN);
+#pragma unroll
+                for (int z = 0; z < NA; z++)
+#pragma unroll
+                    for (int c0 = 0; c0 < TN; c0 += 16) {
+                        uint32_t v[16];
+                        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                                     : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+                                       "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+                                     : "r"(t_lane + z * TN + c0)
+                                     : "memory");
+                        ps_tc_ld_wait();
+#pragma unroll
+                        for (int c = 0; c < 16; c++) {
+                            asm volatile("" : "+r"(v[c])); // (nothing reads it before the wait)
+                            acc[z][c0 + c] += __uint_as_float(v[c]);
+                        }
+                    }
+                ps_tc_fence_before();
+                __syncwarp();
+                if (lane == 0) ps_mbar_arrive(&bar_tmem_empty[tb]);
+            }
+            if (!ok) break;
+            const int n = rt * PT_M + 32 * warp + lane, r0 = a.tile_row0 ? a.tile_row0[ct] : ct * TN, rend = a.tile_end ? a.tile_end[ct] : a.M;
+            const float bias = a.bias && n < a.N ? a.bias[n] : 0.f;
+            float *red = reinterpret_cast<float *>(smem + STAGES * STAGE) + 32 * warp + lane; // (a thread's own)
+#pragma unroll
+            for (int c = 0; c < TN; c++) {
+                red[c * PT_M] = acc[0][c];
+                if (NA == 2) red[(TN + c) * PT_M] = acc[1][c];
+            }
+            const int n_cols = min(TN, rend - r0); // warp-uniform
+            if (a.mode == PT_MODE_EXPERT_DOWN) {
+                int64_t to[(TN + 31) / 32]; // lane: rows lane and lane + 32 of the tile
+                float rw[(TN + 31) / 32];
+#pragma unroll
+                for (int h = 0; h < (TN + 31) / 32; h++) {
+                    const int r = min(r0 + 32 * h + lane, rend - 1);
+                    to[h] = ((int64_t)a.row_token[r] * a.top + a.row_slot[r]) * a.ldc;
+                    rw[h] = a.on_input ? 1.f : a.row_w[r];
+                }
+                for (int c = 0; c < n_cols; c++) {
+                    const int64_t o = __shfl_sync(0xffffffffu, TN > 32 && c >= 32 ? to[(TN - 1) / 32] : to[0], c & 31);
+                    const float rwc = __shfl_sync(0xffffffffu, TN > 32 && c >= 32 ? rw[(TN - 1) / 32] : rw[0], c & 31);
+                    if (n < a.N) a.C[o + n] = red[c * PT_M] * rwc;
+                }
+            } else if (n < a.N) {
+                const bool act1 = a.mode == PT_MODE_EXPERT_UP || (a.act1 && n >= a.act_from);
+                float *to = a.C + (int64_t)r0 * a.ldc + (a.mode == PT_MODE_DENSE && act1 ? n + a.gap : n);
+                if (NA == 2) {
+                    for (int c = 0; c < n_cols; c++) to[(int64_t)c * a.ldc] = pa_expert_act(red[c * PT_M], red[(TN + c) * PT_M], a.act);
+                } else if (act1) {
+                    for (int c = 0; c < n_cols; c++) {
+                        float v = pa_act1(red[c * PT_M] + bias, a.act);
+                        if (a.mul.table) v *= pa_ld(a.mul.table + (int64_t)a.mul.tok[r0 + c] * a.mul.ld + n);
+                        to[(int64_t)c * a.ldc] = v;
+                    }
+                } else {
+                    for (int c = 0; c < n_cols; c++) {
+                        float v = red[c * PT_M] + bias;
+                        if (a.mul.table) v *= pa_ld(a.mul.table + (int64_t)a.mul.tok[r0 + c] * a.mul.ld + n);
+                        to[(int64_t)c * a.ldc] = v;
+                    }
+                }
+            }
+            __syncwarp();
+        }
+    }
+    ps_tc_fence_before();
+    __syncthreads();
+    if (warp == 5) {
+        ps_tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "n"(TM) : "memory");
     }
 }
