@@ -18,7 +18,7 @@
 #define PT_BLOCK (128 * PT_KB * 2) // bytes of one operand block (either side)
 #define PT_THREADS 192
 #define PT_MAX_SEG 6 // operand sets of one product
-#define PT_SMEM (192 * 1024 + 1024)
+#define PT_SMEM (192 * 1024 + 1024 + 2 * 16 * PT_M * 4) // stages, alignment, sixteen columns' sums and table entries
 
 // ---------------------------------------------------------------------------------------------------- operand builders
 // weights [groups][N][K] bf16 row-major -> blocks [group][row tile][k block][k-chunk 8][row 128][8]; zero outside N x K
@@ -134,7 +134,7 @@ struct PtArgs {
 };
 
 template <int NA>
-__global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
+__global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const __grid_constant__ PtArgs a) {
     constexpr int STAGES = NA == 1 ? 6 : 4;
     constexpr int STAGE_BYTES = (NA + 1) * PT_BLOCK;
     extern __shared__ __align__(1024) uint8_t pt_smem_raw[];
@@ -277,23 +277,54 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const PtArgs a) {
                     for (int c = 0; c < 16; c++) mulv[c] = pa_ld(a.mul.table + (int64_t)a.mul.tok[min(r0 + c0 + c, rend - 1)] * a.mul.ld + min(n, n_end - 1));
                 }
                 ps_tc_ld_wait();
-                if (n < n_end) {
+                // the branches of mode and activation lie outside the sixteen copies: a unit's stores are met once, instructions that have to be fetched (with them
+                // inside, a product of 32 units took 22 us, 15 so; 256 tokens of Nufusun at 768 350 and 328)
+                const int left = n_cols - c0;
+                float *to = a.C + (int64_t)(r0 + c0) * a.ldc + n;
+                auto each = [&](auto f) {
+#pragma unroll
+                    for (int c = 0; c < 16; c++)
+                        if (c < left && n < n_end) to[(int64_t)c * a.ldc] = f(c);
+                };
+                auto sum = [&](int c) { return __uint_as_float(v[c]); };
+                if (a.mode == PT_MODE_EXPERT_DOWN) {
+                    const int r = min(r0 + c0 + (lane & 15), rend - 1);
+                    const int64_t mine = ((int64_t)a.row_token[r] * a.top + a.row_slot[r]) * a.ldc;
+                    const float rw = a.on_input ? 1.f : a.row_w[r];
 #pragma unroll
                     for (int c = 0; c < 16; c++) {
-                        const int r = r0 + c0 + c;
-                        if (r >= rend) break;
-                        const float acc = __uint_as_float(v[c]);
-                        if (a.mode == PT_MODE_DENSE) {
-                            const bool act1 = a.act1 && n >= a.act_from;
-                            float val = act1 ? pa_act1(acc + bias, a.act) : acc + bias;
-                            if (NA == 1 && a.mul.table) val *= mulv[c];
-                            a.C[(int64_t)r * a.ldc + (act1 ? n + a.gap : n)] = val;
-                        } else if (a.mode == PT_MODE_EXPERT_UP) {
-                            a.C[(int64_t)r * a.ldc + n] = NA == 2 ? pa_expert_act(acc, __uint_as_float(w2[c]), a.act) : pa_act1(acc, a.act);
-                        } else {
-                            a.C[((int64_t)a.row_token[r] * a.top + a.row_slot[r]) * a.ldc + n] = a.on_input ? acc : acc * a.row_w[r];
-                        }
+                        const int64_t o = __shfl_sync(0xffffffffu, mine, c);
+                        const float f = __shfl_sync(0xffffffffu, rw, c);
+                        if (c < left && n < n_end) a.C[o + n] = sum(c) * f;
                     }
+                } else if (NA == 2) {
+                    PaAct act = a.act;
+                    auto gated = [&](int kind) {
+                        act.kind = kind;
+                        each([&](int c) { return pa_expert_act(sum(c), __uint_as_float(w2[c]), act); });
+                    };
+                    if (act.kind == PS_ACT_RELU) gated(PS_ACT_RELU);
+                    else if (act.kind == PS_ACT_GELU_TANH) gated(PS_ACT_GELU_TANH);
+                    else gated(PS_ACT_SWISH);
+                } else if (a.mode == PT_MODE_DENSE && !a.mul.table && !(a.act1 && n - lane + 31 >= a.act_from)) {
+                    each([&](int c) { return sum(c) + bias; });
+                } else { // one-argument activations, table rows: one copy, the sums by way of shared memory
+                    float *red = reinterpret_cast<float *>(smem + STAGES * STAGE_BYTES) + 32 * warp + lane;
+#pragma unroll
+                    for (int c = 0; c < 16; c++) {
+                        red[c * PT_M] = sum(c);
+                        if (NA == 1 && a.mul.table) red[(16 + c) * PT_M] = mulv[c];
+                    }
+                    const bool act1 = a.mode == PT_MODE_EXPERT_UP || (a.act1 && n >= a.act_from);
+                    if (a.mode == PT_MODE_DENSE && act1) to += a.gap;
+                    if (n < n_end)
+#pragma unroll 2
+                        for (int c = 0; c < min(left, 16); c++) {
+                            float val = a.mode == PT_MODE_DENSE ? red[c * PT_M] + bias : red[c * PT_M];
+                            if (act1) val = pa_act1(val, a.act);
+                            if (NA == 1 && a.mul.table) val *= red[(16 + c) * PT_M];
+                            to[(int64_t)c * a.ldc] = val;
+                        }
                 }
             }
             ps_tc_fence_before();
