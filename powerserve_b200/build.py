@@ -15,7 +15,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libps_cuda.so")
 SOURCES = ["ps_cuda.cu", "ps_arch.cu"]
-HEADERS = ["ps_step.cuh", "ps_tc.cuh", "ps_rw.cuh", "ps_decode.cuh", "ps_kernels.cuh", "ps_math.cuh", "ps_mv32.cuh", "ps_ptx.cuh", "ps_arch.h", "ps_arch_kernels.cuh",
+HEADERS = ["ps_step.cuh", "ps_tc.cuh", "ps_mk.cuh", "ps_rw.cuh", "ps_decode.cuh", "ps_kernels.cuh", "ps_math.cuh", "ps_mv32.cuh", "ps_ptx.cuh", "ps_arch.h", "ps_arch_kernels.cuh",
            "ps_arch_decode.cuh", "ps_arch_tc.cuh", "ps_arch_recur.cuh",
            os.path.join("..", "..", "include", "ps_cuda.h")]
 

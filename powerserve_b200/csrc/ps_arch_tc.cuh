@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const __grid_const
                 }
                 ps_tc_ld_wait();
                 // the branches of mode and activation lie outside the sixteen copies: a unit's stores are met once, instructions that have to be fetched (with them
-                // inside, a product of 32 units took 22 us, 15 so; 256 tokens of Nufusun at 768 350 and 328)
+                // inside, a product of 32 units took 22 us, 15 so; 256 tokens of Nufusun at 768 350 and 320)
                 const int left = n_cols - c0;
                 float *to = a.C + (int64_t)(r0 + c0) * a.ldc + n;
                 auto each = [&](auto f) {

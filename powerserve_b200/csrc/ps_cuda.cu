@@ -5,6 +5,7 @@
 #include "ps_rw.cuh"
 #include "ps_mv32.cuh"
 #include "ps_tc.cuh"
+#include "ps_mk.cuh"
 #include "ps_step.cuh"
 #include "ps_arch.h"
 
@@ -118,13 +119,14 @@ struct ps_cuda_ctx {
     int logits_rows = 0;                // rows of that buffer
     unsigned long long *topk_cand = nullptr; // device top-k scratch: keys of the slices' best, then the result: ids [k], values [k]
     uint32_t *aqs = nullptr, *absp = nullptr;
+    uint8_t *mk_x = nullptr; // activation records of a batch (ps_k_matmul_mk)
     float *ad = nullptr;
     int32_t *tokens_dev = nullptr, *pos_dev = nullptr, *ids_dev = nullptr;
     int32_t *h_tokens = nullptr, *h_pos = nullptr, *h_ids = nullptr; // pinned staging
     float *h_logits = nullptr;                                          // pinned staging for logits
     size_t h_logits_cap = 0;
     // options / counters
-    int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_mt_min = 2, opt_scores_batch_min = 2, opt_give_up = -1;
+    int opt_graph = 1, opt_fused = 1, opt_pdl = 1, opt_ktime = 0, opt_tc = 1, opt_kb = 0, opt_cta_trace = 1, opt_attn_fused = 0, opt_unroll2 = 1, opt_ksplit = 0, opt_defer = 0, opt_rwm_tile = 1, opt_pv_batch_min = 3, opt_mv_kpar = 1, opt_attn_tile = 1, opt_tc_min = 6, opt_mt_min = 2, opt_mk_min = 2, opt_scores_batch_min = 2, opt_give_up = -1;
     bool tc_ok = false;        // tensor-core prefill operands are resident
     uint8_t *tc_b = nullptr;   // B operand blocks of the current activation batch
     float *tc_part = nullptr;  // numbers of the tiles that CTAs share: a slot per CTA, for tiles of up to tc_nt columns
@@ -454,6 +456,33 @@ int matmul_qb(ps_cuda_ctx *ctx, int wtype, int64_t K, int64_t bs, const PsMbSeg 
     }
 }
 
+// The 256-element formats on the tensor cores (ps_k_matmul_mk): column tiles of eight a CTA takes, 0 where ps_k_matmul_qb is the faster one.  A tile's weights are
+// unpacked once whatever its columns, so wide tiles cost little more than narrow ones, but their CTAs are fewer (K x N on columns, us with one / two / four:
+// Q4_K 4096 x 1024 on 32 14.1 / 13.3 / 18, on 128 31 / 21.3 / 20.9; 4096 x 4096 on 16 18.9 / 15.3 / 20.9, on 32 33 / 21.2 / 21, on 128 100 / 64 / 50; Q6_K 45 / 31 / 24 and 160 / 99 / 62).
+// qb: 20, 36, 23, 37, 109; Q6_K 44 and 120.  With two to four columns the two are alike; qb is ahead on large matrices (8192 x 8192 on two: Q4_K 32 and 35 us, Q6_K 43
+// and 52; 4096 x 4096 on two: Q4_K 15.8 and 14.2, Q5_K 15 and 17, Q6_K 17 and 18.7; 4096 x 1024: 15 and 12.6, 14.7 and 14.2, 16.6 and 15.4)
+int mk_tiles(const ps_cuda_ctx *ctx, int wtype, int64_t K, int64_t rows, int bs) {
+    if (!ctx->mk_x || bs < ctx->opt_mk_min || (wtype != 12 && wtype != 13 && wtype != 14)) return 0;
+    if (bs <= 4 && rows * K > (wtype == 12 ? (int64_t)32 << 20 : (int64_t)8 << 20)) return 0;
+    const int64_t n_ct = (bs + 7) / 8, units = (rows + 15) / 16 * n_ct;
+    return n_ct >= 3 && units >= 1024 ? 4 : n_ct >= 2 && units >= 256 ? 2 : 1;
+}
+template <int TYPE, int NT> int launch_mk(ps_cuda_ctx *ctx, PsMkArgs a, int row_tiles) {
+    static bool attr_set[64] = {};
+    constexpr int STAGE = ps_mk_stage<TYPE, NT>(), RED = 8 * 8 * NT * 16 * 4;
+    if (!attr_set[ctx->device]) {
+        PS_CK(cudaFuncSetAttribute(ps_k_matmul_mk<TYPE, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        attr_set[ctx->device] = true;
+    }
+    const int cols = ((a.bs + 7) / 8 + NT - 1) / NT, per_sm = std::min(4, (row_tiles * cols + ctx->n_sm - 1) / ctx->n_sm);
+    a.ns = std::max(2, std::min(std::min(a.nb + 1, 5), 216 * 1024 / per_sm / STAGE));
+    PS_DEP((ps_k_matmul_mk<TYPE, NT>), dim3((unsigned)row_tiles, (unsigned)cols), 128, (size_t)std::max(a.ns * STAGE, RED), a);
+    return 0;
+}
+template <int TYPE> int launch_mk_t(ps_cuda_ctx *ctx, const PsMkArgs &a, int row_tiles, int nt) {
+    return nt == 4 ? launch_mk<TYPE, 4>(ctx, a, row_tiles) : nt == 2 ? launch_mk<TYPE, 2>(ctx, a, row_tiles) : launch_mk<TYPE, 1>(ctx, a, row_tiles);
+}
+
 // quantise bs activation columns of K elements into the context's scratch (type of the WEIGHT decides the format)
 dim3 embed_grid(int64_t tokens, int64_t dim) { return dim3((unsigned)tokens, (unsigned)((dim + 1023) / 1024)); } // four elements a thread
 
@@ -605,6 +634,37 @@ int mt_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t rows, int6
     if (ctx->mv_type == 2) ps_k_mt_pack<2><<<grid, 128, 0, ctx->stream>>>(dst, w, rows, K / 32);
     else ps_k_mt_pack<8><<<grid, 128, 0, ctx->stream>>>(dst, w, rows, K / 32);
     PS_LAUNCH_CK();
+    return 0;
+}
+
+// up to three K-quant matrices that read the same input, quantising included; matrices of one type run in one launch.  *done = false: the other kernels are faster
+int matmul_mk(ps_cuda_ctx *ctx, const ActIn &in, int64_t K, int64_t bs, const PsMbSeg *segs, const int *types, int n_seg, const float *residual, bool *done) {
+    int64_t rows = 0;
+    bool same = true;
+    for (int t = 0; t < n_seg; t++) { rows += segs[t].n; same &= types[t] == types[0]; }
+    for (int t = 0; t < n_seg; t++)
+        if (!mk_tiles(ctx, types[t], K, same ? rows : segs[t].n, (int)std::min<int64_t>(bs, INT32_MAX))) return 0;
+    if (K > ctx->maxK || bs > ctx->d.max_batch) return fail(ctx, PS_CUDA_ERR_INVALID, "activation %lldx%lld exceeds workspace", (long long)K, (long long)bs);
+    if (K % 256) return fail(ctx, PS_CUDA_ERR_INVALID, "K=%lld is not a multiple of 256", (long long)K);
+    if (in.norm) PS_DEP(ps_k_mk_norm_quantize, (unsigned)bs, 512, 0, in.x, in.norm, K, ctx->d.norm_eps, ctx->mk_x);
+    else PS_DEP(ps_k_mk_quantize, dim3((unsigned)((K / 256 + 3) / 4), (unsigned)bs), 128, 0, in.x, in.u, K, ctx->mk_x);
+    for (int t0 = 0; t0 < n_seg;) {
+        PsMkArgs a{};
+        int tiles = 0;
+        rows = 0;
+        for (int t = t0; t < n_seg && (t == t0 || same); t++) {
+            a.seg[a.n_seg] = segs[t];
+            a.seg[a.n_seg++].cta0 = tiles;
+            tiles += (segs[t].n + 15) / 16;
+            rows += segs[t].n;
+        }
+        a.bs = (int)bs; a.nb = (int)(K / 256); a.x = ctx->mk_x; a.residual = residual; a.err = ctx->tc_err_dev;
+        const int nt = mk_tiles(ctx, types[t0], K, rows, (int)bs);
+        const int rc = types[t0] == 12 ? launch_mk_t<12>(ctx, a, tiles, nt) : types[t0] == 13 ? launch_mk_t<13>(ctx, a, tiles, nt) : launch_mk_t<14>(ctx, a, tiles, nt);
+        if (rc) return rc;
+        t0 += a.n_seg;
+    }
+    *done = true;
     return 0;
 }
 
@@ -1536,6 +1596,7 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
     PS_AL(ctx->aqs, ctx->maxK * B);
     PS_AL(ctx->ad, 4 * (ctx->maxK / 32) * B);
     PS_AL(ctx->absp, 4 * (ctx->maxK / 256 + 1) * 4 * B);
+    if (B > 1) PS_AL(ctx->mk_x, ps_mk_x_bytes(ctx->maxK + 255, B));
     PS_AL(ctx->ids_dev, 4 * 4096);
     PS_AL(ctx->ctr_dev, 16);
     { int rc_ = host_buffers(ctx); if (rc_) return bail(rc_); }
@@ -1874,6 +1935,11 @@ int ps_cuda_rmsnorm(ps_cuda_ctx *ctx, float *dst, const float *x, const float *w
 int ps_cuda_matmul(ps_cuda_ctx *ctx, float *dst, const void *w, int wtype, int64_t K, int64_t N, const float *x, int64_t bs) {
     PS_NO_ARCH("ps_cuda_matmul");
     if (bs <= 0 || N <= 0) return fail(ctx, PS_CUDA_ERR_INVALID, "matmul: empty shape");
+    const PsMbSeg sg = {(const uint8_t *)w, dst, nullptr, (int)std::min<int64_t>(N, INT32_MAX), 0};
+    bool done = false;
+    if (N < INT32_MAX - 16)
+        if (int rc = matmul_mk(ctx, {x}, K, bs, &sg, &wtype, 1, nullptr, &done)) return rc;
+    if (done) return 0;
     int rc = quantize_act(ctx, wtype, {x}, K, bs);
     if (rc) return rc;
     return matmul_q(ctx, dst, (const uint8_t *)w, wtype, K, N, bs, nullptr, nullptr);
@@ -2356,10 +2422,12 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             if ((rc = matmul_mt(ctx, {ctx->x, nullptr, ld.attn_norm}, dim, bs, {{ld.mt_q, ctx->q, bias ? ld.q_bias : nullptr, (int)qdim}, {ld.mt_k, ctx->k, bias ? ld.k_bias : nullptr, (int)kvd},
                                 {ld.mt_v, ctx->v, bias ? ld.v_bias : nullptr, (int)kvd}}, nullptr))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.tq, {ctx->x, nullptr, ld.attn_norm}, dim, bs))) return rc;
             const PsMbSeg sg[3] = {{ld.wq, ctx->q, d.qkv_bias ? ld.q_bias : nullptr, (int)qdim, 0}, {ld.wk, ctx->k, d.qkv_bias ? ld.k_bias : nullptr, (int)kvd, 0},
                                    {ld.wv, ctx->v, d.qkv_bias ? ld.v_bias : nullptr, (int)kvd, 0}};
+            const int ty[3] = {ld.tq, ld.tk, ld.tv};
             bool done = false;
+            if (!mo && (rc = matmul_mk(ctx, {ctx->x, nullptr, ld.attn_norm}, dim, bs, sg, ty, 3, nullptr, &done))) return rc;
+            if (!done && (rc = quantize_act(ctx, ld.tq, {ctx->x, nullptr, ld.attn_norm}, dim, bs))) return rc;
             if (mo) {
                 const size_t ob = mv_bytes(ctx->mv_type, 8, dim); // an octet's bytes
                 const PsMbSeg so[3] = {{ld.mv_qkv, ctx->q, sg[0].bias, (int)qdim, 0}, {ld.mv_qkv + ob * (size_t)(qdim / 8), ctx->k, sg[1].bias, (int)kvd, 0},
@@ -2370,7 +2438,6 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             } else if (bs > 1 && ld.tq == ld.tk && ld.tq == ld.tv) {
                 if ((rc = matmul_qb(ctx, ld.tq, dim, bs, sg, 3, nullptr))) return rc;
             } else {
-                const int ty[3] = {ld.tq, ld.tk, ld.tv};
                 for (int t = 0; t < 3; t++)
                     if ((rc = matmul_q(ctx, sg[t].dst, sg[t].w, ty[t], dim, sg[t].n, bs, sg[t].bias, nullptr))) return rc;
             }
@@ -2398,9 +2465,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         } else if (mt) {
             if ((rc = matmul_mt(ctx, {ctx->att}, qdim, bs, {{ld.mt_o, ctx->x, nullptr, (int)dim}}, ctx->x))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.to, {ctx->att}, qdim, bs))) return rc;
             bool done = false;
-            const PsMbSeg so = {ld.mv_o, ctx->x, nullptr, (int)dim, 0};
+            const PsMbSeg so = {ld.mv_o, ctx->x, nullptr, (int)dim, 0}, sg = {ld.wo, ctx->x, nullptr, (int)dim, 0};
+            if (!mo && (rc = matmul_mk(ctx, {ctx->att}, qdim, bs, &sg, &ld.to, 1, ctx->x, &done))) return rc;
+            if (!done && (rc = quantize_act(ctx, ld.to, {ctx->att}, qdim, bs))) return rc;
             if (mo && (rc = matmul_ob(ctx, qdim, bs, &so, 1, ctx->x, &done))) return rc;
             if (!done && (rc = matmul_q(ctx, ctx->x, ld.wo, ld.to, qdim, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wo.att
         }
@@ -2414,15 +2482,17 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         } else if (mt) {
             if ((rc = matmul_mt(ctx, {ctx->x, nullptr, ld.ffn_norm}, dim, bs, {{ld.mt_gate, ctx->g, nullptr, (int)ffn}, {ld.mt_up, ctx->u, nullptr, (int)ffn}}, nullptr))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.tgate, {ctx->x, nullptr, ld.ffn_norm}, dim, bs))) return rc;
+            const PsMbSeg sg[2] = {{ld.wgate, ctx->g, nullptr, (int)ffn, 0}, {ld.wup, ctx->u, nullptr, (int)ffn, 0}};
+            const int ty[2] = {ld.tgate, ld.tup};
             bool done = false;
+            if (!mo && (rc = matmul_mk(ctx, {ctx->x, nullptr, ld.ffn_norm}, dim, bs, sg, ty, 2, nullptr, &done))) return rc;
+            if (!done && (rc = quantize_act(ctx, ld.tgate, {ctx->x, nullptr, ld.ffn_norm}, dim, bs))) return rc;
             if (mo) {
                 const PsMbSeg so[2] = {{ld.mv_gu, ctx->g, nullptr, (int)ffn, 0}, {ld.mv_gu + mv_bytes(ctx->mv_type, 8, dim) * (size_t)(ffn / 8), ctx->u, nullptr, (int)ffn, 0}};
                 if ((rc = matmul_ob(ctx, dim, bs, so, 2, nullptr, &done))) return rc;
             }
             if (done) {
             } else if (bs > 1 && ld.tgate == ld.tup) {
-                const PsMbSeg sg[2] = {{ld.wgate, ctx->g, nullptr, (int)ffn, 0}, {ld.wup, ctx->u, nullptr, (int)ffn, 0}};
                 if ((rc = matmul_qb(ctx, ld.tgate, dim, bs, sg, 2, nullptr))) return rc;
             } else {
                 if ((rc = matmul_q(ctx, ctx->g, ld.wgate, ld.tgate, dim, ffn, bs, nullptr, nullptr))) return rc;
@@ -2439,9 +2509,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         } else if (mt) {
             if ((rc = matmul_mt(ctx, {ctx->g, ctx->u}, ffn, bs, {{ld.mt_down, ctx->x, nullptr, (int)dim}}, ctx->x))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ld.tdown, {ctx->g, ctx->u}, ffn, bs))) return rc;
             bool done = false;
-            const PsMbSeg so = {ld.mv_down, ctx->x, nullptr, (int)dim, 0};
+            const PsMbSeg so = {ld.mv_down, ctx->x, nullptr, (int)dim, 0}, sg = {ld.wdown, ctx->x, nullptr, (int)dim, 0};
+            if (!mo && (rc = matmul_mk(ctx, {ctx->g, ctx->u}, ffn, bs, &sg, &ld.tdown, 1, ctx->x, &done))) return rc;
+            if (!done && (rc = quantize_act(ctx, ld.tdown, {ctx->g, ctx->u}, ffn, bs))) return rc;
             if (mo && (rc = matmul_ob(ctx, ffn, bs, &so, 1, ctx->x, &done))) return rc;
             if (!done && (rc = matmul_q(ctx, ctx->x, ld.wdown, ld.tdown, ffn, dim, bs, nullptr, ctx->x))) return rc; // x = x + Wdown.h
         }
@@ -2456,9 +2527,10 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
         } else if (mt) {
             if ((rc = matmul_mt(ctx, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs, {{ctx->mt_out, ctx->logits, nullptr, d.vocab_size}}, nullptr))) return rc;
         } else {
-            if ((rc = quantize_act(ctx, ctx->t_out, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs))) return rc;
             bool done = false;
-            const PsMbSeg so = {ctx->mv_out, ctx->logits, nullptr, d.vocab_size, 0};
+            const PsMbSeg so = {ctx->mv_out, ctx->logits, nullptr, d.vocab_size, 0}, sg = {ctx->w_out, ctx->logits, nullptr, d.vocab_size, 0};
+            if (!mo && (rc = matmul_mk(ctx, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs, &sg, &ctx->t_out, 1, nullptr, &done))) return rc;
+            if (!done && (rc = quantize_act(ctx, ctx->t_out, {ctx->x, nullptr, ctx->w_out_norm}, dim, bs))) return rc;
             if (mo && (rc = matmul_ob(ctx, dim, bs, &so, 1, nullptr, &done))) return rc;
             if (!done && (rc = matmul_q(ctx, ctx->logits, ctx->w_out, ctx->t_out, dim, d.vocab_size, bs, nullptr, nullptr))) return rc;
         }
@@ -3059,6 +3131,7 @@ int ps_cuda_set_option(ps_cuda_ctx *ctx, const char *name, int value) {
     else if (!strcmp(name, "scores_batch_min")) ctx->opt_scores_batch_min = std::max(1, value); // batches at least this wide use the query-blocked scores kernel
     else if (!strcmp(name, "give_up_warp")) ctx->opt_give_up = value; // tests of the way out of a pipeline whose wait has run out
     else if (!strcmp(name, "tc_min")) ctx->opt_tc_min = std::max(2, value); // narrowest batch that takes the tcgen05 GEMM (narrower ones: multi-column row-walker)
+    else if (!strcmp(name, "mk_min")) ctx->opt_mk_min = std::max(2, value); // narrowest batch of K-quant rows that multiplies on the tensor cores (narrower ones: ps_k_matmul_qb)
     else if (!strcmp(name, "mt_min")) ctx->opt_mt_min = std::max(2, value); // narrowest batch of a 32-block model that multiplies on the tensor cores (narrower ones, and all where its records found no room: ps_k_matmul_ob)
     else if (!strcmp(name, "attn_tile")) ctx->opt_attn_tile = value; // register-tiled scores / P.V kernels for batches (0: the first-generation kernels, for A/B)
     else if (!strcmp(name, "pv_batch_min")) ctx->opt_pv_batch_min = value; // batches at least this wide use the query-blocked P.V kernel (prefill), narrower ones the per-(head, dim) warp kernel
