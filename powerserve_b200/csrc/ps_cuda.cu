@@ -2359,24 +2359,35 @@ static int launch_batch_scores(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs,
     }
     return 0;
 }
-static int launch_batch_pv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int64_t n_kv, int bs, int batch_min) {
+// soft-max of the scores (mask: a tree's bias, or null: the positions) and P.V
+static int launch_batch_pv(ps_cuda_ctx *ctx, int L, int nh, int nkv, int hs, int64_t n_kv, int bs, int batch_min, const float *mask) {
     const int64_t n_ctx = ctx->d.n_ctx;
+    const float kq_scale = 1.0f / sqrtf((float)hs);
+    const bool tile = bs >= batch_min && ctx->opt_attn_tile && hs % PS_PVT_D == 0 && PS_PVT_RING(4) + (size_t)PS_PVT_Q * n_kv * 4 <= 200 * 1024;
+    // The tile kernel takes the soft-max with it where its blocks of eight rows fill the GPU, and on rows short for their number. Per layer, a launch before it -> inside: 1B, 77 rows of
+    // 205 positions 12.9 + 12.0 -> 21.2 us; 8B, 128 of 2048 31.3 + 90 -> 114.7; 0.5B, 32 of 32 5.4 + 4.3 -> 5.2 (passes of 4, 2 and 6 layers 601 -> 588, 984 -> 981, 365 -> 348 us). On the other side a warp's pass over a long row is in nobody's shadow:
+    // 8B, 8 rows of 508 positions +4.6 us, 12 of 1012 +1.7; 1B, 24 of 1924 +7.2; 0.5B, 24 of 274 +0.4 and 8 of 1908 +17
+    const int64_t blocks = (int64_t)((bs + PS_PVT_Q - 1) / PS_PVT_Q) * nh;
+    const bool in_pv = tile && PS_PVT_RING(4) + ps_pvt_rows(n_kv) <= 200 * 1024 && (blocks >= ctx->n_sm || n_kv <= std::max<int64_t>(256, 6 * blocks));
+    const size_t rows = in_pv ? ps_pvt_rows(n_kv) : (size_t)PS_PVT_Q * n_kv * 4;
+    if (!in_pv) PS_DEP(ps_k_softmax_ext, (unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->kq, ctx->kq, mask, ctx->pos_dev, n_kv, bs, kq_scale);
     if (bs >= batch_min && (size_t)PS_PV_QB * n_kv * 4 <= 200 * 1024) {
         static bool pv_attr[64] = {};
         if (!pv_attr[ctx->device]) {
             PS_CK(cudaFuncSetAttribute(ps_k_attn_pv_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-            for (const auto k : {ps_k_attn_pv_tile<true, 4>, ps_k_attn_pv_tile<true, 6>, ps_k_attn_pv_tile<false, 4>}) PS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+            for (const auto k : {ps_k_attn_pv_tile<true, 4, true>, ps_k_attn_pv_tile<true, 6, true>, ps_k_attn_pv_tile<false, 4, true>, ps_k_attn_pv_tile<true, 4, false>,
+                                 ps_k_attn_pv_tile<true, 6, false>, ps_k_attn_pv_tile<false, 4, false>}) PS_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
             pv_attr[ctx->device] = true;
         }
         dim3 grid((unsigned)((bs + PS_PV_QB - 1) / PS_PV_QB), (unsigned)nh);
         const dim3 grid1 = grid;
-        const bool tile = ctx->opt_attn_tile && hs % PS_PVT_D == 0 && PS_PVT_RING(4) + (size_t)PS_PVT_Q * n_kv * 4 <= 200 * 1024;
         if (tile)
             while ((int)(grid.x * grid.y * grid.z) * 2 <= ctx->n_sm * 2 && (int)grid.z * 2 * 8 * PS_PVT_D <= hs) grid.z *= 2; // narrow batch: split the dim groups over more CTAs
         static_assert(PS_PV_QB == PS_PVT_Q, "both P.V kernels block the queries by 8");
-        const bool vec = n_ctx % 4 == 0 && ((uintptr_t)ctx->vct[L] & 15) == 0, deep = vec && PS_PVT_RING(6) + (size_t)PS_PVT_Q * n_kv * 4 <= 112 * 1024; // (two CTAs an SM)
-        const auto pv = deep ? ps_k_attn_pv_tile<true, 6> : vec ? ps_k_attn_pv_tile<true, 4> : ps_k_attn_pv_tile<false, 4>;
-        if (tile) PS_DEP(pv, grid, 256, (deep ? PS_PVT_RING(6) : PS_PVT_RING(4)) + (size_t)PS_PVT_Q * n_kv * 4, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
+        const bool vec = n_ctx % 4 == 0 && ((uintptr_t)ctx->vct[L] & 15) == 0, deep = vec && PS_PVT_RING(6) + rows <= 112 * 1024; // (two CTAs an SM)
+        const auto pv = in_pv ? deep ? ps_k_attn_pv_tile<true, 6, true> : vec ? ps_k_attn_pv_tile<true, 4, true> : ps_k_attn_pv_tile<false, 4, true>
+                              : deep ? ps_k_attn_pv_tile<true, 6, false> : vec ? ps_k_attn_pv_tile<true, 4, false> : ps_k_attn_pv_tile<false, 4, false>;
+        if (tile) PS_DEP(pv, grid, 256, (deep ? PS_PVT_RING(6) : PS_PVT_RING(4)) + rows, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs, mask, ctx->pos_dev, kq_scale);
         else PS_DEP(ps_k_attn_pv_batch, grid1, 256, (size_t)PS_PV_QB * n_kv * 4, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
     } else {
         PS_DEP(ps_k_attn_pv, dim3((unsigned)((hs + 3) / 4), (unsigned)nkv), 128, 0, ctx->att, ctx->vct[L], ctx->kq, hs, nh, nkv, n_kv, n_ctx, bs);
@@ -2454,8 +2465,7 @@ static int forward_ops(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0, int tree
             PS_DEP(pv, dim3((unsigned)((hs + 31) / 32), (unsigned)nkv, (unsigned)bs), 128, 0, ctx->att, pl + d.max_batch, ctx->kq, (int)hs, (int)nh, (int)nkv, ctx->pos_dev, d.n_ctx, cs);
         } else {
         if ((rc = launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs))) return rc;
-        PS_DEP(ps_k_softmax_ext, (unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->kq, ctx->kq, tree ? ctx->tree_bias : nullptr, ctx->pos_dev, n_kv, bs, kq_scale);
-        if ((rc = launch_batch_pv(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs, ctx->opt_pv_batch_min))) return rc;
+        if ((rc = launch_batch_pv(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs, ctx->opt_pv_batch_min, tree ? ctx->tree_bias : nullptr))) return rc;
         }
         if (tc) {
             if ((rc = tc_single(ctx, {ctx->att}, ld.tc_o, (int)dim, (int)qdim, ctx->x, bs, ctx->x))) return rc;
@@ -2606,9 +2616,7 @@ static int forward_ops_tp(ps_cuda_ctx *ctx, int bs, int lm_head, int pos0) {
         }
         if ((rc = launch_rope_kv(ctx, L, (int)nh, (int)nkv, bs))) return rc;
         if ((rc = launch_batch_scores(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs))) return rc;
-        ps_k_softmax_ext<<<(unsigned)(bs * nh), 256, (size_t)n_kv * 4, ctx->stream>>>(ctx->kq, ctx->kq, nullptr, ctx->pos_dev, n_kv, bs, kq_scale);
-        PS_LAUNCH_CK();
-        if ((rc = launch_batch_pv(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs, 0))) return rc;
+        if ((rc = launch_batch_pv(ctx, L, (int)nh, (int)nkv, (int)hs, n_kv, bs, 0, nullptr))) return rc;
         if ((rc = tp_gather_rows(ctx, attb, ctx->att, bs, qdim_l))) return rc;                      // exchange 1: attention output
         if (tc) {
             if ((rc = tc_single(ctx, {attb}, ld.tc_o, (int)dim_l, (int)qdim, xl, bs, xl))) return rc;       // x[rows of this rank] += Wo[rows] . att

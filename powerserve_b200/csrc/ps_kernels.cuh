@@ -1226,17 +1226,23 @@ template <int N> PS_D void ps_cp_async_wait() { asm volatile("cp.async.wait_grou
 // takes eight, which cost shared memory more than everything else in the loop; pairs of queries are packed floats.  DEPTH chunks of a row are on their way:
 // a chunk takes a warp about 200 cycles, memory about 800.  32 heads x 128 queries x 2048 keys, head size 128: 107 us by words, 92 by lines and
 // pairs and four chunks; a pass of two such layers 1108 -> 1082 us with pairs and six
-template <bool VEC, int DEPTH>
+// SOFT: `p` are scores, and the soft-max of the CTA's rows is taken here as well: ps_k_softmax_ext's arithmetic by a warp a row, the doubles of its sum added in another order.  A launch of its
+// own writes and reads the rows once more and is latency on short ones; here a row has one warp instead of eight (launch_batch_pv has the line between them)
+PS_HD size_t ps_pvt_rows(int64_t n_kv) { return (size_t)PS_PVT_Q * (size_t)((n_kv + 31) / 32) * 32 * 4; } // bytes of the probabilities
+template <bool VEC, int DEPTH, bool SOFT>
 __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ out, const float *__restrict__ vct, const float *__restrict__ p,
-                                                            int hs, int n_heads, int n_kv_heads, int64_t n_kv, int64_t n_ctx, int bs) {
+                                                            int hs, int n_heads, int n_kv_heads, int64_t n_kv, int64_t n_ctx, int bs,
+                                                            const float *__restrict__ mask, const int32_t *__restrict__ pos, float scale) {
     ps_grid_dep();
     // [ring: 8 warps][DEPTH][PS_PVT_D][32] V^T chunks, then the probabilities, position-major: s_p4[j] = queries 0..3
     // at position j, s_p4[n_kv + j] = queries 4..7, so a lane fetches its eight probabilities of a chunk with two
-    // conflict-free 16-byte loads off one address register
+    // conflict-free 16-byte loads off one address register; SOFT: [chunk of 32 positions][query][32], whole lines for the warp of a row (eight loads of a chunk: 1 to 2 us a layer where
+    // a CTA has an SM to itself, so not where nothing is gained by it)
     extern __shared__ __align__(16) float4 s_pvt[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     float *const ring = reinterpret_cast<float *>(s_pvt) + warp * (DEPTH * PS_PVT_D * 32);
-    float4 *s_p4 = s_pvt + PS_PVT_RING(DEPTH) / 16;
+    float4 *const s_p4 = s_pvt + PS_PVT_RING(DEPTH) / 16;
+    float *const s_p = reinterpret_cast<float *>(s_p4);
     const int i0 = blockIdx.x * PS_PVT_Q, h = blockIdx.y, g = h / (n_heads / n_kv_heads);
     const int nq = min(PS_PVT_Q, bs - i0);
     const int nkv = (int)n_kv;
@@ -1264,7 +1270,8 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
 #pragma unroll
         for (int k = 0; k < DEPTH - 1; k++) issue(k, k);
     }
-    {
+    float *const row = s_p + warp * 32 + lane; // row i0 + warp: position 32 k + lane is row[256 k]
+    if (!SOFT) {
         const float *pr = p + ((int64_t)h * bs + i0) * n_kv;
         for (int j = tid; j < nkv; j += 256) {
             float e[PS_PVT_Q];
@@ -1273,10 +1280,57 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
             s_p4[j] = make_float4(e[0], e[1], e[2], e[3]);
             s_p4[nkv + j] = make_float4(e[4], e[5], e[6], e[7]);
         }
+    } else if (warp < nq) {
+        const float *pr = p + ((int64_t)h * bs + i0 + warp) * n_kv, *mr = mask ? mask + (int64_t)(i0 + warp) * n_kv : nullptr;
+        const int last = mask ? 0 : pos[i0 + warp];
+        float mx = -INFINITY;
+#pragma unroll 8
+        for (int k = 0; k < (nkv + 31) >> 5; k++) {
+            const int j = 32 * k + lane;
+            if (j < nkv) {
+                const float v = __fadd_rn(__fmul_rn(pr[j], scale), mask ? mr[j] : j <= last ? 0.f : -INFINITY);
+                row[256 * k] = v;
+                mx = fmaxf(mx, v);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(PS_FULL, mx, o));
+        const int n8 = nkv & ~7;
+        double sum = 0.0;
+#pragma unroll 2
+        for (int k = 0; k < (n8 + 31) >> 5; k++) { // eight lanes: one group of eight, ((v4 + v0) + (v6 + v2)) + ((v5 + v1) + (v7 + v3))
+            const bool in = 32 * k + lane < n8;
+            float v = 0.f;
+            if (in) {
+                v = ps_v_expf(__fadd_rn(row[256 * k], -mx));
+                row[256 * k] = v;
+            }
+            v = __fadd_rn(v, __shfl_xor_sync(PS_FULL, v, 4));
+            v = __fadd_rn(v, __shfl_xor_sync(PS_FULL, v, 2));
+            v = __fadd_rn(v, __shfl_xor_sync(PS_FULL, v, 1));
+            if (in && (lane & 7) == 0) sum += (double)v;
+        }
+        if (n8 + lane < nkv) { // scalar tail: libm expf
+            const int j = n8 + lane;
+            float *at = s_p + ((j >> 5) * PS_PVT_Q + warp) * 32 + (j & 31);
+            const float v = ps_expf_glibc(__fadd_rn(*at, -mx));
+            *at = v;
+            sum += (double)v;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(PS_FULL, sum, o);
+        const float inv = (float)(1.0 / sum);
+        __syncwarp();
+#pragma unroll 4
+        for (int k = 0; k < (nkv + 31) >> 5; k++)
+            if (32 * k + lane < nkv) row[256 * k] = __fmul_rn(row[256 * k], inv);
+    } else {
+        for (int k = 0; k < (nkv + 31) >> 5; k++) row[256 * k] = 0.f;
     }
     __syncthreads();
     for (int d0 = d_first; d0 < hs; d0 += d_step) {
-        const ulonglong2 *sp = reinterpret_cast<const ulonglong2 *>(s_p4) + lane;
+        const ulonglong2 *sp4 = reinterpret_cast<const ulonglong2 *>(s_p4) + lane;
+        const float *sp = s_p + lane;
         ps_f2 acc2[PS_PVT_D][PS_PVT_Q / 2]; // [di][pair of queries]
 #pragma unroll
         for (int di = 0; di < PS_PVT_D; di++)
@@ -1290,8 +1344,13 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
             issue(c + DEPTH - 1, slot == 0 ? DEPTH - 1 : slot - 1); // into the slot of the chunk before
             const float *rv = ring + slot * (PS_PVT_D * 32) + lane;
             slot = slot + 1 == DEPTH ? 0 : slot + 1;
-            const ulonglong2 lo = sp[32 * c], hi = sp[nkv + 32 * c];
-            const ps_f2 pp[PS_PVT_Q / 2] = {lo.x, lo.y, hi.x, hi.y};
+            ps_f2 pp[PS_PVT_Q / 2];
+            if (!SOFT) {
+                const ulonglong2 lo = sp4[32 * c], hi = sp4[nkv + 32 * c];
+                pp[0] = lo.x, pp[1] = lo.y, pp[2] = hi.x, pp[3] = hi.y;
+            } else
+#pragma unroll
+            for (int k = 0; k < PS_PVT_Q / 2; k++) pp[k] = ps_f2_pack(sp[c * (PS_PVT_Q * 32) + 64 * k], sp[c * (PS_PVT_Q * 32) + 64 * k + 32]);
 #pragma unroll
             for (int di = 0; di < PS_PVT_D; di++) {
                 const float v = rv[di * 32];
@@ -1331,13 +1390,12 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
         ps_rs_stage<4>(a4, lane & 2, 2);
         const int di = lane >> 2, qb = 4 * (lane & 1) + (lane & 2);
         const float *vrow = vct + ((int64_t)g * hs + d0 + di) * n_ctx;
-        const float *sf = reinterpret_cast<const float *>(s_p4);
 #pragma unroll
         for (int e = 0; e < 2; e++) {
             const int qi = qb + e;
-            const float *pq = sf + (size_t)(qi >> 2) * nkv * 4 + (qi & 3);
+            const float *pq = SOFT ? s_p + (nc * PS_PVT_Q + qi) * 32 : s_p + (size_t)(qi >> 2) * nkv * 4 + (qi & 3) + 4 * np; // from the leftovers' first position
             float sum = a4[e];
-            for (int t = np; t < nkv; t++) sum = __fadd_rn(sum, __fmul_rn(vrow[t], pq[4 * t])); // leftovers: mul, then add, in order
+            for (int t = np; t < nkv; t++) sum = __fadd_rn(sum, __fmul_rn(vrow[t], pq[SOFT ? t - np : 4 * (t - np)])); // leftovers: mul, then add, in order
             if (qi < nq) out[((int64_t)(i0 + qi) * n_heads + h) * hs + d0 + di] = sum;
         }
     }
