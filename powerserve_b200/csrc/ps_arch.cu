@@ -692,7 +692,8 @@ int ps_arch_create(PsArch **out, const ps_cuda_arch_desc *desc, std::string &err
     int dev = 0;
     cudaGetDevice(&dev);
     { int v = 148; if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) a->n_sm = v; }
-    if (cudaFuncSetAttribute(pa_k_dec_scores, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
+    if (cudaFuncSetAttribute(pa_k_softmax_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, PA_SMX_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(pa_k_dec_scores, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(pa_k_dec_pv, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(pa_k_dec_mv<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(pa_k_dec_mv<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024) != cudaSuccess ||
@@ -1303,6 +1304,16 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         PA_LAUNCH();
         return 0;
     };
+    // soft-max of a batch's rows: in shared memory while two CTAs of them share an SM (16 mixed heads: 1 500 keys; eight rows: 3 200) and, with a mix, rows are many and long enough, else in place
+    auto launch_softmax = [&](const PaAttn &at) {
+        int cap = n_kv; // keys of the longest row
+        if (at.window > 0) cap = std::min(cap, at.window);
+        if (at.chunk > 0) cap = std::min(cap, at.chunk);
+        const size_t smem = at.mix ? 4 * (size_t)at.H * (pa_mix_ld(at.H) + cap) : 4 * (size_t)8 * cap;
+        if (smem <= PA_SMX_SMEM && (!at.mix || (bs > a->n_sm / 2 && cap >= 512)))
+            pa_launch_dep(pdl, pa_k_softmax_rows, dim3((unsigned)bs, at.mix ? 1 : cdiv(at.H, 8)), dim3(256), smem, st, at, a->S, io.pos_dev, bs, cap);
+        else pa_launch_dep(pdl, pa_k_mix_softmax, dim3(bs), dim3(256), 4 * (size_t)at.H * at.H, st, at, a->S, io.pos_dev, bs);
+    };
     // scores -> soft-max -> P.V of a batch against the cache rows 0 .. n_kv - 1 (keys before the first query's window are skipped)
     auto attend = [&](const PaAttn &at, const float *q, int ldq, int kd, int li, float *out, int aw) -> int {
         int lo0 = at.window > 0 ? std::max(0, pos0 - at.window + 1) : 0; // the first key the first query sees
@@ -1312,7 +1323,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         const int nv = (at.pool > 0 && n_kv - at.window >= at.pool) ? (n_kv - at.window) / at.pool : 0;
         pa_launch_dep(pdl, pa_k_scores, dim3(tok_tiles + cdiv(nv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st, at, q, ldq, io.kc[li], kd, a->S, io.pos_dev, bs, tile0, tok_tiles);
         PA_LAUNCH();
-        pa_launch_dep(pdl, pa_k_mix_softmax, dim3(bs), dim3(256), 4 * (size_t)at.H * at.H, st, at, a->S, io.pos_dev, bs);
+        launch_softmax(at);
         PA_LAUNCH();
         pa_launch_dep(false, pa_k_pv<!ROUND>, dim3(cdiv(at.dv, PA_TN), cdiv(bs, PA_TM), at.H), blk, 0, st, at, a->S, io.vct[li], out, aw, io.pos_dev, bs);
         PA_LAUNCH();
@@ -2073,7 +2084,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         } else {
             pa_launch_dep(pdl, pa_k_scores, dim3(cdiv(n_kv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st, at, a->qkv, nqkv, io.kc[li], w.kd, a->S, io.pos_dev, bs, 0, (int)cdiv(n_kv, PA_TN));
             PA_LAUNCH();
-            pa_launch_dep(pdl, pa_k_mix_softmax, dim3(bs), dim3(256), 4 * (size_t)H * H, st, at, a->S, io.pos_dev, bs);
+            launch_softmax(at);
             PA_LAUNCH();
             pa_launch_dep(false, pa_k_pv<!ROUND>, dim3(cdiv(dv, PA_TN), cdiv(bs, PA_TM), H), blk, 0, st, at, a->S, io.vct[li], a->att, w.od, io.pos_dev, bs);
             PA_LAUNCH();

@@ -16,6 +16,7 @@
 #define PA_TK 32
 #define PA_LD (PA_TM + 4)
 #define PA_MAX_HEADS 64
+#define PA_SMX_SMEM (100 * 1024) // pa_k_softmax_rows' shared memory at most: two CTAs an SM
 #define PA_MAX_EXPERTS 256
 
 // activation of a gated unit: PS_ACT_SWISH  g' sigmoid(alpha g') (u' + shift) on g' = min(g, limit), u' = clamp(u, +-limit)
@@ -1047,6 +1048,108 @@ __global__ void __launch_bounds__(256) pa_k_mix_softmax(PaAttn at, float *__rest
         if (at.sink) sum += expf(sk - mx);
         const float inv = 1.0f / sum;
         for (int j = lo + lane; j < n; j += 32) row[j] *= inv;
+        for (int j = n + lane; j < n_end; j += 32) row[j] = 0.f;
+        for (int j = lo_tile + lane; j < lo; j += 32) row[j] = 0.f;
+        for (int j = lane; j < nv; j += 32) prow[j] *= inv;
+        for (int j = nv + lane; j < nv_tile; j += 32) prow[j] = 0.f;
+    }
+}
+
+// The same where a query's rows fit shared memory (`cap` keys each: all heads' with a mix, else those of a CTA's eight heads, gridDim.y CTAs a query). In place a row goes to global memory and back
+// three times (a mix: four), a load behind the stores before it, and the mix reads its matrix by words, more of them than products' time. 256 queries x 16 mixed heads x 1024 keys: a pass 297 -> 277 us;
+// without a mix passes of 175 to 450 us are 1 to 9 us shorter. Short or few mixed rows stay above: their time is the fetching of instructions, of which there are more here (24 queries of 26 or of
+// 1048 keys 3 to 5 us longer, 100 of 400 the same, 100 of 1124 12 us shorter, 250 of 550 7)
+PS_HD int pa_mix_ld(int H) { return (H + 3) & ~3; } // floats of a row of the mixing matrix in shared memory
+template <int MAXH>
+__device__ __forceinline__ void pa_mix_shared(const PaAttn &at, const float *S, int i, int lo, int n, const float *Ts, float *rows, int cap) {
+    const int H = at.H, ldT = pa_mix_ld(H);
+    for (int j = lo + threadIdx.x; j < n; j += 256) {
+        float a[MAXH];
+#pragma unroll
+        for (int g = 0; g < MAXH; g++) a[g] = g < H ? S[((int64_t)g * at.B + i) * at.ldS + j] : 0.f;
+#pragma unroll 1
+        for (int h = 0; h < H; h++) {
+            float s = 0.f;
+#pragma unroll
+            for (int g = 0; g < MAXH; g += 4) {
+                if (g >= H) break;
+                const float4 t = *reinterpret_cast<const float4 *>(Ts + h * ldT + g); // (zero past the heads)
+                s = fmaf(t.x, a[g], s);
+                s = fmaf(t.y, a[g + 1], s);
+                s = fmaf(t.z, a[g + 2], s);
+                s = fmaf(t.w, a[g + 3], s);
+            }
+            rows[h * cap + j - lo] = s;
+        }
+    }
+}
+__global__ void __launch_bounds__(256) pa_k_softmax_rows(PaAttn at, float *__restrict__ S, const int32_t *__restrict__ pos, int bs, int cap) {
+    extern __shared__ __align__(16) float Ts[];
+    const int i = blockIdx.x, H = at.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float *const rows = Ts + (at.mix ? H * pa_mix_ld(H) : 0);
+    if (at.mix) // a weight: fetched before the dependency wait
+        for (int h = warp; h < H; h += 8)
+            for (int g = lane; g < pa_mix_ld(H); g += 32) Ts[h * pa_mix_ld(H) + g] = g < H ? at.mix[h * H + g] : 0.f;
+    ps_grid_dep();
+    const int n = pos[i] + 1, n_end = pos[0] + bs, lo = pa_first_key(at, pos[i]);
+    const int lo_tile = pa_tile_first_key(at, pos[0] + i / PA_TM * PA_TM);
+    if (at.mix) {
+        __syncthreads();
+        if (H <= 8) pa_mix_shared<8>(at, S, i, lo, n, Ts, rows, cap);
+        else if (H <= 16) pa_mix_shared<16>(at, S, i, lo, n, Ts, rows, cap);
+        else if (H <= 32) pa_mix_shared<32>(at, S, i, lo, n, Ts, rows, cap);
+        else pa_mix_shared<PA_MAX_HEADS>(at, S, i, lo, n, Ts, rows, cap);
+        __syncthreads();
+    }
+    // pooled blocks: the query's own, and those of its tile's furthest query (P.V walks whole tiles: zeros in between)
+    const int nv = pa_pool_vis(at, pos[i]), nv_tile = pa_pool_vis(at, pos[0] + min(i / PA_TM * PA_TM + PA_TM, bs) - 1);
+    for (int h = blockIdx.y * 8 + warp; h < H; h += 8 * gridDim.y) {
+        float *row = S + ((int64_t)h * at.B + i) * at.ldS, *prow = row + at.pool_off;
+        const float sk = pa_sink_logit(at, h);
+        float mx = at.sink ? sk : -INFINITY;
+        float *const b = rows + (at.mix ? h : warp) * cap; // the row's keys from `lo` on
+        const int m = n - lo;
+        float v[8];
+        for (int j = lane; j < m; j += 256) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = j + 32 * k >= m ? -INFINITY : at.mix ? b[j + 32 * k] : row[lo + j + 32 * k];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                mx = fmaxf(mx, v[k]);
+                if (!at.mix && j + 32 * k < m) b[j + 32 * k] = v[k];
+            }
+        }
+        for (int j = lane; j < nv; j += 32) mx = fmaxf(mx, prow[j]);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        float sum = 0.f;
+        for (int j = lane; j < m; j += 256) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = j + 32 * k < m ? b[j + 32 * k] : -INFINITY;
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (j + 32 * k < m) {
+                    const float e = expf(v[k] - mx);
+                    b[j + 32 * k] = e;
+                    sum += e;
+                }
+        }
+        for (int j = lane; j < nv; j += 32) {
+            const float e = expf(prow[j] - mx);
+            prow[j] = e;
+            sum += e;
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (at.sink) sum += expf(sk - mx);
+        const float inv = 1.0f / sum;
+        for (int j = lane; j < m; j += 256) {
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = j + 32 * k < m ? b[j + 32 * k] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++)
+                if (j + 32 * k < m) row[lo + j + 32 * k] = v[k] * inv;
+        }
         for (int j = n + lane; j < n_end; j += 32) row[j] = 0.f;
         for (int j = lo_tile + lane; j < lo; j += 32) row[j] = 0.f;
         for (int j = lane; j < nv; j += 32) prow[j] *= inv;
