@@ -2725,7 +2725,7 @@ int ps_cuda_forward(ps_cuda_ctx *ctx, const int32_t *tokens, const int32_t *pos,
 // ps_cuda_session_select makes one of them the target of every single-sequence call (forward / decode_greedy / kv_*: prefill
 // and bookkeeping work unchanged), and ps_cuda_forward_sessions advances n sessions by one token each in ONE forward pass -
 // the weight stream is read once for the n columns (Q4_K: multi-column row-walker, tcgen05 GEMM from option tc_min up; other formats:
-// ps_k_matmul_ob or ps_k_matmul_qb), attention
+// ps_k_matmul_mt, ps_k_matmul_mk or ps_k_matmul_qb), attention
 // runs per column over its own session's cache.  A session's logits are bit-identical to decoding it alone with batch 1.
 // The captured steps hold the old set's cache pointers (nothing else does that a switch has to renew: a set brings its pointer table, the
 // opt-in step kernel's table is renewed where it is launched, and a layer-list executor takes the pointers with every pass).  Two pageable copies and a
