@@ -1295,6 +1295,7 @@ __global__ void __launch_bounds__(256, 2) ps_k_attn_pv_tile(float *__restrict__ 
         }
 #pragma unroll
         for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(PS_FULL, mx, o));
+        __syncwarp(); // (the scalar tail reads what other lanes have stored; shuffles order no memory)
         const int n8 = nkv & ~7;
         double sum = 0.0;
 #pragma unroll 2

@@ -39,3 +39,23 @@ def test_same_bits_as_a_launch_of_its_own(name, tmp_path):
     cm.close()
     for a, b, what in zip(got[1], got[0], PORTIONS + [5, 1100]):
         L.assert_bit_equal(a, b, f"{name} {what}")
+
+
+@pytest.mark.parametrize("rest", range(1, 8))
+def test_leftovers_that_other_lanes_stored(rest, tmp_path):
+    """rows whose last one to seven positions begin at lane 8, 16 or 24 of a chunk: the lane that takes the exponential of such a position is not the one that stored its score"""
+    cm = capi.CudaModel(synth.write_model_dir(str(tmp_path), SHAPES["hs64"], seed=6), max_batch=64)
+    toks = synth.random_prompt(500, 300, seed=rest)
+    got = {}
+    for tiled in (0, 1):
+        cm.be.set_option("attn_tile", tiled)
+        got[tiled] = []
+        for n8 in (8, 16, 24, 40, 208):
+            cm.reset()
+            if n8 > 32:
+                cm.prefill(np.r_[toks[:n8 - 8], toks[:1]], 64)
+            lo = cm.position
+            got[tiled].append(cm.forward(toks[lo:n8 + rest]))
+    cm.close()
+    for a, b in zip(got[1], got[0]):
+        L.assert_bit_equal(a, b, f"rest {rest}")
