@@ -73,7 +73,7 @@ int  ps_cuda_device_count(void);
 int  ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc);
 void ps_cuda_destroy(ps_cuda_ctx *ctx);
 const char *ps_cuda_last_error(const ps_cuda_ctx *ctx); /* ctx may be NULL: error of a failed create */
-int  ps_cuda_sync(ps_cuda_ctx *ctx);
+int  ps_cuda_sync(ps_cuda_ctx *ctx); /* waits; PS_CUDA_ERR_CUDA if a kernel since the last report flagged a failure (results invalid) */
 void *ps_cuda_stream(ps_cuda_ctx *ctx);                 /* the cudaStream_t every call enqueues on */
 
 /* ---------------------------------------------------------------------------------------------- memory
@@ -83,7 +83,7 @@ void *ps_cuda_stream(ps_cuda_ctx *ctx);                 /* the cudaStream_t ever
 int   ps_cuda_malloc(ps_cuda_ctx *ctx, size_t bytes, void **dev);
 int   ps_cuda_free(ps_cuda_ctx *ctx, void *dev);
 int   ps_cuda_memcpy_h2d(ps_cuda_ctx *ctx, void *dev, const void *host, size_t bytes);
-int   ps_cuda_memcpy_d2h(ps_cuda_ctx *ctx, void *host, const void *dev, size_t bytes);  /* synchronises */
+int   ps_cuda_memcpy_d2h(ps_cuda_ctx *ctx, void *host, const void *dev, size_t bytes);  /* synchronises, reports like ps_cuda_sync */
 int   ps_cuda_register_weight(ps_cuda_ctx *ctx, const void *host, int type, int64_t ne0, int64_t ne1, void **dev);
 void *ps_cuda_lookup_weight(ps_cuda_ctx *ctx, const void *host);
 int   ps_cuda_unregister_weight(ps_cuda_ctx *ctx, const void *host); /* frees the device copy (model unload) */

@@ -658,7 +658,7 @@ int matmul_mk(ps_cuda_ctx *ctx, const ActIn &in, int64_t K, int64_t bs, const Ps
             tiles += (segs[t].n + 15) / 16;
             rows += segs[t].n;
         }
-        a.bs = (int)bs; a.nb = (int)(K / 256); a.x = ctx->mk_x; a.residual = residual; a.err = ctx->tc_err_dev;
+        a.bs = (int)bs; a.nb = (int)(K / 256); a.x = ctx->mk_x; a.residual = residual; a.err = ctx->tc_err_dev; a.give_up = ctx->opt_give_up;
         const int nt = mk_tiles(ctx, types[t0], K, rows, (int)bs);
         const int rc = types[t0] == 12 ? launch_mk_t<12>(ctx, a, tiles, nt) : types[t0] == 13 ? launch_mk_t<13>(ctx, a, tiles, nt) : launch_mk_t<14>(ctx, a, tiles, nt);
         if (rc) return rc;
@@ -1811,9 +1811,11 @@ int ps_cuda_host_free(void *host) {
     return e == cudaSuccess ? 0 : fail(nullptr, PS_CUDA_ERR_CUDA, "cudaFreeHost failed: %s", cudaGetErrorString(e));
 }
 
+// (a failure that a kernel of the operator table has flagged is reported here or by the copy that fetches its result; the lock: a forward pass in another
+// thread keeps its own flags)
 int ps_cuda_sync(ps_cuda_ctx *ctx) {
-    PS_CK(cudaStreamSynchronize(ctx->stream));
-    return 0;
+    std::lock_guard<std::mutex> lock(ctx->mu);
+    return sync_and_check(ctx);
 }
 
 void *ps_cuda_stream(ps_cuda_ctx *ctx) { return (void *)ctx->stream; }
@@ -1862,10 +1864,10 @@ int ps_cuda_memcpy_h2d(ps_cuda_ctx *ctx, void *dev, const void *host, size_t byt
 }
 
 int ps_cuda_memcpy_d2h(ps_cuda_ctx *ctx, void *host, const void *dev, size_t bytes) {
+    std::lock_guard<std::mutex> lock(ctx->mu);
     PS_CK(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    PS_CK(cudaStreamSynchronize(ctx->stream));
     ctx->d2h += (int64_t)bytes;
-    return 0;
+    return sync_and_check(ctx);
 }
 
 int ps_cuda_register_weight(ps_cuda_ctx *ctx, const void *host, int type, int64_t ne0, int64_t ne1, void **dev) {

@@ -80,7 +80,7 @@ struct PsMkArgs {
     int n_seg, bs, nb, ns; // super-blocks of a row; stages of the ring
     const uint8_t *x;   // activation records
     const float *residual;
-    int *err;
+    int *err, give_up;
 };
 #define PS_MK_MAX_NS 8
 // a row's bytes of one super-block and the 16-byte lines around them; rows lie PITCH apart (an odd number of lines, which spreads them over the banks)
@@ -150,6 +150,7 @@ __global__ void __launch_bounds__(128) ps_k_matmul_mk(const PsMkArgs a) {
     }
     int slot = 0;
     uint32_t phase = 0;
+    if (warp == a.give_up) *a.err = PS_ERR_COPY;
     const uint32_t mine = B::MIN_SCALAR || t == warp ? 0xFFFFFFFFu : 0u; // the mins chain's part of k
     for (int i = 0; i < nb; i++) {
         switch (ns) { // (groups still in flight: a constant of the instruction)

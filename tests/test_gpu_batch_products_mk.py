@@ -78,3 +78,28 @@ def test_scales_that_are_not_finite(be, t):
     got, ref = _product(be, t, np.ascontiguousarray(w.reshape(-1)), K, N, rng.standard_normal(K * bs).astype(np.float32), bs)
     for m in got:
         assert np.array_equal(got[m], ref, equal_nan=True), m
+
+
+@pytest.mark.parametrize("t", TYPES)
+@pytest.mark.parametrize("warp", [0, 3])
+def test_a_warp_that_gives_up_is_reported(be, t, warp):
+    """a product of the operator table whose copies did not arrive: whoever waits for it or fetches it is told, once, and the next product has all bits"""
+    K, N, bs = 512, 40, 6
+    rng = np.random.default_rng(t)
+    w = synth.random_blocks(rng, t, N, K, K ** -0.5).reshape(-1)
+    x = rng.standard_normal(K * bs).astype(np.float32)
+    ref = np.zeros(N * bs, np.float32)
+    L.oracle().ps_or_matmul(t, L.vptr(w), K, N, L.fptr(x), bs, L.fptr(ref))
+    wd, xd, dd = be.register_weight(w, t, K, N), be.upload(x), be.empty(N * bs)
+    for ask in (dd.numpy, be.sync):
+        be.set_option("give_up_warp", warp)
+        be.matmul(dd, wd, t, K, N, xd, bs)
+        with pytest.raises(capi.PsCudaError, match="copy of a batch product"):
+            ask()
+        be.set_option("give_up_warp", -1)
+        be.sync()
+        be.matmul(dd, wd, t, K, N, xd, bs)
+        L.assert_bit_equal(dd.numpy(), ref, f"type {t}, after warp {warp} gave up")
+    xd.free()
+    dd.free()
+    be.unregister_weight(w)
