@@ -80,7 +80,7 @@ struct PsMkArgs {
     int n_seg, bs, nb, ns; // super-blocks of a row; stages of the ring
     const uint8_t *x;   // activation records
     const float *residual;
-    int *err, give_up;
+    int *err;
 };
 #define PS_MK_MAX_NS 8
 // a row's bytes of one super-block and the 16-byte lines around them; rows lie PITCH apart (an odd number of lines, which spreads them over the banks)
@@ -150,7 +150,6 @@ __global__ void __launch_bounds__(128) ps_k_matmul_mk(const PsMkArgs a) {
     }
     int slot = 0;
     uint32_t phase = 0;
-    if (warp == a.give_up) *a.err = PS_ERR_COPY;
     const uint32_t mine = B::MIN_SCALAR || t == warp ? 0xFFFFFFFFu : 0u; // the mins chain's part of k
     for (int i = 0; i < nb; i++) {
         switch (ns) { // (groups still in flight: a constant of the instruction)
@@ -160,7 +159,7 @@ __global__ void __launch_bounds__(128) ps_k_matmul_mk(const PsMkArgs a) {
         default: ps_cp_async_wait<3>(); break; // (ns 5 and more: some wait longer than they must)
         }
         // after a wait that gave up the results are invalid; the loop goes on and waits for the other copies, each within its limit
-        if (!ps_tc_wait(&bar[slot], phase)) *a.err = PS_ERR_COPY;
+        if (!ps_tc_wait(&bar[slot], phase, PS_COPY_POLLS)) *a.err = PS_ERR_COPY;
         __syncthreads(); // everyone's lines have arrived, and everyone has read the slot before
         {
             const int nx = i + ns - 1, sl = slot == 0 ? ns - 1 : slot - 1;

@@ -597,7 +597,7 @@ __global__ void __launch_bounds__(160) ps_k_matmul_mt(const PsMtArgs a) {
         uint32_t phase = 0;
         for (int u = blockIdx.x; u < a.n_units; u += gridDim.x)
             for (int k = 0; k < n_st; k++, n++) {
-                if (n >= ns && !ps_tc_wait_warp(&bar_empty[slot], phase ^ 1)) *a.err = PS_ERR_COPY;
+                if (n >= ns && !ps_tc_wait_warp(&bar_empty[slot], phase ^ 1, PS_COPY_CYCLES)) *a.err = PS_ERR_COPY;
                 if (ps_elect_one()) {
                     if (n >= ahead) weights(u, k, slot);
                     columns(u, k, slot);
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(160) ps_k_matmul_mt(const PsMtArgs a) {
         for (int k = 0; k < n_st; k++) {
             // after a wait that gave up the results are invalid; the loop goes on and waits for the other copies, each within its limit, so that none is in
             // flight when this shared memory becomes another CTA's
-            if (!ps_tc_wait(&bar_full[slot], phase)) *a.err = PS_ERR_COPY;
+            if (!ps_tc_wait(&bar_full[slot], phase, PS_COPY_POLLS)) *a.err = PS_ERR_COPY;
             const uint8_t *st = ps_mt_smem + (size_t)slot * STAGE;
             auto group = [&](int g) {
                 const uint8_t *sw = st + g * WREC;

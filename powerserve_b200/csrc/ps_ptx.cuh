@@ -90,14 +90,18 @@ PS_D bool ps_tc_poll(uint32_t bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity) {
-    for (int spin = 0; spin < (1 << 18); spin++)
+PS_D bool ps_tc_wait(uint64_t *bar, uint32_t parity, int polls = 1 << 18) {
+    for (int spin = 0; spin < polls; spin++)
         if (ps_tc_poll(ps_smem_u32(bar), parity)) return true;
     return false;
 }
 // the same by a converged warp that goes on together: giving up is the warp's decision, not a lane's (elect.sync and the .aligned tcgen05
 // instructions that follow need all lanes).  The limit is a time here, 2^31 SM cycles unless a test asks for less
 #define PS_TC_WAIT_CYCLES 0x80000000u
+// limits where a block goes on after a wait that gave up, and meets the slot of the missing copy again dozens of times: some 30 ms, so that all of them together end
+// within seconds (a copy takes microseconds; a flag that ended the later waits at once cost the kernels 2 to 16 %)
+#define PS_COPY_POLLS (1 << 13)
+#define PS_COPY_CYCLES (1u << 26)
 PS_D uint32_t ps_clock32() {
     uint32_t t;
     asm volatile("mov.u32 %0, %%clock;" : "=r"(t));

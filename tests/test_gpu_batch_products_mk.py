@@ -81,8 +81,7 @@ def test_scales_that_are_not_finite(be, t):
 
 
 @pytest.mark.parametrize("t", TYPES)
-@pytest.mark.parametrize("warp", [0, 3])
-def test_a_warp_that_gives_up_is_reported(be, t, warp):
+def test_a_copy_that_does_not_arrive_is_reported(be, t):
     """a product of the operator table whose copies did not arrive: whoever waits for it or fetches it is told, once, and the next product has all bits"""
     K, N, bs = 512, 40, 6
     rng = np.random.default_rng(t)
@@ -92,14 +91,14 @@ def test_a_warp_that_gives_up_is_reported(be, t, warp):
     L.oracle().ps_or_matmul(t, L.vptr(w), K, N, L.fptr(x), bs, L.fptr(ref))
     wd, xd, dd = be.register_weight(w, t, K, N), be.upload(x), be.empty(N * bs)
     for ask in (dd.numpy, be.sync):
-        be.set_option("give_up_warp", warp)
+        be.set_option("give_up_warp", 0)
         be.matmul(dd, wd, t, K, N, xd, bs)
         with pytest.raises(capi.PsCudaError, match="copy of a batch product"):
             ask()
         be.set_option("give_up_warp", -1)
         be.sync()
         be.matmul(dd, wd, t, K, N, xd, bs)
-        L.assert_bit_equal(dd.numpy(), ref, f"type {t}, after warp {warp} gave up")
+        L.assert_bit_equal(dd.numpy(), ref, f"type {t}, after a failure")
     xd.free()
     dd.free()
     be.unregister_weight(w)
