@@ -4,6 +4,7 @@ is computed in Python, and there is NO fallback — a missing library or device 
 """
 from __future__ import annotations
 
+import atexit
 import ctypes as C
 import json
 import os
@@ -206,14 +207,58 @@ def _i32(a: Sequence[int]) -> np.ndarray:
     return np.ascontiguousarray(np.asarray(a, dtype=np.int32))
 
 
+class _PinnedStore:
+    """Page-locked buffers that no model is using, for all models of the process.  Locking pages takes milliseconds (1 to 4 for 2 MB, 7 to 20 for 16 MB), so a buffer goes from a
+    model that is closed, or has outgrown it, to the next one; sizes go up by factors of two, so that a batch that grows asks for few.  At most four buffers and 32 MB lie here;
+    they are given back when the process ends."""
+    MOST, BYTES = 4, 32 << 20
+    # (1.75 MB, not 2: with what a context locks anyway that fits the 2 MB that the driver locks at a time, and the first call of a model of that size takes 0.7 ms where it took 3.7)
+    SIZES = [64 << 10, 128 << 10, 256 << 10, 512 << 10, 1 << 20, 7 << 18, 4 << 20, 8 << 20, 16 << 20]
+
+    def __init__(self):
+        self.lock, self.idle = threading.RLock(), []    # one lock for the store and its users (an array's finalizer may run inside any of them)
+
+    def take(self, L, n: int):
+        with self.lock:
+            fit = min((b for b in self.idle if b[1] >= n), key=lambda b: b[1], default=None)
+            if fit is not None:
+                self.idle.remove(fit)
+                return fit
+        size, p = next(s for s in self.SIZES if s >= n), C.c_void_p()
+        return (p.value, size) if L.ps_cuda_host_alloc(size, C.byref(p)) == 0 else None
+
+    def give(self, L, buf):
+        with self.lock:
+            if len(self.idle) < self.MOST and sum(b[1] for b in self.idle) + buf[1] <= self.BYTES:
+                self.idle.append(buf)
+                return
+        L.ps_cuda_host_free(buf[0])
+
+    def clear(self, L):
+        with self.lock:
+            rest, self.idle = self.idle, []
+        for b in rest:
+            L.ps_cuda_host_free(b[0])
+
+
+_pinned = _PinnedStore()
+
+
+@atexit.register
+def _give_back(pid=os.getpid()):
+    if _lib is not None and os.getpid() == pid:     # (not in a forked child)
+        _pinned.clear(_lib)
+
+
 class _LogitsPool:
     """Page-locked buffers behind the logits arrays that a model hands out: the device writes them directly (a pageable array takes a second copy on the
-    host, 150 us for 1.6 MB).  At most two buffers of at most 16 MB; an array's buffer comes back when the array and all its views are gone, and is
-    freed if the model has been closed by then.  Whoever keeps more arrays alive, or larger ones, gets ordinary memory."""
-    MOST, LARGEST = 2, 16 << 20
+    host, 150 us for 1.6 MB).  At most two buffers of at most 16 MB; an array's buffer comes back when the array and all its views are gone, and goes to the
+    store if the model has been closed by then.  Whoever keeps more arrays alive, or larger ones, gets ordinary memory.  (The arrays do not own their
+    memory: ndarray.resize in place needs a copy.)"""
+    MOST, LARGEST = 2, _PinnedStore.SIZES[-1]
 
-    def __init__(self, L):
-        self.L, self.lock, self.free, self.made, self.closed = L, threading.RLock(), [], 0, False  # (a finalizer may run inside)
+    def __init__(self, L, store: _PinnedStore = _pinned):
+        self.L, self.store, self.lock, self.free, self.made, self.closed = L, store, store.lock, [], 0, False
 
     def array(self, rows: int, cols: int) -> np.ndarray:
         n = 4 * rows * cols
@@ -225,33 +270,38 @@ class _LogitsPool:
         return np.frombuffer(mem, np.float32).reshape(rows, cols)
 
     def _take(self, n: int):
+        small = None
         with self.lock:
-            fit = next((b for b in self.free if b[1] >= n), None)
-            if fit is None and (self.made < self.MOST or self.free):
-                if self.made == self.MOST:      # a smaller one makes room
-                    self.L.ps_cuda_host_free(self.free.pop()[0])
-                    self.made -= 1
-                p = C.c_void_p()
-                if self.L.ps_cuda_host_alloc(n, C.byref(p)) == 0:
-                    self.made += 1
-                    return p.value, n
-            elif fit is not None:
+            fit = min((b for b in self.free if b[1] >= n), key=lambda b: b[1], default=None)
+            if fit is not None:
                 self.free.remove(fit)
-            return fit
+                return fit
+            if self.made >= self.MOST:
+                if not self.free:
+                    return None
+                small = self.free.pop()     # makes room
+            else:
+                self.made += 1
+        if small is not None:
+            self.store.give(self.L, small)
+        got = self.store.take(self.L, n)    # (outside the lock: it may take milliseconds)
+        if got is None:
+            with self.lock:
+                self.made -= 1
+        return got
 
     def _give(self, buf):
         with self.lock:
-            if self.closed:
-                self.L.ps_cuda_host_free(buf[0])
-            else:
+            if not self.closed:
                 self.free.append(buf)
+                return
+        self.store.give(self.L, buf)
 
     def close(self):
         with self.lock:
-            self.closed = True
-            for b in self.free:
-                self.L.ps_cuda_host_free(b[0])
-            self.free = []
+            self.closed, rest, self.free = True, self.free, []
+        for b in rest:
+            self.store.give(self.L, b)
 
 
 class DeviceBuffer:
