@@ -182,7 +182,8 @@ int ps_cuda_forward_sessions(ps_cuda_ctx *ctx, const int32_t *session_ids, const
 int ps_cuda_decode_greedy(ps_cuda_ctx *ctx, int32_t first_token, int n_steps, int32_t *ids_host);
 /* page-locked host memory: logits buffers in it (of any of the forward calls above) are written by the device directly, others by way of a
  * staging buffer and a copy on the host.  No context is needed; a buffer may outlive the contexts that wrote to it */
-int ps_cuda_host_alloc(size_t bytes, void **host);
+int ps_cuda_host_alloc(size_t bytes, void **host);                    /* on the calling thread's current device */
+int ps_cuda_host_alloc_on(int device, size_t bytes, void **host);     /* that thread's device stays what it is */
 int ps_cuda_host_free(void *host);
 /* device-side logits of the last forward ([bs][vocab]) for callers that sample on the GPU */
 const float *ps_cuda_logits_dev(ps_cuda_ctx *ctx);

@@ -177,6 +177,7 @@ def load_library() -> C.CDLL:
         "ps_cuda_forward_sessions": (ci, [vp, i32p, i32p, ci, ci, fp, i32p]),
         "ps_cuda_logits_dev": (vp, [vp]),
         "ps_cuda_host_alloc": (ci, [C.c_size_t, C.POINTER(vp)]),
+        "ps_cuda_host_alloc_on": (ci, [ci, C.c_size_t, C.POINTER(vp)]),
         "ps_cuda_host_free": (ci, [vp]),
         "ps_cuda_tp_unique_id": (ci, [vp]),
         "ps_cuda_tp_init": (ci, [vp, vp]),
@@ -218,14 +219,14 @@ class _PinnedStore:
     def __init__(self):
         self.lock, self.idle = threading.RLock(), []    # one lock for the store and its users (an array's finalizer may run inside any of them)
 
-    def take(self, L, n: int):
+    def take(self, L, n: int, device: int = 0):
         with self.lock:
             fit = min((b for b in self.idle if b[1] >= n), key=lambda b: b[1], default=None)
             if fit is not None:
                 self.idle.remove(fit)
                 return fit
         size, p = next(s for s in self.SIZES if s >= n), C.c_void_p()
-        return (p.value, size) if L.ps_cuda_host_alloc(size, C.byref(p)) == 0 else None
+        return (p.value, size) if L.ps_cuda_host_alloc_on(device, size, C.byref(p)) == 0 else None
 
     def give(self, L, buf):
         with self.lock:
@@ -257,7 +258,8 @@ class _LogitsPool:
     memory: ndarray.resize in place needs a copy.)"""
     MOST, LARGEST = 2, _PinnedStore.SIZES[-1]
 
-    def __init__(self, L, store: _PinnedStore = _pinned):
+    def __init__(self, L, store: _PinnedStore = _pinned, device: int = 0):
+        self.device = device    # (the calling thread may have chosen none yet: its memory would then be made on device 0, with a context there)
         self.L, self.store, self.lock, self.free, self.made, self.closed = L, store, store.lock, [], 0, False
 
     def array(self, rows: int, cols: int) -> np.ndarray:
@@ -284,7 +286,7 @@ class _LogitsPool:
                 self.made += 1
         if small is not None:
             self.store.give(self.L, small)
-        got = self.store.take(self.L, n)    # (outside the lock: it may take milliseconds)
+        got = self.store.take(self.L, n, self.device)    # (outside the lock: it may take milliseconds)
         if got is None:
             with self.lock:
                 self.made -= 1
@@ -345,7 +347,7 @@ class CudaBackend:
         if rc != 0:
             raise PsCudaError(f"ps_cuda_create failed ({rc}): {self.L.ps_cuda_last_error(None).decode()}")
         self.h = h
-        self.logits_pool = _LogitsPool(self.L)
+        self.logits_pool = _LogitsPool(self.L, device=device)
 
     def _ck(self, rc: int):
         if rc != 0:

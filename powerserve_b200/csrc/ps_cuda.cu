@@ -17,6 +17,7 @@
 #include <initializer_list>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <unordered_map>
 #include <unordered_set>
 #include <vector>
@@ -1520,6 +1521,21 @@ int run_step(ps_cuda_ctx *ctx, bool pick, int n_kv_max) {
     return 0;
 }
 
+
+// page-locked memory belongs to the device it was made on: for another than the calling thread's a helper thread makes and frees it, since a context of the
+// caller's device must not come into being by it, nor that device change
+std::mutex g_host_mu;
+std::unordered_map<void *, int> g_host_device;
+template <typename F> cudaError_t on_device(int device, F f) {
+    int cur = -1;
+    if (cudaGetDevice(&cur) == cudaSuccess && cur == device) return f();
+    cudaError_t e = cudaErrorUnknown;
+    try {
+        std::thread([&] { e = cudaSetDevice(device); if (e == cudaSuccess) e = f(); }).join();
+    } catch (...) {
+    }
+    return e;
+}
 } // namespace
 
 
@@ -1802,14 +1818,48 @@ void ps_cuda_destroy(ps_cuda_ctx *ctx) {
     delete ctx;
 }
 
-int ps_cuda_host_alloc(size_t bytes, void **host) {
+int ps_cuda_host_alloc_on(int device, size_t bytes, void **host) {
     if (!host) return fail(nullptr, PS_CUDA_ERR_INVALID, "null argument");
-    const cudaError_t e = cudaHostAlloc(host, bytes ? bytes : 16, cudaHostAllocPortable);
-    return e == cudaSuccess ? 0 : fail(nullptr, PS_CUDA_ERR_OOM, "cudaHostAlloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+    *host = nullptr;
+    int n = 0;
+    if (cudaGetDeviceCount(&n) != cudaSuccess || device < 0 || device >= n) {
+        cudaGetLastError();
+        return fail(nullptr, PS_CUDA_ERR_INVALID, "host_alloc: device %d out of range [0,%d)", device, n);
+    }
+    void *p = nullptr;
+    const cudaError_t e = on_device(device, [&] { return cudaHostAlloc(&p, bytes ? bytes : 16, cudaHostAllocPortable); });
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(nullptr, PS_CUDA_ERR_OOM, "cudaHostAlloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
+    }
+    try {
+        std::lock_guard<std::mutex> lock(g_host_mu);
+        g_host_device[p] = device;
+    } catch (...) { // (without the note it is freed on the caller's device)
+    }
+    *host = p;
+    return 0;
+}
+int ps_cuda_host_alloc(size_t bytes, void **host) {
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        cudaGetLastError();
+        return fail(nullptr, PS_CUDA_ERR_NO_DEVICE, "host_alloc: no CUDA device");
+    }
+    return ps_cuda_host_alloc_on(device, bytes, host);
 }
 int ps_cuda_host_free(void *host) {
-    const cudaError_t e = cudaFreeHost(host);
-    return e == cudaSuccess ? 0 : fail(nullptr, PS_CUDA_ERR_CUDA, "cudaFreeHost failed: %s", cudaGetErrorString(e));
+    int device = -1;
+    {
+        std::lock_guard<std::mutex> lock(g_host_mu);
+        const auto it = g_host_device.find(host);
+        if (it != g_host_device.end()) { device = it->second; g_host_device.erase(it); }
+    }
+    if (device < 0 && cudaGetDevice(&device) != cudaSuccess) device = 0;
+    const cudaError_t e = on_device(device, [&] { return cudaFreeHost(host); });
+    if (e == cudaSuccess) return 0;
+    cudaGetLastError();
+    return fail(nullptr, PS_CUDA_ERR_CUDA, "cudaFreeHost failed: %s", cudaGetErrorString(e));
 }
 
 // (a failure that a kernel of the operator table has flagged is reported here or by the copy that fetches its result; the lock: a forward pass in another

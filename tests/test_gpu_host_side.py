@@ -2,6 +2,7 @@
 same call into memory of the caller's, and the same operations on one cache; tolerance zero."""
 import ctypes as C
 import gc
+import threading
 
 import numpy as np
 import pytest
@@ -97,3 +98,24 @@ def test_slots_after_a_switch(model):
     model.session_destroy(sids[0])
     with pytest.raises(capi.PsCudaError, match="unknown session"):
         model.session_select(sids[0])
+
+
+def test_page_locked_memory_of_any_thread(model):
+    """made and freed by threads that have chosen no device; what is no such memory, or no device, is refused"""
+    lib, got = model.be.L, []
+
+    def make():
+        p = C.c_void_p()
+        got.append((lib.ps_cuda_host_alloc_on(0, 4096, C.byref(p)), p.value))
+
+    def free():
+        got.append(lib.ps_cuda_host_free(got[0][1]))
+
+    for f in (make, free, free):
+        t = threading.Thread(target=f)
+        t.start()
+        t.join()
+    assert got[0][0] == 0 and got[1] == 0 and got[2] != 0
+    p = C.c_void_p()
+    assert lib.ps_cuda_host_alloc_on(99, 4096, C.byref(p)) != 0 and lib.ps_cuda_host_alloc_on(-1, 4096, C.byref(p)) != 0 and not p.value
+    assert len(model.forward(synth.random_prompt(1000, 3, seed=9))) == 3    # (an error of those calls is not the next one's)

@@ -13,9 +13,10 @@ class FakeLib:
     """page-locked memory of ordinary memory"""
 
     def __init__(self):
-        self.live, self.made, self.fail = {}, 0, False
+        self.live, self.made, self.fail, self.devices = {}, 0, False, []
 
-    def ps_cuda_host_alloc(self, n, out):
+    def ps_cuda_host_alloc_on(self, device, n, out):
+        self.devices.append(device)
         if self.fail:
             return 2
         b = C.create_string_buffer(n)
@@ -129,3 +130,13 @@ def test_threads():
     handed.clear()
     gc.collect()
     assert len(L.live) == len(store.idle) <= store.MOST
+
+
+def test_buffers_are_made_on_the_models_device():
+    """whatever device the calling thread has chosen, or none"""
+    L, store = FakeLib(), capi._PinnedStore()
+    got = []
+    t = threading.Thread(target=lambda: got.append(capi._LogitsPool(L, store, device=3).array(4, 100)))
+    t.start()
+    t.join()
+    assert pinned(got[0]) and L.devices == [3]
