@@ -313,13 +313,21 @@ int stage_call(ps_cuda_ctx *ctx, int bs, bool tree = false) {
     ctx->h2d += (int64_t)bytes;
     return 0;
 }
-// logits of the last pass to the caller; synchronises and checks.  Pinned memory of the caller's is written directly, other memory by way of a pinned
+// logits of the last pass to the caller; synchronises and checks.  Pinned memory of the caller's is written directly, other memory (of which a part may be pinned) by way of a pinned
 // buffer and a copy on the host, which for a few MB takes longer than the transfer (1.6 MB: 150 us and 30)
 int logits_to_host(ps_cuda_ctx *ctx, float *host, size_t bytes) {
-    cudaPointerAttributes at{};
-    const bool direct = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost;
-    if (!direct) {
+    auto locked = [](const void *p) {
+        cudaPointerAttributes at{};
+        if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeHost;
         cudaGetLastError();
+        return false;
+    };
+    bool direct = locked(host) && locked(reinterpret_cast<char *>(host) + bytes - 1);
+    if (direct && cudaMemcpyAsync(host, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess) { // locked at its ends alone, or in pieces
+        cudaGetLastError();
+        direct = false;
+    }
+    if (!direct) {
         if (bytes > ctx->h_logits_cap) {
             if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
             ctx->h_logits = nullptr;
@@ -327,8 +335,8 @@ int logits_to_host(ps_cuda_ctx *ctx, float *host, size_t bytes) {
             PS_CK(cudaMallocHost(&ctx->h_logits, bytes));
             ctx->h_logits_cap = bytes;
         }
+        PS_CK(cudaMemcpyAsync(ctx->h_logits, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     }
-    PS_CK(cudaMemcpyAsync(direct ? host : ctx->h_logits, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     const int rc = sync_and_check(ctx);
     if (rc) return rc;
     if (!direct) memcpy(host, ctx->h_logits, bytes);

@@ -119,3 +119,29 @@ def test_page_locked_memory_of_any_thread(model):
     p = C.c_void_p()
     assert lib.ps_cuda_host_alloc_on(99, 4096, C.byref(p)) != 0 and lib.ps_cuda_host_alloc_on(-1, 4096, C.byref(p)) != 0 and not p.value
     assert len(model.forward(synth.random_prompt(1000, 3, seed=9))) == 3    # (an error of those calls is not the next one's)
+
+
+@pytest.mark.parametrize("pinned", [[(0, 1)], [(1, 1)], [(0, 1), (2, 1)], [(0, 1), (1, 1), (2, 1)], [(0, 3)]])
+def test_arrays_of_which_a_part_is_page_locked(model, pinned):
+    """three pages of a caller's: the first, the middle one, the ends, all in three pieces, all in one piece"""
+    import torch
+
+    rt, toks = torch.cuda.cudart(), synth.random_prompt(1000, 3, seed=3)
+    want = model.forward(toks)
+    raw = np.zeros(5 * 4096, np.uint8)
+    lo = -raw.ctypes.data % 4096
+    out = raw[lo:lo + 12000].view(np.float32)       # 3 x 1000 logits in three pages
+    torch.cuda.init()
+    done = []
+    try:
+        for page, n in pinned:
+            assert int(rt.cudaHostRegister(out.ctypes.data + 4096 * page, 4096 * n, 0)) == 0
+            done.append(out.ctypes.data + 4096 * page)
+        model.reset()
+        t, p = np.asarray(toks, np.int32), np.arange(3, dtype=np.int32)
+        i32p = C.POINTER(C.c_int32)
+        model.be._ck(model.be.L.ps_cuda_forward(model.be.h, t.ctypes.data_as(i32p), p.ctypes.data_as(i32p), 3, 1, out.ctypes.data))
+        L.assert_bit_equal(out.reshape(3, 1000), want, str(pinned))
+    finally:
+        for at in done:
+            rt.cudaHostUnregister(at)
