@@ -1114,7 +1114,7 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
             if (count) return 0;
             int r = aalloc(a, (void **)dst, (size_t)groups * n_rt * nkb * PT_BLOCK, err);
             if (r) return r;
-            pa_k_tc_tile_w<<<dim3((unsigned)nkb, (unsigned)n_rt, (unsigned)groups), 256, 0, stream>>>(*dst, src, N, K, n_rt, nkb, odd);
+            pa_k_tc_tile_w<<<dim3((unsigned)n_rt, (unsigned)nkb, (unsigned)groups), 256, 0, stream>>>(*dst, src, N, K, n_rt, nkb, odd);
             PA_CK(cudaGetLastError());
             return 0;
         };
@@ -1135,7 +1135,7 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
                 if ((rc = aalloc(a, (void **)&w.t_qkv, (size_t)w.seg.rt[w.seg.n] * nkb * PT_BLOCK, err))) return rc;
                 for (int k = 0; k < w.seg.n; k++) {
                     const int n = w.seg.row[k + 1] - w.seg.row[k], n_rt = w.seg.rt[k + 1] - w.seg.rt[k];
-                    pa_k_tc_tile_w<<<dim3((unsigned)nkb, (unsigned)n_rt, 1), 256, 0, stream>>>(w.t_qkv + (size_t)w.seg.rt[k] * nkb * PT_BLOCK, w.wqkv + (size_t)w.seg.row[k] * d.dim, n, d.dim, n_rt, nkb, nullptr);
+                    pa_k_tc_tile_w<<<dim3((unsigned)n_rt, (unsigned)nkb, 1), 256, 0, stream>>>(w.t_qkv + (size_t)w.seg.rt[k] * nkb * PT_BLOCK, w.wqkv + (size_t)w.seg.row[k] * d.dim, n, d.dim, n_rt, nkb, nullptr);
                     PA_CK(cudaGetLastError());
                 }
             } else if ((rc = tile(&w.t_qkv, w.wqkv, 1, w.pw, d.dim))) {

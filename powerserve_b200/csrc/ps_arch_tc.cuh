@@ -24,7 +24,7 @@
 // weights [groups][N][K] bf16 row-major -> blocks [group][row tile][k block][k-chunk 8][row 128][8]; zero outside N x K
 // odd (or null): set if a weight is an infinity or no number
 __global__ void __launch_bounds__(256) pa_k_tc_tile_w(uint8_t *__restrict__ dst, const bf16 *__restrict__ w, int N, int K, int n_rt, int nkb, int *__restrict__ odd) {
-    const int kb = blockIdx.x, rt = blockIdx.y, grp = blockIdx.z;
+    const int kb = blockIdx.y, rt = blockIdx.x, grp = blockIdx.z; // (y ends at 65 535)
     const bf16 *src = w + (int64_t)grp * N * K;
     uint8_t *out = dst + (((int64_t)grp * n_rt + rt) * nkb + kb) * PT_BLOCK;
     for (int c = threadIdx.x; c < 128 * 8; c += 256) {

@@ -639,7 +639,7 @@ int matmul_mt(ps_cuda_ctx *ctx, const ActIn &in, int64_t K, int bs, std::initial
     return ctx->mv_type == 2 ? launch_mt_t<2>(ctx, a) : launch_mt_t<8>(ctx, a);
 }
 int mt_pack(ps_cuda_ctx *ctx, uint8_t *dst, const uint8_t *w, int64_t rows, int64_t K) {
-    const dim3 grid((unsigned)((K / 32 + 3) / 4), (unsigned)((rows + 15) / 16));
+    const dim3 grid((unsigned)((rows + 15) / 16), (unsigned)((K / 32 + 3) / 4));
     if (ctx->mv_type == 2) ps_k_mt_pack<2><<<grid, 128, 0, ctx->stream>>>(dst, w, rows, K / 32);
     else ps_k_mt_pack<8><<<grid, 128, 0, ctx->stream>>>(dst, w, rows, K / 32);
     PS_LAUNCH_CK();

@@ -479,10 +479,10 @@ __global__ void __launch_bounds__(PS_MB_WARPS * 32) ps_k_matmul_ob(const PsMbArg
 template <int TYPE> PS_HD constexpr int ps_mt_wq() { return TYPE == 2 ? 1024 : 2048; }
 template <int TYPE> PS_HD constexpr int ps_mt_wrec() { return ps_mt_wq<TYPE>() + 256; }
 PS_HD size_t ps_mt_w_bytes(int type, int64_t rows, int64_t K) { return (size_t)((rows + 15) / 16) * (size_t)((K / 32 + 3) / 4) * (type == 2 ? ps_mt_wrec<2>() : ps_mt_wrec<8>()); }
-template <int TYPE> __global__ void __launch_bounds__(128) ps_k_mt_pack(uint8_t *__restrict__ dst, const uint8_t *__restrict__ w, int64_t n_rows, int64_t nb) { // grid (groups, tiles)
+template <int TYPE> __global__ void __launch_bounds__(128) ps_k_mt_pack(uint8_t *__restrict__ dst, const uint8_t *__restrict__ w, int64_t n_rows, int64_t nb) { // grid (tiles, groups): y ends at 65 535
     constexpr int SRC = PsMv32<TYPE>::SRC;
-    const int64_t g4 = blockIdx.x, tile = blockIdx.y;
-    uint8_t *out = dst + (tile * gridDim.x + g4) * ps_mt_wrec<TYPE>();
+    const int64_t g4 = blockIdx.y, tile = blockIdx.x;
+    uint8_t *out = dst + (tile * gridDim.y + g4) * ps_mt_wrec<TYPE>();
     const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31, t = lane & 3;
     for (int r = 0; r < 2; r++) {
         const int64_t row = tile * 16 + r * 8 + (lane >> 2);

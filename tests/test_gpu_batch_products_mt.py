@@ -37,3 +37,16 @@ def test_columns(pair, n):
         cm.reset()
         L.assert_bit_equal(cm.forward(tokens), want, f"{n} tokens, mt_min {mt_min}")
     cm.be.set_option("mt_min", 2)
+
+
+def test_more_than_a_million_rows(tmp_path):
+    """a head of 65 535 x 16 rows and more: a launch's y and z end at 65 535"""
+    vocab = 65535 * 16 + 1000
+    shape = synth.ModelShape("mt-rows", "llama", 64, 64, 1, 2, 2, 32, vocab, True, 0, 1e4, 1e-5, gguf.GGML_Q4_0, n_ctx=32)
+    d = synth.write_model_dir(str(tmp_path), shape, seed=8)
+    om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=4)
+    assert cm.be.counter("mv32_ok") == 1
+    tokens = synth.random_prompt(vocab, 3, seed=1)
+    L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), "3 tokens")
+    om.close()
+    cm.close()
