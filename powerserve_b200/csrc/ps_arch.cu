@@ -99,6 +99,7 @@ struct PsArch {
     ps_cuda_arch_desc d{};
     std::vector<PsArchLayer> L;
     std::vector<void *> owned;
+    std::vector<void *> spare; // of them, the operand blocks of float32 mode
     bool bound = false, round = true;
     bf16 *embed = nullptr, *head = nullptr;
     float *final_norm = nullptr;
@@ -186,6 +187,10 @@ int afail(std::string &err, int code, const char *fmt, ...) {
 int aalloc(PsArch *a, void **p, size_t bytes, std::string &err) {
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        if (ps_give_back_others(a) && (e = cudaMalloc(p, bytes)) != cudaSuccess) cudaGetLastError();
+    }
     if (e != cudaSuccess) return afail(err, PS_CUDA_ERR_OOM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
     a->owned.push_back(*p);
     return 0;
@@ -741,6 +746,19 @@ void ps_arch_destroy(PsArch *a) {
     delete a;
 }
 
+bool ps_arch_tiled(const PsArch *a) { return a->tiled; }
+bool ps_arch_give_back(PsArch *a, cudaStream_t stream) {
+    if (a->spare.empty()) return false;
+    cudaStreamSynchronize(stream);
+    for (void *p : a->spare) {
+        a->owned.erase(std::find(a->owned.begin(), a->owned.end(), p));
+        cudaFree(p);
+    }
+    a->spare.clear();
+    a->tiled = false; // (the layers' pointers to them are followed on that condition alone)
+    return true;
+}
+
 size_t ps_arch_k_bytes(const PsArch *a, int layer) {
     const PsArchLayer &w = a->L[(size_t)layer];
     return 4 * (w.k_floats ? (size_t)w.k_floats : (size_t)w.kd * (size_t)a->d.n_ctx);
@@ -1098,6 +1116,7 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
     // tensor-core operand blocks: every matrix once more in the layout the tcgen05 GEMMs stream (ps_arch_tc.cuh).  In float32 mode, whose FMA tiles can do without,
     // a first trip counts the bytes
     size_t need = 0;
+    bool full = false; // float32 mode: the memory was taken meanwhile
     int *odd = nullptr; // float32 mode: a weight that is not finite (its zero parts would turn an infinity into no number)
     for (int trip = a->round ? 1 : 0; trip < 2; trip++) {
         const bool count = trip == 0;
@@ -1111,9 +1130,11 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
         auto tile = [&](uint8_t **dst, const bf16 *src, int groups, int N, int K) -> int {
             const int n_rt = (N + PT_M - 1) / PT_M, nkb = (K + PT_KB - 1) / PT_KB;
             need += (size_t)groups * n_rt * nkb * PT_BLOCK;
-            if (count) return 0;
+            if (count || full) return 0;
             int r = aalloc(a, (void **)dst, (size_t)groups * n_rt * nkb * PT_BLOCK, err);
+            if (r && !a->round) { full = true; return 0; }
             if (r) return r;
+            if (!a->round) a->spare.push_back(*dst);
             pa_k_tc_tile_w<<<dim3((unsigned)n_rt, (unsigned)nkb, (unsigned)groups), 256, 0, stream>>>(*dst, src, N, K, n_rt, nkb, odd);
             PA_CK(cudaGetLastError());
             return 0;
@@ -1158,7 +1179,8 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
         PA_CK(cudaStreamSynchronize(stream));
         int any = 0;
         if (odd) PA_CK(cudaMemcpy(&any, odd, 4, cudaMemcpyDeviceToHost));
-        a->tiled = !any;
+        a->tiled = true;
+        if (any || full) ps_arch_give_back(a, stream);
     }
     for (int i = 0; i < d.n_layers; i++) { // repeated runs: the first run's weights under the run's own description
         PsArchLayer &w = a->L[(size_t)i];

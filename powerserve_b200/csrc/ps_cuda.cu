@@ -11,6 +11,7 @@
 
 #include <dlfcn.h>
 
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -154,7 +155,7 @@ struct ps_cuda_ctx {
     int mv_type = 0;
     uint8_t *mv_out = nullptr;
     bool mt_ok = false;      // weight records of ps_k_matmul_mt are resident
-    uint8_t *mt_out = nullptr, *mt_x = nullptr; // lm_head; activation records of a batch (at the end of the same allocation)
+    uint8_t *mt_mem = nullptr, *mt_out = nullptr, *mt_x = nullptr; // their memory; lm_head's; activation records of a batch (at its end)
     bool ops_graph_ok = false; // any supported mix of weight types: the graph-replayed operator-table decode step applies (decode_step_ops)
     int opt_ops_graph = 1;
     int n_sm = 148;
@@ -249,12 +250,54 @@ int fail(ps_cuda_ctx *c, int code, const char *fmt, ...) {
         if (ctx->arch) return fail(ctx, PS_CUDA_ERR_UNSUPPORTED, what ": not available on a layer-list context"); \
     } while (0)
 
+// Second copies of weights that only make batches faster (the 32-block models' records, a float32 layer list's operand blocks) yield to memory that is asked for
+// later - sessions, further models - on the same device: the batches then take the kernels that do without.  ctx->mu is held
+bool give_back(ps_cuda_ctx *ctx) {
+    bool given = false;
+    if (ctx->mt_mem) {
+        cudaStreamSynchronize(ctx->stream);
+        ctx->owned.erase(std::find(ctx->owned.begin(), ctx->owned.end(), (void *)ctx->mt_mem));
+        given = cudaFree(ctx->mt_mem) == cudaSuccess;
+        ctx->mt_mem = nullptr;
+        ctx->mt_ok = false;
+    }
+    return (ctx->arch && ps_arch_give_back(ctx->arch, ctx->stream)) || given;
+}
+std::mutex g_ctx_mu; // (taken before a context's own, which is only tried: a context at work keeps what it has)
+std::vector<ps_cuda_ctx *> g_ctxs;
+void enlist(ps_cuda_ctx *ctx) {
+    std::lock_guard<std::mutex> lock(g_ctx_mu);
+    try { g_ctxs.push_back(ctx); } catch (...) { } // (it keeps what it has)
+}
+bool give_back_others(const ps_cuda_ctx *self, const PsArch *self_arch) {
+    int device = -1;
+    cudaGetDevice(&device);
+    std::lock_guard<std::mutex> lock(g_ctx_mu);
+    bool given = false;
+    for (ps_cuda_ctx *c : g_ctxs) {
+        if (c == self || c->device != device || (self_arch && c->arch == self_arch)) continue;
+        std::unique_lock<std::mutex> own(c->mu, std::try_to_lock);
+        if (own.owns_lock()) given |= give_back(c);
+    }
+    return given;
+}
+
 int dev_alloc(ps_cuda_ctx *ctx, void **p, size_t bytes) {
     if (bytes == 0) bytes = 16;
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError(); // (or the next launch would seem to have failed)
+        if (give_back_others(ctx, nullptr) && (e = cudaMalloc(p, bytes)) != cudaSuccess) cudaGetLastError();
+    }
     if (e != cudaSuccess) return fail(ctx, PS_CUDA_ERR_OOM, "cudaMalloc(%zu) failed: %s", bytes, cudaGetErrorString(e));
     ctx->owned.push_back(*p);
     return 0;
+}
+// of a call that holds ctx->mu: its own copies yield too
+int dev_alloc_yield(ps_cuda_ctx *ctx, void **p, size_t bytes) {
+    int rc = dev_alloc(ctx, p, bytes);
+    if (rc == PS_CUDA_ERR_OOM && give_back(ctx)) rc = dev_alloc(ctx, p, bytes);
+    return rc;
 }
 
 // Failures detected on the device (tcgen05 pipeline or copy time-out, a peer wait or a grid barrier that gave up) become a C-ABI
@@ -1545,6 +1588,9 @@ template <typename F> cudaError_t on_device(int device, F f) {
     return e;
 }
 } // namespace
+bool ps_give_back_others(const PsArch *self) { return give_back_others(nullptr, self); }
+namespace {
+} // namespace
 
 
 // ====================================================================================================================
@@ -1724,6 +1770,7 @@ int ps_cuda_create(ps_cuda_ctx **out, int device, const ps_cuda_model_desc *desc
     PS_CKC(cudaStreamSynchronize(ctx->stream));
 #undef PS_CKC
 #undef PS_AL
+    enlist(ctx);
     *out = ctx;
     return 0;
 }
@@ -1775,6 +1822,7 @@ int ps_cuda_create_arch(ps_cuda_ctx **out, int device, const ps_cuda_arch_desc *
     if ((rc = ck(cudaEventCreate(&ctx->ev0), "cudaEventCreate")) || (rc = ck(cudaEventCreate(&ctx->ev1), "cudaEventCreate")) ||
         (rc = ck(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize")))
         return bail(rc);
+    enlist(ctx);
     *out = ctx;
     return 0;
 }
@@ -1804,6 +1852,10 @@ int ps_cuda_arch_tap(ps_cuda_ctx *ctx, int layer, float *host, int bs) {
 
 void ps_cuda_destroy(ps_cuda_ctx *ctx) {
     if (!ctx) return;
+    {
+        std::lock_guard<std::mutex> lock(g_ctx_mu);
+        g_ctxs.erase(std::remove(g_ctxs.begin(), g_ctxs.end(), ctx), g_ctxs.end());
+    }
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     for (void *p : ctx->pooled) cudaFreeAsync(p, ctx->stream);
@@ -1895,6 +1947,15 @@ int ps_cuda_malloc(ps_cuda_ctx *ctx, size_t bytes, void **dev) {
     }
     *dev = nullptr;
     cudaError_t e = cudaMallocAsync(dev, std::max<size_t>(bytes, 256), ctx->stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        bool given = give_back_others(ctx, nullptr);
+        {
+            std::lock_guard<std::mutex> lock(ctx->mu);
+            given |= give_back(ctx);
+        }
+        if (given && (e = cudaMallocAsync(dev, std::max<size_t>(bytes, 256), ctx->stream)) != cudaSuccess) cudaGetLastError();
+    }
     if (e != cudaSuccess) return fail(ctx, PS_CUDA_ERR_OOM, "ps_cuda_malloc(%zu): %s", bytes, cudaGetErrorString(e));
     ctx->pooled.insert(*dev);
     return 0;
@@ -2305,10 +2366,9 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
             size_t need = ps_mt_w_bytes(t0, d.vocab_size, dim) + ps_mt_x_bytes(ctx->maxK, d.max_batch), free_b = 0, total_b = 0;
             need += (size_t)d.n_layers * (ps_mt_w_bytes(t0, qdim, dim) + 2 * ps_mt_w_bytes(t0, kvd, dim) + ps_mt_w_bytes(t0, dim, qdim) + 2 * ps_mt_w_bytes(t0, ffn, dim) + ps_mt_w_bytes(t0, dim, ffn));
             PS_CK(cudaMemGetInfo(&free_b, &total_b));
-            ctx->mt_ok = d.max_batch > 1 && need + ((size_t)8 << 30) < free_b;
-            if (ctx->mt_ok) { // (one allocation: seven a layer took longer than the packing)
-                uint8_t *at = nullptr;
-                if ((rc = dev_alloc(ctx, (void **)&at, need))) return rc;
+            ctx->mt_ok = d.max_batch > 1 && need + ((size_t)8 << 30) < free_b && dev_alloc(ctx, (void **)&ctx->mt_mem, need) == 0; // (one allocation: seven a layer took longer than the packing)
+            if (ctx->mt_ok) {
+                uint8_t *at = ctx->mt_mem;
                 auto rec = [&](uint8_t **p, const uint8_t *w, int64_t rows, int64_t K) -> int {
                     *p = at;
                     at += ps_mt_w_bytes(t0, rows, K);
@@ -2815,16 +2875,29 @@ int ps_cuda_session_create(ps_cuda_ctx *ctx, int *session_id) {
     const size_t bytes = 4 * (size_t)d.n_kv_heads * d.head_size * d.n_ctx;
     ps_cuda_ctx::KvSet ks;
     ks.kc.resize(d.n_layers); ks.vct.resize(d.n_layers);
+    auto undo = [&](int rc) { // what has been allocated goes back
+        std::vector<void *> all(ks.kc.begin(), ks.kc.end());
+        all.insert(all.end(), ks.vct.begin(), ks.vct.end());
+        all.push_back(ks.ptrs_dev);
+        cudaStreamSynchronize(ctx->stream);
+        for (void *p : all) {
+            const auto it = p ? std::find(ctx->owned.begin(), ctx->owned.end(), p) : ctx->owned.end();
+            if (it == ctx->owned.end()) continue;
+            ctx->owned.erase(it);
+            cudaFree(p);
+        }
+        return rc;
+    };
     for (int L = 0; L < d.n_layers; L++) {
         int rc;
         const size_t kb = ctx->arch ? ctx->kv_k_bytes[L] : bytes, vb = ctx->arch ? ctx->kv_v_bytes[L] : bytes; // layer-list models: the layer's own widths
-        if ((rc = dev_alloc(ctx, (void **)&ks.kc[L], kb)) || (rc = dev_alloc(ctx, (void **)&ks.vct[L], vb))) return rc;
+        if ((rc = dev_alloc_yield(ctx, (void **)&ks.kc[L], kb)) || (rc = dev_alloc_yield(ctx, (void **)&ks.vct[L], vb))) return undo(rc);
         PS_CK(cudaMemsetAsync(ks.kc[L], 0, kb, ctx->stream));
         PS_CK(cudaMemsetAsync(ks.vct[L], 0, vb, ctx->stream));
     }
     if (!ctx->arch) {
-        int rc = dev_alloc(ctx, (void **)&ks.ptrs_dev, sizeof(float *) * 2 * (size_t)d.n_layers);
-        if (rc || (rc = kv_table(ctx, ks.ptrs_dev, ks.kc, ks.vct))) return rc;
+        int rc = dev_alloc_yield(ctx, (void **)&ks.ptrs_dev, sizeof(float *) * 2 * (size_t)d.n_layers);
+        if (rc || (rc = kv_table(ctx, ks.ptrs_dev, ks.kc, ks.vct))) return undo(rc);
     }
     ks.slot_mask.assign((size_t)d.n_ctx, 1);
     const int id = ctx->next_session++;
@@ -3241,6 +3314,8 @@ int64_t ps_cuda_get_counter(ps_cuda_ctx *ctx, const char *name) {
     if (!strcmp(name, "step_launches")) return ctx->n_step;          // persistent step-kernel launches
     if (!strcmp(name, "step_ok")) return ctx->step_ok ? 1 : 0;
     if (!strcmp(name, "mv32_ok")) return ctx->mv_ok ? 1 : 0;           // all-Q4_0 / all-Q8_0 model: the fused 32-block decode path is bound
+    if (!strcmp(name, "mt_ok")) return ctx->mt_ok ? 1 : 0;             // and the records of its tensor-core batch products are resident
+    if (!strcmp(name, "arch_tiled")) return ctx->arch && ps_arch_tiled(ctx->arch) ? 1 : 0; // a layer list's operand blocks of the tensor-core products are
     if (!strcmp(name, "fused_ok")) return ctx->fused_ok ? 1 : 0;
     if (!strcmp(name, "attn_clusters")) return ctx->attn_clusters;
     if (!strcmp(name, "step_kernel_ns")) return (int64_t)(ctx->kt_ms * 1e6);   // option "ktime": summed CUDA-event time of the step-kernel launches

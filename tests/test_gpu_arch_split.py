@@ -85,6 +85,7 @@ def test_weights_that_are_not_finite(tmp_path):
     build(d, "vanapel", 264, 200, touch)
     toks = [int(v) for v in np.random.default_rng(1).integers(0, 330, 40)]
     m = arch.load_model(d, dtype="float32", max_batch=64, n_ctx=64)
+    assert m.be.counter("arch_tiled") == 0      # (and the blocks are given back)
     got = []
     for tc in (0, 1):
         m.be.set_option("arch_tc", tc)
