@@ -128,6 +128,8 @@ struct PsArch {
     int max_k = 0;
     int opt_tc = 1;     // batches (bs >= 2) run on the tcgen05 GEMMs; 0 = the fp32-FMA tile kernels (on rounded operands in bfloat16 mode)
     bool tiled = false; // the operand blocks of those GEMMs are resident (float32 mode: if HBM has room and every weight is finite)
+    int64_t n_split = 0; // launches of pa_k_tc_gemm3
+    int opt_smx_rows = 1; // soft-max of a batch in shared memory where that pays; 0 = in place (tests compare the two)
     int opt_simple = 0; // 1: every batch width takes the tiled kernels (the single-token kernels are skipped; tests compare the two)
     int n_sm = 148;
     // single-token step: the experts' gate | up product needs only the router logits, so it runs beside the attention kernels
@@ -747,6 +749,7 @@ void ps_arch_destroy(PsArch *a) {
 }
 
 bool ps_arch_tiled(const PsArch *a) { return a->tiled; }
+int64_t ps_arch_split_launches(const PsArch *a) { return a->n_split; }
 bool ps_arch_give_back(PsArch *a, cudaStream_t stream) {
     if (a->spare.empty()) return false;
     cudaStreamSynchronize(stream);
@@ -776,6 +779,7 @@ int ps_arch_set_option(PsArch *a, const char *name, int value) {
     if (!strcmp(name, "arch_simple")) { a->opt_simple = value; return 1; }
     if (!strcmp(name, "arch_taps")) { a->taps_on = value; return 1; }
     if (!strcmp(name, "arch_tc")) { a->opt_tc = value; return 1; }
+    if (!strcmp(name, "arch_smx_rows")) { a->opt_smx_rows = value; return 1; }
     if (!strcmp(name, "arch_fork")) { a->opt_fork = value; return 1; }
     if (!strcmp(name, "arch_pdl")) { a->opt_pdl = value; return 1; }
     if (!strcmp(name, "arch_mv_cap")) { a->opt_mv_cap = value; return 1; }
@@ -1284,6 +1288,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
                       routed ? a->tile_row0 : nullptr, routed ? a->tile_end : nullptr, row_token, row_w);
         PA_LAUNCH();
         const dim3 grid((unsigned)std::min(a->n_sm, g.n_ct * g.n_rt));
+        a->n_split++;
         auto go = [&](void (*kern)(PtArgs), int smem) { pa_launch_dep(pdl, kern, grid, dim3(PT_THREADS), smem, st, g); };
         if (g.a1) tn == 16 ? go(pa_k_tc_gemm3<2, 16>, Pt3<2, 16>::SMEM) : tn == 32 ? go(pa_k_tc_gemm3<2, 32>, Pt3<2, 32>::SMEM) : go(pa_k_tc_gemm3<2, 64>, Pt3<2, 64>::SMEM);
         else tn == 16 ? go(pa_k_tc_gemm3<1, 16>, Pt3<1, 16>::SMEM) : tn == 32 ? go(pa_k_tc_gemm3<1, 32>, Pt3<1, 32>::SMEM) : go(pa_k_tc_gemm3<1, 64>, Pt3<1, 64>::SMEM);
@@ -1332,7 +1337,7 @@ static int forward_t(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_hea
         if (at.window > 0) cap = std::min(cap, at.window);
         if (at.chunk > 0) cap = std::min(cap, at.chunk);
         const size_t smem = at.mix ? 4 * (size_t)at.H * (pa_mix_ld(at.H) + cap) : 4 * (size_t)8 * cap;
-        if (smem <= PA_SMX_SMEM && (!at.mix || (bs > a->n_sm / 2 && cap >= 512)))
+        if (a->opt_smx_rows && smem <= PA_SMX_SMEM && (!at.mix || (bs > a->n_sm / 2 && cap >= 512)))
             pa_launch_dep(pdl, pa_k_softmax_rows, dim3((unsigned)bs, at.mix ? 1 : cdiv(at.H, 8)), dim3(256), smem, st, at, a->S, io.pos_dev, bs, cap);
         else pa_launch_dep(pdl, pa_k_mix_softmax, dim3(bs), dim3(256), 4 * (size_t)at.H * at.H, st, at, a->S, io.pos_dev, bs);
     };

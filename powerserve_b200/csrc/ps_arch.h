@@ -33,6 +33,7 @@ int ps_arch_forward(PsArch *a, const PsArchIO &io, int bs, int pos0, int lm_head
 float *ps_arch_logits(PsArch *a);
 void ps_arch_set_taps(PsArch *a, int on);
 const float *ps_arch_tap(PsArch *a, int layer); // [max_batch][dim] of the last forward, nullptr when taps are off
+int64_t ps_arch_split_launches(const PsArch *a);           // of pa_k_tc_gemm3
 bool ps_arch_tiled(const PsArch *a);                        // operand blocks of the tensor-core batch products are resident
 bool ps_arch_give_back(PsArch *a, cudaStream_t stream);    // in float32 mode they yield to other memory (true: they have); nothing else uses `a` meanwhile
 bool ps_give_back_others(const PsArch *self);              // the other contexts of the device: whether any gave memory back

@@ -139,6 +139,7 @@ struct ps_cuda_ctx {
     int *h_err = nullptr;      // their memory: mapped host memory, so that reading them after every forward / decode takes no copy (a set flag becomes PS_CUDA_ERR_CUDA)
     int *tc_err_dev = nullptr; // = err_dev + 0 (counter "tc_error")
     int64_t n_tc = 0;          // tcgen05 GEMM launches (counter "tc_gemm_launches")
+    int64_t n_mt = 0, n_mk = 0; // ps_k_matmul_mt, ps_k_matmul_mk ("mt_launches", "mk_launches")
     int64_t n_tc_pp[7] = {};   // by a CTA's share of passes: one, two, more (counters "tc_gemm_pass1", "tc_gemm_pass2", "tc_gemm_pass6")
     std::vector<cudaEvent_t> kt_events; // option "ktime": event pairs around every row-walker mat-vec launch
     size_t kt_used = 0;
@@ -528,6 +529,7 @@ template <int TYPE, int NT> int launch_mk(ps_cuda_ctx *ctx, PsMkArgs a, int row_
     }
     const int cols = ((a.bs + 7) / 8 + NT - 1) / NT, per_sm = std::min(4, (row_tiles * cols + ctx->n_sm - 1) / ctx->n_sm);
     a.ns = std::max(2, std::min(std::min(a.nb + 1, 5), 216 * 1024 / per_sm / STAGE));
+    ctx->n_mk++;
     PS_DEP((ps_k_matmul_mk<TYPE, NT>), dim3((unsigned)row_tiles, (unsigned)cols), 128, (size_t)std::max(a.ns * STAGE, RED), a);
     return 0;
 }
@@ -659,6 +661,7 @@ template <int TYPE, int NT> int launch_mt(ps_cuda_ctx *ctx, PsMtArgs a) {
     const int per_sm = std::min(most, (a.n_units + ctx->n_sm - 1) / ctx->n_sm);
     a.ns = std::max(1, std::min(std::min(PS_MT_MAX_NS, (a.nbg + GS - 1) / GS * ((a.n_units + per_sm * ctx->n_sm - 1) / (per_sm * ctx->n_sm))),
                                 std::min((200 * 1024 - RED) / STAGE, (room / per_sm - RED - 1280) / STAGE)));
+    ctx->n_mt++;
     PS_DEP((ps_k_matmul_mt<TYPE, NT>), (unsigned)std::min(a.n_units, per_sm * ctx->n_sm), 160, (size_t)a.ns * STAGE + RED, a);
     return 0;
 }
@@ -3315,6 +3318,9 @@ int64_t ps_cuda_get_counter(ps_cuda_ctx *ctx, const char *name) {
     if (!strcmp(name, "step_ok")) return ctx->step_ok ? 1 : 0;
     if (!strcmp(name, "mv32_ok")) return ctx->mv_ok ? 1 : 0;           // all-Q4_0 / all-Q8_0 model: the fused 32-block decode path is bound
     if (!strcmp(name, "mt_ok")) return ctx->mt_ok ? 1 : 0;             // and the records of its tensor-core batch products are resident
+    if (!strcmp(name, "mt_launches")) return ctx->n_mt;
+    if (!strcmp(name, "mk_launches")) return ctx->n_mk;
+    if (!strcmp(name, "arch_split_launches")) return ctx->arch ? ps_arch_split_launches(ctx->arch) : 0; // float32 products on the tensor cores
     if (!strcmp(name, "arch_tiled")) return ctx->arch && ps_arch_tiled(ctx->arch) ? 1 : 0; // a layer list's operand blocks of the tensor-core products are
     if (!strcmp(name, "fused_ok")) return ctx->fused_ok ? 1 : 0;
     if (!strcmp(name, "attn_clusters")) return ctx->attn_clusters;

@@ -39,9 +39,12 @@ def test_no_further_from_exact_than_fma(tmp_path, family, width, ff):
         return np.concatenate(out)
 
     err = {}
+    assert m.be.counter("arch_tiled") == 1
     for tc in (0, 1):
         m.be.set_option("arch_tc", tc)
+        launches = m.be.counter("arch_split_launches")
         got = run(150)
+        assert (m.be.counter("arch_split_launches") > launches) == bool(tc)
         e = np.sqrt(((got - want) ** 2).mean(-1)) / np.sqrt((want ** 2).mean(-1))
         assert e.max() < 4e-5
         err[tc] = e.mean()

@@ -38,9 +38,12 @@ def pair(request, tmp_path_factory):
     m.close()
 
 
+@pytest.mark.parametrize("tc", [0, 1])  # the tiles, and the tensor cores, which take these products where their operand blocks are resident
 @pytest.mark.parametrize("cuts", [[150], [64], [65, 31], [33, 2], [32, 128]])
-def test_portions(pair, cuts):
+def test_portions(pair, cuts, tc):
     m, toks, ref = pair
+    m.be.set_option("arch_tc", tc)
+    launches = m.be.counter("arch_split_launches")
     m.reset()
     lo, k, out = 0, 0, []
     while lo < len(toks):
@@ -50,6 +53,7 @@ def test_portions(pair, cuts):
     got = np.concatenate(out)
     err = np.sqrt(((got - ref) ** 2).mean(-1)) / np.maximum(np.sqrt((ref ** 2).mean(-1)), 1e-6)
     assert err.max() < 4e-5, (cuts, err.max())
+    assert (m.be.counter("arch_split_launches") > launches) == bool(tc)
 
 
 @pytest.mark.parametrize("family,width,ff", [("vanapel", 248, 3208), ("pidenex", 248, 3208), ("vanapel", 1032, 264)])

@@ -10,6 +10,7 @@ from tests import _libs as L
 from tests import _model as M
 
 pytestmark = pytest.mark.gpu
+OCTETS = 1000   # option mt_min: no batch is so wide, so that all run on the octet copies, as where the tensor cores' records find no room
 
 
 def _shape(quant, dim, ffn, heads, vocab):
@@ -18,13 +19,14 @@ def _shape(quant, dim, ffn, heads, vocab):
 
 @pytest.mark.parametrize("quant", [gguf.GGML_Q8_0, gguf.GGML_Q4_0])
 def test_a_warp_that_gives_up_ends_the_call(quant, tmp_path):
-    """octet copies: one warp of every CTA takes its first piece as not arrived; the call says so and the next one has all bits"""
+    """octet copies and records of the tensor cores: one warp of every CTA takes its first piece as not arrived; the call says so and the next one has all bits"""
     d = synth.write_model_dir(str(tmp_path / "m"), _shape(quant, 256, 512, 4, 512), seed=3)
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=8)
     assert cm.be.counter("mv32_ok") == 1
     tokens = synth.random_prompt(512, 5, seed=1)
     want = om.forward(tokens)
-    for warp in (0, 3):
+    for mt_min, warp in ((OCTETS, 0), (OCTETS, 3), (2, 0), (2, 3)):
+        cm.be.set_option("mt_min", mt_min)
         cm.be.set_option("give_up_warp", warp)
         with pytest.raises(capi.PsCudaError, match="copy of a batch product"):
             cm.forward(tokens)
@@ -37,6 +39,8 @@ def test_a_warp_that_gives_up_ends_the_call(quant, tmp_path):
 
 
 def _product(be, t, w, K, N, x, bs):
+    """on ps_k_matmul_qb, whatever the format and the size"""
+    be.set_option("mk_min", 1000)
     ref = np.zeros(N * bs, np.float32)
     L.oracle().ps_or_matmul(t, L.vptr(w), K, N, L.fptr(x), bs, L.fptr(ref))
     wd = be.register_weight(w, t, K, N)
@@ -67,7 +71,7 @@ def test_infinite_scale_in_the_last_block(t, blocks):
 
 @pytest.mark.parametrize("quant", [gguf.GGML_Q8_0, gguf.GGML_Q4_0])
 def test_infinite_scale_in_the_head(quant, tmp_path, monkeypatch):
-    """the same on octet copies: rows of the head whose last of five blocks has an infinite scale; a logit is infinite where its eight lanes agree"""
+    """the same on octet copies, and on the tensor cores' records: rows of the head whose last of five blocks has an infinite scale; a logit is infinite where its eight lanes agree"""
     def damaged(shape, seed=0, plain=synth.generate_tensors):
         tensors = plain(shape, seed)
         raw = next(d for n, _, _, d in tensors if n == "output.weight").view(np.uint8).reshape(2048, 5, -1)
@@ -81,9 +85,12 @@ def test_infinite_scale_in_the_head(quant, tmp_path, monkeypatch):
     for bs in (2, 4, 8):
         tokens = synth.random_prompt(2048, bs, seed=bs)
         om.reset()
-        cm.reset()
-        want, got = om.forward(tokens), cm.forward(tokens)
-        assert np.isinf(want).any() and np.array_equal(want, got, equal_nan=True)
+        want = om.forward(tokens)
+        for mt_min in (OCTETS, 2):
+            cm.be.set_option("mt_min", mt_min)
+            cm.reset()
+            got = cm.forward(tokens)
+            assert np.isinf(want).any() and np.array_equal(want, got, equal_nan=True)
     om.close()
     cm.close()
 
@@ -107,12 +114,14 @@ def test_long_octets(quant, ffn, tmp_path):
     ps_k_matmul_qb takes it); two and four columns leave more"""
     d = synth.write_model_dir(str(tmp_path / "m"), _shape(quant, 256, ffn, 4, 512), seed=ffn)
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=8)
+    cm.be.set_option("mt_min", OCTETS)
     assert cm.be.counter("mv32_ok") == 1
     for bs in (2, 3, 8):
         tokens = synth.random_prompt(512, bs, seed=bs)
         om.reset()
         cm.reset()
         L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"ffn {ffn} bs {bs}")
+    assert cm.be.counter("mt_launches") == 0
     om.close()
     cm.close()
 
@@ -137,6 +146,7 @@ def test_rows_too_long_for_eight_octets_of_q8_0(tmp_path):
     shape = synth.ModelShape("q8-long-rows", "llama", 1024, 14336, 1, 16, 2, 64, 264, False, 0, 1e4, 1e-5, gguf.GGML_Q8_0, n_ctx=128)
     d = synth.write_model_dir(str(tmp_path), shape, seed=12)
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=80)
+    cm.be.set_option("mt_min", OCTETS)
     took = {}
     for n in (72, 80):
         tokens = synth.random_prompt(264, n, seed=n)
@@ -150,6 +160,7 @@ def test_rows_too_long_for_eight_octets_of_q8_0(tmp_path):
             cm.forward(tokens, lm_head=False)
             best = min(best, time.perf_counter() - t0)
         took[n] = best
+    assert cm.be.counter("mt_launches") == 0
     om.close()
     cm.close()
     assert took[72] < 1.25 * took[80], took
@@ -162,10 +173,12 @@ def test_four_and_eight_columns_a_warp(tmp_path, quant, dim, ffn):
     shape = synth.ModelShape("columns", "llama", dim, ffn, 1, dim // 64, 2, 64, 264, False, 0, 1e4, 1e-5, quant, n_ctx=128)
     d = synth.write_model_dir(str(tmp_path), shape, seed=13)
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=80)
+    cm.be.set_option("mt_min", OCTETS)
     for n in (5, 12, 32, 48, 65, 72):
         tokens = synth.random_prompt(264, n, seed=n)
         om.reset()
         cm.reset()
         L.assert_bit_equal(cm.forward(tokens), om.forward(tokens), f"{n} tokens")
+    assert cm.be.counter("mt_launches") == 0
     om.close()
     cm.close()

@@ -26,7 +26,9 @@ def _product(be, t, w, K, N, x, bs):
     out = {}
     for mk_min in (2, 1000):
         be.set_option("mk_min", mk_min)
+        launches = be.counter("mk_launches")
         be.matmul(dd, wd, t, K, N, xd, bs)
+        assert be.counter("mk_launches") - launches == (mk_min == 2)
         out[mk_min] = dd.numpy()
     be.set_option("mk_min", 2)
     xd.free()

@@ -20,7 +20,7 @@ def pair(request, tmp_path_factory):
     shape = synth.ModelShape("mt-" + name, "qwen2", dim, ffn, 1, nh, nkv, dim // nh, vocab, True, 2, 1e6, 1e-6, quant, n_ctx=128, qkv_bias=True)
     d = synth.write_model_dir(str(tmp_path_factory.mktemp("mt")), shape, seed=8)
     om, cm = M.OracleModel(d), capi.CudaModel(d, max_batch=70)
-    assert cm.be.counter("mv32_ok") == 1
+    assert cm.be.counter("mv32_ok") == 1 and cm.be.counter("mt_ok") == 1
     yield om, cm, vocab
     om.close()
     cm.close()
@@ -35,7 +35,9 @@ def test_columns(pair, n):
     for mt_min in (2, 1000):
         cm.be.set_option("mt_min", mt_min)
         cm.reset()
+        launches = cm.be.counter("mt_launches")
         L.assert_bit_equal(cm.forward(tokens), want, f"{n} tokens, mt_min {mt_min}")
+        assert cm.be.counter("mt_launches") - launches == (5 if mt_min == 2 else 0)
     cm.be.set_option("mt_min", 2)
 
 
