@@ -342,14 +342,18 @@ __global__ void __launch_bounds__(PT_THREADS, 1) pa_k_tc_gemm(const __grid_const
 
 // ---------------------------------------------------------------------------------------------------- float32 mode
 // The same products without rounding.  The weights are bfloat16 as they are; an activation is cut into three bfloat16 parts, its upper, middle and lower
-// eight significant bits (exact, and no part overflows), so that three MMAs whose products are exact replace the FMAs.  What an MMA loses is the low
-// end of the fp32 accumulator (it truncates where an FMA rounds), and that grows with the number of MMAs an accumulator sees and with its size.  So an accumulator takes ONE
-// k block of 64 - lowest parts first, while it is small, the four MMAs of the upper parts last - and the epilogue adds the blocks' sums in fp32 with
-// rounding.  The order of k is the same for every number of tokens and every portion.
-// Error against 64 bits: logits of two 1024-wide Vanapel layers 8e-7 with FMA tiles, 5.8e-7 so (150 tokens at 300).
+// eight significant bits (no part overflows; exact from 2^-103 up, below which a part may be subnormal and at worst 2^-126 is lost), so that three MMAs whose products are exact
+// replace the FMAs.  What an MMA loses is the low end of the fp32 accumulator (it truncates where an FMA rounds), and that grows with the number of MMAs an accumulator sees and
+// with its size.  So an accumulator takes ONE k block of 64 - lowest parts first, while it is small, the four MMAs of the upper parts last - and the epilogue adds the blocks' sums
+// in fp32 with rounding.  The order of k is the same for every number of tokens and every portion.
+// Error against 64 bits, root mean square over the result's: logits of two 1024-wide Vanapel layers 8e-7 with FMA tiles, 5.8e-7 so (150 tokens at 300); one product of K 512 / 2048 / 8192 with
+// weights of both signs, activations of one sign or two, over a binade or ten: 2.1 / 3.0 / 5.8e-7 and 1.2 / 1.6 / 2.4e-7.  Truncation has a direction: where all products of a sum share a sign it
+// does not average out.  Over one binade that is not seen (K 2048 1.1e-7 and 1.0e-7), over ten the sums are 1.1e-7 short: 1.0 / 1.0 / 1.8e-7 with FMAs, 1.2 / 1.4 / 2.0e-7 so.  Bound: the four upper MMAs
+// of a block lose less than an ulp of 1/4 to 4/4 of its sum, together 2.5 * 2^-23.
 // Bound by the epilogue, which drains an accumulator of TN tokens every 12 MMAs (24 with a gate), and by the copies: a stage of 64 k is 16 KB of weights a
 // matrix and 384 B a token.  A unit is 128 output rows x TN tokens, TN as small as fills the GPU: its epilogue is shorter and the weights come from L2.
-// MEASURED
+// 150 tokens, us with the cutting of the activations: K 1024 x 1024 outputs 12 + 4, K 2048 x 1024 20 + 4, gate | up of 2048 from K 1024 21 + 4, head of 4096 from K 1024 15 + 5 (a pass of two
+// layers 606 -> 370)
 #define PT_SPLIT 3
 template <int TN> PS_HD constexpr int pt_xb() { return PT_SPLIT * TN * PT_KB * 2; } // bytes of a tile's k block: [part][k-chunk of 8][token TN][8]
 // activations -> [column tile][k block][part][k-chunk][token][8]; tiles as in pa_k_tc_prep_x

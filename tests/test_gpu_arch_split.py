@@ -96,3 +96,33 @@ def test_weights_that_are_not_finite(tmp_path):
         got.append(m.forward(toks))
     m.close()
     assert np.array_equal(got[0], got[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("K", [512, 2048, 8192])
+@pytest.mark.parametrize("kind", ["one binade", "ten binades", "ten binades, weights of both signs"])
+def test_products_of_one_sign(tmp_path, K, kind):
+    """logits of positive activations (the layer's own outputs are zeros).  Tensor-core accumulation truncates, which has a direction: an accumulator's four upper MMAs lose less than
+    an ulp of 1/4, 2/4, 3/4 and all of a k block's sum, 2.5 * 2^-23 of it, and on average half of that.  With weights of both signs it averages out, and the FMA tiles are further off"""
+    cfg = arch_synth.vanapel_config(K, 330, [arch_synth.vanapel_attention_layer(4, 2, 32, 32, window=40, ff=128, limit=7.0)], groups=1)
+    t = arch_synth.vanapel_weights(cfg, seed=1)
+    rng = np.random.default_rng(K)
+    t["l0.mix.o"], t["l0.mlp.down"] = np.zeros_like(t["l0.mix.o"]), np.zeros_like(t["l0.mlp.down"])
+    spread = 1.0 if kind == "one binade" else 2.0 ** (-10 * rng.random((330, K)))
+    t["embed"] = _vanapel_ref.bf16_round((1 + rng.random((330, K))) * spread)
+    if "both" not in kind:
+        t["head"] = _vanapel_ref.bf16_round((np.abs(rng.standard_normal((330, K))) + 0.1) / K)
+    d = str(tmp_path / "m")
+    arch_synth.write_model_dir(d, cfg, t)
+    toks = [int(v) for v in rng.integers(0, 330, 64)]
+    want = _vanapel_ref.forward(cfg, t, toks)
+    m = arch.load_model(d, dtype="float32", max_batch=64, n_ctx=80)
+    rms = {}
+    for tc in (0, 1):
+        m.be.set_option("arch_tc", tc)
+        m.reset()
+        off = (m.forward(toks) - want) / np.sqrt((want ** 2).mean(-1, keepdims=True))
+        rms[tc] = np.sqrt((off ** 2).mean())
+        if tc:
+            assert abs(off.mean()) < 2.5 * 2.0 ** -23 / 2 + 2.0 ** -25      # and the norm's own rounding
+    m.close()
+    assert rms[1] < (rms[0] if "both" in kind else 1.5 * rms[0]), rms
