@@ -229,11 +229,13 @@ class _PinnedStore:
         return (p.value, size) if L.ps_cuda_host_alloc_on(device, size, C.byref(p)) == 0 else None
 
     def give(self, L, buf):
+        rest = []
         with self.lock:
-            if len(self.idle) < self.MOST and sum(b[1] for b in self.idle) + buf[1] <= self.BYTES:
-                self.idle.append(buf)
-                return
-        L.ps_cuda_host_free(buf[0])
+            self.idle.append(buf)
+            while len(self.idle) > self.MOST or sum(b[1] for b in self.idle) > self.BYTES:
+                rest.append(self.idle.pop(0))   # the one that has lain longest
+        for b in rest:
+            L.ps_cuda_host_free(b[0])
 
     def clear(self, L):
         with self.lock:

@@ -140,3 +140,19 @@ def test_buffers_are_made_on_the_models_device():
     t.start()
     t.join()
     assert pinned(got[0]) and L.devices == [3]
+
+
+def test_what_has_lain_longest_makes_room():
+    """models of one size come after models of another: their buffers stay, whatever lies there"""
+    L, store = FakeLib(), capi._PinnedStore()
+    for rows in (1, 1, 1, 16):
+        pools = [capi._LogitsPool(L, store) for _ in range(3)]
+        arrays = [p.array(rows, 32768) for p in pools]
+        made = L.made
+        del arrays
+        gc.collect()
+        for p in pools:
+            p.close()
+    assert made == 6 and sorted(b[1] for b in store.idle) == [128 << 10] + 3 * [4 << 20] and len(L.live) == 4
+    pools = [capi._LogitsPool(L, store) for _ in range(3)]
+    assert all(pinned(p.array(16, 32768)) for p in pools) and L.made == made
