@@ -99,7 +99,7 @@ struct PsArch {
     ps_cuda_arch_desc d{};
     std::vector<PsArchLayer> L;
     std::vector<void *> owned;
-    std::vector<void *> spare; // of them, the operand blocks of float32 mode
+    std::vector<void *> spare; // the operand blocks of float32 mode
     bool bound = false, round = true;
     bf16 *embed = nullptr, *head = nullptr;
     float *final_norm = nullptr;
@@ -745,6 +745,7 @@ void ps_arch_destroy(PsArch *a) {
     if (a->ev_join) cudaEventDestroy(a->ev_join);
     if (a->side) cudaStreamDestroy(a->side);
     for (void *p : a->owned) cudaFree(p);
+    for (void *p : a->spare) cudaFree(p);
     delete a;
 }
 
@@ -753,10 +754,7 @@ int64_t ps_arch_split_launches(const PsArch *a) { return a->n_split; }
 bool ps_arch_give_back(PsArch *a, cudaStream_t stream) {
     if (a->spare.empty()) return false;
     cudaStreamSynchronize(stream);
-    for (void *p : a->spare) {
-        a->owned.erase(std::find(a->owned.begin(), a->owned.end(), p));
-        cudaFree(p);
-    }
+    for (void *p : a->spare) cudaFree(p);
     a->spare.clear();
     a->tiled = false; // (the layers' pointers to them are followed on that condition alone)
     return true;
@@ -1138,7 +1136,7 @@ int ps_arch_bind(PsArch *a, const ps_cuda_arch_weights *wt, cudaStream_t stream,
             int r = aalloc(a, (void **)dst, (size_t)groups * n_rt * nkb * PT_BLOCK, err);
             if (r && !a->round) { full = true; return 0; }
             if (r) return r;
-            if (!a->round) a->spare.push_back(*dst);
+            if (!a->round) { a->owned.pop_back(); a->spare.push_back(*dst); }
             pa_k_tc_tile_w<<<dim3((unsigned)n_rt, (unsigned)nkb, (unsigned)groups), 256, 0, stream>>>(*dst, src, N, K, n_rt, nkb, odd);
             PA_CK(cudaGetLastError());
             return 0;

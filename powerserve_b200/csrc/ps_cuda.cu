@@ -257,7 +257,6 @@ bool give_back(ps_cuda_ctx *ctx) {
     bool given = false;
     if (ctx->mt_mem) {
         cudaStreamSynchronize(ctx->stream);
-        ctx->owned.erase(std::find(ctx->owned.begin(), ctx->owned.end(), (void *)ctx->mt_mem));
         given = cudaFree(ctx->mt_mem) == cudaSuccess;
         ctx->mt_mem = nullptr;
         ctx->mt_ok = false;
@@ -1864,6 +1863,7 @@ void ps_cuda_destroy(ps_cuda_ctx *ctx) {
     for (void *p : ctx->pooled) cudaFreeAsync(p, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
     for (void *p : ctx->owned) cudaFree(p);
+    if (ctx->mt_mem) cudaFree(ctx->mt_mem);
     if (ctx->h_tokens) cudaFreeHost(ctx->h_tokens);
     if (ctx->h_ids) cudaFreeHost(ctx->h_ids);
     if (ctx->h_err) cudaFreeHost(ctx->h_err);
@@ -2371,6 +2371,7 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
             PS_CK(cudaMemGetInfo(&free_b, &total_b));
             ctx->mt_ok = d.max_batch > 1 && need + ((size_t)8 << 30) < free_b && dev_alloc(ctx, (void **)&ctx->mt_mem, need) == 0; // (one allocation: seven a layer took longer than the packing)
             if (ctx->mt_ok) {
+                ctx->owned.pop_back(); // (another context's thread may give it back, while calls that take no lock add to the list)
                 uint8_t *at = ctx->mt_mem;
                 auto rec = [&](uint8_t **p, const uint8_t *w, int64_t rows, int64_t K) -> int {
                     *p = at;
