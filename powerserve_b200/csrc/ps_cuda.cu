@@ -2268,6 +2268,7 @@ float *ps_cuda_kv_v(ps_cuda_ctx *ctx, int layer) { return (layer >= 0 && layer <
 // ---------------------------------------------------------------------------------------------- whole model
 int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
     PS_NO_ARCH("ps_cuda_bind_model");
+    std::lock_guard<std::mutex> lock(ctx->mu); // (no other context takes the copies that are being made)
     const ps_cuda_model_desc &d = ctx->d;
     const int64_t qdim = (int64_t)d.n_heads * d.head_size, kvd = (int64_t)d.n_kv_heads * d.head_size;
     auto reg = [&](const ps_cuda_tensor &t, int64_t ne0, int64_t ne1, const void **dev, int *type) -> int {
@@ -2342,6 +2343,7 @@ int ps_cuda_bind_model(ps_cuda_ctx *ctx, const ps_cuda_model_weights *w) {
             if (ld.tq != t0 || ld.tk != t0 || ld.tv != t0 || ld.to != t0 || ld.tgate != t0 || ld.tup != t0 || ld.tdown != t0) same = false;
         if (d.dim % 32 || d.ffn_dim % 32 || qdim % 32 || qdim % 8 || kvd % 8 || d.dim % 8 || d.ffn_dim % 8 || d.vocab_size % 8 || d.head_size % 2) same = false;
         ctx->mv_ok = false;
+        give_back(ctx); // (bound before)
         if (same) {
             ctx->mv_type = t0;
             int rc;

@@ -100,6 +100,14 @@ def test_another_context_takes_their_place(blocks):
     other.close()
 
 
+def test_a_second_bind_keeps_one_copy(blocks):
+    toks = synth.random_prompt(1000, 20, seed=1)
+    want = _both(blocks, toks)
+    blocks.be._ck(blocks.be.L.ps_cuda_bind_model(blocks.be.h, C.byref(blocks._w)))
+    assert blocks.be.counter("mt_ok") == 1
+    L.assert_bit_equal(_both(blocks, toks), want, "bound again")
+
+
 def test_buffers_of_the_operator_table_take_their_place(blocks):
     fill = Filler(12 * MB)
     try:
