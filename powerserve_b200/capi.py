@@ -274,9 +274,11 @@ class _LogitsPool:
         return np.frombuffer(mem, np.float32).reshape(rows, cols)
 
     def _take(self, n: int):
-        small = None
+        small = fit = None
         with self.lock:
-            fit = min((b for b in self.free if b[1] >= n), key=lambda b: b[1], default=None)
+            for b in self.free:
+                if b[1] >= n and (fit is None or b[1] < fit[1]):
+                    fit = b
             if fit is not None:
                 self.free.remove(fit)
                 return fit

@@ -359,18 +359,11 @@ int stage_call(ps_cuda_ctx *ctx, int bs, bool tree = false) {
 // logits of the last pass to the caller; synchronises and checks.  Pinned memory of the caller's is written directly, other memory (of which a part may be pinned) by way of a pinned
 // buffer and a copy on the host, which for a few MB takes longer than the transfer (1.6 MB: 150 us and 30)
 int logits_to_host(ps_cuda_ctx *ctx, float *host, size_t bytes) {
-    auto locked = [](const void *p) {
-        cudaPointerAttributes at{};
-        if (cudaPointerGetAttributes(&at, p) == cudaSuccess) return at.type == cudaMemoryTypeHost;
-        cudaGetLastError();
-        return false;
-    };
-    bool direct = locked(host) && locked(reinterpret_cast<char *>(host) + bytes - 1);
-    if (direct && cudaMemcpyAsync(host, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess) { // locked at its ends alone, or in pieces
-        cudaGetLastError();
-        direct = false;
-    }
+    cudaPointerAttributes at{};
+    bool direct = cudaPointerGetAttributes(&at, host) == cudaSuccess && at.type == cudaMemoryTypeHost &&
+                  cudaMemcpyAsync(host, ctx->logits_last, bytes, cudaMemcpyDeviceToHost, ctx->stream) == cudaSuccess; // (refused where it is pinned at its beginning alone, or in pieces)
     if (!direct) {
+        cudaGetLastError();
         if (bytes > ctx->h_logits_cap) {
             if (ctx->h_logits) cudaFreeHost(ctx->h_logits);
             ctx->h_logits = nullptr;
